@@ -171,34 +171,31 @@ def load_kernel_traffic(path=os.path.join(ROOT, "profiles", "counters_per_kernel
 KERNEL_TRAFFIC = load_kernel_traffic()
 
 
-class LaunchRecorder:
-    """Wraps the C-ABI call so that every kernel launch is counted and bracketed by CUDA events on its stream."""
+# device kernel name -> entry point of the library that launches it
+KERNEL_ENTRY = (("gate_cumsum_fwd", "mkda_gate_cumsum_fwd"), ("gate_bwd", "mkda_gate_bwd"), ("reduce_", "mkda_reduce_partials"),
+                ("l2norm_rstd", "mkda_l2norm_rstd"), ("intra_fwd", "mkda_intra_fwd"), ("recur_fwd", "mkda_recur_fwd"),
+                ("out_fwd", "mkda_out_fwd"), ("epilogue_bwd_tiles", "mkda_epilogue_bwd_tiles"), ("epilogue_bwd", "mkda_epilogue_bwd"),
+                ("bwd_dh", "mkda_bwd_dh"), ("bwd_chunk", "mkda_bwd_chunk"), ("qk_grad_finish", "mkda_qk_grad_finish"),
+                ("combine", "mkda_state_combine"), ("warmup_chunks", "mkda_warmup_chunks"))
 
-    def __init__(self, lib_module):
-        self.lib, self.orig, self.events, self.count, self.timing = lib_module, lib_module.call, [], 0, False
 
-    def __enter__(self):
-        def call(name, params, stream):
-            self.count += 1
-            if not self.timing:
-                return self.orig(name, params, stream)
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            self.orig(name, params, stream)
-            e1.record()
-            self.events.append((name, e0, e1))
-        self.lib.call = call
-        return self
-
-    def __exit__(self, *exc):
-        self.lib.call = self.orig
-
-    def totals(self):
-        out = {}
-        for name, e0, e1 in self.events:
-            ms, n = out.get(name, (0.0, 0))
-            out[name] = (ms + e0.elapsed_time(e1), n + 1)
-        return out
+def kernel_times(step, steps):
+    """Device time of the library's kernels over ``steps`` further steps, from the CUDA activity trace (outside the timed region):
+    {entry point: (ms, launches)}."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        for _ in range(steps):
+            step()
+        torch.cuda.synchronize()
+    out = {}
+    for e in prof.events():
+        if e.device_type != torch.autograd.DeviceType.CUDA or "mkda" not in e.name:
+            continue
+        entry = next((v for k, v in KERNEL_ENTRY if k in e.name), None)
+        if entry:
+            ms, n = out.get(entry, (0.0, 0))
+            out[entry] = (ms + e.time_range.elapsed_us() * 1e-3, n + 1)
+    return out
 
 
 class ClockSampler:
@@ -434,68 +431,66 @@ def main():
             dist.barrier()
         torch.cuda.synchronize()
 
-    with LaunchRecorder(_lib) as rec:
-        for _ in range(args.warmup):
-            layer_step(mk, dev, opts, cp)
-        barrier()
-        sampler = ClockSampler(local)
-        if rank == 0:
-            sampler.start()
-        rec.count, rec.timing = 0, True
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        for _ in range(args.steps):
-            layer_step(mk, dev, opts, cp)
-        e1.record()
-        barrier()
-        ms = e0.elapsed_time(e1)
-        launches = rec.count
-        rec.timing = False
-        per_kernel = rec.totals()
-        # end to end: pinned host inputs in, loss out, every step.  As in a training loop with a prefetching loader the
-        # next step's inputs travel on a second stream while the current step computes; all K copies and K loss
-        # read-backs are inside the timed region (the first copy has nothing to hide behind).
-        copy_stream = torch.cuda.Stream()
+    for _ in range(args.warmup):
+        layer_step(mk, dev, opts, cp)
+    barrier()
+    sampler = ClockSampler(local)
+    if rank == 0:
+        sampler.start()
+    launches = _lib.launch_count()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    for _ in range(args.steps):
+        layer_step(mk, dev, opts, cp)
+    e1.record()
+    barrier()
+    ms = e0.elapsed_time(e1)
+    launches = _lib.launch_count() - launches
+    per_kernel = kernel_times(lambda: layer_step(mk, dev, opts, cp), args.steps)
+    # end to end: pinned host inputs in, loss out, every step.  As in a training loop with a prefetching loader the
+    # next step's inputs travel on a second stream while the current step computes; all K copies and K loss
+    # read-backs are inside the timed region (the first copy has nothing to hide behind).
+    copy_stream = torch.cuda.Stream()
 
-        def upload():
-            with torch.cuda.stream(copy_stream):
-                t = {n: x.to(device, non_blocking=True) for n, x in host.items()}
-                ev = torch.cuda.Event()
-                ev.record(copy_stream)
-            return t, ev
+    def upload():
+        with torch.cuda.stream(copy_stream):
+            t = {n: x.to(device, non_blocking=True) for n, x in host.items()}
+            ev = torch.cuda.Event()
+            ev.record(copy_stream)
+        return t, ev
 
-        def e2e_steps(n):
-            nxt = upload()
-            for i in range(n):
-                cur, ev = nxt
-                torch.cuda.current_stream().wait_event(ev)
-                if i + 1 < n:
-                    nxt = upload()
-                loss = layer_step(mk, cur, opts, cp)
-                for x in cur.values():
-                    x.record_stream(torch.cuda.current_stream())
-                loss.item()
+    def e2e_steps(n):
+        nxt = upload()
+        for i in range(n):
+            cur, ev = nxt
+            torch.cuda.current_stream().wait_event(ev)
+            if i + 1 < n:
+                nxt = upload()
+            loss = layer_step(mk, cur, opts, cp)
+            for x in cur.values():
+                x.record_stream(torch.cuda.current_stream())
+            loss.item()
 
-        e2e_steps(2)
-        barrier()
-        # the plain pinned-host -> device copy rate of the same buffers, all ranks at once, for attribution of `e2e`
-        c0, c1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        c0.record()
-        for _ in range(3):
-            tmp = {n: x.to(device, non_blocking=True) for n, x in host.items()}
-        c1.record()
-        barrier()
-        ms_copy = c0.elapsed_time(c1) / 3
-        del tmp
-        f0, f1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        f0.record()
-        e2e_steps(args.steps)
-        f1.record()
-        barrier()
-        ms_e2e = f0.elapsed_time(f1)
-        clocks = sampler.stop() if rank == 0 else None
-        if _lib.device_status() != 0:
-            raise SystemExit("a bounded wait inside a tensor-core kernel expired: the run is invalid")
+    e2e_steps(2)
+    barrier()
+    # the plain pinned-host -> device copy rate of the same buffers, all ranks at once, for attribution of `e2e`
+    c0, c1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    c0.record()
+    for _ in range(3):
+        tmp = {n: x.to(device, non_blocking=True) for n, x in host.items()}
+    c1.record()
+    barrier()
+    ms_copy = c0.elapsed_time(c1) / 3
+    del tmp
+    f0, f1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    f0.record()
+    e2e_steps(args.steps)
+    f1.record()
+    barrier()
+    ms_e2e = f0.elapsed_time(f1)
+    clocks = sampler.stop() if rank == 0 else None
+    if _lib.device_status() != 0:
+        raise SystemExit("a bounded wait inside a tensor-core kernel expired: the run is invalid")
 
     tms = torch.tensor([ms, ms_e2e, ms_copy], device=device, dtype=torch.float64)
     if world > 1:

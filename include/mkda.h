@@ -151,12 +151,14 @@ typedef struct {
     int state_v_first;         /* layout of h0 / ht */
     float* h;                  /* [NC,HV] state tiles: state entering each chunk, or NULL */
     float* Vd;                 /* [NC,HV] chunk tiles: Vd^T, or NULL */
-    float* ht;                 /* [NS,HV,128,128] state leaving each segment, or NULL */
+    float* ht;                 /* [NS or rows of seg_ht,HV,128,128] state leaving each segment, or NULL */
     int want_transition;
     float* mt;                 /* [NS,HV,128,128] transition (row = output K index), needs want_transition */
     const int* warm_start;     /* [NS,HV] from mkda_warmup_chunks, or NULL.  A pass from zero (the segment pre-pass) may start
                                 * at this chunk instead of the segment's first one; where it does, the transition is written
                                 * as zero without being computed. */
+    const int* seg_ht;         /* [NS] row of ht for each segment, -1 = do not store; NULL = identity map */
+    int h0_k_first;            /* 1: h0 is [K,V] whatever state_v_first says (states handed between segments) */
 } MkdaRecurFwd;
 int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream);
 
@@ -326,6 +328,7 @@ typedef struct {
     int reverse;
     float* s_in;               /* [NS,HV,128,128] value entering each segment ([K,V]), or NULL */
     float* s_out;              /* [NG,HV,128,128] value leaving the last (first) segment of each group, or NULL */
+    int carry_v_first; int out_v_first;            /* 1: carry / s_out are [V,K] */
 } MkdaCombine;
 int mkda_state_combine(const MkdaCombine* p, void* stream);
 
@@ -376,6 +379,8 @@ int mkda_device_status(void);
 int mkda_device_status_clear(void);
 
 const char* mkda_last_error(void);
+/* kernel launches issued by this process through the library so far */
+unsigned long long mkda_launch_count(void);
 int mkda_abi_version(void);
 /* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header. */
 int mkda_struct_sizes(int* out, int n);

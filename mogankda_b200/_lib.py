@@ -5,6 +5,7 @@ sizes are checked against ``mkda_struct_sizes`` when the library is loaded.  The
 missing or stale the import of the kernels fails with the build command in the message.
 """
 import ctypes
+import importlib.util
 import os
 import re
 
@@ -63,6 +64,7 @@ class MkdaError(RuntimeError):
 
 
 _libs = {}
+_host = None
 
 
 def load():
@@ -86,6 +88,27 @@ def load():
         raise MkdaError(f"{path} does not match include/mkda.h (struct sizes differ): rebuild with `python -m mogankda_b200.build --force`")
     _libs[variant] = lib
     return lib
+
+
+def host():
+    """The native host path (``_host.so``: argument checks, buffers, launches, autograd node)."""
+    global _host
+    if _host is None:
+        load()                      # checks that the library matches the header before anything is launched through it
+        path = os.path.join(HERE, "_host.so")
+        if not os.path.exists(path):
+            raise MkdaError(f"{path} is missing: build it with `python -m mogankda_b200.build` (no CPU or library fallback exists)")
+        spec = importlib.util.spec_from_file_location("mogankda_b200._host", path)
+        _host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_host)
+    return _host
+
+
+def launch_count():
+    """Kernel launches issued through the library by this process so far."""
+    lib = load()
+    lib.mkda_launch_count.restype = ctypes.c_ulonglong
+    return int(lib.mkda_launch_count())
 
 
 def call(name, params, stream):

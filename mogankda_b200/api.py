@@ -15,7 +15,7 @@ Differences that are extensions, not changes of meaning:
 """
 import torch
 
-from . import ops
+from . import _lib, ops
 from .index import get_layout
 
 CHUNK_SIZE = 64
@@ -25,17 +25,18 @@ CHUNK_SIZE = 64
 AUTO_SEGMENT_CHUNKS = 32
 
 
-class _DeltaRuleFunction(torch.autograd.Function):
-    """forward: gate + cumsum (+beta) -> L2 statistics -> WY preparation -> state pass -> output (+epilogue).
+class _ContextParallelFunction(torch.autograd.Function):
+    """A call whose sequences continue on other ranks: the launches of the native host path (csrc/layer.cpp), with the exchange of
+    ``cp_context`` between the segment pre-pass and the main pass of each direction.
+
+    forward: gate + cumsum (+beta) -> L2 statistics -> WY preparation -> state pass -> output (+epilogue).
     backward: epilogue -> reverse state chain -> WY / state gradients -> intra-chunk gradients -> gate / L2 / GVA."""
 
     @staticmethod
     def forward(ctx, q, k, v, x, beta, A_log, dt_bias, initial_state, ep_w, ep_gate, cfg):
         B, T, HK, K = q.shape
         HV = v.shape[2]
-        dev = q.device
-        lay = get_layout(B, T, cfg["cu_seqlens"], dev, cfg["seg_chunks"], HV if cfg["seg_auto"] else 0,
-                         2.5 if cfg["warmup"] is None else 1.25)
+        lay = get_layout(B, T, cfg["cu_seqlens"], q.device, AUTO_SEGMENT_CHUNKS)
         cp = cfg["cp_context"]
         scale = cfg["scale"]
         q_rstd = k_rstd = None
@@ -48,30 +49,24 @@ class _DeltaRuleFunction(torch.autograd.Function):
                                                     scalar_gate=x.dim() == 3)
         vf = cfg["state_v_first"]
         need_ht = cfg["output_final_state"]
-        ms = m_first = warm_end = None
-        if lay.segmented or cp is not None:
-            # pre-pass from zero: per-segment (state, transition); then the true entering state of every segment
-            warm_start = None
-            if cfg["warmup"] is not None:
-                warm_start, warm_end = ops.warmup_chunks(lay, gl, HK, HV, cfg["warmup"])
-            _, _, hs, ms = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV, store_h=False, store_vd=False,
-                                         want_transition=True, warm_start=warm_start)
-            carry = None
-            if initial_state is not None:
-                carry = initial_state.transpose(-1, -2).contiguous() if vf else initial_state
-            if cp is not None:
-                carry, m_first = cp.forward_carry(hs, ms, carry, lay, HV)
-            s_in, _ = ops.state_combine(lay.grp_seg_off, lay.NG, lay.NS, HV, hs, ms, carry=carry, want_out=False)
-            h, Vd, ht_seg, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV, h0=s_in, state_v_first=False,
-                                             want_ht=need_ht)
-            ht = None
-            if need_ht:
-                ht = ht_seg.index_select(0, torch.nonzero(lay.seg_last >= 0).flatten())
-                if vf:
-                    ht = ht.transpose(-1, -2).contiguous()
-        else:
-            h, Vd, ht, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV, h0=initial_state, state_v_first=vf,
+        # pre-pass from zero: per-segment (state, transition); then the true entering state of every segment
+        warm_start = warm_end = None
+        if cfg["warmup"] is not None:
+            warm_start, warm_end = ops.warmup_chunks(lay, gl, HK, HV, cfg["warmup"])
+        _, _, hs, ms = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV, store_h=False, store_vd=False,
+                                     want_transition=True, warm_start=warm_start)
+        carry = None
+        if initial_state is not None:
+            carry = initial_state.transpose(-1, -2).contiguous() if vf else initial_state
+        carry, m_first = cp.forward_carry(hs, ms, carry, lay, HV)
+        s_in, _ = ops.state_combine(lay.grp_seg_off, lay.NG, lay.NS, HV, hs, ms, carry=carry, want_out=False)
+        h, Vd, ht_seg, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV, h0=s_in, state_v_first=False,
                                          want_ht=need_ht)
+        ht = None
+        if need_ht:
+            ht = ht_seg[[i for i, n in enumerate(lay.host["seg_last"]) if n >= 0]]
+            if vf:
+                ht = ht.transpose(-1, -2).contiguous()
         norm = None
         if cfg["has_ep"]:
             norm = dict(weight=ep_w, gate=ep_gate, act=cfg["ep_act"], eps=cfg["ep_eps"])
@@ -108,26 +103,19 @@ class _DeltaRuleFunction(torch.autograd.Function):
         if dht is not None:
             dht = ops.aligned(dht.float())
         need_dh0 = initial_state is not None and ctx.needs_input_grad[7]
-        if lay.segmented or cp is not None:
-            # pre-pass from zero: only the gradient entering each segment is wanted, nothing per chunk is stored
-            _, _, _, dloc = ops.bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, store=False, dO_in_t=dO_in,
-                                       warm_end=warm_end)
-            carry = None
-            if dht is not None:
-                carry = dht.transpose(-1, -2).contiguous() if vf else dht
-            if cp is not None:
-                carry = cp.backward_carry(dloc, ms, carry, lay, HV, m_first)
-            g_in, dh0 = ops.state_combine(lay.grp_seg_off, lay.NG, lay.NS, HV, dloc, ms, carry=carry, reverse=True,
-                                          want_out=need_dh0 or cp is not None)
-            dh, dVd_t, dO_t, _ = ops.bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, dht=g_in, want_dh0=False,
-                                            dO_in_t=dO_in)
-            if cp is not None:
-                dh0 = cp.finish_backward(dh0)
-            if dh0 is not None and vf:
-                dh0 = dh0.transpose(-1, -2).contiguous()
-        else:
-            dh, dVd_t, dO_t, dh0 = ops.bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, dht=dht,
-                                              state_v_first=vf, want_dh0=need_dh0, dO_in_t=dO_in)
+        # pre-pass from zero: only the gradient entering each segment is wanted, nothing per chunk is stored
+        _, _, _, dloc = ops.bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, store=False, dO_in_t=dO_in,
+                                   warm_end=warm_end)
+        carry = None
+        if dht is not None:
+            carry = dht.transpose(-1, -2).contiguous() if vf else dht
+        carry = cp.backward_carry(dloc, ms, carry, lay, HV, m_first)
+        g_in, dh0 = ops.state_combine(lay.grp_seg_off, lay.NG, lay.NS, HV, dloc, ms, carry=carry, reverse=True)
+        dh, dVd_t, dO_t, _ = ops.bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, dht=g_in, want_dh0=False,
+                                        dO_in_t=dO_in)
+        dh0 = cp.finish_backward(dh0)
+        if dh0 is not None and vf:
+            dh0 = dh0.transpose(-1, -2).contiguous()
         dq_v, dk_v, dgp, dbeta, dv = ops.bwd_chunk(lay, q, k, v, q_rstd, k_rstd, g_c, beta_e, A, h, dh, Vd, dO_t, dVd_t,
                                                    scale, HK, HV, beta, cfg["beta_mode"] == "sigmoid", cfg["beta_scale"],
                                                    scalar_gate=x.dim() == 3)
@@ -146,32 +134,6 @@ class _DeltaRuleFunction(torch.autograd.Function):
         return (dq, dk, dv, dx, dbeta.view_as(beta), d_alog, d_bias, dh0, dw, dgate, None)
 
 
-def _check_common(q, k, v, g, beta, initial_state, cu_seqlens):
-    if not (q.is_cuda and k.is_cuda and v.is_cuda):
-        raise RuntimeError("mogankda_b200 runs on CUDA tensors only (no CPU fallback)")
-    assert q.dtype == k.dtype == v.dtype, "q, k, v must share a dtype"
-    assert q.dtype in (torch.bfloat16, torch.float16, torch.float32), "q, k, v must be bfloat16, float16 or float32"
-    assert q.shape == k.shape and q.dim() == 4 and v.dim() == 4, "q, k [B,T,HK,K]; v [B,T,HV,V]"
-    assert q.shape[-1] == v.shape[-1] == 128, "head dims must be 128"
-    assert v.shape[:2] == q.shape[:2], "q and v disagree on [B,T]"
-    assert v.shape[2] % q.shape[2] == 0, "GVA needs HV % HK == 0"
-    assert g.shape[:3] == v.shape[:3] and (g.dim() == 3 or (g.dim() == 4 and g.shape[3] == 128)), \
-        "g must be [B,T,HV] or [B,T,HV,128]"
-    assert beta.shape == v.shape[:3], "beta must be [B,T,HV]"
-    if cu_seqlens is not None:
-        if q.shape[0] != 1:
-            raise ValueError(f"The batch size is expected to be 1 rather than {q.shape[0]} when using `cu_seqlens`.")
-        n = cu_seqlens.numel() - 1
-    else:
-        n = q.shape[0]
-    if initial_state is not None:
-        assert initial_state.dtype == torch.float32, "initial_state must be float32"
-        if initial_state.shape[0] != n:
-            raise ValueError(f"The number of initial states is expected to be equal to the number of input "
-                             f"sequences, i.e., {n} rather than {initial_state.shape[0]}.")
-        assert tuple(initial_state.shape[1:]) == (v.shape[2], 128, 128), "initial_state must be [N,HV,128,128]"
-
-
 def chunk_delta_rule(q, k, v, g, beta, *, scale=None, initial_state=None, output_final_state=False, cu_seqlens=None,
                      state_v_first=False, gate_mode="precomputed", A_log=None, dt_bias=None, lower_bound=-5.0,
                      beta_mode="precomputed", beta_scale=1.0, use_qk_l2norm_in_kernel=False, output_norm=None,
@@ -184,8 +146,10 @@ def chunk_delta_rule(q, k, v, g, beta, *, scale=None, initial_state=None, output
     """
     if cp_context is not None and getattr(cp_context, "cu_seqlens", None) is not None:
         cu_seqlens = cp_context.cu_seqlens      # the context's local boundaries replace the argument (reference :87-120)
-    _check_common(q, k, v, g, beta, initial_state, cu_seqlens)
-    if gate_mode not in ops.GATE_MODES:
+    host = _lib.host()
+    B, T, HV, _ = host.check(q, k, v, g, beta, initial_state, cu_seqlens)
+    mode = ops.GATE_MODES.get(gate_mode)
+    if mode is None:
         raise ValueError(f"unknown gate_mode {gate_mode!r}")
     if beta_mode not in ("precomputed", "sigmoid"):
         raise ValueError(f"unknown beta_mode {beta_mode!r}")
@@ -193,33 +157,36 @@ def chunk_delta_rule(q, k, v, g, beta, *, scale=None, initial_state=None, output
         assert A_log is not None, "gate_mode='gdn' needs A_log"
         if lower_bound is None and g.dim() == 4:
             lower_bound = -5.0          # the per-channel kernels rely on g >= -5 (reference :338-339)
-    if gate_mode == "eda":
+    elif gate_mode == "eda":
         assert A_log is not None and lower_bound is not None, "gate_mode='eda' needs A_log and lower_bound"
-    if gate_mode == "kimi":
+    elif gate_mode == "kimi":
         assert lower_bound is not None, "gate_mode='kimi' needs lower_bound"
     ep = output_norm
-    if ep is not None and ep.get("act", "silu") not in ops.ACTS:
-        raise ValueError(f"unknown act {ep.get('act')!r}")
-    if cp_context is not None and q.shape[0] != 1:
-        raise ValueError("inter-card CP requires B==1 (varlen).")
+    ep_gate = ep_w = act = eps = None
+    if ep is not None:
+        ep_gate, ep_w, act, eps = ep["gate"], ep.get("weight"), ops.ACTS.get(ep.get("act", "silu")), ep.get("eps", 1e-6)
+        if act is None:
+            raise ValueError(f"unknown act {ep.get('act')!r}")
     if warmup_threshold is not None and not float(warmup_threshold) < 0.0:
         raise ValueError("warmup_threshold must be negative (natural-log units, e.g. -10.0) or None")
-    B, T = q.shape[:2]
-    cfg = dict(scale=float(q.shape[-1] ** -0.5 if scale is None else scale), output_final_state=output_final_state,
-               cu_seqlens=cu_seqlens, state_v_first=state_v_first, gate_mode=gate_mode, lower_bound=lower_bound,
-               beta_mode=beta_mode, beta_scale=float(beta_scale), l2=use_qk_l2norm_in_kernel, has_ep=ep is not None,
-               ep_act=None if ep is None else ep.get("act", "silu"),
-               ep_eps=None if ep is None else ep.get("eps", 1e-6),
-               seg_chunks=AUTO_SEGMENT_CHUNKS if (cp_context is not None or auto_cp) else 0,
-               seg_auto=cp_context is None,          # without CP the chooser in index.wants_segments decides
+    scale = 128 ** -0.5 if scale is None else float(scale)
+    if cp_context is None:
+        # without context parallelism the chooser in index.wants_segments decides whether sequences are cut
+        lay = get_layout(B, T, cu_seqlens, q.device, AUTO_SEGMENT_CHUNKS if auto_cp else 0, HV, 2.5 if warmup_threshold is None else 1.25)
+        return host.layer(q, k, v, g, beta, A_log, dt_bias, initial_state, ep_w, ep_gate, lay.tables, lay.dims, scale, output_final_state,
+                          state_v_first, mode, lower_bound, beta_mode == "sigmoid", beta_scale, use_qk_l2norm_in_kernel, act, eps,
+                          warmup_threshold)
+    if B != 1:
+        raise ValueError("inter-card CP requires B==1 (varlen).")
+    cfg = dict(scale=scale, output_final_state=output_final_state, cu_seqlens=cu_seqlens, state_v_first=state_v_first, gate_mode=gate_mode,
+               lower_bound=lower_bound, beta_mode=beta_mode, beta_scale=float(beta_scale), l2=use_qk_l2norm_in_kernel, has_ep=ep is not None,
+               ep_act=None if ep is None else ep.get("act", "silu"), ep_eps=eps,
                cp_context=cp_context, warmup=None if warmup_threshold is None else float(warmup_threshold))
-    ep_gate = None if ep is None else ep["gate"]
-    ep_w = None if ep is None else ep.get("weight")
     # contiguous and 16-byte aligned operands (a contiguous view at an odd storage offset is copied): what the kernels'
     # vector loads and bulk copies need; the small parameter tensors are realigned where they are used
     al = ops.aligned
-    return _DeltaRuleFunction.apply(al(q), al(k), al(v), al(g), al(beta), A_log, dt_bias, al(initial_state), ep_w,
-                                    al(ep_gate), cfg)
+    return _ContextParallelFunction.apply(al(q), al(k), al(v), al(g), al(beta), A_log, dt_bias, al(initial_state), ep_w,
+                                          al(ep_gate), cfg)
 
 
 def chunk_kda(q, k, v, g, beta, **kwargs):

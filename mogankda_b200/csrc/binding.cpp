@@ -1,0 +1,207 @@
+// The autograd node of a layer call and its Python entry points.
+//
+// Why native: on a short sequence a call is nothing but launches.  Driving the C ABI from Python (ctypes structs, a dozen torch.empty
+// calls, a Python autograd function) took 145 us per forward and 380 us per forward + backward of a 77- / 256-token call whose kernels
+// need 45 / 120 us.
+#include <Python.h>
+
+#include "layer.h"
+
+#include <c10/cuda/CUDAGuard.h>
+#include <pybind11/pybind11.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/edge.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/grad_mode.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include <memory>
+#include <string>
+
+using namespace mkda_host;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+// The inputs are saved as variables (in-place changes are detected, a second backward pass is refused once the buffers are gone), the
+// intermediates as plain memory.
+constexpr int NUM_INPUTS = 10;
+struct DeltaRuleBackward : public torch::autograd::Node {
+    Call call;
+    SavedVariable vars[NUM_INPUTS];
+    std::unique_ptr<Saved> saved;
+
+    std::string name() const override { return "DeltaRuleBackward"; }
+    void release_variables() override {
+        for (auto& v : vars) v.reset_data();
+        saved.reset();
+    }
+    variable_list apply(variable_list&& grads) override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        Inputs in;
+        Tensor* slots[NUM_INPUTS] = {&in.q, &in.k, &in.v, &in.x, &in.beta, &in.A_log, &in.dt_bias, &in.h0, &in.ep_w, &in.ep_gate};
+        for (int i = 0; i < NUM_INPUTS; ++i) *slots[i] = vars[i].unpack();
+        TORCH_CHECK(saved, torch::autograd::ERR_BACKWARD_TWICE);
+        c10::cuda::CUDAGuard guard(call.dev);
+        const Tensor dy = grads[0], dht = grads.size() > 1 ? grads[1] : Tensor();
+        const bool twice = c10::GradMode::is_enabled() && ((dy.defined() && dy.requires_grad()) || (dht.defined() && dht.requires_grad()));
+        Grads g;
+        {
+            at::AutoGradMode off(false);
+            g = run_backward(call, in, *saved, dy, dht, in.A_log.defined() && task_should_compute_output(5),
+                             in.dt_bias.defined() && task_should_compute_output(6), task_should_compute_output(7));
+        }
+        variable_list out = {g.q, g.k, g.v, g.x, g.beta, g.A_log, g.dt_bias, g.h0, g.ep_w, g.ep_gate};
+        for (int i = 0; i < NUM_INPUTS; ++i)
+            if (!task_should_compute_output(i)) out[i] = Tensor();
+        if (twice) {      // gradients of these gradients are not provided: using them has to fail, not to give zeros
+            auto err = std::make_shared<torch::autograd::Error>("chunk_delta_rule: double backward is not supported", torch::autograd::edge_list());
+            for (auto& t : out)
+                if (t.defined()) torch::autograd::set_history(t, err);
+        }
+        return out;
+    }
+};
+
+PyObject* fail(PyObject* type, const std::string& msg) {
+    PyErr_SetString(type, msg.c_str());
+    return nullptr;
+}
+#define REQUIRE(cond, msg) do { if (!(cond)) return fail(PyExc_AssertionError, msg); } while (0)
+
+bool tensor_arg(PyObject* o, Tensor& t) {
+    if (o == Py_None) return true;
+    if (!THPVariable_Check(o)) { PyErr_Format(PyExc_TypeError, "expected a tensor, got %s", Py_TYPE(o)->tp_name); return false; }
+    t = THPVariable_Unpack(o);
+    return true;
+}
+const char NEED_CUDA[] = "mogankda_b200 kernels need CUDA tensors (there is no CPU fallback)";
+
+// check(q, k, v, g, beta, initial_state, cu_seqlens) -> (B, T, HV, device index); raises what the call has to raise
+PyObject* check(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 7) return fail(PyExc_TypeError, "check takes 7 arguments");
+    Tensor q, k, v, g, beta, h0, cu;
+    Tensor* t[7] = {&q, &k, &v, &g, &beta, &h0, &cu};
+    for (int i = 0; i < 7; ++i) {
+        if (!tensor_arg(a[i], *t[i])) return nullptr;
+        if (i < 5 && !t[i]->defined()) return fail(PyExc_TypeError, "q, k, v, g and beta must be tensors");
+    }
+    if (!(q.is_cuda() && k.is_cuda() && v.is_cuda())) return fail(PyExc_RuntimeError, "mogankda_b200 runs on CUDA tensors only (no CPU fallback)");
+    REQUIRE(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(), "q, k, v must share a dtype");
+    REQUIRE(q.scalar_type() == at::kBFloat16 || q.scalar_type() == at::kHalf || q.scalar_type() == at::kFloat, "q, k, v must be bfloat16, float16 or float32");
+    REQUIRE(q.dim() == 4 && v.dim() == 4 && q.sizes() == k.sizes(), "q, k [B,T,HK,K]; v [B,T,HV,V]");
+    REQUIRE(q.size(3) == 128 && v.size(3) == 128, "head dims must be 128");
+    REQUIRE(v.size(0) == q.size(0) && v.size(1) == q.size(1), "q and v disagree on [B,T]");
+    REQUIRE(q.size(2) > 0 && v.size(2) % q.size(2) == 0, "GVA needs HV % HK == 0");
+    REQUIRE((g.dim() == 3 || (g.dim() == 4 && g.size(3) == 128)) && g.size(0) == v.size(0) && g.size(1) == v.size(1) && g.size(2) == v.size(2),
+            "g must be [B,T,HV] or [B,T,HV,128]");
+    REQUIRE(beta.dim() == 3 && beta.size(0) == v.size(0) && beta.size(1) == v.size(1) && beta.size(2) == v.size(2), "beta must be [B,T,HV]");
+    int64_t rows = q.size(0);
+    if (cu.defined()) {
+        if (rows != 1)
+            return fail(PyExc_ValueError, "The batch size is expected to be 1 rather than " + std::to_string(rows) + " when using `cu_seqlens`.");
+        rows = cu.numel() - 1;
+    }
+    if (h0.defined()) {
+        REQUIRE(h0.scalar_type() == at::kFloat, "initial_state must be float32");
+        if (h0.dim() < 1 || h0.size(0) != rows)
+            return fail(PyExc_ValueError, "The number of initial states is expected to be equal to the number of input sequences, i.e., " +
+                                              std::to_string(rows) + " rather than " + std::to_string(h0.dim() ? h0.size(0) : 0) + ".");
+        REQUIRE(h0.dim() == 4 && h0.size(1) == v.size(2) && h0.size(2) == 128 && h0.size(3) == 128, "initial_state must be [N,HV,128,128]");
+    }
+    return Py_BuildValue("(LLLi)", (long long)q.size(0), (long long)q.size(1), (long long)v.size(2), (int)q.device().index());
+    END_HANDLE_TH_ERRORS
+}
+
+// layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all), scale, want_ht,
+//       v_first, gate mode, lower bound or None, beta sigmoid, beta scale, l2, act or None, eps, warm-up threshold or None) -> (o, ht or None)
+PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 23) return fail(PyExc_TypeError, "layer takes 23 arguments");
+    Inputs in;
+    Tensor* slots[NUM_INPUTS] = {&in.q, &in.k, &in.v, &in.x, &in.beta, &in.A_log, &in.dt_bias, &in.h0, &in.ep_w, &in.ep_gate};
+    for (int i = 0; i < NUM_INPUTS; ++i)
+        if (!tensor_arg(a[i], *slots[i])) return nullptr;
+    Tensor tables;
+    if (!tensor_arg(a[10], tables)) return nullptr;
+    Call c;
+    int seg, all;
+    if (!PyArg_ParseTuple(a[11], "iiiii", &c.NC, &c.NS, &c.N, &seg, &all)) return nullptr;
+    c.segmented = seg; c.covers_all = all;
+    c.B = (int)in.q.size(0); c.T = (int)in.q.size(1); c.HK = (int)in.q.size(2); c.HV = (int)in.v.size(2); c.TT = c.B * c.T;
+    c.dev = in.q.device();
+    c.scale = (float)PyFloat_AsDouble(a[12]);
+    c.want_ht = PyObject_IsTrue(a[13]); c.vf = PyObject_IsTrue(a[14]);
+    c.mode = (int)PyLong_AsLong(a[15]);
+    c.lower_bound = a[16] == Py_None ? -3.0e38f : (float)PyFloat_AsDouble(a[16]);
+    c.beta_sigmoid = PyObject_IsTrue(a[17]); c.beta_scale = (float)PyFloat_AsDouble(a[18]); c.l2 = PyObject_IsTrue(a[19]);
+    c.has_ep = a[20] != Py_None;
+    c.act = c.has_ep ? (int)PyLong_AsLong(a[20]) : 0;
+    c.eps = c.has_ep ? (float)PyFloat_AsDouble(a[21]) : 0.f;
+    c.warm = a[22] != Py_None;
+    c.warm_log2 = c.warm ? (float)(PyFloat_AsDouble(a[22]) * 1.4426950408889634) : 0.f;
+    if (PyErr_Occurred()) return nullptr;
+    c.scalar_gate = in.x.dim() == 3;
+    c.qkv_dtype = dtype_code(in.q);
+    dtype_code(in.x); dtype_code(in.beta);
+    if (c.has_ep) {
+        REQUIRE(in.ep_gate.defined(), "the gated norm needs a gate tensor");
+        dtype_code(in.ep_gate);
+        if (in.ep_w.defined()) dtype_code(in.ep_w);
+    }
+    for (Tensor* t : slots)
+        if (t->defined() && !t->is_cuda()) return fail(PyExc_RuntimeError, NEED_CUDA);
+    c.set_tables(tables);
+
+    Tensor out, ht;
+    {
+        pybind11::gil_scoped_release nogil;
+        c10::cuda::CUDAGuard guard(c.dev);
+        for (Tensor* t : {&in.q, &in.k, &in.v, &in.x, &in.beta, &in.h0, &in.ep_gate}) *t = aligned(*t);
+        bool any = false;
+        if (c10::GradMode::is_enabled())
+            for (Tensor* t : slots) any = any || (t->defined() && t->requires_grad());
+        auto saved = std::make_unique<Saved>();
+        std::shared_ptr<DeltaRuleBackward> node;
+        if (any) {
+            node = std::shared_ptr<DeltaRuleBackward>(new DeltaRuleBackward(), torch::autograd::deleteNode);
+            node->set_next_edges(torch::autograd::collect_next_edges(in.q, in.k, in.v, in.x, in.beta, in.A_log, in.dt_bias, in.h0, in.ep_w, in.ep_gate));
+            for (int i = 0; i < NUM_INPUTS; ++i) node->vars[i] = SavedVariable(*slots[i], false);
+        }
+        {
+            at::AutoGradMode off(false);
+            std::tie(out, ht) = run_forward(c, in, any, *saved);
+        }
+        if (any) {
+            node->call = c;
+            node->saved = std::move(saved);
+            torch::autograd::set_history(out, node);
+            if (ht.defined()) torch::autograd::set_history(ht, node);
+        }
+    }
+    PyObject* po = THPVariable_Wrap(out);
+    if (!po) return nullptr;
+    PyObject* ph = Py_None;
+    if (ht.defined()) ph = THPVariable_Wrap(ht);
+    else Py_INCREF(ph);
+    PyObject* res = ph ? PyTuple_Pack(2, po, ph) : nullptr;
+    Py_DECREF(po);
+    Py_XDECREF(ph);
+    return res;
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"check", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check)), METH_FASTCALL, "argument checks of a call"},
+    {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer)), METH_FASTCALL, "one layer call"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "host path of a layer call over libmkda", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }

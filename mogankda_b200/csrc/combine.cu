@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256, 1) combine_kernel(const MkdaCombine p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int kk = (e & 2) ? kr1 : kr0, cc = col0 + nt * 8 + 2 * t + (e & 1);
-                X[nt][e] = src ? src[(size_t)kk * DV + cc] : 0.f;
+                X[nt][e] = src ? (p.carry_v_first ? src[(size_t)cc * DK + kk] : src[(size_t)kk * DV + cc]) : 0.f;
             }
     }
     const int s_beg = p.grp_seg_off[grp], s_end = p.grp_seg_off[grp + 1], n = s_end - s_beg;
@@ -100,8 +100,13 @@ __global__ void __launch_bounds__(256, 1) combine_kernel(const MkdaCombine p) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const int cc = col0 + nt * 8 + 2 * t;
-            *reinterpret_cast<float2*>(out + (size_t)kr0 * DV + cc) = make_float2(X[nt][0], X[nt][1]);
-            *reinterpret_cast<float2*>(out + (size_t)kr1 * DV + cc) = make_float2(X[nt][2], X[nt][3]);
+            if (p.out_v_first) {
+                out[(size_t)cc * DK + kr0] = X[nt][0]; out[(size_t)(cc + 1) * DK + kr0] = X[nt][1];
+                out[(size_t)cc * DK + kr1] = X[nt][2]; out[(size_t)(cc + 1) * DK + kr1] = X[nt][3];
+            } else {
+                *reinterpret_cast<float2*>(out + (size_t)kr0 * DV + cc) = make_float2(X[nt][0], X[nt][1]);
+                *reinterpret_cast<float2*>(out + (size_t)kr1 * DV + cc) = make_float2(X[nt][2], X[nt][3]);
+            }
         }
     }
 }

@@ -4,12 +4,15 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "../../include/mkda.h"
 #include "host.h"
 
 namespace mkda {
 
 static thread_local char g_err[512] = "";
+static std::atomic<unsigned long long> g_launches{0};
 
 int set_error(int code, const char* msg) {
     snprintf(g_err, sizeof(g_err), "%s", msg);
@@ -22,6 +25,7 @@ int check_launch(const char* what) {
         snprintf(g_err, sizeof(g_err), "%s: %s", what, cudaGetErrorString(e));
         return MKDA_ERR_LAUNCH;
     }
+    g_launches.fetch_add(1, std::memory_order_relaxed);
     return MKDA_OK;
 }
 
@@ -113,6 +117,7 @@ extern "C" int mkda_device_status_clear(void) {
     return rc;
 }
 extern "C" const char* mkda_last_error(void) { return mkda::g_err; }
+extern "C" unsigned long long mkda_launch_count(void) { return mkda::g_launches.load(std::memory_order_relaxed); }
 extern "C" int mkda_abi_version(void) { return 4; }
 extern "C" int mkda_struct_sizes(int* out, int n) {
     const int sizes[] = {

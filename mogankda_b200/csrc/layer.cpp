@@ -1,0 +1,266 @@
+// Launches of one layer call: gate + cumsum (+ beta) -> L2 statistics -> WY preparation -> state pass -> output, and the backward
+// pass.  Every intermediate is a torch allocation on the current stream.
+#include "layer.h"
+
+#include <c10/cuda/CUDAStream.h>
+
+#include <limits>
+
+namespace mkda_host {
+
+int dtype_code(const Tensor& t) {
+    switch (t.scalar_type()) {
+        case at::kFloat: return MKDA_F32;
+        case at::kBFloat16: return MKDA_BF16;
+        case at::kHalf: return MKDA_F16;
+        default: break;
+    }
+    TORCH_CHECK_TYPE(false, "unsupported dtype ", t.scalar_type(), "; expected float32, bfloat16 or float16");
+    return -1;
+}
+
+Tensor aligned(const Tensor& t) {
+    if (!t.defined()) return t;
+    Tensor c = t.is_contiguous() ? t : t.contiguous();
+    return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+
+Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev) {
+    return Tensor(at::detail::empty_cuda(sizes, dt, dev, std::nullopt));
+}
+
+namespace {
+
+Tensor aligned_f32(const Tensor& t) {
+    if (!t.defined()) return t;
+    return aligned(t.scalar_type() == at::kFloat ? t : t.to(at::kFloat));
+}
+float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+void check_rc(int rc, const char* what) { TORCH_CHECK(rc == MKDA_OK, what, " failed (", rc, "): ", mkda_last_error()); }
+
+// (row stride, column stride) in elements if `t` [..., 128] can be addressed as rows x 128 with one stride per axis (contiguous
+// tensors, and broadcast views such as the gradient autograd produces for o.sum()); false otherwise
+bool rows_strides(const Tensor& t, int64_t& row, int64_t& col) {
+    int64_t span = -1;
+    row = -1;
+    for (int64_t d = t.dim() - 2; d >= 0; --d) {          // collapse the leading dims from the inside out
+        if (t.size(d) == 1) continue;
+        const int64_t sd = t.stride(d);
+        if (row < 0) row = sd;
+        else if (sd != span) return false;
+        span = sd * t.size(d);
+    }
+    if (row < 0) row = 0;
+    col = t.stride(-1);
+    const int64_t most = std::numeric_limits<int>::max();
+    return !(col == 1 && row % 8) && row <= most && col <= most && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
+
+Tensor reduce(const float* part, int rows, int cols, int group, cudaStream_t st, const at::Device& dev) {
+    Tensor out = new_cuda({cols / group}, at::kFloat, dev);
+    MkdaReduce p{};
+    p.in = part; p.rows = rows; p.cols = cols; p.group = group; p.out = fptr(out);
+    check_rc(mkda_reduce_partials(&p, st), "mkda_reduce_partials");
+    return out;
+}
+
+}  // namespace
+
+std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need_bwd, Saved& s) {
+    cudaStream_t st = c10::cuda::getCurrentCUDAStream();
+    const int64_t row = (int64_t)c.TT * c.HV * 128 * 4, seg_states = (int64_t)c.NS * c.HV * 65536;
+    s.x_alog = aligned_f32(in.A_log);
+    s.x_bias = aligned_f32(in.dt_bias);
+    Arena tmp;
+    Arena& keep = s.arena;
+    float *u = nullptr, *hs = nullptr, *s_in = nullptr;
+    int* warm_start = nullptr;
+    if (c.l2) {
+        keep.want(&s.q_rstd, (int64_t)c.TT * c.HK * 4);
+        keep.want(&s.k_rstd, (int64_t)c.TT * c.HK * 4);
+    }
+    keep.want(&s.g_c, row);
+    keep.want(&s.beta_e, (int64_t)c.TT * c.HV * 4);
+    keep.want(&s.A, c.tiles(MKDA_QUARTER_TILE_BYTES));
+    keep.want(&s.Aqk, c.tiles(MKDA_QUARTER_TILE_BYTES));
+    keep.want(&s.nw, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    keep.want(&s.kbar, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    keep.want(&s.qs, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    keep.want(&s.gl, c.tiles(512));
+    keep.want(&s.h, c.tiles(MKDA_STATE_TILE_BYTES));
+    keep.want(&s.Vd, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    if (c.has_ep && need_bwd) keep.want(&s.o_raw, row);
+    tmp.want(&u, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    if (c.segmented) {
+        keep.want(&s.ms, seg_states);
+        tmp.want(&hs, seg_states);
+        tmp.want(&s_in, seg_states);
+        if (c.warm) {
+            keep.want(&s.warm_end, (int64_t)c.NS * c.HV * 4);
+            tmp.want(&warm_start, (int64_t)c.NS * c.HV * 4);
+        }
+    }
+    keep.allocate(c.dev);
+    tmp.allocate(c.dev);
+    const MkdaLayout L = c.layout();
+
+    if (c.l2) {
+        MkdaL2Norm p{};
+        p.dtype = c.qkv_dtype; p.rows = c.TT * c.HK; p.eps = 1e-6f;
+        p.x = in.q.data_ptr(); p.rstd = s.q_rstd;
+        check_rc(mkda_l2norm_rstd(&p, st), "mkda_l2norm_rstd");
+        p.x = in.k.data_ptr(); p.rstd = s.k_rstd;
+        check_rc(mkda_l2norm_rstd(&p, st), "mkda_l2norm_rstd");
+    }
+    {
+        MkdaGateFwd p{};
+        p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate;
+        p.A_log = fptr(s.x_alog); p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound;
+        p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta); p.beta_sigmoid = c.beta_sigmoid;
+        p.beta_scale = c.beta_scale; p.beta_out = s.beta_e; p.g_c = s.g_c;
+        check_rc(mkda_gate_cumsum_fwd(&p, st), "mkda_gate_cumsum_fwd");
+    }
+    {
+        MkdaIntraFwd p{};
+        p.L = L; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
+        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.scale = c.scale;
+        p.A = s.A; p.Aqk = s.Aqk; p.nw = s.nw; p.u = u; p.kbar = s.kbar; p.qs = s.qs; p.gl = s.gl;
+        check_rc(mkda_intra_fwd(&p, st), "mkda_intra_fwd");
+    }
+    Tensor ht;
+    if (c.want_ht) ht = c.states(c.N);
+    MkdaRecurFwd r{};
+    r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf;
+    if (c.segmented) {
+        // pre-pass from zero: per-segment (state, transition); the prefix combine then gives the state entering every segment
+        if (c.warm) {
+            MkdaWarmup w{};
+            w.L = L; w.gl = s.gl; w.threshold_log2 = c.warm_log2; w.warm_start = warm_start; w.warm_end = s.warm_end;
+            check_rc(mkda_warmup_chunks(&w, st), "mkda_warmup_chunks");
+        }
+        MkdaRecurFwd pre = r;
+        pre.state_v_first = 0; pre.ht = hs; pre.want_transition = 1; pre.mt = s.ms; pre.warm_start = warm_start;
+        check_rc(mkda_recur_fwd(&pre, st), "mkda_recur_fwd");
+        MkdaCombine m{};
+        m.NG = c.N; m.HV = c.HV; m.grp_seg_off = c.grp_off; m.hs = hs; m.ms = s.ms; m.carry = fptr(in.h0); m.s_in = s_in;
+        m.carry_v_first = c.vf;
+        check_rc(mkda_state_combine(&m, st), "mkda_state_combine");
+        r.h0 = s_in; r.h0_k_first = 1; r.seg_ht = c.seg_last;
+    } else {
+        r.h0 = fptr(in.h0);
+    }
+    r.h = s.h; r.Vd = s.Vd; r.ht = fptr(ht);
+    check_rc(mkda_recur_fwd(&r, st), "mkda_recur_fwd");
+
+    Tensor out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type());
+    {
+        MkdaOutFwd p{};
+        p.L = L; p.qs = s.qs; p.Aqk = s.Aqk; p.Vd = s.Vd; p.h = s.h; p.has_norm = c.has_ep;
+        const Tensor w = aligned(in.ep_w);
+        if (c.has_ep) {
+            if (w.defined()) { p.norm_w = w.data_ptr(); p.norm_w_dtype = dtype_code(w); }
+            p.gate = in.ep_gate.data_ptr(); p.gate_dtype = dtype_code(in.ep_gate); p.act = c.act; p.eps = c.eps;
+        }
+        p.o_raw = s.o_raw; p.out = out.data_ptr(); p.out_dtype = dtype_code(out);
+        check_rc(mkda_out_fwd(&p, st), "mkda_out_fwd");
+    }
+    return {out, ht};
+}
+
+Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor dht, bool need_alog, bool need_bias, bool need_h0) {
+    cudaStream_t st = c10::cuda::getCurrentCUDAStream();
+    const MkdaLayout L = c.layout();
+    Grads g;
+    if (!dy.defined()) dy = at::zeros({c.B, c.T, c.HV, 128}, in.q.options().dtype(c.has_ep ? at::kFloat : in.q.scalar_type()));
+    if (dht.defined()) dht = aligned_f32(dht);
+    need_h0 = need_h0 && in.h0.defined();
+
+    Arena tmp;
+    float *dO = nullptr, *dh = nullptr, *dVd = nullptr, *dq_v = nullptr, *dk_v = nullptr, *dgp = nullptr, *part_w = nullptr, *part_b = nullptr,
+          *part_a = nullptr, *dloc = nullptr, *g_in = nullptr;
+    const int64_t tile = MKDA_CHUNK_TILE_BYTES, seg_states = (int64_t)c.NS * c.HV * 65536;
+    const int w_rows = std::min(c.NC * c.HV, MKDA_EPILOGUE_MAX_PART_ROWS);
+    const int g_rows = std::max(1, std::min(c.NC, 256)), g_width = c.scalar_gate ? c.HV : c.HV * 128;
+    tmp.want(&dO, c.tiles(tile));
+    tmp.want(&dh, c.tiles(MKDA_STATE_TILE_BYTES));
+    tmp.want(&dVd, c.tiles(tile));
+    tmp.want(&dq_v, (int64_t)c.NC * c.HK * tile);
+    tmp.want(&dk_v, (int64_t)c.NC * c.HK * tile);
+    tmp.want(&dgp, c.tiles(tile));
+    if (c.has_ep && in.ep_w.defined()) tmp.want(&part_w, (int64_t)w_rows * 512);
+    if (c.mode != MKDA_GATE_PRECOMPUTED) {
+        if (need_bias) tmp.want(&part_b, (int64_t)g_rows * g_width * 4);
+        if (need_alog) tmp.want(&part_a, (int64_t)g_rows * g_width * 4);
+    }
+    if (c.segmented) { tmp.want(&dloc, seg_states); tmp.want(&g_in, seg_states); }
+    tmp.allocate(c.dev);
+
+    MkdaBwdDh d{};
+    d.L = L;
+    if (c.has_ep) {      // dO leaves the epilogue backward in the tile form the tensor-core kernels fetch
+        int64_t rs, cs;
+        if (!rows_strides(dy, rs, cs)) { dy = aligned(dy); rs = 128; cs = 1; }
+        const Tensor w = aligned(in.ep_w);
+        g.ep_gate = c.like_out(in.ep_gate);
+        MkdaEpilogueBwdTiles p{};
+        p.L = L; p.dy = dy.data_ptr(); p.dy_dtype = dtype_code(dy); p.dy_row_stride = (int)rs; p.dy_col_stride = (int)cs; p.o_raw = s.o_raw;
+        if (w.defined()) { p.norm_w = w.data_ptr(); p.norm_w_dtype = dtype_code(w); }
+        p.gate = in.ep_gate.data_ptr(); p.gate_dtype = dtype_code(in.ep_gate); p.act = c.act; p.eps = c.eps;
+        p.dO_t = dO; p.dgate = g.ep_gate.data_ptr(); p.dgate_dtype = dtype_code(g.ep_gate); p.part_rows = w_rows; p.part_w = part_w;
+        check_rc(mkda_epilogue_bwd_tiles(&p, st), "mkda_epilogue_bwd_tiles");
+        if (part_w) g.ep_w = reduce(part_w, w_rows, 128, 1, st, c.dev).to(in.ep_w.scalar_type());
+        d.dO_in_t = dO;
+    } else {
+        dy = aligned(dy);
+        d.d_o = dy.data_ptr(); d.do_dtype = dtype_code(dy);
+    }
+    d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw;
+    if (need_h0) g.h0 = c.states(c.N);
+    MkdaBwdDh full = d;
+    if (c.segmented) {
+        // pre-pass from zero: only the gradient entering each segment is wanted, nothing per chunk is stored
+        d.dh0 = dloc; d.warm_end = s.warm_end;
+        check_rc(mkda_bwd_dh(&d, st), "mkda_bwd_dh");
+        MkdaCombine m{};
+        m.NG = c.N; m.HV = c.HV; m.grp_seg_off = c.grp_off; m.hs = dloc; m.ms = s.ms; m.carry = fptr(dht); m.reverse = 1; m.s_in = g_in;
+        m.s_out = fptr(g.h0); m.carry_v_first = c.vf; m.out_v_first = c.vf;
+        check_rc(mkda_state_combine(&m, st), "mkda_state_combine");
+        full.dht = g_in;
+    } else {
+        full.dht = fptr(dht); full.state_v_first = c.vf; full.dh0 = fptr(g.h0);
+    }
+    full.dh = dh; full.dVd_t = dVd; full.dO_t = c.has_ep ? nullptr : dO;
+    check_rc(mkda_bwd_dh(&full, st), "mkda_bwd_dh");
+    g.v = c.rows_out(c.HV, in.v.scalar_type());
+    g.beta = c.like_out(in.beta);
+    {
+        MkdaBwdChunk p{};
+        p.L = L; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
+        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.A = s.A; p.h = s.h;
+        p.dh = dh; p.Vd = s.Vd; p.dO_t = dO; p.dVd_t = dVd; p.scale = c.scale; p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta);
+        p.beta_sigmoid = c.beta_sigmoid; p.beta_scale = c.beta_scale; p.dq_v = dq_v; p.dk_v = dk_v; p.dgp = dgp; p.dbeta = g.beta.data_ptr();
+        p.dbeta_dtype = dtype_code(g.beta); p.dv = g.v.data_ptr();
+        check_rc(mkda_bwd_chunk(&p, st), "mkda_bwd_chunk");
+    }
+    g.x = c.like_out(in.x);
+    {
+        MkdaGateBwd p{};
+        p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(s.x_alog);
+        p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound; p.dgp = dgp; p.dx = g.x.data_ptr(); p.dx_dtype = dtype_code(g.x);
+        p.part_rows = g_rows; p.part_bias = part_b; p.part_alog = part_a;
+        check_rc(mkda_gate_bwd(&p, st), "mkda_gate_bwd");
+        if (part_b) g.dt_bias = reduce(part_b, g_rows, g_width, 1, st, c.dev).view_as(in.dt_bias).to(in.dt_bias.scalar_type());
+        if (part_a) g.A_log = reduce(part_a, g_rows, g_width, c.scalar_gate ? 1 : 128, st, c.dev).view_as(in.A_log).to(in.A_log.scalar_type());
+    }
+    g.q = c.rows_out(c.HK, in.q.scalar_type());
+    g.k = c.rows_out(c.HK, in.k.scalar_type());
+    {
+        MkdaQkGrad p{};
+        p.L = L; p.dq_v = dq_v; p.dk_v = dk_v; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.x_dtype = c.qkv_dtype;
+        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.dq = g.q.data_ptr(); p.dk = g.k.data_ptr();
+        check_rc(mkda_qk_grad_finish(&p, st), "mkda_qk_grad_finish");
+    }
+    return g;
+}
+
+}  // namespace mkda_host

@@ -30,6 +30,36 @@ __device__ __forceinline__ void publish_operands() {
     umma::fence_after_sync();
 }
 
+// A caller-visible [V,K] state <-> the 32 columns [32 cg, 32 cg + 32) of row `row` that a thread keeps: through a 64 KB shared-memory image
+// (16-byte pieces XOR-swizzled with the row, conflict-free both ways) so that global memory sees whole rows.  Reading or writing the
+// rows thread by thread touches 32 different lines per instruction.  Every thread of the CTA takes part; ends with the image free for the next use after a barrier.
+__device__ __forceinline__ void load_state_rows(const float* __restrict__ src, uint8_t* img, int tid, int row, int cg, float (&s)[32]) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        const int i = tid + n * 512, r = i >> 5, ch = i & 31;
+        *reinterpret_cast<float4*>(img + r * 512 + ((ch ^ (r & 7)) << 4)) = reinterpret_cast<const float4*>(src)[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(img + row * 512 + (((cg * 8 + i) ^ (row & 7)) << 4));
+        s[4 * i] = v.x; s[4 * i + 1] = v.y; s[4 * i + 2] = v.z; s[4 * i + 3] = v.w;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void store_state_rows(float* __restrict__ dst, uint8_t* img, int tid, int row, int cg, const float (&s)[32]) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(img + row * 512 + (((cg * 8 + i) ^ (row & 7)) << 4)) = make_float4(s[4 * i], s[4 * i + 1], s[4 * i + 2], s[4 * i + 3]);
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        const int i = tid + n * 512, r = i >> 5, ch = i & 31;
+        reinterpret_cast<float4*>(dst)[i] = *reinterpret_cast<const float4*>(img + r * 512 + ((ch ^ (r & 7)) << 4));
+    }
+}
+
 constexpr int RECUR_TC_SMEM = 64 * 1024 + 5 * 32 * 1024 + 1024;
 
 __global__ void __launch_bounds__(512, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p) {
@@ -65,22 +95,6 @@ __global__ void __launch_bounds__(512, 1) recur_fwd_tc_kernel(const MkdaRecurFwd
         const int w = p.warm_start[seg * HV + h];
         if (w > c_beg) { cut = true; c_beg = trans ? c_end : w; }
     }
-    {   // initial state: columns [32 cg, 32 cg + 32) of row `row`
-        float s[32];
-        const int h0row = p.seg_h0 ? p.seg_h0[seg] : seg;
-        const float* h0 = (!trans && !cut && p.h0 && h0row >= 0) ? p.h0 + ((size_t)h0row * HV + h) * DK * DV : nullptr;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const int kk = cg * 32 + j;
-            float v = 0.f;
-            if (trans) v = (kk == row && !cut) ? 1.f : 0.f;
-            else if (h0) v = vf ? h0[(size_t)row * DK + kk] : h0[(size_t)kk * DV + row];
-            s[j] = v;
-        }
-        umma::tmem_st32(umma::tmem_addr(tmem, warp, cg * 32), s);
-        umma::tmem_wait_st();
-    }
-
     // nw^T and kbar arrive as the ready-made tiles written by the intra-chunk kernel: two bulk copies per chunk on one
     // barrier (thread 0).  The 128 decay factors of the chunk are read by the first four warps into a register and parked
     // in shared memory at the end of the step: a load stored at once would make those warps (and, at the next barrier,
@@ -107,8 +121,27 @@ __global__ void __launch_bounds__(512, 1) recur_fwd_tc_kernel(const MkdaRecurFwd
     if (c_beg < c_end) {
         fetch(c_beg, 0);
         fetch_u(c_beg);
-        if (tid < DK) sh.gl[0][tid] = gl_next;
     }
+    {   // initial state: columns [32 cg, 32 cg + 32) of row `row`
+        float s[32];
+        const int h0row = p.seg_h0 ? p.seg_h0[seg] : seg;
+        const float* h0 = (!trans && !cut && p.h0 && h0row >= 0) ? p.h0 + ((size_t)h0row * HV + h) * DK * DV : nullptr;
+        if (h0 && vf && !p.h0_k_first) {               // CTA-uniform
+            load_state_rows(h0, sAh, tid, row, cg, s);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const int kk = cg * 32 + j;
+                float v = 0.f;
+                if (trans) v = (kk == row && !cut) ? 1.f : 0.f;
+                else if (h0) v = h0[(size_t)kk * DV + row];
+                s[j] = v;
+            }
+        }
+        umma::tmem_st32(umma::tmem_addr(tmem, warp, cg * 32), s);
+        umma::tmem_wait_st();
+    }
+    if (tid < DK) sh.gl[0][tid] = gl_next;
     for (int c = c_beg; c < c_end; ++c) {
         const int buf = (c - c_beg) & 1;
         const bool more = c + 1 < c_end;
@@ -180,15 +213,16 @@ __global__ void __launch_bounds__(512, 1) recur_fwd_tc_kernel(const MkdaRecurFwd
         umma::tmem_ld32(umma::tmem_addr(tmem, warp, cg * 32), s);
         float* out = nullptr;
         if (trans) { if (p.mt) out = p.mt + ((size_t)seg * HV + h) * DK * DK; }
-        else if (p.ht) out = p.ht + ((size_t)seg * HV + h) * DK * DV;
-        if (out) {
+        else if (p.ht) {
+            const int r = p.seg_ht ? p.seg_ht[seg] : seg;
+            if (r >= 0) out = p.ht + ((size_t)r * HV + h) * DK * DV;
+        }
+        // transition: M[K out][K in] with this thread holding row `row` = K in; state: [K][V] or [V][K]
+        if (out && !trans && vf) {                         // CTA-uniform
+            store_state_rows(out, sAh, tid, row, cg, s);
+        } else if (out) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int kk = cg * 32 + j;
-                // transition: M[K out][K in] with this thread holding row `row` = K in; state: [K][V] or [V][K]
-                if (trans || !vf) out[(size_t)kk * DV + row] = s[j];
-                else out[(size_t)row * DK + kk] = s[j];
-            }
+            for (int j = 0; j < 32; ++j) out[(size_t)(cg * 32 + j) * DV + row] = s[j];
         }
     }
     umma::fence_before_sync();
@@ -266,10 +300,11 @@ __global__ void __launch_bounds__(512, 1) bwd_dh_tc_kernel(const MkdaBwdDh p) {
         float s[32];
         const int drow = p.seg_dht ? p.seg_dht[seg] : seg;
         const float* src = (p.dht && drow >= 0 && !cut) ? p.dht + ((size_t)drow * HV + h) * DK * DV : nullptr;
+        if (src && vf) {                                   // CTA-uniform
+            load_state_rows(src, sAh, tid, row, cg, s);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const int kk = cg * 32 + j;
-            s[j] = src ? (vf ? src[(size_t)row * DK + kk] : src[(size_t)kk * DV + row]) : 0.f;
+            for (int j = 0; j < 32; ++j) s[j] = src ? src[(size_t)(cg * 32 + j) * DV + row] : 0.f;
         }
         umma::tmem_st32(umma::tmem_addr(tmem, warp, cg * 32), s);
         umma::tmem_wait_st();
@@ -380,10 +415,11 @@ __global__ void __launch_bounds__(512, 1) bwd_dh_tc_kernel(const MkdaBwdDh p) {
         float s[32];
         umma::tmem_ld32(umma::tmem_addr(tmem, warp, cg * 32), s);
         float* out = p.dh0 + ((size_t)seg * HV + h) * DK * DV;
+        if (vf) {
+            store_state_rows(out, sAh, tid, row, cg, s);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const int kk = cg * 32 + j;
-            if (vf) out[(size_t)row * DK + kk] = s[j]; else out[(size_t)kk * DV + row] = s[j];
+            for (int j = 0; j < 32; ++j) out[(size_t)(cg * 32 + j) * DV + row] = s[j];
         }
     }
     umma::fence_before_sync();

@@ -9,6 +9,7 @@ like the full sequence (bitwise prefix invariance).
 """
 from dataclasses import dataclass, field
 
+import numpy as np
 import torch
 
 CHUNK = 64
@@ -32,6 +33,8 @@ class Layout:
     segmented: bool
     covers_all: bool            # every token of [0, B*T) belongs to a sequence
     host: dict = field(default_factory=dict)
+    tables: torch.Tensor = None  # int32: the seven tables above, one after the other (what the native host path takes)
+    dims: tuple = ()            # (NC, NS, N, segmented, covers_all)
 
     @property
     def TT(self):
@@ -39,7 +42,7 @@ class Layout:
 
 
 def build_tables(B, T, cu, seg_chunks=0):
-    """Pure-python tables.  ``cu`` is a list of ints or None; ``seg_chunks`` = chunks per segment (0 = no cut)."""
+    """Tables as lists.  ``cu`` is a list of ints or None; ``seg_chunks`` = chunks per segment (0 = no cut)."""
     if cu is None:
         bounds = [(b * T, b * T + T) for b in range(B)]
     else:
@@ -48,26 +51,25 @@ def build_tables(B, T, cu, seg_chunks=0):
         if len(cu) < 1 or cu[0] != 0 or any(cu[i + 1] < cu[i] for i in range(len(cu) - 1)) or cu[-1] > T:
             raise ValueError("cu_seqlens must start at 0, be non-decreasing and end within T")
         bounds = list(zip(cu[:-1], cu[1:]))
-    start, length, seq_off = [], [], [0]
-    seg_off, grp_off, seg_first, seg_last = [0], [0], [], []
-    for n, (s, e) in enumerate(bounds):
-        nc = -(-(e - s) // CHUNK)
-        for i in range(nc):
-            start.append(s + i * CHUNK)
-            length.append(min(CHUNK, e - s - i * CHUNK))
-        base = seq_off[-1]
-        seq_off.append(base + nc)
-        step = seg_chunks if seg_chunks and seg_chunks > 0 else max(nc, 1)
-        cuts = list(range(0, nc, step)) if nc else [0]
-        for j, c0 in enumerate(cuts):
-            seg_off.append(base + min(c0 + step, nc))
-            seg_first.append(n if j == 0 else -1)
-            seg_last.append(n if j == len(cuts) - 1 else -1)
-        grp_off.append(len(seg_off) - 1)
-    covered = sum(e - s for s, e in bounds)
-    return dict(chunk_start=start, chunk_len=length, seq_chunk_off=seq_off, seg_chunk_off=seg_off,
-                grp_seg_off=grp_off, seg_first=seg_first, seg_last=seg_last, N=len(bounds),
-                covers_all=covered == B * T)
+    s, e = np.array(bounds, dtype=np.int64).reshape(-1, 2).T
+    N = len(s)
+    nc = -(-(e - s) // CHUNK)                                  # chunks per sequence
+    seq_off = np.concatenate([[0], np.cumsum(nc)])
+    within = np.arange(seq_off[-1]) - np.repeat(seq_off[:-1], nc)          # index of a chunk inside its sequence
+    start = np.repeat(s, nc) + within * CHUNK
+    length = np.minimum(CHUNK, np.repeat(e, nc) - start)
+    step = np.full(N, seg_chunks, dtype=np.int64) if seg_chunks and seg_chunks > 0 else np.maximum(nc, 1)
+    ns = np.maximum(-(-nc // step), 1)                         # segments per sequence (an empty sequence keeps one)
+    grp_off = np.concatenate([[0], np.cumsum(ns)])
+    seq_of = np.repeat(np.arange(N), ns)
+    j = np.arange(grp_off[-1]) - grp_off[seq_of]
+    seg_end = seq_off[seq_of] + np.minimum((j + 1) * step[seq_of], nc[seq_of])
+    seg_off = np.concatenate([[0], seg_end])
+    seg_first = np.where(j == 0, seq_of, -1)
+    seg_last = np.where(j == ns[seq_of] - 1, seq_of, -1)
+    tb = dict(chunk_start=start, chunk_len=length, seq_chunk_off=seq_off, seg_chunk_off=seg_off,
+              grp_seg_off=grp_off, seg_first=seg_first, seg_last=seg_last)
+    return dict({n: t.tolist() for n, t in tb.items()}, N=N, covers_all=int((e - s).sum()) == B * T)
 
 
 def _sm_count(device=None):
@@ -108,10 +110,11 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
     """Device tables, cached on (shape, identity + version of ``cu_seqlens``, segment policy) like the reference's
     ``tensor_cache`` (mogan_kda/utils/index.py:19-90).  A cache miss reads ``cu_seqlens`` back to the host.
     ``auto_heads`` > 0 lets ``wants_segments`` decide, for that many v-heads, whether ``seg_chunks`` is applied."""
-    key = (B, T, str(device), seg_chunks, auto_heads, cost_ratio)
+    key = (B, T, device, seg_chunks, auto_heads, cost_ratio)
     ver = None if cu_seqlens is None else cu_seqlens._version
-    for i, (k, ref, v, lay) in enumerate(_cache):
-        if k == key and ref is cu_seqlens and v == ver:
+    for i in range(len(_cache) - 1, -1, -1):
+        k, ref, v, lay = _cache[i]
+        if ref is cu_seqlens and v == ver and k == key:
             if i != len(_cache) - 1:
                 _cache.append(_cache.pop(i))          # most recently used last
             return lay
@@ -122,12 +125,17 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
                               cost_ratio):
             seg_chunks = 0
     tb = build_tables(B, T, cu, seg_chunks)
-    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=device)      # noqa: E731
-    lay = Layout(B=B, T=T, N=tb["N"], NC=len(tb["chunk_start"]), NS=len(tb["seg_first"]), NG=tb["N"],
-                 chunk_start=i32(tb["chunk_start"]), chunk_len=i32(tb["chunk_len"]),
-                 seg_chunk_off=i32(tb["seg_chunk_off"]), grp_seg_off=i32(tb["grp_seg_off"]),
-                 seq_chunk_off=i32(tb["seq_chunk_off"]), seg_first=i32(tb["seg_first"]), seg_last=i32(tb["seg_last"]),
-                 segmented=len(tb["seg_first"]) != tb["N"], covers_all=tb["covers_all"], host=tb)
+    # one upload for all seven tables, each padded to a multiple of four entries (16 bytes)
+    names = ("chunk_start", "chunk_len", "seg_chunk_off", "grp_seg_off", "seq_chunk_off", "seg_first", "seg_last")
+    flat, at = [], {}
+    for n in names:
+        at[n] = (len(flat), len(tb[n]))
+        flat += tb[n] + [0] * (-len(tb[n]) % 4)
+    tables = torch.tensor(flat or [0], dtype=torch.int32, device=device)
+    part = {n: tables[o:o + m] for n, (o, m) in at.items()}
+    NC, NS, segmented = len(tb["chunk_start"]), len(tb["seg_first"]), len(tb["seg_first"]) != tb["N"]
+    lay = Layout(B=B, T=T, N=tb["N"], NC=NC, NS=NS, NG=tb["N"], segmented=segmented, covers_all=tb["covers_all"], host=tb, tables=tables,
+                 dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"])), **part)
     if len(_cache) >= _CACHE_MAX:
         _cache.pop(0)
     _cache.append((key, cu_seqlens, ver, lay))
