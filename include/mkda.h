@@ -44,7 +44,7 @@ typedef struct {
 /* Fused gate activation + chunk-local cumsum (log2 domain) + optional beta activation.
  * Replaces kda_gate_cumsum_fwd (mogan_kda/ops/kimi_delta_rule/gate.py:378-406), _beta
  * (mogan_kda/ops/kimi_delta_rule/chunk/__init__.py:184-189) and, for a scalar gate, chunk_local_cumsum
- * (mogan_kda/ops/utils/cumsum.py:296-373) with the result broadcast over the 128 channels. */
+ * (mogan_kda/ops/utils/cumsum.py:296-373). */
 typedef struct {
     MkdaLayout L;
     const void* x; int x_dtype; int scalar_gate;   /* [TT,HV,128] or [TT,HV] */
@@ -54,7 +54,7 @@ typedef struct {
     const void* beta_raw; int beta_dtype;          /* [TT,HV] or NULL (skip beta) */
     int beta_sigmoid; float beta_scale;
     float* beta_out;                               /* [TT,HV] fp32 */
-    float* g_c;                                    /* [TT,HV,128] fp32 */
+    float* g_c;                                    /* [TT,HV,128] fp32 ([TT,HV] if scalar_gate) */
 } MkdaGateFwd;
 int mkda_gate_cumsum_fwd(const MkdaGateFwd* p, void* stream);
 
@@ -66,7 +66,8 @@ typedef struct {
     const void* x; int x_dtype; int scalar_gate;
     const float* A_log; const float* dt_bias;
     int mode; float lower_bound;
-    const float* dgp;          /* [NC,HV] fp32 [64][128] tiles: gradient w.r.t. the log2 cumsum as written by mkda_bwd_chunk */
+    const float* dgp;          /* [NC,HV] fp32 [64][128] tiles: gradient w.r.t. the log2 cumsum as written by mkda_bwd_chunk;
+                                * [NC,HV,64] if scalar_gate */
     void* dx; int dx_dtype;    /* [TT,HV,128] or [TT,HV] */
     int part_rows;             /* number of partial rows R (1 <= R <= NC): chunk c accumulates into row c % R */
     float* part_bias;          /* [R,HV,128] ([R,HV] scalar) partial sums of d/d(x+bias), or NULL */
@@ -101,9 +102,8 @@ typedef struct {
     const void* q; const void* k; const void* v; int qkv_dtype;
     const float* q_rstd; const float* k_rstd;      /* [TT,HK] or NULL */
     const float* g_c; const float* beta;           /* [TT,HV,128], [TT,HV] */
-    int scalar_gate;           /* 1: g_c holds the same value in all 128 channels of a (token, head) (one decay per token, as
-                                * mkda_gate_cumsum_fwd writes it for a [TT,HV] gate): the scalar-gate path is taken, which
-                                * accepts any decay <= 0; 0: per-channel path, contract: decay >= -5 per token */
+    int scalar_gate;           /* 1: one decay per token, g_c is [TT,HV]: the scalar-gate path is taken, which accepts any
+                                * decay <= 0; 0: per-channel path, contract: decay >= -5 per token */
     float scale;
     float* A;      /* [NC,HV] quarter tiles: (I + strictlower(diag(beta) Gamma))^-1 */
     float* Aqk;    /* [NC,HV] quarter tiles: scale * lower(Q K^T with decay) */
@@ -272,7 +272,7 @@ typedef struct {
 int mkda_bwd_dh(const MkdaBwdDh* p, void* stream);
 
 /* Every gradient that is local to a (chunk, v-head) once the state gradients are known, in one kernel:
- *  - through Vd = A diag(beta)(V - k~ S): dv, the WY part of dbeta, dAqk and dL (K3a of bwd_post_kda,
+ *  - through Vd = A diag(beta)(V - k~ S): dv, the WY part of dbeta, dAqk and dL = -strictlower(A^T dVd Vd^T) (K3a of bwd_post_kda,
  *    mogan_kda/ops/kimi_delta_rule/chunk/hopper/bwd_post.py:72-400);
  *  - through the states: the row-local parts of dq, dk and of the gate gradient (K3b, .../bwd_post.py:412-766);
  *  - through the decayed K K^T / Q K^T blocks (bwd_intra_kda, .../hopper/bwd_intra.py:529-600);
@@ -294,7 +294,8 @@ typedef struct {
     float* dq_v; float* dk_v;  /* [NC,HK] fp32 [64 tokens][128] tiles per (chunk, q/k head): the contributions of the HV / HK
                                 * v-heads of the head are added up in the tile (first one stored, the others added in
                                 * order, by the one CTA that owns the head's group); rows past the end are zero */
-    float* dgp;                /* [NC,HV] tiles of the same form per (chunk, v-head): gradient w.r.t. the log2 cumsum */
+    float* dgp;                /* [NC,HV] tiles of the same form per (chunk, v-head): gradient w.r.t. the log2 cumsum; with
+                                * scalar_gate its sum over the channels, [NC,HV,64] */
     void* dbeta; int dbeta_dtype;
     void* dv;                  /* [TT,HV,128] in qkv_dtype */
 } MkdaBwdChunk;

@@ -143,6 +143,28 @@ __device__ __forceinline__ void st4(void* base, int dtype, size_t idx, float4 v)
     }
 }
 
+// 8 consecutive elements, idx % 8 == 0
+template <int DT>
+__device__ __forceinline__ void st8(void* base, size_t idx, const float (&v)[8]) {
+    if (DT == MKDA_F32) {
+        st4(base, DT, idx, make_float4(v[0], v[1], v[2], v[3]));
+        st4(base, DT, idx + 4, make_float4(v[4], v[5], v[6], v[7]));
+        return;
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (DT == MKDA_BF16) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t*>(&b);
+        } else {
+            const __half2 b = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+    }
+    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + idx) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // tensor-core primitive: m16n8k8 TF32, fp32 accumulate.
 // Fragment ownership (g = lane >> 2, t = lane & 3):

@@ -73,6 +73,12 @@ int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned l
     return MKDA_OK;
 }
 
+int kernel_registers(const void* func) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, func) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+    return a.numRegs;
+}
+
 int ensure_smem(const void* func, int bytes, const char* what) {
     // (function, device) pairs whose limit is already raised; a launcher asks before every launch
     struct Done { const void* func; int dev; int bytes; };
@@ -105,6 +111,7 @@ extern "C" int mkda_device_status(void) {
     if (mkda::tc_chunk_status(&f) == 0) any |= f;
     if (mkda::tc_recur_status(&f) == 0) any |= f;
     if (mkda::tc_intra_status(&f) == 0) any |= f;
+    if (mkda::tc_bwd_chunk_status(&f) == 0) any |= f;
     return (int)any;
 }
 extern "C" int mkda_device_status_clear(void) {
@@ -114,6 +121,7 @@ extern "C" int mkda_device_status_clear(void) {
     rc |= mkda::tc_chunk_status_clear();
     rc |= mkda::tc_recur_status_clear();
     rc |= mkda::tc_intra_status_clear();
+    rc |= mkda::tc_bwd_chunk_status_clear();
     return rc;
 }
 extern "C" const char* mkda_last_error(void) { return mkda::g_err; }

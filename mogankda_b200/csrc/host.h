@@ -12,6 +12,8 @@ int check_launch(const char* what);
 // Raises the dynamic shared memory limit of `func` (the attribute is set once per function and device; later calls
 // return at once); returns 0 or an error code.
 int ensure_smem(const void* func, int bytes, const char* what);
+// Registers per thread the kernel is launched with (0 if unknown): a kernel whose warps redistribute registers checks its build with it.
+int kernel_registers(const void* func);
 // Tensor map over a row-major [rows][row_elems] tensor of 2- or 4-byte elements whose boxes are 64 rows x 128 elements, not
 // swizzled: one tiled TMA copy then brings 64 strided 128-element rows (token rows of one head) into shared memory as a dense
 // [64][128] block.  Rows past the end of the tensor read as zeros.  Returns 0, or an error code when the tensor cannot be
@@ -34,6 +36,8 @@ int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream);
 int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream);
+int tc_bwd_chunk_status(unsigned int* out);
+int tc_bwd_chunk_status_clear();
 int tc_intra_status(unsigned int* out);
 int tc_intra_status_clear();
 }  // namespace mkda

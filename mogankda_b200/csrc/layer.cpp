@@ -79,7 +79,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         keep.want(&s.q_rstd, (int64_t)c.TT * c.HK * 4);
         keep.want(&s.k_rstd, (int64_t)c.TT * c.HK * 4);
     }
-    keep.want(&s.g_c, row);
+    keep.want(&s.g_c, c.scalar_gate ? row / 128 : row);
     keep.want(&s.beta_e, (int64_t)c.TT * c.HV * 4);
     keep.want(&s.A, c.tiles(MKDA_QUARTER_TILE_BYTES));
     keep.want(&s.Aqk, c.tiles(MKDA_QUARTER_TILE_BYTES));
@@ -186,7 +186,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     tmp.want(&dVd, c.tiles(tile));
     tmp.want(&dq_v, (int64_t)c.NC * c.HK * tile);
     tmp.want(&dk_v, (int64_t)c.NC * c.HK * tile);
-    tmp.want(&dgp, c.tiles(tile));
+    tmp.want(&dgp, c.tiles(c.scalar_gate ? 256 : tile));
     if (c.has_ep && in.ep_w.defined()) tmp.want(&part_w, (int64_t)w_rows * 512);
     if (c.mode != MKDA_GATE_PRECOMPUTED) {
         if (need_bias) tmp.want(&part_b, (int64_t)g_rows * g_width * 4);

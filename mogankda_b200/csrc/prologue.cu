@@ -61,14 +61,14 @@ __global__ void __launch_bounds__(128, 5) gate_cumsum_fwd_kernel(const MkdaGateF
     __shared__ float4 tot[4][32];
     const float E = p.A_log ? expf(p.A_log[h]) : 1.f;
     float4 bias = splat4(0.f);
-    if (p.dt_bias) bias = p.scalar_gate ? splat4(p.dt_bias[h]) : *reinterpret_cast<const float4*>(p.dt_bias + h * 128 + 4 * lane);
+    if (p.dt_bias) bias = *reinterpret_cast<const float4*>(p.dt_bias + h * 128 + 4 * lane);
     float4 vals[16];
     // all 16 rows of this warp are requested before the first one is used (rows past the end re-read the last one)
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
         const int row = warp * 16 + r, rr = row < len ? row : len - 1;
         const size_t th = (size_t)(start + rr) * HV + h;
-        vals[r] = p.scalar_gate ? splat4(ld1(p.x, XDT, th)) : ld4(p.x, XDT, th * 128 + 4 * lane);
+        vals[r] = ld4(p.x, XDT, th * 128 + 4 * lane);
     }
     float4 run = splat4(0.f);
 #pragma unroll
@@ -104,6 +104,41 @@ __global__ void __launch_bounds__(128, 5) gate_cumsum_fwd_kernel(const MkdaGateF
     }
 }
 
+// One decay per token: grid (NC, blocks of 32 heads), lane = head, warp w owns rows 8w..8w+7.  The inclusive sum has the same form as
+// above (earlier warps' totals in order, plus the running sum inside the warp).  g_c is [TT,HV].
+__global__ void __launch_bounds__(256) gate_cumsum_fwd_scalar_kernel(const MkdaGateFwd p) {
+    const int HV = p.L.HV, c = blockIdx.x, h = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int start = p.L.chunk_start[c], len = p.L.chunk_len[c], hh = h < HV ? h : HV - 1;
+    __shared__ float tot[8][32];
+    const float E = p.A_log ? expf(p.A_log[hh]) : 1.f, bias = p.dt_bias ? p.dt_bias[hh] : 0.f;
+    float v[8], b[8], run = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int row = warp * 8 + r, rr = row < len ? row : len - 1;
+        const size_t th = (size_t)(start + rr) * HV + hh;
+        v[r] = ld1(p.x, p.x_dtype, th);
+        b[r] = p.beta_raw ? ld1(p.beta_raw, p.beta_dtype, th) : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (warp * 8 + r < len) run += gate_value(p.mode, v[r] + bias, E, p.lower_bound);
+        v[r] = run;
+    }
+    tot[warp][lane] = run;
+    __syncthreads();
+    float pre = 0.f;
+    for (int w = 0; w < warp; ++w) pre += tot[w][lane];
+    if (h >= HV) return;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int row = warp * 8 + r;
+        if (row >= len) break;
+        const size_t th = (size_t)(start + row) * HV + h;
+        p.g_c[th] = (pre + v[r]) * RCP_LN2;
+        if (p.beta_raw) p.beta_out[th] = p.beta_sigmoid ? p.beta_scale * sigmoidf_(b[r]) : b[r];
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // backward: same tiling; suffix sums instead of prefix sums.
 // ---------------------------------------------------------------------------------------------------------
@@ -120,7 +155,7 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
     __shared__ float4 red[2][GB_WARPS][32];
     const float E = p.A_log ? expf(p.A_log[h]) : 1.f;
     float4 bias = splat4(0.f);
-    if (p.dt_bias) bias = p.scalar_gate ? splat4(p.dt_bias[h]) : *reinterpret_cast<const float4*>(p.dt_bias + h * 128 + 4 * lane);
+    if (p.dt_bias) bias = *reinterpret_cast<const float4*>(p.dt_bias + h * 128 + 4 * lane);
     float4 pa = splat4(0.f), pb = splat4(0.f);
     for (int c = blockIdx.y; c < p.L.NC; c += gridDim.y) {
         const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
@@ -130,7 +165,7 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
             const int row = warp * GB_ROWS + r, rr = row < len ? row : len - 1;
             vals[r] = *reinterpret_cast<const float4*>(p.dgp + (((size_t)c * HV + h) * CH + rr) * 128 + 4 * lane);
             const size_t th = (size_t)(start + rr) * HV + h;
-            xs[r] = p.scalar_gate ? splat4(ld1(p.x, XDT, th)) : ld4(p.x, XDT, th * 128 + 4 * lane);
+            xs[r] = ld4(p.x, XDT, th * 128 + 4 * lane);
         }
         float4 run = splat4(0.f);
 #pragma unroll
@@ -149,26 +184,16 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
             if (row >= len) continue;                       // warp-uniform
             const size_t th = (size_t)(start + row) * HV + h;
             const float4 dg = add4(vals[r], post);
-            if (p.scalar_gate) {
-                const float dgs = warp_sum(hsum4(dg));
-                float ds, dA;
-                gate_grad(p.mode, xs[r].x + bias.x, E, p.lower_bound, ds, dA);
-                const float dxs = dgs * ds;
-                if (lane == 0) st1(p.dx, p.dx_dtype, th, dxs);
-                pb.x += dxs;
-                pa.x += dgs * dA;
-            } else {
-                const float4 xv = add4(xs[r], bias);
-                float4 ds, dA;
-                gate_grad(p.mode, xv.x, E, p.lower_bound, ds.x, dA.x);
-                gate_grad(p.mode, xv.y, E, p.lower_bound, ds.y, dA.y);
-                gate_grad(p.mode, xv.z, E, p.lower_bound, ds.z, dA.z);
-                gate_grad(p.mode, xv.w, E, p.lower_bound, ds.w, dA.w);
-                const float4 dxv = mul4(dg, ds);
-                st4(p.dx, p.dx_dtype, th * 128 + 4 * lane, dxv);
-                pb = add4(pb, dxv);
-                pa = add4(pa, mul4(dg, dA));
-            }
+            const float4 xv = add4(xs[r], bias);
+            float4 ds, dA;
+            gate_grad(p.mode, xv.x, E, p.lower_bound, ds.x, dA.x);
+            gate_grad(p.mode, xv.y, E, p.lower_bound, ds.y, dA.y);
+            gate_grad(p.mode, xv.z, E, p.lower_bound, ds.z, dA.z);
+            gate_grad(p.mode, xv.w, E, p.lower_bound, ds.w, dA.w);
+            const float4 dxv = mul4(dg, ds);
+            st4(p.dx, p.dx_dtype, th * 128 + 4 * lane, dxv);
+            pb = add4(pb, dxv);
+            pa = add4(pa, mul4(dg, dA));
         }
     }
     if (!p.part_bias && !p.part_alog) return;
@@ -179,15 +204,61 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
         float4 sb = red[0][0][lane], sa = red[1][0][lane];
         for (int w = 1; w < GB_WARPS; ++w) { sb = add4(sb, red[0][w][lane]); sa = add4(sa, red[1][w][lane]); }
         const size_t ch = (size_t)blockIdx.y * HV + h;
-        if (p.scalar_gate) {
-            if (lane == 0) {
-                if (p.part_bias) p.part_bias[ch] = sb.x;
-                if (p.part_alog) p.part_alog[ch] = sa.x;
-            }
-        } else {
-            if (p.part_bias) *reinterpret_cast<float4*>(p.part_bias + ch * 128 + 4 * lane) = sb;
-            if (p.part_alog) *reinterpret_cast<float4*>(p.part_alog + ch * 128 + 4 * lane) = sa;
+        if (p.part_bias) *reinterpret_cast<float4*>(p.part_bias + ch * 128 + 4 * lane) = sb;
+        if (p.part_alog) *reinterpret_cast<float4*>(p.part_alog + ch * 128 + 4 * lane) = sa;
+    }
+}
+
+// One decay per token: dgp is [NC,HV,64], summed over the channels where it was written.  CTA (block of 32 heads, g) walks the chunks g,
+// g + gridDim.y, ...; lane = head, warp w owns rows 8w..8w+7; the [32 heads][64] block of dgp passes through shared memory.
+__global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd p) {
+    const int HV = p.L.HV, h0 = blockIdx.x * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + lane, hh = h < HV ? h : HV - 1;
+    __shared__ float tile[32][CH + 1], tot[8][32], red[2][8][32];
+    const float E = p.A_log ? expf(p.A_log[hh]) : 1.f, bias = p.dt_bias ? p.dt_bias[hh] : 0.f;
+    float pa = 0.f, pb = 0.f;
+    for (int c = blockIdx.y; c < p.L.NC; c += gridDim.y) {
+        const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
+        for (int i = threadIdx.x; i < 32 * CH; i += 256) {
+            const int k = i >> 6;
+            tile[k][i & 63] = h0 + k < HV ? p.dgp[((size_t)c * HV + h0 + k) * CH + (i & 63)] : 0.f;
         }
+        float x[8], v[8], run = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int row = warp * 8 + r, rr = row < len ? row : len - 1;
+            x[r] = ld1(p.x, p.x_dtype, (size_t)(start + rr) * HV + hh);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 7; r >= 0; --r) {
+            if (warp * 8 + r < len) run += tile[lane][warp * 8 + r];
+            v[r] = run;
+        }
+        tot[warp][lane] = run;
+        __syncthreads();                                   // also: the tile may be refilled
+        float post = 0.f;
+        for (int w = 7; w > warp; --w) post += tot[w][lane];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int row = warp * 8 + r;
+            if (row >= len || h >= HV) continue;
+            float ds, dA;
+            gate_grad(p.mode, x[r] + bias, E, p.lower_bound, ds, dA);
+            const float dg = v[r] + post, dx = dg * ds;
+            st1(p.dx, p.dx_dtype, (size_t)(start + row) * HV + h, dx);
+            pb += dx;
+            pa = fmaf(dg, dA, pa);
+        }
+    }
+    if (!p.part_bias && !p.part_alog) return;
+    red[0][warp][lane] = pb;
+    red[1][warp][lane] = pa;
+    __syncthreads();
+    if (warp == 0 && h < HV) {
+        float sb = red[0][0][lane], sa = red[1][0][lane];
+        for (int w = 1; w < 8; ++w) { sb += red[0][w][lane]; sa += red[1][w][lane]; }
+        if (p.part_bias) p.part_bias[(size_t)blockIdx.y * HV + h] = sb;
+        if (p.part_alog) p.part_alog[(size_t)blockIdx.y * HV + h] = sa;
     }
 }
 
@@ -498,6 +569,11 @@ extern "C" int mkda_gate_cumsum_fwd(const MkdaGateFwd* p, void* stream) {
     if (p->mode != MKDA_GATE_PRECOMPUTED && !(p->lower_bound < 0.f)) return set_error(MKDA_ERR_ARG, "gate_cumsum_fwd: lower_bound must be < 0");
     if (p->beta_raw && !p->beta_out) return set_error(MKDA_ERR_ARG, "gate_cumsum_fwd: beta_out missing");
     if (p->L.NC == 0) return MKDA_OK;
+    if (p->x_dtype < MKDA_F32 || p->x_dtype > MKDA_F16) return set_error(MKDA_ERR_ARG, "gate_cumsum_fwd: unsupported dtype");
+    if (p->scalar_gate) {
+        gate_cumsum_fwd_scalar_kernel<<<dim3(p->L.NC, (p->L.HV + 31) / 32), 256, 0, (cudaStream_t)stream>>>(*p);
+        return check_launch("gate_cumsum_fwd");
+    }
     const int grid = p->L.NC * p->L.HV;
     switch (p->x_dtype) {
         case MKDA_F32: gate_cumsum_fwd_kernel<MKDA_F32><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
@@ -516,6 +592,11 @@ extern "C" int mkda_gate_bwd(const MkdaGateBwd* p, void* stream) {
     const dim3 grid(p->L.HV, p->part_rows < p->L.NC ? p->part_rows : p->L.NC);
     if ((p->part_bias || p->part_alog) && (int)grid.y != p->part_rows)
         return set_error(MKDA_ERR_ARG, "gate_bwd: part_rows must not exceed the number of chunks when partials are requested");
+    if (p->x_dtype < MKDA_F32 || p->x_dtype > MKDA_F16) return set_error(MKDA_ERR_ARG, "gate_bwd: unsupported dtype");
+    if (p->scalar_gate) {
+        gate_bwd_scalar_kernel<<<dim3((p->L.HV + 31) / 32, grid.y), 256, 0, (cudaStream_t)stream>>>(*p);
+        return check_launch("gate_bwd");
+    }
     switch (p->x_dtype) {
         case MKDA_F32: gate_bwd_kernel<MKDA_F32><<<grid, 32 * GB_WARPS, 0, (cudaStream_t)stream>>>(*p); break;
         case MKDA_BF16: gate_bwd_kernel<MKDA_BF16><<<grid, 32 * GB_WARPS, 0, (cudaStream_t)stream>>>(*p); break;

@@ -1,0 +1,677 @@
+// bwd_chunk: every gradient that is local to a (chunk, v-head) once the state gradients are known, in one kernel.
+//
+// With S the state entering the chunk, dS' the gradient of the state leaving it, k~ = k 2^g, A = (I + strictlower(diag(beta) Gamma))^-1
+// and Vd = A diag(beta) (V - k~ S) as saved by the forward pass:
+//   dW = A^T dVd          dV = diag(beta) dW          dAqk = lower(dO Vd^T)
+//   dL = -strictlower(A^T dA A^T) with dA = (dVd X^T) diag(beta), X = V - k~ S.  Since A diag(beta) X = Vd this is
+//   dL = -strictlower(dW Vd^T): one product of tiles that exist anyway, instead of rebuilding X and a chain of three products.
+//   dbeta_i = (dW X^T)_ii + (dL Gamma^T)_ii = dW_i . (X - Gamma Vd)_i = (dW Vd^T)_ii / beta_i, because beta (X - Gamma Vd) = Vd: the diagonal of
+//   the same product.  (With a sigmoid the 1 / beta cancels.  A chunk that holds a precomputed beta below 1e-12 takes the long way:
+//   rowsum(dW * V) - rowsum(k~ * (dW S^T)) + rowsum(k * T).)
+// State part (up = 2^g, rest = 2^(g_L - g)):
+//   dq_p = scale (dO S^T) up         dk_p = -beta (dW S^T) up + (Vd dS'^T) rest        dgl = rowsum_v(S * dS')
+// Intra-chunk part, E_ij = 2^(g_i - g_j) per channel (i > j), Wq = scale strictlower(dAqk), dLs = strictlower(dL):
+//   dq_row_i = sum_j Wq_ij k_j E_ij        T_i = sum_j dLs_ij k_j E_ij        dk_col_j = sum_i (Wq_ij q_i + beta_i dLs_ij k_i) E_ij
+//   dq = dq_p + dq_row + scale dAqk_ii k   dk = dk_p + beta T + dk_col + scale dAqk_ii q
+//   dg' = q dq_p + k dk_p (read part) - k (write part) + q dq_row + beta k T - k dk_col, last row += colsum(kbar dkbar) + gl dgl
+// E_ij is factored through the anchor a of i's 16-row block exactly as in the forward kernel (tc_intra.cu).  Channels go on M.  Per row
+// block I (anchor a = 16 I):
+//   row terms   R_I^T[c][r]  = sum_j Kc_I[j][c] W[16 I + r][j]       W = Wq (-> dq_row) or dLs (-> T); N = 16 each
+//   col terms   C_I^T[c][j]  = sum_{i in I} Qr[i][c] Wq[i][j] + beta_i Kr[i][c] dLs[i][j]      N = 16 (I + 1), K = 32 over [Qr; beta Kr]_I
+//
+// Roles: 16 compute warps, one warp that issues every tensor-core product and one that issues every bulk copy, joined by mbarriers only, so
+// that no compute warp waits for an issue slot of the tensor pipe (an N <= 64 product is accepted every ~50 cycles) or for a copy.  Twenty
+// warps start with 96 registers; the compute warps raise theirs to 112, the four others go down to 32 (16 x 32 x 112 + 4 x 32 x 32 = the
+// launch's 61 440).
+//
+// Products in issue order (M = 128 throughout):
+//   dW[tok x v]: two products of A^T (64 rows) with the halves of dVd^T; the second one's operand is moved one 64-group up, so that its result
+//     lands in lanes 64..127 and all warps read dW at once (the other 64 lanes of each accumulator are undefined and unread)
+//   [D1; Z][i x j] = [dO; dW] Vd^T and [Dq | Dk]^T[c x tok] = S [dO; dW]^T over one stacked row tile: dW is written below the dO rows
+//   Db^T[c x tok] = dS' Vd^T, then the row and column terms.
+// What bounds it: the tiles of an item are 272 KB, so no item can be fetched whole while another one is worked on, and an SM draws about
+// 25 B per cycle from HBM.  S, dO, Vd, dVd and A of the next item travel under the epilogue, dS' under the dW phase; k, q and g are
+// requested when that traffic is over and handed to the epilogue through shared memory (requested together with the tiles they wait
+// behind 208 KB of copies: 6 k cycles at the top of every item and as much in the epilogue).
+// Shared memory (KB): S [0,64) -> [Qr; beta Kr] | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> Kc_0, Kc_1 in the dO pieces, raw k
+// and q rows in the dW pieces | Vd^T [128,160) -> Kc_3 | dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Wq; dLs] [160,192), Kc_2 [192,216),
+// scratch [216,224).
+// TMEM columns: dW 0, [D1; Z] 128, later R_I 32 I and C_I 128 + {0, 16, 48, 96}; Dq 320, Dk 384, Db 448.
+#include "host.h"
+#include "intra.cuh"
+
+namespace mkda {
+
+namespace bc {
+constexpr int COMPUTE = 512, THREADS = 640, WARP_MMA = 16, WARP_LOAD = 17, LAUNCH_REGS = 96;
+constexpr int KB = 1024;
+constexpr int S_ = 0, R_ = 64 * KB, V_ = 128 * KB, T_ = 160 * KB, W_ = T_, A_ = 192 * KB, SCR_ = 216 * KB, TILES = 224 * KB;
+constexpr int WD_ = T_, BD_ = V_;                       // [Wq; dLs] 32 KB; scalar gate only: beta dLs, 16 KB
+// 8 KB piece i of dO (hi block 0, hi block 1, lo block 0, lo block 1) and of the dW rows stacked below it
+__host__ __device__ constexpr int o_piece(int i) { return R_ + 16 * KB * i; }
+__host__ __device__ constexpr int w_piece(int i) { return R_ + 16 * KB * i + 8 * KB; }
+// column tiles of the row blocks, 16 (I + 1) rows
+__host__ __device__ constexpr int kc_hi(int I) { return I == 0 ? o_piece(0) : I == 1 ? o_piece(1) : I == 2 ? 192 * KB : V_; }
+__host__ __device__ constexpr int kc_lo(int I) { return I == 0 ? o_piece(0) + 4 * KB : I == 1 ? o_piece(2) : I == 2 ? 204 * KB : V_ + 16 * KB; }
+constexpr int EARLY_GA = o_piece(3);
+// raw 16-bit k (pieces 0, 1) and q (2, 3) rows kept for the epilogue: 32 token rows of 256 bytes per piece
+__device__ __forceinline__ int stash(int which, int tok) { return w_piece(2 * which + (tok >> 5)) + (tok & 31) * 256; }
+__host__ __device__ constexpr int ccol(int I) { return I == 0 ? 128 : I == 1 ? 144 : I == 2 ? 176 : 224; }
+constexpr int DW = 0, D1 = 128, DQ = 320, DKB = 384, DB = 448;      // accumulator columns
+
+struct Shared {
+    uint64_t fullW, fullS, fullT;                       // copies landed: (dVd, A) | (S, dO, Vd) | dS'
+    uint64_t mmW, mmL, mmT, mmI;                        // products done: dW | [D1; Z], Dq, Dk | Db | row and column terms
+    uint64_t opW, opI[4], accFree;                      // compute warps done: dW tile | intra-chunk operands per row block | accumulators and scratch
+    uint32_t tmem;
+    float dgl[DK], beta[CH], rk[CH], rq[CH], diag[CH], gs[CH], dbw[CH];
+};
+constexpr int SMEM = TILES + (int)sizeof(Shared);
+static_assert(SMEM <= 232448, "shared memory of one CTA");
+// scratch of the intra-chunk part and the epilogue, inside the dS' tile (dead by then; the next item's arrives after accFree)
+struct Scratch {
+    float ga[5][DK];                                    // cumsum rows of the four block anchors, [4] = last valid row
+    float col[4][DK];
+    float redg[4][CH], up[CH], re[CH];
+};
+static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
+
+__device__ __forceinline__ bool sync_compute_or(bool x) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 512, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"((uint32_t)x) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(umma::smem_u32(bar)) : "memory");
+}
+// this warp's shared-memory writes and accumulator reads are done: one arrival per warp
+__device__ __forceinline__ void signal(uint64_t* bar, int lane) {
+    umma::fence_async_smem();
+    umma::fence_before_sync();
+    __syncwarp();
+    if (lane == 0) arrive(bar);
+}
+__device__ __forceinline__ void wait_mma(uint64_t* bar, uint32_t parity) {
+    umma::mbar_wait(bar, parity);
+    umma::fence_after_sync();
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(pred));
+    return pred != 0;
+}
+}  // namespace bc
+
+// fire-and-forget fp32 addition in global memory
+__device__ __forceinline__ void red_add(float* addr, float v) {
+    asm volatile("red.global.add.f32 [%0], %1;" :: "l"(addr), "f"(v) : "memory");
+}
+
+// The (chunk, v-head) items of a CTA: groups (chunk, q/k head) gridDim.x apart, heads fastest (CTAs that run together read neighbouring
+// memory), and inside a group the G = HV / HK v-heads that share the q/k head one after the other.  Their dq and dk contributions are
+// summed where they are written: the first v-head of a group stores its fp32 tile, the others add to it (red.global.add.f32 by the same
+// thread to the same address, in the fixed order of the v-heads: deterministic).  The tile lives in L2 between the two passes.
+struct ItemWalk {
+    int grp, j, G, HK, HV, ngroups, stride;
+    __device__ __forceinline__ ItemWalk(const MkdaLayout& L) {
+        HK = L.HK; HV = L.HV; G = HV / HK; ngroups = L.NC * HK; stride = gridDim.x; grp = blockIdx.x; j = 0;
+    }
+    __device__ __forceinline__ bool valid() const { return grp < ngroups; }
+    __device__ __forceinline__ int chunk() const { return grp / HK; }
+    __device__ __forceinline__ int hk() const { return grp % HK; }
+    __device__ __forceinline__ int head() const { return (grp % HK) * G + j; }
+    __device__ __forceinline__ size_t item() const { return (size_t)chunk() * HV + head(); }
+    __device__ __forceinline__ void next() { if (++j == G) { j = 0; grp += stride; } }
+};
+
+// SCALAR (one decay per token): the intra-chunk part contracts the plain k / q rows with weights that already carry
+// E_ij = 2^(g_i - g_j) (i > j, never a positive exponent):  [dq_row | T]^T = K^T [Wq E; dLs E]^T (N = 128),
+// dk_col^T = Q^T (Wq E) + K^T (beta dLs E); no anchors, and any g <= 0 is in range.  TMEM: [dq_row | T] 0, dk_col 128.
+template <bool SCALAR>
+__device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+    using namespace bc;
+    const uint32_t tmem = sh.tmem;
+    uint32_t n = 0;
+    for (ItemWalk w(p.L); w.valid(); w.next(), ++n) {
+        const uint32_t par = n & 1;
+        if (n) wait_mma(&sh.accFree, par ^ 1);
+        umma::mbar_wait(&sh.fullW, par);
+        {
+            const umma::Opnd a_lo = umma::opnd_mn(base + A_, base + A_ + 8192, 64);
+            umma::Opnd a_hi = a_lo;                      // rows 0..63 of the operand read the 8 KB in front of each half
+            a_hi.hi -= 8192; a_hi.lo -= 8192;
+            umma::gemm(tmem + DW, a_lo, umma::opnd_k(base + W_, base + W_ + 16384, 128), 128, 64, 64, 0u);
+            umma::gemm(tmem + DW + 64, a_hi, umma::opnd_k(base + W_, base + W_ + 16384, 128, 64), 128, 64, 64, 0u);
+        }
+        umma::commit(&sh.mmW);
+        umma::mbar_wait(&sh.fullS, par);
+        wait_mma(&sh.opW, par);                          // the dW rows stand below dO
+        const umma::Opnd v_mn = umma::opnd_mn(base + V_, base + V_ + 16384, 128), r_k = umma::opnd_k(base + R_, base + R_ + 32768, 128);
+        umma::gemm(tmem + D1, r_k, v_mn, 128, 64, 128, 0u);
+        umma::gemm(tmem + DQ, umma::opnd_mn(base + S_, base + S_ + 32768, 128), r_k, 128, 128, 128, 0u);
+        umma::commit(&sh.mmL);
+        umma::mbar_wait(&sh.fullT, par);
+        umma::gemm(tmem + DB, umma::opnd_mn(base + T_, base + T_ + 32768, 128), v_mn, 128, 64, 128, 0u);
+        umma::commit(&sh.mmT);
+        uint8_t* sKQ = base + S_;
+        uint8_t* sWD = base + WD_;
+        if (SCALAR) {
+            uint8_t* sBd = base + BD_;
+            wait_mma(&sh.opI[0], par);
+            umma::gemm(tmem + 0, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_k(sWD, sWD + 16384, 128), 128, 128, 64, 0u);
+            umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 64), umma::opnd_mn(sWD, sWD + 16384, 128, 0), 128, 64, 64, 0u);
+            umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_mn(sBd, sBd + 8192, 64, 0), 128, 64, 64, 1u);
+        } else {
+#pragma unroll
+            for (int I = 3; I >= 0; --I) {                 // the column tiles arrive block by block, the largest first
+                wait_mma(&sh.opI[I], par);
+                const int nj = 16 * (I + 1);
+                // both row terms (dq_row | T) of the block in one N = 32 product
+                umma::gemm(tmem + 32 * I, umma::opnd_mn(base + kc_hi(I), base + kc_lo(I), nj), umma::opnd_k(sWD, sWD + 16384, 128, 32 * I), 128, 32, nj, 0u);
+                umma::gemm(tmem + ccol(I), umma::opnd_mn(sKQ, sKQ + 32768, 128, 32 * I), umma::opnd_mn(sWD, sWD + 16384, 128, 32 * I), 128, nj, 32, 0u);
+            }
+        }
+        umma::commit(&sh.mmI);
+    }
+}
+
+// S, dO, Vd, dVd and A of the next item are requested as soon as the intra-chunk products of the current one are done (the epilogue reads
+// accumulators, the scratch and the raw rows only), dS' once dVd and A have been read and the scratch is free.
+template <bool SCALAR>
+__device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+    using namespace bc;
+    auto src = [](const void* t, size_t it, uint32_t bytes, uint32_t off = 0) { return static_cast<const uint8_t*>(t) + it * bytes + off; };
+    uint32_t n = 0;
+    for (ItemWalk w(p.L); w.valid(); w.next(), ++n) {
+        const size_t it = w.item();
+        if (n) umma::mbar_wait(&sh.mmI, (n & 1) ^ 1);
+        umma::mbar_expect_tx(&sh.fullW, umma::CHUNK_TILE_BYTES + umma::QUARTER_TILE_BYTES);
+        umma::bulk_load(base + W_, src(p.dVd_t, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullW);
+        umma::bulk_load(base + A_, src(p.A, it, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES, &sh.fullW);
+        umma::mbar_expect_tx(&sh.fullS, umma::STATE_TILE_BYTES + 2 * umma::CHUNK_TILE_BYTES);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            umma::bulk_load(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
+        umma::bulk_load(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
+        umma::bulk_load(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
+        umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read; those products were issued after the scratch was free
+        umma::mbar_expect_tx(&sh.fullT, umma::STATE_TILE_BYTES);
+        umma::bulk_load(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
+        // Between here and the epilogue nothing else is fetched.  Scalar gate: the next item's tiles start on their way from HBM into L2 (1465 ->
+        // 1388 us on 4 x 16k tokens x 16 heads; its items are short and the copies were late).  With the per-channel gate the same hint
+        // costs 2 % (3.92 -> 4.02 ms on 64k packed tokens x 32 heads).
+        ItemWalk nx = w;
+        nx.next();
+        if (SCALAR && nx.valid()) {
+            const size_t in = nx.item();
+            umma::mbar_wait(&sh.mmT, n & 1);
+            umma::l2_prefetch(src(p.dVd_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
+            umma::l2_prefetch(src(p.A, in, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES);
+            umma::l2_prefetch(src(p.dO_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
+            umma::l2_prefetch(src(p.Vd, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
+            umma::l2_prefetch(src(p.h, in, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES);
+            umma::l2_prefetch(src(p.dh, in, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES);
+        }
+    }
+}
+
+// Compute warps.  Thread (q, lane, cg): accumulator lane `row` = 32 q + lane, columns or rows [16 cg, 16 cg + 16).
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+    using namespace bc;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int q = warp & 3, cg = warp >> 2, row = q * 32 + lane;
+    const int HV = p.L.HV, HK = p.L.HK;
+    const uint32_t tmem = sh.tmem;
+    Scratch& scr = *reinterpret_cast<Scratch*>(base + SCR_);
+    float (*early_ga)[DK] = reinterpret_cast<float (*)[DK]>(base + EARLY_GA);        // anchor rows while the scratch is still dS'
+    constexpr bool STASH = DT != MKDA_F32;                 // fp32 rows do not fit: the epilogue reads them from global memory
+
+    // chunk table entries and the per-row scalars (beta | L2 statistics | scalar gate) travel one item ahead: every address of an item
+    // depends on the former, and a scalar stored where it is requested would be waited for there
+    ItemWalk w(p.L);
+    int next_start = 0, next_len = 1;
+    float ahead0 = 0.f, ahead1 = 0.f;
+    auto row_scalars = [&](const ItemWalk& it) {
+        const int h = it.head(), hk = it.hk(), r = tid & (CH - 1), rr = r < next_len ? r : next_len - 1;
+        const size_t tk = (size_t)(next_start + rr) * HK + hk, tv = (size_t)(next_start + rr) * HV + h;
+        if (tid < CH) {
+            ahead0 = r < next_len ? p.beta[tv] : 0.f;
+        } else if (tid < 2 * CH) {
+            ahead0 = r < next_len ? (p.k_rstd ? p.k_rstd[tk] : 1.f) : 0.f;
+            ahead1 = r < next_len ? (p.q_rstd ? p.q_rstd[tk] : 1.f) : 0.f;
+        } else if (SCALAR && tid < 3 * CH) {
+            ahead0 = p.g_c[tv];                            // rows past the end: the last valid one
+        }
+    };
+    if (w.valid()) {
+        next_start = p.L.chunk_start[w.chunk()]; next_len = p.L.chunk_len[w.chunk()];
+        row_scalars(w);
+    }
+    for (uint32_t n = 0; w.valid(); ++n) {
+        const uint32_t par = n & 1;
+        const int c = w.chunk(), hk = w.hk(), h = w.head(), start = next_start, len = next_len;
+        const size_t item = w.item();
+        const bool first_of_group = w.j == 0;
+        ItemWalk nxt = w;
+        nxt.next();
+        if (nxt.valid() && nxt.grp != w.grp) { next_start = p.L.chunk_start[nxt.chunk()]; next_len = p.L.chunk_len[nxt.chunk()]; }
+
+        bool tiny = false;
+        if (tid < CH) {
+            sh.beta[tid] = ahead0;
+            tiny = !p.beta_sigmoid && tid < len && fabsf(ahead0) < 1e-12f;
+        } else if (tid < 2 * CH) {
+            sh.rk[tid - CH] = ahead0; sh.rq[tid - CH] = ahead1;
+        } else if (SCALAR && tid < 3 * CH) {
+            sh.gs[tid - 2 * CH] = ahead0;
+        }
+        const bool long_way = sync_compute_or(tiny);       // dbeta of this chunk cannot be formed as Z_ii / beta_i
+        if (nxt.valid()) row_scalars(nxt);
+
+        // ---- dW: rows of the stacked tile, dv = beta dW ----
+        wait_mma(&sh.mmW, par);
+        {
+            const int t = row & 63, v0 = (q < 2 ? 0 : 64) + 16 * cg;      // token, first of 16 values
+            float dw[16], x0[8], x1[8];
+            umma::tmem_ld16(umma::tmem_addr(tmem, warp, DW + v0), dw);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { x0[j] = dw[j]; x1[j] = dw[8 + j]; }
+            store_split8(base + R_, base + R_ + 32768, 128, 64 + t, v0 >> 3, x0);
+            store_split8(base + R_, base + R_ + 32768, 128, 64 + t, (v0 >> 3) + 1, x1);
+            signal(&sh.opW, lane);
+            if (long_way) {                                // rowsum(dW * V), the partial sums of the eight warps of a token added in turn
+                float s = 0.f;
+                const size_t tv = ((size_t)(start + (t < len ? t : len - 1)) * HV + h) * 128 + v0;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) s = fmaf(dw[j], ld1(p.v, DT, tv + j), s);
+                for (int k = 0; k < 8; ++k) {
+                    if (k == 2 * cg + (q >> 1)) sh.dbw[t] = k ? sh.dbw[t] + s : s;
+                    sync_compute();
+                }
+            }
+            if (t < len) {
+                const float bt = sh.beta[t];
+                const size_t tv = ((size_t)(start + t) * HV + h) * 128 + v0;
+#pragma unroll
+                for (int j = 0; j < 16; j += 8) {
+                    float o8[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o8[e] = bt * dw[j + e];
+                    st8<DT>(p.dv, tv + j, o8);
+                }
+            }
+        }
+        // ---- k, q, g rows, used once the state products are under way ----
+        Raw8 wk[2], wq[2];
+        float vg[2][8];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int i = tid + m * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
+            const size_t tk = ((size_t)(start + rr) * HK + hk) * 128 + k8 * 8;
+            ldraw8<DT>(p.k, tk, wk[m]);
+            ldraw8<DT>(p.q, tk, wq[m]);
+            if (!SCALAR) ldg8(p.g_c, MKDA_F32, ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[m]);
+        }
+        // ---- dgl[c] = sum_v S[c][v] dS'[c][v] from the two tiles: warp = 8 channels, lanes = v ----
+        umma::mbar_wait(&sh.fullS, par);
+        umma::mbar_wait(&sh.fullT, par);
+        {
+            float acc[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const uint32_t off = umma::tile_chunk_offset(128, lane + 32 * m, warp);
+                const uint4 a4 = *reinterpret_cast<const uint4*>(base + S_ + off), b4 = *reinterpret_cast<const uint4*>(base + S_ + 32768 + off);
+                const uint4 c4 = *reinterpret_cast<const uint4*>(base + T_ + off), d4 = *reinterpret_cast<const uint4*>(base + T_ + 32768 + off);
+                const uint32_t ah[4] = {a4.x, a4.y, a4.z, a4.w}, al[4] = {b4.x, b4.y, b4.z, b4.w};
+                const uint32_t dh[4] = {c4.x, c4.y, c4.z, c4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float s0 = __uint_as_float(ah[e] << 16) + __uint_as_float(al[e] << 16);
+                    const float s1 = __uint_as_float(ah[e] & 0xffff0000u) + __uint_as_float(al[e] & 0xffff0000u);
+                    const float d0 = __uint_as_float(dh[e] << 16) + __uint_as_float(dl[e] << 16);
+                    const float d1 = __uint_as_float(dh[e] & 0xffff0000u) + __uint_as_float(dl[e] & 0xffff0000u);
+                    acc[2 * e] = fmaf(s0, d0, acc[2 * e]);
+                    acc[2 * e + 1] = fmaf(s1, d1, acc[2 * e + 1]);
+                }
+            }
+            warp_colsum(acc, lane);
+            if ((lane & 3) == 0) sh.dgl[warp * 8 + (lane >> 2)] = acc[0];
+        }
+        wait_mma(&sh.mmL, par);
+        if (!SCALAR) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
+                if ((r & 15) == 0) sts8(&early_ga[r >> 4][k8 * 8], vg[m]);
+            }
+        }
+        sync_compute();                                    // every thread has read its part of S; anchor rows visible
+        // ---- [Qr; beta Kr] over S while Db is computed, then the weights and the column tiles ----
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int i = tid + m * 512, r = i >> 4, k8 = i & 15, I0 = r >> 4;
+            const float rk = sh.rk[r], rq = sh.rq[r];
+            float k8v[8], q8v[8];
+            unpack8<DT>(wk[m], k8v);
+            unpack8<DT>(wq[m], q8v);
+            if (STASH) {
+                *reinterpret_cast<uint4*>(base + stash(0, r) + k8 * 16) = wk[m].a;
+                *reinterpret_cast<uint4*>(base + stash(1, r) + k8 * 16) = wq[m].a;
+            }
+            uint8_t* sKQ = base + S_;
+            if (SCALAR) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { k8v[e] *= rk; q8v[e] *= rq; }
+                store_split8(sKQ, sKQ + 32768, 128, r, k8, k8v);
+                store_split8(sKQ, sKQ + 32768, 128, 64 + r, k8, q8v);
+            } else {
+                float ga[8];
+                lds8(&early_ga[I0][k8 * 8], ga);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float f = ex2f_(vg[m][e] - ga[e]);
+                    k8v[e] = k8v[e] * (rk * sh.beta[r]) * f;
+                    q8v[e] = q8v[e] * rq * f;
+                }
+                store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, q8v);
+                store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, k8v);
+            }
+        }
+        wait_mma(&sh.mmT, par);
+        // lanes 0..63 hold D1 = dO Vd^T, lanes 64..127 Z = dW Vd^T = -dL
+        {
+            const int i = row & 63;
+            float d[16];
+            umma::tmem_ld16(umma::tmem_addr(tmem, warp, D1 + cg * 16), d);
+            const float gi = SCALAR ? sh.gs[i] : 0.f, f = q < 2 ? p.scale : -1.f, bt = SCALAR ? sh.beta[i] : 0.f;
+            // rows of the stacked weight tile: per channel 32 I + r = Wq, 32 I + 16 + r = dLs; scalar gate [Wq E; dLs E]
+            const int wrow = SCALAR ? row : 32 * (i >> 4) + (i & 15) + (q < 2 ? 0 : 16);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                float w8[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int j = cg * 16 + hf * 8 + e;
+                    const float E = SCALAR ? ex2f_(fminf(gi - sh.gs[j], 0.f)) : 1.f;
+                    w8[e] = j < i && i < len ? f * d[hf * 8 + e] * E : 0.f;
+                    // diagonals: scale dAqk_ii, and (dW Vd^T)_ii for dbeta (predicated stores: selecting d[i & 15] first makes the compiler
+                    // index it in local memory, which every warp then waits for behind the next barrier)
+                    if (j == i) {
+                        if (q < 2) sh.diag[i] = i < len ? p.scale * d[hf * 8 + e] : 0.f;
+                        else if (!long_way) sh.dbw[i] = d[hf * 8 + e];
+                    }
+                }
+                store_split8(base + WD_, base + WD_ + 16384, 128, wrow, 2 * cg + hf, w8);
+                if (SCALAR && q >= 2) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) w8[e] *= bt;
+                    store_split8(base + BD_, base + BD_ + 8192, 64, i, 2 * cg + hf, w8);
+                }
+            }
+        }
+        if (SCALAR) {
+            if (tid < CH) {
+                const float g = sh.gs[tid];
+                scr.up[tid] = ex2f_(g);
+                scr.re[tid] = ex2f_(sh.gs[CH - 1] - g);
+            }
+            sync_compute();
+        } else {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
+                if ((r & 15) == 0) sts8(&scr.ga[r >> 4][k8 * 8], vg[m]);
+                if (r == CH - 1) sts8(&scr.ga[4][k8 * 8], vg[m]);          // rows past the end carry the last valid row's
+            }
+            sync_compute();
+            float k8v[2][8];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float rk = sh.rk[(tid + m * 512) >> 4];
+                unpack8<DT>(wk[m], k8v[m]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) k8v[m][e] *= rk;
+            }
+            const int k8 = tid & 15, r0 = tid >> 4;        // rows r0 (block 0 or 1) and 32 + r0 (block 2 or 3)
+            float ga[2][8];
+            lds8(&scr.ga[3][k8 * 8], ga[1]);
+#pragma unroll
+            for (int I = 3; I >= 0; --I) {
+                if (I) lds8(&scr.ga[I - 1][k8 * 8], ga[(I - 1) & 1]);      // one block ahead
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int r = r0 + 32 * m;
+                    if (r >= 16 * (I + 1)) continue;       // warp-uniform
+                    float t8[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) t8[e] = k8v[m][e] * ex2f_(ga[I & 1][e] - vg[m][e]);
+                    store_split8(base + kc_hi(I), base + kc_lo(I), 16 * (I + 1), r, k8, t8);
+                }
+                signal(&sh.opI[I], lane);
+            }
+        }
+        if (SCALAR) signal(&sh.opI[0], lane);
+
+        // ---- epilogue: channel `row`, rows 16 cg .. 16 cg + 15; its inputs are fetched while the intra-chunk products run ----
+        // With e = 2^(g - ga[cg]) (the anchor of the row block), ea = 2^ga[cg], h1 = 2^(ga[cg + 1] - g) <= 1 (ga[4] = gL), every decay an element
+        // needs is one of e, 1 / e and h1 times a per-thread factor:
+        //   x = dq_row / e + scale ea Dq     y = T / e - ea Dk     z = h1 (fL Db + sum_{I > cg} f_I C_I) + C_cg / e
+        //   dq = e x + d k     dk = beta e y + z + d q     dg' = q e x + k (beta e y - z)     dbeta term = k e y      (d = scale dAqk_ii)
+        float kq[16], qq[16], gg[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const int i = 16 * cg + r, ii = i < len ? i : len - 1;
+            const size_t tk = ((size_t)(start + ii) * HK + hk) * 128 + row;
+            if (!STASH) {
+                kq[r] = ld1(p.k, DT, tk);
+                qq[r] = ld1(p.q, DT, tk);
+            }
+            if (!SCALAR) gg[r] = p.g_c[((size_t)(start + ii) * HV + h) * 128 + row];
+        }
+        float raw_beta = 0.f;
+        if (tid < len && p.beta_sigmoid) raw_beta = ld1(p.beta_raw, p.beta_dtype, (size_t)(start + tid) * HV + h);
+        float a0 = 0.f, a1 = 0.f, ea = 1.f, fL = 1.f, f2 = 0.f, f3 = 0.f, egL;
+        if (!SCALAR) {
+            a0 = scr.ga[cg][row]; a1 = scr.ga[cg + 1][row];
+            const float gL = scr.ga[4][row];
+            ea = ex2f_(a0); fL = ex2f_(gL - a1); egL = ex2f_(gL);
+            if (cg < 2) f2 = ex2f_(scr.ga[cg + 2][row] - a1);
+            if (cg < 1) f3 = ex2f_(scr.ga[cg + 3][row] - a1);
+        } else {
+            egL = ex2f_(sh.gs[CH - 1]);
+        }
+        const size_t obk = ((size_t)c * HK + hk) * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
+        float* __restrict__ oq = p.dq_v + obk;
+        float* __restrict__ ok = p.dk_v + obk;
+        float* __restrict__ og = SCALAR ? p.dgp + item * CH : p.dgp + item * (size_t)(CH * DK) + row;
+        float cs = 0.f, dg_last = 0.f;
+        wait_mma(&sh.mmI, par);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int c0 = 16 * cg + 8 * hf;
+            float x[8], y[8], z[8], ci[8], t[8];
+            if (SCALAR) {
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DQ + c0), umma::tmem_addr(tmem, warp, c0), t, x);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) x[r] = fmaf(p.scale * scr.up[c0 + r], t[r], x[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DKB + c0), umma::tmem_addr(tmem, warp, 64 + c0), t, y);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) y[r] = fmaf(-scr.up[c0 + r], t[r], y[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DB + c0), umma::tmem_addr(tmem, warp, 128 + c0), t, z);
+            } else {
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DQ + c0), umma::tmem_addr(tmem, warp, 32 * cg + 8 * hf), t, x);
+                const float sa = p.scale * ea;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) x[r] = fmaf(sa, t[r], x[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DKB + c0), umma::tmem_addr(tmem, warp, 32 * cg + 16 + 8 * hf), t, y);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) y[r] = fmaf(-ea, t[r], y[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DB + c0), umma::tmem_addr(tmem, warp, ccol(cg) + c0), t, ci);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) { t[r] *= fL; z[r] = t[r]; }
+                if (cg < 2) {                              // warp-uniform
+                    float u[8], v[8];
+                    umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, ccol(cg + 1) + c0), umma::tmem_addr(tmem, warp, ccol(cg + 2) + c0), u, v);
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) z[r] = fmaf(f2, v[r], z[r] + u[r]);
+                }
+                if (cg == 0 || cg == 2) {
+                    float u[8];
+                    umma::tmem_ld8(umma::tmem_addr(tmem, warp, ccol(3) + c0), u);
+                    const float f = cg == 0 ? f3 : 1.f;
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) z[r] = fmaf(f, u[r], z[r]);
+                }
+            }
+            float bsv[8], dgs[8];                          // bsv: long way only
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int i = c0 + r, rr = 8 * hf + r, ii = i < len ? i : len - 1;
+                const bool ok_row = i < len;
+                float kv, qv;
+                if (STASH) {                               // rows past the end carry the last valid one's
+                    kv = ld1(base + stash(0, i), DT, row);
+                    qv = ld1(base + stash(1, i), DT, row);
+                } else {
+                    kv = kq[rr]; qv = qq[rr];
+                }
+                kv *= sh.rk[ii]; qv *= sh.rq[ii];
+                float ex, ey, zz;
+                if (SCALAR) {
+                    ex = x[r]; ey = y[r];
+                    const float w2 = scr.re[i] * t[r];
+                    zz = w2 + z[r];
+                    if (ok_row) cs = fmaf(kv, w2, cs);
+                } else {
+                    const float g = gg[rr], e = ex2f_(g - a0), ei = ex2f_(a0 - g), h1 = ex2f_(a1 - g);
+                    ex = e * x[r]; ey = e * y[r];
+                    zz = fmaf(h1, z[r], ei * ci[r]);
+                    if (ok_row) cs = fmaf(kv * h1, t[r], cs);
+                }
+                const float bt = sh.beta[i], dgn = sh.diag[i], bey = bt * ey;
+                bsv[r] = kv * ey;
+                const float dg = ok_row ? fmaf(qv, ex, kv * (bey - zz)) : 0.f;
+                const float dq_e = ok_row ? fmaf(dgn, kv, ex) : 0.f;
+                const float dk_e = ok_row ? fmaf(dgn, qv, bey + zz) : 0.f;
+                if (first_of_group) { oq[i * DK] = dq_e; ok[i * DK] = dk_e; }
+                else { red_add(oq + i * DK, dq_e); red_add(ok + i * DK, dk_e); }
+                if (SCALAR) dgs[r] = dg;
+                else if (i == len - 1) dg_last = dg;
+                else og[i * DK] = dg;
+            }
+            if (long_way) {
+                warp_colsum(bsv, lane);
+                for (int k = 0; k < 4; ++k) {
+                    if (k == q && (lane & 3) == 0) sh.dbw[c0 + (lane >> 2)] += bsv[0];
+                    sync_compute();
+                }
+            }
+            if (SCALAR) {
+                warp_colsum(dgs, lane);
+                if ((lane & 3) == 0) scr.redg[q][c0 + (lane >> 2)] = dgs[0];
+            }
+        }
+        // gate term of the last valid row: column sum of the inter-chunk k gradient plus gl dgl
+        if (SCALAR) {
+            if (cg == 0) cs = fmaf(egL, sh.dgl[row], cs);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, o);
+            if (lane == 0) scr.col[0][warp] = cs;
+        } else {
+            scr.col[cg][row] = cs;
+        }
+        sync_compute();
+        if (!SCALAR && cg == (len - 1) >> 4)
+            og[(len - 1) * DK] = dg_last + (((scr.col[0][row] + scr.col[1][row]) + (scr.col[2][row] + scr.col[3][row])) + egL * sh.dgl[row]);
+        if (SCALAR && tid < CH) {
+            float t = (scr.redg[0][tid] + scr.redg[1][tid]) + (scr.redg[2][tid] + scr.redg[3][tid]);
+            if (tid == len - 1) {
+                float e = 0.f;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) e += scr.col[0][k];
+                t += e;
+            }
+            og[tid] = t;
+        }
+        if (tid < len) {
+            float db = sh.dbw[tid];
+            if (p.beta_sigmoid) db *= 1.f - sigmoidf_(raw_beta);          // Z / beta times beta_scale sg (1 - sg), with beta = beta_scale sg
+            else if (!long_way) db /= sh.beta[tid];
+            st1(p.dbeta, p.dbeta_dtype, (size_t)(start + tid) * HV + h, db);
+        }
+        signal(&sh.accFree, lane);
+        w = nxt;
+    }
+}
+
+template <int DT, bool SCALAR>
+__global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p) {
+    using namespace bc;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
+    Shared& sh = *reinterpret_cast<Shared*>(base + TILES);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        if (threadIdx.x == 0) atomicExch(&umma::g_timeout_flag, 1u);
+        return;
+    }
+    if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
+    if (threadIdx.x == 0) {
+        for (uint64_t* b : {&sh.fullW, &sh.fullS, &sh.fullT, &sh.mmW, &sh.mmL, &sh.mmT, &sh.mmI}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.opW, &sh.opI[0], &sh.opI[1], &sh.opI[2], &sh.opI[3], &sh.accFree}) umma::mbar_init(b, COMPUTE / 32);
+        umma::fence_barrier_init();
+    }
+    publish();
+    if (warp >= COMPUTE / 32) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if (warp == WARP_MMA) {
+            if (elect_one()) bwd_chunk_issue<SCALAR>(p, base, sh);
+            __syncwarp();
+        } else if (warp == WARP_LOAD) {
+            if (elect_one()) bwd_chunk_load<SCALAR>(p, base, sh);
+            __syncwarp();
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        bwd_chunk_compute<DT, SCALAR>(p, base, sh);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) umma::tmem_dealloc(sh.tmem, 512);
+}
+
+template <int DT, bool SCALAR>
+static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, cudaStream_t stream) {
+    auto kern = bwd_chunk_tc_kernel<DT, SCALAR>;
+    if (int e = ensure_smem((const void*)kern, bc::SMEM, "bwd_chunk")) return e;
+    static const int regs = kernel_registers((const void*)kern);
+    if (regs < bc::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "bwd_chunk: built with fewer registers than its warps redistribute");
+    const int groups = p->L.NC * p->L.HK;                  // a CTA takes whole (chunk, q/k head) groups
+    kern<<<groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream>>>(*p);
+    return check_launch("bwd_chunk");
+}
+int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream) {
+    switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {
+        case MKDA_F32 * 2: return launch_bwd_chunk_tc_t<MKDA_F32, false>(p, stream);
+        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_t<MKDA_BF16, false>(p, stream);
+        case MKDA_F16 * 2: return launch_bwd_chunk_tc_t<MKDA_F16, false>(p, stream);
+        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_F32, true>(p, stream);
+        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_BF16, true>(p, stream);
+        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_F16, true>(p, stream);
+    }
+    return set_error(MKDA_ERR_ARG, "bwd_chunk: unsupported dtype");
+}
+
+int tc_bwd_chunk_status(unsigned int* out) {
+    return cudaMemcpyFromSymbol(out, umma::g_timeout_flag, sizeof(unsigned int)) == cudaSuccess ? 0 : -1;
+}
+int tc_bwd_chunk_status_clear() {
+    const unsigned int z = 0;
+    return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess ? 0 : -1;
+}
+
+}  // namespace mkda

@@ -67,12 +67,12 @@ def _f32(t):
 
 
 def gate_cumsum_fwd(lay, x, mode, A_log, dt_bias, lower_bound, HV, beta_raw=None, beta_sigmoid=False, beta_scale=1.0):
-    """x [B,T,HV,128] or [B,T,HV] -> (g_c fp32 [TT,HV,128], beta_e fp32 [TT,HV] or None)."""
+    """x [B,T,HV,128] or [B,T,HV] -> (g_c fp32 [TT,HV,128] or [TT,HV], beta_e fp32 [TT,HV] or None)."""
     scalar = x.dim() == 3
     p = STRUCTS["MkdaGateFwd"]()
     p.L = _layout_struct(lay, 1, HV)
     alloc = torch.empty if lay.covers_all else torch.zeros
-    g_c = alloc(lay.TT, HV, 128, dtype=torch.float32, device=x.device)
+    g_c = alloc(*((lay.TT, HV) if scalar else (lay.TT, HV, 128)), dtype=torch.float32, device=x.device)
     p.x, p.x_dtype, p.scalar_gate = _ptr(x), _dt(x), int(scalar)
     A_log, dt_bias = _f32(A_log), _f32(dt_bias)
     p.A_log, p.dt_bias = _ptr(A_log), _ptr(dt_bias)
@@ -328,7 +328,8 @@ def bwd_chunk(lay, q, k, v, q_rstd, k_rstd, g_c, beta_e, A, h, dh, Vd, dO_t, dVd
     dev = q.device
     alloc = torch.empty if lay.covers_all else torch.zeros
     z = lambda H: torch.empty(lay.NC, H, 64, 128, dtype=torch.float32, device=dev)      # noqa: E731  (fp32 [64][128] tiles)
-    dq_v, dk_v, dgp = z(HK), z(HK), z(HV)
+    dq_v, dk_v = z(HK), z(HK)
+    dgp = torch.empty(lay.NC, HV, 64, dtype=torch.float32, device=dev) if scalar_gate else z(HV)
     dbeta = alloc(lay.TT, HV, dtype=beta_raw.dtype, device=dev)
     dv = alloc(lay.TT, HV, 128, dtype=v.dtype, device=dev)
     p = STRUCTS["MkdaBwdChunk"]()
