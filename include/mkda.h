@@ -252,8 +252,8 @@ int mkda_epilogue_bwd_noalloc(const MkdaEpilogueBwdNoAlloc* p, void* stream);
 typedef struct {
     MkdaLayout L;
     const void* d_o; int do_dtype;                 /* [TT,HV,128], or NULL when dO_in_t is given */
-    const float* dO_in_t;      /* [NC,HV] row tiles of dO as written by mkda_epilogue_bwd_tiles, or NULL (then d_o is staged
-                                * through registers and, if dO_t is given, written there in tile form) */
+    const float* dO_in_t;      /* [NC,HV] row tiles of dO as written by mkda_epilogue_bwd_tiles, or NULL (then d_o is first
+                                * written to dO_t, which must be given, in tile form) */
     const float* kbar;         /* [NC,HV] row tiles as written by mkda_intra_fwd */
     const float* qs;           /* [NC,HV] row tiles as written by mkda_intra_fwd */
     const float* gl;           /* [NC,HV,128] as written by mkda_intra_fwd */
@@ -264,7 +264,7 @@ typedef struct {
     int state_v_first;         /* layout of dht / dh0 */
     float* dh;                 /* [NC,HV] state tiles: gradient of the state leaving each chunk, or NULL (not stored) */
     float* dVd_t;              /* [NC,HV] chunk tiles: dVd^T [v][token] (token columns past the end are zero), or NULL */
-    float* dO_t;               /* [NC,HV] row tiles: dO [token][v] as staged for the products (zero rows past the end), or NULL */
+    float* dO_t;               /* [NC,HV] row tiles: dO [token][v] (zero rows past the end); NULL when dO_in_t is given */
     float* dh0;                /* [NS,HV,128,128] gradient of the state entering each segment, or NULL */
     const int* warm_end;       /* [NS,HV] from mkda_warmup_chunks, or NULL: a reverse pass from zero (the segment pre-pass)
                                 * may start below this chunk index instead of at the segment's last chunk */
@@ -357,7 +357,8 @@ int mkda_warmup_chunks(const MkdaWarmup* p, void* stream);
  * {64, 128}.  No counterpart in the reference; used by the tests to validate the tcgen05 plumbing in isolation. */
 typedef struct {
     const float* A; const float* B; float* D; int N; int K;
-    int mode;      /* bit 0: stage B MN-major, bit 1: stage A MN-major (exercises both operand views) */
+    int mode;      /* bit 0: stage B MN-major, bit 1: stage A MN-major (exercises both operand views),
+                    * bit 2: A in tensor memory */
 } MkdaSelfTest;
 int mkda_selftest_umma(const MkdaSelfTest* p, void* stream);
 

@@ -162,7 +162,8 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     {
         pybind11::gil_scoped_release nogil;
         c10::cuda::CUDAGuard guard(c.dev);
-        for (Tensor* t : {&in.q, &in.k, &in.v, &in.x, &in.beta, &in.h0, &in.ep_gate}) *t = aligned(*t);
+        for (Tensor* t : {&in.q, &in.k, &in.v, &in.x, &in.beta, &in.ep_gate}) *t = aligned(*t);
+        in.h0 = aligned(in.h0, 32);
         bool any = false;
         if (c10::GradMode::is_enabled())
             for (Tensor* t : slots) any = any || (t->defined() && t->requires_grad());

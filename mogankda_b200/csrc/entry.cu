@@ -16,7 +16,8 @@ extern "C" int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream) {
 extern "C" int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream) {
     if (!p || !p->nw || !p->u || !p->kbar || !p->gl) return set_error(MKDA_ERR_ARG, "recur_fwd: null argument");
     if (any_misaligned(p->nw, p->u, p->kbar, p->gl, p->h, p->Vd)) return set_error(MKDA_ERR_ARG, "recur_fwd: tensors must be 16-byte aligned");
-    if (p->state_v_first && any_misaligned(p->h0, p->ht)) return set_error(MKDA_ERR_ARG, "recur_fwd: [V,K] states must be 16-byte aligned");
+    if (any_misaligned32(p->h, p->Vd) || (p->state_v_first && any_misaligned32(p->h0, p->ht)))
+        return set_error(MKDA_ERR_ARG, "recur_fwd: saved tiles and [V,K] states must be 32-byte aligned");
     if (p->want_transition && !p->mt) return set_error(MKDA_ERR_ARG, "recur_fwd: want_transition needs mt");
     if (p->L.NS == 0) return MKDA_OK;
     return launch_recur_fwd_tc(p, (cudaStream_t)stream);
@@ -31,13 +32,18 @@ extern "C" int mkda_out_fwd(const MkdaOutFwd* p, void* stream) {
 }
 
 extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) {
-    if (!p || (!p->d_o && !p->dO_in_t) || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw)
+    if (!p || !(p->dO_in_t || (p->d_o && p->dO_t)) || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw)
         return set_error(MKDA_ERR_ARG, "bwd_dh: null argument");
     if (any_misaligned(p->d_o, p->dO_in_t, p->kbar, p->qs, p->gl, p->Aqk, p->nw, p->dh, p->dVd_t, p->dO_t))
         return set_error(MKDA_ERR_ARG, "bwd_dh: tensors must be 16-byte aligned");
-    if (p->state_v_first && any_misaligned(p->dht, p->dh0)) return set_error(MKDA_ERR_ARG, "bwd_dh: [V,K] states must be 16-byte aligned");
+    if (any_misaligned32(p->dh, p->dVd_t) || (p->state_v_first && any_misaligned32(p->dht, p->dh0)))
+        return set_error(MKDA_ERR_ARG, "bwd_dh: saved tiles and [V,K] states must be 32-byte aligned");
     if (p->L.NS == 0) return MKDA_OK;
-    return launch_bwd_dh_tc(p, (cudaStream_t)stream);
+    if (p->dO_in_t) return launch_bwd_dh_tc(p, (cudaStream_t)stream);
+    if (int e = launch_rows_to_tiles(p->L, p->d_o, p->do_dtype, p->dO_t, (cudaStream_t)stream)) return e;
+    MkdaBwdDh q = *p;
+    q.dO_in_t = p->dO_t;
+    return launch_bwd_dh_tc(&q, (cudaStream_t)stream);
 }
 
 extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) {

@@ -25,11 +25,17 @@ template <typename... P>
 inline bool any_misaligned(P... ptrs) {
     return (((reinterpret_cast<uintptr_t>(static_cast<const void*>(ptrs)) & 15) != 0) || ...);
 }
+// ... and the tiles and states that leave in 32-byte pieces
+template <typename... P>
+inline bool any_misaligned32(P... ptrs) {
+    return (((reinterpret_cast<uintptr_t>(static_cast<const void*>(ptrs)) & 31) != 0) || ...);
+}
 // Number of SMs of the current device (cached per device).
 int sm_count();
 int launch_out_fwd_tc(const MkdaOutFwd* p, cudaStream_t stream);
 int tc_chunk_status(unsigned int* out);
 int tc_chunk_status_clear();
+int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void* tiles, cudaStream_t stream);
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream);
 int launch_bwd_dh_tc(const MkdaBwdDh* p, cudaStream_t stream);
 int tc_recur_status(unsigned int* out);

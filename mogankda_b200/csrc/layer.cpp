@@ -19,10 +19,10 @@ int dtype_code(const Tensor& t) {
     return -1;
 }
 
-Tensor aligned(const Tensor& t) {
+Tensor aligned(const Tensor& t, uintptr_t to) {
     if (!t.defined()) return t;
     Tensor c = t.is_contiguous() ? t : t.contiguous();
-    return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+    return reinterpret_cast<uintptr_t>(c.data_ptr()) % to ? c.clone() : c;
 }
 
 Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev) {
@@ -172,7 +172,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     const MkdaLayout L = c.layout();
     Grads g;
     if (!dy.defined()) dy = at::zeros({c.B, c.T, c.HV, 128}, in.q.options().dtype(c.has_ep ? at::kFloat : in.q.scalar_type()));
-    if (dht.defined()) dht = aligned_f32(dht);
+    if (dht.defined()) dht = aligned(aligned_f32(dht), 32);
     need_h0 = need_h0 && in.h0.defined();
 
     Arena tmp;
@@ -212,7 +212,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         d.dO_in_t = dO;
     } else {
         dy = aligned(dy);
-        d.d_o = dy.data_ptr(); d.do_dtype = dtype_code(dy);
+        d.d_o = dy.data_ptr(); d.do_dtype = dtype_code(dy); d.dO_t = dO;
     }
     d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw;
     if (need_h0) g.h0 = c.states(c.N);
@@ -229,7 +229,8 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     } else {
         full.dht = fptr(dht); full.state_v_first = c.vf; full.dh0 = fptr(g.h0);
     }
-    full.dh = dh; full.dVd_t = dVd; full.dO_t = c.has_ep ? nullptr : dO;
+    full.dh = dh; full.dVd_t = dVd;
+    if (c.segmented) full.dO_in_t = dO;                    // already in tile form
     check_rc(mkda_bwd_dh(&full, st), "mkda_bwd_dh");
     g.v = c.rows_out(c.HV, in.v.scalar_type());
     g.beta = c.like_out(in.beta);

@@ -17,7 +17,7 @@ using at::Tensor;
 int dtype_code(const Tensor& t);           // MKDA_F32 / MKDA_BF16 / MKDA_F16; TypeError otherwise
 // The kernels read and write their tensors with 16-byte vector accesses and bulk copies: operands are made contiguous and, where a
 // contiguous view starts at an odd storage offset, copied.
-Tensor aligned(const Tensor& t);
+Tensor aligned(const Tensor& t, uintptr_t to = 16);
 Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev);
 
 // The intermediates of one pass, requested together.  Up to ARENA_SINGLE bytes they share one allocation (a call on a short sequence

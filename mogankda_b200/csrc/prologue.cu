@@ -6,6 +6,7 @@
 #include <stdio.h>
 
 #include "host.h"
+#include "umma.cuh"
 
 namespace mkda {
 
@@ -523,6 +524,29 @@ __global__ void __launch_bounds__(128) epilogue_bwd_tiles_kernel(const MkdaEpilo
     p.part_w[(size_t)blockIdx.x * 128 + threadIdx.x] = t;
 }
 
+// Rows [TT,HV,128] -> row tiles [64 tokens][128] (bf16 hi / lo, rows past the end zero), one CTA per (chunk, v-head), heads fastest.
+template <int DT>
+__global__ void __launch_bounds__(256) rows_to_tiles_kernel(const MkdaLayout L, const void* rows, uint8_t* tiles) {
+    const int HV = L.HV, c = blockIdx.x / HV, h = blockIdx.x - c * HV, start = L.chunk_start[c], len = L.chunk_len[c];
+    uint8_t* tile = tiles + (size_t)blockIdx.x * 32768;
+    const int k8 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+    float v[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 16 * i;
+        ld8(rows, DT, ((size_t)(start + (r < len ? r : len - 1)) * HV + h) * 128 + k8 * 8, v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + 16 * i;
+        if (r >= len) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[i][e] = 0.f;
+        }
+        umma::store_split8(tile, tile + 16384, 64, r, k8, v[i]);
+    }
+}
+
 // Warm-up truncation table: one CTA per (segment, v-head), one thread per key channel (see MkdaWarmup).
 // gl = 2^gL may have underflowed to zero: log2 gives -inf, i.e. fully decayed.
 __global__ void __launch_bounds__(128) warmup_chunks_kernel(const MkdaWarmup p) {
@@ -543,6 +567,19 @@ __global__ void __launch_bounds__(128) warmup_chunks_kernel(const MkdaWarmup p) 
         p.warm_start[seg * HV + h] = ws;
         p.warm_end[seg * HV + h] = we;
     }
+}
+
+int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void* tiles, cudaStream_t stream) {
+    const int grid = L.NC * L.HV;
+    if (grid == 0) return MKDA_OK;
+    uint8_t* t = static_cast<uint8_t*>(tiles);
+    switch (dtype) {
+        case MKDA_F32: rows_to_tiles_kernel<MKDA_F32><<<grid, 256, 0, stream>>>(L, rows, t); break;
+        case MKDA_BF16: rows_to_tiles_kernel<MKDA_BF16><<<grid, 256, 0, stream>>>(L, rows, t); break;
+        case MKDA_F16: rows_to_tiles_kernel<MKDA_F16><<<grid, 256, 0, stream>>>(L, rows, t); break;
+        default: return set_error(MKDA_ERR_ARG, "bwd_dh: unsupported dtype");
+    }
+    return check_launch("rows_to_tiles");
 }
 
 }  // namespace mkda

@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const MkdaSelfTes
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5;
-    if (warp == 0) umma::tmem_alloc(&tmem_slot, 128);
+    if (warp == 0) umma::tmem_alloc(&tmem_slot, 256);
     if (tid == 0) { umma::mbar_init(&bar, 1); umma::fence_barrier_init(); }
     // stage: chunk index i -> (row, 8-column chunk); lanes walk along K for A and along rows for B (both addressings)
     const int a_mn = p.mode & 2, b_mn = p.mode & 1;
@@ -56,12 +56,28 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const MkdaSelfTes
             umma::store_split8(b_hi, b_lo, K, k, n8, v);
         }
     }
+    const bool a_tmem = p.mode & 4;
+    __syncthreads();
+    umma::fence_after_sync();
+    if (a_tmem) {       // A as packed bf16 pairs: thread = row, hi in columns 128.., lo in columns 192..
+        for (int k0 = 0; k0 < K; k0 += 16) {
+            uint32_t h[8], l[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) umma::split2(p.A[(size_t)tid * K + k0 + 2 * e], p.A[(size_t)tid * K + k0 + 2 * e + 1], h[e], l[e]);
+            umma::tmem_st8(umma::tmem_addr(tmem_slot, warp, 128 + k0 / 2), h);
+            umma::tmem_st8(umma::tmem_addr(tmem_slot, warp, 192 + k0 / 2), l);
+        }
+        umma::tmem_wait_st();
+    }
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    if (tid == 0) {
+    if (tid == 0 && a_tmem) {
+        umma::gemm_ta(tmem, tmem + 128, tmem + 192, b_mn ? umma::opnd_mn(b_hi, b_lo, K) : umma::opnd_k(b_hi, b_lo, N), N, K, 0u);
+        umma::commit(&bar);
+    } else if (tid == 0) {
         const umma::Opnd oa = a_mn ? umma::opnd_mn(a_hi, a_lo, K) : umma::opnd_k(a_hi, a_lo, 128);
         const umma::Opnd ob = b_mn ? umma::opnd_mn(b_hi, b_lo, K) : umma::opnd_k(b_hi, b_lo, N);
         umma::gemm(tmem, oa, ob, 128, N, K, 0u);
@@ -77,7 +93,7 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const MkdaSelfTes
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, 128);
+    if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
 // A wait that nothing will ever satisfy: every thread waits on a barrier without arrivals for at most `limit_cycles`,

@@ -82,25 +82,9 @@ __device__ __forceinline__ bool sync_compute_or(bool x) {
     return r != 0;
 }
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(umma::smem_u32(bar)) : "memory");
-}
-// this warp's shared-memory writes and accumulator reads are done: one arrival per warp
-__device__ __forceinline__ void signal(uint64_t* bar, int lane) {
-    umma::fence_async_smem();
-    umma::fence_before_sync();
-    __syncwarp();
-    if (lane == 0) arrive(bar);
-}
-__device__ __forceinline__ void wait_mma(uint64_t* bar, uint32_t parity) {
-    umma::mbar_wait(bar, parity);
-    umma::fence_after_sync();
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(pred));
-    return pred != 0;
-}
+using umma::elect_one;
+using umma::signal;
+using umma::wait_mma;
 }  // namespace bc
 
 // fire-and-forget fp32 addition in global memory

@@ -36,15 +36,15 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
     return r;
 }
+// a pair of fp32 values as packed bf16 pairs: hi = bf16(v), lo = bf16(v - hi)
+__device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& l) {
+    h = pack_bf16x2(a, b);
+    l = pack_bf16x2(a - __uint_as_float(h << 16), b - __uint_as_float(h & 0xffff0000u));
+}
 __device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, int r, int k8, const float (&v)[8]) {
     uint32_t h[4], l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        h[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-        const float ra = v[2 * i] - __uint_as_float(h[i] << 16);
-        const float rb = v[2 * i + 1] - __uint_as_float(h[i] & 0xffff0000u);
-        l[i] = pack_bf16x2(ra, rb);
-    }
+    for (int i = 0; i < 4; ++i) split2(v[2 * i], v[2 * i + 1], h[i], l[i]);
     const uint32_t off = tile_chunk_offset(R, r, k8);
     *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
@@ -138,6 +138,27 @@ __device__ __forceinline__ void gemm(uint32_t tmem_d, const Opnd& a, const Opnd&
     }
 }
 
+// The same products with the A operand in tensor memory: lane = row m, each 32-bit column two consecutive bf16 values of k; `ah` / `al` are
+// the column addresses of its hi and lo parts (KT / 2 columns each).  Nothing of A is fetched from shared memory.
+__device__ __forceinline__ void mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        :: "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void gemm_ta(uint32_t tmem_d, uint32_t ah, uint32_t al, const Opnd& b, int N, int KT, uint32_t accumulate) {
+    const uint32_t idesc = idesc_bf16(128, N, 0, b.mn);
+    const uint64_t bh = opnd_base_desc(b, b.hi), bl = opnd_base_desc(b, b.lo);
+#pragma unroll
+    for (int ks = 0; ks < KT / 16; ++ks) {
+        const uint32_t bo = opnd_step16(b, ks);
+        mma_bf16_ta(tmem_d, al + ks * 8, bh + bo, idesc, accumulate);
+        mma_bf16_ta(tmem_d, ah + ks * 8, bl + bo, idesc, 1u);
+        mma_bf16_ta(tmem_d, ah + ks * 8, bh + bo, idesc, 1u);
+        accumulate = 1u;
+    }
+}
+
 // ---- synchronisation -----------------------------------------------------------------------------------------
 // True in exactly one thread of warp 0 (call with warp 0 converged).  The warp index comes from a shuffle and the lane
 // from elect.sync, so the compiler sees a warp-uniform branch around the MMA issue and can keep the descriptors and
@@ -186,6 +207,34 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     // mkda_device_status_clear().
     const long long limit = *(volatile unsigned int*)&g_timeout_flag ? (1ll << 16) : (1ll << 27);
     return mbar_wait_limited(bar, parity, limit, &g_timeout_flag);
+}
+
+// ---- warp roles ----------------------------------------------------------------------------------------------------
+// Kernels with role-split warps join them through mbarriers: one arrival per producing warp once its shared-memory writes, tensor-memory
+// writes and accumulator reads are done.
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void signal(uint64_t* bar, int lane) {
+    fence_async_smem();
+    fence_before_sync();
+    __syncwarp();
+    if (lane == 0) arrive(bar);
+}
+// the same for a warp that has touched tensor memory only
+__device__ __forceinline__ void signal_tmem(uint64_t* bar, int lane) {
+    fence_before_sync();
+    __syncwarp();
+    if (lane == 0) arrive(bar);
+}
+__device__ __forceinline__ void wait_mma(uint64_t* bar, uint32_t parity) {
+    mbar_wait(bar, parity);
+    fence_after_sync();
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(pred));
+    return pred != 0;
 }
 
 // ---- bulk copies of whole operand tiles ---------------------------------------------------------------------------
@@ -309,6 +358,16 @@ __device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, float (&a)[
                    "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "+r"(s[7]) :: "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) { a[i] = __uint_as_float(r[i]); b[i] = __uint_as_float(s[i]); }
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+           "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 // TMEM address of (lane quadrant of this warp, column)
 __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, int warp, int col) {

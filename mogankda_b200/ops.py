@@ -309,8 +309,8 @@ def bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, *, dht=None, seg_dht=None,
     if store:
         dh = torch.empty(lay.NC, HV, 128, 128, dtype=torch.float32, device=dev)
         dVd_t = torch.empty(lay.NC, HV, 64, 128, dtype=torch.float32, device=dev)
-        if dO_in_t is None:
-            dO_t = torch.empty(lay.NC, HV, 64, 128, dtype=torch.float32, device=dev)
+    if dO_in_t is None:
+        dO_t = torch.empty(lay.NC, HV, 64, 128, dtype=torch.float32, device=dev)
     dh0 = torch.empty(NS, HV, 128, 128, dtype=torch.float32, device=dev) if want_dh0 else None
     p.dh, p.dVd_t, p.dO_t, p.dh0 = _ptr(dh), _ptr(dVd_t), _ptr(None if dO_in_t is not None else dO_t), _ptr(dh0)
     if warm_end is not None:

@@ -23,3 +23,37 @@ def test_precomputed_beta_of_zero_and_near_zero(scalar, dtype):
     lv["beta"][1, 64 * 3 + 20, 1] = 0.0
     compare(run(mk.chunk_delta_rule, lv, do, dht, opts, None),
             run(orc.chunked_delta_rule, lv, do, dht, opts, None, f64=True))
+
+
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("N,K", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_tensor_core_product_with_the_left_operand_in_tensor_memory(b_mn, N, K):
+    """mkda_selftest_umma, mode bit 2: the error must be at the 2^-16 level of the split, as with both operands in shared memory."""
+    from mogankda_b200 import _lib
+    torch.manual_seed(11)
+    A, B, D = torch.randn(128, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.zeros(128, N, device="cuda")
+    p = _lib.STRUCTS["MkdaSelfTest"]()
+    p.A, p.B, p.D, p.N, p.K, p.mode = A.data_ptr(), B.data_ptr(), D.data_ptr(), N, K, 4 | b_mn
+    _lib.call("mkda_selftest_umma", p, torch.cuda.current_stream().cuda_stream)
+    ref = A.double() @ B.double().T
+    assert ((D.double() - ref).abs().max() / ref.abs().max()).item() < 5e-5
+
+
+@pytest.mark.parametrize("offset", [4, 8])
+def test_states_at_odd_storage_offsets(offset):
+    """[V,K] states travel in 32-byte pieces: views 16 and 32 bytes into their storage, and gradients that arrive as such views."""
+    lv, do, dht, opts, epi = make_inputs(B=2, T=150, dtype=torch.bfloat16, gate="eda", seed=43)
+    flat = torch.zeros(lv["h0"].numel() + offset, device="cuda")
+    flat[offset:] = lv["h0"].transpose(-1, -2).reshape(-1)
+    h0 = flat[offset:].view(lv["h0"].shape)
+    up = torch.zeros(dht.numel() + offset, device="cuda")
+    up[offset:] = dht.reshape(-1)
+
+    def call(h0, dht):
+        h0 = h0.detach().requires_grad_(True)
+        o, ht = mk.chunk_delta_rule(lv["q"], lv["k"], lv["v"], lv["g"], lv["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"], initial_state=h0,
+                                    state_v_first=True, **opts)
+        return o, ht, torch.autograd.grad(ht, h0, dht)[0]
+
+    for a, b in zip(call(h0.clone(), dht), call(h0, up[offset:].view(dht.shape))):
+        assert torch.equal(a, b)
