@@ -204,9 +204,24 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     // Bounded by wall time (SM clock): ~70 ms for the first wait that fails on a device, ~35 us afterwards, so a broken
     // launch drains quickly instead of serialising one long timeout per CTA.  The flag stays set until
-    // mkda_device_status_clear().
-    const long long limit = *(volatile unsigned int*)&g_timeout_flag ? (1ll << 16) : (1ll << 27);
-    return mbar_wait_limited(bar, parity, limit, &g_timeout_flag);
+    // mkda_device_status_clear().  It is looked at only by a wait that has already taken ~35 us: read up front it put a global load, i.e.
+    // 0.7 k cycles of latency and thousands under a saturated memory system, in front of every wait of every kernel.
+    const uint32_t addr = smem_u32(bar);
+    const long long t0 = clock64();
+    long long limit = 1ll << 16;
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(addr), "r"(parity), "r"(1000u) : "memory");
+        if (ok) return true;
+        if (clock64() - t0 > limit) {
+            if (limit == (1ll << 27) || *(volatile unsigned int*)&g_timeout_flag) break;
+            limit = 1ll << 27;
+        }
+    }
+    atomicExch(&g_timeout_flag, 1u);
+    return false;
 }
 
 // ---- warp roles ----------------------------------------------------------------------------------------------------
