@@ -176,7 +176,7 @@ KERNEL_ENTRY = (("gate_cumsum_fwd", "mkda_gate_cumsum_fwd"), ("gate_bwd", "mkda_
                 ("l2norm_rstd", "mkda_l2norm_rstd"), ("intra_fwd", "mkda_intra_fwd"), ("recur_fwd", "mkda_recur_fwd"),
                 ("out_fwd", "mkda_out_fwd"), ("epilogue_bwd_tiles", "mkda_epilogue_bwd_tiles"), ("epilogue_bwd", "mkda_epilogue_bwd"),
                 ("bwd_dh", "mkda_bwd_dh"), ("bwd_chunk", "mkda_bwd_chunk"), ("qk_grad_finish", "mkda_qk_grad_finish"),
-                ("combine", "mkda_state_combine"), ("warmup_chunks", "mkda_warmup_chunks"))
+                ("step_fwd", "mkda_step_fwd"), ("combine", "mkda_state_combine"), ("warmup_chunks", "mkda_warmup_chunks"))
 
 
 def kernel_times(step, steps):

@@ -71,7 +71,7 @@ typedef struct {
     void* dx; int dx_dtype;    /* [TT,HV,128] or [TT,HV] */
     int part_rows;             /* number of partial rows R (1 <= R <= NC): chunk c accumulates into row c % R */
     float* part_bias;          /* [R,HV,128] ([R,HV] scalar) partial sums of d/d(x+bias), or NULL */
-    float* part_alog;          /* same shape, partial sums of d/dA_log, or NULL */
+    float* part_alog;          /* [R,HV] partial sums of d/dA_log, or NULL */
 } MkdaGateBwd;
 int mkda_gate_bwd(const MkdaGateBwd* p, void* stream);
 
@@ -83,11 +83,18 @@ typedef struct {
 } MkdaReduce;
 int mkda_reduce_partials(const MkdaReduce* p, void* stream);
 
+/* Up to three such reductions in one launch (a job without `out` is skipped): the parameter gradients of a layer. */
+typedef struct {
+    MkdaReduce job[3];
+} MkdaReduceMulti;
+int mkda_reduce_multi(const MkdaReduceMulti* p, void* stream);
+
 /* rstd[r] = rsqrt(sum_c x[r,c]^2 + eps) for rows of 128.  Replaces l2norm_fwd (mogan_kda/utils/math.py:22-35);
  * the normalised rows themselves are never materialised (consumers multiply by rstd in fp32). */
 typedef struct {
     const void* x; int dtype; int rows; float eps;
     float* rstd;
+    const void* x2; float* rstd2;                  /* a second tensor of the same type and number of rows (q and k), or NULL */
 } MkdaL2Norm;
 int mkda_l2norm_rstd(const MkdaL2Norm* p, void* stream);
 
@@ -178,6 +185,25 @@ typedef struct {
     void* out; int out_dtype;  /* [TT,HV,128] */
 } MkdaOutFwd;
 int mkda_out_fwd(const MkdaOutFwd* p, void* stream);
+
+/* Forward pass over sequences of at most MKDA_STEP_MAX_TOKENS tokens (generation steps): gate, L2 norm, recurrence, output and epilogue in one
+ * kernel, token by token, with the state in registers.  Same results as the chunk kernels up to rounding; nothing is kept for a backward
+ * pass. */
+#define MKDA_STEP_MAX_TOKENS 16
+typedef struct {
+    MkdaLayout L;
+    int N; const int* seq_chunk_off;               /* sequences; [N+1] first chunk of each (at most one chunk per sequence) */
+    int longest;                                   /* tokens of the longest sequence */
+    const void* q; const void* k; const void* v; int qkv_dtype;
+    const void* x; int x_dtype; int scalar_gate;   /* gate input as in MkdaGateFwd */
+    const float* A_log; const float* dt_bias; int mode; float lower_bound;
+    const void* beta; int beta_dtype; int beta_sigmoid; float beta_scale;
+    int l2; float scale;
+    const float* h0; float* ht; int state_v_first; /* [N,HV,128,128] or NULL */
+    int has_norm; const void* norm_w; int norm_w_dtype; const void* gate; int gate_dtype; int act; float eps;      /* as in MkdaOutFwd */
+    void* out; int out_dtype;                      /* [TT,HV,128] */
+} MkdaStepFwd;
+int mkda_step_fwd(const MkdaStepFwd* p, void* stream);
 
 /* Gated RMSNorm backward.  Replaces rmsnorm_gated_bwd (mogan_kda/ops/kimi_delta_rule/epilogue.py:193-205). */
 /* CTA b of the gated RMSNorm backward walks the 64-row groups b, b + R, ... and writes one partial row. */
@@ -298,6 +324,8 @@ typedef struct {
                                 * scalar_gate its sum over the channels, [NC,HV,64] */
     void* dbeta; int dbeta_dtype;
     void* dv;                  /* [TT,HV,128] in qkv_dtype */
+    int per_v_head;            /* 1: dq_v / dk_v are [NC,HV] tiles, one per (chunk, v-head), and the (chunk, v-head) items are spread over the
+                                * CTAs one by one; mkda_qk_grad_finish adds the tiles */
 } MkdaBwdChunk;
 int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream);
 
@@ -311,6 +339,7 @@ typedef struct {
     const void* q; const void* k; int x_dtype;     /* raw q, k [TT,HK,128] */
     const float* q_rstd; const float* k_rstd;      /* [TT,HK], or NULL (no L2 norm) */
     void* dq; void* dk;                            /* [TT,HK,128] in x_dtype; tokens outside every chunk are not written */
+    int per_v_head;                                /* as in MkdaBwdChunk: the HV / HK tiles of each q/k head are added first */
 } MkdaQkGrad;
 int mkda_qk_grad_finish(const MkdaQkGrad* p, void* stream);
 

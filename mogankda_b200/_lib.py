@@ -12,7 +12,7 @@ import re
 HERE = os.path.dirname(os.path.abspath(__file__))
 HEADER = os.path.join(HERE, "..", "include", "mkda.h")
 ENTRY_POINTS = (
-    "mkda_gate_cumsum_fwd", "mkda_gate_bwd", "mkda_reduce_partials", "mkda_l2norm_rstd", "mkda_intra_fwd",
+    "mkda_gate_cumsum_fwd", "mkda_gate_bwd", "mkda_reduce_partials", "mkda_reduce_multi", "mkda_step_fwd", "mkda_l2norm_rstd", "mkda_intra_fwd",
     "mkda_recur_fwd", "mkda_out_fwd", "mkda_epilogue_bwd", "mkda_epilogue_bwd_tiles", "mkda_bwd_dh", "mkda_bwd_chunk",
     "mkda_qk_grad_finish", "mkda_state_combine", "mkda_warmup_chunks", "mkda_selftest_umma", "mkda_selftest_wait", "mkda_epilogue_bwd_noalloc",
 )
@@ -37,8 +37,9 @@ def _parse_header(path=HEADER):
             decl = " ".join(decl.split())
             if not decl:
                 continue
-            m = re.match(r"^(.*?)(\w+)$", decl)
+            m = re.match(r"^(.*?)(\w+)(?:\[(\d+)\])?$", decl)
             ctype_s, fname = m.group(1).strip(), m.group(2)
+            count = int(m.group(3) or 0)
             if "*" in ctype_s:
                 ct = ctypes.c_void_p
             elif ctype_s == "int":
@@ -49,7 +50,7 @@ def _parse_header(path=HEADER):
                 ct = STRUCTS[ctype_s]
             else:
                 raise RuntimeError(f"mkda.h: cannot map type {ctype_s!r} of field {fname}")
-            fields.append((fname, ct))
+            fields.append((fname, ct * count if count else ct))
         STRUCTS[name] = type(name, (ctypes.Structure,), {"_fields_": fields})
         order.append(name)
     return order

@@ -14,7 +14,7 @@ import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-SOURCES = ("host.cu", "entry.cu", "prologue.cu", "combine.cu", "selftest.cu", "tc_chunk.cu", "tc_recur.cu", "tc_intra.cu", "tc_bwd_chunk.cu")
+SOURCES = ("host.cu", "entry.cu", "prologue.cu", "combine.cu", "step.cu", "selftest.cu", "tc_chunk.cu", "tc_recur.cu", "tc_intra.cu", "tc_bwd_chunk.cu")
 HOST_SOURCES = ("layer.cpp", "binding.cpp")
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",

@@ -2,6 +2,7 @@
 // pass.  Every intermediate is a torch allocation on the current stream.
 #include "layer.h"
 
+#include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <limits>
@@ -56,15 +57,34 @@ bool rows_strides(const Tensor& t, int64_t& row, int64_t& col) {
     return !(col == 1 && row % 8) && row <= most && col <= most && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
 }
 
-Tensor reduce(const float* part, int rows, int cols, int group, cudaStream_t st, const at::Device& dev) {
-    Tensor out = new_cuda({cols / group}, at::kFloat, dev);
-    MkdaReduce p{};
-    p.in = part; p.rows = rows; p.cols = cols; p.group = group; p.out = fptr(out);
-    check_rc(mkda_reduce_partials(&p, st), "mkda_reduce_partials");
-    return out;
+// Few (chunk, q/k head) groups: handing a CTA a whole group of v-heads leaves others idle, and the extra tiles the finishing kernel then
+// has to add stay in L2.  Worth it only while the grid is a couple of waves.
+bool spread_v_heads(const Call& c) {
+    const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount, G = c.HV / c.HK;
+    const int64_t groups = (int64_t)c.NC * c.HK;
+    return groups <= 2 * sms && (groups * G + sms - 1) / sms < G * ((groups + sms - 1) / sms);
 }
 
 }  // namespace
+
+std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in) {
+    const Tensor alog = aligned_f32(in.A_log), bias = aligned_f32(in.dt_bias), w = aligned(in.ep_w);
+    Tensor out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type()), ht;
+    if (c.want_ht) ht = c.states(c.N);
+    MkdaStepFwd p{};
+    p.L = c.layout(); p.N = c.N; p.seq_chunk_off = c.seq_off; p.longest = c.longest;
+    p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
+    p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(alog); p.dt_bias = fptr(bias);
+    p.mode = c.mode; p.lower_bound = c.lower_bound; p.beta = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta); p.beta_sigmoid = c.beta_sigmoid;
+    p.beta_scale = c.beta_scale; p.l2 = c.l2; p.scale = c.scale; p.h0 = fptr(in.h0); p.ht = fptr(ht); p.state_v_first = c.vf; p.has_norm = c.has_ep;
+    if (c.has_ep) {
+        if (w.defined()) { p.norm_w = w.data_ptr(); p.norm_w_dtype = dtype_code(w); }
+        p.gate = in.ep_gate.data_ptr(); p.gate_dtype = dtype_code(in.ep_gate); p.act = c.act; p.eps = c.eps;
+    }
+    p.out = out.data_ptr(); p.out_dtype = dtype_code(out);
+    check_rc(mkda_step_fwd(&p, c10::cuda::getCurrentCUDAStream()), "mkda_step_fwd");
+    return {out, ht};
+}
 
 std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need_bwd, Saved& s) {
     cudaStream_t st = c10::cuda::getCurrentCUDAStream();
@@ -107,9 +127,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     if (c.l2) {
         MkdaL2Norm p{};
         p.dtype = c.qkv_dtype; p.rows = c.TT * c.HK; p.eps = 1e-6f;
-        p.x = in.q.data_ptr(); p.rstd = s.q_rstd;
-        check_rc(mkda_l2norm_rstd(&p, st), "mkda_l2norm_rstd");
-        p.x = in.k.data_ptr(); p.rstd = s.k_rstd;
+        p.x = in.q.data_ptr(); p.rstd = s.q_rstd; p.x2 = in.k.data_ptr(); p.rstd2 = s.k_rstd;
         check_rc(mkda_l2norm_rstd(&p, st), "mkda_l2norm_rstd");
     }
     {
@@ -184,13 +202,14 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     tmp.want(&dO, c.tiles(tile));
     tmp.want(&dh, c.tiles(MKDA_STATE_TILE_BYTES));
     tmp.want(&dVd, c.tiles(tile));
-    tmp.want(&dq_v, (int64_t)c.NC * c.HK * tile);
-    tmp.want(&dk_v, (int64_t)c.NC * c.HK * tile);
+    const bool spread = spread_v_heads(c);
+    tmp.want(&dq_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
+    tmp.want(&dk_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
     tmp.want(&dgp, c.tiles(c.scalar_gate ? 256 : tile));
     if (c.has_ep && in.ep_w.defined()) tmp.want(&part_w, (int64_t)w_rows * 512);
     if (c.mode != MKDA_GATE_PRECOMPUTED) {
         if (need_bias) tmp.want(&part_b, (int64_t)g_rows * g_width * 4);
-        if (need_alog) tmp.want(&part_a, (int64_t)g_rows * g_width * 4);
+        if (need_alog) tmp.want(&part_a, (int64_t)g_rows * c.HV * 4);
     }
     if (c.segmented) { tmp.want(&dloc, seg_states); tmp.want(&g_in, seg_states); }
     tmp.allocate(c.dev);
@@ -208,7 +227,6 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         p.gate = in.ep_gate.data_ptr(); p.gate_dtype = dtype_code(in.ep_gate); p.act = c.act; p.eps = c.eps;
         p.dO_t = dO; p.dgate = g.ep_gate.data_ptr(); p.dgate_dtype = dtype_code(g.ep_gate); p.part_rows = w_rows; p.part_w = part_w;
         check_rc(mkda_epilogue_bwd_tiles(&p, st), "mkda_epilogue_bwd_tiles");
-        if (part_w) g.ep_w = reduce(part_w, w_rows, 128, 1, st, c.dev).to(in.ep_w.scalar_type());
         d.dO_in_t = dO;
     } else {
         dy = aligned(dy);
@@ -240,7 +258,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.A = s.A; p.h = s.h;
         p.dh = dh; p.Vd = s.Vd; p.dO_t = dO; p.dVd_t = dVd; p.scale = c.scale; p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta);
         p.beta_sigmoid = c.beta_sigmoid; p.beta_scale = c.beta_scale; p.dq_v = dq_v; p.dk_v = dk_v; p.dgp = dgp; p.dbeta = g.beta.data_ptr();
-        p.dbeta_dtype = dtype_code(g.beta); p.dv = g.v.data_ptr();
+        p.dbeta_dtype = dtype_code(g.beta); p.dv = g.v.data_ptr(); p.per_v_head = spread;
         check_rc(mkda_bwd_chunk(&p, st), "mkda_bwd_chunk");
     }
     g.x = c.like_out(in.x);
@@ -250,15 +268,22 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound; p.dgp = dgp; p.dx = g.x.data_ptr(); p.dx_dtype = dtype_code(g.x);
         p.part_rows = g_rows; p.part_bias = part_b; p.part_alog = part_a;
         check_rc(mkda_gate_bwd(&p, st), "mkda_gate_bwd");
-        if (part_b) g.dt_bias = reduce(part_b, g_rows, g_width, 1, st, c.dev).view_as(in.dt_bias).to(in.dt_bias.scalar_type());
-        if (part_a) g.A_log = reduce(part_a, g_rows, g_width, c.scalar_gate ? 1 : 128, st, c.dev).view_as(in.A_log).to(in.A_log.scalar_type());
+    }
+    if (part_w || part_b || part_a) {                      // the parameter gradients' second stage, in one launch
+        MkdaReduceMulti p{};
+        if (part_w) { g.ep_w = new_cuda({128}, at::kFloat, c.dev); p.job[0] = {part_w, w_rows, 128, 1, fptr(g.ep_w)}; }
+        if (part_b) { g.dt_bias = new_cuda(in.dt_bias.sizes(), at::kFloat, c.dev); p.job[1] = {part_b, g_rows, g_width, 1, fptr(g.dt_bias)}; }
+        if (part_a) { g.A_log = new_cuda(in.A_log.sizes(), at::kFloat, c.dev); p.job[2] = {part_a, g_rows, c.HV, 1, fptr(g.A_log)}; }
+        check_rc(mkda_reduce_multi(&p, st), "mkda_reduce_multi");
+        auto cast = [](Tensor& t, const Tensor& like) { if (t.defined() && t.scalar_type() != like.scalar_type()) t = t.to(like.scalar_type()); };
+        cast(g.ep_w, in.ep_w); cast(g.dt_bias, in.dt_bias); cast(g.A_log, in.A_log);
     }
     g.q = c.rows_out(c.HK, in.q.scalar_type());
     g.k = c.rows_out(c.HK, in.k.scalar_type());
     {
         MkdaQkGrad p{};
         p.L = L; p.dq_v = dq_v; p.dk_v = dk_v; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.x_dtype = c.qkv_dtype;
-        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.dq = g.q.data_ptr(); p.dk = g.k.data_ptr();
+        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.dq = g.q.data_ptr(); p.dk = g.k.data_ptr(); p.per_v_head = spread;
         check_rc(mkda_qk_grad_finish(&p, st), "mkda_qk_grad_finish");
     }
     return g;

@@ -5,6 +5,7 @@
 #include "common.cuh"
 #include <stdio.h>
 
+#include "gate.cuh"
 #include "host.h"
 #include "umma.cuh"
 
@@ -19,34 +20,6 @@ __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// natural-log decay for one element; s = x + dt_bias, E = exp(A_log), lb = lower bound (< 0)
-__device__ __forceinline__ float gate_value(int mode, float s, float E, float lb) {
-    if (mode == MKDA_GATE_GDN) return fmaxf(-E * softplusf_(s), lb);
-    if (mode == MKDA_GATE_KIMI) return lb * sigmoidf_(E * s);
-    if (mode == MKDA_GATE_EDA) return lb + (-lb) * expf_(-(E / fabsf(lb)) * softplusf_(s));
-    return s;
-}
-// d gate / d s  and  d gate / d A_log
-__device__ __forceinline__ void gate_grad(int mode, float s, float E, float lb, float& ds, float& dA) {
-    if (mode == MKDA_GATE_GDN) {
-        const float sp = softplusf_(s);
-        const float keep = (-E * sp >= lb) ? 1.f : 0.f;    // clamp passes no gradient
-        ds = keep * (-E) * sigmoidf_(s);
-        dA = keep * (-E) * sp;
-    } else if (mode == MKDA_GATE_KIMI) {
-        const float u = E * s, sg = sigmoidf_(u), d = lb * sg * (1.f - sg);
-        ds = d * E;
-        dA = d * u;
-    } else if (mode == MKDA_GATE_EDA) {
-        const float sp = softplusf_(s), c = E / fabsf(lb), w = expf_(-c * sp), d = lb * w * c;
-        ds = d * sigmoidf_(s);
-        dA = d * sp;
-    } else {
-        ds = 1.f;
-        dA = 0.f;
-    }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -206,7 +179,8 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
         for (int w = 1; w < GB_WARPS; ++w) { sb = add4(sb, red[0][w][lane]); sa = add4(sa, red[1][w][lane]); }
         const size_t ch = (size_t)blockIdx.y * HV + h;
         if (p.part_bias) *reinterpret_cast<float4*>(p.part_bias + ch * 128 + 4 * lane) = sb;
-        if (p.part_alog) *reinterpret_cast<float4*>(p.part_alog + ch * 128 + 4 * lane) = sa;
+        const float t = warp_sum(hsum4(sa));
+        if (p.part_alog && lane == 0) p.part_alog[ch] = t;
     }
 }
 
@@ -266,51 +240,34 @@ __global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd 
 // ---------------------------------------------------------------------------------------------------------
 // deterministic second-stage reductions
 // ---------------------------------------------------------------------------------------------------------
-// group == 1: block (32, 8); thread (x, y) sums rows y, y+8, ... of column j (four running sums, so that four loads are
-// in flight), then the 8 partials are added in order.
-__global__ void __launch_bounds__(256) reduce_cols_kernel(const float* __restrict__ in, int rows, int cols, float* __restrict__ out) {
-    __shared__ float part[8][33];
-    const int j = blockIdx.x * 32 + threadIdx.x;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    if (j < cols) {
-        int r = threadIdx.y;
-        for (; r + 24 < rows; r += 32) {
-            s0 += in[(size_t)r * cols + j];
-            s1 += in[(size_t)(r + 8) * cols + j];
-            s2 += in[(size_t)(r + 16) * cols + j];
-            s3 += in[(size_t)(r + 24) * cols + j];
+// Up to three jobs in one launch (the parameter gradients of a layer): block = 32 outputs of a job x 32 row lanes.  A lane adds every 32nd
+// term of its output, eight loads in flight; the 32 lanes' sums are then combined by a fixed shuffle tree.  (One launch per job with 8 row
+// lanes, and one block per output for the grouped job, took 43 + 43 us on 64k tokens x 32 heads; this takes 22.)
+__global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
+    __shared__ float part[32][33];
+    int blk = blockIdx.x, job = 0;
+    while (job < 2 && blk >= (p.job[job].cols / p.job[job].group + 31) / 32) { blk -= (p.job[job].cols / p.job[job].group + 31) / 32; ++job; }
+    const MkdaReduce q = p.job[job];
+    const int j = blk * 32 + threadIdx.x, outs = q.cols / q.group, terms = q.rows * q.group;
+    float s = 0.f;
+    if (j < outs) {
+        const float* in = q.in + (size_t)j * q.group;
+        auto at = [&](int t) { return q.group == 1 ? in[(size_t)t * q.cols] : in[(size_t)(t / q.group) * q.cols + t % q.group]; };
+        float a[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) a[e] = 0.f;
+        int t = threadIdx.y;
+        for (; t + 7 * 32 < terms; t += 8 * 32) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] += at(t + e * 32);
         }
-        for (; r < rows; r += 8) s0 += in[(size_t)r * cols + j];
+        for (; t < terms; t += 32) a[0] += at(t);
+        s = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     }
-    part[threadIdx.y][threadIdx.x] = (s0 + s1) + (s2 + s3);
+    part[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
-    if (threadIdx.y == 0 && j < cols) {
-        float t = part[0][threadIdx.x];
-        for (int y = 1; y < 8; ++y) t += part[y][threadIdx.x];
-        out[j] = t;
-    }
-}
-// group > 1: one block of 128 threads per output; warp w walks rows w, w+4, ... and its lanes the group's elements, again
-// with four running sums; lanes, then warps, are combined in a fixed order.
-__global__ void __launch_bounds__(128) reduce_groups_kernel(const float* __restrict__ in, int rows, int cols, int group, float* __restrict__ out) {
-    __shared__ float part[4];
-    const int j = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    for (int i = lane; i < group; i += 32) {
-        const float* col = in + (size_t)j * group + i;
-        int r = warp;
-        for (; r + 12 < rows; r += 16) {
-            s0 += col[(size_t)r * cols];
-            s1 += col[(size_t)(r + 4) * cols];
-            s2 += col[(size_t)(r + 8) * cols];
-            s3 += col[(size_t)(r + 12) * cols];
-        }
-        for (; r < rows; r += 4) s0 += col[(size_t)r * cols];
-    }
-    const float s = warp_sum((s0 + s1) + (s2 + s3));
-    if (lane == 0) part[warp] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) out[j] = (part[0] + part[1]) + (part[2] + part[3]);
+    s = warp_sum(part[threadIdx.x][threadIdx.y]);          // warp y: the 32 partial sums of output y
+    if (threadIdx.x == 0 && blk * 32 + (int)threadIdx.y < outs) q.out[blk * 32 + threadIdx.y] = s;
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -320,12 +277,14 @@ template <int DT>
 __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
     const int lane = threadIdx.x & 31, sub = lane & 15;
     const int row0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + (lane >> 4);
+    const void* x = blockIdx.y ? p.x2 : p.x;
+    float* rstd = blockIdx.y ? p.rstd2 : p.rstd;
     float4 a[4], b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = row0 + 2 * i, rr = row < p.rows ? row : p.rows - 1;
-        a[i] = ld4(p.x, DT, (size_t)rr * 128 + 8 * sub);
-        b[i] = ld4(p.x, DT, (size_t)rr * 128 + 8 * sub + 4);
+        a[i] = ld4(x, DT, (size_t)rr * 128 + 8 * sub);
+        b[i] = ld4(x, DT, (size_t)rr * 128 + 8 * sub + 4);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -333,19 +292,21 @@ __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         const int row = row0 + 2 * i;
-        if (sub == 0 && row < p.rows) p.rstd[row] = 1.f / sqrtf(ss + p.eps);
+        if (sub == 0 && row < p.rows) rstd[row] = 1.f / sqrtf(ss + p.eps);
     }
 }
 
 // L2-norm backward of the q / k gradients.  Block (chunk, q/k head, which of q / k); warp w takes rows w, w + 4, ... of the
 // chunk.  The gradients arrive as the fp32 [64][128] tiles of the chunk backward, already summed over the v-heads of the
 // q/k head (the chunk backward adds them up where it writes them).
+template <bool SPLIT>
 __global__ void __launch_bounds__(128) qk_grad_finish_kernel(const MkdaQkGrad p) {
     const int HK = p.L.HK;
     const int c = blockIdx.x / HK, hk = blockIdx.x - c * HK, which = blockIdx.y;
     const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float* d_v = (which ? p.dk_v : p.dq_v) + ((size_t)c * HK + hk) * CH * 128 + 4 * lane;
+    const int G = SPLIT ? p.L.HV / HK : 1;                 // tiles to add, in the order of the v-heads
+    const float* d_v = (which ? p.dk_v : p.dq_v) + ((size_t)c * HK + hk) * G * CH * 128 + 4 * lane;
     const void* x = which ? p.k : p.q;
     const float* rstd = which ? p.k_rstd : p.q_rstd;
     void* dx = which ? p.dk : p.dq;
@@ -362,6 +323,14 @@ __global__ void __launch_bounds__(128) qk_grad_finish_kernel(const MkdaQkGrad p)
                 xr[u] = ld4(x, p.x_dtype, rowi * 128 + 4 * lane);
             }
         }
+        if (SPLIT)
+            for (int g = 1; g < G; ++g) {
+                float4 t[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) t[u] = *reinterpret_cast<const float4*>(d_v + (size_t)(g * CH + min(r0 + 4 * u, len - 1)) * 128);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] = add4(s[u], t[u]);
+            }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int r = r0 + 4 * u;
@@ -643,21 +612,33 @@ extern "C" int mkda_gate_bwd(const MkdaGateBwd* p, void* stream) {
     return check_launch("gate_bwd");
 }
 
+extern "C" int mkda_reduce_multi(const MkdaReduceMulti* p, void* stream) {
+    if (!p) return set_error(MKDA_ERR_ARG, "reduce_multi: null argument");
+    MkdaReduceMulti q = *p;
+    int blocks = 0;
+    for (MkdaReduce& j : q.job) {
+        if (!j.out || j.cols == 0) { j = MkdaReduce{nullptr, 0, 0, 1, nullptr}; continue; }
+        if (!j.in || j.group < 1 || j.cols % j.group) return set_error(MKDA_ERR_ARG, "reduce_multi: bad argument");
+        blocks += (j.cols / j.group + 31) / 32;
+    }
+    if (blocks == 0) return MKDA_OK;
+    reduce_kernel<<<blocks, dim3(32, 32), 0, (cudaStream_t)stream>>>(q);
+    return check_launch("reduce_multi");
+}
+
 extern "C" int mkda_reduce_partials(const MkdaReduce* p, void* stream) {
-    if (!p || !p->in || !p->out || p->group < 1 || p->cols % p->group) return set_error(MKDA_ERR_ARG, "reduce_partials: bad argument");
-    if (p->cols == 0) return MKDA_OK;
-    if (p->group == 1)
-        reduce_cols_kernel<<<(p->cols + 31) / 32, dim3(32, 8), 0, (cudaStream_t)stream>>>(p->in, p->rows, p->cols, p->out);
-    else
-        reduce_groups_kernel<<<p->cols / p->group, 128, 0, (cudaStream_t)stream>>>(p->in, p->rows, p->cols, p->group, p->out);
-    return check_launch("reduce_partials");
+    if (!p || !p->in || !p->out) return set_error(MKDA_ERR_ARG, "reduce_partials: bad argument");
+    MkdaReduceMulti q{};
+    q.job[0] = *p;
+    return mkda_reduce_multi(&q, stream);
 }
 
 extern "C" int mkda_l2norm_rstd(const MkdaL2Norm* p, void* stream) {
     if (!p || !p->x || !p->rstd) return set_error(MKDA_ERR_ARG, "l2norm_rstd: null argument");
-    if (any_misaligned(p->x)) return set_error(MKDA_ERR_ARG, "l2norm_rstd: x must be 16-byte aligned");
+    if (any_misaligned(p->x, p->x2)) return set_error(MKDA_ERR_ARG, "l2norm_rstd: x must be 16-byte aligned");
+    if (p->x2 && !p->rstd2) return set_error(MKDA_ERR_ARG, "l2norm_rstd: null argument");
     if (p->rows == 0) return MKDA_OK;
-    const int grid = (p->rows + 31) / 32;
+    const dim3 grid((p->rows + 31) / 32, p->x2 ? 2 : 1);
     switch (p->dtype) {
         case MKDA_F32: l2norm_rstd_kernel<MKDA_F32><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
         case MKDA_BF16: l2norm_rstd_kernel<MKDA_BF16><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
@@ -673,7 +654,8 @@ extern "C" int mkda_qk_grad_finish(const MkdaQkGrad* p, void* stream) {
     if (any_misaligned(p->dq_v, p->dk_v, p->dq, p->dk, p->q, p->k)) return set_error(MKDA_ERR_ARG, "qk_grad_finish: tensors must be 16-byte aligned");
     if (p->L.NC == 0) return MKDA_OK;
     const dim3 grid(p->L.NC * p->L.HK, 2);
-    qk_grad_finish_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
+    if (p->per_v_head) qk_grad_finish_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
+    else qk_grad_finish_kernel<false><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
     return check_launch("qk_grad_finish");
 }
 
@@ -729,8 +711,8 @@ extern "C" int mkda_epilogue_bwd_noalloc(const MkdaEpilogueBwdNoAlloc* p, void* 
     q.part_w = scratch;                 // every block overwrites its whole row: nothing has to be cleared first
     epilogue_bwd_kernel<<<nblk, 128, 0, (cudaStream_t)stream>>>(q);
     if (int e = check_launch("epilogue_bwd_noalloc")) return e;
-    reduce_cols_kernel<<<4, dim3(32, 8), 0, (cudaStream_t)stream>>>(scratch, nblk, 128, p->dweight);
-    return check_launch("epilogue_bwd_noalloc (reduce)");
+    const MkdaReduce r{scratch, nblk, 128, 1, p->dweight};
+    return mkda_reduce_partials(&r, stream);
 }
 
 extern "C" int mkda_epilogue_bwd_tiles(const MkdaEpilogueBwdTiles* p, void* stream) {

@@ -96,28 +96,30 @@ __device__ __forceinline__ void red_add(float* addr, float v) {
 // memory), and inside a group the G = HV / HK v-heads that share the q/k head one after the other.  Their dq and dk contributions are
 // summed where they are written: the first v-head of a group stores its fp32 tile, the others add to it (red.global.add.f32 by the same
 // thread to the same address, in the fixed order of the v-heads: deterministic).  The tile lives in L2 between the two passes.
+// SPREAD (few items): a group is one v-head with tiles of its own, so that no CTA works through G of them alone.
+template <bool SPREAD>
 struct ItemWalk {
-    int grp, j, G, HK, HV, ngroups, stride;
+    int grp, j, G, H, HV, ngroups, stride;                 // H groups per chunk; G v-heads per q/k head
     __device__ __forceinline__ ItemWalk(const MkdaLayout& L) {
-        HK = L.HK; HV = L.HV; G = HV / HK; ngroups = L.NC * HK; stride = gridDim.x; grp = blockIdx.x; j = 0;
+        HV = L.HV; G = HV / L.HK; H = SPREAD ? HV : L.HK; ngroups = L.NC * H; stride = gridDim.x; grp = blockIdx.x; j = 0;
     }
     __device__ __forceinline__ bool valid() const { return grp < ngroups; }
-    __device__ __forceinline__ int chunk() const { return grp / HK; }
-    __device__ __forceinline__ int hk() const { return grp % HK; }
-    __device__ __forceinline__ int head() const { return (grp % HK) * G + j; }
+    __device__ __forceinline__ int chunk() const { return grp / H; }
+    __device__ __forceinline__ int head() const { return SPREAD ? grp % H : (grp % H) * G + j; }
+    __device__ __forceinline__ int hk() const { return SPREAD ? grp % H / G : grp % H; }
     __device__ __forceinline__ size_t item() const { return (size_t)chunk() * HV + head(); }
-    __device__ __forceinline__ void next() { if (++j == G) { j = 0; grp += stride; } }
+    __device__ __forceinline__ void next() { if (SPREAD || ++j == G) { j = 0; grp += stride; } }
 };
 
 // SCALAR (one decay per token): the intra-chunk part contracts the plain k / q rows with weights that already carry
 // E_ij = 2^(g_i - g_j) (i > j, never a positive exponent):  [dq_row | T]^T = K^T [Wq E; dLs E]^T (N = 128),
 // dk_col^T = Q^T (Wq E) + K^T (beta dLs E); no anchors, and any g <= 0 is in range.  TMEM: [dq_row | T] 0, dk_col 128.
-template <bool SCALAR>
+template <bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     const uint32_t tmem = sh.tmem;
     uint32_t n = 0;
-    for (ItemWalk w(p.L); w.valid(); w.next(), ++n) {
+    for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
         const uint32_t par = n & 1;
         if (n) wait_mma(&sh.accFree, par ^ 1);
         umma::mbar_wait(&sh.fullW, par);
@@ -162,12 +164,12 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
 
 // S, dO, Vd, dVd and A of the next item are requested as soon as the intra-chunk products of the current one are done (the epilogue reads
 // accumulators, the scratch and the raw rows only), dS' once dVd and A have been read and the scratch is free.
-template <bool SCALAR>
+template <bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     auto src = [](const void* t, size_t it, uint32_t bytes, uint32_t off = 0) { return static_cast<const uint8_t*>(t) + it * bytes + off; };
     uint32_t n = 0;
-    for (ItemWalk w(p.L); w.valid(); w.next(), ++n) {
+    for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
         const size_t it = w.item();
         if (n) umma::mbar_wait(&sh.mmI, (n & 1) ^ 1);
         umma::mbar_expect_tx(&sh.fullW, umma::CHUNK_TILE_BYTES + umma::QUARTER_TILE_BYTES);
@@ -185,7 +187,7 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
         // Between here and the epilogue nothing else is fetched.  Scalar gate: the next item's tiles start on their way from HBM into L2 (1465 ->
         // 1388 us on 4 x 16k tokens x 16 heads; its items are short and the copies were late).  With the per-channel gate the same hint
         // costs 2 % (3.92 -> 4.02 ms on 64k packed tokens x 32 heads).
-        ItemWalk nx = w;
+        ItemWalk<SPREAD> nx = w;
         nx.next();
         if (SCALAR && nx.valid()) {
             const size_t in = nx.item();
@@ -201,7 +203,7 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
 }
 
 // Compute warps.  Thread (q, lane, cg): accumulator lane `row` = 32 q + lane, columns or rows [16 cg, 16 cg + 16).
-template <int DT, bool SCALAR>
+template <int DT, bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -214,10 +216,10 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
 
     // chunk table entries and the per-row scalars (beta | L2 statistics | scalar gate) travel one item ahead: every address of an item
     // depends on the former, and a scalar stored where it is requested would be waited for there
-    ItemWalk w(p.L);
+    ItemWalk<SPREAD> w(p.L);
     int next_start = 0, next_len = 1;
     float ahead0 = 0.f, ahead1 = 0.f;
-    auto row_scalars = [&](const ItemWalk& it) {
+    auto row_scalars = [&](const ItemWalk<SPREAD>& it) {
         const int h = it.head(), hk = it.hk(), r = tid & (CH - 1), rr = r < next_len ? r : next_len - 1;
         const size_t tk = (size_t)(next_start + rr) * HK + hk, tv = (size_t)(next_start + rr) * HV + h;
         if (tid < CH) {
@@ -235,10 +237,10 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     }
     for (uint32_t n = 0; w.valid(); ++n) {
         const uint32_t par = n & 1;
-        const int c = w.chunk(), hk = w.hk(), h = w.head(), start = next_start, len = next_len;
+        const int hk = w.hk(), h = w.head(), start = next_start, len = next_len;
         const size_t item = w.item();
         const bool first_of_group = w.j == 0;
-        ItemWalk nxt = w;
+        ItemWalk<SPREAD> nxt = w;
         nxt.next();
         if (nxt.valid() && nxt.grp != w.grp) { next_start = p.L.chunk_start[nxt.chunk()]; next_len = p.L.chunk_len[nxt.chunk()]; }
 
@@ -468,7 +470,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         } else {
             egL = ex2f_(sh.gs[CH - 1]);
         }
-        const size_t obk = ((size_t)c * HK + hk) * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
+        const size_t obk = (size_t)w.grp * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
         float* __restrict__ oq = p.dq_v + obk;
         float* __restrict__ ok = p.dk_v + obk;
         float* __restrict__ og = SCALAR ? p.dgp + item * CH : p.dgp + item * (size_t)(CH * DK) + row;
@@ -592,7 +594,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     }
 }
 
-template <int DT, bool SCALAR>
+template <int DT, bool SCALAR, bool SPREAD>
 __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p) {
     using namespace bc;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -613,39 +615,43 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
     if (warp >= COMPUTE / 32) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == WARP_MMA) {
-            if (elect_one()) bwd_chunk_issue<SCALAR>(p, base, sh);
+            if (elect_one()) bwd_chunk_issue<SCALAR, SPREAD>(p, base, sh);
             __syncwarp();
         } else if (warp == WARP_LOAD) {
-            if (elect_one()) bwd_chunk_load<SCALAR>(p, base, sh);
+            if (elect_one()) bwd_chunk_load<SCALAR, SPREAD>(p, base, sh);
             __syncwarp();
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        bwd_chunk_compute<DT, SCALAR>(p, base, sh);
+        bwd_chunk_compute<DT, SCALAR, SPREAD>(p, base, sh);
     }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(sh.tmem, 512);
 }
 
-template <int DT, bool SCALAR>
+template <int DT, bool SCALAR, bool SPREAD>
 static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, cudaStream_t stream) {
-    auto kern = bwd_chunk_tc_kernel<DT, SCALAR>;
+    auto kern = bwd_chunk_tc_kernel<DT, SCALAR, SPREAD>;
     if (int e = ensure_smem((const void*)kern, bc::SMEM, "bwd_chunk")) return e;
     static const int regs = kernel_registers((const void*)kern);
     if (regs < bc::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "bwd_chunk: built with fewer registers than its warps redistribute");
-    const int groups = p->L.NC * p->L.HK;                  // a CTA takes whole (chunk, q/k head) groups
+    const int groups = p->L.NC * (SPREAD ? p->L.HV : p->L.HK);              // a CTA takes whole (chunk, q/k head) groups
     kern<<<groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream>>>(*p);
     return check_launch("bwd_chunk");
 }
+template <int DT, bool SCALAR>
+static int launch_bwd_chunk_tc_s(const MkdaBwdChunk* p, cudaStream_t stream) {
+    return p->per_v_head ? launch_bwd_chunk_tc_t<DT, SCALAR, true>(p, stream) : launch_bwd_chunk_tc_t<DT, SCALAR, false>(p, stream);
+}
 int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream) {
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {
-        case MKDA_F32 * 2: return launch_bwd_chunk_tc_t<MKDA_F32, false>(p, stream);
-        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_t<MKDA_BF16, false>(p, stream);
-        case MKDA_F16 * 2: return launch_bwd_chunk_tc_t<MKDA_F16, false>(p, stream);
-        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_F32, true>(p, stream);
-        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_BF16, true>(p, stream);
-        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_t<MKDA_F16, true>(p, stream);
+        case MKDA_F32 * 2: return launch_bwd_chunk_tc_s<MKDA_F32, false>(p, stream);
+        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_s<MKDA_BF16, false>(p, stream);
+        case MKDA_F16 * 2: return launch_bwd_chunk_tc_s<MKDA_F16, false>(p, stream);
+        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F32, true>(p, stream);
+        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_BF16, true>(p, stream);
+        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F16, true>(p, stream);
     }
     return set_error(MKDA_ERR_ARG, "bwd_chunk: unsupported dtype");
 }

@@ -123,11 +123,11 @@ def gate_bwd(lay, x, dgp, mode, A_log, dt_bias, lower_bound, HV, want_bias, want
             part_b = torch.empty(rows, width, dtype=torch.float32, device=x.device)
             p.part_bias = _ptr(part_b)
         if want_alog:
-            part_a = torch.empty(rows, width, dtype=torch.float32, device=x.device)
+            part_a = torch.empty(rows, HV, dtype=torch.float32, device=x.device)
             p.part_alog = _ptr(part_a)
     _lib.call("mkda_gate_bwd", p, _stream())
     d_bias = reduce_partials(part_b, rows, width) if part_b is not None else None
-    d_alog = reduce_partials(part_a, rows, width, 1 if scalar else 128) if part_a is not None else None
+    d_alog = reduce_partials(part_a, rows, HV) if part_a is not None else None
     return dx, d_bias, d_alog
 
 

@@ -57,3 +57,48 @@ def test_states_at_odd_storage_offsets(offset):
 
     for a, b in zip(call(h0.clone(), dht), call(h0, up[offset:].view(dht.shape))):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("case", [
+    dict(B=3, T=1, gate="kimi", dtype=torch.bfloat16, epi="silu"),
+    dict(B=2, T=16, gate="eda", dtype=torch.float32, epi="sigmoid", vfirst=True),
+    dict(B=2, T=17, gate="eda", dtype=torch.float32, epi=None),
+    dict(cu=(0, 1, 1, 6, 22, 22), T=25, gate="gdn", dtype=torch.float16, epi="silu", vfirst=True),
+    dict(B=5, T=2, gate="gdn", scalar=True, dtype=torch.bfloat16, epi=None, vfirst=True),
+    dict(B=1, T=9, gate="precomputed", beta="precomputed", l2=False, dtype=torch.float32, epi=None, h0=False),
+    dict(B=2, T=4, gate="eda", dtype=torch.bfloat16, epi="silu", x_dtype=torch.bfloat16)], ids=str)
+def test_forward_of_very_short_sequences(case):
+    """Without gradients, sequences of up to 16 tokens run token by token (17: the chunk kernels); empty sequences, padding and 4 v-heads on
+    2 q/k heads included."""
+    case = dict(case)
+    vfirst = case.pop("vfirst", False)
+    lv, do, dht, opts, epi = make_inputs(HK=2, HV=4, seed=47, **case)
+    got = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=vfirst, grads=False)
+    end = case["cu"][-1] if "cu" in case else case["T"]
+    cut = {n: (t[:, :end].contiguous() if t.dim() >= 3 and n != "h0" else t) for n, t in lv.items()}
+    ref = run(orc.recurrent_delta_rule, cut, do[:, :end], dht, opts, epi, f64=True, vfirst=vfirst, grads=False)
+    assert (got["o"][:, end:] == 0).all()
+    got["o"] = got["o"][:, :end]
+    compare(got, ref)
+
+
+@pytest.mark.parametrize("NC,G", [(1, 2), (3, 4), (149, 2), (300, 2)])
+def test_few_groups_are_spread_over_v_heads(NC, G):
+    """With few (chunk, q/k head) groups the backward pass gives every v-head tiles of its own, which the finishing kernel adds: the same
+    sums in the same order, so expanding one head's work over more chunks must not change a bit of an earlier chunk."""
+    lv, do, dht, opts, epi = make_inputs(B=NC, T=64, HK=1, HV=G, dtype=torch.float32, gate="eda", seed=53, h0=False, epi=None)
+    full = run(mk.chunk_delta_rule, lv, do, dht, opts, epi)
+    sub = {n: (t[:1].contiguous() if t.dim() >= 3 else t) for n, t in lv.items()}
+    one = run(mk.chunk_delta_rule, sub, do[:1], dht[:1], opts, epi)
+    for n in ("dq", "dk", "dv", "dg", "dbeta"):
+        assert torch.equal(full[n][:1], one[n]), n
+    compare(one, run(orc.chunked_delta_rule, sub, do[:1], dht[:1], opts, epi, f64=True))
+
+
+@pytest.mark.parametrize("rows,cols,group", [(1, 1, 1), (33, 7, 1), (255, 64, 1), (257, 33, 1), (1184, 128, 1), (5, 256, 128), (64, 384, 3)])
+def test_partial_reductions(rows, cols, group):
+    from mogankda_b200 import ops
+    x = torch.randn(rows, cols, device="cuda")
+    got = ops.reduce_partials(x, rows, cols, group)
+    ref = x.double().view(rows, cols // group, group).sum((0, 2))
+    assert got.shape == ref.shape and ((got - ref).abs() <= 1e-6 * x.double().abs().view(rows, cols // group, group).sum((0, 2))).all()
