@@ -131,6 +131,7 @@ KERNEL_FLOPS = {                      # per token per v-head
     "mkda_intra_fwd": 3 * F_CK,                       # Gamma, Q K^T, A (beta [k~ | v]) counted as one C x C x (K|V) product pair
     "mkda_recur_fwd": 2 * F_KV,                       # nw S, kbar^T Vd
     "mkda_out_fwd": F_KV + F_CK,                      # q~ S, Aqk Vd
+    "mkda_chain_fwd": 3 * F_KV + F_CK,                # both in one kernel
     "mkda_bwd_dh": F_CK + 3 * F_KV,                   # Aqk^T dO, kbar dS', q~^T dO, nw^T dVd
     # k~ S, dO Vd^T, A^T dVd, dVd W^T, two C^3 products (Vd comes from the forward pass); dO S^T, dX S^T, Vd dS'^T; row / column
     # terms through Gamma and Q K^T
@@ -140,7 +141,7 @@ KERNEL_FLOPS = {                      # per token per v-head
 # fp32 intermediates, HV = 2 HK), every operand counted once.
 KERNEL_BYTES = {
     "mkda_gate_cumsum_fwd": 1024, "mkda_l2norm_rstd": 128, "mkda_intra_fwd": 3592, "mkda_recur_fwd": 3080,
-    "mkda_out_fwd": 3584, "mkda_epilogue_bwd_tiles": 2048, "mkda_epilogue_bwd": 2048, "mkda_bwd_dh": 3848,
+    "mkda_out_fwd": 3584, "mkda_chain_fwd": 5128, "mkda_epilogue_bwd_tiles": 2048, "mkda_epilogue_bwd": 2048, "mkda_bwd_dh": 3848,
     "mkda_bwd_chunk": 6152, "mkda_gate_bwd": 1536, "mkda_qk_grad_finish": 1024,      # dq / dk tiles are per q/k head: 512 B per v-head
 }
 def load_kernel_traffic(path=os.path.join(ROOT, "profiles", "counters_per_kernel_1b_shape.md")):
@@ -173,7 +174,7 @@ KERNEL_TRAFFIC = load_kernel_traffic()
 
 # device kernel name -> entry point of the library that launches it
 KERNEL_ENTRY = (("gate_cumsum_fwd", "mkda_gate_cumsum_fwd"), ("gate_bwd", "mkda_gate_bwd"), ("reduce_", "mkda_reduce_partials"),
-                ("l2norm_rstd", "mkda_l2norm_rstd"), ("intra_fwd", "mkda_intra_fwd"), ("recur_fwd", "mkda_recur_fwd"),
+                ("l2norm_rstd", "mkda_l2norm_rstd"), ("intra_fwd", "mkda_intra_fwd"), ("recur_fwd", "mkda_recur_fwd"), ("chain_fwd", "mkda_chain_fwd"),
                 ("out_fwd", "mkda_out_fwd"), ("epilogue_bwd_tiles", "mkda_epilogue_bwd_tiles"), ("epilogue_bwd", "mkda_epilogue_bwd"),
                 ("bwd_dh", "mkda_bwd_dh"), ("bwd_chunk", "mkda_bwd_chunk"), ("qk_grad_finish", "mkda_qk_grad_finish"),
                 ("step_fwd", "mkda_step_fwd"), ("combine", "mkda_state_combine"), ("warmup_chunks", "mkda_warmup_chunks"))

@@ -186,6 +186,14 @@ typedef struct {
 } MkdaOutFwd;
 int mkda_out_fwd(const MkdaOutFwd* p, void* stream);
 
+/* mkda_recur_fwd and mkda_out_fwd in one kernel: the output of a chunk is computed in the step that has its state and Vd at hand.  r.h and r.Vd
+ * may be NULL (no backward pass follows: they are then never written); o.h and o.Vd are not used; no transition. */
+typedef struct {
+    MkdaRecurFwd r;
+    MkdaOutFwd o;
+} MkdaChainFwd;
+int mkda_chain_fwd(const MkdaChainFwd* p, void* stream);
+
 /* Forward pass over sequences of at most MKDA_STEP_MAX_TOKENS tokens (generation steps): gate, L2 norm, recurrence, output and epilogue in one
  * kernel, token by token, with the state in registers.  Same results as the chunk kernels up to rounding; nothing is kept for a backward
  * pass. */

@@ -31,6 +31,18 @@ extern "C" int mkda_out_fwd(const MkdaOutFwd* p, void* stream) {
     return launch_out_fwd_tc(p, (cudaStream_t)stream);
 }
 
+extern "C" int mkda_chain_fwd(const MkdaChainFwd* p, void* stream) {
+    if (!p || !p->r.nw || !p->r.u || !p->r.kbar || !p->r.gl || !p->o.qs || !p->o.Aqk || !p->o.out) return set_error(MKDA_ERR_ARG, "chain_fwd: null argument");
+    if (any_misaligned(p->r.nw, p->r.u, p->r.kbar, p->r.gl, p->o.qs, p->o.Aqk, p->o.out, p->o.o_raw, p->o.gate, p->o.norm_w))
+        return set_error(MKDA_ERR_ARG, "chain_fwd: tensors must be 16-byte aligned");
+    if (any_misaligned32(p->r.h, p->r.Vd) || (p->r.state_v_first && any_misaligned32(p->r.h0, p->r.ht)))
+        return set_error(MKDA_ERR_ARG, "chain_fwd: saved tiles and [V,K] states must be 32-byte aligned");
+    if (p->r.want_transition || p->r.warm_start) return set_error(MKDA_ERR_ARG, "chain_fwd: no transition and no truncation in a main pass");
+    if (p->o.has_norm && (!p->o.gate || p->o.out_dtype != MKDA_F32)) return set_error(MKDA_ERR_ARG, "chain_fwd: the gated norm needs a gate tensor and fp32 output");
+    if (p->r.L.NS == 0) return MKDA_OK;
+    return launch_chain_fwd_tc(p, (cudaStream_t)stream);
+}
+
 extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) {
     if (!p || !(p->dO_in_t || (p->d_o && p->dO_t)) || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw)
         return set_error(MKDA_ERR_ARG, "bwd_dh: null argument");

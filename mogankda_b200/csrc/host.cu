@@ -41,7 +41,8 @@ int sm_count() {
     return cached[dev];
 }
 
-int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what) {
+int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what,
+                  int box_rows) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static Encode encode = nullptr;                    // resolved through the runtime: the library does not link against the driver
@@ -62,7 +63,7 @@ int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned l
     }
     const cuuint64_t gdim[2] = {row_elems, rows};
     const cuuint64_t gstride[1] = {pitch};
-    const cuuint32_t box[2] = {128, 64}, estr[2] = {1, 1};
+    const cuuint32_t box[2] = {128, (cuuint32_t)box_rows}, estr[2] = {1, 1};
     const CUresult r = encode(out, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), gdim,
                               gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -130,7 +131,7 @@ extern "C" int mkda_abi_version(void) { return 4; }
 extern "C" int mkda_struct_sizes(int* out, int n) {
     const int sizes[] = {
         (int)sizeof(MkdaLayout),   (int)sizeof(MkdaGateFwd),  (int)sizeof(MkdaGateBwd),     (int)sizeof(MkdaReduce), (int)sizeof(MkdaReduceMulti),
-        (int)sizeof(MkdaL2Norm),   (int)sizeof(MkdaIntraFwd), (int)sizeof(MkdaRecurFwd),    (int)sizeof(MkdaOutFwd), (int)sizeof(MkdaStepFwd),
+        (int)sizeof(MkdaL2Norm),   (int)sizeof(MkdaIntraFwd), (int)sizeof(MkdaRecurFwd),    (int)sizeof(MkdaOutFwd), (int)sizeof(MkdaChainFwd), (int)sizeof(MkdaStepFwd),
         (int)sizeof(MkdaEpilogueBwd), (int)sizeof(MkdaEpilogueBwdTiles), (int)sizeof(MkdaEpilogueBwdNoAlloc), (int)sizeof(MkdaBwdDh), (int)sizeof(MkdaBwdChunk),
         (int)sizeof(MkdaQkGrad),   (int)sizeof(MkdaCombine), (int)sizeof(MkdaWarmup), (int)sizeof(MkdaSelfTest), (int)sizeof(MkdaSelfTestWait)};
     const int cnt = (int)(sizeof(sizes) / sizeof(sizes[0]));

@@ -14,11 +14,12 @@ int check_launch(const char* what);
 int ensure_smem(const void* func, int bytes, const char* what);
 // Registers per thread the kernel is launched with (0 if unknown): a kernel whose warps redistribute registers checks its build with it.
 int kernel_registers(const void* func);
-// Tensor map over a row-major [rows][row_elems] tensor of 2- or 4-byte elements whose boxes are 64 rows x 128 elements, not
-// swizzled: one tiled TMA copy then brings 64 strided 128-element rows (token rows of one head) into shared memory as a dense
+// Tensor map over a row-major [rows][row_elems] tensor of 2- or 4-byte elements whose boxes are `box_rows` (64) rows x 128 elements,
+// not swizzled: one tiled TMA copy then brings 64 strided 128-element rows (token rows of one head) into shared memory as a dense
 // [64][128] block.  Rows past the end of the tensor read as zeros.  Returns 0, or an error code when the tensor cannot be
 // described (base not 16-byte aligned, row pitch not a multiple of 16 bytes, or the driver lacks the encoder).
-int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what);
+int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what,
+                  int box_rows = 64);
 // True if any of the (possibly null) pointers is not 16-byte aligned: the kernels read and write their tensors with
 // 16-byte vector accesses and bulk copies, and a misaligned address would fault the device instead of returning an error.
 template <typename... P>
@@ -37,6 +38,7 @@ int tc_chunk_status(unsigned int* out);
 int tc_chunk_status_clear();
 int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void* tiles, cudaStream_t stream);
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream);
+int launch_chain_fwd_tc(const MkdaChainFwd* p, cudaStream_t stream);
 int launch_bwd_dh_tc(const MkdaBwdDh* p, cudaStream_t stream);
 int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();

@@ -107,8 +107,10 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     keep.want(&s.kbar, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.qs, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.gl, c.tiles(512));
-    keep.want(&s.h, c.tiles(MKDA_STATE_TILE_BYTES));
-    keep.want(&s.Vd, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    if (need_bwd) {
+        keep.want(&s.h, c.tiles(MKDA_STATE_TILE_BYTES));
+        keep.want(&s.Vd, c.tiles(MKDA_CHUNK_TILE_BYTES));
+    }
     if (c.has_ep && need_bwd) keep.want(&s.o_raw, row);
     tmp.want(&u, c.tiles(MKDA_CHUNK_TILE_BYTES));
     if (c.segmented) {
@@ -147,7 +149,10 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     }
     Tensor ht;
     if (c.want_ht) ht = c.states(c.N);
-    MkdaRecurFwd r{};
+    Tensor out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type());
+    const Tensor w = aligned(in.ep_w);
+    MkdaChainFwd p{};
+    MkdaRecurFwd& r = p.r;
     r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf;
     if (c.segmented) {
         // pre-pass from zero: per-segment (state, transition); the prefix combine then gives the state entering every segment
@@ -168,20 +173,14 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         r.h0 = fptr(in.h0);
     }
     r.h = s.h; r.Vd = s.Vd; r.ht = fptr(ht);
-    check_rc(mkda_recur_fwd(&r, st), "mkda_recur_fwd");
-
-    Tensor out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type());
-    {
-        MkdaOutFwd p{};
-        p.L = L; p.qs = s.qs; p.Aqk = s.Aqk; p.Vd = s.Vd; p.h = s.h; p.has_norm = c.has_ep;
-        const Tensor w = aligned(in.ep_w);
-        if (c.has_ep) {
-            if (w.defined()) { p.norm_w = w.data_ptr(); p.norm_w_dtype = dtype_code(w); }
-            p.gate = in.ep_gate.data_ptr(); p.gate_dtype = dtype_code(in.ep_gate); p.act = c.act; p.eps = c.eps;
-        }
-        p.o_raw = s.o_raw; p.out = out.data_ptr(); p.out_dtype = dtype_code(out);
-        check_rc(mkda_out_fwd(&p, st), "mkda_out_fwd");
+    MkdaOutFwd& o = p.o;
+    o.L = L; o.qs = s.qs; o.Aqk = s.Aqk; o.has_norm = c.has_ep;
+    if (c.has_ep) {
+        if (w.defined()) { o.norm_w = w.data_ptr(); o.norm_w_dtype = dtype_code(w); }
+        o.gate = in.ep_gate.data_ptr(); o.gate_dtype = dtype_code(in.ep_gate); o.act = c.act; o.eps = c.eps;
     }
+    o.o_raw = s.o_raw; o.out = out.data_ptr(); o.out_dtype = dtype_code(out);
+    check_rc(mkda_chain_fwd(&p, st), "mkda_chain_fwd");
     return {out, ht};
 }
 

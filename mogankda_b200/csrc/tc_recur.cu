@@ -13,17 +13,18 @@
 // mbarriers, so that nothing but the chain itself is waited for; everything else of a step (saved tiles, which leave as 32-byte pieces
 // straight from registers; the next chunk's u^T; the products that do not depend on the state) is done while products run.
 // 512 threads used to build both operands in shared memory behind CTA-wide barriers: 7.2 - 9.7 k cycles per step.
-#include "common.cuh"
 #include "host.h"
-#include "umma.cuh"
+#include "intra.cuh"
+
+#include <string.h>
 
 namespace mkda {
 
 namespace rc {
-constexpr int COMPUTE = 512, THREADS = 576, WARP_MMA = 16, WARP_LOAD = 17;
+constexpr int COMPUTE = 512, THREADS = 576, WARP_MMA = 16, WARP_LOAD = 17, WARP_STORE = 18, WARP_GATE = 19;
 constexpr int KB = 1024;
 constexpr int SH = 128, SL = 192, VH = 448, VL = 480;      // tensor-memory columns of the left operands (hi, lo)
-constexpr int X = 0, D0 = 256, D1 = 320;                   // fp32 accumulators: state increment, D (two for the forward kernel)
+constexpr int X = 0, D0 = 256, D1 = 320, O = 384;          // fp32 accumulators: state increment, D (two for the forward kernel), output
 
 using umma::signal_tmem;
 using umma::wait_mma;
@@ -103,6 +104,12 @@ __device__ __forceinline__ void save_state_tile(uint8_t* tile, int row, int cg, 
         store_pair(tile + 32768, 128, row, 4 * cg + 2 * i, l + 8 * i);
     }
 }
+// one half (hi or lo) of this thread's part of the state tile in shared memory
+__device__ __forceinline__ void stage_state(uint8_t* tile, int row, int cg, const uint32_t (&w)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(tile + umma::tile_chunk_offset(128, row, 4 * cg + i)) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+}
 // Vd^T (dVd^T) from its accumulator: left operand, and optionally the saved chunk tile
 __device__ __forceinline__ void v_operand(uint32_t tmem, int d_col, int warp, int cg, uint32_t (&h)[8], uint32_t (&l)[8]) {
     float d[16];
@@ -116,30 +123,146 @@ __device__ __forceinline__ void v_operand(uint32_t tmem, int d_col, int warp, in
 }  // namespace rc
 
 // ---------------------------------------------------------------------------------------------------------
-// forward
+// forward.  OUT >= 0: the output O^T = S^T qs^T + Vd^T Aqk^T (qs = scale q 2^g) and its epilogue are computed in the same step.  Both left
+// operands are in tensor memory anyway, the products fill the gaps in which the tensor pipe waits for the chain, and four more warps turn
+// the accumulator into output rows: states and Vd need not travel through HBM to a kernel of their own (and are not written at all when
+// no backward pass follows): 416 -> 320 KB per chunk and head with a backward pass, 400 -> 192 KB without.  OUT = type of the norm's gate,
+// or of the output rows when there is no norm.
+// The epilogue passes 16 rows at a time through shared memory ([row][value], conflict-free both ways): thread v reads its 16 values of the
+// accumulator, then a warp takes four whole rows.  Gate rows come and output rows leave by tiled copies, and the state leaves through a
+// 32 KB stage (hi half, then lo half): with plain loads and stores the load / store queue was what everything waited for (25 k cycles per
+// chunk with thread-per-value accesses, 12 - 22 k with 512-byte rows).
 // ---------------------------------------------------------------------------------------------------------
 struct RecurShared {
-    uint64_t full[2];                                      // nw^T, kbar, u^T tiles and decay factors of a step landed
-    uint64_t opS, opV, mm1, mm2;                           // state operand | Vd operand written; first | second product done
+    uint64_t fullN[2], fullK[2], fullU[2], fullQ, fullA;   // landed: nw^T and decay factors | kbar | u^T | scale q 2^g | Aqk
+    uint64_t opS, opV, uFree, mm1, mm2, mmO, oFree;        // state operand | Vd operand written, u^T used; products done; O accumulator read
+    uint64_t fullG, gFree, ready[2], freed[2];             // gate rows landed | used; state halves staged | read by their copy
     uint32_t tmem;
     __align__(16) float gl[4][DK];                         // four deep: a step's factors are used at the start of the next one
+    __align__(16) float w[DV];                             // weight of the norm
 };
-constexpr int RECUR_BUF = 96 * rc::KB;                     // nw 32, kbar 32, u 32
-constexpr int RECUR_SMEM = 2 * RECUR_BUF + (int)sizeof(RecurShared) + 1024;
+template <bool OUT>
+struct RecurLayout {                                       // the plain recurrence double-buffers every tile
+    static constexpr int D = OUT ? 1 : 2, T = 32 * rc::KB;
+    static constexpr int N = 0, K = N + D * T, U = K + D * T, Q = U + D * T, A = Q + T, S = A + T / 2, G = S + T, STAGE = G + T / 2,
+                         TILES = OUT ? STAGE + 32 * rc::KB : Q, SMEM = TILES + (int)sizeof(RecurShared),
+                         THREADS = OUT ? 768 : 576, REGS = OUT ? 80 : 96;
+    static_assert(SMEM <= 232448, "shared memory of one CTA");
+};
+struct ChainMaps { CUtensorMap gate, raw, out; };          // rows of a head: boxes of 64 (gate) and 16 rows
 
-__global__ void __launch_bounds__(rc::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p) {
+// four consecutive 16-bit values, raw
+template <int DT>
+__device__ __forceinline__ void unpack4(const uint2& r, float (&v)[4]) {
+    v[0] = unpack1<DT>(r.x & 0xffffu); v[1] = unpack1<DT>(r.x >> 16); v[2] = unpack1<DT>(r.y & 0xffffu); v[3] = unpack1<DT>(r.y >> 16);
+}
+
+template <int DT, bool NORM>
+__device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainMaps& maps, RecurShared& sh, uint8_t* base, int h, int c_beg, int n) {
     using namespace rc;
+    using L = RecurLayout<true>;
+    const int HV = o.L.HV, tid = threadIdx.x & 127, w = tid >> 5, lane = tid & 31;
+    const int r = tid >> 3, c = tid & 7;                   // row of a group, 16-byte piece: this thread's values are 4 (c + 8 i) + 0..3
+    const uint32_t acc = umma::tmem_addr(sh.tmem, w, O);
+    const bool silu = o.act == MKDA_ACT_SILU, raw = o.o_raw != nullptr;
+    constexpr int ODT = NORM ? MKDA_F32 : DT;
+    if (NORM) sh.w[tid] = o.norm_w ? ld1(o.norm_w, o.norm_w_dtype, tid) : 1.f;
+    uint32_t buf = 0;
+    for (int k = 0; k < n; ++k) {
+        const int start = o.L.chunk_start[c_beg + k], len = o.L.chunk_len[c_beg + k];
+        if (NORM && DT != MKDA_F32) umma::mbar_wait(&sh.fullG, k & 1);
+        wait_mma(&sh.mmO, k & 1);
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+            if (16 * g >= len) break;
+            float* st = reinterpret_cast<float*>(base + L::STAGE + (buf & 1) * 8192);
+            uint8_t* so = base + L::STAGE + 16384 + (buf & 1) * 8192;
+            {
+                float x[16];
+                umma::tmem_ld16(acc + 16 * g, x);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) st[j * 128 + tid] = x[j];
+            }
+            if (16 * g + 16 >= len) signal_tmem(&sh.oFree, lane);
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            const int row = 16 * g + r;
+            const bool whole = 16 * g + 16 <= len, valid = row < len;
+            const size_t at = ((size_t)(start + (valid ? row : len - 1)) * HV + h) * 128 + 4 * c;
+            float4 x[4];
+            float f = 1.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(st + r * 128 + 4 * (c + 8 * i));
+            if (!whole && raw && valid) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(o.o_raw + at + 32 * i) = x[i];
+            }
+            if (NORM) {
+                float ss = 0.f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ss += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
+#pragma unroll
+                for (int sft = 4; sft > 0; sft >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sft);
+                f = rsqrtf(ss * (1.f / 128.f) + o.eps);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (NORM) {
+                    float z[4];
+                    if (DT == MKDA_F32) {
+                        const float4 z4 = ld4(o.gate, DT, at + 32 * i);
+                        z[0] = z4.x; z[1] = z4.y; z[2] = z4.z; z[3] = z4.w;
+                    } else {
+                        unpack4<DT == MKDA_F32 ? MKDA_BF16 : DT>(*reinterpret_cast<const uint2*>(base + L::G + row * 256 + 8 * (c + 8 * i)), z);
+                    }
+                    const float4 wn = *reinterpret_cast<const float4*>(sh.w + 4 * (c + 8 * i));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float sg = sigmoidf_(z[e]);
+                        z[e] = f * (silu ? z[e] * sg : sg);
+                    }
+                    x[i] = make_float4(x[i].x * wn.x * z[0], x[i].y * wn.y * z[1], x[i].z * wn.z * z[2], x[i].w * wn.w * z[3]);
+                }
+                if (whole) st4(so, ODT, r * 128 + 4 * (c + 8 * i), x[i]);
+                else if (valid) st4(o.out, ODT, at + 32 * i, x[i]);
+            }
+            umma::fence_async_smem();
+            if (tid == 0) umma::bulk_store_wait_read();    // the previous group's rows have left: the other buffers are free behind the barrier
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            if (whole && tid == 0) {
+                if (raw) umma::tma_store_rows(&maps.raw, h * 128, start + 16 * g, st);
+                umma::tma_store_rows(&maps.out, h * 128, start + 16 * g, so);
+                umma::bulk_store_commit();
+            }
+            ++buf;
+        }
+        __syncwarp();
+        if (lane == 0) umma::arrive(&sh.gFree);
+    }
+    if (tid == 0) umma::bulk_store_wait_read();
+}
+
+template <int OUT>
+__device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutFwd& o, const ChainMaps& maps) {
+    using namespace rc;
+    using L = RecurLayout<(OUT >= 0)>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    RecurShared& sh = *reinterpret_cast<RecurShared*>(base + 2 * RECUR_BUF);
+    uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
+    RecurShared& sh = *reinterpret_cast<RecurShared*>(base + L::TILES);
     const bool trans = blockIdx.x == 1;
     const int h = blockIdx.y, seg = blockIdx.z, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-
+    if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        if (tid == 0) atomicExch(&umma::g_timeout_flag, 1u);
+        return;
+    }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (tid == 0) {
-        for (uint64_t* b : {&sh.full[0], &sh.full[1], &sh.mm1, &sh.mm2}) umma::mbar_init(b, 1);
-        for (uint64_t* b : {&sh.opS, &sh.opV}) umma::mbar_init(b, COMPUTE / 32);
+        for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1, &sh.mm2, &sh.mmO,
+                            &sh.fullG, &sh.freed[0], &sh.freed[1]})
+            umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree, &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, COMPUTE / 32);
+        umma::mbar_init(&sh.oFree, 4);
+        umma::mbar_init(&sh.gFree, 4);
         umma::fence_barrier_init();
     }
     umma::fence_before_sync();
@@ -157,37 +280,114 @@ __global__ void __launch_bounds__(rc::THREADS, 1) recur_fwd_tc_kernel(const Mkda
         if (w > c_beg) { cut = true; c_beg = trans ? c_end : w; }
     }
     const int n = c_end - c_beg;
+    auto buf_n = [&](int k) { return base + L::N + (k % L::D) * L::T; };
+    auto buf_k = [&](int k) { return base + L::K + (k % L::D) * L::T; };
+    auto buf_u = [&](int k) { return base + L::U + (k % L::D) * L::T; };
+    const bool save_h = OUT >= 0 && p.h;
 
-    if (warp == WARP_LOAD) {
-        if (umma::elect_one()) {
-            for (int k = 0; k < n; ++k) {
-                if (k >= 2) umma::mbar_wait(&sh.mm2, k & 1);          // step k - 2 is done with its buffer
-                const size_t it = (size_t)(c_beg + k) * HV + h;
-                uint8_t* buf = base + (k & 1) * RECUR_BUF;
-                uint64_t* bar = &sh.full[k & 1];
-                umma::mbar_expect_tx(bar, (trans ? 2 : 3) * umma::CHUNK_TILE_BYTES + DK * 4);
-                umma::bulk_load(buf, reinterpret_cast<const uint8_t*>(p.nw) + it * umma::CHUNK_TILE_BYTES, umma::CHUNK_TILE_BYTES, bar);
-                umma::bulk_load(buf + 32768, reinterpret_cast<const uint8_t*>(p.kbar) + it * umma::CHUNK_TILE_BYTES, umma::CHUNK_TILE_BYTES, bar);
-                umma::bulk_load(sh.gl[k & 3], p.gl + it * DK, DK * 4, bar);
-                if (!trans) umma::bulk_load(buf + 65536, reinterpret_cast<const uint8_t*>(p.u) + it * umma::CHUNK_TILE_BYTES, umma::CHUNK_TILE_BYTES, bar);
+    if (warp >= 16) {
+        if (OUT >= 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+        if (warp == WARP_LOAD) {
+            if (umma::elect_one()) {
+                auto tile = [&](uint8_t* dst, const float* t, int k, uint32_t bytes, uint64_t* bar) {
+                    umma::bulk_load(dst, reinterpret_cast<const uint8_t*>(t) + ((size_t)(c_beg + k) * HV + h) * bytes, bytes, bar);
+                };
+                auto one = [&](uint8_t* dst, const float* t, int k, uint64_t* bar) {
+                    umma::mbar_expect_tx(bar, umma::CHUNK_TILE_BYTES);
+                    tile(dst, t, k, umma::CHUNK_TILE_BYTES, bar);
+                };
+                auto load_n = [&](int k) {
+                    if (k >= n) return;
+                    uint64_t* bar = &sh.fullN[k % L::D];
+                    umma::mbar_expect_tx(bar, umma::CHUNK_TILE_BYTES + DK * 4);
+                    tile(buf_n(k), p.nw, k, umma::CHUNK_TILE_BYTES, bar);
+                    umma::bulk_load(sh.gl[k & 3], p.gl + ((size_t)(c_beg + k) * HV + h) * DK, DK * 4, bar);
+                };
+                auto load_k = [&](int k) { if (k < n) one(buf_k(k), p.kbar, k, &sh.fullK[k % L::D]); };
+                auto load_u = [&](int k) { if (k < n && !trans) one(buf_u(k), p.u, k, &sh.fullU[k % L::D]); };
+                auto load_q = [&](int k) { if (OUT >= 0 && k < n) one(base + L::Q, o.qs, k, &sh.fullQ); };
+                auto load_a = [&](int k) {
+                    if (OUT < 0 || k >= n) return;
+                    umma::mbar_expect_tx(&sh.fullA, umma::QUARTER_TILE_BYTES);
+                    tile(base + L::A, o.Aqk, k, umma::QUARTER_TILE_BYTES, &sh.fullA);
+                };
+                load_u(0); load_n(0); load_k(0); load_q(0); load_a(0);
+                if (L::D > 1) { load_n(1); load_u(1); load_k(1); }
+                if (n > 0) { umma::mbar_wait(&sh.uFree, 0); load_u(L::D); }
+                for (int k = 0; k < n; ++k) {              // each buffer is refilled as soon as its product is done
+                    umma::mbar_wait(&sh.mm1, k & 1);
+                    load_n(k + L::D);
+                    if (k + 1 < n) {
+                        if (L::D > 1) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 1 + L::D); }
+                    }
+                    umma::mbar_wait(&sh.mm2, k & 1);
+                    load_k(k + L::D);
+                    load_q(k + 1);
+                    if (OUT >= 0) {
+                        umma::mbar_wait(&sh.mmO, k & 1);
+                        load_a(k + 1);
+                        if (k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
+                    }
+                }
             }
-        }
-        __syncwarp();
-    } else if (warp == WARP_MMA) {
-        if (umma::elect_one()) {
-            for (int k = 0; k < n; ++k) {
-                const uint8_t* buf = base + (k & 1) * RECUR_BUF;
-                umma::mbar_wait(&sh.full[k & 1], (k >> 1) & 1);
-                wait_mma(&sh.opS, k & 1);
-                umma::gemm_ta(tmem + ((k & 1) ? D1 : D0), tmem + SH, tmem + SL, umma::opnd_mn(buf, buf + 16384, 128), 64, 128, trans ? 0u : 1u);
-                umma::commit(&sh.mm1);
-                wait_mma(&sh.opV, k & 1);
-                umma::gemm_ta(tmem + X, tmem + VH, tmem + VL, umma::opnd_mn(buf + 32768, buf + 49152, 64), 128, 64, 0u);
-                umma::commit(&sh.mm2);
+            __syncwarp();
+        } else if (warp == WARP_MMA) {
+            if (umma::elect_one()) {
+                for (int k = 0; k < n; ++k) {
+                    umma::mbar_wait(&sh.fullN[k % L::D], (k / L::D) & 1);
+                    wait_mma(&sh.opS, k & 1);
+                    umma::gemm_ta(tmem + ((k & 1) ? D1 : D0), tmem + SH, tmem + SL, umma::opnd_mn(buf_n(k), buf_n(k) + 16384, 128), 64, 128, trans ? 0u : 1u);
+                    umma::commit(&sh.mm1);
+                    if (OUT >= 0) {
+                        umma::mbar_wait(&sh.fullQ, k & 1);
+                        if (k) wait_mma(&sh.oFree, (k - 1) & 1);
+                        umma::gemm_ta(tmem + O, tmem + SH, tmem + SL, umma::opnd_k(base + L::Q, base + L::Q + 16384, 64), 64, 128, 0u);
+                    }
+                    umma::mbar_wait(&sh.fullK[k % L::D], (k / L::D) & 1);
+                    wait_mma(&sh.opV, k & 1);
+                    umma::gemm_ta(tmem + X, tmem + VH, tmem + VL, umma::opnd_mn(buf_k(k), buf_k(k) + 16384, 64), 128, 64, 0u);
+                    umma::commit(&sh.mm2);
+                    if (OUT >= 0) {
+                        umma::mbar_wait(&sh.fullA, k & 1);
+                        umma::gemm_ta(tmem + O, tmem + VH, tmem + VL, umma::opnd_k(base + L::A, base + L::A + 8192, 64), 64, 64, 1u);
+                        umma::commit(&sh.mmO);
+                    }
+                }
             }
+            __syncwarp();
+        } else if (OUT >= 0 && warp >= 20) {
+            if (o.has_norm) recur_epilogue<OUT < 0 ? 0 : OUT, true>(o, maps, sh, base, h, c_beg, n);
+            else recur_epilogue<OUT < 0 ? 0 : OUT, false>(o, maps, sh, base, h, c_beg, n);
+        } else if (OUT > 0 && warp == WARP_GATE) {
+            if (o.has_norm && umma::elect_one()) {
+                for (int k = 0; k < n; ++k) {              // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
+                    const int start = o.L.chunk_start[c_beg + k];
+                    if (k) {
+                        umma::tma_prefetch_rows(&maps.gate, h * 128, start);
+                        umma::mbar_wait(&sh.gFree, (k - 1) & 1);
+                    }
+                    umma::mbar_expect_tx(&sh.fullG, 16384);
+                    umma::tma_load_rows(base + L::G, &maps.gate, h * 128, start, &sh.fullG);
+                }
+            }
+            __syncwarp();
+        } else if (OUT >= 0 && warp == WARP_STORE) {
+            if (save_h && umma::elect_one()) {
+                for (int k = 0; k < n; ++k) {
+                    uint8_t* dst = reinterpret_cast<uint8_t*>(p.h) + ((size_t)(c_beg + k) * HV + h) * umma::STATE_TILE_BYTES;
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        umma::mbar_wait(&sh.ready[hf], k & 1);
+                        umma::bulk_store(dst + hf * 32768, base + L::S, 32768);
+                        umma::bulk_store_wait_read();
+                        umma::arrive(&sh.freed[hf]);
+                    }
+                }
+            }
+            __syncwarp();
         }
-        __syncwarp();
     } else {
+        if (OUT >= 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
         const int cg = warp >> 2, row = (warp & 3) * 32 + lane;
         const bool vf = p.state_v_first != 0;
         float s[32];
@@ -200,19 +400,22 @@ __global__ void __launch_bounds__(rc::THREADS, 1) recur_fwd_tc_kernel(const Mkda
         }
         // u^T of step k into the accumulator that its first product adds to
         auto preload_u = [&](int k) {
-            umma::mbar_wait(&sh.full[k & 1], (k >> 1) & 1);
-            if (trans) return;
-            const uint8_t* u = base + (k & 1) * RECUR_BUF + 65536;
-            float a[8];
+            umma::mbar_wait(&sh.fullN[k % L::D], (k / L::D) & 1);      // this thread reads the decay factors that come with nw^T
+            if (!trans) {
+                umma::mbar_wait(&sh.fullU[k % L::D], (k / L::D) & 1);
+                const uint8_t* u = buf_u(k);
+                float a[8];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                umma::load_tile8(u, u + 16384, 128, row, 2 * cg + i, a);
-                uint32_t w[8];
+                for (int i = 0; i < 2; ++i) {
+                    umma::load_tile8(u, u + 16384, 128, row, 2 * cg + i, a);
+                    uint32_t w[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(a[e]);
-                umma::tmem_st8(umma::tmem_addr(tmem, warp, ((k & 1) ? D1 : D0) + cg * 16 + 8 * i), w);
+                    for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(a[e]);
+                    umma::tmem_st8(umma::tmem_addr(tmem, warp, ((k & 1) ? D1 : D0) + cg * 16 + 8 * i), w);
+                }
+                umma::tmem_wait_st();
             }
-            umma::tmem_wait_st();
+            signal_tmem(&sh.uFree, lane);
         };
         if (n > 0) preload_u(0);
         for (int k = 0; k < n; ++k) {
@@ -221,22 +424,31 @@ __global__ void __launch_bounds__(rc::THREADS, 1) recur_fwd_tc_kernel(const Mkda
                 wait_mma(&sh.mm2, (k - 1) & 1);
                 advance_state(umma::tmem_addr(tmem, warp, X + cg * 32), &sh.gl[(k - 1) & 3][cg * 32], s);
             }
-            {
-                uint32_t hi[16], lo[16];
-                state_operand(tmem, warp, cg, s, hi, lo);
-                signal_tmem(&sh.opS, lane);
-                if (p.h && !trans) save_state_tile(reinterpret_cast<uint8_t*>(p.h) + it * umma::STATE_TILE_BYTES, row, cg, hi, lo);
+            uint32_t hi[16], lo[16];
+            state_operand(tmem, warp, cg, s, hi, lo);
+            signal_tmem(&sh.opS, lane);
+            if (save_h) {
+                if (k) umma::mbar_wait(&sh.freed[1], (k - 1) & 1);
+                stage_state(base + L::S, row, cg, hi);
+                umma::signal(&sh.ready[0], lane);
+            } else if (OUT < 0 && p.h && !trans) {
+                save_state_tile(reinterpret_cast<uint8_t*>(p.h) + it * umma::STATE_TILE_BYTES, row, cg, hi, lo);
             }
             wait_mma(&sh.mm1, k & 1);
             {
-                uint32_t hi[8], lo[8];
-                v_operand(tmem, (k & 1) ? D1 : D0, warp, cg, hi, lo);
+                uint32_t vh[8], vl[8];
+                v_operand(tmem, (k & 1) ? D1 : D0, warp, cg, vh, vl);
                 signal_tmem(&sh.opV, lane);
                 if (p.Vd && !trans) {
                     uint8_t* tile = reinterpret_cast<uint8_t*>(p.Vd) + it * umma::CHUNK_TILE_BYTES;
-                    store_pair(tile, 128, row, 2 * cg, hi);
-                    store_pair(tile + 16384, 128, row, 2 * cg, lo);
+                    store_pair(tile, 128, row, 2 * cg, vh);
+                    store_pair(tile + 16384, 128, row, 2 * cg, vl);
                 }
+            }
+            if (save_h) {
+                umma::mbar_wait(&sh.freed[0], k & 1);
+                stage_state(base + L::S, row, cg, lo);
+                umma::signal(&sh.ready[1], lane);
             }
             if (k + 1 < n) preload_u(k + 1);
         }
@@ -257,11 +469,43 @@ __global__ void __launch_bounds__(rc::THREADS, 1) recur_fwd_tc_kernel(const Mkda
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
+__global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p) { recur_body<-1>(p, MkdaOutFwd{}, ChainMaps{}); }
+template <int OUT>
+__global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const __grid_constant__ ChainMaps maps) { recur_body<OUT>(p.r, p.o, maps); }
+
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream) {
+    using L = RecurLayout<false>;
     auto kern = recur_fwd_tc_kernel;
-    if (int e = ensure_smem((const void*)kern, RECUR_SMEM, "recur_fwd")) return e;
-    kern<<<dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), rc::THREADS, RECUR_SMEM, stream>>>(*p);
+    if (int e = ensure_smem((const void*)kern, L::SMEM, "recur_fwd")) return e;
+    kern<<<dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream>>>(*p);
     return check_launch("recur_fwd");
+}
+
+template <int OUT>
+static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, cudaStream_t stream) {
+    using L = RecurLayout<true>;
+    auto kern = chain_fwd_tc_kernel<OUT>;
+    if (int e = ensure_smem((const void*)kern, L::SMEM, "chain_fwd")) return e;
+    static const int regs = kernel_registers((const void*)kern);
+    if (regs < L::REGS) return set_error(MKDA_ERR_LAUNCH, "chain_fwd: built with fewer registers than its warps redistribute");
+    ChainMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    const unsigned long long rows = (unsigned long long)p->o.L.TT, cols = (unsigned long long)p->o.L.HV * 128;
+    int e = 0;
+    if (p->o.has_norm && OUT != MKDA_F32) e = make_rows_map(&maps.gate, p->o.gate, 2, rows, cols, "chain_fwd");
+    if (!e && p->o.o_raw) e = make_rows_map(&maps.raw, p->o.o_raw, 4, rows, cols, "chain_fwd", 16);
+    if (!e) e = make_rows_map(&maps.out, p->o.out, p->o.out_dtype == MKDA_F32 ? 4 : 2, rows, cols, "chain_fwd", 16);
+    if (e) return e;
+    kern<<<dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream>>>(*p, maps);
+    return check_launch("chain_fwd");
+}
+int launch_chain_fwd_tc(const MkdaChainFwd* p, cudaStream_t stream) {
+    switch (p->o.has_norm ? p->o.gate_dtype : p->o.out_dtype) {
+        case MKDA_F32: return launch_chain_fwd_tc_t<MKDA_F32>(p, stream);
+        case MKDA_BF16: return launch_chain_fwd_tc_t<MKDA_BF16>(p, stream);
+        case MKDA_F16: return launch_chain_fwd_tc_t<MKDA_F16>(p, stream);
+    }
+    return set_error(MKDA_ERR_ARG, "chain_fwd: unsupported dtype");
 }
 
 // ---------------------------------------------------------------------------------------------------------
