@@ -118,7 +118,7 @@ PyObject* check(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all, longest), scale, want_ht,
+// layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all, longest, chain), scale, want_ht,
 //       v_first, gate mode, lower bound or None, beta sigmoid, beta scale, l2, act or None, eps, warm-up threshold or None) -> (o, ht or None)
 PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -131,7 +131,7 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!tensor_arg(a[10], tables)) return nullptr;
     Call c;
     int seg, all;
-    if (!PyArg_ParseTuple(a[11], "iiiiii", &c.NC, &c.NS, &c.N, &seg, &all, &c.longest)) return nullptr;
+    if (!PyArg_ParseTuple(a[11], "iiiiiii", &c.NC, &c.NS, &c.N, &seg, &all, &c.longest, &c.chain)) return nullptr;
     c.segmented = seg; c.covers_all = all;
     c.B = (int)in.q.size(0); c.T = (int)in.q.size(1); c.HK = (int)in.q.size(2); c.HV = (int)in.v.size(2); c.TT = c.B * c.T;
     c.dev = in.q.device();
@@ -176,9 +176,10 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         }
         {
             at::AutoGradMode off(false);
-            // Nothing to differentiate and no sequence longer than a handful of tokens: the recurrence itself is cheaper than a 64-row chunk (one
-            // token: 9 instead of 63 us of kernels at 8 sequences x 32 heads).
-            const bool step = !any && c.longest <= MKDA_STEP_MAX_TOKENS && c.N <= 65535;
+            // Running sequences continued by a handful of tokens, nothing to differentiate: the recurrence itself is cheaper than a 64-row chunk
+            // (one token: 9 instead of 63 us of kernels at 8 sequences x 32 heads).  Calls that start from zero keep to the chunk algebra, whose
+            // results for a prefix of a sequence are those of the whole sequence bit for bit.
+            const bool step = !any && in.h0.defined() && c.longest <= MKDA_STEP_MAX_TOKENS && c.N <= 65535;
             std::tie(out, ht) = step ? run_step(c, in) : run_forward(c, in, any, *saved);
         }
         if (any) {

@@ -248,6 +248,19 @@ __device__ __forceinline__ void zero_acc(float (&acc)[NT][4]) {
     for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 }
 
+// Two fp32 operations in one instruction (a pair of registers each): the staging and epilogue code is bound by instruction issue.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 both(float a) { return pack2(a, a); }
+
 // 2^x in one MUFU instruction (max relative error ~2^-22); used where 2^x scales tensor-core operands
 __device__ __forceinline__ float ex2f_(float x) {
     float r;
@@ -261,6 +274,43 @@ __device__ __forceinline__ float ex2f_(float x) {
 __device__ __forceinline__ float expf_(float x) { return ex2f_(x * RCP_LN2); }
 __device__ __forceinline__ float sigmoidf_(float z) { return __fdividef(1.f, 1.f + expf_(-z)); }
 __device__ __forceinline__ float softplusf_(float s) { return fmaxf(s, 0.f) + __log2f(1.f + expf_(-fabsf(s))) * LN2; }
+
+__device__ __forceinline__ float rcpf_(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ f32x2 ex2f2_(f32x2 v) {
+    float a, b;
+    unpack2(v, a, b);
+    return pack2(ex2f_(a), ex2f_(b));
+}
+__device__ __forceinline__ f32x2 sigmoidf2_(f32x2 z) {
+    float a, b;
+    unpack2(add2(ex2f2_(mul2(z, both(-RCP_LN2))), both(1.f)), a, b);
+    return pack2(rcpf_(a), rcpf_(b));
+}
+
+// Gated RMSNorm of a 128-value row.  Two kernels evaluate it (with the state chain, or on its own), chosen by sizes; results must not depend on
+// that choice, so the order of every operation is fixed here.  A row is 32 pieces of four values; piece c + 8 i belongs to column c = 0..7,
+// a column adds its four pieces in order, and the eight columns are then added by a butterfly (xor 4, 2, 1).
+__device__ __forceinline__ float norm_piece(const float4& x) { return __fadd_rn(fmaf(x.x, x.x, __fmul_rn(x.y, x.y)), fmaf(x.z, x.z, __fmul_rn(x.w, x.w))); }
+__device__ __forceinline__ float norm_butterfly(float s) {
+#pragma unroll
+    for (int sft = 4; sft > 0; sft >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, sft));
+    return s;
+}
+__device__ __forceinline__ float norm_rs(float sum, float eps) { return rsqrtf(fmaf(sum, 1.f / 128.f, eps)); }
+__device__ __forceinline__ float4 norm_gate(const float4& x, const float4& w, const float4& z, float rs, bool silu) {
+    f32x2 a = sigmoidf2_(pack2(z.x, z.y)), b = sigmoidf2_(pack2(z.z, z.w));
+    if (silu) { a = mul2(a, pack2(z.x, z.y)); b = mul2(b, pack2(z.z, z.w)); }
+    a = mul2(mul2(a, both(rs)), mul2(pack2(w.x, w.y), pack2(x.x, x.y)));
+    b = mul2(mul2(b, both(rs)), mul2(pack2(w.z, w.w), pack2(x.z, x.w)));
+    float4 r;
+    unpack2(a, r.x, r.y);
+    unpack2(b, r.z, r.w);
+    return r;
+}
 
 // Chunk geometry shared by all chunk-parallel kernels: flattened first token and number of valid rows.
 struct ChunkGeom {

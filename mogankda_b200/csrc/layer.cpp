@@ -65,6 +65,17 @@ bool spread_v_heads(const Call& c) {
     return groups <= 2 * sms && (groups * G + sms - 1) / sms < G * ((groups + sms - 1) / sms);
 }
 
+// Output in the kernel of the state chain, or in one of its own?  In units of 1000 SM cycles per chunk, as measured: a chain step takes 6
+// without the output; with it 8.5 (a backward pass follows) or 6.5, and 12 or 9 when the gated norm is fused; a kernel of its own takes 7
+// (11 with the norm) per chunk and SM and 6 to launch, and has all SMs.  So the separate kernel is the better one where a few long
+// chains leave SMs idle: fp16 4 x 1000 tokens x 8 heads 75 instead of 96 us, 64k packed tokens x 32 heads 2260 instead of 1770 us.
+bool output_in_chain(const Call& c, bool need_bwd) {
+    const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    const double share = (double)c.NC * c.HV / sms, steps = std::max((double)c.chain, share);
+    const double fused = steps * (c.has_ep ? (need_bwd ? 12.0 : 9.0) : (need_bwd ? 8.5 : 6.5));
+    return fused <= steps * 6.0 + share * (c.has_ep ? 11.0 : 7.0) + 6.0;
+}
+
 }  // namespace
 
 std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in) {
@@ -107,7 +118,8 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     keep.want(&s.kbar, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.qs, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.gl, c.tiles(512));
-    if (need_bwd) {
+    const bool fused = output_in_chain(c, need_bwd);
+    if (need_bwd || !fused) {
         keep.want(&s.h, c.tiles(MKDA_STATE_TILE_BYTES));
         keep.want(&s.Vd, c.tiles(MKDA_CHUNK_TILE_BYTES));
     }
@@ -180,7 +192,13 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         o.gate = in.ep_gate.data_ptr(); o.gate_dtype = dtype_code(in.ep_gate); o.act = c.act; o.eps = c.eps;
     }
     o.o_raw = s.o_raw; o.out = out.data_ptr(); o.out_dtype = dtype_code(out);
-    check_rc(mkda_chain_fwd(&p, st), "mkda_chain_fwd");
+    if (fused) {
+        check_rc(mkda_chain_fwd(&p, st), "mkda_chain_fwd");
+    } else {
+        o.h = s.h; o.Vd = s.Vd;
+        check_rc(mkda_recur_fwd(&r, st), "mkda_recur_fwd");
+        check_rc(mkda_out_fwd(&o, st), "mkda_out_fwd");
+    }
     return {out, ht};
 }
 

@@ -51,7 +51,7 @@ struct Arena {
 
 // Options and geometry of a call.
 struct Call {
-    int B, T, HK, HV, N, NC, NS, TT, longest;
+    int B, T, HK, HV, N, NC, NS, TT, longest, chain;
     bool segmented, covers_all, scalar_gate, l2, vf, want_ht, beta_sigmoid, has_ep, warm;
     int mode, act, qkv_dtype;
     float scale, lower_bound, beta_scale, eps, warm_log2;

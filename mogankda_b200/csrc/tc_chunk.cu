@@ -90,8 +90,9 @@ __global__ void __launch_bounds__(512, 1) out_fwd_tc_kernel(const MkdaOutFwd p) 
         const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
         if (umma::mma_issuer()) {
             umma::mbar_wait(&ldbar, k & 1);                // this item's tiles have landed
-            umma::gemm(tmem, umma::opnd_k(a2h, a2l, 128), umma::opnd_k(b2h, b2l, 64), 128, 64, 64, 0u);
-            umma::gemm(tmem, umma::opnd_k(a1h, a1l, 128), umma::opnd_k(b1h, b1l, 64), 128, 64, 128, 1u);
+            // the order of the chain kernel: the results do not depend on which of the two runs
+            umma::gemm(tmem, umma::opnd_k(a1h, a1l, 128), umma::opnd_k(b1h, b1l, 64), 128, 64, 128, 0u);
+            umma::gemm(tmem, umma::opnd_k(a2h, a2l, 128), umma::opnd_k(b2h, b2l, 64), 128, 64, 64, 1u);
             umma::commit(&sh.bar);
         }
         // the row pass (warp w owns rows w, w + 16, ...) fetches its gate values while the products run
@@ -122,18 +123,11 @@ __global__ void __launch_bounds__(512, 1) out_fwd_tc_kernel(const MkdaOutFwd p) 
             const size_t off = ((size_t)(start + r) * HV + h) * 128 + 4 * lane;
             if (p.o_raw) *reinterpret_cast<float4*>(p.o_raw + off) = o;
             if (p.has_norm) {
-                float ss = (o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w);
+                const float pc = norm_piece(o);
+                float ss = __shfl_sync(0xffffffffu, pc, lane & 7);
 #pragma unroll
-                for (int sft = 16; sft > 0; sft >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sft);
-                const float rs = 1.f / sqrtf(ss * (1.f / 128.f) + p.eps);
-                const float zz[4] = {zg[i].x, zg[i].y, zg[i].z, zg[i].w};
-                float a[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float sg = sigmoidf_(zz[e]);
-                    a[e] = p.act == MKDA_ACT_SILU ? zz[e] * sg : sg;
-                }
-                o = make_float4(o.x * rs * w.x * a[0], o.y * rs * w.y * a[1], o.z * rs * w.z * a[2], o.w * rs * w.w * a[3]);
+                for (int j = 1; j < 4; ++j) ss = __fadd_rn(ss, __shfl_sync(0xffffffffu, pc, (lane & 7) + 8 * j));
+                o = norm_gate(o, w, zg[i], norm_rs(norm_butterfly(ss), p.eps), p.act == MKDA_ACT_SILU);
             }
             st4(p.out, p.out_dtype, off, o);
         }

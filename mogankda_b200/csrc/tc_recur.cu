@@ -84,8 +84,8 @@ __device__ __forceinline__ void advance_state(uint32_t taddr, const float* gl, f
         for (int j4 = 0; j4 < 16; j4 += 4) {
             const float4 f = *reinterpret_cast<const float4*>(gl + 16 * hf + j4);
             const int j = 16 * hf + j4;
-            s[j] = fmaf(s[j], f.x, x[j4]); s[j + 1] = fmaf(s[j + 1], f.y, x[j4 + 1]);
-            s[j + 2] = fmaf(s[j + 2], f.z, x[j4 + 2]); s[j + 3] = fmaf(s[j + 3], f.w, x[j4 + 3]);
+            unpack2(fma2(pack2(s[j], s[j + 1]), pack2(f.x, f.y), pack2(x[j4], x[j4 + 1])), s[j], s[j + 1]);
+            unpack2(fma2(pack2(s[j + 2], s[j + 3]), pack2(f.z, f.w), pack2(x[j4 + 2], x[j4 + 3])), s[j + 2], s[j + 3]);
         }
     }
 }
@@ -151,12 +151,6 @@ struct RecurLayout {                                       // the plain recurren
 };
 struct ChainMaps { CUtensorMap gate, raw, out; };          // rows of a head: boxes of 64 (gate) and 16 rows
 
-// four consecutive 16-bit values, raw
-template <int DT>
-__device__ __forceinline__ void unpack4(const uint2& r, float (&v)[4]) {
-    v[0] = unpack1<DT>(r.x & 0xffffu); v[1] = unpack1<DT>(r.x >> 16); v[2] = unpack1<DT>(r.y & 0xffffu); v[3] = unpack1<DT>(r.y >> 16);
-}
-
 template <int DT, bool NORM>
 __device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainMaps& maps, RecurShared& sh, uint8_t* base, int h, int c_beg, int n) {
     using namespace rc;
@@ -197,30 +191,16 @@ __device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainM
                 for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(o.o_raw + at + 32 * i) = x[i];
             }
             if (NORM) {
-                float ss = 0.f;
+                float ss = norm_piece(x[0]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ss += (x[i].x * x[i].x + x[i].y * x[i].y) + (x[i].z * x[i].z + x[i].w * x[i].w);
-#pragma unroll
-                for (int sft = 4; sft > 0; sft >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, sft);
-                f = rsqrtf(ss * (1.f / 128.f) + o.eps);
+                for (int i = 1; i < 4; ++i) ss = __fadd_rn(ss, norm_piece(x[i]));
+                f = norm_rs(norm_butterfly(ss), o.eps);
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 if (NORM) {
-                    float z[4];
-                    if (DT == MKDA_F32) {
-                        const float4 z4 = ld4(o.gate, DT, at + 32 * i);
-                        z[0] = z4.x; z[1] = z4.y; z[2] = z4.z; z[3] = z4.w;
-                    } else {
-                        unpack4<DT == MKDA_F32 ? MKDA_BF16 : DT>(*reinterpret_cast<const uint2*>(base + L::G + row * 256 + 8 * (c + 8 * i)), z);
-                    }
-                    const float4 wn = *reinterpret_cast<const float4*>(sh.w + 4 * (c + 8 * i));
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float sg = sigmoidf_(z[e]);
-                        z[e] = f * (silu ? z[e] * sg : sg);
-                    }
-                    x[i] = make_float4(x[i].x * wn.x * z[0], x[i].y * wn.y * z[1], x[i].z * wn.z * z[2], x[i].w * wn.w * z[3]);
+                    const float4 z = DT == MKDA_F32 ? ld4(o.gate, DT, at + 32 * i) : ld4(base + L::G, DT, row * 128 + 4 * (c + 8 * i));
+                    x[i] = norm_gate(x[i], *reinterpret_cast<const float4*>(sh.w + 4 * (c + 8 * i)), z, f, silu);
                 }
                 if (whole) st4(so, ODT, r * 128 + 4 * (c + 8 * i), x[i]);
                 else if (valid) st4(o.out, ODT, at + 32 * i, x[i]);

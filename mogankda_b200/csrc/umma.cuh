@@ -12,6 +12,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace mkda {
 namespace umma {
 
@@ -39,7 +41,10 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 // a pair of fp32 values as packed bf16 pairs: hi = bf16(v), lo = bf16(v - hi)
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& l) {
     h = pack_bf16x2(a, b);
-    l = pack_bf16x2(a - __uint_as_float(h << 16), b - __uint_as_float(h & 0xffff0000u));
+    // the negated halves: one packed addition instead of two subtractions
+    float ra, rb;
+    unpack2(add2(pack2(a, b), pack2(__uint_as_float((h << 16) ^ 0x80000000u), __uint_as_float((h & 0xffff0000u) ^ 0x80000000u))), ra, rb);
+    l = pack_bf16x2(ra, rb);
 }
 __device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, int r, int k8, const float (&v)[8]) {
     uint32_t h[4], l[4];

@@ -34,7 +34,7 @@ class Layout:
     covers_all: bool            # every token of [0, B*T) belongs to a sequence
     host: dict = field(default_factory=dict)
     tables: torch.Tensor = None  # int32: the seven tables above, one after the other (what the native host path takes)
-    dims: tuple = ()            # (NC, NS, N, segmented, covers_all, tokens of the longest sequence)
+    dims: tuple = ()            # (NC, NS, N, segmented, covers_all, tokens of the longest sequence, chunks of the longest segment)
 
     @property
     def TT(self):
@@ -133,10 +133,12 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
         flat += tb[n] + [0] * (-len(tb[n]) % 4)
     tables = torch.tensor(flat or [0], dtype=torch.int32, device=device)
     longest = T if cu is None else max((e - s for s, e in zip(cu[:-1], cu[1:])), default=0)
+    so = tb["seg_chunk_off"]
+    chain = max((b - a for a, b in zip(so[:-1], so[1:])), default=0)
     part = {n: tables[o:o + m] for n, (o, m) in at.items()}
     NC, NS, segmented = len(tb["chunk_start"]), len(tb["seg_first"]), len(tb["seg_first"]) != tb["N"]
     lay = Layout(B=B, T=T, N=tb["N"], NC=NC, NS=NS, NG=tb["N"], segmented=segmented, covers_all=tb["covers_all"], host=tb, tables=tables,
-                 dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"]), longest), **part)
+                 dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"]), longest, chain), **part)
     if len(_cache) >= _CACHE_MAX:
         _cache.pop(0)
     _cache.append((key, cu_seqlens, ver, lay))

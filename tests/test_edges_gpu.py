@@ -68,7 +68,7 @@ def test_states_at_odd_storage_offsets(offset):
     dict(B=1, T=9, gate="precomputed", beta="precomputed", l2=False, dtype=torch.float32, epi=None, h0=False),
     dict(B=2, T=4, gate="eda", dtype=torch.bfloat16, epi="silu", x_dtype=torch.bfloat16)], ids=str)
 def test_forward_of_very_short_sequences(case):
-    """Without gradients, sequences of up to 16 tokens run token by token (17: the chunk kernels); empty sequences, padding and 4 v-heads on
+    """Without gradients and with an initial state, sequences of up to 16 tokens run token by token (17: the chunk kernels); empty sequences, padding and 4 v-heads on
     2 q/k heads included."""
     case = dict(case)
     vfirst = case.pop("vfirst", False)
@@ -102,3 +102,39 @@ def test_partial_reductions(rows, cols, group):
     got = ops.reduce_partials(x, rows, cols, group)
     ref = x.double().view(rows, cols // group, group).sum((0, 2))
     assert got.shape == ref.shape and ((got - ref).abs() <= 1e-6 * x.double().abs().view(rows, cols // group, group).sum((0, 2))).all()
+
+
+@pytest.mark.parametrize("epi", [None, "silu"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_output_in_the_chain_kernel(dtype, epi):
+    """mkda_chain_fwd against mkda_recur_fwd + mkda_out_fwd: chunks of 1, 15, 16, 17, 48 and 64 rows (its rows leave in groups of 16), states and
+    Vd saved or not.  Which of the two runs depends on the sizes of the call, results must not: bit for bit the same."""
+    from mogankda_b200 import _lib, ops
+    from mogankda_b200.index import get_layout
+    cu = (0, 1, 16, 32, 49, 97, 225, 225, 400)
+    lv, do, dht, opts, _ = make_inputs(cu=cu, T=404, HK=2, HV=4, dtype=dtype, gate="eda", seed=61)
+    lay = get_layout(1, 404, opts["cu_seqlens"], lv["q"].device)
+    rq, rk = ops.l2norm_rstd(lv["q"]), ops.l2norm_rstd(lv["k"])
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "eda", lv["A_log"], lv["dt_bias"], -5.0, 4, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, 128 ** -0.5, 2, 4)
+    h, Vd, ht, _ = ops.recur_fwd(lay, nw, u, kbar, gl, 2, 4, h0=lv["h0"])
+    norm = None if epi is None else dict(weight=lv["ep_w"], gate=lv["ep_gate"], act=epi, eps=1e-6)
+    odt = dtype if epi is None else torch.float32
+    out, raw = ops.out_fwd(lay, qs, Aqk, Vd, h, 2, 4, odt, norm=norm, keep_raw=epi is not None)
+    for save in (True, False):
+        p = _lib.STRUCTS["MkdaChainFwd"]()
+        h2, Vd2, ht2 = torch.empty_like(h), torch.empty_like(Vd), torch.empty_like(ht)
+        out2, raw2 = torch.zeros_like(out), torch.zeros(404, 4, 128, device="cuda")
+        p.r.L = p.o.L = ops._layout_struct(lay, 2, 4)
+        p.r.nw, p.r.u, p.r.kbar, p.r.gl, p.r.h0, p.r.ht = nw.data_ptr(), u.data_ptr(), kbar.data_ptr(), gl.data_ptr(), lv["h0"].data_ptr(), ht2.data_ptr()
+        if save:
+            p.r.h, p.r.Vd = h2.data_ptr(), Vd2.data_ptr()
+        p.o.qs, p.o.Aqk, p.o.out, p.o.out_dtype = qs.data_ptr(), Aqk.data_ptr(), out2.data_ptr(), ops._dt(out2)
+        if epi:
+            p.o.has_norm, p.o.norm_w, p.o.norm_w_dtype, p.o.gate, p.o.gate_dtype = 1, lv["ep_w"].data_ptr(), 0, lv["ep_gate"].data_ptr(), ops._dt(lv["ep_gate"])
+            p.o.act, p.o.eps, p.o.o_raw = ops.ACTS[epi], 1e-6, raw2.data_ptr()
+        _lib.call("mkda_chain_fwd", p, torch.cuda.current_stream().cuda_stream)
+        assert torch.equal(ht, ht2) and (not save or (torch.equal(h, h2) and torch.equal(Vd, Vd2)))
+        if epi:
+            assert torch.equal(raw, raw2)
+        assert torch.equal(out, out2)
