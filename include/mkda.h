@@ -119,6 +119,8 @@ typedef struct {
     float* kbar;   /* [NC,HV] row tiles: k 2^(gL - g) with gL the cumsum at the chunk's last token */
     float* qs;     /* [NC,HV] row tiles: scale q 2^g */
     float* gl;     /* [NC,HV,128] 2^gL, the decay of the state over the whole chunk */
+    int l2; float l2_eps;      /* 1: q and k are L2-normalised here (q_rstd / k_rstd are not read); the statistics of each row are */
+    float* q_rstd_out; float* k_rstd_out;          /* also written, [TT,HK], or NULL */
 } MkdaIntraFwd;
 int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream);
 

@@ -106,7 +106,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     Arena& keep = s.arena;
     float *u = nullptr, *hs = nullptr, *s_in = nullptr;
     int* warm_start = nullptr;
-    if (c.l2) {
+    if (c.l2 && need_bwd) {
         keep.want(&s.q_rstd, (int64_t)c.TT * c.HK * 4);
         keep.want(&s.k_rstd, (int64_t)c.TT * c.HK * 4);
     }
@@ -138,12 +138,6 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     tmp.allocate(c.dev);
     const MkdaLayout L = c.layout();
 
-    if (c.l2) {
-        MkdaL2Norm p{};
-        p.dtype = c.qkv_dtype; p.rows = c.TT * c.HK; p.eps = 1e-6f;
-        p.x = in.q.data_ptr(); p.rstd = s.q_rstd; p.x2 = in.k.data_ptr(); p.rstd2 = s.k_rstd;
-        check_rc(mkda_l2norm_rstd(&p, st), "mkda_l2norm_rstd");
-    }
     {
         MkdaGateFwd p{};
         p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate;
@@ -155,7 +149,8 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     {
         MkdaIntraFwd p{};
         p.L = L; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
-        p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.scale = c.scale;
+        p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.scale = c.scale;
+        p.l2 = c.l2; p.l2_eps = 1e-6f; p.q_rstd_out = s.q_rstd; p.k_rstd_out = s.k_rstd;
         p.A = s.A; p.Aqk = s.Aqk; p.nw = s.nw; p.u = u; p.kbar = s.kbar; p.qs = s.qs; p.gl = s.gl;
         check_rc(mkda_intra_fwd(&p, st), "mkda_intra_fwd");
     }

@@ -46,35 +46,37 @@ constexpr int INTRA_TC_SMEM = RAW_Q + 16384 + 1024;        // operands + (two 32
 static_assert(RAW_G + 32768 <= OPND_BYTES, "k / g rows must fit in the dead part of the operand region");
 static_assert(3 * CH * MLD * 4 <= 53248, "sM / sInv / sP must end below the q rows");
 
-// out[2][4] = A[2 rows][KD] * B[KD][4 columns] with fp32 FMAs in ascending k (the order every entry of the inverse has always
-// been summed in); A rows are `lda` floats apart, B rows `ldb`; all pointers 16-byte aligned.  A 2 x 4 register tile needs
-// 6 shared loads per 32 FMAs: the merges below are bound by shared-memory load issue, not by arithmetic.
+// out[2][4] = A[2 rows][KD] * B[KD][4 columns] with fp32 FMAs in ascending k; A rows are `lda` floats apart, B rows `ldb`; all pointers 16-byte
+// aligned.  A 2 x 4 register tile in few warps keeps the shared-memory loads down, which is what bounds the merges (spreading each sum
+// over four lanes, so that all 16 warps take part, needs 2.5 times the loads and the six products take 4.9 instead of 3.8 k cycles).
 template <int KD>
 __device__ __forceinline__ void mm_tile_2x4(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, float (&out)[2][4]) {
+    f32x2 o[2][2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[i][j] = 0.f;
+    for (int i = 0; i < 2; ++i) o[i][0] = o[i][1] = 0ull;
 #pragma unroll
     for (int k4 = 0; k4 < KD; k4 += 4) {
         const float4 a0 = *reinterpret_cast<const float4*>(A + k4), a1 = *reinterpret_cast<const float4*>(A + lda + k4);
         const float am[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float4 b4 = *reinterpret_cast<const float4*>(B + (k4 + k) * ldb);
-            const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(B + (k4 + k) * ldb);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) out[i][j] = fmaf(am[i][k], bv[j], out[i][j]);
+            for (int i = 0; i < 2; ++i) {
+                o[i][0] = fma2(both(am[i][k]), b.x, o[i][0]);
+                o[i][1] = fma2(both(am[i][k]), b.y, o[i][1]);
+            }
         }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { unpack2(o[i][0], out[i][0], out[i][1]); unpack2(o[i][1], out[i][2], out[i][3]); }
 }
 
 // Inverse of the unit lower-triangular 64 x 64 matrix sM into sInv (fp32, fixed summation order) by recursive halving:
 // the four 16 x 16 diagonal blocks by forward substitution, then the off-diagonal block of each 32 x 32 half and finally
 // the 32 x 32 block below the diagonal, each as  X = -B^-1 (C A^-1)  with A^-1 / B^-1 the inverses above / beside it.
-// Every entry depends on the rows up to its own only, and the order of the sums is fixed by the indices.
+// Every entry depends on the rows up to its own only, and the order of the sums is fixed by the indices.  Blocks (0, 1) and (2, 3) have to
+// be zero on entry; the blocks further above the diagonal are not touched.
 __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, float* __restrict__ sInv, IntraShared& sh) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp < 4 && lane < 16) {
@@ -82,10 +84,16 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
         float x[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
-            float s = (r == lane) ? 1.f : 0.f;
+            float s[4] = {r == lane ? 1.f : 0.f, 0.f, 0.f, 0.f};           // four partial sums: the chain from row to row is what takes the time
 #pragma unroll
-            for (int c = 0; c < r; ++c) s = fmaf(-sM[(o + r) * MLD + o + c], x[c], s);
-            x[r] = s;
+            for (int c = 0; c < r; c += 4) {
+                const float4 m = *reinterpret_cast<const float4*>(sM + (o + r) * MLD + o + c);
+                const float mv[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < r) s[e] = fmaf(-mv[e], x[c + e], s[e]);
+            }
+            x[r] = (s[0] + s[1]) + (s[2] + s[3]);
         }
 #pragma unroll
         for (int r = 0; r < 16; ++r) sInv[(o + r) * MLD + o + lane] = x[r];
@@ -94,15 +102,13 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
     {   // 16 x 16 blocks (1, 0) and (3, 2): 32 threads per block, thread = (row pair, column quad)
         const int hb = tid >> 5, rp = (tid >> 2) & 7, cq = tid & 3;
         const int ro = 32 * hb + 16, co = 32 * hb;            // block origin; A^-1 at (co, co), B^-1 at (ro, ro)
-        float o[2][4];
-        if (tid < 64) {
+        if (tid < 64) {                                       // one warp per block: no CTA-wide barrier inside
+            float o[2][4];
             mm_tile_2x4<16>(sM + (ro + 2 * rp) * MLD + co, MLD, sInv + co * MLD + co + 4 * cq, MLD, o);
 #pragma unroll
             for (int i = 0; i < 2; ++i)
                 *reinterpret_cast<float4*>(&sh.T[16 * hb + 2 * rp + i][4 * cq]) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-        }
-        __syncthreads();
-        if (tid < 64) {
+            __syncwarp();
             mm_tile_2x4<16>(sInv + (ro + 2 * rp) * MLD + ro, MLD, &sh.T[16 * hb][4 * cq], TLD, o);
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -138,7 +144,9 @@ template <int DT, bool SCALAR, bool TMA>
 __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ IntraMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ IntraShared sh;
-    __shared__ __align__(16) float sGa[5][DK];         // cumsum rows of the four block anchors, [4] = last valid row
+    // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
+    // 16 threads of a row read them without bank conflicts
+    __shared__ __align__(16) float sGa[5][DK];
     __shared__ float sGs[CH];                          // SCALAR: the cumsum of every row (rows past the end: the last valid one)
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sKQ = base + KQ_OFF;
@@ -161,19 +169,22 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     // its own, half way through the item, so that they travel while the inverse and the second products run.
     // k and q stay raw (unconverted) in registers until the item starts, so that nothing waits for them here.
     constexpr bool BULK = TMA && DT != MKDA_F32;       // fp32 rows would not fit: they travel through registers
-    float vk[2][8], vq[2][8], vg[2][8], rk[2], rq[2], beta_r = 0.f;
+    f32x2 vk[2][4], vq[2][4], vg[2][4];
+    float rk[2], rq[2], beta_r = 0.f;
     Raw8 wk[2], wq[2];
     uint32_t nin = 0;                                  // phase counter of the input-row barrier
     // the chunk table entries are read one item ahead of load_inputs: every address of an item depends on them
-    int cur_start = 0, cur_len = 1, next_start = 0, next_len = 1;
+    int cur_start = 0, cur_len = 1, cur_c = 0, cur_h = 0, cur_hk = 0, next_start = 0, next_len = 1;
+    const int G = HV / HK;
     auto table_ahead = [&](int it) {
         if (it < total) { next_start = p.L.chunk_start[it / HV]; next_len = p.L.chunk_len[it / HV]; }
     };
     auto load_inputs = [&](int it) {
-        const int c = it / HV, h = it - c * HV, hk = h / (HV / HK);
+        const int c = it / HV, h = it - c * HV, hk = h / G;
+        cur_c = c; cur_h = h; cur_hk = hk;
         const int start = next_start, len = next_len;
         cur_start = start; cur_len = len;
-        if (tid < CH) beta_r = tid < len ? p.beta[(size_t)(start + tid) * HV + h] : 0.f;
+        if (tid < CH) beta_r = p.beta[(size_t)(start + min(tid, len - 1)) * HV + h];
         else if (SCALAR && tid < 2 * CH) beta_r = p.g_c[(size_t)(start + (tid - CH < len ? tid - CH : len - 1)) * HV + h];
         if (BULK && tid == 64) {                       // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
             umma::mbar_expect_tx(&sh.ldin, 16384u + 16384u + (SCALAR ? 0u : 32768u));
@@ -188,10 +199,9 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             if (!BULK) {
                 ldraw8<DT>(p.k, tk * 128 + k8 * 8, wk[n]);
                 ldraw8<DT>(p.q, tk * 128 + k8 * 8, wq[n]);
-                if (!SCALAR) ldg8(p.g_c, MKDA_F32, ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[n]);
+                if (!SCALAR) lds8(p.g_c + ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[n]);
             }
-            rk[n] = r < len ? (p.k_rstd ? p.k_rstd[tk] : 1.f) : 0.f;
-            rq[n] = r < len ? (p.q_rstd ? p.q_rstd[tk] : 1.f) : 0.f;
+            if (!p.l2 && p.k_rstd) { rk[n] = p.k_rstd[tk]; rq[n] = p.q_rstd[tk]; }
         }
     };
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 256);
@@ -204,11 +214,10 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     if ((int)blockIdx.x < total) load_inputs(blockIdx.x);
 
     for (int item = blockIdx.x; item < total; item += stride) {
-    const int c = item / HV, h = item - c * HV;
-    const int start = cur_start, len = cur_len;
+    const int c = cur_c, h = cur_h, hk = cur_hk, start = cur_start, len = cur_len;
     table_ahead(item + stride);
     // ---- phase 0: this item's k, q, g rows into registers; park the anchor rows of g in shared memory ----
-    if (tid < CH) sh.beta[tid] = beta_r;
+    if (tid < CH) sh.beta[tid] = tid < len ? beta_r : 0.f;
     else if (SCALAR && tid < 2 * CH) sGs[tid - CH] = beta_r;
     if (BULK) {
         umma::mbar_wait(&sh.ldin, nin & 1); ++nin;
@@ -220,15 +229,54 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             if (!SCALAR) lds8(reinterpret_cast<const float*>(base + RAW_G + rr * 512 + k8 * 32), vg[n]);
         }
     }
+    float l2sum = 0.f;
+    if (p.l2) {      // L2 statistics: four sums (k, q of two rows) over the 16 threads of a row; lane bits 3 and 2 end up spelling the sum
+        float t[4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            f32x2 x[4];
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                unpack8<DT>(w ? wq[n] : wk[n], x);
+                f32x2 a = mul2(x[0], x[0]);
+#pragma unroll
+                for (int e = 1; e < 4; ++e) a = fma2(x[e], x[e], a);
+                float a0, a1;
+                unpack2(a, a0, a1);
+                t[2 * n + w] = a0 + a1;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float recv = __shfl_xor_sync(0xffffffffu, (lane & 8) ? t[j] : t[j + 2], 8);
+            t[j] = ((lane & 8) ? t[j + 2] : t[j]) + recv;
+        }
+        const float recv = __shfl_xor_sync(0xffffffffu, (lane & 4) ? t[0] : t[1], 4);
+        l2sum = ((lane & 4) ? t[1] : t[0]) + recv;
+        l2sum += __shfl_xor_sync(0xffffffffu, l2sum, 2);
+        l2sum += __shfl_xor_sync(0xffffffffu, l2sum, 1);
+        l2sum = rsqrtf(l2sum + p.l2_eps);
+        const int rr = (tid >> 4) + 4 * (lane & 8);
+        if (p.k_rstd_out && h == hk * G && (lane & 3) == 0 && rr < len)                // the backward pass reads them
+            ((lane & 4) ? p.q_rstd_out : p.k_rstd_out)[(size_t)(start + rr) * HK + hk] = l2sum;
+    }
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-        if (!SCALAR && (r & 15) == 0) sts8(&sGa[r >> 4][k8 * 8], vg[n]);
-        if (!SCALAR && r == len - 1) sts8(&sGa[4][k8 * 8], vg[n]);
+        if (!SCALAR && (r & 15) == 0) sts_halves(sGa[r >> 4], k8, vg[n]);
+        if (!SCALAR && r == len - 1) sts_halves(sGa[4], k8, vg[n]);
         unpack8<DT>(wk[n], vk[n]);
         unpack8<DT>(wq[n], vq[n]);
+        float fk = 1.f, fq = 1.f;
+        if (p.l2) {
+            fk = __shfl_sync(0xffffffffu, l2sum, (lane & 16) | (8 * n));
+            fq = __shfl_sync(0xffffffffu, l2sum, (lane & 16) | (8 * n + 4));
+        } else if (p.k_rstd) {
+            fk = rk[n]; fq = rq[n];
+        }
+        if (r >= len) fk = fq = 0.f;                       // rows past the end are zero
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { vk[n][e] *= rk[n]; vq[n][e] *= rq[n]; }
+        for (int e = 0; e < 4; ++e) { vk[n][e] = mul2(vk[n][e], both(fk)); vq[n][e] = mul2(vq[n][e], both(fq)); }
     }
     if (tid == 0) umma::bulk_store_wait_read();        // the previous item's tiles have left shared memory
     umma::fence_before_sync();
@@ -246,20 +294,19 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const int i = tid + n * 512, r = i >> 4, k8 = i & 15, I0 = r >> 4;
-            float ga[8], t8[8];
-            lds8(&sGa[I0][k8 * 8], ga);
+            f32x2 ga[4], t8[4], e8[4];
+            lds_halves(sGa[I0], k8, ga);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) t8[e] = vk[n][e] * ex2f_(vg[n][e] - ga[e]);
+            for (int e = 0; e < 4; ++e) { e8[e] = ex2f2_(sub2(vg[n][e], ga[e])); t8[e] = mul2(vk[n][e], e8[e]); }
             store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, t8);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) t8[e] = vq[n][e] * ex2f_(vg[n][e] - ga[e]);
+            for (int e = 0; e < 4; ++e) t8[e] = mul2(vq[n][e], e8[e]);
             store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, t8);
 #pragma unroll
             for (int I = 0; I < 4; ++I) {
                 if (I < I0) continue;
-                if (I > I0) lds8(&sGa[I][k8 * 8], ga);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) t8[e] = vk[n][e] * ex2f_(ga[e] - vg[n][e]);
+                if (I > I0) lds_halves(sGa[I], k8, ga);
+                scale_ex2(t8, vk[n], ga, vg[n]);
                 store_split8(base, base + KC_ALL_BYTES, KC_ALL_ROWS, kc_row(I) + r, k8, t8);      // the four column tiles stacked by rows
             }
         }
@@ -287,26 +334,31 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     // The state kernels' scaled operands, as ready-made tiles: kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g,
     // plus gl = 2^gL.  Rows past the end are zero (their k / q were zeroed above).
     {
-        float gLv[8];
-        if (!SCALAR) lds8(&sGa[4][(tid & 15) * 8], gLv);
+        f32x2 gLv[4];
+        if (!SCALAR) lds_halves(sGa[4], tid & 15, gLv);
         const float gLs = SCALAR ? sGs[CH - 1] : 0.f;      // rows past the end carry the last valid one's
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-            float t8[8];
-            const float fk = SCALAR ? ex2f_(gLs - sGs[r]) : 1.f, fq = SCALAR ? p.scale * ex2f_(sGs[r]) : 1.f;
+            f32x2 t8[4];
+            const f32x2 fk = both(SCALAR ? ex2f_(gLs - sGs[r]) : 1.f), fq = both(SCALAR ? p.scale * ex2f_(sGs[r]) : p.scale);
+            if (SCALAR) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) t8[e] = SCALAR ? vk[n][e] * fk : vk[n][e] * ex2f_(gLv[e] - vg[n][e]);
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(vk[n][e], fk);
+            } else {
+                scale_ex2(t8, vk[n], gLv, vg[n]);
+            }
             store_split8(sKB, sKB + 16384, 64, r, k8, t8);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) t8[e] = SCALAR ? vq[n][e] * fq : p.scale * vq[n][e] * ex2f_(vg[n][e]);
+            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vq[n][e], fq) : mul2(mul2(vq[n][e], fq), ex2f2_(vg[n][e]));
             store_split8(sQS, sQS + 16384, 64, r, k8, t8);
         }
         if (SCALAR && tid < DK) p.gl[((size_t)c * HV + h) * 128 + tid] = ex2f_(gLs);
         if (!SCALAR && tid < 16) {
-            float* dst = p.gl + ((size_t)c * HV + h) * 128 + tid * 8;
-            *reinterpret_cast<float4*>(dst) = make_float4(ex2f_(gLv[0]), ex2f_(gLv[1]), ex2f_(gLv[2]), ex2f_(gLv[3]));
-            *reinterpret_cast<float4*>(dst + 4) = make_float4(ex2f_(gLv[4]), ex2f_(gLv[5]), ex2f_(gLv[6]), ex2f_(gLv[7]));
+            f32x2 e8[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) e8[e] = ex2f2_(gLv[e]);
+            sts8(p.gl + ((size_t)c * HV + h) * 128 + tid * 8, e8);
         }
     }
     umma::fence_async_smem();
@@ -323,20 +375,20 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     for (int n = 0; n < 2; ++n) {
         const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
         const float b = sh.beta[r];          // 0 for rows past the end
-        const float fb = SCALAR ? b * ex2f_(sGs[r]) : 0.f;
-        float t8[8];
+        const f32x2 b2 = both(b), fb = both(SCALAR ? b * ex2f_(sGs[r]) : 0.f);
+        f32x2 t8[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) t8[e] = SCALAR ? vk[n][e] * fb : b * vk[n][e] * ex2f_(vg[n][e]);
+        for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vk[n][e], fb) : mul2(mul2(vk[n][e], b2), ex2f2_(vg[n][e]));
         store_split8(sBk, sBk + 16384, 64, r, k8, t8);
         unpack8<DT>(wv[n], t8);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) t8[e] *= b;
+        for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], b2);
         store_split8(sBv, sBv + 16384, 64, r, k8, t8);
     }
     if (tid == 0) umma::bulk_store_wait_read();    // the two tiles under sM / sInv / sP (and the q rows) have left shared memory
     __syncthreads();
     if (item + stride < total) load_inputs(item + stride);     // k, q, g, beta of the next item start travelling
-    for (int i = tid; i < CH * MLD / 4; i += 512) reinterpret_cast<float4*>(sInv)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    sInv[(32 * (tid >> 8) + ((tid >> 4) & 15)) * MLD + 32 * (tid >> 8) + 16 + (tid & 15)] = 0.f;       // blocks (0, 1) and (2, 3)
     if (SCALAR) {                             // lane = row (K rows, then Q rows), cg = 16 columns j: decay applied here, for i >= j only
         float v[16];
         umma::tmem_ld16(umma::tmem_addr(tmem, warp, 16 * cg), v);
@@ -383,6 +435,9 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         const int r = tid >> 3, k8 = tid & 7;
         float a8[8], q8[8];
         lds8(sInv + r * MLD + k8 * 8, a8);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (k8 * 8 + e > r) a8[e] = 0.f;
         lds8(sP + r * MLD + k8 * 8, q8);
         store_split8(sTA, sTA + 8192, 64, r, k8, a8);
         store_split8(sTQ, sTQ + 8192, 64, r, k8, q8);

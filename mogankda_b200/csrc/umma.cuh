@@ -55,6 +55,22 @@ __device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, in
     *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// the same for four packed pairs
+__device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, int r, int k8, const f32x2 (&v)[4]) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a, b;
+        unpack2(v[i], a, b);
+        h[i] = pack_bf16x2(a, b);
+        unpack2(add2(v[i], pack2(__uint_as_float((h[i] << 16) ^ 0x80000000u), __uint_as_float((h[i] & 0xffff0000u) ^ 0x80000000u))), a, b);
+        l[i] = pack_bf16x2(a, b);
+    }
+    const uint32_t off = tile_chunk_offset(R, r, k8);
+    *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
 // reconstruct 8 fp32 values from the hi / lo tiles at (row r, chunk k8)
 __device__ __forceinline__ void load_tile8(const uint8_t* hi, const uint8_t* lo, int R, int r, int k8, float (&v)[8]) {
     const uint32_t off = tile_chunk_offset(R, r, k8);
