@@ -48,6 +48,10 @@ __device__ __forceinline__ void unpack8(const Raw8& r, f32x2 (&v)[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = pack2(f[2 * e], f[2 * e + 1]);
 }
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(umma::smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void publish() {
     umma::fence_async_smem();
     umma::fence_before_sync();

@@ -19,9 +19,10 @@
 namespace mkda {
 
 struct IntraShared {
-    uint64_t bar, ldin;
+    uint64_t bar, bar2, ldin;
     uint32_t tmem;
-    float beta[CH];
+    float beta[2][CH];                                     // of this item and (arriving) the next
+    float rk[CH], rq[CH];                                  // L2 scales of the rows
     __align__(16) float T[32][36];
 };
 constexpr int TLD = 36;
@@ -46,45 +47,21 @@ constexpr int INTRA_TC_SMEM = RAW_Q + 16384 + 1024;        // operands + (two 32
 static_assert(RAW_G + 32768 <= OPND_BYTES, "k / g rows must fit in the dead part of the operand region");
 static_assert(3 * CH * MLD * 4 <= 53248, "sM / sInv / sP must end below the q rows");
 
-// out[2][4] = A[2 rows][KD] * B[KD][4 columns] with fp32 FMAs in ascending k; A rows are `lda` floats apart, B rows `ldb`; all pointers 16-byte
-// aligned.  A 2 x 4 register tile in few warps keeps the shared-memory loads down, which is what bounds the merges (spreading each sum
-// over four lanes, so that all 16 warps take part, needs 2.5 times the loads and the six products take 4.9 instead of 3.8 k cycles).
-template <int KD>
-__device__ __forceinline__ void mm_tile_2x4(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, float (&out)[2][4]) {
-    f32x2 o[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) o[i][0] = o[i][1] = 0ull;
-#pragma unroll
-    for (int k4 = 0; k4 < KD; k4 += 4) {
-        const float4 a0 = *reinterpret_cast<const float4*>(A + k4), a1 = *reinterpret_cast<const float4*>(A + lda + k4);
-        const float am[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(B + (k4 + k) * ldb);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                o[i][0] = fma2(both(am[i][k]), b.x, o[i][0]);
-                o[i][1] = fma2(both(am[i][k]), b.y, o[i][1]);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) { unpack2(o[i][0], out[i][0], out[i][1]); unpack2(o[i][1], out[i][2], out[i][3]); }
-}
-
-// Inverse of the unit lower-triangular 64 x 64 matrix sM into sInv (fp32, fixed summation order) by recursive halving:
+// Inverse of the unit lower-triangular 64 x 64 matrix sM into sInv (fixed summation order) by recursive halving:
 // the four 16 x 16 diagonal blocks by forward substitution, then the off-diagonal block of each 32 x 32 half and finally
 // the 32 x 32 block below the diagonal, each as  X = -B^-1 (C A^-1)  with A^-1 / B^-1 the inverses above / beside it.
 // Every entry depends on the rows up to its own only, and the order of the sums is fixed by the indices.  Blocks (0, 1) and (2, 3) have to
 // be zero on entry; the blocks further above the diagonal are not touched.
+// The merges are TF32 products with error compensation (three products, fp32 accumulation: ~2^-21 per product), one 16 x 8 tile per warp:
+// fragments need a quarter of the shared-memory loads of fp32 register tiles, which bounded them (1.05 k cycles per 32 x 32 product).
 __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, float* __restrict__ sInv, IntraShared& sh) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp < 4 && lane < 16) {
-        const int o = 16 * warp;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    if (warp < 2) {
+        const int o = 32 * warp + (lane & 16), col = lane & 15;
         float x[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
-            float s[4] = {r == lane ? 1.f : 0.f, 0.f, 0.f, 0.f};           // four partial sums: the chain from row to row is what takes the time
+            float s[4] = {r == col ? 1.f : 0.f, 0.f, 0.f, 0.f};            // four partial sums: the chain from row to row is what takes the time
 #pragma unroll
             for (int c = 0; c < r; c += 4) {
                 const float4 m = *reinterpret_cast<const float4*>(sM + (o + r) * MLD + o + c);
@@ -96,42 +73,44 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
             x[r] = (s[0] + s[1]) + (s[2] + s[3]);
         }
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sInv[(o + r) * MLD + o + lane] = x[r];
-    }
-    __syncthreads();
-    {   // 16 x 16 blocks (1, 0) and (3, 2): 32 threads per block, thread = (row pair, column quad)
-        const int hb = tid >> 5, rp = (tid >> 2) & 7, cq = tid & 3;
-        const int ro = 32 * hb + 16, co = 32 * hb;            // block origin; A^-1 at (co, co), B^-1 at (ro, ro)
-        if (tid < 64) {                                       // one warp per block: no CTA-wide barrier inside
-            float o[2][4];
-            mm_tile_2x4<16>(sM + (ro + 2 * rp) * MLD + co, MLD, sInv + co * MLD + co + 4 * cq, MLD, o);
+        for (int r = 0; r < 16; ++r) sInv[(o + r) * MLD + o + col] = x[r];
+        __syncwarp();
+        // 16 x 16 block (1, 0) or (3, 2): both of its diagonal blocks are this warp's
+        const int ro = 32 * warp + 16, co = 32 * warp;
+        float* T = &sh.T[16 * warp][0];
+        float acc[2][4];
+        zero_acc(acc);
+        warp_mma<2, 3, MLD, 1, MLD, 1>(acc, sM + ro * MLD + co, sInv + co * MLD + co, 16);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<float4*>(&sh.T[16 * hb + 2 * rp + i][4 * cq]) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-            __syncwarp();
-            mm_tile_2x4<16>(sInv + (ro + 2 * rp) * MLD + ro, MLD, &sh.T[16 * hb][4 * cq], TLD, o);
+        for (int nt = 0; nt < 2; ++nt) {
+            *reinterpret_cast<float2*>(T + g * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][0], acc[nt][1]);
+            *reinterpret_cast<float2*>(T + (g + 8) * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][2], acc[nt][3]);
+        }
+        __syncwarp();
+        zero_acc(acc);
+        warp_mma<2, 3, MLD, 1, TLD, 1>(acc, sInv + ro * MLD + ro, T, 16);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<float4*>(sInv + (ro + 2 * rp + i) * MLD + co + 4 * cq) = make_float4(-o[i][0], -o[i][1], -o[i][2], -o[i][3]);
+        for (int nt = 0; nt < 2; ++nt) {
+            *reinterpret_cast<float2*>(sInv + (ro + g) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][0], -acc[nt][1]);
+            *reinterpret_cast<float2*>(sInv + (ro + g + 8) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][2], -acc[nt][3]);
         }
     }
     __syncthreads();
-    {   // 32 x 32 block (rows 32.., columns 0..31): 128 threads, thread = (row pair, column quad)
-        const int rp = tid >> 3, cq = tid & 7;
-        float o[2][4];
-        if (tid < 128) {
-            mm_tile_2x4<32>(sM + (32 + 2 * rp) * MLD, MLD, sInv + 4 * cq, MLD, o);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<float4*>(&sh.T[2 * rp + i][4 * cq]) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-        }
-        __syncthreads();
-        if (tid < 128) {
-            mm_tile_2x4<32>(sInv + (32 + 2 * rp) * MLD + 32, MLD, &sh.T[0][4 * cq], TLD, o);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<float4*>(sInv + (32 + 2 * rp + i) * MLD + 4 * cq) = make_float4(-o[i][0], -o[i][1], -o[i][2], -o[i][3]);
-        }
+    // 32 x 32 block (rows 32.., columns 0..31): eight warps, one 16 x 8 tile each
+    const int m0 = 16 * ((warp >> 2) & 1), n0 = 8 * (warp & 3);
+    float acc[1][4];
+    if (warp < 8) {
+        zero_acc(acc);
+        warp_mma<1, 3, MLD, 1, MLD, 1>(acc, sM + (32 + m0) * MLD, sInv + n0, 32);
+        *reinterpret_cast<float2*>(&sh.T[m0 + g][n0 + 2 * t]) = make_float2(acc[0][0], acc[0][1]);
+        *reinterpret_cast<float2*>(&sh.T[m0 + g + 8][n0 + 2 * t]) = make_float2(acc[0][2], acc[0][3]);
+    }
+    __syncthreads();
+    if (warp < 8) {
+        zero_acc(acc);
+        warp_mma<1, 3, MLD, 1, TLD, 1>(acc, sInv + (32 + m0) * MLD + 32, &sh.T[0][n0], 32);
+        *reinterpret_cast<float2*>(sInv + (32 + m0 + g) * MLD + n0 + 2 * t) = make_float2(-acc[0][0], -acc[0][1]);
+        *reinterpret_cast<float2*>(sInv + (32 + m0 + g + 8) * MLD + n0 + 2 * t) = make_float2(-acc[0][2], -acc[0][3]);
     }
     __syncthreads();
 }
@@ -147,7 +126,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
     // 16 threads of a row read them without bank conflicts
     __shared__ __align__(16) float sGa[5][DK];
-    __shared__ float sGs[CH];                          // SCALAR: the cumsum of every row (rows past the end: the last valid one)
+    __shared__ float sGsb[2][CH];                      // SCALAR: the cumsum of every row (rows past the end: the last valid one)
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sKQ = base + KQ_OFF;
     float* sM = reinterpret_cast<float*>(base + OPND_BYTES);
@@ -164,61 +143,59 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int q = warp & 3, cg = warp >> 2, row = q * 32 + lane;
 
-    // Persistent: one CTA per SM walks the (chunk, v-head) items gridDim.x apart, heads fastest.  The k, q, g rows (and beta,
-    // the L2 statistics) of the NEXT item are requested into registers as soon as the current item has no more use for
-    // its own, half way through the item, so that they travel while the inverse and the second products run.
-    // k and q stay raw (unconverted) in registers until the item starts, so that nothing waits for them here.
+    // Persistent: one CTA per SM walks the (chunk, v-head) items gridDim.x apart, heads fastest.  The k, q, g rows of the NEXT item are
+    // requested as soon as the current item has no more use for their place, half way through the item, so that they travel while the
+    // inverse and the second products run.  beta (and a scalar gate's cumsum) come by asynchronous copies into the other half of a double
+    // buffer: a value that is loaded into a register under a condition is waited for where the paths join again (2 k cycles per item).
     constexpr bool BULK = TMA && DT != MKDA_F32;       // fp32 rows would not fit: they travel through registers
     f32x2 vk[2][4], vq[2][4], vg[2][4];
-    float rk[2], rq[2], beta_r = 0.f;
     Raw8 wk[2], wq[2];
     uint32_t nin = 0;                                  // phase counter of the input-row barrier
-    // the chunk table entries are read one item ahead of load_inputs: every address of an item depends on them
-    int cur_start = 0, cur_len = 1, cur_c = 0, cur_h = 0, cur_hk = 0, next_start = 0, next_len = 1;
-    const int G = HV / HK;
-    auto table_ahead = [&](int it) {
-        if (it < total) { next_start = p.L.chunk_start[it / HV]; next_len = p.L.chunk_len[it / HV]; }
-    };
-    auto load_inputs = [&](int it) {
-        const int c = it / HV, h = it - c * HV, hk = h / G;
-        cur_c = c; cur_h = h; cur_hk = hk;
-        const int start = next_start, len = next_len;
-        cur_start = start; cur_len = len;
-        if (tid < CH) beta_r = p.beta[(size_t)(start + min(tid, len - 1)) * HV + h];
-        else if (SCALAR && tid < 2 * CH) beta_r = p.g_c[(size_t)(start + (tid - CH < len ? tid - CH : len - 1)) * HV + h];
-        if (BULK && tid == 64) {                       // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
+    struct Item { int c, h, hk, start, len; } cur, nxt;
+    const int G = HV / HK, dc = stride / HV, dh = stride - dc * HV;
+    const float rG = 1.f / (float)G;
+    auto advance = [&](Item& i) { i.c += dc; i.h += dh; if (i.h >= HV) { i.h -= HV; ++i.c; } i.hk = (int)(((float)i.h + 0.5f) * rG); };
+    auto table = [&](Item& i) { const int c = min(i.c, p.L.NC - 1); i.start = p.L.chunk_start[c]; i.len = p.L.chunk_len[c]; };
+    auto load_inputs = [&](const Item& i, int buf) {
+        if (tid < CH) cp_async4(&sh.beta[buf][tid], p.beta + (size_t)(i.start + min(tid, i.len - 1)) * HV + i.h);
+        else if (SCALAR && tid < 2 * CH) cp_async4(&sGsb[buf][tid - CH], p.g_c + (size_t)(i.start + min(tid - CH, i.len - 1)) * HV + i.h);
+        if (BULK && tid == 128) {                      // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
             umma::mbar_expect_tx(&sh.ldin, 16384u + 16384u + (SCALAR ? 0u : 32768u));
-            umma::tma_load_rows(base + RAW_K, &maps.k, hk * 128, start, &sh.ldin);
-            umma::tma_load_rows(base + RAW_Q, &maps.q, hk * 128, start, &sh.ldin);
-            if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, h * 128, start, &sh.ldin);
+            umma::tma_load_rows(base + RAW_K, &maps.k, i.hk * 128, i.start, &sh.ldin);
+            umma::tma_load_rows(base + RAW_Q, &maps.q, i.hk * 128, i.start, &sh.ldin);
+            if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, i.h * 128, i.start, &sh.ldin);
         }
+        if (!BULK) {
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int i = tid + n * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
-            const size_t tk = (size_t)(start + rr) * HK + hk;
-            if (!BULK) {
+            for (int n = 0; n < 2; ++n) {
+                const int r = (tid + n * 512) >> 4, k8 = tid & 15, rr = min(r, i.len - 1);
+                const size_t tk = (size_t)(i.start + rr) * HK + i.hk;
                 ldraw8<DT>(p.k, tk * 128 + k8 * 8, wk[n]);
                 ldraw8<DT>(p.q, tk * 128 + k8 * 8, wq[n]);
-                if (!SCALAR) lds8(p.g_c + ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[n]);
+                if (!SCALAR) lds8(p.g_c + ((size_t)(i.start + rr) * HV + i.h) * 128 + k8 * 8, vg[n]);
             }
-            if (!p.l2 && p.k_rstd) { rk[n] = p.k_rstd[tk]; rq[n] = p.q_rstd[tk]; }
         }
     };
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 256);
-    if (tid == 0) { umma::mbar_init(&sh.bar, 1); umma::mbar_init(&sh.ldin, 1); umma::fence_barrier_init(); }
+    if (tid == 0) { umma::mbar_init(&sh.bar, 1); umma::mbar_init(&sh.bar2, 1); umma::mbar_init(&sh.ldin, 1); umma::fence_barrier_init(); }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
-    table_ahead(blockIdx.x);
-    if ((int)blockIdx.x < total) load_inputs(blockIdx.x);
+    cur.c = blockIdx.x / HV; cur.h = blockIdx.x - cur.c * HV; cur.hk = cur.h / G;
+    table(cur);
+    if ((int)blockIdx.x < total) load_inputs(cur, 0);
+    nxt = cur;
+    advance(nxt);
 
-    for (int item = blockIdx.x; item < total; item += stride) {
-    const int c = cur_c, h = cur_h, hk = cur_hk, start = cur_start, len = cur_len;
-    table_ahead(item + stride);
+    for (int item = blockIdx.x, it = 0; item < total; item += stride, ++it) {
+    const int c = cur.c, h = cur.h, hk = cur.hk, start = cur.start, len = cur.len;
+    float* sBeta = sh.beta[it & 1];
+    const float* sGs = sGsb[it & 1];
+    table(nxt);                                        // the chunk table entries are read ahead of load_inputs: every address depends on them
     // ---- phase 0: this item's k, q, g rows into registers; park the anchor rows of g in shared memory ----
-    if (tid < CH) sh.beta[tid] = tid < len ? beta_r : 0.f;
-    else if (SCALAR && tid < 2 * CH) sGs[tid - CH] = beta_r;
+    cp_async_wait_all();
+    if (tid < CH && tid >= len) sBeta[tid] = 0.f;
     if (BULK) {
         umma::mbar_wait(&sh.ldin, nin & 1); ++nin;
 #pragma unroll
@@ -229,54 +206,17 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             if (!SCALAR) lds8(reinterpret_cast<const float*>(base + RAW_G + rr * 512 + k8 * 32), vg[n]);
         }
     }
-    float l2sum = 0.f;
-    if (p.l2) {      // L2 statistics: four sums (k, q of two rows) over the 16 threads of a row; lane bits 3 and 2 end up spelling the sum
-        float t[4];
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            f32x2 x[4];
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                unpack8<DT>(w ? wq[n] : wk[n], x);
-                f32x2 a = mul2(x[0], x[0]);
-#pragma unroll
-                for (int e = 1; e < 4; ++e) a = fma2(x[e], x[e], a);
-                float a0, a1;
-                unpack2(a, a0, a1);
-                t[2 * n + w] = a0 + a1;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const float recv = __shfl_xor_sync(0xffffffffu, (lane & 8) ? t[j] : t[j + 2], 8);
-            t[j] = ((lane & 8) ? t[j + 2] : t[j]) + recv;
-        }
-        const float recv = __shfl_xor_sync(0xffffffffu, (lane & 4) ? t[0] : t[1], 4);
-        l2sum = ((lane & 4) ? t[1] : t[0]) + recv;
-        l2sum += __shfl_xor_sync(0xffffffffu, l2sum, 2);
-        l2sum += __shfl_xor_sync(0xffffffffu, l2sum, 1);
-        l2sum = rsqrtf(l2sum + p.l2_eps);
-        const int rr = (tid >> 4) + 4 * (lane & 8);
-        if (p.k_rstd_out && h == hk * G && (lane & 3) == 0 && rr < len)                // the backward pass reads them
-            ((lane & 4) ? p.q_rstd_out : p.k_rstd_out)[(size_t)(start + rr) * HK + hk] = l2sum;
-    }
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
         if (!SCALAR && (r & 15) == 0) sts_halves(sGa[r >> 4], k8, vg[n]);
         if (!SCALAR && r == len - 1) sts_halves(sGa[4], k8, vg[n]);
+        if (r >= len) {                                    // rows past the end are zero
+            wk[n].a = wq[n].a = make_uint4(0, 0, 0, 0);
+            if (DT == MKDA_F32) wk[n].b = wq[n].b = make_uint4(0, 0, 0, 0);
+        }
         unpack8<DT>(wk[n], vk[n]);
         unpack8<DT>(wq[n], vq[n]);
-        float fk = 1.f, fq = 1.f;
-        if (p.l2) {
-            fk = __shfl_sync(0xffffffffu, l2sum, (lane & 16) | (8 * n));
-            fq = __shfl_sync(0xffffffffu, l2sum, (lane & 16) | (8 * n + 4));
-        } else if (p.k_rstd) {
-            fk = rk[n]; fq = rq[n];
-        }
-        if (r >= len) fk = fq = 0.f;                       // rows past the end are zero
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { vk[n][e] = mul2(vk[n][e], both(fk)); vq[n][e] = mul2(vq[n][e], both(fq)); }
     }
     if (tid == 0) umma::bulk_store_wait_read();        // the previous item's tiles have left shared memory
     umma::fence_before_sync();
@@ -323,6 +263,55 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         }
         umma::commit(&sh.bar);
     }
+    // The L2 scales are applied to what comes out (Gamma and Q K^T are bilinear in the rows) and to the tiles below: finding them takes no
+    // time while the products run.  Four sums (k, q of two rows) over the 16 threads of a row; lane bits 3 and 2 end up spelling the sum.
+    float fk[2] = {1.f, 1.f}, fq[2] = {1.f, 1.f};
+    if (p.l2) {
+        float t[4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            f32x2 a = mul2(vk[n][0], vk[n][0]), b = mul2(vq[n][0], vq[n][0]);
+#pragma unroll
+            for (int e = 1; e < 4; ++e) { a = fma2(vk[n][e], vk[n][e], a); b = fma2(vq[n][e], vq[n][e], b); }
+            float a0, a1, b0, b1;
+            unpack2(a, a0, a1);
+            unpack2(b, b0, b1);
+            t[2 * n] = a0 + a1;
+            t[2 * n + 1] = b0 + b1;
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float recv = __shfl_xor_sync(0xffffffffu, (lane & 8) ? t[j] : t[j + 2], 8);
+            t[j] = ((lane & 8) ? t[j + 2] : t[j]) + recv;
+        }
+        const float recv = __shfl_xor_sync(0xffffffffu, (lane & 4) ? t[0] : t[1], 4);
+        float s = ((lane & 4) ? t[1] : t[0]) + recv;
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s = rsqrtf(s + p.l2_eps);
+        const int rr = (tid >> 4) + 4 * (lane & 8);
+        if ((lane & 3) == 0) {
+            ((lane & 4) ? sh.rq : sh.rk)[rr] = s;
+            if (p.k_rstd_out && h == hk * G && rr < len)                   // the backward pass reads them
+                ((lane & 4) ? p.q_rstd_out : p.k_rstd_out)[(size_t)(start + rr) * HK + hk] = s;
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            fk[n] = __shfl_sync(0xffffffffu, s, (lane & 16) | (8 * n));
+            fq[n] = __shfl_sync(0xffffffffu, s, (lane & 16) | (8 * n + 4));
+        }
+    } else {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int r = (tid + n * 512) >> 4;
+            if (p.k_rstd) {
+                const size_t tk = (size_t)(start + min(r, len - 1)) * HK + hk;
+                fk[n] = p.k_rstd[tk];
+                fq[n] = p.q_rstd[tk];
+            }
+            if ((lane & 15) == 0) { sh.rk[r] = fk[n]; sh.rq[r] = fq[n]; }
+        }
+    }
     // v for phase 3 is fetched while the products run
     Raw8 wv[2];
 #pragma unroll
@@ -341,16 +330,18 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         for (int n = 0; n < 2; ++n) {
             const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
             f32x2 t8[4];
-            const f32x2 fk = both(SCALAR ? ex2f_(gLs - sGs[r]) : 1.f), fq = both(SCALAR ? p.scale * ex2f_(sGs[r]) : p.scale);
+            const f32x2 sk = both(SCALAR ? fk[n] * ex2f_(gLs - sGs[r]) : fk[n]), sq = both(SCALAR ? fq[n] * p.scale * ex2f_(sGs[r]) : fq[n] * p.scale);
             if (SCALAR) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) t8[e] = mul2(vk[n][e], fk);
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(vk[n][e], sk);
             } else {
                 scale_ex2(t8, vk[n], gLv, vg[n]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], sk);
             }
             store_split8(sKB, sKB + 16384, 64, r, k8, t8);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vq[n][e], fq) : mul2(mul2(vq[n][e], fq), ex2f2_(vg[n][e]));
+            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vq[n][e], sq) : mul2(mul2(vq[n][e], sq), ex2f2_(vg[n][e]));
             store_split8(sQS, sQS + 16384, 64, r, k8, t8);
         }
         if (SCALAR && tid < DK) p.gl[((size_t)c * HV + h) * 128 + tid] = ex2f_(gLs);
@@ -374,11 +365,11 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-        const float b = sh.beta[r];          // 0 for rows past the end
-        const f32x2 b2 = both(b), fb = both(SCALAR ? b * ex2f_(sGs[r]) : 0.f);
+        const float b = sBeta[r];            // 0 for rows past the end
+        const f32x2 b2 = both(b), fb = both(SCALAR ? b * fk[n] * ex2f_(sGs[r]) : b * fk[n]);
         f32x2 t8[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vk[n][e], fb) : mul2(mul2(vk[n][e], b2), ex2f2_(vg[n][e]));
+        for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vk[n][e], fb) : mul2(mul2(vk[n][e], fb), ex2f2_(vg[n][e]));
         store_split8(sBk, sBk + 16384, 64, r, k8, t8);
         unpack8<DT>(wv[n], t8);
 #pragma unroll
@@ -387,13 +378,13 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     }
     if (tid == 0) umma::bulk_store_wait_read();    // the two tiles under sM / sInv / sP (and the q rows) have left shared memory
     __syncthreads();
-    if (item + stride < total) load_inputs(item + stride);     // k, q, g, beta of the next item start travelling
+    if (item + stride < total) load_inputs(nxt, (it & 1) ^ 1);     // k, q, g, beta of the next item start travelling
     sInv[(32 * (tid >> 8) + ((tid >> 4) & 15)) * MLD + 32 * (tid >> 8) + 16 + (tid & 15)] = 0.f;       // blocks (0, 1) and (2, 3)
     if (SCALAR) {                             // lane = row (K rows, then Q rows), cg = 16 columns j: decay applied here, for i >= j only
         float v[16];
         umma::tmem_ld16(umma::tmem_addr(tmem, warp, 16 * cg), v);
         const int i = row & 63;
-        const float gi = sGs[i], bi = sh.beta[i];
+        const float gi = sGs[i], bi = q < 2 ? sBeta[i] * sh.rk[i] : p.scale * sh.rq[i];
         float* dst = (q < 2 ? sM : sP) + i * MLD + 16 * cg;
 #pragma unroll
         for (int j4 = 0; j4 < 16; j4 += 4) {
@@ -402,8 +393,9 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             for (int e = 0; e < 4; ++e) {
                 const int j = 16 * cg + j4 + e;
                 const float E = ex2f_(fminf(gi - sGs[j], 0.f));
-                if (q < 2) o4[e] = j < i ? bi * v[j4 + e] * E : (j == i ? 1.f : 0.f);
-                else o4[e] = j <= i ? p.scale * v[j4 + e] * E : 0.f;
+                const float w = bi * v[j4 + e] * E * sh.rk[j];
+                if (q < 2) o4[e] = j < i ? w : (j == i ? 1.f : 0.f);
+                else o4[e] = j <= i ? w : 0.f;
             }
             *reinterpret_cast<float4*>(dst + j4) = make_float4(o4[0], o4[1], o4[2], o4[3]);
         }
@@ -414,7 +406,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
 #pragma unroll
         for (int e = 0; e < 16; ++e) v[e] = 0.f;
         if (cg <= I) umma::tmem_ld16(umma::tmem_addr(tmem, warp, kc_row(I) + 16 * cg), v);      // warp-uniform condition
-        const float bi = sh.beta[i];
+        const float bi = isq ? p.scale * sh.rq[i] : sBeta[i] * sh.rk[i];
         float* dst = (isq ? sP : sM) + i * MLD + 16 * cg;
 #pragma unroll
         for (int j4 = 0; j4 < 16; j4 += 4) {
@@ -422,8 +414,9 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int j = 16 * cg + j4 + e;
-                if (isq) o4[e] = j <= i ? p.scale * v[j4 + e] : 0.f;
-                else o4[e] = j < i ? bi * v[j4 + e] : (j == i ? 1.f : 0.f);
+                const float w = bi * v[j4 + e] * sh.rk[j];
+                if (isq) o4[e] = j <= i ? w : 0.f;
+                else o4[e] = j < i ? w : (j == i ? 1.f : 0.f);
             }
             *reinterpret_cast<float4*>(dst + j4) = make_float4(o4[0], o4[1], o4[2], o4[3]);
         }
@@ -451,10 +444,11 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     if (umma::mma_issuer()) {
         const umma::Opnd bA = umma::opnd_k(sTA, sTA + 8192, 64);
         umma::gemm(tmem + 128, umma::opnd_mn(sBk, sBk + 16384, 64), bA, 128, 64, 64, 0u);
+        umma::commit(&sh.bar2);                        // nw^T is read out while the u^T products run
         umma::gemm(tmem + 192, umma::opnd_mn(sBv, sBv + 16384, 64), bA, 128, 64, 64, 0u);
         umma::commit(&sh.bar);
     }
-    umma::mbar_wait(&sh.bar, 1);
+    umma::mbar_wait(&sh.bar2, it & 1);
     umma::fence_after_sync();
     {   // nw^T [K index][tok] leaves as a ready-made chunk tile (the serial kernels fetch it with one bulk copy; token
         // columns past the end are exact zeros: beta is 0 there)
@@ -464,7 +458,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         for (int j = 0; j < 16; ++j) {
             if (j < 8) n0[j] = -a[j]; else n1[j - 8] = -a[j];
         }
-        store_split8(base, base + 16384, 128, row, 2 * cg, n0);          // every operand tile is dead by now
+        store_split8(base, base + 16384, 128, row, 2 * cg, n0);          // beta k~ is dead
         store_split8(base, base + 16384, 128, row, 2 * cg + 1, n1);
     }
     umma::fence_async_smem();
@@ -473,6 +467,8 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     {   // u^T [v][tok] leaves the same way (token columns past the end are exact zeros: A has identity rows there and
         // beta v zero rows), built next to the nw tile while that one is being copied
         float b[16], u0[8], u1[8];
+        umma::mbar_wait(&sh.bar, 1);
+        umma::fence_after_sync();
         umma::tmem_ld16(umma::tmem_addr(tmem, warp, 192 + 16 * cg), b);
 #pragma unroll
         for (int j = 0; j < 8; ++j) { u0[j] = b[j]; u1[j] = b[8 + j]; }
@@ -482,6 +478,8 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     umma::fence_async_smem();
     __syncthreads();
     if (tid == 0) umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base + 32768, umma::CHUNK_TILE_BYTES);
+    cur = nxt;
+    advance(nxt);
     }   // items
     if (tid == 0) umma::bulk_store_wait_read();
     umma::fence_before_sync();
