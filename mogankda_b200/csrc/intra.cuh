@@ -26,6 +26,10 @@ __device__ __forceinline__ void sts8(float* p, const f32x2 (&v)[4]) {
     *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]);
     *reinterpret_cast<ulonglong2*>(p + 4) = make_ulonglong2(v[2], v[3]);
 }
+__device__ __forceinline__ void lds4(const float* p, f32x2 (&v)[2]) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p);
+    v[0] = a.x; v[1] = a.y;
+}
 // channels 8 k8 .. 8 k8 + 7 of a 128-float row that is stored as two planes: the lower, then the upper four of every eight
 __device__ __forceinline__ void lds_halves(const float* row, int k8, f32x2 (&v)[4]) {
     const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + 4 * k8), b = *reinterpret_cast<const ulonglong2*>(row + 64 + 4 * k8);

@@ -32,11 +32,15 @@
 // What bounds it: the tiles of an item are 272 KB, so no item can be fetched whole while another one is worked on, and an SM draws about
 // 25 B per cycle from HBM.  S, dO, Vd, dVd and A of the next item travel under the epilogue, dS' under the dW phase; k, q and g are
 // requested when that traffic is over and handed to the epilogue through shared memory (requested together with the tiles they wait
-// behind 208 KB of copies: 6 k cycles at the top of every item and as much in the epilogue).
+// behind 208 KB of copies: 6 k cycles at the top of every item and as much in the epilogue).  The products' operand reads, the copies and the
+// compute warps' own accesses share the 128 B per cycle of shared memory: some 23 k cycles of the 25 k an item takes.
+// dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
+// 64k packed tokens x 32 heads: 3.80 -> 3.25 ms by that, by operand descriptors that no longer spill in the issuing warp, by row scalars
+// read four at a time and by the L2 hint in the copy warp; 4 x 16k x 16 heads, scalar gate: 1355 -> 1250 us.
 // Shared memory (KB): S [0,64) -> [Qr; beta Kr] | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> Kc_0, Kc_1 in the dO pieces, raw k
 // and q rows in the dW pieces | Vd^T [128,160) -> Kc_3 | dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Wq; dLs] [160,192), Kc_2 [192,216),
 // scratch [216,224).
-// TMEM columns: dW 0, [D1; Z] 128, later R_I 32 I and C_I 128 + {0, 16, 48, 96}; Dq 320, Dk 384, Db 448.
+// TMEM columns: [D1; Z] 128, later C_I 128 + {0, 16, 48, 96}; dW 320, later Dq 320 and Dk 384; R_I 32 I; Db 448.
 #include "host.h"
 #include "intra.cuh"
 
@@ -57,22 +61,23 @@ constexpr int EARLY_GA = o_piece(3);
 // raw 16-bit k (pieces 0, 1) and q (2, 3) rows kept for the epilogue: 32 token rows of 256 bytes per piece
 __device__ __forceinline__ int stash(int which, int tok) { return w_piece(2 * which + (tok >> 5)) + (tok & 31) * 256; }
 __host__ __device__ constexpr int ccol(int I) { return I == 0 ? 128 : I == 1 ? 144 : I == 2 ? 176 : 224; }
-constexpr int DW = 0, D1 = 128, DQ = 320, DKB = 384, DB = 448;      // accumulator columns
+constexpr int D1 = 128, DQ = 320, DKB = 384, DW = DQ, DB = 448;     // accumulator columns; dW of the next item takes the place of Dq and Dk
 
 struct Shared {
     uint64_t fullW, fullS, fullT;                       // copies landed: (dVd, A) | (S, dO, Vd) | dS'
-    uint64_t mmW, mmL, mmT, mmI;                        // products done: dW | [D1; Z], Dq, Dk | Db | row and column terms
-    uint64_t opW, opI[4], accFree;                      // compute warps done: dW tile | intra-chunk operands per row block | accumulators and scratch
+    uint64_t mmW, mmL, mmT, mmI[4];                     // products done: dW | [D1; Z], Dq, Dk | Db | row and column terms of block I and the later ones
+    uint64_t opW, opI[4], accFree;                      // compute warps done: dW tile | intra-chunk operands per row block | scratch
     uint32_t tmem;
-    float dgl[DK], beta[CH], rk[CH], rq[CH], diag[CH], gs[CH], dbw[CH];
+    alignas(16) float dgl[DK];
+    float beta[CH], rk[CH], rq[CH], diag[CH], gs[CH], up[CH], dbw[CH];
 };
 constexpr int SMEM = TILES + (int)sizeof(Shared);
 static_assert(SMEM <= 232448, "shared memory of one CTA");
 // scratch of the intra-chunk part and the epilogue, inside the dS' tile (dead by then; the next item's arrives after accFree)
 struct Scratch {
-    float ga[5][DK];                                    // cumsum rows of the four block anchors, [4] = last valid row
+    float ga[5][DK];                                    // the anchor rows again, for the epilogue
     float col[4][DK];
-    float redg[4][CH], up[CH], re[CH];
+    float redg[4][CH], re[CH];
 };
 static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
 
@@ -97,42 +102,57 @@ __device__ __forceinline__ void red_add(float* addr, float v) {
 // summed where they are written: the first v-head of a group stores its fp32 tile, the others add to it (red.global.add.f32 by the same
 // thread to the same address, in the fixed order of the v-heads: deterministic).  The tile lives in L2 between the two passes.
 // SPREAD (few items): a group is one v-head with tiles of its own, so that no CTA works through G of them alone.
+// The walk goes on by additions: every warp takes it for every item, and an integer division is some 40 instructions.
 template <bool SPREAD>
 struct ItemWalk {
-    int grp, j, G, H, HV, ngroups, stride;                 // H groups per chunk; G v-heads per q/k head
+    int c, gr, j, G, H, HV, NC, dc, dg;                    // H groups per chunk; G v-heads per q/k head
     __device__ __forceinline__ ItemWalk(const MkdaLayout& L) {
-        HV = L.HV; G = HV / L.HK; H = SPREAD ? HV : L.HK; ngroups = L.NC * H; stride = gridDim.x; grp = blockIdx.x; j = 0;
+        HV = L.HV; G = HV / L.HK; H = SPREAD ? HV : L.HK; NC = L.NC; j = 0;
+        c = blockIdx.x / H; gr = blockIdx.x - c * H; dc = gridDim.x / H; dg = gridDim.x - dc * H;
     }
-    __device__ __forceinline__ bool valid() const { return grp < ngroups; }
-    __device__ __forceinline__ int chunk() const { return grp / H; }
-    __device__ __forceinline__ int head() const { return SPREAD ? grp % H : (grp % H) * G + j; }
-    __device__ __forceinline__ int hk() const { return SPREAD ? grp % H / G : grp % H; }
-    __device__ __forceinline__ size_t item() const { return (size_t)chunk() * HV + head(); }
-    __device__ __forceinline__ void next() { if (SPREAD || ++j == G) { j = 0; grp += stride; } }
+    __device__ __forceinline__ bool valid() const { return c < NC; }
+    __device__ __forceinline__ int chunk() const { return c; }
+    __device__ __forceinline__ int head() const { return SPREAD ? gr : gr * G + j; }
+    __device__ __forceinline__ int hk() const { return SPREAD ? gr / G : gr; }
+    __device__ __forceinline__ size_t group() const { return (size_t)c * H + gr; }
+    __device__ __forceinline__ size_t item() const { return (size_t)c * HV + head(); }
+    __device__ __forceinline__ void next() {
+        if (SPREAD || ++j == G) {
+            j = 0; c += dc; gr += dg;
+            if (gr >= H) { gr -= H; ++c; }
+        }
+    }
 };
 
 // SCALAR (one decay per token): the intra-chunk part contracts the plain k / q rows with weights that already carry
 // E_ij = 2^(g_i - g_j) (i > j, never a positive exponent):  [dq_row | T]^T = K^T [Wq E; dLs E]^T (N = 128),
 // dk_col^T = Q^T (Wq E) + K^T (beta dLs E); no anchors, and any g <= 0 is in range.  TMEM: [dq_row | T] 0, dk_col 128.
 template <bool SCALAR, bool SPREAD>
-__device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+__device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* smem, bc::Shared& sh) {
     using namespace bc;
     const uint32_t tmem = sh.tmem;
+    uint8_t* base = smem;
+    // The base passes through an empty statement in front of each group of products: kept in registers over the loop, the operand
+    // descriptors of all of them spill (the warp has 32).
+    auto fresh = [&]() { base = smem; asm volatile("" : "+l"(base)); };
     uint32_t n = 0;
-    for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
-        const uint32_t par = n & 1;
-        if (n) wait_mma(&sh.accFree, par ^ 1);
+    auto product_dW = [&](uint32_t par) {
         umma::mbar_wait(&sh.fullW, par);
-        {
-            const umma::Opnd a_lo = umma::opnd_mn(base + A_, base + A_ + 8192, 64);
-            umma::Opnd a_hi = a_lo;                      // rows 0..63 of the operand read the 8 KB in front of each half
-            a_hi.hi -= 8192; a_hi.lo -= 8192;
-            umma::gemm(tmem + DW, a_lo, umma::opnd_k(base + W_, base + W_ + 16384, 128), 128, 64, 64, 0u);
-            umma::gemm(tmem + DW + 64, a_hi, umma::opnd_k(base + W_, base + W_ + 16384, 128, 64), 128, 64, 64, 0u);
-        }
+        fresh();
+        const umma::Opnd a_lo = umma::opnd_mn(base + A_, base + A_ + 8192, 64);
+        umma::Opnd a_hi = a_lo;                          // rows 0..63 of the operand read the 8 KB in front of each half
+        a_hi.hi -= 8192; a_hi.lo -= 8192;
+        umma::gemm(tmem + DW, a_lo, umma::opnd_k(base + W_, base + W_ + 16384, 128), 128, 64, 64, 0u);
+        umma::gemm(tmem + DW + 64, a_hi, umma::opnd_k(base + W_, base + W_ + 16384, 128, 64), 128, 64, 64, 0u);
         umma::commit(&sh.mmW);
+    };
+    ItemWalk<SPREAD> w(p.L);
+    if (w.valid()) product_dW(0);
+    for (; w.valid(); ++n) {
+        const uint32_t par = n & 1;
         umma::mbar_wait(&sh.fullS, par);
-        wait_mma(&sh.opW, par);                          // the dW rows stand below dO
+        wait_mma(&sh.opW, par);                          // the dW rows stand below dO; the previous item's accumulators have been read
+        fresh();
         const umma::Opnd v_mn = umma::opnd_mn(base + V_, base + V_ + 16384, 128), r_k = umma::opnd_k(base + R_, base + R_ + 32768, 128);
         umma::gemm(tmem + D1, r_k, v_mn, 128, 64, 128, 0u);
         umma::gemm(tmem + DQ, umma::opnd_mn(base + S_, base + S_ + 32768, 128), r_k, 128, 128, 128, 0u);
@@ -140,38 +160,46 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
         umma::mbar_wait(&sh.fullT, par);
         umma::gemm(tmem + DB, umma::opnd_mn(base + T_, base + T_ + 32768, 128), v_mn, 128, 64, 128, 0u);
         umma::commit(&sh.mmT);
-        uint8_t* sKQ = base + S_;
-        uint8_t* sWD = base + WD_;
+        fresh();
         if (SCALAR) {
+            uint8_t* sKQ = base + S_;
+            uint8_t* sWD = base + WD_;
             uint8_t* sBd = base + BD_;
             wait_mma(&sh.opI[0], par);
-            umma::gemm(tmem + 0, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_k(sWD, sWD + 16384, 128), 128, 128, 64, 0u);
+            umma::gemm(tmem + 0, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_k(sWD, sWD + 16384, 128), 128, 128, 64, 1u);
             umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 64), umma::opnd_mn(sWD, sWD + 16384, 128, 0), 128, 64, 64, 0u);
             umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_mn(sBd, sBd + 8192, 64, 0), 128, 64, 64, 1u);
         } else {
 #pragma unroll
             for (int I = 3; I >= 0; --I) {                 // the column tiles arrive block by block, the largest first
                 wait_mma(&sh.opI[I], par);
+                fresh();
+                uint8_t* sKQ = base + S_;
+                uint8_t* sWD = base + WD_;
                 const int nj = 16 * (I + 1);
-                // both row terms (dq_row | T) of the block in one N = 32 product
-                umma::gemm(tmem + 32 * I, umma::opnd_mn(base + kc_hi(I), base + kc_lo(I), nj), umma::opnd_k(sWD, sWD + 16384, 128, 32 * I), 128, 32, nj, 0u);
+                // both row terms (dq_row | T) of the block in one N = 32 product, on top of the state terms
+                umma::gemm(tmem + 32 * I, umma::opnd_mn(base + kc_hi(I), base + kc_lo(I), nj), umma::opnd_k(sWD, sWD + 16384, 128, 32 * I), 128, 32, nj, 1u);
                 umma::gemm(tmem + ccol(I), umma::opnd_mn(sKQ, sKQ + 32768, 128, 32 * I), umma::opnd_mn(sWD, sWD + 16384, 128, 32 * I), 128, nj, 32, 0u);
+                if (I) umma::commit(&sh.mmI[I]);
             }
         }
-        umma::commit(&sh.mmI);
+        umma::commit(&sh.mmI[0]);
+        w.next();
+        if (w.valid()) product_dW(par ^ 1);              // under the epilogue of this item; Dq and Dk were read before opI
     }
 }
 
 // S, dO, Vd, dVd and A of the next item are requested as soon as the intra-chunk products of the current one are done (the epilogue reads
 // accumulators, the scratch and the raw rows only), dS' once dVd and A have been read and the scratch is free.
-template <bool SCALAR, bool SPREAD>
+template <bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     auto src = [](const void* t, size_t it, uint32_t bytes, uint32_t off = 0) { return static_cast<const uint8_t*>(t) + it * bytes + off; };
+    const bool from_hbm = (size_t)p.L.NC * p.L.HV > (256u << 20) / (272u << 10);          // twice L2 (126 MB)
     uint32_t n = 0;
-    for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
+    for (ItemWalk<SPREAD> w(p.L); w.valid(); ++n) {
         const size_t it = w.item();
-        if (n) umma::mbar_wait(&sh.mmI, (n & 1) ^ 1);
+        if (n) umma::mbar_wait(&sh.mmI[0], (n & 1) ^ 1);
         umma::mbar_expect_tx(&sh.fullW, umma::CHUNK_TILE_BYTES + umma::QUARTER_TILE_BYTES);
         umma::bulk_load(base + W_, src(p.dVd_t, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullW);
         umma::bulk_load(base + A_, src(p.A, it, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES, &sh.fullW);
@@ -181,17 +209,17 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
             umma::bulk_load(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
         umma::bulk_load(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
         umma::bulk_load(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
-        umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read; those products were issued after the scratch was free
+        umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read
+        if (n) umma::mbar_wait(&sh.accFree, (n & 1) ^ 1);    // ... and the scratch
         umma::mbar_expect_tx(&sh.fullT, umma::STATE_TILE_BYTES);
         umma::bulk_load(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
-        // Between here and the epilogue nothing else is fetched.  Scalar gate: the next item's tiles start on their way from HBM into L2 (1465 ->
-        // 1388 us on 4 x 16k tokens x 16 heads; its items are short and the copies were late).  With the per-channel gate the same hint
-        // costs 2 % (3.92 -> 4.02 ms on 64k packed tokens x 32 heads).
-        ItemWalk<SPREAD> nx = w;
-        nx.next();
-        if (SCALAR && nx.valid()) {
-            const size_t in = nx.item();
-            umma::mbar_wait(&sh.mmT, n & 1);
+        // Between here and the epilogue there is no room for another tile and nothing would be fetched: the next item's tiles start on their
+        // way from HBM into L2 (3.47 -> 3.23 ms on 64k packed tokens x 32 heads, 1315 -> 1250 us on 4 x 16k x 16 heads with a scalar gate).
+        // Not where the tiles of all items come close to fitting into L2 as they are: 512 items lose 3 % by it.
+        w.next();
+        if (from_hbm && w.valid()) {
+            const size_t in = w.item();
+            umma::mbar_wait(&sh.mmL, n & 1);
             umma::l2_prefetch(src(p.dVd_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
             umma::l2_prefetch(src(p.A, in, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES);
             umma::l2_prefetch(src(p.dO_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
@@ -211,7 +239,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     const int HV = p.L.HV, HK = p.L.HK;
     const uint32_t tmem = sh.tmem;
     Scratch& scr = *reinterpret_cast<Scratch*>(base + SCR_);
-    float (*early_ga)[DK] = reinterpret_cast<float (*)[DK]>(base + EARLY_GA);        // anchor rows while the scratch is still dS'
+    // cumsum rows of the four block anchors while the scratch is still dS', over dead dO rows; both copies stored as halves
+    const int ga_col = ((row >> 3) << 2) + (row & 3) + ((row & 4) << 4);
+    float (*early_ga)[DK] = reinterpret_cast<float (*)[DK]>(base + EARLY_GA);
     constexpr bool STASH = DT != MKDA_F32;                 // fp32 rows do not fit: the epilogue reads them from global memory
 
     // chunk table entries and the per-row scalars (beta | L2 statistics | scalar gate) travel one item ahead: every address of an item
@@ -242,7 +272,10 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         const bool first_of_group = w.j == 0;
         ItemWalk<SPREAD> nxt = w;
         nxt.next();
-        if (nxt.valid() && nxt.grp != w.grp) { next_start = p.L.chunk_start[nxt.chunk()]; next_len = p.L.chunk_len[nxt.chunk()]; }
+        {                                                  // loaded unconditionally, so in flight until used
+            const int c = nxt.valid() ? nxt.chunk() : w.chunk();
+            next_start = p.L.chunk_start[c]; next_len = p.L.chunk_len[c];
+        }
 
         bool tiny = false;
         if (tid < CH) {
@@ -252,9 +285,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             sh.rk[tid - CH] = ahead0; sh.rq[tid - CH] = ahead1;
         } else if (SCALAR && tid < 3 * CH) {
             sh.gs[tid - 2 * CH] = ahead0;
+            sh.up[tid - 2 * CH] = ex2f_(ahead0);
         }
         const bool long_way = sync_compute_or(tiny);       // dbeta of this chunk cannot be formed as Z_ii / beta_i
-        if (nxt.valid()) row_scalars(nxt);
 
         // ---- dW: rows of the stacked tile, dv = beta dW ----
         wait_mma(&sh.mmW, par);
@@ -291,39 +324,31 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         }
         // ---- k, q, g rows, used once the state products are under way ----
         Raw8 wk[2], wq[2];
-        float vg[2][8];
+        f32x2 vg[2][4];
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
             const int i = tid + m * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
             const size_t tk = ((size_t)(start + rr) * HK + hk) * 128 + k8 * 8;
             ldraw8<DT>(p.k, tk, wk[m]);
             ldraw8<DT>(p.q, tk, wq[m]);
-            if (!SCALAR) ldg8(p.g_c, MKDA_F32, ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[m]);
+            if (!SCALAR) lds8(p.g_c + ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[m]);
         }
         // ---- dgl[c] = sum_v S[c][v] dS'[c][v] from the two tiles: warp = 8 channels, lanes = v ----
         umma::mbar_wait(&sh.fullS, par);
         umma::mbar_wait(&sh.fullT, par);
         {
-            float acc[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+            f32x2 sum[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                const uint32_t off = umma::tile_chunk_offset(128, lane + 32 * m, warp);
-                const uint4 a4 = *reinterpret_cast<const uint4*>(base + S_ + off), b4 = *reinterpret_cast<const uint4*>(base + S_ + 32768 + off);
-                const uint4 c4 = *reinterpret_cast<const uint4*>(base + T_ + off), d4 = *reinterpret_cast<const uint4*>(base + T_ + 32768 + off);
-                const uint32_t ah[4] = {a4.x, a4.y, a4.z, a4.w}, al[4] = {b4.x, b4.y, b4.z, b4.w};
-                const uint32_t dh[4] = {c4.x, c4.y, c4.z, c4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
+                f32x2 s2[4], d2[4];
+                umma::load_tile8(base + S_, base + S_ + 32768, 128, lane + 32 * m, warp, s2);
+                umma::load_tile8(base + T_, base + T_ + 32768, 128, lane + 32 * m, warp, d2);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float s0 = __uint_as_float(ah[e] << 16) + __uint_as_float(al[e] << 16);
-                    const float s1 = __uint_as_float(ah[e] & 0xffff0000u) + __uint_as_float(al[e] & 0xffff0000u);
-                    const float d0 = __uint_as_float(dh[e] << 16) + __uint_as_float(dl[e] << 16);
-                    const float d1 = __uint_as_float(dh[e] & 0xffff0000u) + __uint_as_float(dl[e] & 0xffff0000u);
-                    acc[2 * e] = fmaf(s0, d0, acc[2 * e]);
-                    acc[2 * e + 1] = fmaf(s1, d1, acc[2 * e + 1]);
-                }
+                for (int e = 0; e < 4; ++e) sum[e] = fma2(s2[e], d2[e], sum[e]);
             }
+            float acc[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) unpack2(sum[e], acc[2 * e], acc[2 * e + 1]);
             warp_colsum(acc, lane);
             if ((lane & 3) == 0) sh.dgl[warp * 8 + (lane >> 2)] = acc[0];
         }
@@ -332,7 +357,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
-                if ((r & 15) == 0) sts8(&early_ga[r >> 4][k8 * 8], vg[m]);
+                if ((r & 15) == 0) sts_halves(early_ga[r >> 4], k8, vg[m]);
             }
         }
         sync_compute();                                    // every thread has read its part of S; anchor rows visible
@@ -341,7 +366,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         for (int m = 0; m < 2; ++m) {
             const int i = tid + m * 512, r = i >> 4, k8 = i & 15, I0 = r >> 4;
             const float rk = sh.rk[r], rq = sh.rq[r];
-            float k8v[8], q8v[8];
+            f32x2 k8v[4], q8v[4];
             unpack8<DT>(wk[m], k8v);
             unpack8<DT>(wq[m], q8v);
             if (STASH) {
@@ -351,21 +376,43 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             uint8_t* sKQ = base + S_;
             if (SCALAR) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) { k8v[e] *= rk; q8v[e] *= rq; }
+                for (int e = 0; e < 4; ++e) { k8v[e] = mul2(k8v[e], both(rk)); q8v[e] = mul2(q8v[e], both(rq)); }
                 store_split8(sKQ, sKQ + 32768, 128, r, k8, k8v);
                 store_split8(sKQ, sKQ + 32768, 128, 64 + r, k8, q8v);
             } else {
-                float ga[8];
-                lds8(&early_ga[I0][k8 * 8], ga);
+                const f32x2 kb = both(rk * sh.beta[r]), qb = both(rq);
+                f32x2 ga[4];
+                lds_halves(early_ga[I0], k8, ga);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float f = ex2f_(vg[m][e] - ga[e]);
-                    k8v[e] = k8v[e] * (rk * sh.beta[r]) * f;
-                    q8v[e] = q8v[e] * rq * f;
+                for (int e = 0; e < 4; ++e) {
+                    const f32x2 f = ex2f2_(sub2(vg[m][e], ga[e]));
+                    k8v[e] = mul2(mul2(k8v[e], kb), f);
+                    q8v[e] = mul2(mul2(q8v[e], qb), f);
                 }
                 store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, q8v);
                 store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, k8v);
             }
+        }
+        // ---- the state terms of dq and of T become the starting values of the row products: scale ea Dq and -ea Dk of the block in its
+        // 32 columns (over the old dW).  Dq and Dk are free from here on ----
+        {
+            const float ea = SCALAR ? 1.f : ex2f_(early_ga[cg][ga_col]);
+            const f32x2 sa = both(p.scale * ea), na = both(-ea);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int c0 = 16 * cg + 8 * hf;
+                f32x2 t[4], u[4];
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DQ + c0), umma::tmem_addr(tmem, warp, DKB + c0), t, u);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    f32x2 ft = sa, fu = na;
+                    if (SCALAR) { const f32x2 up = pack2(sh.up[c0 + 2 * e], sh.up[c0 + 2 * e + 1]); ft = mul2(sa, up); fu = mul2(na, up); }
+                    t[e] = mul2(ft, t[e]); u[e] = mul2(fu, u[e]);
+                }
+                umma::tmem_st8(umma::tmem_addr(tmem, warp, SCALAR ? c0 : 32 * cg + 8 * hf), t);
+                umma::tmem_st8(umma::tmem_addr(tmem, warp, SCALAR ? 64 + c0 : 32 * cg + 16 + 8 * hf), u);
+            }
+            umma::tmem_wait_st();
         }
         wait_mma(&sh.mmT, par);
         // lanes 0..63 hold D1 = dO Vd^T, lanes 64..127 Z = dW Vd^T = -dL
@@ -400,41 +447,37 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             }
         }
         if (SCALAR) {
-            if (tid < CH) {
-                const float g = sh.gs[tid];
-                scr.up[tid] = ex2f_(g);
-                scr.re[tid] = ex2f_(sh.gs[CH - 1] - g);
-            }
-            sync_compute();
+            if (tid < CH) scr.re[tid] = ex2f_(sh.gs[CH - 1] - sh.gs[tid]);
         } else {
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
-                if ((r & 15) == 0) sts8(&scr.ga[r >> 4][k8 * 8], vg[m]);
-                if (r == CH - 1) sts8(&scr.ga[4][k8 * 8], vg[m]);          // rows past the end carry the last valid row's
+                if ((r & 15) == 0) sts_halves(scr.ga[r >> 4], k8, vg[m]);
+                if (r == CH - 1) sts_halves(scr.ga[4], k8, vg[m]);         // rows past the end carry the last valid row's
             }
-            sync_compute();
-            float k8v[2][8];
+        }
+        sync_compute();                                    // diag, dbw, scratch
+        if (!SCALAR) {
+            f32x2 k8v[2][4];
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const float rk = sh.rk[(tid + m * 512) >> 4];
                 unpack8<DT>(wk[m], k8v[m]);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) k8v[m][e] *= rk;
+                for (int e = 0; e < 4; ++e) k8v[m][e] = mul2(k8v[m][e], both(rk));
             }
             const int k8 = tid & 15, r0 = tid >> 4;        // rows r0 (block 0 or 1) and 32 + r0 (block 2 or 3)
-            float ga[2][8];
-            lds8(&scr.ga[3][k8 * 8], ga[1]);
+            f32x2 ga[2][4];
+            lds_halves(scr.ga[3], k8, ga[1]);
 #pragma unroll
             for (int I = 3; I >= 0; --I) {
-                if (I) lds8(&scr.ga[I - 1][k8 * 8], ga[(I - 1) & 1]);      // one block ahead
+                if (I) lds_halves(scr.ga[I - 1], k8, ga[(I - 1) & 1]);      // one block ahead
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
                     const int r = r0 + 32 * m;
                     if (r >= 16 * (I + 1)) continue;       // warp-uniform
-                    float t8[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) t8[e] = k8v[m][e] * ex2f_(ga[I & 1][e] - vg[m][e]);
+                    f32x2 t8[4];
+                    scale_ex2(t8, k8v[m], ga[I & 1], vg[m]);
                     store_split8(base + kc_hi(I), base + kc_lo(I), 16 * (I + 1), r, k8, t8);
                 }
                 signal(&sh.opI[I], lane);
@@ -445,9 +488,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         // ---- epilogue: channel `row`, rows 16 cg .. 16 cg + 15; its inputs are fetched while the intra-chunk products run ----
         // With e = 2^(g - ga[cg]) (the anchor of the row block), ea = 2^ga[cg], h1 = 2^(ga[cg + 1] - g) <= 1 (ga[4] = gL), every decay an element
         // needs is one of e, 1 / e and h1 times a per-thread factor:
-        //   x = dq_row / e + scale ea Dq     y = T / e - ea Dk     z = h1 (fL Db + sum_{I > cg} f_I C_I) + C_cg / e
+        //   x = dq_row / e + scale ea Dq and y = T / e - ea Dk as accumulated     z = h1 (fL Db + sum_{I > cg} f_I C_I) + C_cg / e
         //   dq = e x + d k     dk = beta e y + z + d q     dg' = q e x + k (beta e y - z)     dbeta term = k e y      (d = scale dAqk_ii)
-        float kq[16], qq[16], gg[16];
+        float kq[STASH ? 1 : 16], qq[STASH ? 1 : 16], gg[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
             const int i = 16 * cg + r, ii = i < len ? i : len - 1;
@@ -458,96 +501,100 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             }
             if (!SCALAR) gg[r] = p.g_c[((size_t)(start + ii) * HV + h) * 128 + row];
         }
+        if (nxt.valid()) row_scalars(nxt);
         float raw_beta = 0.f;
         if (tid < len && p.beta_sigmoid) raw_beta = ld1(p.beta_raw, p.beta_dtype, (size_t)(start + tid) * HV + h);
-        float a0 = 0.f, a1 = 0.f, ea = 1.f, fL = 1.f, f2 = 0.f, f3 = 0.f, egL;
+        float a0 = 0.f, a1 = 0.f, fL = 1.f, f2 = 0.f, f3 = 0.f, egL;
         if (!SCALAR) {
-            a0 = scr.ga[cg][row]; a1 = scr.ga[cg + 1][row];
-            const float gL = scr.ga[4][row];
-            ea = ex2f_(a0); fL = ex2f_(gL - a1); egL = ex2f_(gL);
-            if (cg < 2) f2 = ex2f_(scr.ga[cg + 2][row] - a1);
-            if (cg < 1) f3 = ex2f_(scr.ga[cg + 3][row] - a1);
+            a0 = scr.ga[cg][ga_col]; a1 = scr.ga[cg + 1][ga_col];
+            const float gL = scr.ga[4][ga_col];
+            fL = ex2f_(gL - a1); egL = ex2f_(gL);
+            if (cg < 2) f2 = ex2f_(scr.ga[cg + 2][ga_col] - a1);
+            if (cg < 1) f3 = ex2f_(scr.ga[cg + 3][ga_col] - a1);
         } else {
             egL = ex2f_(sh.gs[CH - 1]);
         }
-        const size_t obk = (size_t)w.grp * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
+        const size_t obk = w.group() * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
         float* __restrict__ oq = p.dq_v + obk;
         float* __restrict__ ok = p.dk_v + obk;
         float* __restrict__ og = SCALAR ? p.dgp + item * CH : p.dgp + item * (size_t)(CH * DK) + row;
-        float cs = 0.f, dg_last = 0.f;
-        wait_mma(&sh.mmI, par);
+        f32x2 cs2 = 0;
+        float dg_last = 0.f;
+        wait_mma(&sh.mmI[SCALAR ? 0 : cg], par);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int c0 = 16 * cg + 8 * hf;
-            float x[8], y[8], z[8], ci[8], t[8];
+            f32x2 x[4], y[4], z[4], ci[4], t[4];
             if (SCALAR) {
-                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DQ + c0), umma::tmem_addr(tmem, warp, c0), t, x);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) x[r] = fmaf(p.scale * scr.up[c0 + r], t[r], x[r]);
-                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DKB + c0), umma::tmem_addr(tmem, warp, 64 + c0), t, y);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) y[r] = fmaf(-scr.up[c0 + r], t[r], y[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, c0), umma::tmem_addr(tmem, warp, 64 + c0), x, y);
                 umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DB + c0), umma::tmem_addr(tmem, warp, 128 + c0), t, z);
             } else {
-                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DQ + c0), umma::tmem_addr(tmem, warp, 32 * cg + 8 * hf), t, x);
-                const float sa = p.scale * ea;
-#pragma unroll
-                for (int r = 0; r < 8; ++r) x[r] = fmaf(sa, t[r], x[r]);
-                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DKB + c0), umma::tmem_addr(tmem, warp, 32 * cg + 16 + 8 * hf), t, y);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) y[r] = fmaf(-ea, t[r], y[r]);
+                umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, 32 * cg + 8 * hf), umma::tmem_addr(tmem, warp, 32 * cg + 16 + 8 * hf), x, y);
                 umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, DB + c0), umma::tmem_addr(tmem, warp, ccol(cg) + c0), t, ci);
 #pragma unroll
-                for (int r = 0; r < 8; ++r) { t[r] *= fL; z[r] = t[r]; }
+                for (int r = 0; r < 4; ++r) { t[r] = mul2(t[r], both(fL)); z[r] = t[r]; }
                 if (cg < 2) {                              // warp-uniform
-                    float u[8], v[8];
+                    f32x2 u[4], v[4];
                     umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, ccol(cg + 1) + c0), umma::tmem_addr(tmem, warp, ccol(cg + 2) + c0), u, v);
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) z[r] = fmaf(f2, v[r], z[r] + u[r]);
+                    for (int r = 0; r < 4; ++r) z[r] = fma2(both(f2), v[r], add2(z[r], u[r]));
                 }
                 if (cg == 0 || cg == 2) {
-                    float u[8];
+                    f32x2 u[4];
                     umma::tmem_ld8(umma::tmem_addr(tmem, warp, ccol(3) + c0), u);
                     const float f = cg == 0 ? f3 : 1.f;
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) z[r] = fmaf(f, u[r], z[r]);
+                    for (int r = 0; r < 4; ++r) z[r] = fma2(both(f), u[r], z[r]);
                 }
             }
-            float bsv[8], dgs[8];                          // bsv: long way only
+            // Rows past the end: sh.rk and sh.rq are 0 there, every other factor is finite.  bsv: long way only.
+            float bsv[8], dgs[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int i = c0 + r, rr = 8 * hf + r, ii = i < len ? i : len - 1;
-                const bool ok_row = i < len;
-                float kv, qv;
-                if (STASH) {                               // rows past the end carry the last valid one's
-                    kv = ld1(base + stash(0, i), DT, row);
-                    qv = ld1(base + stash(1, i), DT, row);
-                } else {
-                    kv = kq[rr]; qv = qq[rr];
+            for (int r4 = 0; r4 < 2; ++r4) {               // the rows' scalars four at a time: one broadcast read each instead of four
+                f32x2 rk4[2], rq4[2], bt4[2], dn4[2], re4[2];
+                lds4(sh.rk + c0 + 4 * r4, rk4); lds4(sh.rq + c0 + 4 * r4, rq4); lds4(sh.beta + c0 + 4 * r4, bt4); lds4(sh.diag + c0 + 4 * r4, dn4);
+                if (SCALAR) lds4(scr.re + c0 + 4 * r4, re4);
+#pragma unroll
+                for (int r2 = 0; r2 < 2; ++r2) {
+                    const int pr = 2 * r4 + r2, i = c0 + 2 * pr, rr = 8 * hf + 2 * pr;
+                    f32x2 kv, qv;
+                    if (STASH) {
+                        kv = pack2(ld1(base + stash(0, i), DT, row), ld1(base + stash(0, i + 1), DT, row));
+                        qv = pack2(ld1(base + stash(1, i), DT, row), ld1(base + stash(1, i + 1), DT, row));
+                    } else {
+                        kv = pack2(kq[rr], kq[rr + 1]); qv = pack2(qq[rr], qq[rr + 1]);
+                    }
+                    kv = mul2(kv, rk4[r2]); qv = mul2(qv, rq4[r2]);
+                    f32x2 ex, ey, zz;
+                    if (SCALAR) {
+                        ex = x[pr]; ey = y[pr];
+                        const f32x2 w2 = mul2(re4[r2], t[pr]);
+                        zz = add2(w2, z[pr]);
+                        cs2 = fma2(kv, w2, cs2);
+                    } else {
+                        const f32x2 g = pack2(gg[rr], gg[rr + 1]);
+                        const f32x2 e = ex2f2_(sub2(g, both(a0))), ei = ex2f2_(sub2(both(a0), g)), h1 = ex2f2_(sub2(both(a1), g));
+                        ex = mul2(e, x[pr]); ey = mul2(e, y[pr]);
+                        zz = fma2(h1, z[pr], mul2(ei, ci[pr]));
+                        cs2 = fma2(mul2(kv, h1), t[pr], cs2);
+                    }
+                    const f32x2 bey = mul2(bt4[r2], ey);
+                    const f32x2 dg2 = fma2(qv, ex, mul2(kv, sub2(bey, zz))), dq2 = fma2(dn4[r2], kv, ex), dk2 = fma2(dn4[r2], qv, add2(bey, zz));
+                    float dgv[2], dqv[2], dkv[2];
+                    unpack2(mul2(kv, ey), bsv[2 * pr], bsv[2 * pr + 1]);
+                    unpack2(dg2, dgv[0], dgv[1]); unpack2(dq2, dqv[0], dqv[1]); unpack2(dk2, dkv[0], dkv[1]);
+#pragma unroll
+                    for (int o = 0; o < 2; ++o) {
+                        const int io = i + o;
+                        const bool ok_row = io < len;
+                        const float dg = ok_row ? dgv[o] : 0.f, dq_e = ok_row ? dqv[o] : 0.f, dk_e = ok_row ? dkv[o] : 0.f;
+                        if (first_of_group) { oq[io * DK] = dq_e; ok[io * DK] = dk_e; }
+                        else { red_add(oq + io * DK, dq_e); red_add(ok + io * DK, dk_e); }
+                        if (SCALAR) dgs[2 * pr + o] = dg;
+                        else if (io == len - 1) dg_last = dg;
+                        else og[io * DK] = dg;
+                    }
                 }
-                kv *= sh.rk[ii]; qv *= sh.rq[ii];
-                float ex, ey, zz;
-                if (SCALAR) {
-                    ex = x[r]; ey = y[r];
-                    const float w2 = scr.re[i] * t[r];
-                    zz = w2 + z[r];
-                    if (ok_row) cs = fmaf(kv, w2, cs);
-                } else {
-                    const float g = gg[rr], e = ex2f_(g - a0), ei = ex2f_(a0 - g), h1 = ex2f_(a1 - g);
-                    ex = e * x[r]; ey = e * y[r];
-                    zz = fmaf(h1, z[r], ei * ci[r]);
-                    if (ok_row) cs = fmaf(kv * h1, t[r], cs);
-                }
-                const float bt = sh.beta[i], dgn = sh.diag[i], bey = bt * ey;
-                bsv[r] = kv * ey;
-                const float dg = ok_row ? fmaf(qv, ex, kv * (bey - zz)) : 0.f;
-                const float dq_e = ok_row ? fmaf(dgn, kv, ex) : 0.f;
-                const float dk_e = ok_row ? fmaf(dgn, qv, bey + zz) : 0.f;
-                if (first_of_group) { oq[i * DK] = dq_e; ok[i * DK] = dk_e; }
-                else { red_add(oq + i * DK, dq_e); red_add(ok + i * DK, dk_e); }
-                if (SCALAR) dgs[r] = dg;
-                else if (i == len - 1) dg_last = dg;
-                else og[i * DK] = dg;
             }
             if (long_way) {
                 warp_colsum(bsv, lane);
@@ -561,6 +608,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                 if ((lane & 3) == 0) scr.redg[q][c0 + (lane >> 2)] = dgs[0];
             }
         }
+        float cs, cs_odd;
+        unpack2(cs2, cs, cs_odd);
+        cs += cs_odd;
         // gate term of the last valid row: column sum of the inter-chunk k gradient plus gl dgl
         if (SCALAR) {
             if (cg == 0) cs = fmaf(egL, sh.dgl[row], cs);
@@ -607,7 +657,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
     }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (threadIdx.x == 0) {
-        for (uint64_t* b : {&sh.fullW, &sh.fullS, &sh.fullT, &sh.mmW, &sh.mmL, &sh.mmT, &sh.mmI}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.fullW, &sh.fullS, &sh.fullT, &sh.mmW, &sh.mmL, &sh.mmT, &sh.mmI[0], &sh.mmI[1], &sh.mmI[2], &sh.mmI[3]}) umma::mbar_init(b, 1);
         for (uint64_t* b : {&sh.opW, &sh.opI[0], &sh.opI[1], &sh.opI[2], &sh.opI[3], &sh.accFree}) umma::mbar_init(b, COMPUTE / 32);
         umma::fence_barrier_init();
     }
@@ -618,7 +668,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
             if (elect_one()) bwd_chunk_issue<SCALAR, SPREAD>(p, base, sh);
             __syncwarp();
         } else if (warp == WARP_LOAD) {
-            if (elect_one()) bwd_chunk_load<SCALAR, SPREAD>(p, base, sh);
+            if (elect_one()) bwd_chunk_load<SPREAD>(p, base, sh);
             __syncwarp();
         }
     } else {

@@ -82,6 +82,15 @@ __device__ __forceinline__ void load_tile8(const uint8_t* hi, const uint8_t* lo,
         v[2 * e + 1] = __uint_as_float(hw[e] & 0xffff0000u) + __uint_as_float(lw[e] & 0xffff0000u);
     }
 }
+__device__ __forceinline__ void load_tile8(const uint8_t* hi, const uint8_t* lo, int R, int r, int k8, f32x2 (&v)[4]) {
+    const uint32_t off = tile_chunk_offset(R, r, k8);
+    const uint4 a = *reinterpret_cast<const uint4*>(hi + off), b = *reinterpret_cast<const uint4*>(lo + off);
+    const uint32_t hw[4] = {a.x, a.y, a.z, a.w}, lw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        v[e] = add2(pack2(__uint_as_float(hw[e] << 16), __uint_as_float(hw[e] & 0xffff0000u)),
+                    pack2(__uint_as_float(lw[e] << 16), __uint_as_float(lw[e] & 0xffff0000u)));
+}
 
 // ---- descriptors ---------------------------------------------------------------------------------------------
 // shared-memory matrix descriptor: K-major, SWIZZLE_128B, 8-row groups 1024 B apart (SBO = 64 x 16 B), version 1
@@ -404,6 +413,19 @@ __device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, float (&a)[
 #pragma unroll
     for (int i = 0; i < 8; ++i) { a[i] = __uint_as_float(r[i]); b[i] = __uint_as_float(s[i]); }
 }
+// the same as packed pairs
+__device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, f32x2 (&a)[4], f32x2 (&b)[4]) {
+    float x[8], y[8];
+    tmem_ld8x2(ta, tb, x, y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { a[i] = pack2(x[2 * i], x[2 * i + 1]); b[i] = pack2(y[2 * i], y[2 * i + 1]); }
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, f32x2 (&v)[4]) {
+    float x[8];
+    tmem_ld8(taddr, x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = pack2(x[2 * i], x[2 * i + 1]);
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -413,6 +435,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                  :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const f32x2 (&v)[4]) {
+    float f[8];
+    uint32_t r[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { unpack2(v[i], f[2 * i], f[2 * i + 1]); r[2 * i] = __float_as_uint(f[2 * i]); r[2 * i + 1] = __float_as_uint(f[2 * i + 1]); }
+    tmem_st8(taddr, r);
 }
 // TMEM address of (lane quadrant of this warp, column)
 __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, int warp, int col) {

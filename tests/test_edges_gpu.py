@@ -95,6 +95,19 @@ def test_few_groups_are_spread_over_v_heads(NC, G):
     compare(one, run(orc.chunked_delta_rule, sub, do[:1], dht[:1], opts, epi, f64=True))
 
 
+@pytest.mark.parametrize("scalar", [False, True])
+def test_next_items_brought_into_l2(scalar):
+    """From 964 (chunk, v-head) items on the backward kernel hints the next item's tiles into L2, and a CTA walks several items: no bit of the
+    gradients may differ from those of the same heads in calls of 510 items."""
+    lv, do, dht, opts, epi = make_inputs(T=64 * 16 + 21, HK=60, HV=60, dtype=torch.bfloat16, gate="precomputed", scalar=scalar, beta="precomputed", h0=False, epi=None, seed=71)
+    full = run(mk.chunk_delta_rule, lv, do, dht, opts, epi)
+    for h in (slice(0, 30), slice(30, 60)):
+        sub = {n: t[:, :, h].contiguous() for n, t in lv.items()}
+        part = run(mk.chunk_delta_rule, sub, do[:, :, h].contiguous(), dht[:, h].contiguous(), opts, epi)
+        for n in ("dq", "dk", "dv", "dg", "dbeta"):
+            assert torch.equal(full[n][:, :, h], part[n]), n
+
+
 @pytest.mark.parametrize("rows,cols,group", [(1, 1, 1), (33, 7, 1), (255, 64, 1), (257, 33, 1), (1184, 128, 1), (5, 256, 128), (64, 384, 3)])
 def test_partial_reductions(rows, cols, group):
     from mogankda_b200 import ops
