@@ -210,9 +210,10 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
         umma::bulk_load(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
         umma::bulk_load(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
         umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read
-        if (n) umma::mbar_wait(&sh.accFree, (n & 1) ^ 1);    // ... and the scratch
         umma::mbar_expect_tx(&sh.fullT, umma::STATE_TILE_BYTES);
-        umma::bulk_load(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
+        umma::bulk_load(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), SCR_ - T_, &sh.fullT);
+        if (n) umma::mbar_wait(&sh.accFree, (n & 1) ^ 1);    // the last 8 KB are the scratch of the previous item's epilogue
+        umma::bulk_load(base + SCR_, src(p.dh, it, umma::STATE_TILE_BYTES, SCR_ - T_), umma::STATE_TILE_BYTES - (SCR_ - T_), &sh.fullT);
         // Between here and the epilogue there is no room for another tile and nothing would be fetched: the next item's tiles start on their
         // way from HBM into L2 (3.47 -> 3.23 ms on 64k packed tokens x 32 heads, 1315 -> 1250 us on 4 x 16k x 16 heads with a scalar gate).
         // Not where the tiles of all items come close to fitting into L2 as they are: 512 items lose 3 % by it.
@@ -242,6 +243,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     // cumsum rows of the four block anchors while the scratch is still dS', over dead dO rows; both copies stored as halves
     const int ga_col = ((row >> 3) << 2) + (row & 3) + ((row & 4) << 4);
     float (*early_ga)[DK] = reinterpret_cast<float (*)[DK]>(base + EARLY_GA);
+    // the two token rows of a thread, of blocks 0 and 3 or 1 and 2: a row of block B enters 4 - B column tiles, so each thread writes five
+    auto staged_row = [&](int m) { return m ? 32 + ((tid >> 4) ^ 16) : tid >> 4; };
     constexpr bool STASH = DT != MKDA_F32;                 // fp32 rows do not fit: the epilogue reads them from global memory
 
     // chunk table entries and the per-row scalars (beta | L2 statistics | scalar gate) travel one item ahead: every address of an item
@@ -327,7 +330,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         f32x2 vg[2][4];
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            const int i = tid + m * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
+            const int r = staged_row(m), k8 = tid & 15, rr = r < len ? r : len - 1;
             const size_t tk = ((size_t)(start + rr) * HK + hk) * 128 + k8 * 8;
             ldraw8<DT>(p.k, tk, wk[m]);
             ldraw8<DT>(p.q, tk, wq[m]);
@@ -356,7 +359,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         if (!SCALAR) {
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
-                const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
+                const int r = staged_row(m), k8 = tid & 15;
                 if ((r & 15) == 0) sts_halves(early_ga[r >> 4], k8, vg[m]);
             }
         }
@@ -364,7 +367,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         // ---- [Qr; beta Kr] over S while Db is computed, then the weights and the column tiles ----
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            const int i = tid + m * 512, r = i >> 4, k8 = i & 15, I0 = r >> 4;
+            const int r = staged_row(m), k8 = tid & 15, I0 = r >> 4;
             const float rk = sh.rk[r], rq = sh.rq[r];
             f32x2 k8v[4], q8v[4];
             unpack8<DT>(wk[m], k8v);
@@ -451,7 +454,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         } else {
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
-                const int i = tid + m * 512, r = i >> 4, k8 = i & 15;
+                const int r = staged_row(m), k8 = tid & 15;
                 if ((r & 15) == 0) sts_halves(scr.ga[r >> 4], k8, vg[m]);
                 if (r == CH - 1) sts_halves(scr.ga[4], k8, vg[m]);         // rows past the end carry the last valid row's
             }
@@ -461,12 +464,12 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             f32x2 k8v[2][4];
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
-                const float rk = sh.rk[(tid + m * 512) >> 4];
+                const float rk = sh.rk[staged_row(m)];
                 unpack8<DT>(wk[m], k8v[m]);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) k8v[m][e] = mul2(k8v[m][e], both(rk));
             }
-            const int k8 = tid & 15, r0 = tid >> 4;        // rows r0 (block 0 or 1) and 32 + r0 (block 2 or 3)
+            const int k8 = tid & 15;
             f32x2 ga[2][4];
             lds_halves(scr.ga[3], k8, ga[1]);
 #pragma unroll
@@ -474,7 +477,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                 if (I) lds_halves(scr.ga[I - 1], k8, ga[(I - 1) & 1]);      // one block ahead
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
-                    const int r = r0 + 32 * m;
+                    const int r = staged_row(m);
                     if (r >= 16 * (I + 1)) continue;       // warp-uniform
                     f32x2 t8[4];
                     scale_ex2(t8, k8v[m], ga[I & 1], vg[m]);
