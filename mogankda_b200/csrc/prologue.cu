@@ -240,15 +240,18 @@ __global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd 
 // ---------------------------------------------------------------------------------------------------------
 // deterministic second-stage reductions
 // ---------------------------------------------------------------------------------------------------------
-// Up to three jobs in one launch (the parameter gradients of a layer): block = 32 outputs of a job x 32 row lanes.  A lane adds every 32nd
-// term of its output, eight loads in flight; the 32 lanes' sums are then combined by a fixed shuffle tree.  (One launch per job with 8 row
-// lanes, and one block per output for the grouped job, took 43 + 43 us on 64k tokens x 32 heads; this takes 22.)
+// Up to three jobs in one launch (the parameter gradients of a layer): block = 8 outputs of a job x 128 row lanes.  A lane adds every 128th
+// term of its output, eight loads in flight; the 128 lanes' sums are then combined by a fixed shuffle tree.  What takes the time is the
+// latency of a lane's rounds of loads: the widest job has 128 outputs of 1184 terms, which 32 outputs x 32 lanes gave to four SMs in five
+// rounds (21 us).
+constexpr int RED_OUTS = 8, RED_LANES = 128;
+__host__ __device__ inline int reduce_blocks(const MkdaReduce& j) { return (j.cols / j.group + RED_OUTS - 1) / RED_OUTS; }
 __global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
-    __shared__ float part[32][33];
+    __shared__ float part[RED_OUTS][RED_LANES + 4];
     int blk = blockIdx.x, job = 0;
-    while (job < 2 && blk >= (p.job[job].cols / p.job[job].group + 31) / 32) { blk -= (p.job[job].cols / p.job[job].group + 31) / 32; ++job; }
+    while (job < 2 && blk >= reduce_blocks(p.job[job])) { blk -= reduce_blocks(p.job[job]); ++job; }
     const MkdaReduce q = p.job[job];
-    const int j = blk * 32 + threadIdx.x, outs = q.cols / q.group, terms = q.rows * q.group;
+    const int o = threadIdx.x & (RED_OUTS - 1), l = threadIdx.x / RED_OUTS, j = blk * RED_OUTS + o, outs = q.cols / q.group, terms = q.rows * q.group;
     float s = 0.f;
     if (j < outs) {
         const float* in = q.in + (size_t)j * q.group;
@@ -256,18 +259,19 @@ __global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
         float a[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) a[e] = 0.f;
-        int t = threadIdx.y;
-        for (; t + 7 * 32 < terms; t += 8 * 32) {
+        for (int t = l; t < terms; t += 8 * RED_LANES) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) a[e] += at(t + e * 32);
+            for (int e = 0; e < 8; ++e)
+                if (t + e * RED_LANES < terms) a[e] += at(t + e * RED_LANES);
         }
-        for (; t < terms; t += 32) a[0] += at(t);
         s = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     }
-    part[threadIdx.y][threadIdx.x] = s;
+    part[o][l] = s;
     __syncthreads();
-    s = warp_sum(part[threadIdx.x][threadIdx.y]);          // warp y: the 32 partial sums of output y
-    if (threadIdx.x == 0 && blk * 32 + (int)threadIdx.y < outs) q.out[blk * 32 + threadIdx.y] = s;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w >= RED_OUTS || blk * RED_OUTS + w >= outs) return;
+    s = warp_sum((part[w][lane] + part[w][lane + 32]) + (part[w][lane + 64] + part[w][lane + 96]));
+    if (lane == 0) q.out[blk * RED_OUTS + w] = s;
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -619,10 +623,10 @@ extern "C" int mkda_reduce_multi(const MkdaReduceMulti* p, void* stream) {
     for (MkdaReduce& j : q.job) {
         if (!j.out || j.cols == 0) { j = MkdaReduce{nullptr, 0, 0, 1, nullptr}; continue; }
         if (!j.in || j.group < 1 || j.cols % j.group) return set_error(MKDA_ERR_ARG, "reduce_multi: bad argument");
-        blocks += (j.cols / j.group + 31) / 32;
+        blocks += reduce_blocks(j);
     }
     if (blocks == 0) return MKDA_OK;
-    reduce_kernel<<<blocks, dim3(32, 32), 0, (cudaStream_t)stream>>>(q);
+    reduce_kernel<<<blocks, RED_OUTS * RED_LANES, 0, (cudaStream_t)stream>>>(q);
     return check_launch("reduce_multi");
 }
 
