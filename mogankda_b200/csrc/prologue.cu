@@ -29,6 +29,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ---------------------------------------------------------------------------------------------------------
 template <int XDT>
 __global__ void __launch_bounds__(128, 5) gate_cumsum_fwd_kernel(const MkdaGateFwd p) {
+    follow_stream();
     const int HV = p.L.HV, c = blockIdx.x / HV, h = blockIdx.x - c * HV;
     const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(128, 5) gate_cumsum_fwd_kernel(const MkdaGateF
 // One decay per token: grid (NC, blocks of 32 heads), lane = head, warp w owns rows 8w..8w+7.  The inclusive sum has the same form as
 // above (earlier warps' totals in order, plus the running sum inside the warp).  g_c is [TT,HV].
 __global__ void __launch_bounds__(256) gate_cumsum_fwd_scalar_kernel(const MkdaGateFwd p) {
+    follow_stream();
     const int HV = p.L.HV, c = blockIdx.x, h = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int start = p.L.chunk_start[c], len = p.L.chunk_len[c], hh = h < HV ? h : HV - 1;
     __shared__ float tot[8][32];
@@ -123,6 +125,7 @@ __global__ void __launch_bounds__(256) gate_cumsum_fwd_scalar_kernel(const MkdaG
 constexpr int GB_WARPS = 16, GB_ROWS = CH / GB_WARPS;
 template <int XDT>
 __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGateBwd p) {
+    follow_stream();
     const int h = blockIdx.x, HV = p.L.HV;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ float4 tot[GB_WARPS][32];
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
 // One decay per token: dgp is [NC,HV,64], summed over the channels where it was written.  CTA (block of 32 heads, g) walks the chunks g,
 // g + gridDim.y, ...; lane = head, warp w owns rows 8w..8w+7; the [32 heads][64] block of dgp passes through shared memory.
 __global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd p) {
+    follow_stream();
     const int HV = p.L.HV, h0 = blockIdx.x * 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + lane, hh = h < HV ? h : HV - 1;
     __shared__ float tile[32][CH + 1], tot[8][32], red[2][8][32];
     const float E = p.A_log ? expf(p.A_log[hh]) : 1.f, bias = p.dt_bias ? p.dt_bias[hh] : 0.f;
@@ -247,6 +251,7 @@ __global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd 
 constexpr int RED_OUTS = 8, RED_LANES = 128;
 __host__ __device__ inline int reduce_blocks(const MkdaReduce& j) { return (j.cols / j.group + RED_OUTS - 1) / RED_OUTS; }
 __global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
+    follow_stream();
     __shared__ float part[RED_OUTS][RED_LANES + 4];
     int blk = blockIdx.x, job = 0;
     while (job < 2 && blk >= reduce_blocks(p.job[job])) { blk -= reduce_blocks(p.job[job]); ++job; }
@@ -279,6 +284,7 @@ __global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
 // ---------------------------------------------------------------------------------------------------------
 template <int DT>
 __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
+    follow_stream();
     const int lane = threadIdx.x & 31, sub = lane & 15;
     const int row0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + (lane >> 4);
     const void* x = blockIdx.y ? p.x2 : p.x;
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
 // q/k head (the chunk backward adds them up where it writes them).
 template <bool SPLIT>
 __global__ void __launch_bounds__(128) qk_grad_finish_kernel(const MkdaQkGrad p) {
+    follow_stream();
     const int HK = p.L.HK;
     const int c = blockIdx.x / HK, hk = blockIdx.x - c * HK, which = blockIdx.y;
     const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
@@ -357,6 +364,7 @@ __global__ void __launch_bounds__(128) qk_grad_finish_kernel(const MkdaQkGrad p)
 //   dz = dy n w a'(z);  dw = sum dy n a
 // ---------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) epilogue_bwd_kernel(const MkdaEpilogueBwd p) {
+    follow_stream();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ float4 red[4][32];
     float4 w = splat4(1.f);
@@ -414,6 +422,7 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 // DYMODE: how dy is addressed: 0 = dense rows (16-byte loads), 1 = one value per row (column stride 0), 2 = any strides
 template <int DYMODE>
 __global__ void __launch_bounds__(128) epilogue_bwd_tiles_kernel(const MkdaEpilogueBwdTiles p) {
+    follow_stream();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 15, hw = lane >> 4;
     __shared__ float red[8][128];
     const int HV = p.L.HV, total = p.L.NC * HV;
@@ -500,6 +509,7 @@ __global__ void __launch_bounds__(128) epilogue_bwd_tiles_kernel(const MkdaEpilo
 // Rows [TT,HV,128] -> row tiles [64 tokens][128] (bf16 hi / lo, rows past the end zero), one CTA per (chunk, v-head), heads fastest.
 template <int DT>
 __global__ void __launch_bounds__(256) rows_to_tiles_kernel(const MkdaLayout L, const void* rows, uint8_t* tiles) {
+    follow_stream();
     const int HV = L.HV, c = blockIdx.x / HV, h = blockIdx.x - c * HV, start = L.chunk_start[c], len = L.chunk_len[c];
     uint8_t* tile = tiles + (size_t)blockIdx.x * 32768;
     const int k8 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
@@ -523,6 +533,7 @@ __global__ void __launch_bounds__(256) rows_to_tiles_kernel(const MkdaLayout L, 
 // Warm-up truncation table: one CTA per (segment, v-head), one thread per key channel (see MkdaWarmup).
 // gl = 2^gL may have underflowed to zero: log2 gives -inf, i.e. fully decayed.
 __global__ void __launch_bounds__(128) warmup_chunks_kernel(const MkdaWarmup p) {
+    follow_stream();
     const int seg = blockIdx.x, h = blockIdx.y, ch = threadIdx.x, HV = p.L.HV;
     const int c_beg = p.L.seg_chunk_off[seg], c_end = p.L.seg_chunk_off[seg + 1];
     int ws = c_beg, we = c_end;
@@ -547,9 +558,9 @@ int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void*
     if (grid == 0) return MKDA_OK;
     uint8_t* t = static_cast<uint8_t*>(tiles);
     switch (dtype) {
-        case MKDA_F32: rows_to_tiles_kernel<MKDA_F32><<<grid, 256, 0, stream>>>(L, rows, t); break;
-        case MKDA_BF16: rows_to_tiles_kernel<MKDA_BF16><<<grid, 256, 0, stream>>>(L, rows, t); break;
-        case MKDA_F16: rows_to_tiles_kernel<MKDA_F16><<<grid, 256, 0, stream>>>(L, rows, t); break;
+        case MKDA_F32: launch(rows_to_tiles_kernel<MKDA_F32>, grid, 256, 0, stream, L, rows, t); break;
+        case MKDA_BF16: launch(rows_to_tiles_kernel<MKDA_BF16>, grid, 256, 0, stream, L, rows, t); break;
+        case MKDA_F16: launch(rows_to_tiles_kernel<MKDA_F16>, grid, 256, 0, stream, L, rows, t); break;
         default: return set_error(MKDA_ERR_ARG, "bwd_dh: unsupported dtype");
     }
     return check_launch("rows_to_tiles");
@@ -569,7 +580,7 @@ extern "C" int mkda_warmup_chunks(const MkdaWarmup* p, void* stream) {
     if (!p || !p->gl || !p->warm_start || !p->warm_end || !p->L.seg_chunk_off) return set_error(MKDA_ERR_ARG, "warmup_chunks: null argument");
     if (!(p->threshold_log2 < 0.f)) return set_error(MKDA_ERR_ARG, "warmup_chunks: the threshold must be negative");
     if (p->L.NS == 0 || p->L.HV == 0) return MKDA_OK;
-    warmup_chunks_kernel<<<dim3(p->L.NS, p->L.HV), 128, 0, (cudaStream_t)stream>>>(*p);
+    launch(warmup_chunks_kernel, dim3(p->L.NS, p->L.HV), 128, 0, (cudaStream_t)stream, *p);
     return check_launch("warmup_chunks");
 }
 
@@ -581,14 +592,14 @@ extern "C" int mkda_gate_cumsum_fwd(const MkdaGateFwd* p, void* stream) {
     if (p->L.NC == 0) return MKDA_OK;
     if (p->x_dtype < MKDA_F32 || p->x_dtype > MKDA_F16) return set_error(MKDA_ERR_ARG, "gate_cumsum_fwd: unsupported dtype");
     if (p->scalar_gate) {
-        gate_cumsum_fwd_scalar_kernel<<<dim3(p->L.NC, (p->L.HV + 31) / 32), 256, 0, (cudaStream_t)stream>>>(*p);
+        launch(gate_cumsum_fwd_scalar_kernel, dim3(p->L.NC, (p->L.HV + 31) / 32), 256, 0, (cudaStream_t)stream, *p);
         return check_launch("gate_cumsum_fwd");
     }
     const int grid = p->L.NC * p->L.HV;
     switch (p->x_dtype) {
-        case MKDA_F32: gate_cumsum_fwd_kernel<MKDA_F32><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_BF16: gate_cumsum_fwd_kernel<MKDA_BF16><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_F16: gate_cumsum_fwd_kernel<MKDA_F16><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
+        case MKDA_F32: launch(gate_cumsum_fwd_kernel<MKDA_F32>, grid, 128, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_BF16: launch(gate_cumsum_fwd_kernel<MKDA_BF16>, grid, 128, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_F16: launch(gate_cumsum_fwd_kernel<MKDA_F16>, grid, 128, 0, (cudaStream_t)stream, *p); break;
         default: return set_error(MKDA_ERR_ARG, "gate_cumsum_fwd: unsupported dtype");
     }
     return check_launch("gate_cumsum_fwd");
@@ -604,13 +615,13 @@ extern "C" int mkda_gate_bwd(const MkdaGateBwd* p, void* stream) {
         return set_error(MKDA_ERR_ARG, "gate_bwd: part_rows must not exceed the number of chunks when partials are requested");
     if (p->x_dtype < MKDA_F32 || p->x_dtype > MKDA_F16) return set_error(MKDA_ERR_ARG, "gate_bwd: unsupported dtype");
     if (p->scalar_gate) {
-        gate_bwd_scalar_kernel<<<dim3((p->L.HV + 31) / 32, grid.y), 256, 0, (cudaStream_t)stream>>>(*p);
+        launch(gate_bwd_scalar_kernel, dim3((p->L.HV + 31) / 32, grid.y), 256, 0, (cudaStream_t)stream, *p);
         return check_launch("gate_bwd");
     }
     switch (p->x_dtype) {
-        case MKDA_F32: gate_bwd_kernel<MKDA_F32><<<grid, 32 * GB_WARPS, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_BF16: gate_bwd_kernel<MKDA_BF16><<<grid, 32 * GB_WARPS, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_F16: gate_bwd_kernel<MKDA_F16><<<grid, 32 * GB_WARPS, 0, (cudaStream_t)stream>>>(*p); break;
+        case MKDA_F32: launch(gate_bwd_kernel<MKDA_F32>, grid, 32 * GB_WARPS, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_BF16: launch(gate_bwd_kernel<MKDA_BF16>, grid, 32 * GB_WARPS, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_F16: launch(gate_bwd_kernel<MKDA_F16>, grid, 32 * GB_WARPS, 0, (cudaStream_t)stream, *p); break;
         default: return set_error(MKDA_ERR_ARG, "gate_bwd: unsupported dtype");
     }
     return check_launch("gate_bwd");
@@ -626,7 +637,7 @@ extern "C" int mkda_reduce_multi(const MkdaReduceMulti* p, void* stream) {
         blocks += reduce_blocks(j);
     }
     if (blocks == 0) return MKDA_OK;
-    reduce_kernel<<<blocks, RED_OUTS * RED_LANES, 0, (cudaStream_t)stream>>>(q);
+    launch(reduce_kernel, blocks, RED_OUTS * RED_LANES, 0, (cudaStream_t)stream, q);
     return check_launch("reduce_multi");
 }
 
@@ -644,9 +655,9 @@ extern "C" int mkda_l2norm_rstd(const MkdaL2Norm* p, void* stream) {
     if (p->rows == 0) return MKDA_OK;
     const dim3 grid((p->rows + 31) / 32, p->x2 ? 2 : 1);
     switch (p->dtype) {
-        case MKDA_F32: l2norm_rstd_kernel<MKDA_F32><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_BF16: l2norm_rstd_kernel<MKDA_BF16><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
-        case MKDA_F16: l2norm_rstd_kernel<MKDA_F16><<<grid, 128, 0, (cudaStream_t)stream>>>(*p); break;
+        case MKDA_F32: launch(l2norm_rstd_kernel<MKDA_F32>, grid, 128, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_BF16: launch(l2norm_rstd_kernel<MKDA_BF16>, grid, 128, 0, (cudaStream_t)stream, *p); break;
+        case MKDA_F16: launch(l2norm_rstd_kernel<MKDA_F16>, grid, 128, 0, (cudaStream_t)stream, *p); break;
         default: return set_error(MKDA_ERR_ARG, "l2norm_rstd: unsupported dtype");
     }
     return check_launch("l2norm_rstd");
@@ -658,8 +669,8 @@ extern "C" int mkda_qk_grad_finish(const MkdaQkGrad* p, void* stream) {
     if (any_misaligned(p->dq_v, p->dk_v, p->dq, p->dk, p->q, p->k)) return set_error(MKDA_ERR_ARG, "qk_grad_finish: tensors must be 16-byte aligned");
     if (p->L.NC == 0) return MKDA_OK;
     const dim3 grid(p->L.NC * p->L.HK, 2);
-    if (p->per_v_head) qk_grad_finish_kernel<true><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
-    else qk_grad_finish_kernel<false><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
+    if (p->per_v_head) launch(qk_grad_finish_kernel<true>, grid, 128, 0, (cudaStream_t)stream, *p);
+    else launch(qk_grad_finish_kernel<false>, grid, 128, 0, (cudaStream_t)stream, *p);
     return check_launch("qk_grad_finish");
 }
 
@@ -713,7 +724,7 @@ extern "C" int mkda_epilogue_bwd_noalloc(const MkdaEpilogueBwdNoAlloc* p, void* 
     q.norm_w_dtype = p->norm_w_dtype; q.gate = p->gate; q.gate_dtype = p->gate_dtype; q.act = p->act; q.eps = p->eps;
     q.d_o = p->d_o; q.dgate = p->dgate; q.dgate_dtype = p->dgate_dtype;
     q.part_w = scratch;                 // every block overwrites its whole row: nothing has to be cleared first
-    epilogue_bwd_kernel<<<nblk, 128, 0, (cudaStream_t)stream>>>(q);
+    launch(epilogue_bwd_kernel, nblk, 128, 0, (cudaStream_t)stream, q);
     if (int e = check_launch("epilogue_bwd_noalloc")) return e;
     const MkdaReduce r{scratch, nblk, 128, 1, p->dweight};
     return mkda_reduce_partials(&r, stream);
@@ -729,15 +740,15 @@ extern "C" int mkda_epilogue_bwd_tiles(const MkdaEpilogueBwdTiles* p, void* stre
     if (items == 0) return MKDA_OK;
     const int grid = items < MKDA_EPILOGUE_MAX_PART_ROWS ? items : MKDA_EPILOGUE_MAX_PART_ROWS;
     if (p->part_w && p->part_rows != grid) return set_error(MKDA_ERR_ARG, "epilogue_bwd_tiles: part_rows must be min(NC * HV, MKDA_EPILOGUE_MAX_PART_ROWS)");
-    if (p->dy_col_stride == 1) epilogue_bwd_tiles_kernel<0><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
-    else if (p->dy_col_stride == 0) epilogue_bwd_tiles_kernel<1><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
-    else epilogue_bwd_tiles_kernel<2><<<grid, 128, 0, (cudaStream_t)stream>>>(*p);
+    if (p->dy_col_stride == 1) launch(epilogue_bwd_tiles_kernel<0>, grid, 128, 0, (cudaStream_t)stream, *p);
+    else if (p->dy_col_stride == 0) launch(epilogue_bwd_tiles_kernel<1>, grid, 128, 0, (cudaStream_t)stream, *p);
+    else launch(epilogue_bwd_tiles_kernel<2>, grid, 128, 0, (cudaStream_t)stream, *p);
     return check_launch("epilogue_bwd_tiles");
 }
 
 extern "C" int mkda_epilogue_bwd(const MkdaEpilogueBwd* p, void* stream) {
     if (!p || !p->dy || !p->o_raw || !p->gate || !p->d_o || !p->dgate) return set_error(MKDA_ERR_ARG, "epilogue_bwd: null argument");
     if (p->rows == 0) return MKDA_OK;
-    epilogue_bwd_kernel<<<epilogue_part_rows(p->rows), 128, 0, (cudaStream_t)stream>>>(*p);
+    launch(epilogue_bwd_kernel, epilogue_part_rows(p->rows), 128, 0, (cudaStream_t)stream, *p);
     return check_launch("epilogue_bwd");
 }

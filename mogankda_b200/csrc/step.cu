@@ -24,6 +24,7 @@ __device__ __forceinline__ float warp_sum_f(float x) {
 }
 
 __global__ void __launch_bounds__(256, 2) step_fwd_kernel(const MkdaStepFwd p) {
+    follow_stream();
     __shared__ __align__(16) StepShared sh;
     const int h = blockIdx.x, n = blockIdx.y, HV = p.L.HV, HK = p.L.HK, hk = h / (HV / HK);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -150,6 +151,6 @@ extern "C" int mkda_step_fwd(const MkdaStepFwd* p, void* stream) {
         if (dt < MKDA_F32 || dt > MKDA_F16) return set_error(MKDA_ERR_ARG, "step_fwd: unsupported dtype");
     if (p->N == 0 || p->L.HV == 0) return MKDA_OK;
     if (p->N > 65535) return set_error(MKDA_ERR_ARG, "step_fwd: too many sequences");
-    step_fwd_kernel<<<dim3(p->L.HV, p->N), 256, 0, (cudaStream_t)stream>>>(*p);
+    launch(step_fwd_kernel, dim3(p->L.HV, p->N), 256, 0, (cudaStream_t)stream, *p);
     return check_launch("step_fwd");
 }

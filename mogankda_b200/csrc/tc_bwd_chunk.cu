@@ -655,6 +655,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
     Shared& sh = *reinterpret_cast<Shared*>(base + TILES);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        follow_stream();
         if (threadIdx.x == 0) atomicExch(&umma::g_timeout_flag, 1u);
         return;
     }
@@ -665,6 +666,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
         umma::fence_barrier_init();
     }
     publish();
+    follow_stream();
     if (warp >= COMPUTE / 32) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == WARP_MMA) {
@@ -690,7 +692,7 @@ static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, cudaStream_t stream) {
     static const int regs = kernel_registers((const void*)kern);
     if (regs < bc::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "bwd_chunk: built with fewer registers than its warps redistribute");
     const int groups = p->L.NC * (SPREAD ? p->L.HV : p->L.HK);              // a CTA takes whole (chunk, q/k head) groups
-    kern<<<groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream>>>(*p);
+    launch(kern, groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream, *p);
     return check_launch("bwd_chunk");
 }
 template <int DT, bool SCALAR>

@@ -78,11 +78,12 @@ __global__ void __launch_bounds__(512, 1) out_fwd_tc_kernel(const MkdaOutFwd p) 
     if (tid == 0) {
         umma::mbar_init(&ldbar, 1);
         umma::fence_barrier_init();
-        if ((int)blockIdx.x < total) request(blockIdx.x);
     }
+    const uint32_t tmem = tc_operands_ready(&sh);
+    follow_stream();
+    if (tid == 0 && (int)blockIdx.x < total) request(blockIdx.x);
     float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
     if (p.has_norm && p.norm_w) w = ld4(p.norm_w, p.norm_w_dtype, 4 * lane);
-    const uint32_t tmem = tc_operands_ready(&sh);
 
     int k = 0;
     for (int item = blockIdx.x; item < total; item += stride, ++k) {
@@ -149,7 +150,7 @@ static int launch_out_fwd_tc_t(const MkdaOutFwd* p, cudaStream_t stream) {
     auto kern = out_fwd_tc_kernel<GDT>;
     if (int e = ensure_smem((const void*)kern, OUT_TC_SMEM, "out_fwd")) return e;
     const int items = p->L.NC * p->L.HV;
-    kern<<<items < sm_count() ? items : sm_count(), 512, OUT_TC_SMEM, stream>>>(*p);
+    launch(kern, items < sm_count() ? items : sm_count(), 512, OUT_TC_SMEM, stream, *p);
     return check_launch("out_fwd");
 }
 int launch_out_fwd_tc(const MkdaOutFwd* p, cudaStream_t stream) {

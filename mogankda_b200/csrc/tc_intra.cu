@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
+    follow_stream();
     cur.c = blockIdx.x / HV; cur.h = blockIdx.x - cur.c * HV; cur.hk = cur.h / G;
     table(cur);
     if ((int)blockIdx.x < total) load_inputs(cur, 0);
@@ -500,7 +501,7 @@ static int launch_intra_fwd_tc_tt(const MkdaIntraFwd* p, const IntraMaps& maps, 
     auto kern = intra_fwd_tc_kernel<DT, SCALAR, TMA>;
     if (int e = ensure_smem((const void*)kern, INTRA_TC_SMEM, "intra_fwd")) return e;
     const int items = p->L.NC * p->L.HV;
-    kern<<<items < sm_count() ? items : sm_count(), 512, INTRA_TC_SMEM, stream>>>(*p, maps);
+    launch(kern, items < sm_count() ? items : sm_count(), 512, INTRA_TC_SMEM, stream, *p, maps);
     return check_launch("intra_fwd");
 }
 template <int DT, bool SCALAR>

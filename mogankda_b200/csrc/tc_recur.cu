@@ -232,6 +232,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     const int h = blockIdx.y, seg = blockIdx.z, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        follow_stream();
         if (tid == 0) atomicExch(&umma::g_timeout_flag, 1u);
         return;
     }
@@ -249,6 +250,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
+    follow_stream();
 
     // Warm-up truncation (a pass from zero only): where the decay accumulated from chunk warm_start to the segment's end
     // hides everything before it, the pass starts there; the transition is then zero and its CTA visits no chunk.
@@ -457,7 +459,7 @@ int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream) {
     using L = RecurLayout<false>;
     auto kern = recur_fwd_tc_kernel;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "recur_fwd")) return e;
-    kern<<<dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream>>>(*p);
+    launch(kern, dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream, *p);
     return check_launch("recur_fwd");
 }
 
@@ -476,7 +478,7 @@ static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, cudaStream_t stream) {
     if (!e && p->o.o_raw) e = make_rows_map(&maps.raw, p->o.o_raw, 4, rows, cols, "chain_fwd", 16);
     if (!e) e = make_rows_map(&maps.out, p->o.out, p->o.out_dtype == MKDA_F32 ? 4 : 2, rows, cols, "chain_fwd", 16);
     if (e) return e;
-    kern<<<dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream>>>(*p, maps);
+    launch(kern, dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream, *p, maps);
     return check_launch("chain_fwd");
 }
 int launch_chain_fwd_tc(const MkdaChainFwd* p, cudaStream_t stream) {
@@ -512,6 +514,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     const int h = blockIdx.y, seg = blockIdx.z, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        follow_stream();
         if (tid == 0) atomicExch(&umma::g_timeout_flag, 1u);
         return;
     }
@@ -525,6 +528,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
+    follow_stream();
 
     // Warm-up truncation (a pass from zero only): the reverse chain starts below chunk warm_end where the decay accumulated
     // over the segment's first chunks hides every later contribution from the segment's entrance.
@@ -638,7 +642,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
 int launch_bwd_dh_tc(const MkdaBwdDh* p, cudaStream_t stream) {
     auto kern = bwd_dh_tc_kernel;
     if (int e = ensure_smem((const void*)kern, DH_SMEM, "bwd_dh")) return e;
-    kern<<<dim3(1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream>>>(*p);
+    launch(kern, dim3(1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream, *p);
     return check_launch("bwd_dh");
 }
 
