@@ -21,7 +21,7 @@ namespace mkda {
 struct IntraShared {
     uint64_t bar, bar2, ldin;
     uint32_t tmem;
-    float beta[2][CH];                                     // of this item and (arriving) the next
+    __align__(16) float beta[2][CH];                       // of this item and (arriving) the next
     float rk[CH], rq[CH];                                  // L2 scales of the rows
     __align__(16) float T[32][36];
 };
@@ -36,16 +36,17 @@ constexpr int KQ_OFF = 81920;                              // [128][128] hi 32 K
 constexpr int OPND_BYTES = KQ_OFF + 65536;                 // 144 KB
 // The 16-bit k, q and the g rows of the NEXT item arrive by tiled copy (one 64 x 128 box per tensor) while the current item's
 // inverse and second products run: k and g rows in the upper 48 KB of the [Kr; Qr] tile, dead once the first products are
-// done, q rows behind sP.  They are read back into registers before the next item's operands are staged over them.  (Loads
+// done, q rows over the kbar tile as soon as that has left.  They are read back into registers before the next item's operands are staged over them.  (Loads
 // into registers at that point are accepted only as fast as their data returns and occupied every thread for a fifth of
 // the item; one small bulk copy per row is slower still.)
 struct IntraMaps { CUtensorMap k, q, g; };
 constexpr int RAW_K = 98304;                               // [64][128] 16-bit, 16 KB
 constexpr int RAW_G = RAW_K + 16384;                       // [64][128] fp32, 32 KB
-constexpr int RAW_Q = OPND_BYTES + 53248;                  // [64][128] 16-bit, 16 KB
-constexpr int INTRA_TC_SMEM = RAW_Q + 16384 + 1024;        // operands + (two 32 KB hand-over tiles, later sM / sInv / sP) + q rows
+constexpr int RAW_Q = OPND_BYTES;                          // [64][128] 16-bit, 16 KB, over the kbar tile
+constexpr int INTRA_TC_SMEM = OPND_BYTES + 32768 + 2 * CH * MLD * 4 + 1024;        // operands, kbar tile, scale q 2^g tile (later sM / sInv)
 static_assert(RAW_G + 32768 <= OPND_BYTES, "k / g rows must fit in the dead part of the operand region");
-static_assert(3 * CH * MLD * 4 <= 53248, "sM / sInv / sP must end below the q rows");
+static_assert(2 * CH * MLD * 4 >= 32768, "the scale q 2^g tile must fit below the end");
+constexpr int STORER = 256;                                // the thread that issues every bulk store: its warp has no part in the inverse
 
 // Inverse of the unit lower-triangular 64 x 64 matrix sM into sInv (fixed summation order) by recursive halving:
 // the four 16 x 16 diagonal blocks by forward substitution, then the off-diagonal block of each 32 x 32 half and finally
@@ -125,19 +126,18 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     __shared__ IntraShared sh;
     // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
     // 16 threads of a row read them without bank conflicts
-    __shared__ __align__(16) float sGa[5][DK];
-    __shared__ float sGsb[2][CH];                      // SCALAR: the cumsum of every row (rows past the end: the last valid one)
+    __shared__ __align__(16) float sGa[5][DK], sStep[2][DK];      // anchor rows; 2^(ga[I] - ga[I - 1]) of I = 2, 3
+    __shared__ __align__(16) float sGsb[2][CH];                      // SCALAR: the cumsum of every row (rows past the end: the last valid one)
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sKQ = base + KQ_OFF;
-    float* sM = reinterpret_cast<float*>(base + OPND_BYTES);
+    float* sM = reinterpret_cast<float*>(base + OPND_BYTES + 32768);
     float* sInv = sM + CH * MLD;
-    float* sP = sInv + CH * MLD;
     uint8_t* sBk = base;                               // phase 3: beta k~ [j][K index], hi 16 KB + lo 16 KB
     uint8_t* sBv = base + 32768;                       // beta v [j][v]
     uint8_t* sTA = base + 65536;                       // A [i][j], hi 8 KB + lo 8 KB
     uint8_t* sTQ = base + 81920;                       // Aqk [i][j], hi 8 KB + lo 8 KB (only copied out)
-    uint8_t* sKB = base + OPND_BYTES;                  // kbar [tok][K index] hi + lo (32 KB), only copied out; under sM ...
-    uint8_t* sQS = sKB + 32768;                        // scale q 2^g [tok][K index] hi + lo (32 KB), likewise
+    uint8_t* sKB = base + OPND_BYTES;                  // kbar [tok][K index] hi + lo (32 KB), only copied out; later the q rows of the next item
+    uint8_t* sQS = sKB + 32768;                        // scale q 2^g [tok][K index] hi + lo (32 KB), likewise; under sM and sInv
 
     const int HV = p.L.HV, HK = p.L.HK, total = p.L.NC * HV, stride = gridDim.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -162,7 +162,6 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         if (BULK && tid == 128) {                      // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
             umma::mbar_expect_tx(&sh.ldin, 16384u + 16384u + (SCALAR ? 0u : 32768u));
             umma::tma_load_rows(base + RAW_K, &maps.k, i.hk * 128, i.start, &sh.ldin);
-            umma::tma_load_rows(base + RAW_Q, &maps.q, i.hk * 128, i.start, &sh.ldin);
             if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, i.h * 128, i.start, &sh.ldin);
         }
         if (!BULK) {
@@ -176,6 +175,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             }
         }
     };
+    auto load_q = [&](const Item& i) { umma::tma_load_rows(base + RAW_Q, &maps.q, i.hk * 128, i.start, &sh.ldin); };
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 256);
     if (tid == 0) { umma::mbar_init(&sh.bar, 1); umma::mbar_init(&sh.bar2, 1); umma::mbar_init(&sh.ldin, 1); umma::fence_barrier_init(); }
     umma::fence_before_sync();
@@ -185,7 +185,10 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     follow_stream();
     cur.c = blockIdx.x / HV; cur.h = blockIdx.x - cur.c * HV; cur.hk = cur.h / G;
     table(cur);
-    if ((int)blockIdx.x < total) load_inputs(cur, 0);
+    if ((int)blockIdx.x < total) {
+        load_inputs(cur, 0);
+        if (BULK && tid == STORER) load_q(cur);
+    }
     nxt = cur;
     advance(nxt);
 
@@ -212,6 +215,15 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
         if (!SCALAR && (r & 15) == 0) sts_halves(sGa[r >> 4], k8, vg[n]);
         if (!SCALAR && r == len - 1) sts_halves(sGa[4], k8, vg[n]);
+        if (!SCALAR && (r & 15) == 0 && r >= 32) {
+            const int rp = r - 16 < len ? r - 16 : len - 1;
+            f32x2 prev[4];
+            if (BULK) lds8(reinterpret_cast<const float*>(base + RAW_G + rp * 512 + k8 * 32), prev);
+            else lds8(p.g_c + ((size_t)(start + rp) * HV + h) * 128 + k8 * 8, prev);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) prev[e] = ex2f2_(sub2(vg[n][e], prev[e]));
+            sts_halves(sStep[(r >> 4) - 2], k8, prev);
+        }
         if (r >= len) {                                    // rows past the end are zero
             wk[n].a = wq[n].a = make_uint4(0, 0, 0, 0);
             if (DT == MKDA_F32) wk[n].b = wq[n].b = make_uint4(0, 0, 0, 0);
@@ -219,7 +231,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         unpack8<DT>(wk[n], vk[n]);
         unpack8<DT>(wq[n], vq[n]);
     }
-    if (tid == 0) umma::bulk_store_wait_read();        // the previous item's tiles have left shared memory
+    if (tid == STORER) umma::bulk_store_wait_read();   // the previous item's tiles have left shared memory
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -246,8 +258,14 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
 #pragma unroll
             for (int I = 0; I < 4; ++I) {
                 if (I < I0) continue;
-                if (I > I0) lds_halves(sGa[I], k8, ga);
-                scale_ex2(t8, vk[n], ga, vg[n]);
+                if (I <= I0 + 1) {
+                    if (I > I0) lds_halves(sGa[I], k8, ga);
+                    scale_ex2(t8, vk[n], ga, vg[n]);
+                } else {                                   // a step of decay (<= 1) further down the anchors: exponentials are what bounds this phase
+                    lds_halves(sStep[I - 2], k8, ga);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], ga[e]);
+                }
                 store_split8(base, base + KC_ALL_BYTES, KC_ALL_ROWS, kc_row(I) + r, k8, t8);      // the four column tiles stacked by rows
             }
         }
@@ -355,10 +373,10 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     }
     umma::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (tid == STORER) {                               // qs first: its place is needed first
         const size_t it = (size_t)c * HV + h;
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + it * umma::CHUNK_TILE_BYTES, sKB, umma::CHUNK_TILE_BYTES);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + it * umma::CHUNK_TILE_BYTES, sQS, umma::CHUNK_TILE_BYTES);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + it * umma::CHUNK_TILE_BYTES, sKB, umma::CHUNK_TILE_BYTES);
     }
     umma::mbar_wait(&sh.bar, 0);
     umma::fence_after_sync();
@@ -377,29 +395,41 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], b2);
         store_split8(sBv, sBv + 16384, 64, r, k8, t8);
     }
-    if (tid == 0) umma::bulk_store_wait_read();    // the two tiles under sM / sInv / sP (and the q rows) have left shared memory
+    if (tid == STORER) umma::bulk_store_wait_read_but<1>();        // the tile under sM / sInv has left shared memory
     __syncthreads();
     if (item + stride < total) load_inputs(nxt, (it & 1) ^ 1);     // k, q, g, beta of the next item start travelling
     sInv[(32 * (tid >> 8) + ((tid >> 4) & 15)) * MLD + 32 * (tid >> 8) + 16 + (tid & 15)] = 0.f;       // blocks (0, 1) and (2, 3)
+    auto store_row16 = [](float* dst, const float (&o)[16]) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+    };
+    auto store_aqk = [&](int i, const float (&o)[16]) {        // Aqk leaves as a ready-made [row][column] operand tile (rows past the end: zeros)
+        float lo[8], hi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { lo[j] = o[j]; hi[j] = o[8 + j]; }
+        store_split8(sTQ, sTQ + 8192, 64, i, 2 * cg, lo);
+        store_split8(sTQ, sTQ + 8192, 64, i, 2 * cg + 1, hi);
+    };
     if (SCALAR) {                             // lane = row (K rows, then Q rows), cg = 16 columns j: decay applied here, for i >= j only
         float v[16];
         umma::tmem_ld16(umma::tmem_addr(tmem, warp, 16 * cg), v);
         const int i = row & 63;
         const float gi = sGs[i], bi = q < 2 ? sBeta[i] * sh.rk[i] : p.scale * sh.rq[i];
-        float* dst = (q < 2 ? sM : sP) + i * MLD + 16 * cg;
+        float o[16];
 #pragma unroll
         for (int j4 = 0; j4 < 16; j4 += 4) {
-            float o4[4];
+            const float4 g4 = *reinterpret_cast<const float4*>(sGs + 16 * cg + j4), r4 = *reinterpret_cast<const float4*>(sh.rk + 16 * cg + j4);
+            const float gj[4] = {g4.x, g4.y, g4.z, g4.w}, rj[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int j = 16 * cg + j4 + e;
-                const float E = ex2f_(fminf(gi - sGs[j], 0.f));
-                const float w = bi * v[j4 + e] * E * sh.rk[j];
-                if (q < 2) o4[e] = j < i ? w : (j == i ? 1.f : 0.f);
-                else o4[e] = j <= i ? w : 0.f;
+                const float E = ex2f_(fminf(gi - gj[e], 0.f));
+                const float w = bi * v[j4 + e] * E * rj[e];
+                o[j4 + e] = j < i ? w : j > i ? 0.f : q < 2 ? 1.f : w;
             }
-            *reinterpret_cast<float4*>(dst + j4) = make_float4(o4[0], o4[1], o4[2], o4[3]);
         }
+        if (q < 2) store_row16(sM + i * MLD + 16 * cg, o);
+        else store_aqk(i, o);
     } else {                                  // warp quadrant = row block I (lanes: 16 rows of Gamma, then 16 rows of Q K^T), cg = 16 columns j
         const int I = q, i = 16 * I + (lane & 15);
         const bool isq = lane >= 16;
@@ -408,40 +438,42 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         for (int e = 0; e < 16; ++e) v[e] = 0.f;
         if (cg <= I) umma::tmem_ld16(umma::tmem_addr(tmem, warp, kc_row(I) + 16 * cg), v);      // warp-uniform condition
         const float bi = isq ? p.scale * sh.rq[i] : sBeta[i] * sh.rk[i];
-        float* dst = (isq ? sP : sM) + i * MLD + 16 * cg;
+        float o[16];
 #pragma unroll
         for (int j4 = 0; j4 < 16; j4 += 4) {
-            float o4[4];
+            const float4 r4 = *reinterpret_cast<const float4*>(sh.rk + 16 * cg + j4);
+            const float rj[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int j = 16 * cg + j4 + e;
-                const float w = bi * v[j4 + e] * sh.rk[j];
-                if (isq) o4[e] = j <= i ? w : 0.f;
-                else o4[e] = j < i ? w : (j == i ? 1.f : 0.f);
+                const float w = bi * v[j4 + e] * rj[e];
+                o[j4 + e] = j < i ? w : j > i ? 0.f : isq ? w : 1.f;
             }
-            *reinterpret_cast<float4*>(dst + j4) = make_float4(o4[0], o4[1], o4[2], o4[3]);
+        }
+        if (isq) store_aqk(i, o);
+        else store_row16(sM + i * MLD + 16 * cg, o);
+    }
+    umma::fence_async_smem();
+    __syncthreads();
+    if (tid == STORER) {
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTQ, umma::QUARTER_TILE_BYTES);
+        if (BULK && item + stride < total) {
+            umma::bulk_store_wait_read_but<1>();       // the kbar tile has left
+            load_q(nxt);
         }
     }
-    __syncthreads();
     invert_unit_lower(sM, sInv, sh);
-    {   // A as the B operand of phase 3; A and Aqk also leave as ready-made [row][column] operand tiles (rows past the end:
-        // identity rows of A, zero rows of Aqk)
+    {   // A as the B operand of phase 3; it also leaves as a ready-made [row][column] operand tile (rows past the end: identity rows)
         const int r = tid >> 3, k8 = tid & 7;
-        float a8[8], q8[8];
+        float a8[8];
         lds8(sInv + r * MLD + k8 * 8, a8);
 #pragma unroll
         for (int e = 0; e < 8; ++e)
             if (k8 * 8 + e > r) a8[e] = 0.f;
-        lds8(sP + r * MLD + k8 * 8, q8);
         store_split8(sTA, sTA + 8192, 64, r, k8, a8);
-        store_split8(sTQ, sTQ + 8192, 64, r, k8, q8);
     }
     publish();
-    if (tid == 0) {
-        const size_t it = (size_t)c * HV + h;
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.A) + it * umma::QUARTER_TILE_BYTES, sTA, umma::QUARTER_TILE_BYTES);
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + it * umma::QUARTER_TILE_BYTES, sTQ, umma::QUARTER_TILE_BYTES);
-    }
+    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.A) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTA, umma::QUARTER_TILE_BYTES);
     if (umma::mma_issuer()) {
         const umma::Opnd bA = umma::opnd_k(sTA, sTA + 8192, 64);
         umma::gemm(tmem + 128, umma::opnd_mn(sBk, sBk + 16384, 64), bA, 128, 64, 64, 0u);
@@ -464,7 +496,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     }
     umma::fence_async_smem();
     __syncthreads();
-    if (tid == 0) umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base, umma::CHUNK_TILE_BYTES);
+    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base, umma::CHUNK_TILE_BYTES);
     {   // u^T [v][tok] leaves the same way (token columns past the end are exact zeros: A has identity rows there and
         // beta v zero rows), built next to the nw tile while that one is being copied
         float b[16], u0[8], u1[8];
@@ -478,11 +510,11 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     }
     umma::fence_async_smem();
     __syncthreads();
-    if (tid == 0) umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base + 32768, umma::CHUNK_TILE_BYTES);
+    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base + 32768, umma::CHUNK_TILE_BYTES);
     cur = nxt;
     advance(nxt);
     }   // items
-    if (tid == 0) umma::bulk_store_wait_read();
+    if (tid == STORER) umma::bulk_store_wait_read();
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 256);

@@ -320,6 +320,9 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" :: "l"(gdst), "r"(smem_u32(smem_src)), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// ... all but the latest N
+template <int N>
+__device__ __forceinline__ void bulk_store_wait_read_but() { asm volatile("cp.async.bulk.wait_group.read %0;" :: "n"(N) : "memory"); }
 __device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // Hint: bring `bytes` (multiple of 16) from the 16-byte aligned global address into L2; nothing waits for it.
