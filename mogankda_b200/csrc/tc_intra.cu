@@ -19,13 +19,19 @@
 namespace mkda {
 
 struct IntraShared {
-    uint64_t bar, bar2, ldin;
+    uint64_t ldin, op1, op2;                               // rows landed | operands of the first, second products written (16 warps)
+    uint64_t mm1, mmN, mmU;                                // products done: [Gamma; Q K^T], nw^T, u^T
     uint32_t tmem;
     __align__(16) float beta[2][CH];                       // of this item and (arriving) the next
     float rk[CH], rq[CH];                                  // L2 scales of the rows
     __align__(16) float T[32][36];
 };
 constexpr int TLD = 36;
+// 16 compute warps and one that issues the products (of a warpgroup of its own).  The tensor pipe accepts a product as slowly as it executes
+// them: the compute warp that issued used to come 1.4 k cycles after the others (of 19.7 k per item).  Registers as in bwd_chunk:
+// 16 x 32 x 112 + 4 x 32 x 32 = the 640 x 96 of the launch.
+constexpr int INTRA_THREADS = 640, INTRA_WARP_MMA = 16, INTRA_LAUNCH_REGS = 96;
+__device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
 constexpr int MLD = 68;
 // the four column tiles stacked by rows into one 160-row tile (hi 40 KB, then lo)
@@ -34,6 +40,7 @@ constexpr int KC_ALL_ROWS = 160;
 constexpr int KC_ALL_BYTES = KC_ALL_ROWS * 128 * 2;        // one of hi / lo
 constexpr int KQ_OFF = 81920;                              // [128][128] hi 32 KB, lo 32 KB
 constexpr int OPND_BYTES = KQ_OFF + 65536;                 // 144 KB
+constexpr int TA_OFF = 65536;                              // A, over the dead column tiles
 // The 16-bit k, q and the g rows of the NEXT item arrive by tiled copy (one 64 x 128 box per tensor) while the current item's
 // inverse and second products run: k and g rows in the upper 48 KB of the [Kr; Qr] tile, dead once the first products are
 // done, q rows over the kbar tile as soon as that has left.  They are read back into registers before the next item's operands are staged over them.  (Loads
@@ -96,7 +103,7 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
             *reinterpret_cast<float2*>(sInv + (ro + g + 8) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][2], -acc[nt][3]);
         }
     }
-    __syncthreads();
+    sync_compute();
     // 32 x 32 block (rows 32.., columns 0..31): eight warps, one 16 x 8 tile each
     const int m0 = 16 * ((warp >> 2) & 1), n0 = 8 * (warp & 3);
     float acc[1][4];
@@ -106,14 +113,44 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
         *reinterpret_cast<float2*>(&sh.T[m0 + g][n0 + 2 * t]) = make_float2(acc[0][0], acc[0][1]);
         *reinterpret_cast<float2*>(&sh.T[m0 + g + 8][n0 + 2 * t]) = make_float2(acc[0][2], acc[0][3]);
     }
-    __syncthreads();
+    sync_compute();
     if (warp < 8) {
         zero_acc(acc);
         warp_mma<1, 3, MLD, 1, TLD, 1>(acc, sInv + (32 + m0) * MLD + 32, &sh.T[0][n0], 32);
         *reinterpret_cast<float2*>(sInv + (32 + m0 + g) * MLD + n0 + 2 * t) = make_float2(-acc[0][0], -acc[0][1]);
         *reinterpret_cast<float2*>(sInv + (32 + m0 + g + 8) * MLD + n0 + 2 * t) = make_float2(-acc[0][2], -acc[0][3]);
     }
-    __syncthreads();
+    sync_compute();
+}
+
+// The issuing thread.  The base passes through an empty statement in front of each group of products: kept in registers over the loop, the
+// operand descriptors of all of them would spill.
+template <bool SCALAR>
+__device__ __forceinline__ void intra_issue(uint8_t* smem, uint32_t tmem, int total, IntraShared& sh) {
+    uint8_t* base = smem;
+    auto fresh = [&]() { base = smem; asm volatile("" : "+l"(base)); };
+    uint32_t it = 0;
+    for (int item = blockIdx.x; item < total; item += gridDim.x, ++it) {
+        umma::wait_mma(&sh.op1, it & 1);
+        fresh();
+        uint8_t* sKQ = base + KQ_OFF;
+        if (SCALAR) {      // D[m][j]: lanes 0..63 = K K^T rows, lanes 64..127 = Q K^T rows; columns j = K rows of the same tile
+            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(sKQ, sKQ + 32768, 128), 128, 64, 128, 0u);
+        } else {
+            // ONE product over the stacked column tiles: D[32 I + t][kc_row(I') + j].  Only the blocks I' = I are meaningful (the
+            // anchors of the two operands match there) and read back; the others are finite and ignored.  An MMA costs
+            // (4 KB of A + 32 N bytes of B) / 128 B per cycle, so N = 160 once is far cheaper than N = 32 four times.
+            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(base, base + KC_ALL_BYTES, KC_ALL_ROWS), 128, KC_ALL_ROWS, 128, 0u);
+        }
+        umma::commit(&sh.mm1);
+        umma::wait_mma(&sh.op2, it & 1);
+        fresh();
+        const umma::Opnd bA = umma::opnd_k(base + TA_OFF, base + TA_OFF + 8192, 64);
+        umma::gemm(tmem + 128, umma::opnd_mn(base, base + 16384, 64), bA, 128, 64, 64, 0u);
+        umma::commit(&sh.mmN);
+        umma::gemm(tmem + 192, umma::opnd_mn(base + 32768, base + 32768 + 16384, 64), bA, 128, 64, 64, 0u);
+        umma::commit(&sh.mmU);
+    }
 }
 
 // SCALAR: the gate is one decay per token (the same cumsum in all 128 channels).  It then commutes with the contraction
@@ -121,7 +158,7 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
 // [K; Q] tile) and the decay is applied to the accumulators, element by element and for i >= j only: nothing is anchored,
 // no exponent is ever positive, and any g <= 0 is in range (the per-channel path needs g >= -5 per token).
 template <int DT, bool SCALAR, bool TMA>
-__global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ IntraMaps maps) {
+__global__ void __launch_bounds__(INTRA_THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ IntraMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ IntraShared sh;
     // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
@@ -134,7 +171,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     float* sInv = sM + CH * MLD;
     uint8_t* sBk = base;                               // phase 3: beta k~ [j][K index], hi 16 KB + lo 16 KB
     uint8_t* sBv = base + 32768;                       // beta v [j][v]
-    uint8_t* sTA = base + 65536;                       // A [i][j], hi 8 KB + lo 8 KB
+    uint8_t* sTA = base + TA_OFF;                       // A [i][j], hi 8 KB + lo 8 KB
     uint8_t* sTQ = base + 81920;                       // Aqk [i][j], hi 8 KB + lo 8 KB (only copied out)
     uint8_t* sKB = base + OPND_BYTES;                  // kbar [tok][K index] hi + lo (32 KB), only copied out; later the q rows of the next item
     uint8_t* sQS = sKB + 32768;                        // scale q 2^g [tok][K index] hi + lo (32 KB), likewise; under sM and sInv
@@ -177,12 +214,22 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     };
     auto load_q = [&](const Item& i) { umma::tma_load_rows(base + RAW_Q, &maps.q, i.hk * 128, i.start, &sh.ldin); };
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 256);
-    if (tid == 0) { umma::mbar_init(&sh.bar, 1); umma::mbar_init(&sh.bar2, 1); umma::mbar_init(&sh.ldin, 1); umma::fence_barrier_init(); }
+    if (tid == 0) { 
+        for (uint64_t* b : {&sh.ldin, &sh.mm1, &sh.mmN, &sh.mmU}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.op1, &sh.op2}) umma::mbar_init(b, 16);
+        umma::fence_barrier_init();
+    }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
+    if (warp >= INTRA_WARP_MMA) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if (warp == INTRA_WARP_MMA && umma::elect_one()) intra_issue<SCALAR>(base, tmem, total, sh);
+        __syncwarp();
+    } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     cur.c = blockIdx.x / HV; cur.h = blockIdx.x - cur.c * HV; cur.hk = cur.h / G;
     table(cur);
     if ((int)blockIdx.x < total) {
@@ -233,7 +280,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
     }
     if (tid == STORER) umma::bulk_store_wait_read();   // the previous item's tiles have left shared memory
     umma::fence_before_sync();
-    __syncthreads();
+    sync_compute();
     umma::fence_after_sync();
     // ---- operands ---------------------------------------------------------------------------------------------------
     if (SCALAR) {          // one stacked tile: rows 0..63 = k, rows 64..127 = q (L2 statistics applied, zero past the end)
@@ -270,18 +317,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             }
         }
     }
-    publish();
-    if (umma::mma_issuer()) {
-        if (SCALAR) {      // D[m][j]: lanes 0..63 = K K^T rows, lanes 64..127 = Q K^T rows; columns j = K rows of the same tile
-            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(sKQ, sKQ + 32768, 128), 128, 64, 128, 0u);
-        } else {
-            // ONE product over the stacked column tiles: D[32 I + t][kc_row(I') + j].  Only the blocks I' = I are meaningful (the
-            // anchors of the two operands match there) and read back; the others are finite and ignored.  An MMA costs
-            // (4 KB of A + 32 N bytes of B) / 128 B per cycle, so N = 160 once is far cheaper than N = 32 four times.
-            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(base, base + KC_ALL_BYTES, KC_ALL_ROWS), 128, KC_ALL_ROWS, 128, 0u);
-        }
-        umma::commit(&sh.bar);
-    }
+    umma::signal(&sh.op1, lane);
     // The L2 scales are applied to what comes out (Gamma and Q K^T are bilinear in the rows) and to the tiles below: finding them takes no
     // time while the products run.  Four sums (k, q of two rows) over the 16 threads of a row; lane bits 3 and 2 end up spelling the sum.
     float fk[2] = {1.f, 1.f}, fq[2] = {1.f, 1.f};
@@ -372,14 +408,13 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         }
     }
     umma::fence_async_smem();
-    __syncthreads();
+    sync_compute();
     if (tid == STORER) {                               // qs first: its place is needed first
         const size_t it = (size_t)c * HV + h;
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + it * umma::CHUNK_TILE_BYTES, sQS, umma::CHUNK_TILE_BYTES);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + it * umma::CHUNK_TILE_BYTES, sKB, umma::CHUNK_TILE_BYTES);
     }
-    umma::mbar_wait(&sh.bar, 0);
-    umma::fence_after_sync();
+    umma::wait_mma(&sh.mm1, it & 1);
     // phase-3 operands over the dead phase-1 tiles: beta k 2^g and beta v (rows past the end are zero)
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
@@ -396,7 +431,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         store_split8(sBv, sBv + 16384, 64, r, k8, t8);
     }
     if (tid == STORER) umma::bulk_store_wait_read_but<1>();        // the tile under sM / sInv has left shared memory
-    __syncthreads();
+    sync_compute();
     if (item + stride < total) load_inputs(nxt, (it & 1) ^ 1);     // k, q, g, beta of the next item start travelling
     sInv[(32 * (tid >> 8) + ((tid >> 4) & 15)) * MLD + 32 * (tid >> 8) + 16 + (tid & 15)] = 0.f;       // blocks (0, 1) and (2, 3)
     auto store_row16 = [](float* dst, const float (&o)[16]) {
@@ -454,7 +489,7 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         else store_row16(sM + i * MLD + 16 * cg, o);
     }
     umma::fence_async_smem();
-    __syncthreads();
+    sync_compute();
     if (tid == STORER) {
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTQ, umma::QUARTER_TILE_BYTES);
         if (BULK && item + stride < total) {
@@ -472,17 +507,13 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
             if (k8 * 8 + e > r) a8[e] = 0.f;
         store_split8(sTA, sTA + 8192, 64, r, k8, a8);
     }
-    publish();
-    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.A) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTA, umma::QUARTER_TILE_BYTES);
-    if (umma::mma_issuer()) {
-        const umma::Opnd bA = umma::opnd_k(sTA, sTA + 8192, 64);
-        umma::gemm(tmem + 128, umma::opnd_mn(sBk, sBk + 16384, 64), bA, 128, 64, 64, 0u);
-        umma::commit(&sh.bar2);                        // nw^T is read out while the u^T products run
-        umma::gemm(tmem + 192, umma::opnd_mn(sBv, sBv + 16384, 64), bA, 128, 64, 64, 0u);
-        umma::commit(&sh.bar);
+    umma::signal(&sh.op2, lane);
+    if (tid == STORER) {
+        umma::mbar_wait(&sh.op2, it & 1);                  // all of A is there
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.A) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTA, umma::QUARTER_TILE_BYTES);
     }
-    umma::mbar_wait(&sh.bar2, it & 1);
-    umma::fence_after_sync();
+    // nw^T is read out while the u^T products run
+    umma::wait_mma(&sh.mmN, it & 1);
     {   // nw^T [K index][tok] leaves as a ready-made chunk tile (the serial kernels fetch it with one bulk copy; token
         // columns past the end are exact zeros: beta is 0 there)
         float a[16], n0[8], n1[8];
@@ -495,13 +526,12 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         store_split8(base, base + 16384, 128, row, 2 * cg + 1, n1);
     }
     umma::fence_async_smem();
-    __syncthreads();
+    sync_compute();
     if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base, umma::CHUNK_TILE_BYTES);
     {   // u^T [v][tok] leaves the same way (token columns past the end are exact zeros: A has identity rows there and
         // beta v zero rows), built next to the nw tile while that one is being copied
         float b[16], u0[8], u1[8];
-        umma::mbar_wait(&sh.bar, 1);
-        umma::fence_after_sync();
+        umma::wait_mma(&sh.mmU, it & 1);
         umma::tmem_ld16(umma::tmem_addr(tmem, warp, 192 + 16 * cg), b);
 #pragma unroll
         for (int j = 0; j < 8; ++j) { u0[j] = b[j]; u1[j] = b[8 + j]; }
@@ -509,12 +539,13 @@ __global__ void __launch_bounds__(512, 1) intra_fwd_tc_kernel(const MkdaIntraFwd
         store_split8(base + 32768, base + 32768 + 16384, 128, row, 2 * cg + 1, u1);
     }
     umma::fence_async_smem();
-    __syncthreads();
+    sync_compute();
     if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base + 32768, umma::CHUNK_TILE_BYTES);
     cur = nxt;
     advance(nxt);
     }   // items
     if (tid == STORER) umma::bulk_store_wait_read();
+    }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 256);
@@ -533,7 +564,9 @@ static int launch_intra_fwd_tc_tt(const MkdaIntraFwd* p, const IntraMaps& maps, 
     auto kern = intra_fwd_tc_kernel<DT, SCALAR, TMA>;
     if (int e = ensure_smem((const void*)kern, INTRA_TC_SMEM, "intra_fwd")) return e;
     const int items = p->L.NC * p->L.HV;
-    launch(kern, items < sm_count() ? items : sm_count(), 512, INTRA_TC_SMEM, stream, *p, maps);
+    static const int regs = kernel_registers((const void*)kern);
+    if (regs < INTRA_LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
+    launch(kern, items < sm_count() ? items : sm_count(), INTRA_THREADS, INTRA_TC_SMEM, stream, *p, maps);
     return check_launch("intra_fwd");
 }
 template <int DT, bool SCALAR>
