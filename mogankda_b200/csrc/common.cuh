@@ -185,7 +185,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 }
 
 __device__ __forceinline__ void mma_tf32_raw(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
@@ -246,6 +246,46 @@ __device__ __forceinline__ void warp_mma(float (&acc)[NT][4], const float* __res
             mma_frag<PREC>(acc[nt], fa, fb);
         }
     }
+}
+
+// The same with acc = A * B for a short Kd known at compile time: all fragments are loaded first, and the three products of the compensation
+// are summed apart, so that the chain of products is a third as long.
+template <int NT, int KD, int ARS, int ACS, int BKS, int BNS>
+__device__ __forceinline__ void warp_mma_short(float (&acc)[NT][4], const float* __restrict__ A, const float* __restrict__ B) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const float* ap = A + g * ARS + t * ACS;
+    const float* bp = B + t * BKS + g * BNS;
+    FragA<3> fa[KD / 8];
+    FragB<3> fb[KD / 8][NT];
+#pragma unroll
+    for (int k = 0; k < KD / 8; ++k) {
+        fa[k].set(0, ap[8 * k * ACS]);
+        fa[k].set(1, ap[8 * ARS + 8 * k * ACS]);
+        fa[k].set(2, ap[(8 * k + 4) * ACS]);
+        fa[k].set(3, ap[8 * ARS + (8 * k + 4) * ACS]);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            fb[k][nt].set(0, bp[8 * k * BKS + nt * 8 * BNS]);
+            fb[k][nt].set(1, bp[(8 * k + 4) * BKS + nt * 8 * BNS]);
+        }
+    }
+    float lh[NT][4], hl[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) lh[nt][e] = hl[nt][e] = acc[nt][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KD / 8; ++k)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            mma_tf32_raw(lh[nt], fa[k].lo, fb[k][nt].hi);
+            mma_tf32_raw(hl[nt], fa[k].hi, fb[k][nt].lo);
+            mma_tf32_raw(acc[nt], fa[k].hi, fb[k][nt].hi);
+        }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nt][e] += lh[nt][e] + hl[nt][e];
 }
 
 template <int NT>

@@ -87,16 +87,14 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
         const int ro = 32 * warp + 16, co = 32 * warp;
         float* T = &sh.T[16 * warp][0];
         float acc[2][4];
-        zero_acc(acc);
-        warp_mma<2, 3, MLD, 1, MLD, 1>(acc, sM + ro * MLD + co, sInv + co * MLD + co, 16);
+        warp_mma_short<2, 16, MLD, 1, MLD, 1>(acc, sM + ro * MLD + co, sInv + co * MLD + co);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
             *reinterpret_cast<float2*>(T + g * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][0], acc[nt][1]);
             *reinterpret_cast<float2*>(T + (g + 8) * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][2], acc[nt][3]);
         }
         __syncwarp();
-        zero_acc(acc);
-        warp_mma<2, 3, MLD, 1, TLD, 1>(acc, sInv + ro * MLD + ro, T, 16);
+        warp_mma_short<2, 16, MLD, 1, TLD, 1>(acc, sInv + ro * MLD + ro, T);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
             *reinterpret_cast<float2*>(sInv + (ro + g) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][0], -acc[nt][1]);
@@ -104,19 +102,18 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
         }
     }
     sync_compute();
-    // 32 x 32 block (rows 32.., columns 0..31): eight warps, one 16 x 8 tile each
+    // 32 x 32 block (rows 32.., columns 0..31): eight warps, one 16 x 8 tile each.  (Leaving out the products with zero blocks needs the code
+    // of several lengths and made the whole kernel 5 % slower: it is fetched anew for every item.)
     const int m0 = 16 * ((warp >> 2) & 1), n0 = 8 * (warp & 3);
     float acc[1][4];
     if (warp < 8) {
-        zero_acc(acc);
-        warp_mma<1, 3, MLD, 1, MLD, 1>(acc, sM + (32 + m0) * MLD, sInv + n0, 32);
+        warp_mma_short<1, 32, MLD, 1, MLD, 1>(acc, sM + (32 + m0) * MLD, sInv + n0);
         *reinterpret_cast<float2*>(&sh.T[m0 + g][n0 + 2 * t]) = make_float2(acc[0][0], acc[0][1]);
         *reinterpret_cast<float2*>(&sh.T[m0 + g + 8][n0 + 2 * t]) = make_float2(acc[0][2], acc[0][3]);
     }
     sync_compute();
     if (warp < 8) {
-        zero_acc(acc);
-        warp_mma<1, 3, MLD, 1, TLD, 1>(acc, sInv + (32 + m0) * MLD + 32, &sh.T[0][n0], 32);
+        warp_mma_short<1, 32, MLD, 1, TLD, 1>(acc, sInv + (32 + m0) * MLD + 32, &sh.T[0][n0]);
         *reinterpret_cast<float2*>(sInv + (32 + m0 + g) * MLD + n0 + 2 * t) = make_float2(-acc[0][0], -acc[0][1]);
         *reinterpret_cast<float2*>(sInv + (32 + m0 + g + 8) * MLD + n0 + 2 * t) = make_float2(-acc[0][2], -acc[0][3]);
     }
