@@ -100,18 +100,6 @@ __device__ __forceinline__ void unpack8(const Raw8& r, float (&v)[8]) {
         }
     }
 }
-// one element, raw (zero-extended for the 16-bit types) and widened later
-template <int DT>
-__device__ __forceinline__ uint32_t ldraw1(const void* base, size_t idx) {
-    if (DT == MKDA_F32) return static_cast<const uint32_t*>(base)[idx];
-    return static_cast<const uint16_t*>(base)[idx];
-}
-template <int DT>
-__device__ __forceinline__ float unpack1(uint32_t w) {
-    if (DT == MKDA_F32) return __uint_as_float(w);
-    if (DT == MKDA_BF16) return __uint_as_float(w << 16);
-    return __half2float(__ushort_as_half(static_cast<unsigned short>(w)));
-}
 
 __device__ __forceinline__ float ld1(const void* base, int dtype, size_t idx) {
     if (dtype == MKDA_F32) return static_cast<const float*>(base)[idx];
@@ -125,15 +113,6 @@ __device__ __forceinline__ void st1(void* base, int dtype, size_t idx, float v) 
     else static_cast<__half*>(base)[idx] = __float2half_rn(v);
 }
 
-__device__ __forceinline__ void st2(void* base, int dtype, size_t idx, float a, float b) {   // idx % 2 == 0
-    if (dtype == MKDA_F32) {
-        *reinterpret_cast<float2*>(static_cast<float*>(base) + idx) = make_float2(a, b);
-    } else if (dtype == MKDA_BF16) {
-        *reinterpret_cast<__nv_bfloat162*>(static_cast<__nv_bfloat16*>(base) + idx) = __floats2bfloat162_rn(a, b);
-    } else {
-        *reinterpret_cast<__half2*>(static_cast<__half*>(base) + idx) = __floats2half2_rn(a, b);
-    }
-}
 
 __device__ __forceinline__ void st4(void* base, int dtype, size_t idx, float4 v) {          // idx % 4 == 0
     if (dtype == MKDA_F32) {
@@ -191,72 +170,33 @@ __device__ __forceinline__ void mma_tf32_raw(float (&d)[4], const uint32_t (&a)[
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-template <int PREC>
+// a value as two TF32 parts
 struct FragA {
-    uint32_t hi[4];
-    uint32_t lo[PREC == 3 ? 4 : 1];
+    uint32_t hi[4], lo[4];
     __device__ __forceinline__ void set(int i, float x) {
         hi[i] = to_tf32(x);
-        if (PREC == 3) lo[i] = to_tf32(x - __uint_as_float(hi[i]));
+        lo[i] = to_tf32(x - __uint_as_float(hi[i]));
     }
 };
-template <int PREC>
 struct FragB {
-    uint32_t hi[2];
-    uint32_t lo[PREC == 3 ? 2 : 1];
+    uint32_t hi[2], lo[2];
     __device__ __forceinline__ void set(int i, float x) {
         hi[i] = to_tf32(x);
-        if (PREC == 3) lo[i] = to_tf32(x - __uint_as_float(hi[i]));
+        lo[i] = to_tf32(x - __uint_as_float(hi[i]));
     }
 };
 
-template <int PREC>
-__device__ __forceinline__ void mma_frag(float (&d)[4], const FragA<PREC>& a, const FragB<PREC>& b) {
-    if (PREC == 3) {
-        uint32_t alo[4] = {a.lo[0], a.lo[PREC == 3 ? 1 : 0], a.lo[PREC == 3 ? 2 : 0], a.lo[PREC == 3 ? 3 : 0]};
-        uint32_t blo[2] = {b.lo[0], b.lo[PREC == 3 ? 1 : 0]};
-        mma_tf32_raw(d, alo, b.hi);
-        mma_tf32_raw(d, a.hi, blo);
-    }
-    mma_tf32_raw(d, a.hi, b.hi);
-}
-
-// acc[NT][4] += A(16 x Kd) * B(Kd x 8*NT) for one warp.
+// acc[NT][4] = A(16 x KD) * B(KD x 8*NT) for one warp, KD a small multiple of 8.
 //   A(m, k) = A[m * ARS + k * ACS]   (pointer already offset to the warp's first row)
 //   B(k, n) = B[k * BKS + n * BNS]   (pointer already offset to the warp's first column)
-// Kd must be a multiple of 8.
-template <int NT, int PREC, int ARS, int ACS, int BKS, int BNS>
-__device__ __forceinline__ void warp_mma(float (&acc)[NT][4], const float* __restrict__ A,
-                                         const float* __restrict__ B, int Kd) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const float* ap = A + g * ARS + t * ACS;
-    const float* bp = B + t * BKS + g * BNS;
-#pragma unroll 2
-    for (int k0 = 0; k0 < Kd; k0 += 8) {
-        FragA<PREC> fa;
-        fa.set(0, ap[k0 * ACS]);
-        fa.set(1, ap[8 * ARS + k0 * ACS]);
-        fa.set(2, ap[(k0 + 4) * ACS]);
-        fa.set(3, ap[8 * ARS + (k0 + 4) * ACS]);
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            FragB<PREC> fb;
-            fb.set(0, bp[k0 * BKS + nt * 8 * BNS]);
-            fb.set(1, bp[(k0 + 4) * BKS + nt * 8 * BNS]);
-            mma_frag<PREC>(acc[nt], fa, fb);
-        }
-    }
-}
-
-// The same with acc = A * B for a short Kd known at compile time: all fragments are loaded first, and the three products of the compensation
-// are summed apart, so that the chain of products is a third as long.
+// All fragments are loaded first, and the three products of the compensation are summed apart, so that the chain of products is short.
 template <int NT, int KD, int ARS, int ACS, int BKS, int BNS>
 __device__ __forceinline__ void warp_mma_short(float (&acc)[NT][4], const float* __restrict__ A, const float* __restrict__ B) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const float* ap = A + g * ARS + t * ACS;
     const float* bp = B + t * BKS + g * BNS;
-    FragA<3> fa[KD / 8];
-    FragB<3> fb[KD / 8][NT];
+    FragA fa[KD / 8];
+    FragB fb[KD / 8][NT];
 #pragma unroll
     for (int k = 0; k < KD / 8; ++k) {
         fa[k].set(0, ap[8 * k * ACS]);
@@ -286,12 +226,6 @@ __device__ __forceinline__ void warp_mma_short(float (&acc)[NT][4], const float*
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[nt][e] += lh[nt][e] + hl[nt][e];
-}
-
-template <int NT>
-__device__ __forceinline__ void zero_acc(float (&acc)[NT][4]) {
-#pragma unroll
-    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 }
 
 // Two fp32 operations in one instruction (a pair of registers each): the staging and epilogue code is bound by instruction issue.
@@ -358,15 +292,5 @@ __device__ __forceinline__ float4 norm_gate(const float4& x, const float4& w, co
     return r;
 }
 
-// Chunk geometry shared by all chunk-parallel kernels: flattened first token and number of valid rows.
-struct ChunkGeom {
-    int start, len;
-};
-__device__ __forceinline__ ChunkGeom chunk_geom(const int* chunk_start, const int* chunk_len, int c) {
-    ChunkGeom gmt;
-    gmt.start = chunk_start[c];
-    gmt.len = chunk_len[c];
-    return gmt;
-}
 
 }  // namespace mkda

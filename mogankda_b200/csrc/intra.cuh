@@ -7,9 +7,6 @@ namespace mkda {
 
 using umma::store_split8;
 
-__device__ __forceinline__ void ldg8(const void* base, int dtype, size_t idx, float (&v)[8]) {
-    ld8(base, dtype, idx, v);
-}
 __device__ __forceinline__ void lds8(const float* p, float (&v)[8]) {
     const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;

@@ -1,4 +1,4 @@
-// Intra-chunk forward kernel on the Blackwell tensor cores: WY preparation.  One CTA (16 warps) per (chunk, v-head).
+// Intra-chunk forward kernel on the Blackwell tensor cores: WY preparation.  A persistent CTA per SM walks the (chunk, v-head) items.
 //
 //   Gamma_ij = sum_c k_ic k_jc 2^(g_ic - g_jc)  (i > j)        Aqk_ij = scale sum_c q_ic k_jc 2^(g_ic - g_jc)  (i >= j)
 //   A  = (I + strictlower(diag(beta) Gamma))^-1
@@ -11,8 +11,8 @@
 // (their g as the last valid row's), so they produce identity rows in A and are never stored.
 //   row operand     Kr[i] = k_i 2^(g_i - g_a(i)),  Qr[i] = q_i 2^(g_i - g_a(i))      one tile for all 64 rows
 //   column operand  Kc_I[j] = k_j 2^(g_aI - g_j),  j < 16 (I + 1)                    one tile per row block
-// With M = 128 mandatory, the column operand goes on M:  D_I[j][r] = Kc_I[j] . [Kr_I; Qr_I][r]  (N = 32, K = 128);
-// lanes j >= 16 (I + 1) read whatever follows the tile and are ignored (a D row depends on its own A row only).
+// What bounds it: the chain of phases of an item with one CTA per SM (18 k cycles; the item's own bytes take 8 k at 25 B per cycle).
+// Packed 6 k prefill x 32 heads 288 -> 236 us (with the L2 statistics, formerly a kernel), 32 k tokens 1373 -> 1120 us.
 #include "host.h"
 #include "intra.cuh"
 

@@ -132,10 +132,6 @@ __device__ __forceinline__ Opnd opnd_mn(const void* hi, const void* lo, int rows
     o.mn = 1;
     return o;
 }
-__device__ __forceinline__ uint64_t opnd_desc(const Opnd& o, uint32_t base, int ks) {
-    if (o.mn) return make_desc(base + ks * 2048, o.blk >> 4);
-    return make_desc(base + (ks >> 2) * o.blk + (ks & 3) * 32);
-}
 
 // D[M x N] (+)= A[M x 16] * B[N x 16]^T, one elected thread
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -330,14 +326,6 @@ __device__ __forceinline__ void l2_prefetch(const void* gsrc, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(gsrc), "r"(bytes) : "memory");
 }
 
-// One thread: initialise `bar` and start the asynchronous fetch of state tile `idx` of the array `tiles` into `smem_dst`
-// (1024-byte aligned).  Waiters use mbar_wait(bar, 0) after a CTA-wide barrier that follows this call.
-__device__ __forceinline__ void fetch_state_tile(uint64_t* bar, void* smem_dst, const void* tiles, size_t idx) {
-    mbar_init(bar, 1);
-    fence_barrier_init();
-    mbar_expect_tx(bar, STATE_TILE_BYTES);
-    bulk_load(smem_dst, static_cast<const uint8_t*>(tiles) + idx * STATE_TILE_BYTES, STATE_TILE_BYTES, bar);
-}
 
 // ---- tensor memory -------------------------------------------------------------------------------------------
 // one full warp allocates `ncols` (power of two >= 32) columns and publishes the base address through `slot`
@@ -348,7 +336,6 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 32 lanes x 32 columns: thread t of the warp receives columns [col, col+32) of TMEM lane (quadrant base + t)
@@ -365,20 +352,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
-        "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        :: "r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-           "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-           "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-           "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
-           "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-           "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-           "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
-           "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
-        : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
