@@ -128,6 +128,16 @@ __device__ __forceinline__ void st4(void* base, int dtype, size_t idx, float4 v)
     }
 }
 
+// two values rounded to the 16-bit type DT, in one word
+template <int DT>
+__device__ __forceinline__ uint32_t pack16(float a, float b) {
+    if (DT == MKDA_BF16) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&v);
+    }
+    const __half2 v = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
 // 8 consecutive elements, idx % 8 == 0
 template <int DT>
 __device__ __forceinline__ void st8(void* base, size_t idx, const float (&v)[8]) {
@@ -138,16 +148,14 @@ __device__ __forceinline__ void st8(void* base, size_t idx, const float (&v)[8])
     }
     uint32_t w[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        if (DT == MKDA_BF16) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-            w[e] = *reinterpret_cast<const uint32_t*>(&b);
-        } else {
-            const __half2 b = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-            w[e] = *reinterpret_cast<const uint32_t*>(&b);
-        }
-    }
+    for (int e = 0; e < 4; ++e) w[e] = pack16<DT>(v[2 * e], v[2 * e + 1]);
     *reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + idx) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// 32 bytes in one store, `dst` 32-byte aligned
+__device__ __forceinline__ void st32b(void* dst, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------

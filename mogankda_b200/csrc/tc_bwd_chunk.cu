@@ -245,6 +245,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     float (*early_ga)[DK] = reinterpret_cast<float (*)[DK]>(base + EARLY_GA);
     // the two token rows of a thread, of blocks 0 and 3 or 1 and 2: a row of block B enters 4 - B column tiles, so each thread writes five
     auto staged_row = [&](int m) { return m ? 32 + ((tid >> 4) ^ 16) : tid >> 4; };
+    const bool dv_sectors = (reinterpret_cast<uintptr_t>(p.dv) & 31) == 0;
     constexpr bool STASH = DT != MKDA_F32;                 // fp32 rows do not fit: the epilogue reads them from global memory
 
     // chunk table entries and the per-row scalars (beta | L2 statistics | scalar gate) travel one item ahead: every address of an item
@@ -316,12 +317,19 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             if (t < len) {
                 const float bt = sh.beta[t];
                 const size_t tv = ((size_t)(start + t) * HV + h) * 128 + v0;
+                if (DT != MKDA_F32 && dv_sectors) {        // a lane's 16 values are one 32-byte sector (1B shape 215 -> 213 us, short documents 266 -> 262)
+                    uint32_t o[8];
 #pragma unroll
-                for (int j = 0; j < 16; j += 8) {
-                    float o8[8];
+                    for (int j = 0; j < 8; ++j) o[j] = pack16<DT>(bt * dw[2 * j], bt * dw[2 * j + 1]);
+                    st32b(static_cast<uint16_t*>(p.dv) + tv, o);
+                } else {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) o8[e] = bt * dw[j + e];
-                    st8<DT>(p.dv, tv + j, o8);
+                    for (int j = 0; j < 16; j += 8) {
+                        float o8[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o8[e] = bt * dw[j + e];
+                        st8<DT>(p.dv, tv + j, o8);
+                    }
                 }
             }
         }

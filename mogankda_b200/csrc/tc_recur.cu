@@ -29,11 +29,7 @@ constexpr int X = 0, D0 = 256, D1 = 320, O = 384;          // fp32 accumulators:
 using umma::signal_tmem;
 using umma::wait_mma;
 
-// 32 bytes to global memory in one piece
-__device__ __forceinline__ void st32b(void* dst, const uint32_t (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 :: "l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-}
+// 32 bytes of fp32 in one load, `src` 32-byte aligned
 __device__ __forceinline__ void ld32b(const void* src, float* v) {
     uint32_t w[8];
     asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

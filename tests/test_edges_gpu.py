@@ -117,6 +117,32 @@ def test_partial_reductions(rows, cols, group):
     assert got.shape == ref.shape and ((got - ref).abs() <= 1e-6 * x.double().abs().view(rows, cols // group, group).sum((0, 2))).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_value_gradient_on_a_16_byte_boundary(dtype, monkeypatch):
+    """mkda_bwd_chunk stores dv in 32-byte pieces where its address allows that, in 16-byte pieces otherwise: the same bits, and none beside
+    them.  Chunks of 1, 64 and 35 rows."""
+    from mogankda_b200 import _lib, ops
+    from mogankda_b200.index import get_layout
+    lv, do, _, opts, _ = make_inputs(cu=(0, 1, 100), T=100, HK=1, HV=2, dtype=dtype, gate="eda", h0=False, epi=None, seed=83)
+    lay = get_layout(1, 100, opts["cu_seqlens"], lv["q"].device)
+    rq, rk = ops.l2norm_rstd(lv["q"]), ops.l2norm_rstd(lv["k"])
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "eda", lv["A_log"], lv["dt_bias"], -5.0, 2, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, 128 ** -0.5, 1, 2)
+    h, Vd, _, _ = ops.recur_fwd(lay, nw, u, kbar, gl, 1, 2)
+    dh, dVd_t, dO_t, _ = ops.bwd_dh(lay, do.to(dtype), kbar, qs, gl, Aqk, nw, 1, 2)
+    args = (lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, A, h, dh, Vd, dO_t, dVd_t, 128 ** -0.5, 1, 2, lv["beta"], True, 2.0)
+    dv = ops.bwd_chunk(*args)[4]
+    buf = torch.full((100 * 2 * 128 + 16,), 7.0, dtype=dtype, device="cuda")
+    call = _lib.call
+
+    def shifted(name, p, stream):
+        p.dv = buf.data_ptr() + 16
+        return call(name, p, stream)
+    monkeypatch.setattr(_lib, "call", shifted)
+    ops.bwd_chunk(*args)
+    assert torch.equal(buf[8:-8].view_as(dv), dv) and (buf[:8] == 7).all() and (buf[-8:] == 7).all()
+
+
 @pytest.mark.parametrize("epi", [None, "silu"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_output_in_the_chain_kernel(dtype, epi):
