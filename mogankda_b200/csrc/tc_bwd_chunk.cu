@@ -5,9 +5,10 @@
 //   dW = A^T dVd          dV = diag(beta) dW          dAqk = lower(dO Vd^T)
 //   dL = -strictlower(A^T dA A^T) with dA = (dVd X^T) diag(beta), X = V - k~ S.  Since A diag(beta) X = Vd this is
 //   dL = -strictlower(dW Vd^T): one product of tiles that exist anyway, instead of rebuilding X and a chain of three products.
-//   dbeta_i = (dW X^T)_ii + (dL Gamma^T)_ii = dW_i . (X - Gamma Vd)_i = (dW Vd^T)_ii / beta_i, because beta (X - Gamma Vd) = Vd: the diagonal of
-//   the same product.  (With a sigmoid the 1 / beta cancels.  A chunk that holds a precomputed beta below 1e-12 takes the long way:
-//   rowsum(dW * V) - rowsum(k~ * (dW S^T)) + rowsum(k * T).)
+//   dbeta_i = (dW X^T)_ii + (dL Gamma^T)_ii = rowsum(dW * V) - rowsum(k~ * (dW S^T)) + rowsum(k * T).  (It also is (dW Vd^T)_ii / beta_i, the
+//   diagonal of the product above, for nothing; but Vd carries the errors of the state chain where V is exact: over 50 cases that came to 1.16
+//   times the error against fp64, up to 6.4e-6 instead of 3.7e-6.  So V is read (213 -> 228 us at the 1B shape, 262 -> 273 on short documents),
+//   and what the bf16 halves leave of dW, 2.4e-6 of the sum, is kept as a third part.)
 // State part (up = 2^g, rest = 2^(g_L - g)):
 //   dq_p = scale (dO S^T) up         dk_p = -beta (dW S^T) up + (Vd dS'^T) rest        dgl = rowsum_v(S * dS')
 // Intra-chunk part, E_ij = 2^(g_i - g_j) per channel (i > j), Wq = scale strictlower(dAqk), dLs = strictlower(dL):
@@ -58,10 +59,13 @@ __host__ __device__ constexpr int w_piece(int i) { return R_ + 16 * KB * i + 8 *
 __host__ __device__ constexpr int kc_hi(int I) { return I == 0 ? o_piece(0) : I == 1 ? o_piece(1) : I == 2 ? 192 * KB : V_; }
 __host__ __device__ constexpr int kc_lo(int I) { return I == 0 ? o_piece(0) + 4 * KB : I == 1 ? o_piece(2) : I == 2 ? 204 * KB : V_ + 16 * KB; }
 constexpr int EARLY_GA = o_piece(3);
+// over dead dO rows (pieces 0, 1): what the bf16 halves leave of dW, [64][128] bf16, 16-byte chunks swizzled with the row
+__device__ __forceinline__ int rest_chunk(int t, int k8) { return o_piece(t >> 5) + (t & 31) * 256 + ((k8 ^ (t & 7)) << 4); }
 // raw 16-bit k (pieces 0, 1) and q (2, 3) rows kept for the epilogue: 32 token rows of 256 bytes per piece
 __device__ __forceinline__ int stash(int which, int tok) { return w_piece(2 * which + (tok >> 5)) + (tok & 31) * 256; }
 __host__ __device__ constexpr int ccol(int I) { return I == 0 ? 128 : I == 1 ? 144 : I == 2 ? 176 : 224; }
-constexpr int D1 = 128, DQ = 320, DKB = 384, DW = DQ, DB = 448;     // accumulator columns; dW of the next item takes the place of Dq and Dk
+// accumulator columns; dW of the next item takes the place of Dq and Dk; its rest waits in DWR (free until the column products)
+constexpr int D1 = 128, DWR = 192, DQ = 320, DKB = 384, DW = DQ, DB = 448;
 
 struct Shared {
     uint64_t fullW, fullS, fullT;                       // copies landed: (dVd, A) | (S, dO, Vd) | dS'
@@ -69,7 +73,7 @@ struct Shared {
     uint64_t opW, opI[4], accFree;                      // compute warps done: dW tile | intra-chunk operands per row block | scratch
     uint32_t tmem;
     alignas(16) float dgl[DK];
-    float beta[CH], rk[CH], rq[CH], diag[CH], gs[CH], up[CH], dbw[CH];
+    float beta[CH], rk[CH], rq[CH], diag[CH], gs[CH], up[CH], dbw[CH];        // dbw: rowsum(dW * V)
 };
 constexpr int SMEM = TILES + (int)sizeof(Shared);
 static_assert(SMEM <= 232448, "shared memory of one CTA");
@@ -77,15 +81,10 @@ static_assert(SMEM <= 232448, "shared memory of one CTA");
 struct Scratch {
     float ga[5][DK];                                    // the anchor rows again, for the epilogue
     float col[4][DK];
-    float redg[4][CH], re[CH];
+    float redg[4][CH], redb[4][CH], re[CH];
 };
 static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
 
-__device__ __forceinline__ bool sync_compute_or(bool x) {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 512, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"((uint32_t)x) : "memory");
-    return r != 0;
-}
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 using umma::elect_one;
 using umma::signal;
@@ -281,39 +280,34 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             next_start = p.L.chunk_start[c]; next_len = p.L.chunk_len[c];
         }
 
-        bool tiny = false;
         if (tid < CH) {
             sh.beta[tid] = ahead0;
-            tiny = !p.beta_sigmoid && tid < len && fabsf(ahead0) < 1e-12f;
         } else if (tid < 2 * CH) {
             sh.rk[tid - CH] = ahead0; sh.rq[tid - CH] = ahead1;
         } else if (SCALAR && tid < 3 * CH) {
             sh.gs[tid - 2 * CH] = ahead0;
             sh.up[tid - 2 * CH] = ex2f_(ahead0);
         }
-        const bool long_way = sync_compute_or(tiny);       // dbeta of this chunk cannot be formed as Z_ii / beta_i
+        sync_compute();
 
         // ---- dW: rows of the stacked tile, dv = beta dW ----
         wait_mma(&sh.mmW, par);
         {
             const int t = row & 63, v0 = (q < 2 ? 0 : 64) + 16 * cg;      // token, first of 16 values
-            float dw[16], x0[8], x1[8];
+            float dw[16];
+            uint32_t rest[8];
             umma::tmem_ld16(umma::tmem_addr(tmem, warp, DW + v0), dw);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { x0[j] = dw[j]; x1[j] = dw[8 + j]; }
-            store_split8(base + R_, base + R_ + 32768, 128, 64 + t, v0 >> 3, x0);
-            store_split8(base + R_, base + R_ + 32768, 128, 64 + t, (v0 >> 3) + 1, x1);
-            signal(&sh.opW, lane);
-            if (long_way) {                                // rowsum(dW * V), the partial sums of the eight warps of a token added in turn
-                float s = 0.f;
-                const size_t tv = ((size_t)(start + (t < len ? t : len - 1)) * HV + h) * 128 + v0;
+            for (int m = 0; m < 2; ++m) {
+                uint32_t hi[4], lo[4];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) s = fmaf(dw[j], ld1(p.v, DT, tv + j), s);
-                for (int k = 0; k < 8; ++k) {
-                    if (k == 2 * cg + (q >> 1)) sh.dbw[t] = k ? sh.dbw[t] + s : s;
-                    sync_compute();
-                }
+                for (int e = 0; e < 4; ++e) umma::split3(dw[8 * m + 2 * e], dw[8 * m + 2 * e + 1], hi[e], lo[e], rest[4 * m + e]);
+                const uint32_t off = umma::tile_chunk_offset(128, 64 + t, (v0 >> 3) + m);
+                *reinterpret_cast<uint4*>(base + R_ + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(base + R_ + 32768 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
+            umma::tmem_st8(umma::tmem_addr(tmem, warp, DWR + 8 * cg), rest);
+            signal(&sh.opW, lane);
             if (t < len) {
                 const float bt = sh.beta[t];
                 const size_t tv = ((size_t)(start + t) * HV + h) * 128 + v0;
@@ -333,8 +327,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                 }
             }
         }
-        // ---- k, q, g rows, used once the state products are under way ----
-        Raw8 wk[2], wq[2];
+        // ---- k, q, g, v rows, used once the state products are under way ----
+        Raw8 wk[2], wq[2], wv[2];
         f32x2 vg[2][4];
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
@@ -342,6 +336,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             const size_t tk = ((size_t)(start + rr) * HK + hk) * 128 + k8 * 8;
             ldraw8<DT>(p.k, tk, wk[m]);
             ldraw8<DT>(p.q, tk, wq[m]);
+            ldraw8<DT>(p.v, ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, wv[m]);
             if (!SCALAR) lds8(p.g_c + ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, vg[m]);
         }
         // ---- dgl[c] = sum_v S[c][v] dS'[c][v] from the two tiles: warp = 8 channels, lanes = v ----
@@ -364,6 +359,26 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             if ((lane & 3) == 0) sh.dgl[warp * 8 + (lane >> 2)] = acc[0];
         }
         wait_mma(&sh.mmL, par);
+        {
+            uint32_t r8[8];
+            umma::tmem_wait_st();
+            umma::tmem_ld8(umma::tmem_addr(tmem, warp, DWR + 8 * cg), r8);
+            const int t = row & 63, k8 = (q < 2 ? 0 : 8) + 2 * cg;
+            *reinterpret_cast<uint4*>(base + rest_chunk(t, k8)) = make_uint4(r8[0], r8[1], r8[2], r8[3]);
+            *reinterpret_cast<uint4*>(base + rest_chunk(t, k8 + 1)) = make_uint4(r8[4], r8[5], r8[6], r8[7]);
+        }
+        // ---- rowsum(dW * V), as far as the halves of dW in the stacked tile go; the rest of dW over dead dO rows ----
+        umma::mbar_wait(&sh.opW, par);                     // all of dW is there
+        f32x2 dwv[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            f32x2 d2[4], v2[4];
+            umma::load_tile8(base + R_, base + R_ + 32768, 128, 64 + staged_row(m), tid & 15, d2);
+            unpack8<DT>(wv[m], v2);
+            dwv[m] = mul2(d2[0], v2[0]);
+#pragma unroll
+            for (int e = 1; e < 4; ++e) dwv[m] = fma2(d2[e], v2[e], dwv[m]);
+        }
         if (!SCALAR) {
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
@@ -371,7 +386,29 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                 if ((r & 15) == 0) sts_halves(early_ga[r >> 4], k8, vg[m]);
             }
         }
-        sync_compute();                                    // every thread has read its part of S; anchor rows visible
+        sync_compute();                                    // every thread has read its part of S; anchor rows and the rest of dW visible
+        {
+            float t2[2];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                f32x2 d2[4], v2[4];
+                Raw8 r;
+                r.a = *reinterpret_cast<const uint4*>(base + rest_chunk(staged_row(m), tid & 15));
+                unpack8<MKDA_BF16>(r, d2);
+                unpack8<DT>(wv[m], v2);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dwv[m] = fma2(d2[e], v2[e], dwv[m]);
+                float a0, a1;
+                unpack2(dwv[m], a0, a1);
+                t2[m] = a0 + a1;
+            }
+            // 16 threads per row; lane bit 3 ends up choosing between the thread's two rows
+            const float recv = __shfl_xor_sync(0xffffffffu, (lane & 8) ? t2[0] : t2[1], 8);
+            float t = ((lane & 8) ? t2[1] : t2[0]) + recv;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if ((lane & 7) == 0) sh.dbw[staged_row((lane >> 3) & 1)] = t;
+        }
         // ---- [Qr; beta Kr] over S while Db is computed, then the weights and the column tiles ----
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
@@ -442,12 +479,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                     const int j = cg * 16 + hf * 8 + e;
                     const float E = SCALAR ? ex2f_(fminf(gi - sh.gs[j], 0.f)) : 1.f;
                     w8[e] = j < i && i < len ? f * d[hf * 8 + e] * E : 0.f;
-                    // diagonals: scale dAqk_ii, and (dW Vd^T)_ii for dbeta (predicated stores: selecting d[i & 15] first makes the compiler
-                    // index it in local memory, which every warp then waits for behind the next barrier)
-                    if (j == i) {
-                        if (q < 2) sh.diag[i] = i < len ? p.scale * d[hf * 8 + e] : 0.f;
-                        else if (!long_way) sh.dbw[i] = d[hf * 8 + e];
-                    }
+                    // the diagonal scale dAqk_ii (a predicated store: selecting d[i & 15] first makes the compiler index it in local
+                    // memory, which every warp then waits for behind the next barrier)
+                    if (j == i && q < 2) sh.diag[i] = i < len ? p.scale * d[hf * 8 + e] : 0.f;
                 }
                 store_split8(base + WD_, base + WD_ + 16384, 128, wrow, 2 * cg + hf, w8);
                 if (SCALAR && q >= 2) {
@@ -467,7 +501,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                 if (r == CH - 1) sts_halves(scr.ga[4], k8, vg[m]);         // rows past the end carry the last valid row's
             }
         }
-        sync_compute();                                    // diag, dbw, scratch
+        sync_compute();                                    // diag, scratch
         if (!SCALAR) {
             f32x2 k8v[2][4];
 #pragma unroll
@@ -558,7 +592,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                     for (int r = 0; r < 4; ++r) z[r] = fma2(both(f), u[r], z[r]);
                 }
             }
-            // Rows past the end: sh.rk and sh.rq are 0 there, every other factor is finite.  bsv: long way only.
+            // Rows past the end: sh.rk and sh.rq are 0 there, every other factor is finite.
             float bsv[8], dgs[8];
 #pragma unroll
             for (int r4 = 0; r4 < 2; ++r4) {               // the rows' scalars four at a time: one broadcast read each instead of four
@@ -607,13 +641,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                     }
                 }
             }
-            if (long_way) {
-                warp_colsum(bsv, lane);
-                for (int k = 0; k < 4; ++k) {
-                    if (k == q && (lane & 3) == 0) sh.dbw[c0 + (lane >> 2)] += bsv[0];
-                    sync_compute();
-                }
-            }
+            warp_colsum(bsv, lane);
+            if ((lane & 3) == 0) scr.redb[q][c0 + (lane >> 2)] = bsv[0];
             if (SCALAR) {
                 warp_colsum(dgs, lane);
                 if ((lane & 3) == 0) scr.redg[q][c0 + (lane >> 2)] = dgs[0];
@@ -645,9 +674,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             og[tid] = t;
         }
         if (tid < len) {
-            float db = sh.dbw[tid];
-            if (p.beta_sigmoid) db *= 1.f - sigmoidf_(raw_beta);          // Z / beta times beta_scale sg (1 - sg), with beta = beta_scale sg
-            else if (!long_way) db /= sh.beta[tid];
+            float db = sh.dbw[tid] + ((scr.redb[0][tid] + scr.redb[1][tid]) + (scr.redb[2][tid] + scr.redb[3][tid]));
+            if (p.beta_sigmoid) db *= sh.beta[tid] * (1.f - sigmoidf_(raw_beta));          // beta = beta_scale sg: its derivative is beta (1 - sg)
             st1(p.dbeta, p.dbeta_dtype, (size_t)(start + tid) * HV + h, db);
         }
         signal(&sh.accFree, lane);
