@@ -6,11 +6,13 @@
 //
 // Range / prefix invariance: the per-channel decay 2^(g_i - g_j) does not factor out of the contraction over channels,
 // so each 16-row block I uses its first row a = 16 I as anchor: row operand k_i 2^(g_i - g_a) (<= 1), column operand
-// k_j 2^(g_a - g_j) (<= 1 for j < a, <= 2^(15*5/ln2) inside the diagonal block).  An output element (i, j) therefore
-// depends on rows i, j and a <= i only, never on later rows.  Rows past the end of the sequence are staged as zeros
+// k_j 2^(g_a - g_j) (<= |k| for j < a, <= 2^(15*5/ln2) |k| = 2^108 |k| inside the diagonal block).  An output element (i, j) therefore
+// depends on rows i, j and a <= i only, never on later rows.  The rows are staged as they come, the L2 scales applied to what comes out, so |k|
+// is whatever the caller's scale is: 2^48 goes from the column to the row operands (exact, and nothing in range changes by it), which leaves room
+// for every row whose sum of squares is finite and keeps the low halves of small rows out of the subnormals.  Rows past the end of the sequence are staged as zeros
 // (their g as the last valid row's), so they produce identity rows in A and are never stored.
-//   row operand     Kr[i] = k_i 2^(g_i - g_a(i)),  Qr[i] = q_i 2^(g_i - g_a(i))      one tile for all 64 rows
-//   column operand  Kc_I[j] = k_j 2^(g_aI - g_j),  j < 16 (I + 1)                    one tile per row block
+//   row operand     Kr[i] = k_i 2^(48 + g_i - g_a(i)),  Qr[i] = q_i 2^(48 + g_i - g_a(i))      one tile for all 64 rows
+//   column operand  Kc_I[j] = k_j 2^(g_aI - g_j - 48),  j < 16 (I + 1)                         one tile per row block
 // What bounds it: the chain of phases of an item with one CTA per SM (18 k cycles; the item's own bytes take 8 k at 25 B per cycle).
 // Packed 6 k prefill x 32 heads 288 -> 236 us (with the L2 statistics, formerly a kernel), 32 k tokens 1373 -> 1120 us.
 #include "host.h"
@@ -34,6 +36,7 @@ constexpr int INTRA_THREADS = 640, INTRA_WARP_MMA = 16, INTRA_LAUNCH_REGS = 96;
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
 constexpr int MLD = 68;
+constexpr float ROW_UP = 0x1p48f, COL_DOWN = 0x1p-48f;      // column operand: 108 + 64 - 48 < 127, row operand: 64 + 48 < 127 for |k| < 2^64
 // the four column tiles stacked by rows into one 160-row tile (hi 40 KB, then lo)
 __host__ __device__ constexpr int kc_row(int I) { return I == 0 ? 0 : I == 1 ? 16 : I == 2 ? 48 : 96; }
 constexpr int KC_ALL_ROWS = 160;
@@ -294,17 +297,20 @@ __global__ void __launch_bounds__(INTRA_THREADS, 1) intra_fwd_tc_kernel(const Mk
             f32x2 ga[4], t8[4], e8[4];
             lds_halves(sGa[I0], k8, ga);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { e8[e] = ex2f2_(sub2(vg[n][e], ga[e])); t8[e] = mul2(vk[n][e], e8[e]); }
+            for (int e = 0; e < 4; ++e) { e8[e] = mul2(ex2f2_(sub2(vg[n][e], ga[e])), both(ROW_UP)); t8[e] = mul2(vk[n][e], e8[e]); }
             store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, t8);
 #pragma unroll
             for (int e = 0; e < 4; ++e) t8[e] = mul2(vq[n][e], e8[e]);
             store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, t8);
+            f32x2 kd[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) kd[e] = mul2(vk[n][e], both(COL_DOWN));
 #pragma unroll
             for (int I = 0; I < 4; ++I) {
                 if (I < I0) continue;
                 if (I <= I0 + 1) {
                     if (I > I0) lds_halves(sGa[I], k8, ga);
-                    scale_ex2(t8, vk[n], ga, vg[n]);
+                    scale_ex2(t8, kd, ga, vg[n]);
                 } else {                                   // a step of decay (<= 1) further down the anchors: exponentials are what bounds this phase
                     lds_halves(sStep[I - 2], k8, ga);
 #pragma unroll

@@ -190,3 +190,15 @@ def test_beta_gradient_keeps_the_accuracy_of_v(scalar, bound):
     got = run(mk.chunk_delta_rule, lv, do, dht, opts, None)["dbeta"].double()
     ref = run(orc.chunked_delta_rule, lv, do, dht, opts, None, f64=True)["dbeta"]
     assert ((got - ref).norm() / ref.norm()).item() < bound
+
+
+@pytest.mark.parametrize("size", [1e-4, 1e-3, 1.0, 1e3, 1e7, 1e12])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("decay", [-5.0, -0.5])
+def test_l2_norm_takes_rows_of_any_size(dtype, size, decay):
+    """With the L2 norm in the kernels the scale of the raw q and k rows is the caller's: the anchored operands (decay factors up to 2^108 at the
+    bound of -5 per token) must neither overflow nor lose their low halves.  Three full chunks and a ragged one."""
+    lv, do, dht, opts, _ = make_inputs(T=64 * 3 + 21, HK=1, HV=2, dtype=dtype, gate="precomputed", epi=None, seed=97)
+    lv["g"] = torch.full_like(lv["g"], decay)
+    lv["q"], lv["k"] = (lv["q"].float() * size).to(dtype), (lv["k"].float() * size).to(dtype)
+    compare(run(mk.chunk_delta_rule, lv, do, dht, opts, None), run(orc.chunked_delta_rule, lv, do, dht, opts, None, f64=True))
