@@ -171,6 +171,7 @@ def chunk_delta_rule(q, k, v, g, beta, *, scale=None, initial_state=None, output
         ep_gate, ep_w, act, eps = ep["gate"], ep.get("weight"), ops.ACTS.get(ep.get("act", "silu")), ep.get("eps", 1e-6)
         if act is None:
             raise ValueError(f"unknown act {ep.get('act')!r}")
+    host.check_params(v, g, A_log, dt_bias, ep_w, ep_gate)
     if warmup_threshold is not None and not float(warmup_threshold) < 0.0:
         raise ValueError("warmup_threshold must be negative (natural-log units, e.g. -10.0) or None")
     scale = 128 ** -0.5 if scale is None else float(scale)

@@ -118,6 +118,24 @@ PyObject* check(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// check_params(v, g, A_log, dt_bias, norm weight, norm gate): the kernels take the sizes of these tensors from v and g, for reading them and
+// for writing their gradients
+PyObject* check_params(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 6) return fail(PyExc_TypeError, "check_params takes 6 arguments");
+    Tensor v, g, alog, bias, w, gate;
+    Tensor* t[6] = {&v, &g, &alog, &bias, &w, &gate};
+    for (int i = 0; i < 6; ++i)
+        if (!tensor_arg(a[i], *t[i])) return nullptr;
+    const int64_t HV = v.size(2);
+    REQUIRE(!alog.defined() || alog.numel() == HV, "A_log must have one element per v-head");
+    REQUIRE(!bias.defined() || bias.numel() == (g.dim() == 3 ? HV : HV * 128), "dt_bias must have one element per v-head and, for a per-channel gate, key channel");
+    REQUIRE(!w.defined() || w.numel() == 128, "the weight of the gated norm must have 128 elements");
+    REQUIRE(!gate.defined() || gate.numel() == v.numel(), "the gate of the gated norm must have as many elements as v");
+    Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
+}
+
 // layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all, longest, chain), scale, want_ht,
 //       v_first, gate mode, lower bound or None, beta sigmoid, beta scale, l2, act or None, eps, warm-up threshold or None) -> (o, ht or None)
 PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -203,6 +221,7 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyMethodDef methods[] = {
     {"check", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check)), METH_FASTCALL, "argument checks of a call"},
+    {"check_params", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check_params)), METH_FASTCALL, "sizes of the parameter tensors"},
     {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(layer)), METH_FASTCALL, "one layer call"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "host path of a layer call over libmkda", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -88,3 +88,21 @@ def test_entry_points_reject_misaligned_tensors_without_launching():
     q.dk = 0x30008
     assert lib.mkda_qk_grad_finish(ctypes.byref(q), None) == -1
     assert b"16-byte aligned" in lib.mkda_last_error()
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+def test_parameter_tensors_of_other_sizes_are_refused(lib, scalar):
+    """The kernels take the sizes of A_log, dt_bias and the norm's tensors from v and g; a smaller one would be read, and its gradient written,
+    past its end."""
+    from mogankda_b200 import _lib
+    check, HV = _lib.host().check_params, 4
+    v = torch.zeros(1, 8, HV, 128)
+    g = v[..., 0] if scalar else v
+    A, bias, w = torch.zeros(HV), torch.zeros(HV if scalar else HV * 128), torch.zeros(128)
+    for good in ((None,) * 4, (A, bias, w, v), (A.view(1, 1, HV, 1), bias.view(HV, -1), w.view(1, 128), v.view(8, HV * 128))):
+        check(v, g, *good)
+    other_bias = torch.zeros(HV * 128 if scalar else HV)
+    for bad in ((A[:-1], None, None, None), (A.repeat(2), None, None, None), (None, other_bias, None, None), (None, bias[:-1], None, None),
+                (None, None, w[:64], None), (None, None, None, v[:, :7]), (None, None, None, v[..., 0])):
+        with pytest.raises(AssertionError):
+            check(v, g, *bad)

@@ -202,3 +202,14 @@ def test_l2_norm_takes_rows_of_any_size(dtype, size, decay):
     lv["g"] = torch.full_like(lv["g"], decay)
     lv["q"], lv["k"] = (lv["q"].float() * size).to(dtype), (lv["k"].float() * size).to(dtype)
     compare(run(mk.chunk_delta_rule, lv, do, dht, opts, None), run(orc.chunked_delta_rule, lv, do, dht, opts, None, f64=True))
+
+
+def test_calls_with_parameters_of_other_sizes_are_refused():
+    lv, _, _, opts, _ = make_inputs(T=70, dtype=torch.bfloat16, gate="eda", epi="silu", h0=False, seed=101)
+    call = lambda A, b, w, z: mk.chunk_kda(lv["q"], lv["k"], lv["v"], lv["g"], lv["beta"], A_log=A, dt_bias=b,          # noqa: E731
+                                           output_norm=dict(weight=w, gate=z, act="silu"), **opts)
+    good = (lv["A_log"], lv["dt_bias"], lv["ep_w"], lv["ep_gate"])
+    call(*good)
+    for i, bad in enumerate((lv["A_log"][:3], lv["dt_bias"][:, 0], lv["ep_w"][:64], lv["ep_gate"][:, :69])):
+        with pytest.raises(AssertionError):
+            call(*good[:i], bad.contiguous(), *good[i + 1:])
