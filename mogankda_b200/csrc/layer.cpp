@@ -210,7 +210,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
           *part_a = nullptr, *dloc = nullptr, *g_in = nullptr;
     const int64_t tile = MKDA_CHUNK_TILE_BYTES, seg_states = (int64_t)c.NS * c.HV * 65536;
     const int w_rows = std::min(c.NC * c.HV, MKDA_EPILOGUE_MAX_PART_ROWS);
-    const int g_rows = std::max(1, std::min(c.NC, 256)), g_width = c.scalar_gate ? c.HV : c.HV * 128;
+    const int g_rows = std::min(c.NC, 256), g_width = c.scalar_gate ? c.HV : c.HV * 128;
     tmp.want(&dO, c.tiles(tile));
     tmp.want(&dh, c.tiles(MKDA_STATE_TILE_BYTES));
     tmp.want(&dVd, c.tiles(tile));
@@ -278,10 +278,10 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         MkdaGateBwd p{};
         p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(s.x_alog);
         p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound; p.dgp = dgp; p.dx = g.x.data_ptr(); p.dx_dtype = dtype_code(g.x);
-        p.part_rows = g_rows; p.part_bias = part_b; p.part_alog = part_a;
+        p.part_rows = std::max(g_rows, 1); p.part_bias = part_b; p.part_alog = part_a;
         check_rc(mkda_gate_bwd(&p, st), "mkda_gate_bwd");
     }
-    if (part_w || part_b || part_a) {                      // the parameter gradients' second stage, in one launch
+    if (part_w || part_b || part_a) {                      // the parameter gradients' second stage, in one launch (no chunk: sums of no rows)
         MkdaReduceMulti p{};
         if (part_w) { g.ep_w = new_cuda({128}, at::kFloat, c.dev); p.job[0] = {part_w, w_rows, 128, 1, fptr(g.ep_w)}; }
         if (part_b) { g.dt_bias = new_cuda(in.dt_bias.sizes(), at::kFloat, c.dev); p.job[1] = {part_b, g_rows, g_width, 1, fptr(g.dt_bias)}; }

@@ -118,12 +118,13 @@ def gate_bwd(lay, x, dgp, mode, A_log, dt_bias, lower_bound, HV, want_bias, want
     rows = max(1, min(lay.NC, 256))
     p.part_rows = rows
     part_b = part_a = None
+    alloc = torch.empty if lay.NC else torch.zeros          # without a chunk the kernel writes no partial row
     if mode != "precomputed":
         if want_bias:
-            part_b = torch.empty(rows, width, dtype=torch.float32, device=x.device)
+            part_b = alloc(rows, width, dtype=torch.float32, device=x.device)
             p.part_bias = _ptr(part_b)
         if want_alog:
-            part_a = torch.empty(rows, HV, dtype=torch.float32, device=x.device)
+            part_a = alloc(rows, HV, dtype=torch.float32, device=x.device)
             p.part_alog = _ptr(part_a)
     _lib.call("mkda_gate_bwd", p, _stream())
     d_bias = reduce_partials(part_b, rows, width) if part_b is not None else None

@@ -213,3 +213,22 @@ def test_calls_with_parameters_of_other_sizes_are_refused():
     for i, bad in enumerate((lv["A_log"][:3], lv["dt_bias"][:, 0], lv["ep_w"][:64], lv["ep_gate"][:, :69])):
         with pytest.raises(AssertionError):
             call(*good[:i], bad.contiguous(), *good[i + 1:])
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+def test_gradients_of_a_batch_without_tokens_are_zero(scalar):
+    """Only empty sequences (padding tokens on a data-parallel rank): no kernel writes a partial sum, and every gradient is exactly zero, that of
+    the initial state the upstream one.  Freed memory full of NaN stands ready for whatever is allocated."""
+    from mogankda_b200 import ops
+    from mogankda_b200.index import get_layout
+    lv, do, dht, opts, epi = make_inputs(cu=(0, 0, 0), T=7, dtype=torch.bfloat16, gate="eda", scalar=scalar, epi="silu", seed=103)
+    for n in (1 << 9, 1 << 12, 1 << 16, 1 << 20, 1 << 24):
+        junk = [torch.full((n,), float("nan"), device="cuda") for _ in range(4)]
+        del junk
+    got = run(mk.chunk_delta_rule, lv, do, dht, opts, epi)
+    assert torch.equal(got.pop("dh0"), dht) and torch.equal(got.pop("ht"), lv["h0"])
+    for n, t in got.items():
+        assert (t == 0).all(), n
+    lay = get_layout(1, 7, opts["cu_seqlens"], do.device)
+    _, db, da = ops.gate_bwd(lay, lv["g"], torch.empty(1, device="cuda"), "eda", lv["A_log"], lv["dt_bias"], -5.0, 4, True, True)
+    assert (db == 0).all() and (da == 0).all()
