@@ -27,18 +27,30 @@ using torch::autograd::variable_list;
 
 namespace {
 
-// The inputs are saved as variables (in-place changes are detected, a second backward pass is refused once the buffers are gone), the
-// intermediates as plain memory.
+// Inputs and intermediates are saved as variables: in-place changes are detected, a second backward pass is refused once the buffers are gone,
+// and saved-tensor hooks (activation checkpointing, offloading) get all of it.  The blocks that hold the intermediates may come back from a hook
+// at another place: the pointers into them are taken again.
 constexpr int NUM_INPUTS = 10;
 struct DeltaRuleBackward : public torch::autograd::Node {
     Call call;
     SavedVariable vars[NUM_INPUTS];
+    std::vector<SavedVariable> blocks;                     // saved->arena.keep
+    std::vector<int64_t> block_bytes;
     std::unique_ptr<Saved> saved;
 
     std::string name() const override { return "DeltaRuleBackward"; }
     void release_variables() override {
         for (auto& v : vars) v.reset_data();
+        for (auto& b : blocks) b.reset_data();
         saved.reset();
+    }
+    void save(std::unique_ptr<Saved> s) {
+        saved = std::move(s);
+        for (const Tensor& t : saved->arena.keep) {
+            blocks.emplace_back(t, false);
+            block_bytes.push_back(t.numel());
+        }
+        saved->arena.keep.clear();
     }
     variable_list apply(variable_list&& grads) override {
         std::lock_guard<std::mutex> lock(mutex_);
@@ -47,6 +59,15 @@ struct DeltaRuleBackward : public torch::autograd::Node {
         for (int i = 0; i < NUM_INPUTS; ++i) *slots[i] = vars[i].unpack();
         TORCH_CHECK(saved, torch::autograd::ERR_BACKWARD_TWICE);
         c10::cuda::CUDAGuard guard(call.dev);
+        std::vector<Tensor>& keep = saved->arena.keep;
+        struct Release { std::vector<Tensor>& t; ~Release() { t.clear(); } } release{keep};      // the saved variables hold the blocks
+        for (size_t i = 0; i < blocks.size(); ++i) {
+            const Tensor t = blocks[i].unpack();
+            TORCH_CHECK(t.scalar_type() == at::kByte && t.numel() == block_bytes[i] && t.device() == call.dev,
+                        "chunk_delta_rule: a saved-tensor hook returned another tensor than was saved");
+            keep.push_back(aligned(t, 256));
+        }
+        saved->arena.point();
         const Tensor dy = grads[0], dht = grads.size() > 1 ? grads[1] : Tensor();
         const bool twice = c10::GradMode::is_enabled() && ((dy.defined() && dy.requires_grad()) || (dht.defined() && dht.requires_grad()));
         Grads g;
@@ -202,7 +223,7 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         }
         if (any) {
             node->call = c;
-            node->saved = std::move(saved);
+            node->save(std::move(saved));
             torch::autograd::set_history(out, node);
             if (ht.defined()) torch::autograd::set_history(ht, node);
         }

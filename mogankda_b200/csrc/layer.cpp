@@ -100,8 +100,7 @@ std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in) {
 std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need_bwd, Saved& s) {
     cudaStream_t st = c10::cuda::getCurrentCUDAStream();
     const int64_t row = (int64_t)c.TT * c.HV * 128 * 4, seg_states = (int64_t)c.NS * c.HV * 65536;
-    s.x_alog = aligned_f32(in.A_log);
-    s.x_bias = aligned_f32(in.dt_bias);
+    const Tensor alog = aligned_f32(in.A_log), bias = aligned_f32(in.dt_bias);
     Arena tmp;
     Arena& keep = s.arena;
     float *u = nullptr, *hs = nullptr, *s_in = nullptr;
@@ -141,7 +140,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     {
         MkdaGateFwd p{};
         p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate;
-        p.A_log = fptr(s.x_alog); p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound;
+        p.A_log = fptr(alog); p.dt_bias = fptr(bias); p.mode = c.mode; p.lower_bound = c.lower_bound;
         p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta); p.beta_sigmoid = c.beta_sigmoid;
         p.beta_scale = c.beta_scale; p.beta_out = s.beta_e; p.g_c = s.g_c;
         check_rc(mkda_gate_cumsum_fwd(&p, st), "mkda_gate_cumsum_fwd");
@@ -275,9 +274,10 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     }
     g.x = c.like_out(in.x);
     {
+        const Tensor alog = aligned_f32(in.A_log), bias = aligned_f32(in.dt_bias);
         MkdaGateBwd p{};
-        p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(s.x_alog);
-        p.dt_bias = fptr(s.x_bias); p.mode = c.mode; p.lower_bound = c.lower_bound; p.dgp = dgp; p.dx = g.x.data_ptr(); p.dx_dtype = dtype_code(g.x);
+        p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(alog);
+        p.dt_bias = fptr(bias); p.mode = c.mode; p.lower_bound = c.lower_bound; p.dgp = dgp; p.dx = g.x.data_ptr(); p.dx_dtype = dtype_code(g.x);
         p.part_rows = std::max(g_rows, 1); p.part_bias = part_b; p.part_alog = part_a;
         check_rc(mkda_gate_bwd(&p, st), "mkda_gate_bwd");
     }

@@ -25,27 +25,27 @@ Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev)
 // blocks one by one.
 constexpr int64_t ARENA_SINGLE = 64 << 20;
 struct Arena {
-    struct Req { void** dst; int64_t bytes; };
+    struct Req { void** dst; int64_t bytes, offset; size_t block; };
     std::vector<Req> reqs;
     std::vector<Tensor> keep;
     template <typename T>
-    void want(T** dst, int64_t bytes) { reqs.push_back({reinterpret_cast<void**>(dst), (std::max<int64_t>(bytes, 1) + 255) / 256 * 256}); }
+    void want(T** dst, int64_t bytes) { reqs.push_back({reinterpret_cast<void**>(dst), (std::max<int64_t>(bytes, 1) + 255) / 256 * 256, 0, 0}); }
     void allocate(const at::Device& dev) {
         int64_t total = 0;
         for (const auto& r : reqs) total += r.bytes;
         const bool single = total <= ARENA_SINGLE;
         if (single && total) keep.push_back(new_cuda({total}, at::kByte, dev));
-        char* base = single && total ? static_cast<char*>(keep.back().data_ptr()) : nullptr;
-        for (const auto& r : reqs) {
-            if (single) {
-                *r.dst = base;
-                base += r.bytes;
-            } else {
-                keep.push_back(new_cuda({r.bytes}, at::kByte, dev));
-                *r.dst = keep.back().data_ptr();
-            }
+        int64_t at = 0;
+        for (auto& r : reqs) {
+            if (!single) keep.push_back(new_cuda({r.bytes}, at::kByte, dev));
+            r.block = keep.size() - 1;
+            r.offset = single ? at : 0;
+            at += r.bytes;
         }
-        reqs.clear();
+        point();
+    }
+    void point() {                         // the pointers into the blocks of `keep`, which may have been elsewhere in between
+        for (const auto& r : reqs) *r.dst = static_cast<char*>(keep[r.block].data_ptr()) + r.offset;
     }
 };
 
@@ -81,7 +81,6 @@ struct Call {
 // What the forward pass leaves for the backward pass (pointers into `arena`).
 struct Saved {
     Arena arena;
-    Tensor x_alog, x_bias;                 // the parameter tensors as the kernels read them (fp32)
     float *q_rstd = nullptr, *k_rstd = nullptr, *g_c = nullptr, *beta_e = nullptr, *A = nullptr, *Aqk = nullptr, *nw = nullptr,
           *kbar = nullptr, *qs = nullptr, *gl = nullptr, *h = nullptr, *Vd = nullptr, *o_raw = nullptr, *ms = nullptr;
     int* warm_end = nullptr;

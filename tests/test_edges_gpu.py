@@ -232,3 +232,47 @@ def test_gradients_of_a_batch_without_tokens_are_zero(scalar):
     lay = get_layout(1, 7, opts["cu_seqlens"], do.device)
     _, db, da = ops.gate_bwd(lay, lv["g"], torch.empty(1, device="cuda"), "eda", lv["A_log"], lv["dt_bias"], -5.0, 4, True, True)
     assert (db == 0).all() and (da == 0).all()
+
+
+def _training_call(T, epi, seed):
+    lv, do, dht, opts, epi = make_inputs(T=T, HK=2, HV=4, dtype=torch.bfloat16, gate="eda", epi=epi, seed=seed)
+    x = {n: t.clone().requires_grad_(True) for n, t in lv.items()}
+    norm = None if epi is None else dict(weight=x["ep_w"], gate=x["ep_gate"], act=epi)
+    f = lambda q: mk.chunk_delta_rule(q, x["k"], x["v"], x["g"], x["beta"], A_log=x["A_log"], dt_bias=x["dt_bias"], initial_state=x["h0"],          # noqa: E731
+                                      output_norm=norm, **opts)
+    grads = lambda o, ht: torch.autograd.grad((o, ht), list(x.values()), (do.to(o.dtype), dht))          # noqa: E731
+    return f, x["q"], grads
+
+
+# intermediates in one block | in a block each | sequences cut into segments
+@pytest.mark.parametrize("T,epi", [(130, "silu"), (130, None), (64 * 80, "silu"), (64 * 300 + 9, None)])
+def test_saved_tensor_hooks_get_the_intermediates(T, epi):
+    """Offloading moves everything the backward pass needs, and what a hook brings back from another place is used: the same bits."""
+    f, q, grads = _training_call(T, epi, 107)
+    ref = grads(*f(q))
+    sizes = []
+
+    def pack(t):
+        sizes.append(t.numel() * t.element_size())
+        return t.cpu()
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        o, ht = f(q)
+    chunk_heads = (T + 63) // 64 * 4
+    assert sum(sizes) > chunk_heads * (65536 + 4 * 32768)          # states, nw, kbar, qs, Vd are among them
+    for a, b in zip(ref, grads(o, ht)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,epi", [(130, "silu"), (64 * 80, "silu"), (64 * 300 + 9, None)])
+def test_activation_checkpointing_frees_the_intermediates(T, epi):
+    import gc
+    from torch.utils.checkpoint import checkpoint
+    f, q, grads = _training_call(T, epi, 109)
+    ref = grads(*f(q))
+    gc.collect()
+    before = torch.cuda.memory_allocated()
+    o, ht = checkpoint(f, q, use_reentrant=False)
+    held = torch.cuda.memory_allocated() - before - o.numel() * o.element_size() - ht.numel() * 4
+    assert held < 1 << 16, held
+    for a, b in zip(ref, grads(o, ht)):
+        assert torch.equal(a, b)
