@@ -193,8 +193,11 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         dtype_code(in.ep_gate);
         if (in.ep_w.defined()) dtype_code(in.ep_w);
     }
-    for (Tensor* t : slots)
+    for (Tensor* t : slots) {
         if (t->defined() && !t->is_cuda()) return fail(PyExc_RuntimeError, NEED_CUDA);
+        // a node without a forward-mode formula would drop the tangent without a word
+        if (t->defined() && t->_fw_grad(0).defined()) return fail(PyExc_NotImplementedError, "chunk_delta_rule: forward-mode AD is not supported");
+    }
     c.set_tables(tables);
 
     Tensor out, ht;

@@ -276,3 +276,14 @@ def test_activation_checkpointing_frees_the_intermediates(T, epi):
     assert held < 1 << 16, held
     for a, b in zip(ref, grads(o, ht)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("grads", [False, True])
+def test_forward_mode_ad_is_refused(grads):
+    """... not answered without a tangent, whichever tensor carries it."""
+    import torch.autograd.forward_ad as fwad
+    f, q, _ = _training_call(70, None, 113)
+    with torch.set_grad_enabled(grads), fwad.dual_level():
+        with pytest.raises(NotImplementedError):
+            f(fwad.make_dual(q, torch.ones_like(q)))
+    f(q)
