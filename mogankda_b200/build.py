@@ -80,8 +80,10 @@ def build(force=False, verbose=False):
     host = os.path.join(HERE, "_host.so")
     if force or host_jobs or not _newer(host, [*host_objs, out]):
         torch_lib = os.path.join(torch_dir, "lib")
+        # The C++ runtime that torch has loaded, by name: a compiler that brings only an archive of it would put a second copy into the module,
+        # whose streams have no locale (the first number in an error message ended the process)
         subprocess.check_call([cxx, "-shared", "-o", host, *host_objs, "-L" + HERE, "-lmkda", "-L" + torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu",
-                               "-ltorch_cuda", "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib])
+                               "-ltorch_cuda", "-ltorch", "-ltorch_python", "-l:libstdc++.so.6", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib])
     return out
 
 

@@ -106,3 +106,14 @@ def test_parameter_tensors_of_other_sizes_are_refused(lib, scalar):
                 (None, None, w[:64], None), (None, None, None, v[:, :7]), (None, None, None, v[..., 0])):
         with pytest.raises(AssertionError):
             check(v, g, *bad)
+
+
+@pytest.mark.parametrize("name", ["_host.so", "libmkda.so"])
+def test_modules_share_the_cxx_runtime_of_the_process(lib, name):
+    """A second, private copy of the C++ runtime has streams without a locale: formatting a number for an error message crashed the process."""
+    import subprocess
+    path = os.path.join(ROOT, "mogankda_b200", name)
+    needed = subprocess.run(["readelf", "-d", path], capture_output=True, text=True, check=True).stdout
+    symbols = subprocess.run(["nm", "-D", "--defined-only", path], capture_output=True, text=True, check=True).stdout
+    assert "libstdc++.so.6" in needed
+    assert "_ZNSo9_M_insertIlEERSoT_" not in symbols          # std::ostream::_M_insert<long>
