@@ -27,6 +27,24 @@ using torch::autograd::variable_list;
 
 namespace {
 
+// An error of the library is a mogankda_b200._lib.MkdaError, in the forward call and out of the autograd engine.  Called without the GIL.
+template <typename F>
+auto library_call(F f) {
+    try {
+        return f();
+    } catch (const LibraryError& e) {
+        pybind11::gil_scoped_acquire gil;
+        PyObject* mod = PyImport_ImportModule("mogankda_b200._lib");
+        PyObject* type = mod ? PyObject_GetAttrString(mod, "MkdaError") : nullptr;
+        if (type) PyErr_SetString(type, e.what());
+        Py_XDECREF(type);
+        Py_XDECREF(mod);
+        python_error err;
+        err.persist();
+        throw err;
+    }
+}
+
 // Inputs and intermediates are saved as variables: in-place changes are detected, a second backward pass is refused once the buffers are gone,
 // and saved-tensor hooks (activation checkpointing, offloading) get all of it.  The blocks that hold the intermediates may come back from a hook
 // at another place: the pointers into them are taken again.
@@ -73,8 +91,10 @@ struct DeltaRuleBackward : public torch::autograd::Node {
         Grads g;
         {
             at::AutoGradMode off(false);
-            g = run_backward(call, in, *saved, dy, dht, in.A_log.defined() && task_should_compute_output(5),
-                             in.dt_bias.defined() && task_should_compute_output(6), task_should_compute_output(7));
+            g = library_call([&] {
+                return run_backward(call, in, *saved, dy, dht, in.A_log.defined() && task_should_compute_output(5),
+                                    in.dt_bias.defined() && task_should_compute_output(6), task_should_compute_output(7));
+            });
         }
         variable_list out = {g.q, g.k, g.v, g.x, g.beta, g.A_log, g.dt_bias, g.h0, g.ep_w, g.ep_gate};
         for (int i = 0; i < NUM_INPUTS; ++i)
@@ -222,7 +242,7 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
             // (one token: 9 instead of 63 us of kernels at 8 sequences x 32 heads).  Calls that start from zero keep to the chunk algebra, whose
             // results for a prefix of a sequence are those of the whole sequence bit for bit.
             const bool step = !any && in.h0.defined() && c.longest <= MKDA_STEP_MAX_TOKENS && c.N <= 65535;
-            std::tie(out, ht) = step ? run_step(c, in) : run_forward(c, in, any, *saved);
+            std::tie(out, ht) = library_call([&] { return step ? run_step(c, in) : run_forward(c, in, any, *saved); });
         }
         if (any) {
             node->call = c;

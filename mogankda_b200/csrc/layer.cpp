@@ -37,7 +37,9 @@ Tensor aligned_f32(const Tensor& t) {
     return aligned(t.scalar_type() == at::kFloat ? t : t.to(at::kFloat));
 }
 float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
-void check_rc(int rc, const char* what) { TORCH_CHECK(rc == MKDA_OK, what, " failed (", rc, "): ", mkda_last_error()); }
+void check_rc(int rc, const char* what) {
+    if (rc != MKDA_OK) throw LibraryError(std::string(what) + " failed (" + std::to_string(rc) + "): " + mkda_last_error());
+}
 
 // (row stride, column stride) in elements if `t` [..., 128] can be addressed as rows x 128 with one stride per axis (contiguous
 // tensors, and broadcast views such as the gradient autograd produces for o.sum()); false otherwise

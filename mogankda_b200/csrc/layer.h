@@ -5,6 +5,8 @@
 #include <ATen/cuda/EmptyTensor.h>
 
 #include <algorithm>
+#include <stdexcept>
+#include <string>
 #include <utility>
 #include <vector>
 
@@ -14,6 +16,7 @@ namespace mkda_host {
 
 using at::Tensor;
 
+struct LibraryError : std::runtime_error { using std::runtime_error::runtime_error; };      // an entry point of libmkda returned an error
 int dtype_code(const Tensor& t);           // MKDA_F32 / MKDA_BF16 / MKDA_F16; TypeError otherwise
 // The kernels read and write their tensors with 16-byte vector accesses and bulk copies: operands are made contiguous and, where a
 // contiguous view starts at an odd storage offset, copied.

@@ -287,3 +287,15 @@ def test_forward_mode_ad_is_refused(grads):
         with pytest.raises(NotImplementedError):
             f(fwad.make_dual(q, torch.ones_like(q)))
     f(q)
+
+
+def test_errors_of_the_library_are_mkda_errors():
+    """A lower bound that is not negative is refused by the kernels' entry points, on the chunk path and on the path of a few tokens."""
+    from mogankda_b200 import _lib
+    lv, _, _, opts, _ = make_inputs(T=70, dtype=torch.bfloat16, gate="kimi", epi=None, h0=False, seed=127)
+    for T in (70, 3):
+        cut = {n: t[:, :T].contiguous() for n, t in lv.items() if t.dim() > 2}
+        h0 = torch.zeros(1, 4, 128, 128, device="cuda") if T == 3 else None
+        with torch.no_grad(), pytest.raises(_lib.MkdaError, match="lower_bound"):
+            mk.chunk_kda(cut["q"], cut["k"], cut["v"], cut["g"], cut["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"], initial_state=h0,
+                         **dict(opts, lower_bound=1.0))
