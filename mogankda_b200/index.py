@@ -7,6 +7,7 @@ and the segments are stitched by the state-combine kernel (the same mechanism ca
 GPUs).  The segment length never depends on the sequence length, so a prefix of a sequence is segmented exactly
 like the full sequence (bitwise prefix invariance).
 """
+import threading
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -104,6 +105,18 @@ def wants_segments(chunks_per_seq, HV, seg_chunks, sm_count=None, cost_ratio=2.5
 # way every step) can never hit an old entry, and an in-place edit changes the version.
 _cache = []
 _CACHE_MAX = 16
+_cache_lock = threading.Lock()      # held for list operations only, never for a read-back or an upload
+
+
+def _cached(key, cu_seqlens, ver):
+    with _cache_lock:
+        for i in range(len(_cache) - 1, -1, -1):
+            k, ref, v, lay = _cache[i]
+            if ref is cu_seqlens and v == ver and k == key:
+                if i != len(_cache) - 1:
+                    _cache.append(_cache.pop(i))          # most recently used last
+                return lay
+    return None
 
 
 def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=2.5):
@@ -112,12 +125,9 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
     ``auto_heads`` > 0 lets ``wants_segments`` decide, for that many v-heads, whether ``seg_chunks`` is applied."""
     key = (B, T, device, seg_chunks, auto_heads, cost_ratio)
     ver = None if cu_seqlens is None else cu_seqlens._version
-    for i in range(len(_cache) - 1, -1, -1):
-        k, ref, v, lay = _cache[i]
-        if ref is cu_seqlens and v == ver and k == key:
-            if i != len(_cache) - 1:
-                _cache.append(_cache.pop(i))          # most recently used last
-            return lay
+    lay = _cached(key, cu_seqlens, ver)
+    if lay is not None:
+        return lay
     cu = None if cu_seqlens is None else [int(x) for x in cu_seqlens.tolist()]
     if auto_heads > 0:
         lens = [T] * B if cu is None else [e - s for s, e in zip(cu[:-1], cu[1:])]
@@ -139,7 +149,8 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
     NC, NS, segmented = len(tb["chunk_start"]), len(tb["seg_first"]), len(tb["seg_first"]) != tb["N"]
     lay = Layout(B=B, T=T, N=tb["N"], NC=NC, NS=NS, NG=tb["N"], segmented=segmented, covers_all=tb["covers_all"], host=tb, tables=tables,
                  dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"]), longest, chain), **part)
-    if len(_cache) >= _CACHE_MAX:
-        _cache.pop(0)
-    _cache.append((key, cu_seqlens, ver, lay))
+    with _cache_lock:
+        if len(_cache) >= _CACHE_MAX:
+            _cache.pop(0)
+        _cache.append((key, cu_seqlens, ver, lay))
     return lay

@@ -86,3 +86,33 @@ def test_layout_cache_is_keyed_on_tensor_identity_not_on_its_address():
     c = fresh[0]
     c[1] = 64                                                           # in-place edit: the version counter moves
     assert index.get_layout(1, 256, c, "cpu").chunk_len.tolist()[0] == 64
+
+
+def test_layout_cache_is_safe_with_several_threads():
+    """Forward calls on several threads (one per device) share the cache: more boundaries than it holds, looked up and evicted at the same time."""
+    import sys
+    import threading
+    import torch
+    from mogankda_b200 import index
+    cus = [torch.tensor([0, 10 + i, 256], dtype=torch.int32) for i in range(40)]
+    errors = []
+
+    def work(k):
+        try:
+            for r in range(400):
+                i = (r * 7 + k * 13) % 40
+                assert index.get_layout(1, 256, cus[i], "cpu").chunk_len.tolist()[0] == 10 + i
+                index.get_layout(1, 256, cus[k], "cpu")
+        except Exception as e:
+            errors.append(e)
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not errors and len(index._cache) <= index._CACHE_MAX
