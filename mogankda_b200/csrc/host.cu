@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/mkda.h"
 #include "host.h"
@@ -30,7 +31,7 @@ int check_launch(const char* what) {
 }
 
 int sm_count() {
-    static int cached[64] = {0};
+    static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
     if (!cached[dev]) {
@@ -45,7 +46,8 @@ int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned l
                   int box_rows) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Encode encode = nullptr;                    // resolved through the runtime: the library does not link against the driver
+    static std::atomic<Encode> resolved{nullptr};      // through the runtime: the library does not link against the driver
+    Encode encode = resolved.load(std::memory_order_relaxed);
     if (!encode) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -55,6 +57,7 @@ int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned l
             return MKDA_ERR_LAUNCH;
         }
         encode = reinterpret_cast<Encode>(fn);
+        resolved.store(encode, std::memory_order_relaxed);
     }
     const unsigned long long pitch = row_elems * (unsigned long long)elem_bytes;
     if ((reinterpret_cast<uintptr_t>(base) & 15) || (pitch & 15) || row_elems < 128 || rows == 0) {
@@ -81,12 +84,15 @@ int kernel_registers(const void* func) {
 }
 
 int ensure_smem(const void* func, int bytes, const char* what) {
-    // (function, device) pairs whose limit is already raised; a launcher asks before every launch
+    // (function, device) pairs whose limit is already raised; a launcher asks before every launch.  Launches come from several threads: callers
+    // that have released the GIL, and the autograd engine's thread of each device.
     struct Done { const void* func; int dev; int bytes; };
     static Done done[256];
     static int ndone = 0;
+    static std::mutex mutex;
     int dev = 0;
     (void)cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mutex);
     for (int i = 0; i < ndone; ++i)
         if (done[i].func == func && done[i].dev == dev && done[i].bytes >= bytes) return MKDA_OK;
     cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -95,7 +101,7 @@ int ensure_smem(const void* func, int bytes, const char* what) {
         (void)cudaGetLastError();
         return MKDA_ERR_LAUNCH;
     }
-    if (ndone < 256) done[ndone++] = Done{func, dev, bytes};      // single-threaded host, as the reference assumes
+    if (ndone < 256) done[ndone++] = Done{func, dev, bytes};
     return MKDA_OK;
 }
 

@@ -5,6 +5,8 @@
 #include "common.cuh"
 #include <stdio.h>
 
+#include <atomic>
+
 #include "gate.cuh"
 #include "host.h"
 #include "umma.cuh"
@@ -682,7 +684,7 @@ extern "C" int mkda_qk_grad_finish(const MkdaQkGrad* p, void* stream) {
 // ---------------------------------------------------------------------------------------------------------
 static __device__ __align__(256) float g_noalloc_scratch[(MKDA_NOALLOC_MAX_ROWS / 64) * 128];
 static_assert(MKDA_NOALLOC_MAX_ROWS / 64 >= MKDA_EPILOGUE_MAX_PART_ROWS, "the built-in scratch must hold every partial row");
-static float* g_noalloc_ptr[64] = {nullptr};          // device address of the scratch, per device ordinal
+static std::atomic<float*> g_noalloc_ptr[64];          // device address of the scratch, per device ordinal
 
 static int noalloc_scratch(float** out) {
     int dev = -1;
