@@ -424,6 +424,11 @@ const char* mkda_last_error(void);
 unsigned long long mkda_launch_count(void);
 int mkda_abi_version(void);
 /* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header. */
+#define MKDA_STRUCTS(X) \
+    X(MkdaLayout) X(MkdaGateFwd) X(MkdaGateBwd) X(MkdaReduce) X(MkdaReduceMulti) X(MkdaL2Norm) \
+    X(MkdaIntraFwd) X(MkdaRecurFwd) X(MkdaOutFwd) X(MkdaChainFwd) X(MkdaStepFwd) X(MkdaEpilogueBwd) \
+    X(MkdaEpilogueBwdTiles) X(MkdaEpilogueBwdNoAlloc) X(MkdaBwdDh) X(MkdaBwdChunk) X(MkdaQkGrad) X(MkdaCombine) \
+    X(MkdaWarmup) X(MkdaSelfTest) X(MkdaSelfTestWait)
 int mkda_struct_sizes(int* out, int n);
 
 #ifdef __cplusplus

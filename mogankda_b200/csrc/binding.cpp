@@ -272,4 +272,15 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "host path of a layer call
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+#define MKDA_SIZE(S) (int)sizeof(S),
+    const int built[] = {MKDA_STRUCTS(MKDA_SIZE)};
+    constexpr int n = sizeof(built) / sizeof(built[0]);
+    int have[n];
+    if (mkda_struct_sizes(have, n) != n || !std::equal(have, have + n, built)) {
+        PyErr_SetString(PyExc_ImportError, "_host.so and libmkda.so were built from different include/mkda.h (struct sizes differ): rebuild with "
+                                           "`python -m mogankda_b200.build --force`");
+        return nullptr;
+    }
+    return PyModule_Create(&module);
+}

@@ -135,11 +135,8 @@ extern "C" const char* mkda_last_error(void) { return mkda::g_err; }
 extern "C" unsigned long long mkda_launch_count(void) { return mkda::g_launches.load(std::memory_order_relaxed); }
 extern "C" int mkda_abi_version(void) { return 4; }
 extern "C" int mkda_struct_sizes(int* out, int n) {
-    const int sizes[] = {
-        (int)sizeof(MkdaLayout),   (int)sizeof(MkdaGateFwd),  (int)sizeof(MkdaGateBwd),     (int)sizeof(MkdaReduce), (int)sizeof(MkdaReduceMulti),
-        (int)sizeof(MkdaL2Norm),   (int)sizeof(MkdaIntraFwd), (int)sizeof(MkdaRecurFwd),    (int)sizeof(MkdaOutFwd), (int)sizeof(MkdaChainFwd), (int)sizeof(MkdaStepFwd),
-        (int)sizeof(MkdaEpilogueBwd), (int)sizeof(MkdaEpilogueBwdTiles), (int)sizeof(MkdaEpilogueBwdNoAlloc), (int)sizeof(MkdaBwdDh), (int)sizeof(MkdaBwdChunk),
-        (int)sizeof(MkdaQkGrad),   (int)sizeof(MkdaCombine), (int)sizeof(MkdaWarmup), (int)sizeof(MkdaSelfTest), (int)sizeof(MkdaSelfTestWait)};
+#define MKDA_SIZE(S) (int)sizeof(S),
+    const int sizes[] = {MKDA_STRUCTS(MKDA_SIZE)};
     const int cnt = (int)(sizeof(sizes) / sizeof(sizes[0]));
     for (int i = 0; i < n && i < cnt; ++i) out[i] = sizes[i];
     return cnt;

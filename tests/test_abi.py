@@ -117,3 +117,19 @@ def test_modules_share_the_cxx_runtime_of_the_process(lib, name):
     symbols = subprocess.run(["nm", "-D", "--defined-only", path], capture_output=True, text=True, check=True).stdout
     assert "libstdc++.so.6" in needed
     assert "_ZNSo9_M_insertIlEERSoT_" not in symbols          # std::ostream::_M_insert<long>
+
+
+def test_a_host_module_of_another_header_is_refused(lib, tmp_path):
+    """_host.so has the struct layouts compiled in: against a library with others (here a preloaded mkda_struct_sizes that reports others) the
+    import has to fail."""
+    import subprocess
+    import sys
+    src, so = tmp_path / "other.c", tmp_path / "other.so"
+    src.write_text("int mkda_struct_sizes(int* out, int n) { for (int i = 0; i < n; ++i) out[i] = 8; return n; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(src), "-o", str(so)], check=True)
+    code = ("import torch, importlib.util\nspec = importlib.util.spec_from_file_location('mogankda_b200._host', 'mogankda_b200/_host.so')\n"
+            "importlib.util.module_from_spec(spec)")
+    for preload, ok in (("", True), (str(so), False)):
+        run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, LD_PRELOAD=preload), capture_output=True, text=True)
+        assert (run.returncode == 0) == ok, run.stderr
+        assert ok or "struct sizes differ" in run.stderr
