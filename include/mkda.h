@@ -94,7 +94,6 @@ int mkda_reduce_multi(const MkdaReduceMulti* p, void* stream);
 typedef struct {
     const void* x; int dtype; int rows; float eps;
     float* rstd;
-    const void* x2; float* rstd2;                  /* a second tensor of the same type and number of rows (q and k), or NULL */
 } MkdaL2Norm;
 int mkda_l2norm_rstd(const MkdaL2Norm* p, void* stream);
 

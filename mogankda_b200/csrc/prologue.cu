@@ -289,14 +289,12 @@ __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
     follow_stream();
     const int lane = threadIdx.x & 31, sub = lane & 15;
     const int row0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + (lane >> 4);
-    const void* x = blockIdx.y ? p.x2 : p.x;
-    float* rstd = blockIdx.y ? p.rstd2 : p.rstd;
     float4 a[4], b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = row0 + 2 * i, rr = row < p.rows ? row : p.rows - 1;
-        a[i] = ld4(x, DT, (size_t)rr * 128 + 8 * sub);
-        b[i] = ld4(x, DT, (size_t)rr * 128 + 8 * sub + 4);
+        a[i] = ld4(p.x, DT, (size_t)rr * 128 + 8 * sub);
+        b[i] = ld4(p.x, DT, (size_t)rr * 128 + 8 * sub + 4);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -304,7 +302,7 @@ __global__ void __launch_bounds__(128) l2norm_rstd_kernel(const MkdaL2Norm p) {
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         const int row = row0 + 2 * i;
-        if (sub == 0 && row < p.rows) rstd[row] = 1.f / sqrtf(ss + p.eps);
+        if (sub == 0 && row < p.rows) p.rstd[row] = 1.f / sqrtf(ss + p.eps);
     }
 }
 
@@ -652,10 +650,9 @@ extern "C" int mkda_reduce_partials(const MkdaReduce* p, void* stream) {
 
 extern "C" int mkda_l2norm_rstd(const MkdaL2Norm* p, void* stream) {
     if (!p || !p->x || !p->rstd) return set_error(MKDA_ERR_ARG, "l2norm_rstd: null argument");
-    if (any_misaligned(p->x, p->x2)) return set_error(MKDA_ERR_ARG, "l2norm_rstd: x must be 16-byte aligned");
-    if (p->x2 && !p->rstd2) return set_error(MKDA_ERR_ARG, "l2norm_rstd: null argument");
+    if (any_misaligned(p->x)) return set_error(MKDA_ERR_ARG, "l2norm_rstd: x must be 16-byte aligned");
     if (p->rows == 0) return MKDA_OK;
-    const dim3 grid((p->rows + 31) / 32, p->x2 ? 2 : 1);
+    const int grid = (p->rows + 31) / 32;
     switch (p->dtype) {
         case MKDA_F32: launch(l2norm_rstd_kernel<MKDA_F32>, grid, 128, 0, (cudaStream_t)stream, *p); break;
         case MKDA_BF16: launch(l2norm_rstd_kernel<MKDA_BF16>, grid, 128, 0, (cudaStream_t)stream, *p); break;
