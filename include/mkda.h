@@ -197,12 +197,13 @@ int mkda_chain_fwd(const MkdaChainFwd* p, void* stream);
 
 /* Forward pass over sequences of at most MKDA_STEP_MAX_TOKENS tokens (generation steps): gate, L2 norm, recurrence, output and epilogue in one
  * kernel, token by token, with the state in registers.  Same results as the chunk kernels up to rounding; nothing is kept for a backward
- * pass. */
+ * pass.  A sequence's results depend on that sequence only. */
 #define MKDA_STEP_MAX_TOKENS 16
 typedef struct {
     MkdaLayout L;
     int N; const int* seq_chunk_off;               /* sequences; [N+1] first chunk of each (at most one chunk per sequence) */
     int longest;                                   /* tokens of the longest sequence */
+    int short_only;                                /* 1: longer (and empty) sequences are left alone, out and ht of theirs included */
     const void* q; const void* k; const void* v; int qkv_dtype;
     const void* x; int x_dtype; int scalar_gate;   /* gate input as in MkdaGateFwd */
     const float* A_log; const float* dt_bias; int mode; float lower_bound;

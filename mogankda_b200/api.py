@@ -144,9 +144,10 @@ def chunk_delta_rule(q, k, v, g, beta, *, scale=None, initial_state=None, output
     unless ``gate_mode="precomputed"``, then the natural-log per-token decay, contract g >= -5); beta [B,T,HV].
     Returns ``(o, final_state)``: o in q.dtype, or float32 when ``output_norm`` is given.
 
-    A forward-only call that continues running sequences (``initial_state``) by at most 16 tokens is computed token by token, which
-    agrees with the chunked computation to rounding; every other call gives a prefix of a sequence bit for bit what the same tokens give
-    inside the longer sequence.
+    A sequence that a forward-only call (no gradient wanted) continues from its ``initial_state`` by at most 16 tokens is computed token by
+    token, which agrees with the chunked computation to rounding.  That holds for each sequence by itself: its results do not depend on what
+    else is in the batch, but their last bits do depend on whether gradients are wanted, and they are not those of the same tokens inside a
+    longer continuation.  Everything else gives a prefix of a sequence bit for bit what the same tokens give inside the longer sequence.
     """
     if cp_context is not None and getattr(cp_context, "cu_seqlens", None) is not None:
         cu_seqlens = cp_context.cu_seqlens      # the context's local boundaries replace the argument (reference :87-120)

@@ -177,7 +177,7 @@ PyObject* check_params(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all, longest, chain), scale, want_ht,
+// layer(q, k, v, g, beta, A_log, dt_bias, initial_state, norm weight, norm gate, tables, (NC, NS, N, segmented, covers_all, longest, chain, few), scale, want_ht,
 //       v_first, gate mode, lower bound or None, beta sigmoid, beta scale, l2, act or None, eps, warm-up threshold or None) -> (o, ht or None)
 PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -190,7 +190,7 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!tensor_arg(a[10], tables)) return nullptr;
     Call c;
     int seg, all;
-    if (!PyArg_ParseTuple(a[11], "iiiiiii", &c.NC, &c.NS, &c.N, &seg, &all, &c.longest, &c.chain)) return nullptr;
+    if (!PyArg_ParseTuple(a[11], "iiiiiiii", &c.NC, &c.NS, &c.N, &seg, &all, &c.longest, &c.chain, &c.few)) return nullptr;
     c.segmented = seg; c.covers_all = all;
     c.B = (int)in.q.size(0); c.T = (int)in.q.size(1); c.HK = (int)in.q.size(2); c.HV = (int)in.v.size(2); c.TT = c.B * c.T;
     c.dev = in.q.device();
@@ -239,10 +239,14 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         {
             at::AutoGradMode off(false);
             // Running sequences continued by a handful of tokens, nothing to differentiate: the recurrence itself is cheaper than a 64-row chunk
-            // (one token: 9 instead of 63 us of kernels at 8 sequences x 32 heads).  Calls that start from zero keep to the chunk algebra, whose
-            // results for a prefix of a sequence are those of the whole sequence bit for bit.
-            const bool step = !any && in.h0.defined() && c.longest <= MKDA_STEP_MAX_TOKENS && c.N <= 65535;
-            std::tie(out, ht) = library_call([&] { return step ? run_step(c, in) : run_forward(c, in, any, *saved); });
+            // (step.cu).  The choice is made for each sequence by itself, so that its results do not depend on what else is in the batch: in
+            // a mixed batch the steps go over the chunk kernels' results.  Sequences that start from zero keep to the chunk algebra, whose results
+            // for a prefix of a sequence are those of the whole sequence bit for bit.
+            const bool steps = !any && in.h0.defined();
+            library_call([&] {
+                if (!steps || c.longest > MKDA_STEP_MAX_TOKENS) std::tie(out, ht) = run_forward(c, in, any, *saved);
+                if (steps && (!out.defined() || c.few)) run_step(c, in, out, ht);
+            });
         }
         if (any) {
             node->call = c;

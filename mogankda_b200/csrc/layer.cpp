@@ -80,11 +80,14 @@ bool output_in_chain(const Call& c, bool need_bwd) {
 
 }  // namespace
 
-std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in) {
+void run_step(const Call& c, const Inputs& in, Tensor& out, Tensor& ht) {
     const Tensor alog = aligned_f32(in.A_log), bias = aligned_f32(in.dt_bias), w = aligned(in.ep_w);
-    Tensor out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type()), ht;
-    if (c.want_ht) ht = c.states(c.N);
     MkdaStepFwd p{};
+    p.short_only = out.defined();
+    if (!out.defined()) {
+        out = c.rows_out(c.HV, c.has_ep ? at::kFloat : in.q.scalar_type());
+        if (c.want_ht) ht = c.states(c.N);
+    }
     p.L = c.layout(); p.N = c.N; p.seq_chunk_off = c.seq_off; p.longest = c.longest;
     p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
     p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate; p.A_log = fptr(alog); p.dt_bias = fptr(bias);
@@ -96,7 +99,6 @@ std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in) {
     }
     p.out = out.data_ptr(); p.out_dtype = dtype_code(out);
     check_rc(mkda_step_fwd(&p, c10::cuda::getCurrentCUDAStream()), "mkda_step_fwd");
-    return {out, ht};
 }
 
 std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need_bwd, Saved& s) {

@@ -54,7 +54,7 @@ struct Arena {
 
 // Options and geometry of a call.
 struct Call {
-    int B, T, HK, HV, N, NC, NS, TT, longest, chain;
+    int B, T, HK, HV, N, NC, NS, TT, longest, chain, few;          // few: sequences of 1 to MKDA_STEP_MAX_TOKENS tokens
     bool segmented, covers_all, scalar_gate, l2, vf, want_ht, beta_sigmoid, has_ep, warm;
     int mode, act, qkv_dtype;
     float scale, lower_bound, beta_scale, eps, warm_log2;
@@ -92,7 +92,8 @@ struct Saved {
 struct Inputs { Tensor q, k, v, x, beta, A_log, dt_bias, h0, ep_w, ep_gate; };
 struct Grads { Tensor q, k, v, x, beta, A_log, dt_bias, h0, ep_w, ep_gate; };
 
-std::pair<Tensor, Tensor> run_step(const Call& c, const Inputs& in);
+// Every sequence token by token (undefined `out`: allocated here), or only those of a few tokens over the results of run_forward.
+void run_step(const Call& c, const Inputs& in, Tensor& out, Tensor& ht);
 std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need_bwd, Saved& s);
 Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor dht, bool need_alog, bool need_bias, bool need_h0);
 

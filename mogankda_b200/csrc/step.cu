@@ -5,6 +5,8 @@
 // everything in between, gate and L2 norm included, stays on chip.
 // What bounds it: 128 KB of state traffic per CTA.  The chunk path spends the same traffic several times over (operand tiles of 64 rows of
 // which a few are real, and five launches): 63 us of kernels for one token of 8 sequences x 32 heads, against 9 us here (33.5 MB of states).
+// Up to how many tokens: a token costs 1.6 us there, a chunk the same for any number of rows.  16 tokens, whole call with cold caches, here
+// and by chunks: 43 / 52 us (8 sequences x 32 heads), 221 / 316 us (64 x 32), 29 / 30 us (1 x 32); one token 18 / 50, 80 / 306, 14 / 30.
 #include "common.cuh"
 #include "gate.cuh"
 #include "host.h"
@@ -26,12 +28,13 @@ __device__ __forceinline__ float warp_sum_f(float x) {
 __global__ void __launch_bounds__(256, 2) step_fwd_kernel(const MkdaStepFwd p) {
     follow_stream();
     __shared__ __align__(16) StepShared sh;
-    const int h = blockIdx.x, n = blockIdx.y, HV = p.L.HV, HK = p.L.HK, hk = h / (HV / HK);
+    const int HV = p.L.HV, HK = p.L.HK, n = blockIdx.x / HV, h = blockIdx.x - n * HV, hk = h / (HV / HK);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int vi = tid & 127, half = tid >> 7;
     const int c = p.seq_chunk_off[n];
-    const bool any = p.seq_chunk_off[n + 1] > c;           // an empty sequence hands its state through
-    const int start = any ? p.L.chunk_start[c] : 0, len = any ? p.L.chunk_len[c] : 0;
+    const int chunks = p.seq_chunk_off[n + 1] - c;         // an empty sequence hands its state through
+    const int start = chunks ? p.L.chunk_start[c] : 0, len = chunks ? p.L.chunk_len[c] : 0;
+    if (p.short_only && (chunks != 1 || len > STEP_MAX)) return;
 
     // the state: 64 loads in flight per thread while the tokens are prepared
     float S[64];
@@ -146,11 +149,10 @@ extern "C" int mkda_step_fwd(const MkdaStepFwd* p, void* stream) {
     if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "step_fwd: HV must be a multiple of HK");
     if (p->has_norm && !p->gate) return set_error(MKDA_ERR_ARG, "step_fwd: the gated norm needs a gate tensor");
     if (p->mode != MKDA_GATE_PRECOMPUTED && !(p->lower_bound < 0.f)) return set_error(MKDA_ERR_ARG, "step_fwd: lower_bound must be < 0");
-    if (p->longest > STEP_MAX) return set_error(MKDA_ERR_ARG, "step_fwd: a sequence is longer than MKDA_STEP_MAX_TOKENS");
+    if (!p->short_only && p->longest > STEP_MAX) return set_error(MKDA_ERR_ARG, "step_fwd: a sequence is longer than MKDA_STEP_MAX_TOKENS");
     for (int dt : {p->qkv_dtype, p->x_dtype, p->beta_dtype, p->out_dtype})
         if (dt < MKDA_F32 || dt > MKDA_F16) return set_error(MKDA_ERR_ARG, "step_fwd: unsupported dtype");
     if (p->N == 0 || p->L.HV == 0) return MKDA_OK;
-    if (p->N > 65535) return set_error(MKDA_ERR_ARG, "step_fwd: too many sequences");
-    launch(step_fwd_kernel, dim3(p->L.HV, p->N), 256, 0, (cudaStream_t)stream, *p);
+    launch(step_fwd_kernel, p->N * p->L.HV, 256, 0, (cudaStream_t)stream, *p);
     return check_launch("step_fwd");
 }

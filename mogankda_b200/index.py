@@ -13,6 +13,8 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from ._lib import ENUMS
+
 CHUNK = 64
 
 
@@ -35,7 +37,8 @@ class Layout:
     covers_all: bool            # every token of [0, B*T) belongs to a sequence
     host: dict = field(default_factory=dict)
     tables: torch.Tensor = None  # int32: the seven tables above, one after the other (what the native host path takes)
-    dims: tuple = ()            # (NC, NS, N, segmented, covers_all, tokens of the longest sequence, chunks of the longest segment)
+    dims: tuple = ()            # (NC, NS, N, segmented, covers_all, tokens of the longest sequence,
+    #                             chunks of the longest segment, sequences of 1 to MKDA_STEP_MAX_TOKENS tokens)
 
     @property
     def TT(self):
@@ -129,8 +132,8 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
     if lay is not None:
         return lay
     cu = None if cu_seqlens is None else [int(x) for x in cu_seqlens.tolist()]
+    lens = [T] * B if cu is None else [e - s for s, e in zip(cu[:-1], cu[1:])]
     if auto_heads > 0:
-        lens = [T] * B if cu is None else [e - s for s, e in zip(cu[:-1], cu[1:])]
         if not wants_segments([-(-n // CHUNK) for n in lens], auto_heads, seg_chunks, _sm_count(device) if str(device) != "cpu" else None,
                               cost_ratio):
             seg_chunks = 0
@@ -142,13 +145,14 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
         at[n] = (len(flat), len(tb[n]))
         flat += tb[n] + [0] * (-len(tb[n]) % 4)
     tables = torch.tensor(flat or [0], dtype=torch.int32, device=device)
-    longest = T if cu is None else max((e - s for s, e in zip(cu[:-1], cu[1:])), default=0)
+    longest = T if cu is None else max(lens, default=0)
+    few = sum(0 < n <= ENUMS["MKDA_STEP_MAX_TOKENS"] for n in lens)
     so = tb["seg_chunk_off"]
     chain = max((b - a for a, b in zip(so[:-1], so[1:])), default=0)
     part = {n: tables[o:o + m] for n, (o, m) in at.items()}
     NC, NS, segmented = len(tb["chunk_start"]), len(tb["seg_first"]), len(tb["seg_first"]) != tb["N"]
     lay = Layout(B=B, T=T, N=tb["N"], NC=NC, NS=NS, NG=tb["N"], segmented=segmented, covers_all=tb["covers_all"], host=tb, tables=tables,
-                 dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"]), longest, chain), **part)
+                 dims=(NC, NS, tb["N"], int(segmented), int(tb["covers_all"]), longest, chain, few), **part)
     with _cache_lock:
         if len(_cache) >= _CACHE_MAX:
             _cache.pop(0)

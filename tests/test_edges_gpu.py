@@ -299,3 +299,23 @@ def test_errors_of_the_library_are_mkda_errors():
         with torch.no_grad(), pytest.raises(_lib.MkdaError, match="lower_bound"):
             mk.chunk_kda(cut["q"], cut["k"], cut["v"], cut["g"], cut["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"], initial_state=h0,
                          **dict(opts, lower_bound=1.0))
+
+
+@pytest.mark.parametrize("epi", [None, "silu"])
+@pytest.mark.parametrize("vfirst", [False, True])
+def test_a_short_continuation_does_not_depend_on_the_rest_of_the_batch(epi, vfirst):
+    """Forward-only calls with states: sequences of 0, 1, 5, 16 (token by token), 17, 40 and 100 tokens (chunks) packed together and padding behind
+    them give the bits that each gives alone."""
+    cu = (0, 5, 45, 45, 46, 62, 79, 179)
+    lv, do, dht, opts, _ = make_inputs(cu=cu, T=183, HK=2, HV=4, dtype=torch.bfloat16, gate="eda", epi=epi, seed=131)
+    alone = dict(opts, cu_seqlens=None)
+    got = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=vfirst, grads=False)
+    assert (got["o"][:, 179:] == 0).all()
+    for n, (a, b) in enumerate(zip(cu[:-1], cu[1:])):
+        if a == b:
+            h0 = lv["h0"][n].transpose(-1, -2) if vfirst else lv["h0"][n]
+            assert torch.equal(got["ht"][n], h0)
+            continue
+        sub = {m: (t[n:n + 1] if m == "h0" else t[:, a:b].contiguous() if t.dim() >= 3 else t) for m, t in lv.items()}
+        one = run(mk.chunk_delta_rule, sub, do[:, a:b], dht[n:n + 1], alone, epi, vfirst=vfirst, grads=False)
+        assert torch.equal(got["o"][:, a:b], one["o"]) and torch.equal(got["ht"][n:n + 1], one["ht"]), (n, b - a)
