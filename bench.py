@@ -126,23 +126,22 @@ def layer_step(mk, dev, opts, cp=None):
 # precision-split or recompute multipliers, no triangular discount) and algorithmic bytes of the streaming kernels.
 # ----------------------------------------------------------------------------------------------------------
 C_, K_, V_ = 64, 128, 128
-F_CK, F_KV, F_CC = 2 * C_ * K_, 2 * K_ * V_, 2 * C_ * C_
+F_CK, F_KV = 2 * C_ * K_, 2 * K_ * V_
 KERNEL_FLOPS = {                      # per token per v-head
     "mkda_intra_fwd": 3 * F_CK,                       # Gamma, Q K^T, A (beta [k~ | v]) counted as one C x C x (K|V) product pair
     "mkda_recur_fwd": 2 * F_KV,                       # nw S, kbar^T Vd
     "mkda_out_fwd": F_KV + F_CK,                      # q~ S, Aqk Vd
     "mkda_chain_fwd": 3 * F_KV + F_CK,                # both in one kernel
     "mkda_bwd_dh": F_CK + 3 * F_KV,                   # Aqk^T dO, kbar dS', q~^T dO, nw^T dVd
-    # k~ S, dO Vd^T, A^T dVd, dVd W^T, two C^3 products (Vd comes from the forward pass); dO S^T, dX S^T, Vd dS'^T; row / column
-    # terms through Gamma and Q K^T
-    "mkda_bwd_chunk": 4 * F_KV + 7 * F_CK + 2 * F_CC,
+    # A^T dVd, dO Vd^T, dW Vd^T; dO S^T, dW S^T, Vd dS'^T; row and column terms through Gamma and Q K^T
+    "mkda_bwd_chunk": 3 * F_KV + 7 * F_CK,
 }
 # Algorithmic bytes per token per v-head: each kernel's own tensor I/O at the default workload (bf16 q/k/v/gate,
 # fp32 intermediates, HV = 2 HK), every operand counted once.
 KERNEL_BYTES = {
     "mkda_gate_cumsum_fwd": 1024, "mkda_l2norm_rstd": 128, "mkda_intra_fwd": 3592, "mkda_recur_fwd": 3080,
     "mkda_out_fwd": 3584, "mkda_chain_fwd": 5128, "mkda_epilogue_bwd_tiles": 2048, "mkda_epilogue_bwd": 2048, "mkda_bwd_dh": 3848,
-    "mkda_bwd_chunk": 6152, "mkda_gate_bwd": 1536, "mkda_qk_grad_finish": 1024,      # dq / dk tiles are per q/k head: 512 B per v-head
+    "mkda_bwd_chunk": 6408, "mkda_gate_bwd": 1536, "mkda_qk_grad_finish": 1024,      # dq / dk tiles are per q/k head: 512 B per v-head
 }
 def load_kernel_traffic(path=os.path.join(ROOT, "profiles", "counters_per_kernel_1b_shape.md")):
     """DRAM traffic per token per v-head of every kernel, read from the committed ncu summary (its table has the columns

@@ -423,7 +423,8 @@ const char* mkda_last_error(void);
 /* kernel launches issued by this process through the library so far */
 unsigned long long mkda_launch_count(void);
 int mkda_abi_version(void);
-/* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header. */
+/* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header: the sizes, not the version
+ * above, tell one build's layouts from another's. */
 #define MKDA_STRUCTS(X) \
     X(MkdaLayout) X(MkdaGateFwd) X(MkdaGateBwd) X(MkdaReduce) X(MkdaReduceMulti) X(MkdaL2Norm) \
     X(MkdaIntraFwd) X(MkdaRecurFwd) X(MkdaOutFwd) X(MkdaChainFwd) X(MkdaStepFwd) X(MkdaEpilogueBwd) \

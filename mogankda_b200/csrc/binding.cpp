@@ -2,7 +2,8 @@
 //
 // Why native: on a short sequence a call is nothing but launches.  Driving the C ABI from Python (ctypes structs, a dozen torch.empty
 // calls, a Python autograd function) took 145 us per forward and 380 us per forward + backward of a 77- / 256-token call whose kernels
-// need 45 / 120 us.
+// need 45 / 120 us.  A C++ node has none of the checks of a Python autograd function: saved-tensor hooks, forward-mode AD and a second
+// differentiation are seen to below.
 #include <Python.h>
 
 #include "layer.h"

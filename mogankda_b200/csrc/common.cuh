@@ -1,9 +1,9 @@
 // Shared device helpers for the KDA / GDN kernels (sm_100a).
 //
-// Numerics policy: every contraction runs on the tensor cores with the error-compensated three-product split
-// (a = hi + lo, a*b ~ lo_a*hi_b + hi_a*lo_b + hi_a*hi_b) and fp32 accumulation: bf16 halves on tcgen05 in the chunk
-// kernels (umma.cuh), TF32 halves on mma.sync in the small prefix-combine kernel (PREC = 3 below; PREC = 1 is the plain
-// single product).  Inputs may be fp32, bf16 or fp16 in global memory; they are widened to fp32 when staged.
+// Numerics policy: the contractions of the chunk kernels run on the tensor cores with the error-compensated three-product split
+// (a = hi + lo, a*b ~ lo_a*hi_b + hi_a*lo_b + hi_a*hi_b) and fp32 accumulation: bf16 halves on tcgen05 (umma.cuh), and TF32 halves on
+// mma.sync in the 16- and 32-row merges of the triangular inverse (warp_mma_short below).  The prefix combine and the step kernel are plain
+// fp32.  Inputs may be fp32, bf16 or fp16 in global memory; they are widened to fp32 when staged.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

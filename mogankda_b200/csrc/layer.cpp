@@ -1,4 +1,4 @@
-// Launches of one layer call: gate + cumsum (+ beta) -> L2 statistics -> WY preparation -> state pass -> output, and the backward
+// Launches of one layer call: gate + cumsum (+ beta) -> L2 statistics and WY preparation -> state pass and output, and the backward
 // pass.  Every intermediate is a torch allocation on the current stream.
 #include "layer.h"
 

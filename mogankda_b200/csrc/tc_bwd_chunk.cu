@@ -7,7 +7,7 @@
 //   dL = -strictlower(dW Vd^T): one product of tiles that exist anyway, instead of rebuilding X and a chain of three products.
 //   dbeta_i = (dW X^T)_ii + (dL Gamma^T)_ii = rowsum(dW * V) - rowsum(k~ * (dW S^T)) + rowsum(k * T).  (It also is (dW Vd^T)_ii / beta_i, the
 //   diagonal of the product above, for nothing; but Vd carries the errors of the state chain where V is exact: over 50 cases that came to 1.16
-//   times the error against fp64, up to 6.4e-6 instead of 3.7e-6.  So V is read (213 -> 228 us at the 1B shape, 262 -> 273 on short documents),
+//   times the error against fp64, up to 6.4e-6 instead of 3.7e-6.  So V is read (213 -> 228 us at the 1B shape, 3.15 -> 3.37 ms on 64k packed tokens),
 //   and what the bf16 halves leave of dW, 2.4e-6 of the sum, is kept as a third part.)
 // State part (up = 2^g, rest = 2^(g_L - g)):
 //   dq_p = scale (dO S^T) up         dk_p = -beta (dW S^T) up + (Vd dS'^T) rest        dgl = rowsum_v(S * dS')
@@ -36,8 +36,8 @@
 // behind 208 KB of copies: 6 k cycles at the top of every item and as much in the epilogue).  The products' operand reads, the copies and the
 // compute warps' own accesses share the 128 B per cycle of shared memory: some 23 k cycles of the 25 k an item takes.
 // dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
-// 64k packed tokens x 32 heads: 3.80 -> 3.25 ms by that, by operand descriptors that no longer spill in the issuing warp, by row scalars
-// read four at a time and by the L2 hint in the copy warp; 4 x 16k x 16 heads, scalar gate: 1355 -> 1250 us.
+// 64k packed tokens x 32 heads: 3.80 -> 3.25 ms (3.37 with the reading of V) by that, by operand descriptors that no longer spill in the issuing warp, by row scalars
+// read four at a time and by the L2 hint in the copy warp; 4 x 16k x 16 heads, scalar gate: 1355 -> 1250 us (1275).
 // Shared memory (KB): S [0,64) -> [Qr; beta Kr] | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> Kc_0, Kc_1 in the dO pieces, raw k
 // and q rows in the dW pieces | Vd^T [128,160) -> Kc_3 | dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Wq; dLs] [160,192), Kc_2 [192,216),
 // scratch [216,224).

@@ -91,7 +91,9 @@ def wants_segments(chunks_per_seq, HV, seg_chunks, sm_count=None, cost_ratio=2.5
     set by the longest sequence (critical path) unless there is so much work that the even share of all chunk steps over
     the SMs is longer still.  Cutting spreads the steps evenly but adds the state + transition pre-pass in the forward
     direction and a second pass in the backward direction, about 2.5 x the serial work over a layer step, plus the prefix
-    combine.  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
+    combine.  (The 2.5 was measured with earlier serial kernels.  With today's, counters at 45 + 42 + 42 chunks x 16 heads give 444 us for
+    the cut calls against an estimate of 310 uncut, at the kernels' 3.2 + 3.7 us per chunk: the line lies too low for few heads and
+    sequences of 33 to about 75 chunks.)  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
     warm-up truncation, which shortens the two extra passes to a few chunks wherever the gate decays).  Decided from the
     lengths alone (host), never from data; it plays the role of the reference's intra-card CP decision
     (mogan_kda/ops/gated_delta_rule/chunk/cp/context.py:252-283, cp/autocp/decision.py:54-123)."""

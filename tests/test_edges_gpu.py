@@ -68,8 +68,8 @@ def test_states_at_odd_storage_offsets(offset):
     dict(B=1, T=9, gate="precomputed", beta="precomputed", l2=False, dtype=torch.float32, epi=None, h0=False),
     dict(B=2, T=4, gate="eda", dtype=torch.bfloat16, epi="silu", x_dtype=torch.bfloat16)], ids=str)
 def test_forward_of_very_short_sequences(case):
-    """Without gradients and with an initial state, sequences of up to 16 tokens run token by token (17: the chunk kernels); empty sequences, padding and 4 v-heads on
-    2 q/k heads included."""
+    """Without gradients and with an initial state, sequences of up to 16 tokens run token by token; 17 tokens, and a sequence that starts from
+    zero, take the chunk kernels.  Empty sequences, padding and 4 v-heads on 2 q/k heads included."""
     case = dict(case)
     vfirst = case.pop("vfirst", False)
     lv, do, dht, opts, epi = make_inputs(HK=2, HV=4, seed=47, **case)
