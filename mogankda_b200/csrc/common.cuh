@@ -236,6 +236,40 @@ __device__ __forceinline__ void warp_mma_short(float (&acc)[NT][4], const float*
         for (int e = 0; e < 4; ++e) acc[nt][e] += lh[nt][e] + hl[nt][e];
 }
 
+// acc[2][4] = A(16 x 16) * B(16 x 16) for one warp with A as the accumulators of an earlier product (its columns 2 t, 2 t + 1 of every eight
+// taken as the terms t, t + 4), B(k, n) = B[k * ld + n]
+__device__ __forceinline__ void warp_mma_chained(float (&acc)[2][4], const float (&A)[2][4], const float* __restrict__ B, int ld) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    FragA fa[2];
+    FragB fb[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        fa[k].set(0, A[k][0]); fa[k].set(1, A[k][2]); fa[k].set(2, A[k][1]); fa[k].set(3, A[k][3]);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            fb[k][nt].set(0, B[(8 * k + 2 * t) * ld + 8 * nt + g]);
+            fb[k][nt].set(1, B[(8 * k + 2 * t + 1) * ld + 8 * nt + g]);
+        }
+    }
+    float lh[2][4], hl[2][4];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) lh[nt][e] = hl[nt][e] = acc[nt][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            mma_tf32_raw(lh[nt], fa[k].lo, fb[k][nt].hi);
+            mma_tf32_raw(hl[nt], fa[k].hi, fb[k][nt].lo);
+            mma_tf32_raw(acc[nt], fa[k].hi, fb[k][nt].hi);
+        }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nt][e] += lh[nt][e] + hl[nt][e];
+}
+
 // Two fp32 operations in one instruction (a pair of registers each): the staging and epilogue code is bound by instruction issue.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float a, float b) {

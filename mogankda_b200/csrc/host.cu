@@ -43,7 +43,7 @@ int sm_count() {
 }
 
 int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what,
-                  int box_rows) {
+                  int box_rows, int box_cols) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static std::atomic<Encode> resolved{nullptr};      // through the runtime: the library does not link against the driver
@@ -66,9 +66,10 @@ int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned l
     }
     const cuuint64_t gdim[2] = {row_elems, rows};
     const cuuint64_t gstride[1] = {pitch};
-    const cuuint32_t box[2] = {128, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, estr[2] = {1, 1};
     const CUresult r = encode(out, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), gdim,
-                              gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         snprintf(g_err, sizeof(g_err), "%s: cuTensorMapEncodeTiled failed (%d)", what, (int)r);

@@ -16,10 +16,11 @@ int ensure_smem(const void* func, int bytes, const char* what);
 int kernel_registers(const void* func);
 // Tensor map over a row-major [rows][row_elems] tensor of 2- or 4-byte elements whose boxes are `box_rows` (64) rows x 128 elements,
 // not swizzled: one tiled TMA copy then brings 64 strided 128-element rows (token rows of one head) into shared memory as a dense
-// [64][128] block.  Rows past the end of the tensor read as zeros.  Returns 0, or an error code when the tensor cannot be
+// [64][128] block.  box_cols = 64 (2-byte elements): boxes of 64 elements with the 128-byte swizzle, a column block of an operand tile
+// (umma.cuh).  Rows past the end of the tensor read as zeros.  Returns 0, or an error code when the tensor cannot be
 // described (base not 16-byte aligned, row pitch not a multiple of 16 bytes, or the driver lacks the encoder).
 int make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, unsigned long long rows, unsigned long long row_elems, const char* what,
-                  int box_rows = 64);
+                  int box_rows = 64, int box_cols = 128);
 // True if any of the (possibly null) pointers is not 16-byte aligned: the kernels read and write their tensors with
 // 16-byte vector accesses and bulk copies, and a misaligned address would fault the device instead of returning an error.
 template <typename... P>

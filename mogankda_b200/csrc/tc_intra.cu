@@ -2,7 +2,7 @@
 //
 //   Gamma_ij = sum_c k_ic k_jc 2^(g_ic - g_jc)  (i > j)        Aqk_ij = scale sum_c q_ic k_jc 2^(g_ic - g_jc)  (i >= j)
 //   A  = (I + strictlower(diag(beta) Gamma))^-1
-//   nw = -A diag(beta) (k 2^g)                                  u = A diag(beta) v
+//   nw = -(A diag(beta)) (k 2^g)                                u = (A diag(beta)) v
 //
 // Range / prefix invariance: the per-channel decay 2^(g_i - g_j) does not factor out of the contraction over channels,
 // so each 16-row block I uses its first row a = 16 I as anchor: row operand k_i 2^(g_i - g_a) (<= 1), column operand
@@ -13,69 +13,354 @@
 // (their g as the last valid row's), so they produce identity rows in A and are never stored.
 //   row operand     Kr[i] = k_i 2^(48 + g_i - g_a(i)),  Qr[i] = q_i 2^(48 + g_i - g_a(i))      one tile for all 64 rows
 //   column operand  Kc_I[j] = k_j 2^(g_aI - g_j - 48),  j < 16 (I + 1)                         one tile per row block
-// What bounds it: the chain of phases of an item with one CTA per SM (18 k cycles; the item's own bytes take 8 k at 25 B per cycle).
-// Packed 6 k prefill x 32 heads 288 -> 236 us (with the L2 statistics, formerly a kernel), 32 k tokens 1373 -> 1120 us.
+//
+// What bounds it: the phases of an item depend on each other, and only one item's operands (144 KB) fit.  So the phases are split between two
+// groups of warps that work on neighbouring items:
+//   X, 16 warps, item n + 1: rows in -> operands -> (while [Gamma; Q K^T] is computed) L2 scales; nw, u of item n from their accumulators ->
+//                            kbar, scale q 2^g and k 2^g tiles
+//   Y, 4 or 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, A diag(beta)
+// and four warps of one working thread each: products of X, products of Y, copies of X, copies of Y.  All are joined by mbarriers.
+// beta is folded into A, so that v itself is the operand: 16-bit rows arrive by a swizzled tiled copy, bf16 ones as a ready-made tile
+// that needs one product less per k-step (it has no low half).
+// Shared memory is what X is then bound by (11 to 12 k of the 13 k cycles of an item, 18 k before, move operands, tiles and rows); with few items
+// the latency of an item counts, and twice as many warps in Y shorten it.
+// 6 k packed tokens x 32 heads 240 -> 196 us, 32 k tokens x 32 heads 1110 -> 825, scalar gate 4 x 2000 tokens x 16 heads 129 -> 89.
 #include "host.h"
 #include "intra.cuh"
 
+#include <string.h>
+
 namespace mkda {
 
-struct IntraShared {
-    uint64_t ldin, op1, op2;                               // rows landed | operands of the first, second products written (16 warps)
-    uint64_t mm1, mmN, mmU;                                // products done: [Gamma; Q K^T], nw^T, u^T
-    uint32_t tmem;
-    __align__(16) float beta[2][CH];                       // of this item and (arriving) the next
-    float rk[CH], rq[CH];                                  // L2 scales of the rows
-    __align__(16) float T[32][36];
+namespace in {
+constexpr int X_WARPS = 16;
+// YW warps of Y.  Registers of the launch, of X and of Y; the last four warps go down to 40 (the sums are those of the launch).
+template <int YW>
+struct Warps {
+    static constexpr int THREADS = 32 * (X_WARPS + YW + 4), LAUNCH_REGS = YW == 4 ? 80 : 72, X_REGS = LAUNCH_REGS + 8, Y_REGS = YW == 4 ? 88 : 72;
+    static_assert(X_WARPS * X_REGS + YW * Y_REGS + 4 * 40 <= (X_WARPS + YW + 4) * LAUNCH_REGS, "registers of the launch");
 };
-constexpr int TLD = 36;
-// 16 compute warps and one that issues the products (of a warpgroup of its own).  The tensor pipe accepts a product as slowly as it executes
-// them: the compute warp that issued used to come 1.4 k cycles after the others (of 19.7 k per item).  Registers as in bwd_chunk:
-// 16 x 32 x 112 + 4 x 32 x 32 = the 640 x 96 of the launch.
-constexpr int INTRA_THREADS = 640, INTRA_WARP_MMA = 16, INTRA_LAUNCH_REGS = 96;
-__device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-
-constexpr int MLD = 68;
 constexpr float ROW_UP = 0x1p48f, COL_DOWN = 0x1p-48f;      // column operand: 108 + 64 - 48 < 127, row operand: 64 + 48 < 127 for |k| < 2^64
 // the four column tiles stacked by rows into one 160-row tile (hi 40 KB, then lo)
-__host__ __device__ constexpr int kc_row(int I) { return I == 0 ? 0 : I == 1 ? 16 : I == 2 ? 48 : 96; }
-constexpr int KC_ALL_ROWS = 160;
-constexpr int KC_ALL_BYTES = KC_ALL_ROWS * 128 * 2;        // one of hi / lo
-constexpr int KQ_OFF = 81920;                              // [128][128] hi 32 KB, lo 32 KB
-constexpr int OPND_BYTES = KQ_OFF + 65536;                 // 144 KB
-constexpr int TA_OFF = 65536;                              // A, over the dead column tiles
-// The 16-bit k, q and the g rows of the NEXT item arrive by tiled copy (one 64 x 128 box per tensor) while the current item's
-// inverse and second products run: k and g rows in the upper 48 KB of the [Kr; Qr] tile, dead once the first products are
-// done, q rows over the kbar tile as soon as that has left.  They are read back into registers before the next item's operands are staged over them.  (Loads
-// into registers at that point are accepted only as fast as their data returns and occupied every thread for a fifth of
-// the item; one small bulk copy per row is slower still.)
-struct IntraMaps { CUtensorMap k, q, g; };
-constexpr int RAW_K = 98304;                               // [64][128] 16-bit, 16 KB
-constexpr int RAW_G = RAW_K + 16384;                       // [64][128] fp32, 32 KB
-constexpr int RAW_Q = OPND_BYTES;                          // [64][128] 16-bit, 16 KB, over the kbar tile
-constexpr int INTRA_TC_SMEM = OPND_BYTES + 32768 + 2 * CH * MLD * 4 + 1024;        // operands, kbar tile, scale q 2^g tile (later sM / sInv)
-static_assert(RAW_G + 32768 <= OPND_BYTES, "k / g rows must fit in the dead part of the operand region");
-static_assert(2 * CH * MLD * 4 >= 32768, "the scale q 2^g tile must fit below the end");
-constexpr int STORER = 256;                                // the thread that issues every bulk store: its warp has no part in the inverse
+__host__ __device__ constexpr int kc_row(int I) { return 8 * I * (I + 1); }
+constexpr int KC_ROWS = 160, KC_BYTES = KC_ROWS * 128 * 2;  // one of hi / lo
+constexpr int KQ = 2 * KC_BYTES;                            // [Kr; Qr] [128][128]: hi 32 KB, lo 32 KB
+// Over both once their products are done: the hand-over tiles kbar, scale q 2^g and Aqk of the item over the column tiles (written last, half
+// 0 in front of Aqk), the rows of the next one (dense [64][128] blocks) over [Kr; Qr].  fp32 rows do not fit: q waits until kbar has left.
+constexpr int KB = 0, QS = 32768, AQ = 65536, RAW_G = KQ;
+template <int DT, bool SCALAR>
+struct Rows {
+    static constexpr int BYTES = DT == MKDA_F32 ? 32768 : 16384, PITCH = BYTES / CH;
+    static constexpr bool LATE_Q = DT == MKDA_F32 && !SCALAR;
+    static constexpr int K = SCALAR ? KQ : KQ + 32768, Q = LATE_Q ? KB : K + BYTES;
+    static_assert(LATE_Q || Q + BYTES <= KQ + 65536, "rows of the next item");
+};
+// Y's own: k 2^g [j][K index] (then nw^T), v [j][v] (bf16: 16 KB) and A diag(beta) [i][j] (then u^T over both), the triangular matrix
+constexpr int BK = KQ + 65536, V_ = BK + 32768, AB = V_ + 16384, T_ = AB, UT = V_, M_ = AB + 16384;
+constexpr int LD = 36, MB = 32 * LD;                        // I + L as three 32 x 32 blocks: (0, 0), (1, 0), (1, 1)
+constexpr int TILES = M_ + 3 * MB * 4;
+constexpr int D1 = 0, D1_COLS = 160, NW = 320, U = 384;      // accumulator columns (two of [Gamma; Q K^T]: Y is an item behind)
 
-// Inverse of the unit lower-triangular 64 x 64 matrix sM into sInv (fixed summation order) by recursive halving:
-// the four 16 x 16 diagonal blocks by forward substitution, then the off-diagonal block of each 32 x 32 half and finally
-// the 32 x 32 block below the diagonal, each as  X = -B^-1 (C A^-1)  with A^-1 / B^-1 the inverses above / beside it.
-// Every entry depends on the rows up to its own only, and the order of the sums is fixed by the indices.  Blocks (0, 1) and (2, 3) have to
-// be zero on entry; the blocks further above the diagonal are not touched.
-// The merges are TF32 products with error compensation (three products, fp32 accumulation: ~2^-21 per product), one 16 x 8 tile per warp:
-// fragments need a quarter of the shared-memory loads of fp32 register tiles, which bounded them (1.05 k cycles per 32 x 32 product).
-__device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, float* __restrict__ sInv, IntraShared& sh) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    if (warp < 2) {
-        const int o = 32 * warp + (lane & 16), col = lane & 15;
+struct Shared {
+    uint64_t ldin, fullV;                                   // rows | v landed
+    uint64_t op1[2], mm1;                                   // operands of channel half 0, 1 written; [Gamma; Q K^T] done
+    uint64_t rows, acc, hand, khFree;                       // row scales | Aqk | kbar, scale q 2^g, k 2^g written; the first two tiles and Aqk have left
+    uint64_t opA, opV, mmV, mmN, mmU;                       // A diag(beta) written | (v in two halves: low half written, high half used) | nw^T, u^T done
+    uint64_t nwReady, uReady, bkFree, abFree;               // nw^T, u^T staged | have left
+    uint32_t tmem;
+    __align__(16) float beta[2][CH];                        // Y is an item behind
+    struct { int item, start, len, h, hk; } info[4];        // of the items, by the warp that requests their rows
+    __align__(16) float rs[2][CH], part[2][CH];             // L2 scales of the k, q rows (first the sums of half their channels); of the other half
+    // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
+    // threads of a row read them without bank conflicts.  2^(ga[I] - ga[I - 1]) of I = 2, 3
+    __align__(16) float ga[5][DK], step[2][DK];
+};
+constexpr int SMEM = TILES + (int)sizeof(Shared);
+static_assert(SMEM <= 232448, "shared memory of one CTA");
+
+struct Maps { CUtensorMap k, q, g, v; };
+
+__device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+template <int YW>
+__device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, %0;" :: "n"(32 * YW) : "memory"); }
+
+// The items of a CTA: gridDim.x apart, heads fastest (the threads that request copies walk them; the others read `info`).
+struct Walk {
+    int c, h, hk, start, len, dc, dh, HV, NC;
+    float rG;
+    const MkdaLayout& L;
+    __device__ __forceinline__ Walk(const MkdaLayout& l) : L(l) {
+        HV = l.HV; NC = l.NC;
+        c = blockIdx.x / HV; h = blockIdx.x - c * HV; dc = gridDim.x / HV; dh = gridDim.x - dc * HV;
+        rG = 1.f / (float)(HV / l.HK);
+        table();
+    }
+    __device__ __forceinline__ void table() {
+        hk = (int)(((float)h + 0.5f) * rG);
+        const int i = min(c, NC - 1);
+        start = L.chunk_start[i]; len = L.chunk_len[i];
+    }
+    __device__ __forceinline__ bool valid() const { return c < NC; }
+    __device__ __forceinline__ int item() const { return c * HV + h; }
+    __device__ __forceinline__ void next() {
+        c += dc; h += dh;
+        if (h >= HV) { h -= HV; ++c; }
+        table();
+    }
+};
+__device__ __forceinline__ int item_count(const MkdaLayout& L) { return (L.NC * L.HV - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x; }
+
+// eight consecutive floats by the threads c = 0..7 of a row: the two 16-byte halves in an order that keeps the eight off each other's banks
+__device__ __forceinline__ void lds8_swapped(const float* p, bool s, f32x2 (&v)[4]) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p + (s ? 4 : 0)), b = *reinterpret_cast<const ulonglong2*>(p + (s ? 0 : 4));
+    v[0] = s ? b.x : a.x; v[1] = s ? b.y : a.y; v[2] = s ? a.x : b.x; v[3] = s ? a.y : b.y;
+}
+template <int DT>
+__device__ __forceinline__ void lds_raw8(const uint8_t* row, int k8, Raw8& r) {
+    if (DT == MKDA_F32) {
+        r.a = *reinterpret_cast<const uint4*>(row + k8 * 32);
+        r.b = *reinterpret_cast<const uint4*>(row + k8 * 32 + 16);
+    } else {
+        r.a = *reinterpret_cast<const uint4*>(row + k8 * 16);
+    }
+}
+}  // namespace in
+
+// ---- X ----------------------------------------------------------------------------------------------------------------------------------
+// Thread: eight channels of the first half of row r = tid / 8 and eight of the second half of row r ^ 48: the products of channels 0..63 run
+// while the operands of 64..127 are written, and as a row of block B enters 4 - B column tiles, each thread writes five.
+// SCALAR: the gate is one decay per token (the same cumsum in all 128 channels).  It then commutes with the contraction
+// over channels, Gamma_ij = (k_i . k_j) 2^(g_i - g_j), so the products are plain K K^T / Q K^T (one product over a stacked
+// [K; Q] tile; bf16 rows have no low half) and the decay is applied to the accumulators, element by element and for i >= j only: nothing is
+// anchored, no exponent is ever positive, and any g <= 0 is in range (the per-channel path needs g >= -5 per token).
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, uint32_t tmem, in::Shared& sh) {
+    using namespace in;
+    using R = Rows<DT, SCALAR>;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c8 = tid & 7;
+    const bool odd = c8 & 4;
+    auto row_of = [&](int hf) { return hf ? (tid >> 3) ^ 48 : tid >> 3; };
+    uint8_t* sKQ = base + KQ;
+    // nw^T [K index][tok] and u^T [v][tok] of an item leave as ready-made chunk tiles over their operands (the serial kernels fetch them with one
+    // bulk copy; token columns past the end are exact zeros: beta is 0 there)
+    auto read_out = [&](int it) {
+        auto stage = [&](int col, uint8_t* tile, float sign) {
+            float a[16];
+            umma::tmem_ld16(umma::tmem_addr(tmem, warp, col + 16 * (warp >> 2)), a);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                float o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = sign * a[8 * m + j];
+                store_split8(tile, tile + 16384, 128, (warp & 3) * 32 + lane, 2 * (warp >> 2) + m, o);
+            }
+        };
+        umma::wait_mma(&sh.mmN, it & 1);
+        stage(NW, base + BK, -1.f);
+        umma::signal(&sh.nwReady, lane);
+        umma::wait_mma(&sh.mmU, it & 1);
+        stage(U, base + UT, 1.f);
+        umma::signal(&sh.uReady, lane);
+    };
+    const int count = item_count(p.L);
+    for (int it = 0; it < count; ++it) {
+        const uint32_t par = it & 1;
+        float* beta = sh.beta[par];
+        float* gs = &sh.ga[0][0] + par * CH;                // SCALAR: the cumsum of every row, two items (rows past the end: the last valid one)
+        // ---- this item's rows into registers; park the anchor rows of g ----
+        umma::mbar_wait(&sh.ldin, par);
+        const int len = sh.info[it & 3].len;
+        Raw8 wk[2], wq[2];
+        f32x2 vg[2][4];
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = row_of(hf), rr = r < len ? r : len - 1, k8 = c8 + 8 * hf;
+            lds_raw8<DT>(base + R::K + rr * R::PITCH, k8, wk[hf]);
+            lds_raw8<DT>(base + R::Q + rr * R::PITCH, k8, wq[hf]);
+            if (r >= len) {                                 // rows past the end are zero
+                wk[hf].a = wq[hf].a = make_uint4(0, 0, 0, 0);
+                if (DT == MKDA_F32) wk[hf].b = wq[hf].b = make_uint4(0, 0, 0, 0);
+            }
+            if (!SCALAR) {
+                const float* g = reinterpret_cast<const float*>(base + RAW_G) + k8 * 8;
+                lds8_swapped(g + rr * 128, odd, vg[hf]);
+                if (it && hf == 0) umma::mbar_wait(&sh.hand, par ^ 1);             // nobody reads the previous item's last row any more
+                if ((r & 15) == 0) sts_halves(sh.ga[r >> 4], k8, vg[hf]);
+                if (r == len - 1) sts_halves(sh.ga[4], k8, vg[hf]);
+                if ((r & 15) == 0 && r >= 32) {
+                    f32x2 prev[4];
+                    lds8_swapped(g + (r - 16 < len ? r - 16 : len - 1) * 128, odd, prev);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) prev[e] = ex2f2_(sub2(vg[hf][e], prev[e]));
+                    sts_halves(sh.step[(r >> 4) - 2], k8, prev);
+                }
+            }
+        }
+        {   // beta (and a scalar gate's cumsum), used once the products are done
+            const size_t HV = p.L.HV;
+            const int i = sh.info[it & 3].start + min(tid & (CH - 1), len - 1), h = sh.info[it & 3].h;
+            if (tid < CH) cp_async4(&beta[tid], p.beta + i * HV + h);
+            else if (SCALAR && tid < 2 * CH) cp_async4(gs + tid - CH, p.g_c + i * HV + h);
+        }
+        umma::fence_before_sync();
+        sync_x();
+        umma::fence_after_sync();
+        // ---- operands, half by half ----
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = row_of(hf), I0 = r >> 4, k8 = c8 + 8 * hf;
+            if (SCALAR && DT == MKDA_BF16) {                // rows 0..63 = k, rows 64..127 = q, zero past the end
+                *reinterpret_cast<uint4*>(sKQ + umma::tile_chunk_offset(128, r, k8)) = wk[hf].a;
+                *reinterpret_cast<uint4*>(sKQ + umma::tile_chunk_offset(128, 64 + r, k8)) = wq[hf].a;
+            } else if (SCALAR) {
+                f32x2 x8[4];
+                unpack8<DT>(wk[hf], x8);
+                store_split8(sKQ, sKQ + 32768, 128, r, k8, x8);
+                unpack8<DT>(wq[hf], x8);
+                store_split8(sKQ, sKQ + 32768, 128, 64 + r, k8, x8);
+            } else {
+                f32x2 x8[4], d[4], e8[4], t8[4];
+                lds_halves(sh.ga[I0], k8, d);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { d[e] = sub2(vg[hf][e], d[e]); e8[e] = mul2(ex2f2_(d[e]), both(ROW_UP)); }
+                unpack8<DT>(wk[hf], x8);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(x8[e], e8[e]);
+                store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, t8);
+                unpack8<DT>(wq[hf], x8);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(x8[e], e8[e]);
+                store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, t8);
+                unpack8<DT>(wk[hf], x8);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { x8[e] = mul2(x8[e], both(COL_DOWN)); t8[e] = mul2(x8[e], ex2f2_(mul2(d[e], both(-1.f)))); }
+                if (it && hf == 0) umma::mbar_wait(&sh.khFree, par ^ 1);           // the tiles under the column tiles have left
+                store_split8(base, base + KC_BYTES, KC_ROWS, kc_row(I0) + r, k8, t8);
+#pragma unroll
+                for (int I = 1; I < 4; ++I) {
+                    if (I <= I0) continue;                  // warp-uniform
+                    if (I == I0 + 1) {
+                        lds_halves(sh.ga[I], k8, d);
+                        scale_ex2(t8, x8, d, vg[hf]);
+                    } else {                                // a step of decay (<= 1) further down the anchors instead of one more exponential
+                        lds_halves(sh.step[I - 2], k8, d);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], d[e]);
+                    }
+                    store_split8(base, base + KC_BYTES, KC_ROWS, kc_row(I) + r, k8, t8);
+                }
+            }
+            umma::signal(&sh.op1[hf], lane);
+        }
+        // ---- L2 scales, while the products run: they are applied to what comes out (Gamma and Q K^T are bilinear in the rows) and to the tiles
+        // below.  Four sums (k, q of two half rows) over eight threads; lane bit 2 ends up choosing the half, bit 1 between k and q ----
+        if (SCALAR && it) umma::mbar_wait(&sh.khFree, par ^ 1);     // Y has used the previous item's
+        if (p.l2) {
+            float t[2][2];
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                f32x2 x8[4], a = 0;
+                float a0, a1;
+                unpack8<DT>(wk[hf], x8);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a = fma2(x8[e], x8[e], a);
+                unpack2(a, a0, a1);
+                t[hf][0] = a0 + a1;
+                a = 0;
+                unpack8<DT>(wq[hf], x8);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) a = fma2(x8[e], x8[e], a);
+                unpack2(a, a0, a1);
+                t[hf][1] = a0 + a1;
+            }
+            float u[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) u[j] = (odd ? t[1][j] : t[0][j]) + __shfl_xor_sync(0xffffffffu, odd ? t[0][j] : t[1][j], 4);
+            float s = (c8 & 2 ? u[1] : u[0]) + __shfl_xor_sync(0xffffffffu, c8 & 2 ? u[0] : u[1], 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            if (!(c8 & 1)) (odd ? sh.part : sh.rs)[(c8 >> 1) & 1][row_of(odd)] = s;
+            sync_x();
+            if (tid < 2 * CH) {
+                const int i = tid & (CH - 1), x = tid >> 6;
+                s = rsqrtf(sh.rs[x][i] + sh.part[x][i] + p.l2_eps);
+                sh.rs[x][i] = s;
+                const int HK = p.L.HK, hk = sh.info[it & 3].hk;
+                if (p.k_rstd_out && sh.info[it & 3].h == hk * (p.L.HV / HK) && i < len)        // the backward pass reads them
+                    (x ? p.q_rstd_out : p.k_rstd_out)[(size_t)(sh.info[it & 3].start + i) * HK + hk] = s;
+            }
+        } else if (tid < 2 * CH) {
+            const int i = tid & (CH - 1), x = tid >> 6;
+            sh.rs[x][i] = p.k_rstd ? (x ? p.q_rstd : p.k_rstd)[(size_t)(sh.info[it & 3].start + min(i, len - 1)) * p.L.HK + sh.info[it & 3].hk] : 1.f;
+        }
+        cp_async_wait_all();
+        if (tid < CH && tid >= len) beta[tid] = 0.f;
+        __syncwarp();
+        if (lane == 0) umma::arrive(&sh.rows);
+        if (it) read_out(it - 1);
+        umma::wait_mma(&sh.mm1, par);
+        umma::mbar_wait(&sh.rows, par);
+        // ---- over the dead operands: the state kernels' scaled operands, kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g; k 2^g for Y ----
+        const float gLs = SCALAR ? gs[CH - 1] : 0.f;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = row_of(hf), k8 = c8 + 8 * hf;
+            const float up = SCALAR ? ex2f_(gs[r]) : 1.f, fk = sh.rs[0][r], fq = sh.rs[1][r] * p.scale;
+            const f32x2 sk = both(SCALAR ? fk * ex2f_(gLs - gs[r]) : fk), sq = both(SCALAR ? fq * up : fq), sb = both(SCALAR ? fk * up : fk);
+            f32x2 t8[4], e8[4], x8[4];
+            unpack8<DT>(wk[hf], x8);
+            if (SCALAR) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) t8[e] = mul2(x8[e], sk);
+            } else {
+                lds_halves(sh.ga[4], k8, e8);
+                scale_ex2(t8, x8, e8, vg[hf]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { t8[e] = mul2(t8[e], sk); e8[e] = ex2f2_(vg[hf][e]); }
+            }
+            store_split8(base + KB, base + KB + 16384, 64, r, k8, t8);
+            unpack8<DT>(wq[hf], t8);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(t8[e], sq) : mul2(mul2(t8[e], sq), e8[e]);
+            store_split8(base + QS, base + QS + 16384, 64, r, k8, t8);
+            if (it && hf == 0) umma::mbar_wait(&sh.bkFree, par ^ 1);               // nw^T of the previous item has left
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(x8[e], sb) : mul2(mul2(x8[e], sb), e8[e]);
+            store_split8(base + BK, base + BK + 16384, 64, r, k8, t8);
+        }
+        const size_t item = sh.info[it & 3].item;
+        if (SCALAR && tid < DK) p.gl[item * 128 + tid] = ex2f_(gLs);
+        if (!SCALAR && warp == X_WARPS - 1 && lane < 16) {
+            f32x2 gL[4];
+            lds_halves(sh.ga[4], lane, gL);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) gL[e] = ex2f2_(gL[e]);
+            sts8(p.gl + item * 128 + lane * 8, gL);
+        }
+        umma::signal(&sh.hand, lane);
+    }
+    read_out(count - 1);
+}
+
+// ---- Y ----------------------------------------------------------------------------------------------------------------------------------
+// Inverse of the unit lower-triangular matrix in place (fixed summation order) by recursive halving: the four 16 x 16 diagonal blocks by
+// forward substitution, then the off-diagonal block of each 32 x 32 half and finally the 32 x 32 block below the diagonal, each as
+// X = -B^-1 C A^-1  with A^-1 / B^-1 the inverses above / beside it.  Every entry depends on the rows up to its own only, and the order of the
+// sums is fixed by the indices.  The merges are TF32 products with error compensation (three products, fp32 accumulation: ~2^-21 per product).
+// T = 32 rows of scratch, free once `free` completes.
+template <int YW>
+__device__ __forceinline__ void invert_unit_lower(float* M, float* T, uint64_t* free, int it) {
+    using namespace in;
+    const int y = (threadIdx.x >> 5) & (YW - 1), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    if (y < 2) {
+        float* D = M + y * 2 * MB;
+        const int o = lane & 16, col = lane & 15;
         float x[16];
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
             float s[4] = {r == col ? 1.f : 0.f, 0.f, 0.f, 0.f};            // four partial sums: the chain from row to row is what takes the time
 #pragma unroll
             for (int c = 0; c < r; c += 4) {
-                const float4 m = *reinterpret_cast<const float4*>(sM + (o + r) * MLD + o + c);
+                const float4 m = *reinterpret_cast<const float4*>(D + (o + r) * LD + o + c);
                 const float mv[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
@@ -83,140 +368,314 @@ __device__ __forceinline__ void invert_unit_lower(const float* __restrict__ sM, 
             }
             x[r] = (s[0] + s[1]) + (s[2] + s[3]);
         }
-#pragma unroll
-        for (int r = 0; r < 16; ++r) sInv[(o + r) * MLD + o + col] = x[r];
         __syncwarp();
-        // 16 x 16 block (1, 0) or (3, 2): both of its diagonal blocks are this warp's
-        const int ro = 32 * warp + 16, co = 32 * warp;
-        float* T = &sh.T[16 * warp][0];
-        float acc[2][4];
-        warp_mma_short<2, 16, MLD, 1, MLD, 1>(acc, sM + ro * MLD + co, sInv + co * MLD + co);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) D[(o + r) * LD + o + col] = x[r];
+        __syncwarp();
+        // (B^-1 C) A^-1: the first product stays in registers as the left operand of the second, whose terms are summed in the order in which an
+        // accumulator's columns lie (2 t, 2 t + 1 of every eight in the place of t, t + 4)
+        float acc[2][4], z[2][4];
+        warp_mma_short<2, 16, LD, 1, LD, 1>(acc, D + 16 * LD + 16, D + 16 * LD);
+        warp_mma_chained(z, acc, D, LD);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-            *reinterpret_cast<float2*>(T + g * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][0], acc[nt][1]);
-            *reinterpret_cast<float2*>(T + (g + 8) * TLD + 8 * nt + 2 * t) = make_float2(acc[nt][2], acc[nt][3]);
+            *reinterpret_cast<float2*>(D + (16 + g) * LD + 8 * nt + 2 * t) = make_float2(-z[nt][0], -z[nt][1]);
+            *reinterpret_cast<float2*>(D + (24 + g) * LD + 8 * nt + 2 * t) = make_float2(-z[nt][2], -z[nt][3]);
         }
-        __syncwarp();
-        warp_mma_short<2, 16, MLD, 1, TLD, 1>(acc, sInv + ro * MLD + ro, T);
+    }
+    if (it) umma::mbar_wait(free, (it & 1) ^ 1);
+    sync_y<YW>();
+    // 32 x 32 block (rows 32.., columns 0..31) in tiles of 16 x 8
+    auto product = [&](const float* A, const float* B, float* D, float sign) {
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            *reinterpret_cast<float2*>(sInv + (ro + g) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][0], -acc[nt][1]);
-            *reinterpret_cast<float2*>(sInv + (ro + g + 8) * MLD + co + 8 * nt + 2 * t) = make_float2(-acc[nt][2], -acc[nt][3]);
+        for (int i = y; i < 8; i += YW) {
+            const int m0 = 16 * (i >> 2), n0 = 8 * (i & 3);
+            float acc[1][4];
+            warp_mma_short<1, 32, LD, 1, LD, 1>(acc, A + m0 * LD, B + n0);
+            *reinterpret_cast<float2*>(D + (m0 + g) * LD + n0 + 2 * t) = make_float2(sign * acc[0][0], sign * acc[0][1]);
+            *reinterpret_cast<float2*>(D + (m0 + g + 8) * LD + n0 + 2 * t) = make_float2(sign * acc[0][2], sign * acc[0][3]);
         }
-    }
-    sync_compute();
-    // 32 x 32 block (rows 32.., columns 0..31): eight warps, one 16 x 8 tile each.  (Leaving out the products with zero blocks needs the code
-    // of several lengths and made the whole kernel 5 % slower: it is fetched anew for every item.)
-    const int m0 = 16 * ((warp >> 2) & 1), n0 = 8 * (warp & 3);
-    float acc[1][4];
-    if (warp < 8) {
-        warp_mma_short<1, 32, MLD, 1, MLD, 1>(acc, sM + (32 + m0) * MLD, sInv + n0);
-        *reinterpret_cast<float2*>(&sh.T[m0 + g][n0 + 2 * t]) = make_float2(acc[0][0], acc[0][1]);
-        *reinterpret_cast<float2*>(&sh.T[m0 + g + 8][n0 + 2 * t]) = make_float2(acc[0][2], acc[0][3]);
-    }
-    sync_compute();
-    if (warp < 8) {
-        warp_mma_short<1, 32, MLD, 1, TLD, 1>(acc, sInv + (32 + m0) * MLD + 32, &sh.T[0][n0]);
-        *reinterpret_cast<float2*>(sInv + (32 + m0 + g) * MLD + n0 + 2 * t) = make_float2(-acc[0][0], -acc[0][1]);
-        *reinterpret_cast<float2*>(sInv + (32 + m0 + g + 8) * MLD + n0 + 2 * t) = make_float2(-acc[0][2], -acc[0][3]);
-    }
-    sync_compute();
+        sync_y<YW>();
+    };
+    product(M + MB, M, T, 1.f);
+    product(M + 2 * MB, T, M + MB, -1.f);
 }
 
-// The issuing thread.  The base passes through an empty statement in front of each group of products: kept in registers over the loop, the
-// operand descriptors of all of them would spill.
-template <bool SCALAR>
-__device__ __forceinline__ void intra_issue(uint8_t* smem, uint32_t tmem, int total, IntraShared& sh) {
-    uint8_t* base = smem;
-    auto fresh = [&]() { base = smem; asm volatile("" : "+l"(base)); };
-    uint32_t it = 0;
-    for (int item = blockIdx.x; item < total; item += gridDim.x, ++it) {
-        umma::wait_mma(&sh.op1, it & 1);
-        fresh();
-        uint8_t* sKQ = base + KQ_OFF;
-        if (SCALAR) {      // D[m][j]: lanes 0..63 = K K^T rows, lanes 64..127 = Q K^T rows; columns j = K rows of the same tile
-            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(sKQ, sKQ + 32768, 128), 128, 64, 128, 0u);
-        } else {
-            // ONE product over the stacked column tiles: D[32 I + t][kc_row(I') + j].  Only the blocks I' = I are meaningful (the
-            // anchors of the two operands match there) and read back; the others are finite and ignored.  An MMA costs
-            // (4 KB of A + 32 N bytes of B) / 128 B per cycle, so N = 160 once is far cheaper than N = 32 four times.
-            umma::gemm(tmem, umma::opnd_k(sKQ, sKQ + 32768, 128), umma::opnd_k(base, base + KC_ALL_BYTES, KC_ALL_ROWS), 128, KC_ALL_ROWS, 128, 0u);
-        }
-        umma::commit(&sh.mm1);
-        umma::wait_mma(&sh.op2, it & 1);
-        fresh();
-        const umma::Opnd bA = umma::opnd_k(base + TA_OFF, base + TA_OFF + 8192, 64);
-        umma::gemm(tmem + 128, umma::opnd_mn(base, base + 16384, 64), bA, 128, 64, 64, 0u);
-        umma::commit(&sh.mmN);
-        umma::gemm(tmem + 192, umma::opnd_mn(base + 32768, base + 32768 + 16384, 64), bA, 128, 64, 64, 0u);
-        umma::commit(&sh.mmU);
-    }
-}
-
-// SCALAR: the gate is one decay per token (the same cumsum in all 128 channels).  It then commutes with the contraction
-// over channels, Gamma_ij = (k_i . k_j) 2^(g_i - g_j), so the products are plain K K^T / Q K^T (one product over a stacked
-// [K; Q] tile) and the decay is applied to the accumulators, element by element and for i >= j only: nothing is anchored,
-// no exponent is ever positive, and any g <= 0 is in range (the per-channel path needs g >= -5 per token).
-template <int DT, bool SCALAR, bool TMA>
-__global__ void __launch_bounds__(INTRA_THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ IntraMaps maps) {
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ IntraShared sh;
-    // cumsum rows of the four block anchors, [4] = last valid row; first the lower then the upper four of every eight channels, so that the
-    // 16 threads of a row read them without bank conflicts
-    __shared__ __align__(16) float sGa[5][DK], sStep[2][DK];      // anchor rows; 2^(ga[I] - ga[I - 1]) of I = 2, 3
-    __shared__ __align__(16) float sGsb[2][CH];                      // SCALAR: the cumsum of every row (rows past the end: the last valid one)
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sKQ = base + KQ_OFF;
-    float* sM = reinterpret_cast<float*>(base + OPND_BYTES + 32768);
-    float* sInv = sM + CH * MLD;
-    uint8_t* sBk = base;                               // phase 3: beta k~ [j][K index], hi 16 KB + lo 16 KB
-    uint8_t* sBv = base + 32768;                       // beta v [j][v]
-    uint8_t* sTA = base + TA_OFF;                       // A [i][j], hi 8 KB + lo 8 KB
-    uint8_t* sTQ = base + 81920;                       // Aqk [i][j], hi 8 KB + lo 8 KB (only copied out)
-    uint8_t* sKB = base + OPND_BYTES;                  // kbar [tok][K index] hi + lo (32 KB), only copied out; later the q rows of the next item
-    uint8_t* sQS = sKB + 32768;                        // scale q 2^g [tok][K index] hi + lo (32 KB), likewise; under sM and sInv
-
-    const int HV = p.L.HV, HK = p.L.HK, total = p.L.NC * HV, stride = gridDim.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int q = warp & 3, cg = warp >> 2, row = q * 32 + lane;
-
-    // Persistent: one CTA per SM walks the (chunk, v-head) items gridDim.x apart, heads fastest.  The k, q, g rows of the NEXT item are
-    // requested as soon as the current item has no more use for their place, half way through the item, so that they travel while the
-    // inverse and the second products run.  beta (and a scalar gate's cumsum) come by asynchronous copies into the other half of a double
-    // buffer: a value that is loaded into a register under a condition is waited for where the paths join again (2 k cycles per item).
-    constexpr bool BULK = TMA && DT != MKDA_F32;       // fp32 rows would not fit: they travel through registers
-    f32x2 vk[2][4], vq[2][4], vg[2][4];
-    Raw8 wk[2], wq[2];
-    uint32_t nin = 0;                                  // phase counter of the input-row barrier
-    struct Item { int c, h, hk, start, len; } cur, nxt;
-    const int G = HV / HK, dc = stride / HV, dh = stride - dc * HV;
-    const float rG = 1.f / (float)G;
-    auto advance = [&](Item& i) { i.c += dc; i.h += dh; if (i.h >= HV) { i.h -= HV; ++i.c; } i.hk = (int)(((float)i.h + 0.5f) * rG); };
-    auto table = [&](Item& i) { const int c = min(i.c, p.L.NC - 1); i.start = p.L.chunk_start[c]; i.len = p.L.chunk_len[c]; };
-    auto load_inputs = [&](const Item& i, int buf) {
-        if (tid < CH) cp_async4(&sh.beta[buf][tid], p.beta + (size_t)(i.start + min(tid, i.len - 1)) * HV + i.h);
-        else if (SCALAR && tid < 2 * CH) cp_async4(&sGsb[buf][tid - CH], p.g_c + (size_t)(i.start + min(tid - CH, i.len - 1)) * HV + i.h);
-        if (BULK && tid == 128) {                      // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
-            umma::mbar_expect_tx(&sh.ldin, 16384u + 16384u + (SCALAR ? 0u : 32768u));
-            umma::tma_load_rows(base + RAW_K, &maps.k, i.hk * 128, i.start, &sh.ldin);
-            if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, i.h * 128, i.start, &sh.ldin);
-        }
-        if (!BULK) {
+template <int DT, bool SCALAR, int YW>
+__device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, uint32_t tmem, in::Shared& sh) {
+    using namespace in;
+    constexpr int YT = 32 * YW;
+    const int tid = threadIdx.x & (YT - 1), warp = threadIdx.x >> 5, lane = tid & 31, q = warp & 3;
+    const size_t HV = p.L.HV;
+    float* M = reinterpret_cast<float*>(base + M_);
+    const int count = item_count(p.L);
+    for (int it = 0; it < count; ++it) {
+        const uint32_t par = it & 1;
+        const float* beta = sh.beta[par];
+        const float* gs = &sh.ga[0][0] + par * CH;
+        // ---- I + L and Aqk from the accumulators ----
+        // per channel: warp quadrant = row block (16 rows of Gamma, then 16 rows of Q K^T); scalar gate: 64 rows of K K^T, then of Q K^T
+        umma::mbar_wait(&sh.rows, par);
+        umma::wait_mma(&sh.mm1, par);
+        const int len = sh.info[it & 3].len;
+        {
+            const int i = SCALAR ? (q & 1) * 32 + lane : 16 * q + (lane & 15);
+            const bool isq = SCALAR ? q >= 2 : lane >= 16;
+            const float bi = isq ? p.scale * sh.rs[1][i] : beta[i] * sh.rs[0][i], gi = SCALAR ? gs[i] : 0.f;
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                const int r = (tid + n * 512) >> 4, k8 = tid & 15, rr = min(r, i.len - 1);
-                const size_t tk = (size_t)(i.start + rr) * HK + i.hk;
-                ldraw8<DT>(p.k, tk * 128 + k8 * 8, wk[n]);
-                ldraw8<DT>(p.q, tk * 128 + k8 * 8, wq[n]);
-                if (!SCALAR) lds8(p.g_c + ((size_t)(i.start + rr) * HV + i.h) * 128 + k8 * 8, vg[n]);
+            for (int cg = YW == 4 ? 0 : 2 * ((warp >> 2) & 1), last = cg + 16 / YW; cg < last; ++cg) {
+                float v[16];
+                if (SCALAR || cg <= q) {                     // warp-uniform
+                    umma::tmem_ld16(umma::tmem_addr(tmem, warp, D1 + par * D1_COLS + (SCALAR ? 0 : kc_row(q)) + 16 * cg), v);
+#pragma unroll
+                    for (int j4 = 0; j4 < 16; j4 += 4) {
+                        const float4 r4 = *reinterpret_cast<const float4*>(sh.rs[0] + 16 * cg + j4);
+                        const float rj[4] = {r4.x, r4.y, r4.z, r4.w};
+                        float E[4] = {1.f, 1.f, 1.f, 1.f};
+                        if (SCALAR) {
+                            const float4 g4 = *reinterpret_cast<const float4*>(gs + 16 * cg + j4);
+                            const float gj[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) E[e] = ex2f_(fminf(gi - gj[e], 0.f));
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int j = 16 * cg + j4 + e;
+                            const float x = SCALAR ? bi * v[j4 + e] * E[e] * rj[e] : bi * v[j4 + e] * rj[e];
+                            v[j4 + e] = j < i ? x : j > i ? 0.f : isq ? x : 1.f;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                }
+                if (isq) {                                   // Aqk leaves as a ready-made [row][column] operand tile (rows past the end: zeros)
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        float o[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) o[j] = v[8 * m + j];
+                        store_split8(base + AQ, base + AQ + 8192, 64, i, 2 * cg + m, o);
+                    }
+                } else if (SCALAR ? q == 1 || cg < 2 : cg <= (q | 1)) {      // the blocks (0, 1) and (2, 3) above the diagonal are read as zeros
+                    float* d = M + (i < 32 ? 0 : cg < 2 ? MB : 2 * MB) + (i & 31) * LD + 16 * (cg & 1);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(d + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
             }
         }
+        umma::signal(&sh.acc, lane);
+        sync_y<YW>();
+        invert_unit_lower<YW>(M, reinterpret_cast<float*>(base + T_), &sh.abFree, it);         // there u^T of the previous item may still be leaving
+        // A leaves as a ready-made [row][column] operand tile (rows past the end: identity rows); A diag(beta) is the operand of nw and u
+        uint8_t* At = reinterpret_cast<uint8_t*>(p.A) + (size_t)sh.info[it & 3].item * umma::QUARTER_TILE_BYTES;
+        const int k8 = tid & 7;
+        f32x2 b8[4];
+        lds8_swapped(beta + 8 * k8, k8 & 4, b8);
+#pragma unroll
+        for (int m = 0; m < 16 / YW; ++m) {
+            const int r = 4 * YW * m + (tid >> 3);
+            float a8[8];
+            if (m < 8 / YW && k8 >= 4) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) a8[e] = 0.f;
+            } else {
+                f32x2 a[4];
+                lds8_swapped(M + (m < 8 / YW ? 0 : k8 < 4 ? MB : 2 * MB) + (r & 31) * LD + 8 * (k8 & 3), k8 & 2, a);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) unpack2(a[e], a8[2 * e], a8[2 * e + 1]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (k8 * 8 + e > r) a8[e] = 0.f;
+            }
+            store_split8(At, At + 8192, 64, r, k8, a8);
+            f32x2 ab[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ab[e] = mul2(pack2(a8[2 * e], a8[2 * e + 1]), b8[e]);
+            store_split8(base + AB, base + AB + 8192, 64, r, k8, ab);
+        }
+        if (DT == MKDA_BF16) {
+            if (len < CH) {                                  // rows past the end belong to another sequence
+                umma::mbar_wait(&sh.fullV, par);
+                for (int i = len * 16 + tid; i < CH * 16; i += YT)
+                    *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(0, 0, 0, 0);
+            }
+            umma::signal(&sh.opA, lane);
+        } else {
+            // v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
+            constexpr int N = 32 / YW;
+            uint32_t lo[N][4];
+            if (DT == MKDA_F16) umma::mbar_wait(&sh.fullV, par);
+#pragma unroll
+            for (int m = 0; m < N; m += 4) {
+                Raw8 raw[4];
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const int i = tid + YT * (m + n), r = i >> 4;
+                    if (DT == MKDA_F16) raw[n].a = *reinterpret_cast<const uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15));
+                    else ldraw8<DT>(p.v, ((size_t)(sh.info[it & 3].start + min(r, len - 1)) * HV + sh.info[it & 3].h) * 128 + (i & 15) * 8, raw[n]);
+                }
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const int i = tid + YT * (m + n), r = i >> 4;
+                    float v8[8];
+                    unpack8<DT>(raw[n], v8);
+                    uint32_t hi[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        umma::split2(v8[2 * e], v8[2 * e + 1], hi[e], lo[m + n][e]);
+                        if (r >= len) hi[e] = lo[m + n][e] = 0u;
+                    }
+                    *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                }
+            }
+            umma::signal(&sh.opA, lane);
+            umma::wait_mma(&sh.mmV, par);
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const int i = tid + YT * n;
+                *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(lo[n][0], lo[n][1], lo[n][2], lo[n][3]);
+            }
+            umma::signal(&sh.opV, lane);
+        }
+        sync_y<YW>();                                            // the matrix has been read
+    }
+}
+
+// ---- the four warps of one thread each ---------------------------------------------------------------------------------------------------
+// The base passes through an empty statement in front of each group of products: kept in registers over the loop, the operand descriptors of
+// all of them would spill.
+__device__ __forceinline__ uint8_t* fresh(uint8_t* smem) {
+    asm volatile("" : "+l"(smem));
+    return smem;
+}
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, uint32_t tmem, in::Shared& sh) {
+    using namespace in;
+    const int count = item_count(p.L);
+    for (int it = 0; it < count; ++it) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            umma::wait_mma(&sh.op1[hf], it & 1);
+            uint8_t* base = fresh(smem);
+            uint8_t* kq = base + KQ + hf * 16384;
+            if (SCALAR) {      // D[m][j]: lanes 0..63 = K K^T rows, lanes 64..127 = Q K^T rows; columns j = K rows of the same tile
+                const umma::Opnd o = umma::opnd_k(kq, DT == MKDA_BF16 ? nullptr : kq + 32768, 128);
+                umma::gemm(tmem + D1 + (it & 1) * D1_COLS, o, o, 128, 64, 64, hf);
+            } else {
+                // ONE product over the stacked column tiles: D[32 I + t][kc_row(I') + j].  Only the blocks I' = I are meaningful (the
+                // anchors of the two operands match there) and read back; the others are finite and ignored.  An MMA costs
+                // (4 KB of A + 32 N bytes of B) / 128 B per cycle, so N = 160 once is far cheaper than N = 32 four times.
+                uint8_t* kc = base + hf * KC_ROWS * 128;
+                umma::gemm(tmem + D1 + (it & 1) * D1_COLS, umma::opnd_k(kq, kq + 32768, 128), umma::opnd_k(kc, kc + KC_BYTES, KC_ROWS), 128, KC_ROWS, 64, hf);
+            }
+        }
+        umma::commit(&sh.mm1);
+    }
+}
+template <int DT>
+__device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, uint32_t tmem, in::Shared& sh) {
+    using namespace in;
+    const int count = item_count(p.L);
+    for (int it = 0; it < count; ++it) {
+        const uint32_t par = it & 1;
+        umma::wait_mma(&sh.hand, par);                      // k 2^g
+        umma::wait_mma(&sh.opA, par);
+        if (DT == MKDA_BF16) umma::mbar_wait(&sh.fullV, par);
+        uint8_t* base = fresh(smem);
+        const umma::Opnd ab = umma::opnd_k(base + AB, base + AB + 8192, 64), v = umma::opnd_mn(base + V_, nullptr, 64);
+        if (DT != MKDA_BF16) {
+            umma::gemm(tmem + U, v, ab, 128, 64, 64, 0u);
+            umma::commit(&sh.mmV);
+            umma::wait_mma(&sh.opV, par);
+            umma::Opnd hi = ab;
+            hi.lo = 0;
+            umma::gemm(tmem + U, v, hi, 128, 64, 64, 1u);
+            umma::commit(&sh.mmU);
+        }
+        umma::gemm(tmem + NW, umma::opnd_mn(base + BK, base + BK + 16384, 64), ab, 128, 64, 64, 0u);
+        umma::commit(&sh.mmN);
+        if (DT == MKDA_BF16) {
+            umma::gemm(tmem + U, v, ab, 128, 64, 64, 0u);
+            umma::commit(&sh.mmU);
+        }
+    }
+}
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+    using namespace in;
+    using R = Rows<DT, SCALAR>;
+    // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
+    auto load_q = [&](const Walk& w) { umma::tma_load_rows(base + R::Q, &maps.q, w.hk * 128, w.start, &sh.ldin); };
+    auto load_rows = [&](const Walk& w, int it) {
+        auto& i = sh.info[it & 3];
+        i.item = w.item(); i.start = w.start; i.len = w.len; i.h = w.h; i.hk = w.hk;
+        umma::mbar_expect_tx(&sh.ldin, 2 * R::BYTES + (SCALAR ? 0u : 32768u));
+        if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, w.h * 128, w.start, &sh.ldin);
+        umma::tma_load_rows(base + R::K, &maps.k, w.hk * 128, w.start, &sh.ldin);
+        if (!R::LATE_Q) load_q(w);
     };
-    auto load_q = [&](const Item& i) { umma::tma_load_rows(base + RAW_Q, &maps.q, i.hk * 128, i.start, &sh.ldin); };
-    if (warp == 0) umma::tmem_alloc(&sh.tmem, 256);
-    if (tid == 0) { 
-        for (uint64_t* b : {&sh.ldin, &sh.mm1, &sh.mmN, &sh.mmU}) umma::mbar_init(b, 1);
-        for (uint64_t* b : {&sh.op1, &sh.op2}) umma::mbar_init(b, 16);
+    Walk w(p.L);
+    load_rows(w, 0);
+    if (R::LATE_Q) load_q(w);
+    for (int it = 0; w.valid(); ++it) {
+        const size_t item = w.item();
+        w.next();
+        umma::mbar_wait(&sh.mm1, it & 1);                   // the operands are dead
+        if (w.valid()) load_rows(w, it + 1);
+        umma::mbar_wait(&sh.acc, it & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + item * umma::QUARTER_TILE_BYTES, base + AQ, umma::QUARTER_TILE_BYTES);
+        umma::mbar_wait(&sh.hand, it & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + item * umma::CHUNK_TILE_BYTES, base + KB, umma::CHUNK_TILE_BYTES);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + item * umma::CHUNK_TILE_BYTES, base + QS, umma::CHUNK_TILE_BYTES);
+        umma::bulk_store_wait_read();
+        umma::arrive(&sh.khFree);
+        if (R::LATE_Q && w.valid()) load_q(w);
+    }
+}
+template <int DT>
+__device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+    using namespace in;
+    auto load_v = [&](const Walk& w) {                      // two boxes of 64 channels: a [64][128] operand tile as it stands
+        if (DT == MKDA_F32) return;
+        umma::mbar_expect_tx(&sh.fullV, 16384);
+        umma::tma_load_rows(base + V_, &maps.v, w.h * 128, w.start, &sh.fullV);
+        umma::tma_load_rows(base + V_ + 8192, &maps.v, w.h * 128 + 64, w.start, &sh.fullV);
+    };
+    Walk w(p.L);
+    load_v(w);
+    for (uint32_t it = 0; w.valid(); ++it) {
+        const size_t item = w.item();
+        w.next();
+        umma::mbar_wait(&sh.nwReady, it & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + item * umma::CHUNK_TILE_BYTES, base + BK, umma::CHUNK_TILE_BYTES);
+        umma::mbar_wait(&sh.uReady, it & 1);
+        umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + item * umma::CHUNK_TILE_BYTES, base + UT, umma::CHUNK_TILE_BYTES);
+        umma::bulk_store_wait_read_but<1>();
+        umma::arrive(&sh.bkFree);
+        umma::bulk_store_wait_read();
+        umma::arrive(&sh.abFree);
+        if (w.valid()) load_v(w);
+    }
+}
+
+template <int DT, bool SCALAR, int YW>
+__global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ in::Maps maps) {
+    using namespace in;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
+    Shared& sh = *reinterpret_cast<Shared*>(base + TILES);
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        follow_stream();
+        if (threadIdx.x == 0) atomicExch(&umma::g_timeout_flag, 1u);
+        return;
+    }
+    if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
+    if (threadIdx.x == 0) {
+        for (uint64_t* b : {&sh.ldin, &sh.fullV, &sh.mm1, &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.op1[0], &sh.op1[1], &sh.rows, &sh.hand, &sh.nwReady, &sh.uReady}) umma::mbar_init(b, X_WARPS);
+        for (uint64_t* b : {&sh.opA, &sh.opV, &sh.acc}) umma::mbar_init(b, YW);
         umma::fence_barrier_init();
     }
     umma::fence_before_sync();
@@ -224,334 +683,27 @@ __global__ void __launch_bounds__(INTRA_THREADS, 1) intra_fwd_tc_kernel(const Mk
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
-    if (warp >= INTRA_WARP_MMA) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
-        if (warp == INTRA_WARP_MMA && umma::elect_one()) intra_issue<SCALAR>(base, tmem, total, sh);
+    if (warp < X_WARPS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(Warps<YW>::X_REGS));
+        intra_x<DT, SCALAR>(p, base, tmem, sh);
+    } else if (warp < X_WARPS + YW) {
+        if (YW == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(Warps<YW>::Y_REGS));
+        intra_y<DT, SCALAR, YW>(p, base, tmem, sh);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (umma::elect_one()) {
+            switch (warp - X_WARPS - YW) {
+                case 0: intra_mm1<DT, SCALAR>(p, base, tmem, sh); break;
+                case 1: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
+                case 2: intra_copy_y<DT>(p, maps, base, sh); break;
+                default: intra_mm3<DT>(p, base, tmem, sh);
+            }
+        }
         __syncwarp();
-    } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-    cur.c = blockIdx.x / HV; cur.h = blockIdx.x - cur.c * HV; cur.hk = cur.h / G;
-    table(cur);
-    if ((int)blockIdx.x < total) {
-        load_inputs(cur, 0);
-        if (BULK && tid == STORER) load_q(cur);
-    }
-    nxt = cur;
-    advance(nxt);
-
-    for (int item = blockIdx.x, it = 0; item < total; item += stride, ++it) {
-    const int c = cur.c, h = cur.h, hk = cur.hk, start = cur.start, len = cur.len;
-    float* sBeta = sh.beta[it & 1];
-    const float* sGs = sGsb[it & 1];
-    table(nxt);                                        // the chunk table entries are read ahead of load_inputs: every address depends on them
-    // ---- phase 0: this item's k, q, g rows into registers; park the anchor rows of g in shared memory ----
-    cp_async_wait_all();
-    if (tid < CH && tid >= len) sBeta[tid] = 0.f;
-    if (BULK) {
-        umma::mbar_wait(&sh.ldin, nin & 1); ++nin;
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int i = tid + n * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
-            wk[n].a = *reinterpret_cast<const uint4*>(base + RAW_K + rr * 256 + k8 * 16);
-            wq[n].a = *reinterpret_cast<const uint4*>(base + RAW_Q + rr * 256 + k8 * 16);
-            if (!SCALAR) lds8(reinterpret_cast<const float*>(base + RAW_G + rr * 512 + k8 * 32), vg[n]);
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-        if (!SCALAR && (r & 15) == 0) sts_halves(sGa[r >> 4], k8, vg[n]);
-        if (!SCALAR && r == len - 1) sts_halves(sGa[4], k8, vg[n]);
-        if (!SCALAR && (r & 15) == 0 && r >= 32) {
-            const int rp = r - 16 < len ? r - 16 : len - 1;
-            f32x2 prev[4];
-            if (BULK) lds8(reinterpret_cast<const float*>(base + RAW_G + rp * 512 + k8 * 32), prev);
-            else lds8(p.g_c + ((size_t)(start + rp) * HV + h) * 128 + k8 * 8, prev);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) prev[e] = ex2f2_(sub2(vg[n][e], prev[e]));
-            sts_halves(sStep[(r >> 4) - 2], k8, prev);
-        }
-        if (r >= len) {                                    // rows past the end are zero
-            wk[n].a = wq[n].a = make_uint4(0, 0, 0, 0);
-            if (DT == MKDA_F32) wk[n].b = wq[n].b = make_uint4(0, 0, 0, 0);
-        }
-        unpack8<DT>(wk[n], vk[n]);
-        unpack8<DT>(wq[n], vq[n]);
-    }
-    if (tid == STORER) umma::bulk_store_wait_read();   // the previous item's tiles have left shared memory
-    umma::fence_before_sync();
-    sync_compute();
-    umma::fence_after_sync();
-    // ---- operands ---------------------------------------------------------------------------------------------------
-    if (SCALAR) {          // one stacked tile: rows 0..63 = k, rows 64..127 = q (L2 statistics applied, zero past the end)
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-            store_split8(sKQ, sKQ + 32768, 128, r, k8, vk[n]);
-            store_split8(sKQ, sKQ + 32768, 128, 64 + r, k8, vq[n]);
-        }
-    } else {
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int i = tid + n * 512, r = i >> 4, k8 = i & 15, I0 = r >> 4;
-            f32x2 ga[4], t8[4], e8[4];
-            lds_halves(sGa[I0], k8, ga);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { e8[e] = mul2(ex2f2_(sub2(vg[n][e], ga[e])), both(ROW_UP)); t8[e] = mul2(vk[n][e], e8[e]); }
-            store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + (r & 15), k8, t8);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) t8[e] = mul2(vq[n][e], e8[e]);
-            store_split8(sKQ, sKQ + 32768, 128, 32 * I0 + 16 + (r & 15), k8, t8);
-            f32x2 kd[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) kd[e] = mul2(vk[n][e], both(COL_DOWN));
-#pragma unroll
-            for (int I = 0; I < 4; ++I) {
-                if (I < I0) continue;
-                if (I <= I0 + 1) {
-                    if (I > I0) lds_halves(sGa[I], k8, ga);
-                    scale_ex2(t8, kd, ga, vg[n]);
-                } else {                                   // a step of decay (<= 1) further down the anchors: exponentials are what bounds this phase
-                    lds_halves(sStep[I - 2], k8, ga);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], ga[e]);
-                }
-                store_split8(base, base + KC_ALL_BYTES, KC_ALL_ROWS, kc_row(I) + r, k8, t8);      // the four column tiles stacked by rows
-            }
-        }
-    }
-    umma::signal(&sh.op1, lane);
-    // The L2 scales are applied to what comes out (Gamma and Q K^T are bilinear in the rows) and to the tiles below: finding them takes no
-    // time while the products run.  Four sums (k, q of two rows) over the 16 threads of a row; lane bits 3 and 2 end up spelling the sum.
-    float fk[2] = {1.f, 1.f}, fq[2] = {1.f, 1.f};
-    if (p.l2) {
-        float t[4];
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            f32x2 a = mul2(vk[n][0], vk[n][0]), b = mul2(vq[n][0], vq[n][0]);
-#pragma unroll
-            for (int e = 1; e < 4; ++e) { a = fma2(vk[n][e], vk[n][e], a); b = fma2(vq[n][e], vq[n][e], b); }
-            float a0, a1, b0, b1;
-            unpack2(a, a0, a1);
-            unpack2(b, b0, b1);
-            t[2 * n] = a0 + a1;
-            t[2 * n + 1] = b0 + b1;
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const float recv = __shfl_xor_sync(0xffffffffu, (lane & 8) ? t[j] : t[j + 2], 8);
-            t[j] = ((lane & 8) ? t[j + 2] : t[j]) + recv;
-        }
-        const float recv = __shfl_xor_sync(0xffffffffu, (lane & 4) ? t[0] : t[1], 4);
-        float s = ((lane & 4) ? t[1] : t[0]) + recv;
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s = rsqrtf(s + p.l2_eps);
-        const int rr = (tid >> 4) + 4 * (lane & 8);
-        if ((lane & 3) == 0) {
-            ((lane & 4) ? sh.rq : sh.rk)[rr] = s;
-            if (p.k_rstd_out && h == hk * G && rr < len)                   // the backward pass reads them
-                ((lane & 4) ? p.q_rstd_out : p.k_rstd_out)[(size_t)(start + rr) * HK + hk] = s;
-        }
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            fk[n] = __shfl_sync(0xffffffffu, s, (lane & 16) | (8 * n));
-            fq[n] = __shfl_sync(0xffffffffu, s, (lane & 16) | (8 * n + 4));
-        }
-    } else {
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int r = (tid + n * 512) >> 4;
-            if (p.k_rstd) {
-                const size_t tk = (size_t)(start + min(r, len - 1)) * HK + hk;
-                fk[n] = p.k_rstd[tk];
-                fq[n] = p.q_rstd[tk];
-            }
-            if ((lane & 15) == 0) { sh.rk[r] = fk[n]; sh.rq[r] = fq[n]; }
-        }
-    }
-    // v for phase 3 is fetched while the products run
-    Raw8 wv[2];
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        const int i = tid + n * 512, r = i >> 4, k8 = i & 15, rr = r < len ? r : len - 1;
-        ldraw8<DT>(p.v, ((size_t)(start + rr) * HV + h) * 128 + k8 * 8, wv[n]);
-    }
-    // ... and so are the hand-over tiles, built and sent off in the shadow of the products
-    // The state kernels' scaled operands, as ready-made tiles: kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g,
-    // plus gl = 2^gL.  Rows past the end are zero (their k / q were zeroed above).
-    {
-        f32x2 gLv[4];
-        if (!SCALAR) lds_halves(sGa[4], tid & 15, gLv);
-        const float gLs = SCALAR ? sGs[CH - 1] : 0.f;      // rows past the end carry the last valid one's
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-            f32x2 t8[4];
-            const f32x2 sk = both(SCALAR ? fk[n] * ex2f_(gLs - sGs[r]) : fk[n]), sq = both(SCALAR ? fq[n] * p.scale * ex2f_(sGs[r]) : fq[n] * p.scale);
-            if (SCALAR) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) t8[e] = mul2(vk[n][e], sk);
-            } else {
-                scale_ex2(t8, vk[n], gLv, vg[n]);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], sk);
-            }
-            store_split8(sKB, sKB + 16384, 64, r, k8, t8);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vq[n][e], sq) : mul2(mul2(vq[n][e], sq), ex2f2_(vg[n][e]));
-            store_split8(sQS, sQS + 16384, 64, r, k8, t8);
-        }
-        if (SCALAR && tid < DK) p.gl[((size_t)c * HV + h) * 128 + tid] = ex2f_(gLs);
-        if (!SCALAR && tid < 16) {
-            f32x2 e8[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) e8[e] = ex2f2_(gLv[e]);
-            sts8(p.gl + ((size_t)c * HV + h) * 128 + tid * 8, e8);
-        }
-    }
-    umma::fence_async_smem();
-    sync_compute();
-    if (tid == STORER) {                               // qs first: its place is needed first
-        const size_t it = (size_t)c * HV + h;
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + it * umma::CHUNK_TILE_BYTES, sQS, umma::CHUNK_TILE_BYTES);
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + it * umma::CHUNK_TILE_BYTES, sKB, umma::CHUNK_TILE_BYTES);
-    }
-    umma::wait_mma(&sh.mm1, it & 1);
-    // phase-3 operands over the dead phase-1 tiles: beta k 2^g and beta v (rows past the end are zero)
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        const int i = tid + n * 512, r = i >> 4, k8 = i & 15;
-        const float b = sBeta[r];            // 0 for rows past the end
-        const f32x2 b2 = both(b), fb = both(SCALAR ? b * fk[n] * ex2f_(sGs[r]) : b * fk[n]);
-        f32x2 t8[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(vk[n][e], fb) : mul2(mul2(vk[n][e], fb), ex2f2_(vg[n][e]));
-        store_split8(sBk, sBk + 16384, 64, r, k8, t8);
-        unpack8<DT>(wv[n], t8);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) t8[e] = mul2(t8[e], b2);
-        store_split8(sBv, sBv + 16384, 64, r, k8, t8);
-    }
-    if (tid == STORER) umma::bulk_store_wait_read_but<1>();        // the tile under sM / sInv has left shared memory
-    sync_compute();
-    if (item + stride < total) load_inputs(nxt, (it & 1) ^ 1);     // k, q, g, beta of the next item start travelling
-    sInv[(32 * (tid >> 8) + ((tid >> 4) & 15)) * MLD + 32 * (tid >> 8) + 16 + (tid & 15)] = 0.f;       // blocks (0, 1) and (2, 3)
-    auto store_row16 = [](float* dst, const float (&o)[16]) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
-    };
-    auto store_aqk = [&](int i, const float (&o)[16]) {        // Aqk leaves as a ready-made [row][column] operand tile (rows past the end: zeros)
-        float lo[8], hi[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { lo[j] = o[j]; hi[j] = o[8 + j]; }
-        store_split8(sTQ, sTQ + 8192, 64, i, 2 * cg, lo);
-        store_split8(sTQ, sTQ + 8192, 64, i, 2 * cg + 1, hi);
-    };
-    if (SCALAR) {                             // lane = row (K rows, then Q rows), cg = 16 columns j: decay applied here, for i >= j only
-        float v[16];
-        umma::tmem_ld16(umma::tmem_addr(tmem, warp, 16 * cg), v);
-        const int i = row & 63;
-        const float gi = sGs[i], bi = q < 2 ? sBeta[i] * sh.rk[i] : p.scale * sh.rq[i];
-        float o[16];
-#pragma unroll
-        for (int j4 = 0; j4 < 16; j4 += 4) {
-            const float4 g4 = *reinterpret_cast<const float4*>(sGs + 16 * cg + j4), r4 = *reinterpret_cast<const float4*>(sh.rk + 16 * cg + j4);
-            const float gj[4] = {g4.x, g4.y, g4.z, g4.w}, rj[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = 16 * cg + j4 + e;
-                const float E = ex2f_(fminf(gi - gj[e], 0.f));
-                const float w = bi * v[j4 + e] * E * rj[e];
-                o[j4 + e] = j < i ? w : j > i ? 0.f : q < 2 ? 1.f : w;
-            }
-        }
-        if (q < 2) store_row16(sM + i * MLD + 16 * cg, o);
-        else store_aqk(i, o);
-    } else {                                  // warp quadrant = row block I (lanes: 16 rows of Gamma, then 16 rows of Q K^T), cg = 16 columns j
-        const int I = q, i = 16 * I + (lane & 15);
-        const bool isq = lane >= 16;
-        float v[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = 0.f;
-        if (cg <= I) umma::tmem_ld16(umma::tmem_addr(tmem, warp, kc_row(I) + 16 * cg), v);      // warp-uniform condition
-        const float bi = isq ? p.scale * sh.rq[i] : sBeta[i] * sh.rk[i];
-        float o[16];
-#pragma unroll
-        for (int j4 = 0; j4 < 16; j4 += 4) {
-            const float4 r4 = *reinterpret_cast<const float4*>(sh.rk + 16 * cg + j4);
-            const float rj[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = 16 * cg + j4 + e;
-                const float w = bi * v[j4 + e] * rj[e];
-                o[j4 + e] = j < i ? w : j > i ? 0.f : isq ? w : 1.f;
-            }
-        }
-        if (isq) store_aqk(i, o);
-        else store_row16(sM + i * MLD + 16 * cg, o);
-    }
-    umma::fence_async_smem();
-    sync_compute();
-    if (tid == STORER) {
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTQ, umma::QUARTER_TILE_BYTES);
-        if (BULK && item + stride < total) {
-            umma::bulk_store_wait_read_but<1>();       // the kbar tile has left
-            load_q(nxt);
-        }
-    }
-    invert_unit_lower(sM, sInv, sh);
-    {   // A as the B operand of phase 3; it also leaves as a ready-made [row][column] operand tile (rows past the end: identity rows)
-        const int r = tid >> 3, k8 = tid & 7;
-        float a8[8];
-        lds8(sInv + r * MLD + k8 * 8, a8);
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-            if (k8 * 8 + e > r) a8[e] = 0.f;
-        store_split8(sTA, sTA + 8192, 64, r, k8, a8);
-    }
-    umma::signal(&sh.op2, lane);
-    if (tid == STORER) {
-        umma::mbar_wait(&sh.op2, it & 1);                  // all of A is there
-        umma::bulk_store(reinterpret_cast<uint8_t*>(p.A) + ((size_t)c * HV + h) * umma::QUARTER_TILE_BYTES, sTA, umma::QUARTER_TILE_BYTES);
-    }
-    // nw^T is read out while the u^T products run
-    umma::wait_mma(&sh.mmN, it & 1);
-    {   // nw^T [K index][tok] leaves as a ready-made chunk tile (the serial kernels fetch it with one bulk copy; token
-        // columns past the end are exact zeros: beta is 0 there)
-        float a[16], n0[8], n1[8];
-        umma::tmem_ld16(umma::tmem_addr(tmem, warp, 128 + 16 * cg), a);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            if (j < 8) n0[j] = -a[j]; else n1[j - 8] = -a[j];
-        }
-        store_split8(base, base + 16384, 128, row, 2 * cg, n0);          // beta k~ is dead
-        store_split8(base, base + 16384, 128, row, 2 * cg + 1, n1);
-    }
-    umma::fence_async_smem();
-    sync_compute();
-    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base, umma::CHUNK_TILE_BYTES);
-    {   // u^T [v][tok] leaves the same way (token columns past the end are exact zeros: A has identity rows there and
-        // beta v zero rows), built next to the nw tile while that one is being copied
-        float b[16], u0[8], u1[8];
-        umma::wait_mma(&sh.mmU, it & 1);
-        umma::tmem_ld16(umma::tmem_addr(tmem, warp, 192 + 16 * cg), b);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { u0[j] = b[j]; u1[j] = b[8 + j]; }
-        store_split8(base + 32768, base + 32768 + 16384, 128, row, 2 * cg, u0);
-        store_split8(base + 32768, base + 32768 + 16384, 128, row, 2 * cg + 1, u1);
-    }
-    umma::fence_async_smem();
-    sync_compute();
-    if (tid == STORER) umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + ((size_t)c * HV + h) * umma::CHUNK_TILE_BYTES, base + 32768, umma::CHUNK_TILE_BYTES);
-    cur = nxt;
-    advance(nxt);
-    }   // items
-    if (tid == STORER) umma::bulk_store_wait_read();
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, 256);
+    if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
 int tc_intra_status(unsigned int* out) {
@@ -562,26 +714,33 @@ int tc_intra_status_clear() {
     return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess ? 0 : -1;
 }
 
-template <int DT, bool SCALAR, bool TMA>
-static int launch_intra_fwd_tc_tt(const MkdaIntraFwd* p, const IntraMaps& maps, cudaStream_t stream) {
-    auto kern = intra_fwd_tc_kernel<DT, SCALAR, TMA>;
-    if (int e = ensure_smem((const void*)kern, INTRA_TC_SMEM, "intra_fwd")) return e;
-    const int items = p->L.NC * p->L.HV;
+template <int DT, bool SCALAR, int YW>
+static int launch_intra_fwd_tc_w(const MkdaIntraFwd* p, cudaStream_t stream) {
+    using W = in::Warps<YW>;
+    auto kern = intra_fwd_tc_kernel<DT, SCALAR, YW>;
+    if (int e = ensure_smem((const void*)kern, in::SMEM, "intra_fwd")) return e;
     static const int regs = kernel_registers((const void*)kern);
-    if (regs < INTRA_LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
-    launch(kern, items < sm_count() ? items : sm_count(), INTRA_THREADS, INTRA_TC_SMEM, stream, *p, maps);
+    if (regs < W::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
+    in::Maps maps;
+    memset(&maps, 0, sizeof(maps));
+    const unsigned long long rows = (unsigned long long)p->L.TT, k_cols = (unsigned long long)p->L.HK * 128, v_cols = (unsigned long long)p->L.HV * 128;
+    constexpr int ES = DT == MKDA_F32 ? 4 : 2;
+    int e = make_rows_map(&maps.k, p->k, ES, rows, k_cols, "intra_fwd");
+    if (!e) e = make_rows_map(&maps.q, p->q, ES, rows, k_cols, "intra_fwd");
+    if (!e && !SCALAR) e = make_rows_map(&maps.g, p->g_c, 4, rows, v_cols, "intra_fwd");
+    if (!e && DT != MKDA_F32) e = make_rows_map(&maps.v, p->v, 2, rows, v_cols, "intra_fwd", CH, 64);
+    if (e) return e;
+    const int items = p->L.NC * p->L.HV;
+    launch(kern, items < sm_count() ? items : sm_count(), W::THREADS, in::SMEM, stream, *p, maps);
     return check_launch("intra_fwd");
 }
+// Eight warps in Y where Y is what is waited for: with a scalar gate, whose X writes a fifth of the operands (4 x 2000 tokens x 16 heads 103 -> 95 us),
+// and with up to four items per SM (fp16 4 x 1000 tokens x 8 heads 50 -> 45 us, 77 tokens 18.4 -> 17.4).  Else X is bound by shared memory, and eight
+// warps cost more than they bring (32 k tokens x 32 heads 825 -> 930 us).  The results are the same bit for bit.
 template <int DT, bool SCALAR>
 static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, cudaStream_t stream) {
-    IntraMaps maps;
-    memset(&maps, 0, sizeof(maps));
-    // 16-bit rows travel by tiled copy when the tensors can be described (16-byte aligned); otherwise through registers
-    if (DT != MKDA_F32 && make_rows_map(&maps.k, p->k, 2, (unsigned long long)p->L.TT, (unsigned long long)p->L.HK * 128, "intra_fwd") == MKDA_OK &&
-        make_rows_map(&maps.q, p->q, 2, (unsigned long long)p->L.TT, (unsigned long long)p->L.HK * 128, "intra_fwd") == MKDA_OK &&
-        (SCALAR || make_rows_map(&maps.g, p->g_c, 4, (unsigned long long)p->L.TT, (unsigned long long)p->L.HV * 128, "intra_fwd") == MKDA_OK))
-        return launch_intra_fwd_tc_tt<DT, SCALAR, true>(p, maps, stream);
-    return launch_intra_fwd_tc_tt<DT, SCALAR, false>(p, maps, stream);
+    if (SCALAR || (long long)p->L.NC * p->L.HV <= 4ll * sm_count()) return launch_intra_fwd_tc_w<DT, SCALAR, 8>(p, stream);
+    return launch_intra_fwd_tc_w<DT, SCALAR, SCALAR ? 8 : 4>(p, stream);
 }
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream) {
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {

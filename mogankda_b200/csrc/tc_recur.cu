@@ -27,6 +27,7 @@ constexpr int SH = 128, SL = 192, VH = 448, VL = 480;      // tensor-memory colu
 constexpr int X = 0, D0 = 256, D1 = 320, O = 384;          // fp32 accumulators: state increment, D (two for the forward kernel), output
 
 using umma::signal_tmem;
+using umma::store_pair;
 using umma::wait_mma;
 
 // 32 bytes of fp32 in one load, `src` 32-byte aligned
@@ -36,15 +37,6 @@ __device__ __forceinline__ void ld32b(const void* src, float* v) {
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src));
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
-}
-// Two neighbouring 16-byte chunks k8, k8 + 1 (k8 even) of row r of an operand tile: they fill one aligned 32-byte piece, in an order that
-// the swizzle takes from the row's parity.
-__device__ __forceinline__ void store_pair(uint8_t* tile, int R, int r, int k8, const uint32_t* w) {
-    uint32_t o[8];
-    const bool odd = r & 1;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { o[i] = odd ? w[4 + i] : w[i]; o[4 + i] = odd ? w[i] : w[4 + i]; }
-    st32b(tile + (umma::tile_chunk_offset(R, r, k8) & ~16u), o);
 }
 // The state <-> caller-visible memory: thread (row, cg) holds columns [32 cg, 32 cg + 32) of row `row` (v).
 __device__ __forceinline__ void load_state(const float* __restrict__ src, bool v_first, int row, int cg, float (&s)[32]) {

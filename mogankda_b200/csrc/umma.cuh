@@ -80,6 +80,16 @@ __device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, in
     *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// Two neighbouring 16-byte chunks k8, k8 + 1 (k8 even) of row r of an operand tile: they fill one aligned 32-byte piece, in an order that
+// the swizzle takes from the row's parity.
+__device__ __forceinline__ void store_pair(uint8_t* tile, int R, int r, int k8, const uint32_t* w) {
+    uint32_t o[8];
+    const bool odd = r & 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { o[i] = odd ? w[4 + i] : w[i]; o[4 + i] = odd ? w[i] : w[4 + i]; }
+    st32b(tile + (tile_chunk_offset(R, r, k8) & ~16u), o);
+}
+
 // reconstruct 8 fp32 values from the hi / lo tiles at (row r, chunk k8)
 __device__ __forceinline__ void load_tile8(const uint8_t* hi, const uint8_t* lo, int R, int r, int k8, float (&v)[8]) {
     const uint32_t off = tile_chunk_offset(R, r, k8);
