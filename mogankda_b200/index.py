@@ -91,17 +91,18 @@ def wants_segments(chunks_per_seq, HV, seg_chunks, sm_count=None, cost_ratio=2.5
     set by the longest sequence (critical path) unless there is so much work that the even share of all chunk steps over
     the SMs is longer still.  Cutting spreads the steps evenly but adds the state + transition pre-pass in the forward
     direction and a second pass in the backward direction, about 2.5 x the serial work over a layer step, plus the prefix
-    combine.  (The 2.5 was measured with earlier serial kernels.  With today's, counters at 45 + 42 + 42 chunks x 16 heads give 444 us for
-    the cut calls against an estimate of 310 uncut, at the kernels' 3.2 + 3.7 us per chunk: the line lies too low for few heads and
-    sequences of 33 to about 75 chunks.)  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
-    warm-up truncation, which shortens the two extra passes to a few chunks wherever the gate decays).  Decided from the
+    combine.  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
+    warm-up truncation, which shortens the two extra passes to a few chunks wherever the gate decays).  With few chains the four passes of a
+    cut call take a segment each however small the share is: about 374 us for segments of 32 chunks, at 2.1 us per chunk for the pre-pass and 3
+    for the others, against 6 us per chunk uncut; without the pre-passes about 205.  So sequences of up to two segments (1.25 where truncation is
+    allowed) are left alone.  45 + 42 + 42 chunks x 16 heads took 415 us in the serial kernels and combines when cut, 280 uncut.  Decided from the
     lengths alone (host), never from data; it plays the role of the reference's intra-card CP decision
     (mogan_kda/ops/gated_delta_rule/chunk/cp/context.py:252-283, cp/autocp/decision.py:54-123)."""
     longest = max(chunks_per_seq, default=0)
     if seg_chunks <= 0 or longest <= seg_chunks:
         return False
     even_share = sum(chunks_per_seq) * HV / (sm_count or _sm_count())
-    return longest > cost_ratio * even_share
+    return longest > max(cost_ratio * even_share, (0.5 + 0.6 * cost_ratio) * seg_chunks)
 
 
 # Entries: (static key, the cu_seqlens tensor itself, its version counter, layout).  The entry keeps the tensor alive
