@@ -141,8 +141,8 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
         const umma::Opnd a_lo = umma::opnd_mn(base + A_, base + A_ + 8192, 64);
         umma::Opnd a_hi = a_lo;                          // rows 0..63 of the operand read the 8 KB in front of each half
         a_hi.hi -= 8192; a_hi.lo -= 8192;
-        umma::gemm(tmem + DW, a_lo, umma::opnd_k(base + W_, base + W_ + 16384, 128), 128, 64, 64, 0u);
-        umma::gemm(tmem + DW + 64, a_hi, umma::opnd_k(base + W_, base + W_ + 16384, 128, 64), 128, 64, 64, 0u);
+        umma::gemm<true>(tmem + DW, a_lo, umma::opnd_k(base + W_, base + W_ + 16384, 128), 128, 64, 64, 0u);
+        umma::gemm<true>(tmem + DW + 64, a_hi, umma::opnd_k(base + W_, base + W_ + 16384, 128, 64), 128, 64, 64, 0u);
         umma::commit(&sh.mmW);
     };
     ItemWalk<SPREAD> w(p.L);
@@ -153,11 +153,11 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
         wait_mma(&sh.opW, par);                          // the dW rows stand below dO; the previous item's accumulators have been read
         fresh();
         const umma::Opnd v_mn = umma::opnd_mn(base + V_, base + V_ + 16384, 128), r_k = umma::opnd_k(base + R_, base + R_ + 32768, 128);
-        umma::gemm(tmem + D1, r_k, v_mn, 128, 64, 128, 0u);
-        umma::gemm(tmem + DQ, umma::opnd_mn(base + S_, base + S_ + 32768, 128), r_k, 128, 128, 128, 0u);
+        umma::gemm<true>(tmem + D1, r_k, v_mn, 128, 64, 128, 0u);
+        umma::gemm<true>(tmem + DQ, umma::opnd_mn(base + S_, base + S_ + 32768, 128), r_k, 128, 128, 128, 0u);
         umma::commit(&sh.mmL);
         umma::mbar_wait(&sh.fullT, par);
-        umma::gemm(tmem + DB, umma::opnd_mn(base + T_, base + T_ + 32768, 128), v_mn, 128, 64, 128, 0u);
+        umma::gemm<true>(tmem + DB, umma::opnd_mn(base + T_, base + T_ + 32768, 128), v_mn, 128, 64, 128, 0u);
         umma::commit(&sh.mmT);
         fresh();
         if (SCALAR) {
@@ -165,9 +165,9 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
             uint8_t* sWD = base + WD_;
             uint8_t* sBd = base + BD_;
             wait_mma(&sh.opI[0], par);
-            umma::gemm(tmem + 0, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_k(sWD, sWD + 16384, 128), 128, 128, 64, 1u);
-            umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 64), umma::opnd_mn(sWD, sWD + 16384, 128, 0), 128, 64, 64, 0u);
-            umma::gemm(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_mn(sBd, sBd + 8192, 64, 0), 128, 64, 64, 1u);
+            umma::gemm<true>(tmem + 0, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_k(sWD, sWD + 16384, 128), 128, 128, 64, 1u);
+            umma::gemm<true>(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 64), umma::opnd_mn(sWD, sWD + 16384, 128, 0), 128, 64, 64, 0u);
+            umma::gemm<true>(tmem + 128, umma::opnd_mn(sKQ, sKQ + 32768, 128, 0), umma::opnd_mn(sBd, sBd + 8192, 64, 0), 128, 64, 64, 1u);
         } else {
 #pragma unroll
             for (int I = 3; I >= 0; --I) {                 // the column tiles arrive block by block, the largest first
@@ -177,8 +177,8 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
                 uint8_t* sWD = base + WD_;
                 const int nj = 16 * (I + 1);
                 // both row terms (dq_row | T) of the block in one N = 32 product, on top of the state terms
-                umma::gemm(tmem + 32 * I, umma::opnd_mn(base + kc_hi(I), base + kc_lo(I), nj), umma::opnd_k(sWD, sWD + 16384, 128, 32 * I), 128, 32, nj, 1u);
-                umma::gemm(tmem + ccol(I), umma::opnd_mn(sKQ, sKQ + 32768, 128, 32 * I), umma::opnd_mn(sWD, sWD + 16384, 128, 32 * I), 128, nj, 32, 0u);
+                umma::gemm<true>(tmem + 32 * I, umma::opnd_mn(base + kc_hi(I), base + kc_lo(I), nj), umma::opnd_k(sWD, sWD + 16384, 128, 32 * I), 128, 32, nj, 1u);
+                umma::gemm<true>(tmem + ccol(I), umma::opnd_mn(sKQ, sKQ + 32768, 128, 32 * I), umma::opnd_mn(sWD, sWD + 16384, 128, 32 * I), 128, nj, 32, 0u);
                 if (I) umma::commit(&sh.mmI[I]);
             }
         }

@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
             auto ahead = [&](int k) {
                 uint8_t* t = base + (k & 1) * DH_SET + 65536;
                 umma::mbar_wait(&sh.fullA[k & 1], (k >> 1) & 1);
-                umma::gemm(tmem + D0, dO_mn(k), umma::opnd_mn(t, t + 8192, 64), 128, 64, 64, 0u);
+                umma::gemm<true>(tmem + D0, dO_mn(k), umma::opnd_mn(t, t + 8192, 64), 128, 64, 64, 0u);
             };
             if (n > 0) ahead(0);
             for (int k = 0; k < n; ++k) {
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
                 umma::gemm_ta(tmem + D0, tmem + SH, tmem + SL, umma::opnd_k(base + DH_K, base + DH_K + 16384, 64), 64, 128, 1u);
                 umma::commit(&sh.mm1);
                 uint8_t* qs = base + (k & 1) * DH_SET + 32768;
-                umma::gemm(tmem + X, dO_mn(k), umma::opnd_mn(qs, qs + 16384, 64), 128, 128, 64, 0u);
+                umma::gemm<true>(tmem + X, dO_mn(k), umma::opnd_mn(qs, qs + 16384, 64), 128, 128, 64, 0u);
                 umma::mbar_wait(&sh.fullN, k & 1);
                 wait_mma(&sh.opV, k & 1);
                 umma::gemm_ta(tmem + X, tmem + VH, tmem + VL, umma::opnd_k(base + DH_N, base + DH_N + 16384, 128), 128, 64, 1u);

@@ -160,6 +160,20 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The same for the second last and the last product in a row with the same A: fetched once
+__device__ __forceinline__ void mma_bf16_fill(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}"
+        :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_bf16_lastuse(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}"
+        :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 // D[M x N] (+)= A B^T over KT (multiple of 16) with the hi/lo split; products whose lo tile is absent are skipped.
 // The four base descriptors are built once; a k-step only adds its byte offset (>> 4) to the start-address field, so
 // the issuing thread spends a handful of instructions per MMA (KT is a literal at every call site: the loop unrolls).
@@ -169,6 +183,10 @@ __device__ __forceinline__ uint64_t opnd_base_desc(const Opnd& o, uint32_t addr)
 __device__ __forceinline__ uint32_t opnd_step16(const Opnd& o, int ks) {       // offset of k-step ks in 16-byte units
     return o.mn ? (uint32_t)(ks * 128) : (uint32_t)(((ks >> 2) * o.blk + (ks & 3) * 32) >> 4);
 }
+// ONE_ISSUER: no other thread of the CTA issues products, so that the high half of A may stay in the collector buffer from its first to its second
+// product: a third of A's fetches less, where shared memory is what bounds the kernel (bwd_chunk 231 -> 223 us at the 1B shape, 1285 -> 1200 for
+// 4 x 16 k tokens x 16 heads with a scalar gate).
+template <bool ONE_ISSUER = false>
 __device__ __forceinline__ void gemm(uint32_t tmem_d, const Opnd& a, const Opnd& b, int M, int N, int KT, uint32_t accumulate) {
     const uint32_t idesc = idesc_bf16(M, N, a.mn, b.mn);
     const uint64_t ah = opnd_base_desc(a, a.hi), al = opnd_base_desc(a, a.lo);
@@ -177,8 +195,13 @@ __device__ __forceinline__ void gemm(uint32_t tmem_d, const Opnd& a, const Opnd&
     for (int ks = 0; ks < KT / 16; ++ks) {
         const uint32_t ao = opnd_step16(a, ks), bo = opnd_step16(b, ks);
         if (a.lo) { mma_bf16(tmem_d, al + ao, bh + bo, idesc, accumulate); accumulate = 1u; }
-        if (b.lo) { mma_bf16(tmem_d, ah + ao, bl + bo, idesc, accumulate); accumulate = 1u; }
-        mma_bf16(tmem_d, ah + ao, bh + bo, idesc, accumulate);
+        if (b.lo) {
+            if (ONE_ISSUER) mma_bf16_fill(tmem_d, ah + ao, bl + bo, idesc, accumulate);
+            else mma_bf16(tmem_d, ah + ao, bl + bo, idesc, accumulate);
+            accumulate = 1u;
+        }
+        if (ONE_ISSUER && b.lo) mma_bf16_lastuse(tmem_d, ah + ao, bh + bo, idesc, accumulate);
+        else mma_bf16(tmem_d, ah + ao, bh + bo, idesc, accumulate);
         accumulate = 1u;
     }
 }
