@@ -78,9 +78,11 @@ __device__ __forceinline__ void advance_state(uint32_t taddr, const float* gl, f
     }
 }
 // the state as the left operand of the next products
-__device__ __forceinline__ void state_operand(uint32_t tmem, int warp, int cg, const float (&s)[32], uint32_t (&h)[16], uint32_t (&l)[16]) {
+__device__ __forceinline__ void state_operand(uint32_t tmem, int warp, int cg, const float (&s)[32], uint32_t (&h)[16], uint32_t (&l)[16],
+                                              uint64_t* used = nullptr, uint32_t parity = 0) {        // `used`: completes once the old one has been read
 #pragma unroll
     for (int i = 0; i < 16; ++i) umma::split2(s[2 * i], s[2 * i + 1], h[i], l[i]);
+    if (used) wait_mma(used, parity);
     umma::tmem_st16(umma::tmem_addr(tmem, warp, SH + cg * 16), h);
     umma::tmem_st16(umma::tmem_addr(tmem, warp, SL + cg * 16), l);
     umma::tmem_wait_st();
@@ -123,7 +125,7 @@ __device__ __forceinline__ void v_operand(uint32_t tmem, int d_col, int warp, in
 // ---------------------------------------------------------------------------------------------------------
 struct RecurShared {
     uint64_t fullN[2], fullK[2], fullU[2], fullQ, fullA;   // landed: nw^T and decay factors | kbar | u^T | scale q 2^g | Aqk
-    uint64_t opS, opV, uFree, mm1, mm2, mmO, oFree;        // state operand | Vd operand written, u^T used; products done; O accumulator read
+    uint64_t opS, opV, uFree, mm1, mm2, mmS, mmO, oFree;   // state operand | Vd operand written, u^T used; products done; O accumulator read
     uint64_t fullG, gFree, ready[2], freed[2];             // gate rows landed | used; state halves staged | read by their copy
     uint32_t tmem;
     __align__(16) float gl[4][DK];                         // four deep: a step's factors are used at the start of the next one
@@ -226,7 +228,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (tid == 0) {
-        for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1, &sh.mm2, &sh.mmO,
+        for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1, &sh.mm2, &sh.mmS, &sh.mmO,
                             &sh.fullG, &sh.freed[0], &sh.freed[1]})
             umma::mbar_init(b, 1);
         for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree, &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, COMPUTE / 32);
@@ -250,10 +252,18 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
         if (w > c_beg) { cut = true; c_beg = trans ? c_end : w; }
     }
     const int n = c_end - c_beg;
-    auto buf_n = [&](int k) { return base + L::N + (k % L::D) * L::T; };
+    const bool save_h = OUT >= 0 && p.h;
+    // Where the chain itself is what takes the time (no norm: a short epilogue), the output's products stand behind the chain's, and without
+    // states to save their place is a second buffer for nw^T, which each step starts with.  In the gap in front of X the products held X up
+    // whenever their tile or their accumulator was late: 5.4 -> 4.7 k cycles per step (scalar gate, 64 chains of 32 steps: 107 -> 95 us; of 256
+    // steps with states saved: 1073 -> 971).  With the norm the epilogue or HBM is the bound, and the other order is faster by 5 %.
+    const bool late = OUT >= 0 && !o.has_norm;
+    const int dn = L::D > 1 || (late && !save_h) ? 2 : 1;
+    auto buf_n = [&](int k) { return base + (L::D > 1 ? L::N + (k & 1) * L::T : (k & 1) && dn == 2 ? L::S : L::N); };
+    auto n_bar = [&](int k) { return &sh.fullN[dn == 2 ? k & 1 : 0]; };
+    auto n_par = [&](int k) { return (uint32_t)(dn == 2 ? k >> 1 : k) & 1; };
     auto buf_k = [&](int k) { return base + L::K + (k % L::D) * L::T; };
     auto buf_u = [&](int k) { return base + L::U + (k % L::D) * L::T; };
-    const bool save_h = OUT >= 0 && p.h;
 
     if (warp >= 16) {
         if (OUT >= 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
@@ -268,7 +278,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                 };
                 auto load_n = [&](int k) {
                     if (k >= n) return;
-                    uint64_t* bar = &sh.fullN[k % L::D];
+                    uint64_t* bar = n_bar(k);
                     umma::mbar_expect_tx(bar, umma::CHUNK_TILE_BYTES + DK * 4);
                     tile(buf_n(k), p.nw, k, umma::CHUNK_TILE_BYTES, bar);
                     umma::bulk_load(sh.gl[k & 3], p.gl + ((size_t)(c_beg + k) * HV + h) * DK, DK * 4, bar);
@@ -282,21 +292,24 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                     tile(base + L::A, o.Aqk, k, umma::QUARTER_TILE_BYTES, &sh.fullA);
                 };
                 load_u(0); load_n(0); load_k(0); load_q(0); load_a(0);
-                if (L::D > 1) { load_n(1); load_u(1); load_k(1); }
+                if (dn > 1) load_n(1);
+                if (L::D > 1) { load_u(1); load_k(1); }
                 if (n > 0) { umma::mbar_wait(&sh.uFree, 0); load_u(L::D); }
                 for (int k = 0; k < n; ++k) {              // each buffer is refilled as soon as its product is done
                     umma::mbar_wait(&sh.mm1, k & 1);
-                    load_n(k + L::D);
+                    load_n(k + dn);
                     if (k + 1 < n) {
                         if (L::D > 1) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 1 + L::D); }
                     }
                     umma::mbar_wait(&sh.mm2, k & 1);
                     load_k(k + L::D);
-                    load_q(k + 1);
                     if (OUT >= 0) {
+                        if (late && k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
+                        umma::mbar_wait(&sh.mmS, k & 1);
+                        load_q(k + 1);
                         umma::mbar_wait(&sh.mmO, k & 1);
                         load_a(k + 1);
-                        if (k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
+                        if (!late && k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
                     }
                 }
             }
@@ -304,20 +317,23 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
         } else if (warp == WARP_MMA) {
             if (umma::elect_one()) {
                 for (int k = 0; k < n; ++k) {
-                    umma::mbar_wait(&sh.fullN[k % L::D], (k / L::D) & 1);
+                    umma::mbar_wait(n_bar(k), n_par(k));
                     wait_mma(&sh.opS, k & 1);
                     umma::gemm_ta(tmem + ((k & 1) ? D1 : D0), tmem + SH, tmem + SL, umma::opnd_mn(buf_n(k), buf_n(k) + 16384, 128), 64, 128, trans ? 0u : 1u);
                     umma::commit(&sh.mm1);
-                    if (OUT >= 0) {
+                    auto output = [&]() {
                         umma::mbar_wait(&sh.fullQ, k & 1);
                         if (k) wait_mma(&sh.oFree, (k - 1) & 1);
                         umma::gemm_ta(tmem + O, tmem + SH, tmem + SL, umma::opnd_k(base + L::Q, base + L::Q + 16384, 64), 64, 128, 0u);
-                    }
+                        umma::commit(&sh.mmS);
+                    };
+                    if (OUT >= 0 && !late) output();
                     umma::mbar_wait(&sh.fullK[k % L::D], (k / L::D) & 1);
                     wait_mma(&sh.opV, k & 1);
                     umma::gemm_ta(tmem + X, tmem + VH, tmem + VL, umma::opnd_mn(buf_k(k), buf_k(k) + 16384, 64), 128, 64, 0u);
                     umma::commit(&sh.mm2);
                     if (OUT >= 0) {
+                        if (late) output();
                         umma::mbar_wait(&sh.fullA, k & 1);
                         umma::gemm_ta(tmem + O, tmem + VH, tmem + VL, umma::opnd_k(base + L::A, base + L::A + 8192, 64), 64, 64, 1u);
                         umma::commit(&sh.mmO);
@@ -370,7 +386,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
         }
         // u^T of step k into the accumulator that its first product adds to
         auto preload_u = [&](int k) {
-            umma::mbar_wait(&sh.fullN[k % L::D], (k / L::D) & 1);      // this thread reads the decay factors that come with nw^T
+            umma::mbar_wait(n_bar(k), n_par(k));                       // this thread reads the decay factors that come with nw^T
             if (!trans) {
                 umma::mbar_wait(&sh.fullU[k % L::D], (k / L::D) & 1);
                 const uint8_t* u = buf_u(k);
@@ -395,7 +411,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                 advance_state(umma::tmem_addr(tmem, warp, X + cg * 32), &sh.gl[(k - 1) & 3][cg * 32], s);
             }
             uint32_t hi[16], lo[16];
-            state_operand(tmem, warp, cg, s, hi, lo);
+            state_operand(tmem, warp, cg, s, hi, lo, late && k ? &sh.mmS : nullptr, (k - 1) & 1);
             signal_tmem(&sh.opS, lane);
             if (save_h) {
                 if (k) umma::mbar_wait(&sh.freed[1], (k - 1) & 1);
