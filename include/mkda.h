@@ -167,6 +167,7 @@ typedef struct {
                                 * as zero without being computed. */
     const int* seg_ht;         /* [NS] row of ht for each segment, -1 = do not store; NULL = identity map */
     int h0_k_first;            /* 1: h0 is [K,V] whatever state_v_first says (states handed between segments) */
+    const int* seg_order;      /* [NS] a permutation: the order in which the segments are started on, or NULL: as they lie */
 } MkdaRecurFwd;
 int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream);
 
@@ -304,6 +305,7 @@ typedef struct {
     float* dh0;                /* [NS,HV,128,128] gradient of the state entering each segment, or NULL */
     const int* warm_end;       /* [NS,HV] from mkda_warmup_chunks, or NULL: a reverse pass from zero (the segment pre-pass)
                                 * may start below this chunk index instead of at the segment's last chunk */
+    const int* seg_order;      /* [NS] a permutation: the order in which the segments are started on, or NULL: as they lie */
 } MkdaBwdDh;
 int mkda_bwd_dh(const MkdaBwdDh* p, void* stream);
 

@@ -78,6 +78,12 @@ bool output_in_chain(const Call& c, bool need_bwd) {
     return fused <= steps * 6.0 + share * (c.has_ep ? 11.0 : 7.0) + 6.0;
 }
 
+// Segments longest first, unless all of them run at once.  In the order of the documents a long one that starts late is waited for at the end:
+// 22 documents of 1 to 19 chunks x 32 heads 156 -> 146 us, 86 of up to 76 chunks 1813 -> 1720 (forward) and 1270 -> 1221 (backward).
+const int* segment_order(const Call& c) {
+    return (int64_t)c.NS * c.HV > at::cuda::getCurrentDeviceProperties()->multiProcessorCount ? c.seg_order : nullptr;
+}
+
 }  // namespace
 
 void run_step(const Call& c, const Inputs& in, Tensor& out, Tensor& ht) {
@@ -163,7 +169,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     const Tensor w = aligned(in.ep_w);
     MkdaChainFwd p{};
     MkdaRecurFwd& r = p.r;
-    r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf;
+    r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf; r.seg_order = segment_order(c);
     if (c.segmented) {
         // pre-pass from zero: per-segment (state, transition); the prefix combine then gives the state entering every segment
         if (c.warm) {
@@ -247,7 +253,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         dy = aligned(dy);
         d.d_o = dy.data_ptr(); d.do_dtype = dtype_code(dy); d.dO_t = dO;
     }
-    d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw;
+    d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw; d.seg_order = segment_order(c);
     if (need_h0) g.h0 = c.states(c.N);
     MkdaBwdDh full = d;
     if (c.segmented) {

@@ -58,8 +58,8 @@ struct Call {
     bool segmented, covers_all, scalar_gate, l2, vf, want_ht, beta_sigmoid, has_ep, warm;
     int mode, act, qkv_dtype;
     float scale, lower_bound, beta_scale, eps, warm_log2;
-    Tensor tables;                         // index.py: seven int32 tables, each padded to a multiple of four entries
-    const int *chunk_start, *chunk_len, *seg_off, *grp_off, *seq_off, *seg_last;
+    Tensor tables;                         // index.py: eight int32 tables, each padded to a multiple of four entries
+    const int *chunk_start, *chunk_len, *seg_off, *grp_off, *seq_off, *seg_last, *seg_order;
     at::Device dev = at::Device(at::kCUDA);
 
     MkdaLayout layout() const { return MkdaLayout{TT, NC, NS, HK, HV, chunk_start, chunk_len, seg_off}; }
@@ -70,6 +70,7 @@ struct Call {
         chunk_start = next(NC); chunk_len = next(NC); seg_off = next(NS + 1); grp_off = next(N + 1); seq_off = next(N + 1);
         next(NS);
         seg_last = next(NS);
+        seg_order = next(NS);
     }
     int64_t tiles(int64_t bytes) const { return (int64_t)NC * HV * bytes; }
     Tensor rows_out(int64_t heads, at::ScalarType dt) const {      // [B,T,heads,128]; tokens outside every sequence are zero

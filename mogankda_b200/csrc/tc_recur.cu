@@ -219,7 +219,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
     RecurShared& sh = *reinterpret_cast<RecurShared*>(base + L::TILES);
     const bool trans = blockIdx.x == 1;
-    const int h = blockIdx.y, seg = blockIdx.z, HV = p.L.HV;
+    const int h = blockIdx.y, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
         follow_stream();
@@ -241,6 +241,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
+    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
 
     // Warm-up truncation (a pass from zero only): where the decay accumulated from chunk warm_start to the segment's end
     // hides everything before it, the pass starts there; the transition is then zero and its CTA visits no chunk.
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
     DhShared& sh = *reinterpret_cast<DhShared*>(base + DH_TILES);
-    const int h = blockIdx.y, seg = blockIdx.z, HV = p.L.HV;
+    const int h = blockIdx.y, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
         follow_stream();
@@ -533,6 +534,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
+    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
 
     // Warm-up truncation (a pass from zero only): the reverse chain starts below chunk warm_end where the decay accumulated
     // over the segment's first chunks hides every later contribution from the segment's entrance.

@@ -33,10 +33,11 @@ class Layout:
     seq_chunk_off: torch.Tensor  # int32 [N+1]  (segments == sequences view)
     seg_first: torch.Tensor     # int32 [NS]: sequence id if the segment opens its sequence, else -1
     seg_last: torch.Tensor      # int32 [NS]: sequence id if the segment closes its sequence, else -1
+    seg_order: torch.Tensor     # int32 [NS]: the segments, longest first
     segmented: bool
     covers_all: bool            # every token of [0, B*T) belongs to a sequence
     host: dict = field(default_factory=dict)
-    tables: torch.Tensor = None  # int32: the seven tables above, one after the other (what the native host path takes)
+    tables: torch.Tensor = None  # int32: the eight tables above, one after the other (what the native host path takes)
     dims: tuple = ()            # (NC, NS, N, segmented, covers_all, tokens of the longest sequence,
     #                             chunks of the longest segment, sequences of 1 to MKDA_STEP_MAX_TOKENS tokens)
 
@@ -72,7 +73,7 @@ def build_tables(B, T, cu, seg_chunks=0):
     seg_first = np.where(j == 0, seq_of, -1)
     seg_last = np.where(j == ns[seq_of] - 1, seq_of, -1)
     tb = dict(chunk_start=start, chunk_len=length, seq_chunk_off=seq_off, seg_chunk_off=seg_off,
-              grp_seg_off=grp_off, seg_first=seg_first, seg_last=seg_last)
+              grp_seg_off=grp_off, seg_first=seg_first, seg_last=seg_last, seg_order=np.argsort(-np.diff(seg_off), kind="stable"))
     return dict({n: t.tolist() for n, t in tb.items()}, N=N, covers_all=int((e - s).sum()) == B * T)
 
 
@@ -141,8 +142,8 @@ def get_layout(B, T, cu_seqlens, device, seg_chunks=0, auto_heads=0, cost_ratio=
                               cost_ratio):
             seg_chunks = 0
     tb = build_tables(B, T, cu, seg_chunks)
-    # one upload for all seven tables, each padded to a multiple of four entries (16 bytes)
-    names = ("chunk_start", "chunk_len", "seg_chunk_off", "grp_seg_off", "seq_chunk_off", "seg_first", "seg_last")
+    # one upload for all eight tables, each padded to a multiple of four entries (16 bytes)
+    names = ("chunk_start", "chunk_len", "seg_chunk_off", "grp_seg_off", "seq_chunk_off", "seg_first", "seg_last", "seg_order")
     flat, at = [], {}
     for n in names:
         at[n] = (len(flat), len(tb[n]))

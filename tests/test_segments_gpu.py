@@ -26,3 +26,24 @@ def test_sequences_around_two_segments(chunks, decay, warm):
     if warm is not None and decay > -1e-3 and chunks > 64:
         exact = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True)
         assert all(torch.equal(t, got[n]) for n, t in exact.items())
+
+
+def test_longest_first_changes_nothing():
+    """More (document, head) chains than SMs are started longest first: every document, its states included, has the bits of its own call."""
+    lens, HV = (70, 1, 200, 64, 129, 0, 70, 333), 32
+    cu = [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, dht, opts, epi = make_inputs(T=cu[-1], HK=16, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi=None, seed=29)
+    lay = get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, 32, HV)
+    assert not lay.segmented and len(lens) * HV > torch.cuda.get_device_properties(0).multi_processor_count
+    assert lay.host["seg_order"] == [7, 2, 4, 0, 6, 1, 3, 5]              # by chunks: 6, 4, 3, 2, 2, 1, 1, 0
+    got = run(mk.chunk_delta_rule, lv, do, dht, opts, epi)
+    for d, n in enumerate(lens):
+        if n == 0:
+            continue
+        s, e = cu[d], cu[d + 1]
+        sub = {k: (t[:, s:e].contiguous() if t.dim() >= 3 and t.shape[1] == cu[-1] else t) for k, t in lv.items()}
+        sub["h0"] = lv["h0"][d:d + 1].contiguous()
+        one = run(mk.chunk_delta_rule, sub, do[:, s:e].contiguous(), dht[d:d + 1].contiguous(), dict(opts, cu_seqlens=None), epi)
+        assert torch.equal(got["ht"][d:d + 1], one["ht"]) and torch.equal(got["dh0"][d:d + 1], one["dh0"])
+        for k in ("o", "dq", "dk", "dv", "dg", "dbeta"):
+            assert torch.equal(got[k][:, s:e], one[k]), (k, d)
