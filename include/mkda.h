@@ -144,7 +144,7 @@ int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream);
 #define MKDA_QUARTER_TILE_BYTES 16384
 
 /* Serial state recurrence per (segment, v-head):  Vd = u + nw S;  S <- diag(gl) S + kbar^T Vd.
- * With want_transition a second CTA per (segment, v-head) carries the segment's K x K transition matrix (same
+ * With want_transition a second chain per (segment, v-head) carries the segment's K x K transition matrix (same
  * recurrence with u = 0 started from the identity).  Replaces the state part of fused_fwd_kda
  * (mogan_kda/ops/kimi_delta_rule/chunk/hopper/fused_fwd.py:523-616) and, for context parallelism, the role of
  * fused_gdr_h (mogan_kda/ops/gated_delta_rule/chunk/blackwell/prepare_h.py:336-403). */

@@ -460,7 +460,224 @@ __global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_k
 template <int OUT>
 __global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const __grid_constant__ ChainMaps maps) { recur_body<OUT>(p.r, p.o, maps); }
 
+// ---------------------------------------------------------------------------------------------------------
+// The pre-pass of a cut call: state from zero and transition of a segment in ONE CTA, when there are more of them than SMs.  A chain of its own
+// waits most of its 3.9 k cycles per step for its own operands, products and barriers (the tensor pipe is busy for 1.5 k, HBM at 3.6 TB/s);
+// two side by side fill each other's gaps and share the nw^T and kbar tiles.  Eight warps per chain (thread = one lane x 64 columns).  Tensor
+// memory has room for both because operands lie where the accumulators were read: 16 columns of an accumulator become the 8 + 8 columns of hi
+// and lo halves of the same 16 terms, by the thread that read them.  Every sum is formed in the order of the single chain: the same bits.
+// 32 k tokens x 32 heads (512 pairs of 32 steps) 450 -> 339 us, 64 k 980 -> 655.  With fewer chains than SMs both run at once anyway, 2.1 us per
+// step instead of 2.7.
+// ---------------------------------------------------------------------------------------------------------
+namespace pr {
+constexpr int THREADS = 640, WARP_MMA = 16, WARP_LOAD = 17, LAUNCH_REGS = 96, T = 32 * rc::KB;
+constexpr int N = 0, K = 2 * T, U = 4 * T, TILES = 6 * T;
+struct Shared {
+    uint64_t fullN[2], fullK[2], fullU[2], uFree;
+    uint64_t opS[2], opV[2], mm1[2], mm2[2];                // per chain: state operand | Vd operand written; products done
+    uint32_t tmem;
+    __align__(16) float gl[4][DK];
+};
+constexpr int SMEM = TILES + (int)sizeof(Shared);
+static_assert(SMEM <= 232448, "shared memory of one CTA");
+// accumulator columns: S and the state increment of chain c; D and V (two for the state, whose D starts as u^T)
+__device__ __forceinline__ int sx(int c) { return 128 * c; }
+__device__ __forceinline__ int dv(int c, int k) { return c ? 384 : 256 + 64 * (k & 1); }
+
+// D (+)= A B^T with A as pairs of 8-column hi and lo groups
+__device__ __forceinline__ void gemm_pairs(uint32_t tmem_d, uint32_t a, const umma::Opnd& b, int N_, int KT, uint32_t accumulate) {
+    const uint32_t idesc = umma::idesc_bf16(128, N_, 0, b.mn);
+    const uint64_t bh = umma::opnd_base_desc(b, b.hi), bl = umma::opnd_base_desc(b, b.lo);
+#pragma unroll
+    for (int ks = 0; ks < KT / 16; ++ks) {
+        const uint32_t bo = umma::opnd_step16(b, ks), ah = a + 16 * ks, al = ah + 8;
+        umma::mma_bf16_ta(tmem_d, al, bh + bo, idesc, accumulate);
+        umma::mma_bf16_ta(tmem_d, ah, bl + bo, idesc, 1u);
+        umma::mma_bf16_ta(tmem_d, ah, bh + bo, idesc, 1u);
+        accumulate = 1u;
+    }
+}
+// 16 values -> their hi and lo groups in the 16 columns at `taddr`
+__device__ __forceinline__ void store_pairs(uint32_t taddr, const float* v) {
+    uint32_t h[8], l[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) umma::split2(v[2 * i], v[2 * i + 1], h[i], l[i]);
+    umma::tmem_st8(taddr, h);
+    umma::tmem_st8(taddr + 8, l);
+}
+}  // namespace pr
+
+__global__ void __launch_bounds__(pr::THREADS, 1) recur_pair_tc_kernel(const MkdaRecurFwd p) {
+    using namespace pr;
+    using umma::signal_tmem;
+    using umma::wait_mma;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
+    Shared& sh = *reinterpret_cast<Shared*>(base + TILES);
+    const int h = blockIdx.y, HV = p.L.HV;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
+        follow_stream();
+        if (tid == 0) atomicExch(&umma::g_timeout_flag, 1u);
+        return;
+    }
+    if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            for (uint64_t* b : {&sh.fullN[i], &sh.fullK[i], &sh.fullU[i], &sh.mm1[i], &sh.mm2[i]}) umma::mbar_init(b, 1);
+            for (uint64_t* b : {&sh.opS[i], &sh.opV[i]}) umma::mbar_init(b, 8);
+        }
+        umma::mbar_init(&sh.uFree, 8);
+        umma::fence_barrier_init();
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = sh.tmem;
+    follow_stream();
+    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
+    const int c_beg = p.L.seg_chunk_off[seg], n = p.L.seg_chunk_off[seg + 1] - c_beg;
+    if (warp >= 16) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if (warp == WARP_LOAD) {
+            if (umma::elect_one()) {
+                auto tile = [&](int off, const float* t, int k, uint64_t* bar) {
+                    umma::bulk_load(base + off + (k & 1) * T, reinterpret_cast<const uint8_t*>(t) + ((size_t)(c_beg + k) * HV + h) * umma::CHUNK_TILE_BYTES,
+                                    umma::CHUNK_TILE_BYTES, bar);
+                };
+                auto load_n = [&](int k) {
+                    if (k >= n) return;
+                    umma::mbar_expect_tx(&sh.fullN[k & 1], umma::CHUNK_TILE_BYTES + DK * 4);
+                    tile(N, p.nw, k, &sh.fullN[k & 1]);
+                    umma::bulk_load(sh.gl[k & 3], p.gl + ((size_t)(c_beg + k) * HV + h) * DK, DK * 4, &sh.fullN[k & 1]);
+                };
+                auto load = [&](int off, const float* t, int k, uint64_t* bars) {
+                    if (k >= n) return;
+                    umma::mbar_expect_tx(&bars[k & 1], umma::CHUNK_TILE_BYTES);
+                    tile(off, t, k, &bars[k & 1]);
+                };
+                for (int k = 0; k < 2; ++k) { load(U, p.u, k, sh.fullU); load_n(k); load(K, p.kbar, k, sh.fullK); }
+                for (int k = 0; k < n; ++k) {              // each buffer is refilled as soon as both chains are done with it
+                    umma::mbar_wait(&sh.uFree, k & 1);
+                    load(U, p.u, k + 2, sh.fullU);
+                    umma::mbar_wait(&sh.mm1[1], k & 1);
+                    load_n(k + 2);
+                    umma::mbar_wait(&sh.mm2[1], k & 1);
+                    load(K, p.kbar, k + 2, sh.fullK);
+                }
+            }
+            __syncwarp();
+        } else if (warp == WARP_MMA) {
+            if (umma::elect_one()) {
+                for (int k = 0; k < n; ++k) {
+                    uint8_t *bn = base + N + (k & 1) * T, *bk = base + K + (k & 1) * T;
+                    umma::mbar_wait(&sh.fullN[k & 1], (k >> 1) & 1);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        wait_mma(&sh.opS[c], k & 1);
+                        gemm_pairs(tmem + dv(c, k), tmem + sx(c), umma::opnd_mn(bn, bn + 16384, 128), 64, 128, c ? 0u : 1u);
+                        umma::commit(&sh.mm1[c]);
+                    }
+                    umma::mbar_wait(&sh.fullK[k & 1], (k >> 1) & 1);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        wait_mma(&sh.opV[c], k & 1);
+                        gemm_pairs(tmem + sx(c), tmem + dv(c, k), umma::opnd_mn(bk, bk + 16384, 64), 128, 64, 0u);
+                        umma::commit(&sh.mm2[c]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        const int c = warp >> 3, half = (warp >> 2) & 1, row = (warp & 3) * 32 + lane, col = 64 * half;
+        float s[64];                                       // columns col .. col + 63 of lane `row`
+#pragma unroll
+        for (int j = 0; j < 64; ++j) s[j] = c && col + j == row ? 1.f : 0.f;
+        auto advance = [&](int k, int b) {                 // s <- s gl + increment of step k, 16 columns
+            float x[16];
+            umma::tmem_ld16(umma::tmem_addr(tmem, warp, sx(c) + col + 16 * b), x);
+            const float* gl = &sh.gl[k & 3][col + 16 * b];
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(gl + j);
+                float* t = s + 16 * b + j;
+                unpack2(fma2(pack2(t[0], t[1]), pack2(f.x, f.y), pack2(x[j], x[j + 1])), t[0], t[1]);
+                unpack2(fma2(pack2(t[2], t[3]), pack2(f.z, f.w), pack2(x[j + 2], x[j + 3])), t[2], t[3]);
+            }
+        };
+        auto preload_u = [&](int k) {                      // u^T of step k into the accumulator that its first product adds to
+            umma::mbar_wait(&sh.fullU[k & 1], (k >> 1) & 1);
+            const uint8_t* u = base + U + (k & 1) * T;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float a[8];
+                umma::load_tile8(u, u + 16384, 128, row, 4 * half + i, a);
+                uint32_t w[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(a[e]);
+                umma::tmem_st8(umma::tmem_addr(tmem, warp, dv(0, k) + 32 * half + 8 * i), w);
+            }
+            umma::tmem_wait_st();
+            signal_tmem(&sh.uFree, lane);
+        };
+        if (c == 0 && n > 0) preload_u(0);
+        for (int k = 0; k < n; ++k) {
+            umma::mbar_wait(&sh.fullN[k & 1], (k >> 1) & 1);           // this thread reads the decay factors that come with nw^T
+            if (k) wait_mma(&sh.mm2[c], (k - 1) & 1);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (k) advance(k - 1, b);
+                store_pairs(umma::tmem_addr(tmem, warp, sx(c) + col + 16 * b), s + 16 * b);
+            }
+            umma::tmem_wait_st();
+            signal_tmem(&sh.opS[c], lane);
+            wait_mma(&sh.mm1[c], k & 1);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                float d[16];
+                const uint32_t at = umma::tmem_addr(tmem, warp, dv(c, k) + 32 * half + 16 * b);
+                umma::tmem_ld16(at, d);
+                store_pairs(at, d);
+            }
+            umma::tmem_wait_st();
+            signal_tmem(&sh.opV[c], lane);
+            if (c == 0 && k + 1 < n) preload_u(k + 1);
+        }
+        if (n > 0) {
+            wait_mma(&sh.mm2[c], (n - 1) & 1);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) advance(n - 1, b);
+        }
+        // transition: M[K out][K in] with this thread holding row `row` = K in; state: [K][V] or [V][K]
+        float* dst = nullptr;
+        if (c) {
+            dst = p.mt + ((size_t)seg * HV + h) * DK * DK;
+        } else if (p.ht) {
+            const int r = p.seg_ht ? p.seg_ht[seg] : seg;
+            if (r >= 0) dst = p.ht + ((size_t)r * HV + h) * DK * DV;
+        }
+        if (dst) {
+            const bool vf = !c && p.state_v_first;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) dst[vf ? (size_t)row * DK + col + j : (size_t)(col + j) * DV + row] = s[j];
+        }
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) umma::tmem_dealloc(tmem, 512);
+}
+
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream) {
+    if (p->want_transition && !p->h && !p->Vd && !p->h0 && !p->warm_start && 2ll * p->L.HV * p->L.NS > sm_count()) {
+        auto pair = recur_pair_tc_kernel;
+        if (int e = ensure_smem((const void*)pair, pr::SMEM, "recur_fwd")) return e;
+        static const int regs = kernel_registers((const void*)pair);
+        if (regs < pr::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "recur_fwd: built with fewer registers than its warps redistribute");
+        launch(pair, dim3(1, p->L.HV, p->L.NS), pr::THREADS, pr::SMEM, stream, *p);
+        return check_launch("recur_fwd");
+    }
     using L = RecurLayout<false>;
     auto kern = recur_fwd_tc_kernel;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "recur_fwd")) return e;

@@ -47,3 +47,21 @@ def test_longest_first_changes_nothing():
         assert torch.equal(got["ht"][d:d + 1], one["ht"]) and torch.equal(got["dh0"][d:d + 1], one["dh0"])
         for k in ("o", "dq", "dk", "dv", "dg", "dbeta"):
             assert torch.equal(got[k][:, s:e], one[k]), (k, d)
+
+
+@pytest.mark.parametrize("lens", [(1,), (64,), (65, 1), (64 * 9 + 1, 0, 130)])
+def test_state_and_transition_in_one_cta(lens):
+    """More than one (segment, head) pair per two SMs: mkda_recur_fwd carries state and transition of a pair in one CTA; with a state to start
+    from (here zero) in two.  Segments of 0 to 3 chunks, ragged ends: the same bits."""
+    from mogankda_b200 import ops
+    cu, HV = [0, *torch.tensor(lens).cumsum(0).tolist()], 80
+    lv, _, _, opts, _ = make_inputs(T=cu[-1], HK=HV, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi=None, h0=False, seed=31)
+    lay = get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, 3)
+    assert 2 * HV * lay.NS > torch.cuda.get_device_properties(0).multi_processor_count
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "kimi", lv["A_log"], lv["dt_bias"], -5.0, HV, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    rq, rk = ops.l2norm_rstd(lv["q"]), ops.l2norm_rstd(lv["k"])
+    _, _, nw, u, kbar, _, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, 128 ** -0.5, HV, HV)
+    kw = dict(store_h=False, store_vd=False, want_transition=True)
+    _, _, ht, mt = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, **kw)
+    _, _, ht2, mt2 = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, h0=torch.zeros(lay.NS, HV, 128, 128, device="cuda"), **kw)
+    assert torch.equal(ht, ht2) and torch.equal(mt, mt2) and torch.isfinite(ht).all() and torch.isfinite(mt).all()
