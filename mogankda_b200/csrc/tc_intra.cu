@@ -20,8 +20,9 @@
 //                            kbar, scale q 2^g and k 2^g tiles
 //   Y, 4 or 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, A diag(beta)
 // and four warps of one working thread each: products of X, products of Y, copies of X, copies of Y.  All are joined by mbarriers.
-// beta is folded into A, so that v itself is the operand: 16-bit rows arrive by a swizzled tiled copy, bf16 ones as a ready-made tile
-// that needs one product less per k-step (it has no low half).
+// bf16: beta is folded into A, so that v itself is the operand, a ready-made tile by a swizzled tiled copy that needs one product less per k-step
+// (it has no low half).  Other types have halves to round anyway: beta goes to v and k 2^g, and the diagonal of A stays exact (with it in A the
+// error against fp64 was 1.08 times as large in fp32 gradients, 1.2 in final states).
 // Shared memory is what X is then bound by (11 to 12 k of the 13 k cycles of an item, 18 k before, move operands, tiles and rows); with few items
 // the latency of an item counts, and twice as many warps in Y shorten it.
 // 6 k packed tokens x 32 heads 240 -> 196 us, 32 k tokens x 32 heads 1110 -> 825, scalar gate 4 x 2000 tokens x 16 heads 129 -> 89.
@@ -304,8 +305,8 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int r = row_of(hf), k8 = c8 + 8 * hf;
-            const float up = SCALAR ? ex2f_(gs[r]) : 1.f, fk = sh.rs[0][r], fq = sh.rs[1][r] * p.scale;
-            const f32x2 sk = both(SCALAR ? fk * ex2f_(gLs - gs[r]) : fk), sq = both(SCALAR ? fq * up : fq), sb = both(SCALAR ? fk * up : fk);
+            const float up = SCALAR ? ex2f_(gs[r]) : 1.f, fk = sh.rs[0][r], fq = sh.rs[1][r] * p.scale, fb = DT == MKDA_BF16 ? fk : fk * beta[r];
+            const f32x2 sk = both(SCALAR ? fk * ex2f_(gLs - gs[r]) : fk), sq = both(SCALAR ? fq * up : fq), sb = both(SCALAR ? fb * up : fb);
             f32x2 t8[4], e8[4], x8[4];
             unpack8<DT>(wk[hf], x8);
             if (SCALAR) {
@@ -491,7 +492,10 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             store_split8(At, At + 8192, 64, r, k8, a8);
             f32x2 ab[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) ab[e] = mul2(pack2(a8[2 * e], a8[2 * e + 1]), b8[e]);
+            for (int e = 0; e < 4; ++e) {
+                ab[e] = pack2(a8[2 * e], a8[2 * e + 1]);
+                if (DT == MKDA_BF16) ab[e] = mul2(ab[e], b8[e]);
+            }
             store_split8(base + AB, base + AB + 8192, 64, r, k8, ab);
         }
         if (DT == MKDA_BF16) {
@@ -502,7 +506,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             }
             umma::signal(&sh.opA, lane);
         } else {
-            // v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
+            // beta v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
             constexpr int N = 32 / YW;
             uint32_t lo[N][4];
             if (DT == MKDA_F16) umma::mbar_wait(&sh.fullV, par);
@@ -520,10 +524,11 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
                     const int i = tid + YT * (m + n), r = i >> 4;
                     float v8[8];
                     unpack8<DT>(raw[n], v8);
+                    const float b = beta[r];
                     uint32_t hi[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        umma::split2(v8[2 * e], v8[2 * e + 1], hi[e], lo[m + n][e]);
+                        umma::split2(b * v8[2 * e], b * v8[2 * e + 1], hi[e], lo[m + n][e]);
                         if (r >= len) hi[e] = lo[m + n][e] = 0u;
                     }
                     *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
