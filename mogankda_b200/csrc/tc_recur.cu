@@ -507,7 +507,7 @@ __device__ __forceinline__ void store_pairs(uint32_t taddr, const float* v) {
 }
 }  // namespace pr
 
-__global__ void __launch_bounds__(pr::THREADS, 1) recur_pair_tc_kernel(const MkdaRecurFwd p) {
+__global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const MkdaRecurFwd p) {
     using namespace pr;
     using umma::signal_tmem;
     using umma::wait_mma;
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_pair_tc_kernel(const Mkd
 
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream) {
     if (p->want_transition && !p->h && !p->Vd && !p->h0 && !p->warm_start && 2ll * p->L.HV * p->L.NS > sm_count()) {
-        auto pair = recur_pair_tc_kernel;
+        auto pair = recur_fwd_pair_tc_kernel;
         if (int e = ensure_smem((const void*)pair, pr::SMEM, "recur_fwd")) return e;
         static const int regs = kernel_registers((const void*)pair);
         if (regs < pr::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "recur_fwd: built with fewer registers than its warps redistribute");
