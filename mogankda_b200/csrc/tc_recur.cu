@@ -473,8 +473,9 @@ namespace pr {
 constexpr int THREADS = 640, WARP_MMA = 16, WARP_LOAD = 17, LAUNCH_REGS = 96, T = 32 * rc::KB;
 constexpr int N = 0, K = 2 * T, U = 4 * T, TILES = 6 * T;
 struct Shared {
-    uint64_t fullN[2], fullK[2], fullU[2], uFree;
-    uint64_t opS[2], opV[2], mm1[2], mm2[2];                // per chain: state operand | Vd operand written; products done
+    // One barrier per buffer (k & 1): its next phase needs the copy that the wait for this one releases, however late the copying thread comes.
+    uint64_t fullN[2], fullK[2], fullU[2], uFree[2];
+    uint64_t opS[2], opV[2], mm1[2][2], mm2[2][2];          // per chain: state operand | Vd operand written; products done
     uint32_t tmem;
     __align__(16) float gl[4][DK];
 };
@@ -524,10 +525,9 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
-            for (uint64_t* b : {&sh.fullN[i], &sh.fullK[i], &sh.fullU[i], &sh.mm1[i], &sh.mm2[i]}) umma::mbar_init(b, 1);
-            for (uint64_t* b : {&sh.opS[i], &sh.opV[i]}) umma::mbar_init(b, 8);
+            for (uint64_t* b : {&sh.fullN[i], &sh.fullK[i], &sh.fullU[i], &sh.mm1[0][i], &sh.mm1[1][i], &sh.mm2[0][i], &sh.mm2[1][i]}) umma::mbar_init(b, 1);
+            for (uint64_t* b : {&sh.opS[i], &sh.opV[i], &sh.uFree[i]}) umma::mbar_init(b, 8);
         }
-        umma::mbar_init(&sh.uFree, 8);
         umma::fence_barrier_init();
     }
     umma::fence_before_sync();
@@ -558,11 +558,11 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
                 };
                 for (int k = 0; k < 2; ++k) { load(U, p.u, k, sh.fullU); load_n(k); load(K, p.kbar, k, sh.fullK); }
                 for (int k = 0; k < n; ++k) {              // each buffer is refilled as soon as both chains are done with it
-                    umma::mbar_wait(&sh.uFree, k & 1);
+                    umma::mbar_wait(&sh.uFree[k & 1], (k >> 1) & 1);
                     load(U, p.u, k + 2, sh.fullU);
-                    umma::mbar_wait(&sh.mm1[1], k & 1);
+                    umma::mbar_wait(&sh.mm1[1][k & 1], (k >> 1) & 1);
                     load_n(k + 2);
-                    umma::mbar_wait(&sh.mm2[1], k & 1);
+                    umma::mbar_wait(&sh.mm2[1][k & 1], (k >> 1) & 1);
                     load(K, p.kbar, k + 2, sh.fullK);
                 }
             }
@@ -576,14 +576,14 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
                     for (int c = 0; c < 2; ++c) {
                         wait_mma(&sh.opS[c], k & 1);
                         gemm_pairs(tmem + dv(c, k), tmem + sx(c), umma::opnd_mn(bn, bn + 16384, 128), 64, 128, c ? 0u : 1u);
-                        umma::commit(&sh.mm1[c]);
+                        umma::commit(&sh.mm1[c][k & 1]);
                     }
                     umma::mbar_wait(&sh.fullK[k & 1], (k >> 1) & 1);
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         wait_mma(&sh.opV[c], k & 1);
                         gemm_pairs(tmem + sx(c), tmem + dv(c, k), umma::opnd_mn(bk, bk + 16384, 64), 128, 64, 0u);
-                        umma::commit(&sh.mm2[c]);
+                        umma::commit(&sh.mm2[c][k & 1]);
                     }
                 }
             }
@@ -620,12 +620,12 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
                 umma::tmem_st8(umma::tmem_addr(tmem, warp, dv(0, k) + 32 * half + 8 * i), w);
             }
             umma::tmem_wait_st();
-            signal_tmem(&sh.uFree, lane);
+            signal_tmem(&sh.uFree[k & 1], lane);
         };
         if (c == 0 && n > 0) preload_u(0);
         for (int k = 0; k < n; ++k) {
             umma::mbar_wait(&sh.fullN[k & 1], (k >> 1) & 1);           // this thread reads the decay factors that come with nw^T
-            if (k) wait_mma(&sh.mm2[c], (k - 1) & 1);
+            if (k) wait_mma(&sh.mm2[c][(k - 1) & 1], ((k - 1) >> 1) & 1);
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 if (k) advance(k - 1, b);
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
             }
             umma::tmem_wait_st();
             signal_tmem(&sh.opS[c], lane);
-            wait_mma(&sh.mm1[c], k & 1);
+            wait_mma(&sh.mm1[c][k & 1], (k >> 1) & 1);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 float d[16];
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
             if (c == 0 && k + 1 < n) preload_u(k + 1);
         }
         if (n > 0) {
-            wait_mma(&sh.mm2[c], (n - 1) & 1);
+            wait_mma(&sh.mm2[c][(n - 1) & 1], ((n - 1) >> 1) & 1);
 #pragma unroll
             for (int b = 0; b < 4; ++b) advance(n - 1, b);
         }

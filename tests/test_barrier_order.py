@@ -1,0 +1,176 @@
+"""CPU: no wait of the warp-specialised kernels rests on timing.
+
+An mbarrier is waited for by the parity of a phase: the wait has to be made before the NEXT phase of the barrier completes, or it blocks on the phase
+after that.  So for every wait something must keep the next phase from completing until the waiter has passed.  The roles of the kernels that carry
+the state are restated here as sequences of arrivals and waits; every role is held in front of each of its waits while all
+others run as far as they can (copies and products complete at once), and the barrier it is held at must not have gone past the phase it waits for.
+The system is monotone, so this covers every schedule.
+
+How many barriers stand behind a name (one per buffer slot, or one in all) is read from the kernels' shared structs.  Warps that act alike are two
+agents, so that one of them may be late.
+"""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mogankda_b200", "csrc")
+STEPS = 7
+
+
+def _slots(source, struct):
+    """{barrier: barriers per chain or item} of the uint64_t members of a kernel's shared struct."""
+    text = open(os.path.join(CSRC, source)).read()
+    body = re.search(r"struct %s \{(.*?)\n\};" % struct, text, re.S)[1]
+    found = {}
+    for line in re.findall(r"uint64_t ([^;]*);", body):
+        for name, dims in re.findall(r"(\w+)((?:\[\d+\])*)", line):
+            found[name] = [int(d) for d in re.findall(r"\d+", dims)]
+    return found
+
+
+class Roles:
+    """Agents: name -> [("wait" | "arrive", barrier, phase)].  `slots`: barriers behind a name that takes a step number."""
+
+    def __init__(self, slots):
+        self.slots, self.count, self.agents = slots, {}, {}
+
+    def at(self, name, k):
+        n = self.slots.get(name, 1)
+        return (name, k % n), k // n
+
+    def agent(self, name):
+        ops = self.agents.setdefault(name, [])
+
+        def wait(bar, k):
+            ops.append(("wait", *self.at(bar, k)))
+
+        def arrive(bar, k):
+            ops.append(("arrive", self.at(bar, k)[0], None))
+        return wait, arrive
+
+    def run(self, held=None, at=None):
+        """Arrivals per barrier when nobody can go on; every agent has to come to its end if none is held."""
+        pos, got = dict.fromkeys(self.agents, 0), {}
+        moved = True
+        while moved:
+            moved = False
+            for name, ops in self.agents.items():
+                while pos[name] < len(ops) and not (name == held and pos[name] == at):
+                    what, bar, phase = ops[pos[name]]
+                    if what == "wait":
+                        if got.get(bar, 0) // self.count.get(bar[0], 1) <= phase:
+                            break
+                    else:
+                        got[bar] = got.get(bar, 0) + 1
+                    pos[name] += 1
+                    moved = True
+        if held is None:
+            assert all(pos[n] == len(ops) for n, ops in self.agents.items()), {n: ops[pos[n]] for n, ops in self.agents.items() if pos[n] < len(ops)}
+        return got
+
+    def late_waits(self):
+        """The waits that could be made too late: (agent, barrier)."""
+        self.run()
+        bad = set()
+        for name, ops in self.agents.items():
+            for i, (what, bar, phase) in enumerate(ops):
+                if what == "wait" and not bar[0].startswith("sync"):
+                    if self.run(name, i).get(bar, 0) // self.count.get(bar[0], 1) > phase + 1:
+                        bad.add((name, bar[0]))
+        return sorted(bad)
+
+
+def _per_step(dims, chains=1):
+    """Barriers per step: the last dimension of an array (the first one of a pair's is the chain)."""
+    return {n: (d[-1] if len(d) == chains else 1) for n, d in dims.items()}
+
+
+def pair(dims, n=STEPS):
+    """recur_fwd_pair: two chains (0: state, 1: transition) with common tiles, all double-buffered."""
+    slots = {}
+    for name in ("fullN", "fullK", "fullU", "uFree"):
+        slots[name] = dims[name][0] if dims[name] else 1
+    for name in ("opS", "opV", "mm1", "mm2"):
+        for c in range(2):
+            slots[f"{name}{c}"] = dims[name][1] if len(dims[name]) > 1 else 1
+    r = Roles(slots)
+    r.count = {"uFree": 2, **{f"op{x}{c}": 2 for x in "SV" for c in range(2)}}
+    wait, arrive = r.agent("load")
+
+    def load(bar, k):
+        if k < n:
+            arrive(bar, k)
+    for k in range(2):
+        load("fullU", k), load("fullN", k), load("fullK", k)
+    for k in range(n):
+        wait("uFree", k), load("fullU", k + 2)
+        wait("mm11", k), load("fullN", k + 2)
+        wait("mm21", k), load("fullK", k + 2)
+    wait, arrive = r.agent("mma")
+    for k in range(n):
+        wait("fullN", k)
+        for c in "01":
+            wait("opS" + c, k), arrive("mm1" + c, k)
+        wait("fullK", k)
+        for c in "01":
+            wait("opV" + c, k), arrive("mm2" + c, k)
+    for c in "01":
+        for w in "ab":
+            wait, arrive = r.agent(f"chain{c}{w}")
+
+            def preload_u(k):
+                if c == "0" and k < n:
+                    wait("fullU", k), arrive("uFree", k)
+            preload_u(0)
+            for k in range(n):
+                wait("fullN", k)
+                if k:
+                    wait("mm2" + c, k - 1)
+                arrive("opS" + c, k)
+                wait("mm1" + c, k)
+                arrive("opV" + c, k)
+                preload_u(k + 1)
+            wait("mm2" + c, n - 1)
+    return r
+
+
+def reverse(dims, n=STEPS):
+    """bwd_dh."""
+    r = Roles({k: (d[0] if d else 1) for k, d in dims.items()})
+    r.count = {"opS": 2, "opV": 2}
+    wait, arrive = r.agent("load")
+    arrive("fullA", 0), arrive("fullK", 0), arrive("fullN", 0), arrive("fullA", 1)
+    for k in range(n - 1):
+        wait("mm1", k), arrive("fullK", k + 1)
+        wait("mm2", k), arrive("fullN", k + 1)
+        if k + 2 < n:
+            arrive("fullA", k + 2)
+    wait, arrive = r.agent("mma")
+    wait("fullA", 0)
+    for k in range(n):
+        wait("fullK", k), wait("opS", k), arrive("mm1", k)
+        wait("fullN", k), wait("opV", k), arrive("mm2", k)
+        if k + 1 < n:
+            wait("fullA", k + 1)
+    for w in "ab":
+        wait, arrive = r.agent("state" + w)
+        for k in range(n):
+            if k:
+                wait("mm2", k - 1)
+            arrive("opS", k)
+            wait("fullA", k), wait("mm1", k), arrive("opV", k)
+        wait("mm2", n - 1)
+    return r
+
+
+def test_a_wait_that_rests_on_timing_is_found():
+    """The pair kernel with one barrier in all for u^T used and for each product: the copying thread may come to its waits two phases late."""
+    dims = dict(fullN=[2], fullK=[2], fullU=[2], uFree=[], opS=[2], opV=[2], mm1=[2], mm2=[2])
+    assert ("load", "uFree") in pair(dims).late_waits()
+
+
+def test_recur_fwd_pair():
+    assert pair(_slots("tc_recur.cu", "Shared")).late_waits() == []
+
+
+def test_bwd_dh():
+    assert reverse(_slots("tc_recur.cu", "DhShared")).late_waits() == []
