@@ -125,7 +125,9 @@ __device__ __forceinline__ void v_operand(uint32_t tmem, int d_col, int warp, in
 // ---------------------------------------------------------------------------------------------------------
 struct RecurShared {
     uint64_t fullN[2], fullK[2], fullU[2], fullQ, fullA;   // landed: nw^T and decay factors | kbar | u^T | scale q 2^g | Aqk
-    uint64_t opS, opV, uFree, mm1, mm2, mmS, mmO, oFree;   // state operand | Vd operand written, u^T used; products done; O accumulator read
+    uint64_t opS, opV, mmS, mmO, oFree;                    // state operand | Vd operand written; output products done; O accumulator read
+    uint64_t uFree[2], mm1[2], mm2[2];                     // u^T used; the chain's products done.  Of even and odd steps: where their tiles have two
+                                                           // buffers, the next step's could complete before the copying thread waits for this one's
     uint64_t fullG, gFree, ready[2], freed[2];             // gate rows landed | used; state halves staged | read by their copy
     uint32_t tmem;
     __align__(16) float gl[4][DK];                         // four deep: a step's factors are used at the start of the next one
@@ -228,10 +230,10 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (tid == 0) {
-        for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1, &sh.mm2, &sh.mmS, &sh.mmO,
-                            &sh.fullG, &sh.freed[0], &sh.freed[1]})
+        for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1[0], &sh.mm1[1],
+                            &sh.mm2[0], &sh.mm2[1], &sh.mmS, &sh.mmO, &sh.fullG, &sh.freed[0], &sh.freed[1]})
             umma::mbar_init(b, 1);
-        for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree, &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, COMPUTE / 32);
+        for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree[0], &sh.uFree[1], &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, COMPUTE / 32);
         umma::mbar_init(&sh.oFree, 4);
         umma::mbar_init(&sh.gFree, 4);
         umma::fence_barrier_init();
@@ -263,6 +265,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     auto buf_n = [&](int k) { return base + (L::D > 1 ? L::N + (k & 1) * L::T : (k & 1) && dn == 2 ? L::S : L::N); };
     auto n_bar = [&](int k) { return &sh.fullN[dn == 2 ? k & 1 : 0]; };
     auto n_par = [&](int k) { return (uint32_t)(dn == 2 ? k >> 1 : k) & 1; };
+    auto step_par = [](int k) { return (uint32_t)(k >> 1) & 1; };      // of the barriers of even and odd steps
     auto buf_k = [&](int k) { return base + L::K + (k % L::D) * L::T; };
     auto buf_u = [&](int k) { return base + L::U + (k % L::D) * L::T; };
 
@@ -295,22 +298,21 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                 load_u(0); load_n(0); load_k(0); load_q(0); load_a(0);
                 if (dn > 1) load_n(1);
                 if (L::D > 1) { load_u(1); load_k(1); }
-                if (n > 0) { umma::mbar_wait(&sh.uFree, 0); load_u(L::D); }
+                if (n > 0) { umma::mbar_wait(&sh.uFree[0], 0); load_u(L::D); }
                 for (int k = 0; k < n; ++k) {              // each buffer is refilled as soon as its product is done
-                    umma::mbar_wait(&sh.mm1, k & 1);
+                    auto u_free = [&]() { umma::mbar_wait(&sh.uFree[(k + 1) & 1], step_par(k + 1)); };
+                    umma::mbar_wait(&sh.mm1[k & 1], step_par(k));
                     load_n(k + dn);
-                    if (k + 1 < n) {
-                        if (L::D > 1) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 1 + L::D); }
-                    }
-                    umma::mbar_wait(&sh.mm2, k & 1);
+                    if (L::D > 1 && k + 1 < n) { u_free(); load_u(k + 1 + L::D); }
+                    umma::mbar_wait(&sh.mm2[k & 1], step_par(k));
                     load_k(k + L::D);
                     if (OUT >= 0) {
-                        if (late && k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
+                        if (late && k + 1 < n) { u_free(); load_u(k + 2); }
                         umma::mbar_wait(&sh.mmS, k & 1);
                         load_q(k + 1);
                         umma::mbar_wait(&sh.mmO, k & 1);
                         load_a(k + 1);
-                        if (!late && k + 1 < n) { umma::mbar_wait(&sh.uFree, (k + 1) & 1); load_u(k + 2); }
+                        if (!late && k + 1 < n) { u_free(); load_u(k + 2); }
                     }
                 }
             }
@@ -321,7 +323,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                     umma::mbar_wait(n_bar(k), n_par(k));
                     wait_mma(&sh.opS, k & 1);
                     umma::gemm_ta(tmem + ((k & 1) ? D1 : D0), tmem + SH, tmem + SL, umma::opnd_mn(buf_n(k), buf_n(k) + 16384, 128), 64, 128, trans ? 0u : 1u);
-                    umma::commit(&sh.mm1);
+                    umma::commit(&sh.mm1[k & 1]);
                     auto output = [&]() {
                         umma::mbar_wait(&sh.fullQ, k & 1);
                         if (k) wait_mma(&sh.oFree, (k - 1) & 1);
@@ -332,7 +334,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                     umma::mbar_wait(&sh.fullK[k % L::D], (k / L::D) & 1);
                     wait_mma(&sh.opV, k & 1);
                     umma::gemm_ta(tmem + X, tmem + VH, tmem + VL, umma::opnd_mn(buf_k(k), buf_k(k) + 16384, 64), 128, 64, 0u);
-                    umma::commit(&sh.mm2);
+                    umma::commit(&sh.mm2[k & 1]);
                     if (OUT >= 0) {
                         if (late) output();
                         umma::mbar_wait(&sh.fullA, k & 1);
@@ -402,13 +404,13 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
                 }
                 umma::tmem_wait_st();
             }
-            signal_tmem(&sh.uFree, lane);
+            signal_tmem(&sh.uFree[k & 1], lane);
         };
         if (n > 0) preload_u(0);
         for (int k = 0; k < n; ++k) {
             const size_t it = (size_t)(c_beg + k) * HV + h;
             if (k) {
-                wait_mma(&sh.mm2, (k - 1) & 1);
+                wait_mma(&sh.mm2[(k - 1) & 1], step_par(k - 1));
                 advance_state(umma::tmem_addr(tmem, warp, X + cg * 32), &sh.gl[(k - 1) & 3][cg * 32], s);
             }
             uint32_t hi[16], lo[16];
@@ -421,7 +423,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
             } else if (OUT < 0 && p.h && !trans) {
                 save_state_tile(reinterpret_cast<uint8_t*>(p.h) + it * umma::STATE_TILE_BYTES, row, cg, hi, lo);
             }
-            wait_mma(&sh.mm1, k & 1);
+            wait_mma(&sh.mm1[k & 1], step_par(k));
             {
                 uint32_t vh[8], vl[8];
                 v_operand(tmem, (k & 1) ? D1 : D0, warp, cg, vh, vl);
@@ -440,7 +442,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
             if (k + 1 < n) preload_u(k + 1);
         }
         if (n > 0) {
-            wait_mma(&sh.mm2, (n - 1) & 1);
+            wait_mma(&sh.mm2[(n - 1) & 1], step_par(n - 1));
             advance_state(umma::tmem_addr(tmem, warp, X + cg * 32), &sh.gl[(n - 1) & 3][cg * 32], s);
         }
         // transition: M[K out][K in] with this thread holding row `row` = K in; state: [K][V] or [V][K]

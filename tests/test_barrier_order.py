@@ -12,6 +12,8 @@ agents, so that one of them may be late.
 import os
 import re
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mogankda_b200", "csrc")
 STEPS = 7
 
@@ -79,11 +81,6 @@ class Roles:
         return sorted(bad)
 
 
-def _per_step(dims, chains=1):
-    """Barriers per step: the last dimension of an array (the first one of a pair's is the chain)."""
-    return {n: (d[-1] if len(d) == chains else 1) for n, d in dims.items()}
-
-
 def pair(dims, n=STEPS):
     """recur_fwd_pair: two chains (0: state, 1: transition) with common tiles, all double-buffered."""
     slots = {}
@@ -133,6 +130,100 @@ def pair(dims, n=STEPS):
     return r
 
 
+def chain(dims, out, norm=False, save_h=False, n=STEPS):
+    """recur_fwd (out = False: every tile double-buffered) and chain_fwd (one buffer each; without a norm and without states to save two of nw^T)."""
+    late = out and not norm
+    D = 1 if out else 2
+    dn = 2 if D == 2 or (late and not save_h) else 1
+    slots = {k: (d[0] if d else 1) for k, d in dims.items()}
+    slots.update(fullN=dn, fullK=D, fullU=D, ready=1, freed=1)
+    r = Roles(slots)
+    r.count = {"opS": 2, "opV": 2, "uFree": 2, "oFree": 2, "gFree": 2, "ready0": 2, "ready1": 2}
+    wait, arrive = r.agent("load")
+
+    def load(bar, k):
+        if k < n:
+            arrive(bar, k)
+    load("fullU", 0), load("fullN", 0), load("fullK", 0)
+    if out:
+        load("fullQ", 0), load("fullA", 0)
+    if dn > 1:
+        load("fullN", 1)
+    if D > 1:
+        load("fullU", 1), load("fullK", 1)
+    wait("uFree", 0), load("fullU", D)
+    for k in range(n):
+        wait("mm1", k), load("fullN", k + dn)
+        if k + 1 < n and D > 1:
+            wait("uFree", k + 1), load("fullU", k + 1 + D)
+        wait("mm2", k), load("fullK", k + D)
+        if out:
+            if late and k + 1 < n:
+                wait("uFree", k + 1), load("fullU", k + 2)
+            wait("mmS", k), load("fullQ", k + 1)
+            wait("mmO", k), load("fullA", k + 1)
+            if not late and k + 1 < n:
+                wait("uFree", k + 1), load("fullU", k + 2)
+    wait, arrive = r.agent("mma")
+
+    def output(k):
+        wait("fullQ", k)
+        if k:
+            wait("oFree", k - 1)
+        arrive("mmS", k)
+    for k in range(n):
+        wait("fullN", k), wait("opS", k), arrive("mm1", k)
+        if out and not late:
+            output(k)
+        wait("fullK", k), wait("opV", k), arrive("mm2", k)
+        if out:
+            if late:
+                output(k)
+            wait("fullA", k), arrive("mmO", k)
+    if out:
+        for w in "ab":
+            wait, arrive = r.agent("epilogue" + w)
+            for k in range(n):
+                if norm:
+                    wait("fullG", k)
+                wait("mmO", k), arrive("oFree", k), arrive("gFree", k)
+        if norm:
+            wait, arrive = r.agent("gate")
+            for k in range(n):
+                if k:
+                    wait("gFree", k - 1)
+                arrive("fullG", k)
+        if save_h:
+            wait, arrive = r.agent("store")
+            for k in range(n):
+                for hf in "01":
+                    wait("ready" + hf, k), arrive("freed" + hf, k)
+    for w in "ab":
+        wait, arrive = r.agent("state" + w)
+
+        def preload_u(k):
+            wait("fullN", k), wait("fullU", k), arrive("uFree", k)
+        preload_u(0)
+        for k in range(n):
+            if k:
+                wait("mm2", k - 1)
+                if late:
+                    wait("mmS", k - 1)
+            arrive("opS", k)
+            if save_h:
+                if k:
+                    wait("freed1", k - 1)
+                arrive("ready0", k)
+            wait("mm1", k)
+            arrive("opV", k)
+            if save_h:
+                wait("freed0", k), arrive("ready1", k)
+            if k + 1 < n:
+                preload_u(k + 1)
+        wait("mm2", n - 1)
+    return r
+
+
 def reverse(dims, n=STEPS):
     """bwd_dh."""
     r = Roles({k: (d[0] if d else 1) for k, d in dims.items()})
@@ -170,6 +261,11 @@ def test_a_wait_that_rests_on_timing_is_found():
 
 def test_recur_fwd_pair():
     assert pair(_slots("tc_recur.cu", "Shared")).late_waits() == []
+
+
+@pytest.mark.parametrize("out,norm,save_h", [(False, False, False), (True, True, False), (True, True, True), (True, False, False), (True, False, True)])
+def test_recur_fwd_and_chain_fwd(out, norm, save_h):
+    assert chain(_slots("tc_recur.cu", "RecurShared"), out, norm, save_h).late_waits() == []
 
 
 def test_bwd_dh():
