@@ -64,7 +64,8 @@ constexpr int D1 = 0, D1_COLS = 160, NW = 320, U = 384;      // accumulator colu
 
 struct Shared {
     uint64_t ldin, fullV;                                   // rows | v landed
-    uint64_t op1[2], mm1;                                   // operands of channel half 0, 1 written; [Gamma; Q K^T] done
+    uint64_t op1[2], mm1[2];                                // operands of channel half 0, 1 written; [Gamma; Q K^T] done, one per accumulator buffer:
+                                                            // a scalar gate's can be done for the next item before Y comes to wait for this one's
     uint64_t rows, acc, hand, khFree;                       // row scales | Aqk | kbar, scale q 2^g, k 2^g written; the first two tiles and Aqk have left
     uint64_t opA, opV, mmV, mmN, mmU;                       // A diag(beta) written | (v in two halves: low half written, high half used) | nw^T, u^T done
     uint64_t nwReady, uReady, bkFree, abFree;               // nw^T, u^T staged | have left
@@ -298,7 +299,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
         __syncwarp();
         if (lane == 0) umma::arrive(&sh.rows);
         if (it) read_out(it - 1);
-        umma::wait_mma(&sh.mm1, par);
+        umma::wait_mma(&sh.mm1[par], (it >> 1) & 1);
         umma::mbar_wait(&sh.rows, par);
         // ---- over the dead operands: the state kernels' scaled operands, kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g; k 2^g for Y ----
         const float gLs = SCALAR ? gs[CH - 1] : 0.f;
@@ -417,7 +418,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
         // ---- I + L and Aqk from the accumulators ----
         // per channel: warp quadrant = row block (16 rows of Gamma, then 16 rows of Q K^T); scalar gate: 64 rows of K K^T, then of Q K^T
         umma::mbar_wait(&sh.rows, par);
-        umma::wait_mma(&sh.mm1, par);
+        umma::wait_mma(&sh.mm1[par], (it >> 1) & 1);
         const int len = sh.info[it & 3].len;
         {
             const int i = SCALAR ? (q & 1) * 32 + lane : 16 * q + (lane & 15);
@@ -575,7 +576,7 @@ __device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, 
                 umma::gemm(tmem + D1 + (it & 1) * D1_COLS, umma::opnd_k(kq, kq + 32768, 128), umma::opnd_k(kc, kc + KC_BYTES, KC_ROWS), 128, KC_ROWS, 64, hf);
             }
         }
-        umma::commit(&sh.mm1);
+        umma::commit(&sh.mm1[it & 1]);
     }
 }
 template <int DT>
@@ -626,7 +627,7 @@ __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Ma
     for (int it = 0; w.valid(); ++it) {
         const size_t item = w.item();
         w.next();
-        umma::mbar_wait(&sh.mm1, it & 1);                   // the operands are dead
+        umma::mbar_wait(&sh.mm1[it & 1], (it >> 1) & 1);    // the operands are dead
         if (w.valid()) load_rows(w, it + 1);
         umma::mbar_wait(&sh.acc, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + item * umma::QUARTER_TILE_BYTES, base + AQ, umma::QUARTER_TILE_BYTES);
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel
     }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (threadIdx.x == 0) {
-        for (uint64_t* b : {&sh.ldin, &sh.fullV, &sh.mm1, &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.ldin, &sh.fullV, &sh.mm1[0], &sh.mm1[1], &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
         for (uint64_t* b : {&sh.op1[0], &sh.op1[1], &sh.rows, &sh.hand, &sh.nwReady, &sh.uReady}) umma::mbar_init(b, X_WARPS);
         for (uint64_t* b : {&sh.opA, &sh.opV, &sh.acc}) umma::mbar_init(b, YW);
         umma::fence_barrier_init();

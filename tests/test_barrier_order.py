@@ -2,7 +2,7 @@
 
 An mbarrier is waited for by the parity of a phase: the wait has to be made before the NEXT phase of the barrier completes, or it blocks on the phase
 after that.  So for every wait something must keep the next phase from completing until the waiter has passed.  The roles of the kernels that carry
-the state are restated here as sequences of arrivals and waits; every role is held in front of each of its waits while all
+the state and of the WY preparation are restated here as sequences of arrivals and waits; every role is held in front of each of its waits while all
 others run as far as they can (copies and products complete at once), and the barrier it is held at must not have gone past the phase it waits for.
 The system is monotone, so this covers every schedule.
 
@@ -253,6 +253,89 @@ def reverse(dims, n=STEPS):
     return r
 
 
+def intra(dims, dtype, scalar, n=STEPS):
+    """intra_fwd: X and Y on neighbouring items, two threads that issue products, two that copy."""
+    late_q = dtype == "fp32" and not scalar
+    slots = {k: (d[0] if d else 1) for k, d in dims.items()}
+    slots["op1"] = 1                                       # [2] are the halves of the channels
+    r = Roles(slots)
+    x_bars, y_bars = ("op1h0", "op1h1", "rows", "hand", "nwReady", "uReady", "syncA", "syncB"), ("opA", "opV", "acc", "syncY", "syncI")
+    r.count = {**dict.fromkeys(x_bars, 2), **dict.fromkeys(y_bars, 2), "ldin": 2}
+    for w in "ab":
+        wait, arrive = r.agent("X" + w)
+
+        def read_out(k):
+            wait("mmN", k), arrive("nwReady", k)
+            wait("mmU", k), arrive("uReady", k)
+        for k in range(n):
+            wait("ldin", k)
+            if not scalar and k:
+                wait("hand", k - 1)
+            arrive("syncA", k), wait("syncA", k)
+            if not scalar and k:
+                wait("khFree", k - 1)
+            arrive("op1h0", k), arrive("op1h1", k)
+            if scalar and k:
+                wait("khFree", k - 1)
+            arrive("syncB", k), wait("syncB", k)
+            arrive("rows", k)
+            if k:
+                read_out(k - 1)
+            wait("mm1", k), wait("rows", k)
+            if k:
+                wait("bkFree", k - 1)
+            arrive("hand", k)
+        read_out(n - 1)
+        wait, arrive = r.agent("Y" + w)
+        for k in range(n):
+            wait("rows", k), wait("mm1", k)
+            arrive("acc", k)
+            arrive("syncY", k), wait("syncY", k)
+            if k:
+                wait("abFree", k - 1)
+            arrive("syncI", k), wait("syncI", k)
+            if dtype != "fp32":
+                wait("fullV", k)
+            arrive("opA", k)
+            if dtype != "bf16":
+                wait("mmV", k), arrive("opV", k)
+    wait, arrive = r.agent("products X")
+    for k in range(n):
+        wait("op1h0", k), wait("op1h1", k), arrive("mm1", k)
+    wait, arrive = r.agent("products Y")
+    for k in range(n):
+        wait("hand", k), wait("opA", k)
+        if dtype == "bf16":
+            wait("fullV", k), arrive("mmN", k), arrive("mmU", k)
+        else:
+            arrive("mmV", k), wait("opV", k), arrive("mmU", k), arrive("mmN", k)
+    wait, arrive = r.agent("copies X")
+
+    def load_rows(k):
+        if k < n:
+            arrive("ldin", k)
+            if not late_q:
+                arrive("ldin", k)
+    load_rows(0)
+    if late_q:
+        arrive("ldin", 0)
+    for k in range(n):
+        wait("mm1", k), load_rows(k + 1)
+        wait("acc", k), wait("hand", k)
+        arrive("khFree", k)
+        if late_q and k + 1 < n:
+            arrive("ldin", k + 1)
+    wait, arrive = r.agent("copies Y")
+    if dtype != "fp32":
+        arrive("fullV", 0)
+    for k in range(n):
+        wait("nwReady", k), wait("uReady", k)
+        arrive("bkFree", k), arrive("abFree", k)
+        if dtype != "fp32" and k + 1 < n:
+            arrive("fullV", k + 1)
+    return r
+
+
 def test_a_wait_that_rests_on_timing_is_found():
     """The pair kernel with one barrier in all for u^T used and for each product: the copying thread may come to its waits two phases late."""
     dims = dict(fullN=[2], fullK=[2], fullU=[2], uFree=[], opS=[2], opV=[2], mm1=[2], mm2=[2])
@@ -270,3 +353,9 @@ def test_recur_fwd_and_chain_fwd(out, norm, save_h):
 
 def test_bwd_dh():
     assert reverse(_slots("tc_recur.cu", "DhShared")).late_waits() == []
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+@pytest.mark.parametrize("dtype", ["bf16", "fp16", "fp32"])
+def test_intra_fwd(dtype, scalar):
+    assert intra(_slots("tc_intra.cu", "Shared"), dtype, scalar).late_waits() == []
