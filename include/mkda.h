@@ -167,9 +167,11 @@ typedef struct {
                                 * as zero without being computed. */
     const int* seg_ht;         /* [NS] row of ht for each segment, -1 = do not store; NULL = identity map */
     int h0_k_first;            /* 1: h0 is [K,V] whatever state_v_first says (states handed between segments) */
-    const int* seg_order;      /* [NS] a permutation: the order in which the segments are started on, or NULL: as they lie */
 } MkdaRecurFwd;
 int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream);
+/* The same with the segments started on in the order of seg_order, [NS], a permutation (NULL: as they lie).  Here, in mkda_chain_fwd_ordered and
+ * in mkda_bwd_dh_ordered an argument and not a field: the structs keep their layouts for hosts built against an earlier header. */
+int mkda_recur_fwd_ordered(const MkdaRecurFwd* p, const int* seg_order, void* stream);
 
 /* Chunk-parallel output  o = qs h + Aqk Vd  (qs = scale q 2^g) with the optional gated RMSNorm epilogue fused.
  * Replaces the output part of fused_fwd_kda and rmsnorm_gated_fwd
@@ -195,6 +197,7 @@ typedef struct {
     MkdaOutFwd o;
 } MkdaChainFwd;
 int mkda_chain_fwd(const MkdaChainFwd* p, void* stream);
+int mkda_chain_fwd_ordered(const MkdaChainFwd* p, const int* seg_order, void* stream);
 
 /* Forward pass over sequences of at most MKDA_STEP_MAX_TOKENS tokens (generation steps): gate, L2 norm, recurrence, output and epilogue in one
  * kernel, token by token, with the state in registers.  Same results as the chunk kernels up to rounding; nothing is kept for a backward
@@ -305,9 +308,9 @@ typedef struct {
     float* dh0;                /* [NS,HV,128,128] gradient of the state entering each segment, or NULL */
     const int* warm_end;       /* [NS,HV] from mkda_warmup_chunks, or NULL: a reverse pass from zero (the segment pre-pass)
                                 * may start below this chunk index instead of at the segment's last chunk */
-    const int* seg_order;      /* [NS] a permutation: the order in which the segments are started on, or NULL: as they lie */
 } MkdaBwdDh;
 int mkda_bwd_dh(const MkdaBwdDh* p, void* stream);
+int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, void* stream);
 
 /* Every gradient that is local to a (chunk, v-head) once the state gradients are known, in one kernel:
  *  - through Vd = A diag(beta)(V - k~ S): dv, the WY part of dbeta, dAqk and dL = -strictlower(A^T dVd Vd^T) (K3a of bwd_post_kda,
@@ -425,8 +428,8 @@ const char* mkda_last_error(void);
 /* kernel launches issued by this process through the library so far */
 unsigned long long mkda_launch_count(void);
 int mkda_abi_version(void);
-/* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header: the sizes, not the version
- * above, tell one build's layouts from another's. */
+/* sizeof() of every parameter struct, in declaration order, so bindings can verify their mirror of this header.  Layouts change with the version
+ * above only, from version 4 on. */
 #define MKDA_STRUCTS(X) \
     X(MkdaLayout) X(MkdaGateFwd) X(MkdaGateBwd) X(MkdaReduce) X(MkdaReduceMulti) X(MkdaL2Norm) \
     X(MkdaIntraFwd) X(MkdaRecurFwd) X(MkdaOutFwd) X(MkdaChainFwd) X(MkdaStepFwd) X(MkdaEpilogueBwd) \

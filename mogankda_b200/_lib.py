@@ -16,6 +16,7 @@ ENTRY_POINTS = (
     "mkda_recur_fwd", "mkda_out_fwd", "mkda_epilogue_bwd", "mkda_epilogue_bwd_tiles", "mkda_bwd_dh", "mkda_bwd_chunk",
     "mkda_qk_grad_finish", "mkda_state_combine", "mkda_warmup_chunks", "mkda_selftest_umma", "mkda_selftest_wait", "mkda_epilogue_bwd_noalloc",
 )
+ORDERED_ENTRY_POINTS = ("mkda_recur_fwd_ordered", "mkda_chain_fwd_ordered", "mkda_bwd_dh_ordered")      # with the order of the segments
 ENUMS = {}
 STRUCTS = {}
 
@@ -78,10 +79,10 @@ def load():
         raise MkdaError(f"{path} is missing: build it with `python -m mogankda_b200.build` (no CPU or library fallback exists)")
     lib = ctypes.CDLL(path)
     lib.mkda_last_error.restype = ctypes.c_char_p
-    for name in ENTRY_POINTS:
+    for name in ENTRY_POINTS + ORDERED_ENTRY_POINTS:
         fn = getattr(lib, name)
         fn.restype = ctypes.c_int
-        fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+        fn.argtypes = [ctypes.c_void_p] * (3 if name in ORDERED_ENTRY_POINTS else 2)
     n = len(STRUCT_ORDER)
     sizes = (ctypes.c_int * n)()
     cnt = lib.mkda_struct_sizes(sizes, n)
@@ -112,9 +113,9 @@ def launch_count():
     return int(lib.mkda_launch_count())
 
 
-def call(name, params, stream):
+def call(name, params, *args):
     lib = load()
-    rc = getattr(lib, name)(ctypes.byref(params), ctypes.c_void_p(stream))
+    rc = getattr(lib, name)(ctypes.byref(params), *(ctypes.c_void_p(a) for a in args))
     if rc != 0:
         raise MkdaError(f"{name} failed ({rc}): {lib.mkda_last_error().decode()}")
 

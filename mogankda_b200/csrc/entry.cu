@@ -13,15 +13,16 @@ extern "C" int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream) {
     return launch_intra_fwd_tc(p, (cudaStream_t)stream);
 }
 
-extern "C" int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream) {
+extern "C" int mkda_recur_fwd_ordered(const MkdaRecurFwd* p, const int* seg_order, void* stream) {
     if (!p || !p->nw || !p->u || !p->kbar || !p->gl) return set_error(MKDA_ERR_ARG, "recur_fwd: null argument");
     if (any_misaligned(p->nw, p->u, p->kbar, p->gl, p->h, p->Vd)) return set_error(MKDA_ERR_ARG, "recur_fwd: tensors must be 16-byte aligned");
     if (any_misaligned32(p->h, p->Vd) || (p->state_v_first && any_misaligned32(p->h0, p->ht)))
         return set_error(MKDA_ERR_ARG, "recur_fwd: saved tiles and [V,K] states must be 32-byte aligned");
     if (p->want_transition && !p->mt) return set_error(MKDA_ERR_ARG, "recur_fwd: want_transition needs mt");
     if (p->L.NS == 0) return MKDA_OK;
-    return launch_recur_fwd_tc(p, (cudaStream_t)stream);
+    return launch_recur_fwd_tc(p, seg_order, (cudaStream_t)stream);
 }
+extern "C" int mkda_recur_fwd(const MkdaRecurFwd* p, void* stream) { return mkda_recur_fwd_ordered(p, nullptr, stream); }
 
 extern "C" int mkda_out_fwd(const MkdaOutFwd* p, void* stream) {
     if (!p || !p->qs || !p->Aqk || !p->Vd || !p->h || !p->out) return set_error(MKDA_ERR_ARG, "out_fwd: null argument");
@@ -31,7 +32,7 @@ extern "C" int mkda_out_fwd(const MkdaOutFwd* p, void* stream) {
     return launch_out_fwd_tc(p, (cudaStream_t)stream);
 }
 
-extern "C" int mkda_chain_fwd(const MkdaChainFwd* p, void* stream) {
+extern "C" int mkda_chain_fwd_ordered(const MkdaChainFwd* p, const int* seg_order, void* stream) {
     if (!p || !p->r.nw || !p->r.u || !p->r.kbar || !p->r.gl || !p->o.qs || !p->o.Aqk || !p->o.out) return set_error(MKDA_ERR_ARG, "chain_fwd: null argument");
     if (any_misaligned(p->r.nw, p->r.u, p->r.kbar, p->r.gl, p->o.qs, p->o.Aqk, p->o.out, p->o.o_raw, p->o.gate, p->o.norm_w))
         return set_error(MKDA_ERR_ARG, "chain_fwd: tensors must be 16-byte aligned");
@@ -40,10 +41,11 @@ extern "C" int mkda_chain_fwd(const MkdaChainFwd* p, void* stream) {
     if (p->r.want_transition || p->r.warm_start) return set_error(MKDA_ERR_ARG, "chain_fwd: no transition and no truncation in a main pass");
     if (p->o.has_norm && (!p->o.gate || p->o.out_dtype != MKDA_F32)) return set_error(MKDA_ERR_ARG, "chain_fwd: the gated norm needs a gate tensor and fp32 output");
     if (p->r.L.NS == 0) return MKDA_OK;
-    return launch_chain_fwd_tc(p, (cudaStream_t)stream);
+    return launch_chain_fwd_tc(p, seg_order, (cudaStream_t)stream);
 }
+extern "C" int mkda_chain_fwd(const MkdaChainFwd* p, void* stream) { return mkda_chain_fwd_ordered(p, nullptr, stream); }
 
-extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) {
+extern "C" int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, void* stream) {
     if (!p || !(p->dO_in_t || (p->d_o && p->dO_t)) || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw)
         return set_error(MKDA_ERR_ARG, "bwd_dh: null argument");
     if (any_misaligned(p->d_o, p->dO_in_t, p->kbar, p->qs, p->gl, p->Aqk, p->nw, p->dh, p->dVd_t, p->dO_t))
@@ -51,12 +53,13 @@ extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) {
     if (any_misaligned32(p->dh, p->dVd_t) || (p->state_v_first && any_misaligned32(p->dht, p->dh0)))
         return set_error(MKDA_ERR_ARG, "bwd_dh: saved tiles and [V,K] states must be 32-byte aligned");
     if (p->L.NS == 0) return MKDA_OK;
-    if (p->dO_in_t) return launch_bwd_dh_tc(p, (cudaStream_t)stream);
+    if (p->dO_in_t) return launch_bwd_dh_tc(p, seg_order, (cudaStream_t)stream);
     if (int e = launch_rows_to_tiles(p->L, p->d_o, p->do_dtype, p->dO_t, (cudaStream_t)stream)) return e;
     MkdaBwdDh q = *p;
     q.dO_in_t = p->dO_t;
-    return launch_bwd_dh_tc(&q, (cudaStream_t)stream);
+    return launch_bwd_dh_tc(&q, seg_order, (cudaStream_t)stream);
 }
+extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) { return mkda_bwd_dh_ordered(p, nullptr, stream); }
 
 extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) {
     if (!p || !p->q || !p->k || !p->v || !p->g_c || !p->beta || !p->A || !p->h || !p->dh || !p->Vd || !p->dO_t || !p->dVd_t ||

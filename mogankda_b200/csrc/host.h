@@ -49,9 +49,9 @@ int launch_out_fwd_tc(const MkdaOutFwd* p, cudaStream_t stream);
 int tc_chunk_status(unsigned int* out);
 int tc_chunk_status_clear();
 int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void* tiles, cudaStream_t stream);
-int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream);
-int launch_chain_fwd_tc(const MkdaChainFwd* p, cudaStream_t stream);
-int launch_bwd_dh_tc(const MkdaBwdDh* p, cudaStream_t stream);
+int launch_recur_fwd_tc(const MkdaRecurFwd* p, const int* seg_order, cudaStream_t stream);
+int launch_chain_fwd_tc(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream);
+int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stream);
 int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream);

@@ -146,6 +146,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     keep.allocate(c.dev);
     tmp.allocate(c.dev);
     const MkdaLayout L = c.layout();
+    const int* order = segment_order(c);
 
     {
         MkdaGateFwd p{};
@@ -169,7 +170,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     const Tensor w = aligned(in.ep_w);
     MkdaChainFwd p{};
     MkdaRecurFwd& r = p.r;
-    r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf; r.seg_order = segment_order(c);
+    r.L = L; r.nw = s.nw; r.u = u; r.kbar = s.kbar; r.gl = s.gl; r.state_v_first = c.vf;
     if (c.segmented) {
         // pre-pass from zero: per-segment (state, transition); the prefix combine then gives the state entering every segment
         if (c.warm) {
@@ -179,7 +180,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         }
         MkdaRecurFwd pre = r;
         pre.state_v_first = 0; pre.ht = hs; pre.want_transition = 1; pre.mt = s.ms; pre.warm_start = warm_start;
-        check_rc(mkda_recur_fwd(&pre, st), "mkda_recur_fwd");
+        check_rc(mkda_recur_fwd_ordered(&pre, order, st), "mkda_recur_fwd");
         MkdaCombine m{};
         m.NG = c.N; m.HV = c.HV; m.grp_seg_off = c.grp_off; m.hs = hs; m.ms = s.ms; m.carry = fptr(in.h0); m.s_in = s_in;
         m.carry_v_first = c.vf;
@@ -197,10 +198,10 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     }
     o.o_raw = s.o_raw; o.out = out.data_ptr(); o.out_dtype = dtype_code(out);
     if (fused) {
-        check_rc(mkda_chain_fwd(&p, st), "mkda_chain_fwd");
+        check_rc(mkda_chain_fwd_ordered(&p, order, st), "mkda_chain_fwd");
     } else {
         o.h = s.h; o.Vd = s.Vd;
-        check_rc(mkda_recur_fwd(&r, st), "mkda_recur_fwd");
+        check_rc(mkda_recur_fwd_ordered(&r, order, st), "mkda_recur_fwd");
         check_rc(mkda_out_fwd(&o, st), "mkda_out_fwd");
     }
     return {out, ht};
@@ -209,6 +210,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
 Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor dht, bool need_alog, bool need_bias, bool need_h0) {
     cudaStream_t st = c10::cuda::getCurrentCUDAStream();
     const MkdaLayout L = c.layout();
+    const int* order = segment_order(c);
     Grads g;
     if (!dy.defined()) dy = at::zeros({c.B, c.T, c.HV, 128}, in.q.options().dtype(c.has_ep ? at::kFloat : in.q.scalar_type()));
     if (dht.defined()) dht = aligned(aligned_f32(dht), 32);
@@ -253,13 +255,13 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         dy = aligned(dy);
         d.d_o = dy.data_ptr(); d.do_dtype = dtype_code(dy); d.dO_t = dO;
     }
-    d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw; d.seg_order = segment_order(c);
+    d.kbar = s.kbar; d.qs = s.qs; d.gl = s.gl; d.Aqk = s.Aqk; d.nw = s.nw;
     if (need_h0) g.h0 = c.states(c.N);
     MkdaBwdDh full = d;
     if (c.segmented) {
         // pre-pass from zero: only the gradient entering each segment is wanted, nothing per chunk is stored
         d.dh0 = dloc; d.warm_end = s.warm_end;
-        check_rc(mkda_bwd_dh(&d, st), "mkda_bwd_dh");
+        check_rc(mkda_bwd_dh_ordered(&d, order, st), "mkda_bwd_dh");
         MkdaCombine m{};
         m.NG = c.N; m.HV = c.HV; m.grp_seg_off = c.grp_off; m.hs = dloc; m.ms = s.ms; m.carry = fptr(dht); m.reverse = 1; m.s_in = g_in;
         m.s_out = fptr(g.h0); m.carry_v_first = c.vf; m.out_v_first = c.vf;
@@ -270,7 +272,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     }
     full.dh = dh; full.dVd_t = dVd;
     if (c.segmented) full.dO_in_t = dO;                    // already in tile form
-    check_rc(mkda_bwd_dh(&full, st), "mkda_bwd_dh");
+    check_rc(mkda_bwd_dh_ordered(&full, order, st), "mkda_bwd_dh");
     g.v = c.rows_out(c.HV, in.v.scalar_type());
     g.beta = c.like_out(in.beta);
     {

@@ -214,7 +214,7 @@ __device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainM
 }
 
 template <int OUT>
-__device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutFwd& o, const ChainMaps& maps) {
+__device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg_order, const MkdaOutFwd& o, const ChainMaps& maps) {
     using namespace rc;
     using L = RecurLayout<(OUT >= 0)>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -243,7 +243,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
-    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
+    const int seg = seg_order ? seg_order[blockIdx.z] : blockIdx.z;
 
     // Warm-up truncation (a pass from zero only): where the decay accumulated from chunk warm_start to the segment's end
     // hides everything before it, the pass starts there; the transition is then zero and its CTA visits no chunk.
@@ -458,9 +458,13 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const MkdaOutF
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-__global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p) { recur_body<-1>(p, MkdaOutFwd{}, ChainMaps{}); }
+__global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p, const int* seg_order) {
+    recur_body<-1>(p, seg_order, MkdaOutFwd{}, ChainMaps{});
+}
 template <int OUT>
-__global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const __grid_constant__ ChainMaps maps) { recur_body<OUT>(p.r, p.o, maps); }
+__global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const int* seg_order, const __grid_constant__ ChainMaps maps) {
+    recur_body<OUT>(p.r, seg_order, p.o, maps);
+}
 
 // ---------------------------------------------------------------------------------------------------------
 // The pre-pass of a cut call: state from zero and transition of a segment in ONE CTA, when there are more of them than SMs.  A chain of its own
@@ -510,7 +514,7 @@ __device__ __forceinline__ void store_pairs(uint32_t taddr, const float* v) {
 }
 }  // namespace pr
 
-__global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const MkdaRecurFwd p) {
+__global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const MkdaRecurFwd p, const int* seg_order) {
     using namespace pr;
     using umma::signal_tmem;
     using umma::wait_mma;
@@ -537,7 +541,7 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
-    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
+    const int seg = seg_order ? seg_order[blockIdx.z] : blockIdx.z;
     const int c_beg = p.L.seg_chunk_off[seg], n = p.L.seg_chunk_off[seg + 1] - c_beg;
     if (warp >= 16) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
@@ -671,24 +675,24 @@ __global__ void __launch_bounds__(pr::THREADS, 1) recur_fwd_pair_tc_kernel(const
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-int launch_recur_fwd_tc(const MkdaRecurFwd* p, cudaStream_t stream) {
+int launch_recur_fwd_tc(const MkdaRecurFwd* p, const int* seg_order, cudaStream_t stream) {
     if (p->want_transition && !p->h && !p->Vd && !p->h0 && !p->warm_start && 2ll * p->L.HV * p->L.NS > sm_count()) {
         auto pair = recur_fwd_pair_tc_kernel;
         if (int e = ensure_smem((const void*)pair, pr::SMEM, "recur_fwd")) return e;
         static const int regs = kernel_registers((const void*)pair);
         if (regs < pr::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "recur_fwd: built with fewer registers than its warps redistribute");
-        launch(pair, dim3(1, p->L.HV, p->L.NS), pr::THREADS, pr::SMEM, stream, *p);
+        launch(pair, dim3(1, p->L.HV, p->L.NS), pr::THREADS, pr::SMEM, stream, *p, seg_order);
         return check_launch("recur_fwd");
     }
     using L = RecurLayout<false>;
     auto kern = recur_fwd_tc_kernel;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "recur_fwd")) return e;
-    launch(kern, dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream, *p);
+    launch(kern, dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream, *p, seg_order);
     return check_launch("recur_fwd");
 }
 
 template <int OUT>
-static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, cudaStream_t stream) {
+static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
     using L = RecurLayout<true>;
     auto kern = chain_fwd_tc_kernel<OUT>;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "chain_fwd")) return e;
@@ -702,14 +706,14 @@ static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, cudaStream_t stream) {
     if (!e && p->o.o_raw) e = make_rows_map(&maps.raw, p->o.o_raw, 4, rows, cols, "chain_fwd", 16);
     if (!e) e = make_rows_map(&maps.out, p->o.out, p->o.out_dtype == MKDA_F32 ? 4 : 2, rows, cols, "chain_fwd", 16);
     if (e) return e;
-    launch(kern, dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream, *p, maps);
+    launch(kern, dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream, *p, seg_order, maps);
     return check_launch("chain_fwd");
 }
-int launch_chain_fwd_tc(const MkdaChainFwd* p, cudaStream_t stream) {
+int launch_chain_fwd_tc(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
     switch (p->o.has_norm ? p->o.gate_dtype : p->o.out_dtype) {
-        case MKDA_F32: return launch_chain_fwd_tc_t<MKDA_F32>(p, stream);
-        case MKDA_BF16: return launch_chain_fwd_tc_t<MKDA_BF16>(p, stream);
-        case MKDA_F16: return launch_chain_fwd_tc_t<MKDA_F16>(p, stream);
+        case MKDA_F32: return launch_chain_fwd_tc_t<MKDA_F32>(p, seg_order, stream);
+        case MKDA_BF16: return launch_chain_fwd_tc_t<MKDA_BF16>(p, seg_order, stream);
+        case MKDA_F16: return launch_chain_fwd_tc_t<MKDA_F16>(p, seg_order, stream);
     }
     return set_error(MKDA_ERR_ARG, "chain_fwd: unsupported dtype");
 }
@@ -730,7 +734,7 @@ constexpr int DH_K = 2 * DH_SET, DH_N = DH_K + 32 * rc::KB, DH_TILES = DH_N + 32
 constexpr int DH_SMEM = DH_TILES + (int)sizeof(DhShared);
 static_assert(DH_SMEM <= 232448, "shared memory of one CTA");
 
-__global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwdDh p) {
+__global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwdDh p, const int* seg_order) {
     using namespace rc;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     umma::fence_after_sync();
     const uint32_t tmem = sh.tmem;
     follow_stream();
-    const int seg = p.seg_order ? p.seg_order[blockIdx.z] : blockIdx.z;
+    const int seg = seg_order ? seg_order[blockIdx.z] : blockIdx.z;
 
     // Warm-up truncation (a pass from zero only): the reverse chain starts below chunk warm_end where the decay accumulated
     // over the segment's first chunks hides every later contribution from the segment's entrance.
@@ -864,10 +868,10 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-int launch_bwd_dh_tc(const MkdaBwdDh* p, cudaStream_t stream) {
+int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stream) {
     auto kern = bwd_dh_tc_kernel;
     if (int e = ensure_smem((const void*)kern, DH_SMEM, "bwd_dh")) return e;
-    launch(kern, dim3(1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream, *p);
+    launch(kern, dim3(1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream, *p, seg_order);
     return check_launch("bwd_dh");
 }
 

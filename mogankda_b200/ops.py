@@ -175,9 +175,9 @@ def warmup_chunks(lay, gl, HK, HV, threshold):
 
 
 def recur_fwd(lay, nw, u, kbar, gl, HK, HV, *, h0=None, seg_h0=None, state_v_first=False, store_h=True,
-              store_vd=True, want_ht=True, want_transition=False, segments=True, warm_start=None):
+              store_vd=True, want_ht=True, want_transition=False, segments=True, warm_start=None, seg_order=None):
     """Runs the serial state pass over the layout's segments (or whole sequences with ``segments=False``).
-    ``warm_start`` (from ``warmup_chunks``) shortens a pass from zero.
+    ``warm_start`` (from ``warmup_chunks``) shortens a pass from zero; ``seg_order``: the order in which the segments are started on.
     Returns (h [NC,HV] state tiles or None, Vd [NC,HV] chunk tiles or None, ht [NS,HV,128,128] or None, mt or None)."""
     dev = nw.device
     NS = lay.NS if segments else lay.N
@@ -194,7 +194,7 @@ def recur_fwd(lay, nw, u, kbar, gl, HK, HV, *, h0=None, seg_h0=None, state_v_fir
         if h0 is not None or store_h or store_vd or not segments:
             raise ValueError("warm_start applies to a pass from zero that stores nothing per chunk")
         p.warm_start = _ptr(warm_start, torch.int32)
-    _lib.call("mkda_recur_fwd", p, _stream())
+    _lib.call("mkda_recur_fwd_ordered", p, _ptr(seg_order, torch.int32), _stream())
     return h, Vd, ht, mt
 
 
@@ -290,11 +290,11 @@ def epilogue_bwd_tiles(lay, dy, o_raw, weight, gate, act, eps, HV):
 
 
 def bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, *, dht=None, seg_dht=None,
-           state_v_first=False, want_dh0=True, segments=True, store=True, dO_in_t=None, warm_end=None):
+           state_v_first=False, want_dh0=True, segments=True, store=True, dO_in_t=None, warm_end=None, seg_order=None):
     """Reverse state chain.  dO comes either as rows ``d_o`` [TT,HV,128] or as the row tiles ``dO_in_t`` of
     ``epilogue_bwd_tiles``.  With ``store`` the per-chunk results leave as tiles for ``bwd_chunk``: dh (state tiles), dVd^T
     (chunk tiles) and, for row input, the staged dO (row tiles); a pre-pass that only wants the segment-level gradient
-    passes ``store=False``.  Returns (dh, dVd_t, dO_t, dh0) with dO_t = ``dO_in_t`` when that was given."""
+    passes ``store=False``.  ``seg_order`` as in ``recur_fwd``.  Returns (dh, dVd_t, dO_t, dh0) with dO_t = ``dO_in_t`` when that was given."""
     dev = nw.device
     NS = lay.NS if segments else lay.N
     p = STRUCTS["MkdaBwdDh"]()
@@ -318,7 +318,7 @@ def bwd_dh(lay, d_o, kbar, qs, gl, Aqk, nw, HK, HV, *, dht=None, seg_dht=None,
         if dht is not None or store or not segments:
             raise ValueError("warm_end applies to a reverse pass from zero that stores nothing per chunk")
         p.warm_end = _ptr(warm_end, torch.int32)
-    _lib.call("mkda_bwd_dh", p, _stream())
+    _lib.call("mkda_bwd_dh_ordered", p, _ptr(seg_order, torch.int32), _stream())
     return dh, dVd_t, dO_t, dh0
 
 

@@ -40,6 +40,18 @@ def test_struct_sizes_match_header(lib):
     assert lib.mkda_abi_version() == 4
 
 
+# bytes of every parameter struct, by version: a host built against an earlier header of the same version hands over these and no more
+LAYOUTS = {4: dict(MkdaLayout=48, MkdaGateFwd=128, MkdaGateBwd=128, MkdaReduce=32, MkdaReduceMulti=96, MkdaL2Norm=32, MkdaIntraFwd=200, MkdaRecurFwd=168,
+                   MkdaOutFwd=152, MkdaChainFwd=320, MkdaStepFwd=256, MkdaEpilogueBwd=104, MkdaEpilogueBwdTiles=152, MkdaEpilogueBwdNoAlloc=104,
+                   MkdaBwdDh=176, MkdaBwdChunk=256, MkdaQkGrad=128, MkdaCombine=72, MkdaWarmup=80, MkdaSelfTest=40, MkdaSelfTestWait=16)}
+
+
+def test_struct_layouts_belong_to_the_version(lib):
+    """A field more in a struct is read from behind what such a host passes."""
+    from mogankda_b200 import _lib
+    assert {n: ctypes.sizeof(_lib.STRUCTS[n]) for n in _lib.STRUCT_ORDER} == LAYOUTS[lib.mkda_abi_version()]
+
+
 def test_null_arguments_are_rejected_without_launch(lib):
     from mogankda_b200 import _lib
     p = _lib.STRUCTS["MkdaIntraFwd"]()
