@@ -192,9 +192,12 @@ def test_padding_tokens_past_the_last_sequence_are_zero():
 
 
 def test_long_sequences_are_segmented_and_match():
-    """T > 32 chunks: the state + transition pre-pass, the prefix combine and the main pass replace the single serial
+    """T > 64 chunks: the state + transition pre-pass, the prefix combine and the main pass replace the single serial
     recurrence; same numbers within tolerance, and the uncut path still agrees with the oracle."""
-    lv, do, dht, opts, epi = make_inputs(B=1, T=2048 + 64 * 5 + 7, dtype=torch.float32, gate="eda", seed=13, HV=2)
+    from mogankda_b200.index import get_layout
+    T = 64 * 69 + 7
+    lv, do, dht, opts, epi = make_inputs(B=1, T=T, dtype=torch.float32, gate="eda", seed=13, HV=2)
+    assert get_layout(1, T, None, lv["q"].device, 32, 2).segmented
     seg = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True)
     ref = run(orc.chunked_delta_rule, lv, do, dht, opts, epi, f64=True, vfirst=True)
     compare(seg, ref)

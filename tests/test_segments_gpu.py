@@ -5,20 +5,20 @@ import torch
 
 import mogankda_b200 as mk
 from mogankda_b200.index import get_layout
-from tests.common import check, make_inputs, run
+from oracle import kda_oracle as orc
+from tests.common import check, compare, make_inputs, run
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("warm", [None, -10.0])
-@pytest.mark.parametrize("chunks,decay", [(64, -1e-4), (65, -1e-4), (65, -0.5)])
+@pytest.mark.parametrize("chunks,decay,warm", [(64, -1e-4, -10.0), (65, -1e-4, None), (65, -1e-4, -10.0), (65, -0.5, None), (65, -0.5, -10.0)])
 def test_sequences_around_two_segments(chunks, decay, warm):
     """Weak decay: truncation skips nothing and the results are bit for bit those of the cut call without it.  Strong decay: the pre-passes are
     truncated.  All against the uncut call."""
     lv, do, dht, opts, epi = make_inputs(B=1, T=64 * chunks - 23, dtype=torch.float32, gate="precomputed", seed=15, HV=2)
     lv["g"] = torch.full_like(lv["g"], decay)
-    ratio = 2.5 if warm is None else 1.25
-    assert get_layout(1, 64 * chunks - 23, None, lv["q"].device, 32, 2, ratio).segmented == (chunks > 64 or warm is not None)
+    cut = lambda ratio: get_layout(1, 64 * chunks - 23, None, lv["q"].device, 32, 2, ratio).segmented      # noqa: E731
+    assert cut(2.5) == (chunks > 64) and cut(1.25)                    # without and with truncation
     flat = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True, auto_cp=False)
     got = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True, warmup_threshold=warm)
     for n, t in flat.items():
@@ -49,19 +49,47 @@ def test_longest_first_changes_nothing():
             assert torch.equal(got[k][:, s:e], one[k]), (k, d)
 
 
-@pytest.mark.parametrize("lens", [(1,), (64,), (65, 1), (64 * 9 + 1, 0, 130)])
-def test_state_and_transition_in_one_cta(lens):
+def test_cut_batch_with_segments_of_unequal_length():
+    """More (segment, head) chains than SMs and a natural order that is not longest first: every pass of a cut batch, forward and backward, is
+    started on in another order.  Against the oracle, states in and out."""
+    lens, HV = (64 * 69 + 7, 64 * 3, 64 * 40 + 1, *(64 * (1 + i % 8) - 5 * i for i in range(14))), 8
+    cu = [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, dht, opts, epi = make_inputs(T=cu[-1], HK=4, HV=HV, cu=tuple(cu), dtype=torch.float32, gate="kimi", seed=37)
+    lay = get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, 32, HV)
+    assert lay.segmented and lay.NS * HV > torch.cuda.get_device_properties(0).multi_processor_count
+    assert lay.host["seg_order"][:4] == [0, 1, 4, 5]                      # 32, 32, 32 and 9 chunks; 6 and 3 lie between
+    compare(run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True), run(orc.chunked_delta_rule, lv, do, dht, opts, epi, f64=True, vfirst=True))
+
+
+@pytest.mark.parametrize("vfirst", [False, True])
+@pytest.mark.parametrize("lens,seg", [((1,), 3), ((64,), 3), ((65, 1), 3), ((64 * 9 + 1, 0, 130), 3), ((64 * 45 - 3, 300), 32)])
+def test_state_and_transition_in_one_cta(lens, seg, vfirst, monkeypatch):
     """More than one (segment, head) pair per two SMs: mkda_recur_fwd carries state and transition of a pair in one CTA; with a state to start
-    from (here zero) in two.  Segments of 0 to 3 chunks, ragged ends: the same bits."""
-    from mogankda_b200 import ops
+    from (here zero) in two.  Segments of 0 to 3 and of 5 to 32 chunks, ragged ends, started on in any order, final states of the last and of the
+    first segment only and swapped: the same bits."""
+    from mogankda_b200 import _lib, ops
     cu, HV = [0, *torch.tensor(lens).cumsum(0).tolist()], 80
     lv, _, _, opts, _ = make_inputs(T=cu[-1], HK=HV, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi=None, h0=False, seed=31)
-    lay = get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, 3)
+    lay = get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, seg)
     assert 2 * HV * lay.NS > torch.cuda.get_device_properties(0).multi_processor_count
     g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "kimi", lv["A_log"], lv["dt_bias"], -5.0, HV, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
     rq, rk = ops.l2norm_rstd(lv["q"]), ops.l2norm_rstd(lv["k"])
     _, _, nw, u, kbar, _, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, 128 ** -0.5, HV, HV)
-    kw = dict(store_h=False, store_vd=False, want_transition=True)
-    _, _, ht, mt = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, **kw)
-    _, _, ht2, mt2 = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, h0=torch.zeros(lay.NS, HV, 128, 128, device="cuda"), **kw)
+    kw = dict(store_h=False, store_vd=False, want_transition=True, state_v_first=vfirst)
+    order = torch.randperm(lay.NS, generator=torch.Generator().manual_seed(7)).int().cuda()
+    zero = torch.zeros(lay.NS, HV, 128, 128, device="cuda")
+    _, _, ht, mt = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, seg_order=order, **kw)
+    _, _, ht2, mt2 = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, h0=zero, **kw)
     assert torch.equal(ht, ht2) and torch.equal(mt, mt2) and torch.isfinite(ht).all() and torch.isfinite(mt).all()
+    rows = torch.full((lay.NS,), -1, dtype=torch.int32, device="cuda")
+    rows[0], rows[-1] = lay.NS - 1, 0
+    call, empty = _lib.call, torch.empty
+
+    def chosen(name, p, *args):
+        p.seg_ht = rows.data_ptr()
+        return call(name, p, *args)
+    monkeypatch.setattr(_lib, "call", chosen)
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, **k).fill_(7.0))
+    _, _, ht3, mt3 = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, **kw)
+    assert torch.equal(ht3[-1], ht[0]) and torch.equal(ht3[0], ht[-1]) and (ht3[1:-1] == 7).all() and torch.equal(mt3, mt)
+    assert _lib.device_status() == 0

@@ -13,6 +13,12 @@ from oracle import kda_oracle as orc
 from tests.common import compare, make_inputs, run
 
 pytestmark = pytest.mark.gpu
+LONG = 64 * 69 + 7
+
+
+def _is_cut(ratio):
+    """Whether LONG tokens x 2 heads are cut into segments at that cost ratio (index.wants_segments)."""
+    return get_layout(1, LONG, None, torch.device("cuda"), 32, 2, ratio).segmented
 
 
 def _table(seg_off, gl, thr_log2):
@@ -62,9 +68,10 @@ def test_warmup_table_matches_the_restatement():
 
 
 def test_truncated_prepass_stays_within_tolerance_of_the_exact_oracle():
-    """38 chunks = two segments; the eda gate of the generator decays by far more than e^-10 per segment, so the state +
+    """70 chunks = three segments; the eda gate of the generator decays by far more than e^-10 per segment, so the state +
     transition pre-pass visits a few chunks only.  Everything, gradients included, against the exact oracle."""
-    lv, do, dht, opts, epi = make_inputs(B=1, T=2048 + 64 * 5 + 7, dtype=torch.float32, gate="eda", seed=13, HV=2)
+    lv, do, dht, opts, epi = make_inputs(B=1, T=LONG, dtype=torch.float32, gate="eda", seed=13, HV=2)
+    assert _is_cut(2.5) and _is_cut(1.25)                              # without and with truncation
     cut = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True, warmup_threshold=-10.0)
     ref = run(orc.chunked_delta_rule, lv, do, dht, opts, epi, f64=True, vfirst=True)
     compare(cut, ref)
@@ -78,7 +85,8 @@ def test_truncated_prepass_stays_within_tolerance_of_the_exact_oracle():
 
 def test_truncation_changes_nothing_where_the_decay_is_weak():
     """Per-token decay of 1e-4: 2048 tokens accumulate -0.2, far above the threshold; every result is bitwise the exact one."""
-    lv, do, dht, opts, epi = make_inputs(B=1, T=2048 + 64 * 5 + 7, dtype=torch.float32, gate="precomputed", seed=14, HV=2)
+    lv, do, dht, opts, epi = make_inputs(B=1, T=LONG, dtype=torch.float32, gate="precomputed", seed=14, HV=2)
+    assert _is_cut(2.5) and _is_cut(1.25)
     lv["g"] = torch.full_like(lv["g"], -1e-4)
     exact = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True)
     cut = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=True, warmup_threshold=-10.0)
