@@ -2,7 +2,7 @@
 //
 //   Gamma_ij = sum_c k_ic k_jc 2^(g_ic - g_jc)  (i > j)        Aqk_ij = scale sum_c q_ic k_jc 2^(g_ic - g_jc)  (i >= j)
 //   A  = (I + strictlower(diag(beta) Gamma))^-1
-//   nw = -(A diag(beta)) (k 2^g)                                u = (A diag(beta)) v
+//   nw = -A diag(beta) (k 2^g)                                  u = A diag(beta) v
 //
 // Range / prefix invariance: the per-channel decay 2^(g_i - g_j) does not factor out of the contraction over channels,
 // so each 16-row block I uses its first row a = 16 I as anchor: row operand k_i 2^(g_i - g_a) (<= 1), column operand
@@ -17,12 +17,12 @@
 // What bounds it: the phases of an item depend on each other, and only one item's operands (144 KB) fit.  So the phases are split between two
 // groups of warps that work on neighbouring items:
 //   X, 16 warps, item n + 1: rows in -> operands -> (while [Gamma; Q K^T] is computed) L2 scales; nw, u of item n from their accumulators ->
-//                            kbar, scale q 2^g and k 2^g tiles
-//   Y, 4 or 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, A diag(beta)
+//                            kbar, scale q 2^g and beta k 2^g tiles
+//   Y, 4 or 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, beta v
 // and four warps of one working thread each: products of X, products of Y, copies of X, copies of Y.  All are joined by mbarriers.
-// bf16: beta is folded into A, so that v itself is the operand, a ready-made tile by a swizzled tiled copy that needs one product less per k-step
-// (it has no low half).  Other types have halves to round anyway: beta goes to v and k 2^g, and the diagonal of A stays exact (with it in A the
-// error against fp64 was 1.08 times as large in fp32 gradients, 1.2 in final states).
+// beta goes to v and k 2^g and not into A, whose diagonal stays exact.  With A diag(beta) as the operand a bf16 v would be one as it stands and take a
+// product less per k-step (6 to 12 % of the kernel), but a rounded beta on the diagonal is an error that all 128 values of a row have in common:
+// dh0 1.03 times as far from fp64 (geometric mean of 90 bf16 layers; 1.4 at worst), fp32 gradients 1.08, final states 1.2.
 // Shared memory is what X is then bound by (11 to 12 k of the 13 k cycles of an item, 18 k before, move operands, tiles and rows); with few items
 // the latency of an item counts, and twice as many warps in Y shorten it.
 // 6 k packed tokens x 32 heads 240 -> 196 us, 32 k tokens x 32 heads 1110 -> 825, scalar gate 4 x 2000 tokens x 16 heads 129 -> 89.
@@ -56,8 +56,8 @@ struct Rows {
     static constexpr int K = SCALAR ? KQ : KQ + 32768, Q = LATE_Q ? KB : K + BYTES;
     static_assert(LATE_Q || Q + BYTES <= KQ + 65536, "rows of the next item");
 };
-// Y's own: k 2^g [j][K index] (then nw^T), v [j][v] (bf16: 16 KB) and A diag(beta) [i][j] (then u^T over both), the triangular matrix
-constexpr int BK = KQ + 65536, V_ = BK + 32768, AB = V_ + 16384, T_ = AB, UT = V_, M_ = AB + 16384;
+// Y's own: beta k 2^g [j][K index] (then nw^T), half of beta v [j][v] (16-bit: v before) and A [i][j] (then u^T over both), the triangular matrix
+constexpr int BK = KQ + 65536, V_ = BK + 32768, A_ = V_ + 16384, T_ = A_, UT = V_, M_ = A_ + 16384;
 constexpr int LD = 36, MB = 32 * LD;                        // I + L as three 32 x 32 blocks: (0, 0), (1, 0), (1, 1)
 constexpr int TILES = M_ + 3 * MB * 4;
 constexpr int D1 = 0, D1_COLS = 160, NW = 320, U = 384;      // accumulator columns (two of [Gamma; Q K^T]: Y is an item behind)
@@ -66,8 +66,8 @@ struct Shared {
     uint64_t ldin, fullV;                                   // rows | v landed
     uint64_t op1[2], mm1[2];                                // operands of channel half 0, 1 written; [Gamma; Q K^T] done, one per accumulator buffer:
                                                             // a scalar gate's can be done for the next item before Y comes to wait for this one's
-    uint64_t rows, acc, hand, khFree;                       // row scales | Aqk | kbar, scale q 2^g, k 2^g written; the first two tiles and Aqk have left
-    uint64_t opA, opV, mmV, mmN, mmU;                       // A diag(beta) written | (v in two halves: low half written, high half used) | nw^T, u^T done
+    uint64_t rows, acc, hand, khFree;                       // row scales | Aqk | kbar, scale q 2^g, beta k 2^g written; the first two tiles and Aqk have left
+    uint64_t opA, opV, mmV, mmN, mmU;                       // A and the high half of beta v | the low half written; high half used | nw^T, u^T done
     uint64_t nwReady, uReady, bkFree, abFree;               // nw^T, u^T staged | have left
     uint32_t tmem;
     __align__(16) float beta[2][CH];                        // Y is an item behind
@@ -144,7 +144,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
     auto row_of = [&](int hf) { return hf ? (tid >> 3) ^ 48 : tid >> 3; };
     uint8_t* sKQ = base + KQ;
     // nw^T [K index][tok] and u^T [v][tok] of an item leave as ready-made chunk tiles over their operands (the serial kernels fetch them with one
-    // bulk copy; token columns past the end are exact zeros: beta is 0 there)
+    // bulk copy; token columns past the end are exact zeros: rows of beta v and beta k are zero there)
     auto read_out = [&](int it) {
         auto stage = [&](int col, uint8_t* tile, float sign) {
             float a[16];
@@ -301,12 +301,12 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
         if (it) read_out(it - 1);
         umma::wait_mma(&sh.mm1[par], (it >> 1) & 1);
         umma::mbar_wait(&sh.rows, par);
-        // ---- over the dead operands: the state kernels' scaled operands, kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g; k 2^g for Y ----
+        // ---- over the dead operands: the state kernels' scaled operands, kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g; beta k 2^g for Y ----
         const float gLs = SCALAR ? gs[CH - 1] : 0.f;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int r = row_of(hf), k8 = c8 + 8 * hf;
-            const float up = SCALAR ? ex2f_(gs[r]) : 1.f, fk = sh.rs[0][r], fq = sh.rs[1][r] * p.scale, fb = DT == MKDA_BF16 ? fk : fk * beta[r];
+            const float up = SCALAR ? ex2f_(gs[r]) : 1.f, fk = sh.rs[0][r], fq = sh.rs[1][r] * p.scale, fb = fk * beta[r];
             const f32x2 sk = both(SCALAR ? fk * ex2f_(gLs - gs[r]) : fk), sq = both(SCALAR ? fq * up : fq), sb = both(SCALAR ? fb * up : fb);
             f32x2 t8[4], e8[4], x8[4];
             unpack8<DT>(wk[hf], x8);
@@ -469,11 +469,9 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
         umma::signal(&sh.acc, lane);
         sync_y<YW>();
         invert_unit_lower<YW>(M, reinterpret_cast<float*>(base + T_), &sh.abFree, it);         // there u^T of the previous item may still be leaving
-        // A leaves as a ready-made [row][column] operand tile (rows past the end: identity rows); A diag(beta) is the operand of nw and u
+        // A leaves as a ready-made [row][column] operand tile (rows past the end: identity rows) and is the operand of nw and u
         uint8_t* At = reinterpret_cast<uint8_t*>(p.A) + (size_t)sh.info[it & 3].item * umma::QUARTER_TILE_BYTES;
         const int k8 = tid & 7;
-        f32x2 b8[4];
-        lds8_swapped(beta + 8 * k8, k8 & 4, b8);
 #pragma unroll
         for (int m = 0; m < 16 / YW; ++m) {
             const int r = 4 * YW * m + (tid >> 3);
@@ -491,59 +489,44 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
                     if (k8 * 8 + e > r) a8[e] = 0.f;
             }
             store_split8(At, At + 8192, 64, r, k8, a8);
-            f32x2 ab[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                ab[e] = pack2(a8[2 * e], a8[2 * e + 1]);
-                if (DT == MKDA_BF16) ab[e] = mul2(ab[e], b8[e]);
-            }
-            store_split8(base + AB, base + AB + 8192, 64, r, k8, ab);
+            store_split8(base + A_, base + A_ + 8192, 64, r, k8, a8);
         }
-        if (DT == MKDA_BF16) {
-            if (len < CH) {                                  // rows past the end belong to another sequence
-                umma::mbar_wait(&sh.fullV, par);
-                for (int i = len * 16 + tid; i < CH * 16; i += YT)
-                    *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(0, 0, 0, 0);
+        // beta v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
+        constexpr int N = 32 / YW;
+        uint32_t lo[N][4];
+        if (DT != MKDA_F32) umma::mbar_wait(&sh.fullV, par);
+#pragma unroll
+        for (int m = 0; m < N; m += 4) {
+            Raw8 raw[4];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int i = tid + YT * (m + n), r = i >> 4;
+                if (DT != MKDA_F32) raw[n].a = *reinterpret_cast<const uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15));
+                else ldraw8<DT>(p.v, ((size_t)(sh.info[it & 3].start + min(r, len - 1)) * HV + sh.info[it & 3].h) * 128 + (i & 15) * 8, raw[n]);
             }
-            umma::signal(&sh.opA, lane);
-        } else {
-            // beta v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
-            constexpr int N = 32 / YW;
-            uint32_t lo[N][4];
-            if (DT == MKDA_F16) umma::mbar_wait(&sh.fullV, par);
 #pragma unroll
-            for (int m = 0; m < N; m += 4) {
-                Raw8 raw[4];
+            for (int n = 0; n < 4; ++n) {
+                const int i = tid + YT * (m + n), r = i >> 4;
+                float v8[8];
+                unpack8<DT>(raw[n], v8);
+                const float b = beta[r];
+                uint32_t hi[4];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const int i = tid + YT * (m + n), r = i >> 4;
-                    if (DT == MKDA_F16) raw[n].a = *reinterpret_cast<const uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15));
-                    else ldraw8<DT>(p.v, ((size_t)(sh.info[it & 3].start + min(r, len - 1)) * HV + sh.info[it & 3].h) * 128 + (i & 15) * 8, raw[n]);
+                for (int e = 0; e < 4; ++e) {
+                    umma::split2(b * v8[2 * e], b * v8[2 * e + 1], hi[e], lo[m + n][e]);
+                    if (r >= len) hi[e] = lo[m + n][e] = 0u;
                 }
-#pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const int i = tid + YT * (m + n), r = i >> 4;
-                    float v8[8];
-                    unpack8<DT>(raw[n], v8);
-                    const float b = beta[r];
-                    uint32_t hi[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        umma::split2(b * v8[2 * e], b * v8[2 * e + 1], hi[e], lo[m + n][e]);
-                        if (r >= len) hi[e] = lo[m + n][e] = 0u;
-                    }
-                    *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                }
+                *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             }
-            umma::signal(&sh.opA, lane);
-            umma::wait_mma(&sh.mmV, par);
-#pragma unroll
-            for (int n = 0; n < N; ++n) {
-                const int i = tid + YT * n;
-                *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(lo[n][0], lo[n][1], lo[n][2], lo[n][3]);
-            }
-            umma::signal(&sh.opV, lane);
         }
+        umma::signal(&sh.opA, lane);
+        umma::wait_mma(&sh.mmV, par);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int i = tid + YT * n;
+            *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(lo[n][0], lo[n][1], lo[n][2], lo[n][3]);
+        }
+        umma::signal(&sh.opV, lane);
         sync_y<YW>();                                            // the matrix has been read
     }
 }
@@ -579,32 +562,24 @@ __device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, 
         umma::commit(&sh.mm1[it & 1]);
     }
 }
-template <int DT>
 __device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, uint32_t tmem, in::Shared& sh) {
     using namespace in;
     const int count = item_count(p.L);
     for (int it = 0; it < count; ++it) {
         const uint32_t par = it & 1;
-        umma::wait_mma(&sh.hand, par);                      // k 2^g
+        umma::wait_mma(&sh.hand, par);                      // beta k 2^g
         umma::wait_mma(&sh.opA, par);
-        if (DT == MKDA_BF16) umma::mbar_wait(&sh.fullV, par);
         uint8_t* base = fresh(smem);
-        const umma::Opnd ab = umma::opnd_k(base + AB, base + AB + 8192, 64), v = umma::opnd_mn(base + V_, nullptr, 64);
-        if (DT != MKDA_BF16) {
-            umma::gemm(tmem + U, v, ab, 128, 64, 64, 0u);
-            umma::commit(&sh.mmV);
-            umma::wait_mma(&sh.opV, par);
-            umma::Opnd hi = ab;
-            hi.lo = 0;
-            umma::gemm(tmem + U, v, hi, 128, 64, 64, 1u);
-            umma::commit(&sh.mmU);
-        }
-        umma::gemm(tmem + NW, umma::opnd_mn(base + BK, base + BK + 16384, 64), ab, 128, 64, 64, 0u);
+        const umma::Opnd a = umma::opnd_k(base + A_, base + A_ + 8192, 64), v = umma::opnd_mn(base + V_, nullptr, 64);
+        umma::gemm(tmem + U, v, a, 128, 64, 64, 0u);
+        umma::commit(&sh.mmV);
+        umma::wait_mma(&sh.opV, par);
+        umma::Opnd hi = a;
+        hi.lo = 0;
+        umma::gemm(tmem + U, v, hi, 128, 64, 64, 1u);
+        umma::commit(&sh.mmU);
+        umma::gemm(tmem + NW, umma::opnd_mn(base + BK, base + BK + 16384, 64), a, 128, 64, 64, 0u);
         umma::commit(&sh.mmN);
-        if (DT == MKDA_BF16) {
-            umma::gemm(tmem + U, v, ab, 128, 64, 64, 0u);
-            umma::commit(&sh.mmU);
-        }
     }
 }
 template <int DT, bool SCALAR>
@@ -642,7 +617,7 @@ __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Ma
 template <int DT>
 __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     using namespace in;
-    auto load_v = [&](const Walk& w) {                      // two boxes of 64 channels: a [64][128] operand tile as it stands
+    auto load_v = [&](const Walk& w) {                      // two boxes of 64 channels: rows in the layout of an operand tile
         if (DT == MKDA_F32) return;
         umma::mbar_expect_tx(&sh.fullV, 16384);
         umma::tma_load_rows(base + V_, &maps.v, w.h * 128, w.start, &sh.fullV);
@@ -702,7 +677,7 @@ __global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel
                 case 0: intra_mm1<DT, SCALAR>(p, base, tmem, sh); break;
                 case 1: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
                 case 2: intra_copy_y<DT>(p, maps, base, sh); break;
-                default: intra_mm3<DT>(p, base, tmem, sh);
+                default: intra_mm3(p, base, tmem, sh);
             }
         }
         __syncwarp();

@@ -297,18 +297,14 @@ def intra(dims, dtype, scalar, n=STEPS):
             if dtype != "fp32":
                 wait("fullV", k)
             arrive("opA", k)
-            if dtype != "bf16":
-                wait("mmV", k), arrive("opV", k)
+            wait("mmV", k), arrive("opV", k)
     wait, arrive = r.agent("products X")
     for k in range(n):
         wait("op1h0", k), wait("op1h1", k), arrive("mm1", k)
     wait, arrive = r.agent("products Y")
     for k in range(n):
         wait("hand", k), wait("opA", k)
-        if dtype == "bf16":
-            wait("fullV", k), arrive("mmN", k), arrive("mmU", k)
-        else:
-            arrive("mmV", k), wait("opV", k), arrive("mmU", k), arrive("mmN", k)
+        arrive("mmV", k), wait("opV", k), arrive("mmU", k), arrive("mmN", k)
     wait, arrive = r.agent("copies X")
 
     def load_rows(k):
@@ -356,6 +352,6 @@ def test_bwd_dh():
 
 
 @pytest.mark.parametrize("scalar", [False, True])
-@pytest.mark.parametrize("dtype", ["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("dtype", ["fp16", "fp32"])
 def test_intra_fwd(dtype, scalar):
     assert intra(_slots("tc_intra.cu", "Shared"), dtype, scalar).late_waits() == []

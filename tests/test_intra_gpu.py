@@ -28,6 +28,24 @@ def _call(lens, q, k, v, g, be, scalar):
 
 @pytest.mark.parametrize("scalar", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_rows_have_no_error_in_common(dtype, scalar):
+    """Sequences of one token: u = beta v, nw = -beta (k 2^g).  Each of their 128 values is rounded twice (as an operand and as a result) to 16
+    mantissa bits, 2^-17 at most: the part of the error that a row has in common is an average of 128 such, 2^-16 / 128^0.5 (root mean square over
+    the rows, at most).  A beta that is itself rounded to 16 bits moves the whole row, and the norm behind it passes that on to dh0."""
+    T, gen = 1200, torch.Generator(device="cuda").manual_seed(11)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")                        # noqa: E731
+    q, k, v = r(1, T, HK, 128).to(dtype), r(1, T, HK, 128).to(dtype), r(1, T, HV, 128).to(dtype)
+    be, g = torch.rand(T, HV, generator=gen, device="cuda"), -torch.rand(T, HV, *(() if scalar else (128,)), generator=gen, device="cuda")
+    got = _call((1,) * T, q, k, v, g, be, scalar)[2]
+    kn = k[0].double() * torch.rsqrt((k[0].double() ** 2).sum(-1, keepdim=True) + 1e-6)
+    gd = g.double() if not scalar else g.double()[..., None]
+    for x, y in ((got[2], -kn.repeat_interleave(HV // HK, 1) * torch.exp2(gd) * be[..., None]), (got[3], v[0].double() * be[..., None])):
+        common = (x.double() * y).sum(-1) / (y * y).sum(-1) - 1
+        assert common.square().mean().sqrt().item() <= 2.0 ** -16 / 128 ** 0.5
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_ragged_chunks(dtype, scalar):
     T, gen = sum(LENS), torch.Generator(device="cuda").manual_seed(5)
     r = lambda *s: torch.randn(*s, generator=gen, device="cuda")                        # noqa: E731
