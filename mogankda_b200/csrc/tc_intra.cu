@@ -18,14 +18,13 @@
 // groups of warps that work on neighbouring items:
 //   X, 16 warps, item n + 1: rows in -> operands -> (while [Gamma; Q K^T] is computed) L2 scales; nw, u of item n from their accumulators ->
 //                            kbar, scale q 2^g and beta k 2^g tiles
-//   Y, 4 or 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, beta v
+//   Y, 8 warps, item n:      I + L and Aqk from the accumulators -> inverse (a chain of latencies that used to hold up 16 warps) -> A, beta v
 // and four warps of one working thread each: products of X, products of Y, copies of X, copies of Y.  All are joined by mbarriers.
 // beta goes to v and k 2^g and not into A, whose diagonal stays exact.  With A diag(beta) as the operand a bf16 v would be one as it stands and take a
 // product less per k-step (6 to 12 % of the kernel), but a rounded beta on the diagonal is an error that all 128 values of a row have in common:
 // dh0 1.03 times as far from fp64 (geometric mean of 90 bf16 layers; 1.4 at worst), fp32 gradients 1.08, final states 1.2.
-// Shared memory is what X is then bound by (11 to 12 k of the 13 k cycles of an item, 18 k before, move operands, tiles and rows); with few items
-// the latency of an item counts, and twice as many warps in Y shorten it.
-// 6 k packed tokens x 32 heads 240 -> 196 us, 32 k tokens x 32 heads 1110 -> 825, scalar gate 4 x 2000 tokens x 16 heads 129 -> 89.
+// An item takes 12 to 13 k cycles (18 k before): shared memory (operands, tiles and rows of X) and the latency of Y are about as long.
+// 6 k packed tokens x 32 heads 240 -> 190 us, 32 k tokens x 32 heads 1121 -> 860, scalar gate 4 x 2000 tokens x 16 heads 129 -> 99.
 #include "host.h"
 #include "intra.cuh"
 
@@ -34,13 +33,12 @@
 namespace mkda {
 
 namespace in {
-constexpr int X_WARPS = 16;
-// YW warps of Y.  Registers of the launch, of X and of Y; the last four warps go down to 40 (the sums are those of the launch).
-template <int YW>
-struct Warps {
-    static constexpr int THREADS = 32 * (X_WARPS + YW + 4), LAUNCH_REGS = YW == 4 ? 80 : 72, X_REGS = LAUNCH_REGS + 8, Y_REGS = YW == 4 ? 88 : 72;
-    static_assert(X_WARPS * X_REGS + YW * Y_REGS + 4 * 40 <= (X_WARPS + YW + 4) * LAUNCH_REGS, "registers of the launch");
-};
+// Eight warps of Y: the latency of its phases is what an item takes, also where X keeps shared memory busy.  Eight against four, per-channel gate, from 0.2 to
+// 220 items per SM: 3 to 12 % faster throughout, bf16, fp16 and fp32 (bf16 6 k packed tokens x 32 heads 219 -> 190 us, 32 k tokens 1005 -> 860).
+constexpr int X_WARPS = 16, Y_WARPS = 8, THREADS = 32 * (X_WARPS + Y_WARPS + 4);
+// registers of the launch (Y keeps them), of X and of the last four warps
+constexpr int LAUNCH_REGS = 72, X_REGS = 80, ISSUE_REGS = 40;
+static_assert(X_WARPS * X_REGS + Y_WARPS * LAUNCH_REGS + 4 * ISSUE_REGS <= (X_WARPS + Y_WARPS + 4) * LAUNCH_REGS, "registers of the launch");
 constexpr float ROW_UP = 0x1p48f, COL_DOWN = 0x1p-48f;      // column operand: 108 + 64 - 48 < 127, row operand: 64 + 48 < 127 for |k| < 2^64
 // the four column tiles stacked by rows into one 160-row tile (hi 40 KB, then lo)
 __host__ __device__ constexpr int kc_row(int I) { return 8 * I * (I + 1); }
@@ -83,8 +81,8 @@ static_assert(SMEM <= 232448, "shared memory of one CTA");
 struct Maps { CUtensorMap k, q, g, v; };
 
 __device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-template <int YW>
-__device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, %0;" :: "n"(32 * YW) : "memory"); }
+__device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
+static_assert(X_WARPS == 16 && Y_WARPS == 8, "threads of the named barriers");
 
 // The items of a CTA: gridDim.x apart, heads fastest (the threads that request copies walk them; the others read `info`).
 struct Walk {
@@ -349,10 +347,9 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
 // X = -B^-1 C A^-1  with A^-1 / B^-1 the inverses above / beside it.  Every entry depends on the rows up to its own only, and the order of the
 // sums is fixed by the indices.  The merges are TF32 products with error compensation (three products, fp32 accumulation: ~2^-21 per product).
 // T = 32 rows of scratch, free once `free` completes.
-template <int YW>
 __device__ __forceinline__ void invert_unit_lower(float* M, float* T, uint64_t* free, int it) {
     using namespace in;
-    const int y = (threadIdx.x >> 5) & (YW - 1), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int y = (threadIdx.x >> 5) & (Y_WARPS - 1), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (y < 2) {
         float* D = M + y * 2 * MB;
         const int o = lane & 16, col = lane & 15;
@@ -386,27 +383,24 @@ __device__ __forceinline__ void invert_unit_lower(float* M, float* T, uint64_t* 
         }
     }
     if (it) umma::mbar_wait(free, (it & 1) ^ 1);
-    sync_y<YW>();
-    // 32 x 32 block (rows 32.., columns 0..31) in tiles of 16 x 8
+    sync_y();
+    // 32 x 32 block (rows 32.., columns 0..31): a tile of 16 x 8 per warp
+    const int m0 = 16 * (y >> 2), n0 = 8 * (y & 3);
     auto product = [&](const float* A, const float* B, float* D, float sign) {
-#pragma unroll
-        for (int i = y; i < 8; i += YW) {
-            const int m0 = 16 * (i >> 2), n0 = 8 * (i & 3);
-            float acc[1][4];
-            warp_mma_short<1, 32, LD, 1, LD, 1>(acc, A + m0 * LD, B + n0);
-            *reinterpret_cast<float2*>(D + (m0 + g) * LD + n0 + 2 * t) = make_float2(sign * acc[0][0], sign * acc[0][1]);
-            *reinterpret_cast<float2*>(D + (m0 + g + 8) * LD + n0 + 2 * t) = make_float2(sign * acc[0][2], sign * acc[0][3]);
-        }
-        sync_y<YW>();
+        float acc[1][4];
+        warp_mma_short<1, 32, LD, 1, LD, 1>(acc, A + m0 * LD, B + n0);
+        *reinterpret_cast<float2*>(D + (m0 + g) * LD + n0 + 2 * t) = make_float2(sign * acc[0][0], sign * acc[0][1]);
+        *reinterpret_cast<float2*>(D + (m0 + g + 8) * LD + n0 + 2 * t) = make_float2(sign * acc[0][2], sign * acc[0][3]);
+        sync_y();
     };
     product(M + MB, M, T, 1.f);
     product(M + 2 * MB, T, M + MB, -1.f);
 }
 
-template <int DT, bool SCALAR, int YW>
+template <int DT, bool SCALAR>
 __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, uint32_t tmem, in::Shared& sh) {
     using namespace in;
-    constexpr int YT = 32 * YW;
+    constexpr int YT = 32 * Y_WARPS;
     const int tid = threadIdx.x & (YT - 1), warp = threadIdx.x >> 5, lane = tid & 31, q = warp & 3;
     const size_t HV = p.L.HV;
     float* M = reinterpret_cast<float*>(base + M_);
@@ -425,7 +419,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             const bool isq = SCALAR ? q >= 2 : lane >= 16;
             const float bi = isq ? p.scale * sh.rs[1][i] : beta[i] * sh.rs[0][i], gi = SCALAR ? gs[i] : 0.f;
 #pragma unroll
-            for (int cg = YW == 4 ? 0 : 2 * ((warp >> 2) & 1), last = cg + 16 / YW; cg < last; ++cg) {
+            for (int cg = 2 * ((warp >> 2) & 1), last = cg + 2; cg < last; ++cg) {
                 float v[16];
                 if (SCALAR || cg <= q) {                     // warp-uniform
                     umma::tmem_ld16(umma::tmem_addr(tmem, warp, D1 + par * D1_COLS + (SCALAR ? 0 : kc_row(q)) + 16 * cg), v);
@@ -467,21 +461,21 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             }
         }
         umma::signal(&sh.acc, lane);
-        sync_y<YW>();
-        invert_unit_lower<YW>(M, reinterpret_cast<float*>(base + T_), &sh.abFree, it);         // there u^T of the previous item may still be leaving
+        sync_y();
+        invert_unit_lower(M, reinterpret_cast<float*>(base + T_), &sh.abFree, it);         // there u^T of the previous item may still be leaving
         // A leaves as a ready-made [row][column] operand tile (rows past the end: identity rows) and is the operand of nw and u
         uint8_t* At = reinterpret_cast<uint8_t*>(p.A) + (size_t)sh.info[it & 3].item * umma::QUARTER_TILE_BYTES;
         const int k8 = tid & 7;
 #pragma unroll
-        for (int m = 0; m < 16 / YW; ++m) {
-            const int r = 4 * YW * m + (tid >> 3);
+        for (int m = 0; m < 2; ++m) {
+            const int r = 32 * m + (tid >> 3);
             float a8[8];
-            if (m < 8 / YW && k8 >= 4) {
+            if (m == 0 && k8 >= 4) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) a8[e] = 0.f;
             } else {
                 f32x2 a[4];
-                lds8_swapped(M + (m < 8 / YW ? 0 : k8 < 4 ? MB : 2 * MB) + (r & 31) * LD + 8 * (k8 & 3), k8 & 2, a);
+                lds8_swapped(M + (m == 0 ? 0 : k8 < 4 ? MB : 2 * MB) + (r & 31) * LD + 8 * (k8 & 3), k8 & 2, a);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) unpack2(a[e], a8[2 * e], a8[2 * e + 1]);
 #pragma unroll
@@ -492,32 +486,29 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             store_split8(base + A_, base + A_ + 8192, 64, r, k8, a8);
         }
         // beta v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there
-        constexpr int N = 32 / YW;
+        constexpr int N = 4;
         uint32_t lo[N][4];
         if (DT != MKDA_F32) umma::mbar_wait(&sh.fullV, par);
+        Raw8 raw[N];
 #pragma unroll
-        for (int m = 0; m < N; m += 4) {
-            Raw8 raw[4];
+        for (int n = 0; n < N; ++n) {
+            const int i = tid + YT * n, r = i >> 4;
+            if (DT != MKDA_F32) raw[n].a = *reinterpret_cast<const uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15));
+            else ldraw8<DT>(p.v, ((size_t)(sh.info[it & 3].start + min(r, len - 1)) * HV + sh.info[it & 3].h) * 128 + (i & 15) * 8, raw[n]);
+        }
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                const int i = tid + YT * (m + n), r = i >> 4;
-                if (DT != MKDA_F32) raw[n].a = *reinterpret_cast<const uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15));
-                else ldraw8<DT>(p.v, ((size_t)(sh.info[it & 3].start + min(r, len - 1)) * HV + sh.info[it & 3].h) * 128 + (i & 15) * 8, raw[n]);
+        for (int n = 0; n < N; ++n) {
+            const int i = tid + YT * n, r = i >> 4;
+            float v8[8];
+            unpack8<DT>(raw[n], v8);
+            const float b = beta[r];
+            uint32_t hi[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                umma::split2(b * v8[2 * e], b * v8[2 * e + 1], hi[e], lo[n][e]);
+                if (r >= len) hi[e] = lo[n][e] = 0u;
             }
-#pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                const int i = tid + YT * (m + n), r = i >> 4;
-                float v8[8];
-                unpack8<DT>(raw[n], v8);
-                const float b = beta[r];
-                uint32_t hi[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    umma::split2(b * v8[2 * e], b * v8[2 * e + 1], hi[e], lo[m + n][e]);
-                    if (r >= len) hi[e] = lo[m + n][e] = 0u;
-                }
-                *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            }
+            *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }
         umma::signal(&sh.opA, lane);
         umma::wait_mma(&sh.mmV, par);
@@ -527,7 +518,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, i >> 4, i & 15)) = make_uint4(lo[n][0], lo[n][1], lo[n][2], lo[n][3]);
         }
         umma::signal(&sh.opV, lane);
-        sync_y<YW>();                                            // the matrix has been read
+        sync_y();                                            // the matrix has been read
     }
 }
 
@@ -640,8 +631,8 @@ __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Ma
     }
 }
 
-template <int DT, bool SCALAR, int YW>
-__global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ in::Maps maps) {
+template <int DT, bool SCALAR>
+__global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ in::Maps maps) {
     using namespace in;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
@@ -656,7 +647,7 @@ __global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel
     if (threadIdx.x == 0) {
         for (uint64_t* b : {&sh.ldin, &sh.fullV, &sh.mm1[0], &sh.mm1[1], &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
         for (uint64_t* b : {&sh.op1[0], &sh.op1[1], &sh.rows, &sh.hand, &sh.nwReady, &sh.uReady}) umma::mbar_init(b, X_WARPS);
-        for (uint64_t* b : {&sh.opA, &sh.opV, &sh.acc}) umma::mbar_init(b, YW);
+        for (uint64_t* b : {&sh.opA, &sh.opV, &sh.acc}) umma::mbar_init(b, Y_WARPS);
         umma::fence_barrier_init();
     }
     umma::fence_before_sync();
@@ -665,15 +656,14 @@ __global__ void __launch_bounds__(in::Warps<YW>::THREADS, 1) intra_fwd_tc_kernel
     const uint32_t tmem = sh.tmem;
     follow_stream();
     if (warp < X_WARPS) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(Warps<YW>::X_REGS));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(X_REGS));
         intra_x<DT, SCALAR>(p, base, tmem, sh);
-    } else if (warp < X_WARPS + YW) {
-        if (YW == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(Warps<YW>::Y_REGS));
-        intra_y<DT, SCALAR, YW>(p, base, tmem, sh);
+    } else if (warp < X_WARPS + Y_WARPS) {
+        intra_y<DT, SCALAR>(p, base, tmem, sh);
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(ISSUE_REGS));
         if (umma::elect_one()) {
-            switch (warp - X_WARPS - YW) {
+            switch (warp - X_WARPS - Y_WARPS) {
                 case 0: intra_mm1<DT, SCALAR>(p, base, tmem, sh); break;
                 case 1: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
                 case 2: intra_copy_y<DT>(p, maps, base, sh); break;
@@ -695,13 +685,12 @@ int tc_intra_status_clear() {
     return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess ? 0 : -1;
 }
 
-template <int DT, bool SCALAR, int YW>
-static int launch_intra_fwd_tc_w(const MkdaIntraFwd* p, cudaStream_t stream) {
-    using W = in::Warps<YW>;
-    auto kern = intra_fwd_tc_kernel<DT, SCALAR, YW>;
+template <int DT, bool SCALAR>
+static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, cudaStream_t stream) {
+    auto kern = intra_fwd_tc_kernel<DT, SCALAR>;
     if (int e = ensure_smem((const void*)kern, in::SMEM, "intra_fwd")) return e;
     static const int regs = kernel_registers((const void*)kern);
-    if (regs < W::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
+    if (regs < in::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
     in::Maps maps;
     memset(&maps, 0, sizeof(maps));
     const unsigned long long rows = (unsigned long long)p->L.TT, k_cols = (unsigned long long)p->L.HK * 128, v_cols = (unsigned long long)p->L.HV * 128;
@@ -712,16 +701,8 @@ static int launch_intra_fwd_tc_w(const MkdaIntraFwd* p, cudaStream_t stream) {
     if (!e && DT != MKDA_F32) e = make_rows_map(&maps.v, p->v, 2, rows, v_cols, "intra_fwd", CH, 64);
     if (e) return e;
     const int items = p->L.NC * p->L.HV;
-    launch(kern, items < sm_count() ? items : sm_count(), W::THREADS, in::SMEM, stream, *p, maps);
+    launch(kern, items < sm_count() ? items : sm_count(), in::THREADS, in::SMEM, stream, *p, maps);
     return check_launch("intra_fwd");
-}
-// Eight warps in Y where Y is what is waited for: with a scalar gate, whose X writes a fifth of the operands (4 x 2000 tokens x 16 heads 103 -> 95 us),
-// and with up to four items per SM (fp16 4 x 1000 tokens x 8 heads 50 -> 45 us, 77 tokens 18.4 -> 17.4).  Else X is bound by shared memory, and eight
-// warps cost more than they bring (32 k tokens x 32 heads 825 -> 930 us).  The results are the same bit for bit.
-template <int DT, bool SCALAR>
-static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, cudaStream_t stream) {
-    if (SCALAR || (long long)p->L.NC * p->L.HV <= 4ll * sm_count()) return launch_intra_fwd_tc_w<DT, SCALAR, 8>(p, stream);
-    return launch_intra_fwd_tc_w<DT, SCALAR, SCALAR ? 8 : 4>(p, stream);
 }
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream) {
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {

@@ -1,5 +1,5 @@
-"""GPU: mkda_intra_fwd over ragged chunks.  Sequences of 1, 15, 16, 17, 33, 63, 64, 65 and 100 tokens once (few items: eight warps take the
-inverse) and thirty times over (four warps, several items per CTA, all buffers reused): the same bits everywhere, the fp64 chunk algebra, and
+"""GPU: mkda_intra_fwd over ragged chunks.  Sequences of 1, 15, 16, 17, 33, 63, 64, 65 and 100 tokens once (one item per
+CTA) and thirty times over (several, all buffers reused): the same bits everywhere, the fp64 chunk algebra, and
 nothing of a neighbour that holds infinities."""
 import pytest
 import torch
