@@ -35,7 +35,7 @@ namespace mkda {
 namespace in {
 // Eight warps of Y: the latency of its phases is what an item takes, also where X keeps shared memory busy.  Eight against four, per-channel gate, from 0.2 to
 // 220 items per SM: 3 to 12 % faster throughout, bf16, fp16 and fp32 (bf16 6 k packed tokens x 32 heads 219 -> 190 us, 32 k tokens 1005 -> 860).
-constexpr int X_WARPS = 16, Y_WARPS = 8, THREADS = 32 * (X_WARPS + Y_WARPS + 4);
+constexpr int X_WARPS = 16, Y_WARPS = 8, COPY_X = 1, THREADS = 32 * (X_WARPS + Y_WARPS + 4);
 // registers of the launch (Y keeps them), of X and of the last four warps
 constexpr int LAUNCH_REGS = 72, X_REGS = 80, ISSUE_REGS = 40;
 static_assert(X_WARPS * X_REGS + Y_WARPS * LAUNCH_REGS + 4 * ISSUE_REGS <= (X_WARPS + Y_WARPS + 4) * LAUNCH_REGS, "registers of the launch");
@@ -562,39 +562,48 @@ __device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, 
         umma::wait_mma(&sh.opA, par);
         uint8_t* base = fresh(smem);
         const umma::Opnd a = umma::opnd_k(base + A_, base + A_ + 8192, 64), v = umma::opnd_mn(base + V_, nullptr, 64);
+        auto product_nw = [&]() {
+            umma::gemm(tmem + NW, umma::opnd_mn(base + BK, base + BK + 16384, 64), a, 128, 64, 64, 0u);
+            umma::commit(&sh.mmN);
+        };
         umma::gemm(tmem + U, v, a, 128, 64, 64, 0u);
         umma::commit(&sh.mmV);
+        // Of the last item nw comes first, under Y's writing of the low half (77 tokens 13.8 -> 13.4 us).  In front of other items that would hold up
+        // what waits for u: 14 items per SM 123 -> 129 us
+        if (it + 1 == count) product_nw();
         umma::wait_mma(&sh.opV, par);
         umma::Opnd hi = a;
         hi.lo = 0;
         umma::gemm(tmem + U, v, hi, 128, 64, 64, 1u);
         umma::commit(&sh.mmU);
-        umma::gemm(tmem + NW, umma::opnd_mn(base + BK, base + BK + 16384, 64), a, 128, 64, 64, 0u);
-        umma::commit(&sh.mmN);
+        if (it + 1 < count) product_nw();
     }
+}
+// rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void request_q(const in::Walk& w, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+    umma::tma_load_rows(base + in::Rows<DT, SCALAR>::Q, &maps.q, w.hk * 128, w.start, &sh.ldin);
+}
+template <int DT, bool SCALAR>
+__device__ __forceinline__ void request_rows(const in::Walk& w, int it, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+    using R = in::Rows<DT, SCALAR>;
+    auto& i = sh.info[it & 3];
+    i.item = w.item(); i.start = w.start; i.len = w.len; i.h = w.h; i.hk = w.hk;
+    umma::mbar_expect_tx(&sh.ldin, 2 * R::BYTES + (SCALAR ? 0u : 32768u));
+    if (!SCALAR) umma::tma_load_rows(base + in::RAW_G, &maps.g, w.h * 128, w.start, &sh.ldin);
+    umma::tma_load_rows(base + R::K, &maps.k, w.hk * 128, w.start, &sh.ldin);
+    if (!R::LATE_Q) request_q<DT, SCALAR>(w, maps, base, sh);
 }
 template <int DT, bool SCALAR>
 __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     using namespace in;
     using R = Rows<DT, SCALAR>;
-    // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
-    auto load_q = [&](const Walk& w) { umma::tma_load_rows(base + R::Q, &maps.q, w.hk * 128, w.start, &sh.ldin); };
-    auto load_rows = [&](const Walk& w, int it) {
-        auto& i = sh.info[it & 3];
-        i.item = w.item(); i.start = w.start; i.len = w.len; i.h = w.h; i.hk = w.hk;
-        umma::mbar_expect_tx(&sh.ldin, 2 * R::BYTES + (SCALAR ? 0u : 32768u));
-        if (!SCALAR) umma::tma_load_rows(base + RAW_G, &maps.g, w.h * 128, w.start, &sh.ldin);
-        umma::tma_load_rows(base + R::K, &maps.k, w.hk * 128, w.start, &sh.ldin);
-        if (!R::LATE_Q) load_q(w);
-    };
-    Walk w(p.L);
-    load_rows(w, 0);
-    if (R::LATE_Q) load_q(w);
+    Walk w(p.L);                                            // the first item's rows are on their way
     for (int it = 0; w.valid(); ++it) {
         const size_t item = w.item();
         w.next();
         umma::mbar_wait(&sh.mm1[it & 1], (it >> 1) & 1);    // the operands are dead
-        if (w.valid()) load_rows(w, it + 1);
+        if (w.valid()) request_rows<DT, SCALAR>(w, it + 1, maps, base, sh);
         umma::mbar_wait(&sh.acc, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + item * umma::QUARTER_TILE_BYTES, base + AQ, umma::QUARTER_TILE_BYTES);
         umma::mbar_wait(&sh.hand, it & 1);
@@ -602,7 +611,7 @@ __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Ma
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + item * umma::CHUNK_TILE_BYTES, base + QS, umma::CHUNK_TILE_BYTES);
         umma::bulk_store_wait_read();
         umma::arrive(&sh.khFree);
-        if (R::LATE_Q && w.valid()) load_q(w);
+        if (R::LATE_Q && w.valid()) request_q<DT, SCALAR>(w, maps, base, sh);
     }
 }
 template <int DT>
@@ -645,10 +654,23 @@ __global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const Mkda
     }
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (threadIdx.x == 0) {
-        for (uint64_t* b : {&sh.ldin, &sh.fullV, &sh.mm1[0], &sh.mm1[1], &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
+        for (uint64_t* b : {&sh.fullV, &sh.mm1[0], &sh.mm1[1], &sh.khFree, &sh.mmV, &sh.mmN, &sh.mmU, &sh.bkFree, &sh.abFree}) umma::mbar_init(b, 1);
         for (uint64_t* b : {&sh.op1[0], &sh.op1[1], &sh.rows, &sh.hand, &sh.nwReady, &sh.uReady}) umma::mbar_init(b, X_WARPS);
         for (uint64_t* b : {&sh.opA, &sh.opV, &sh.acc}) umma::mbar_init(b, Y_WARPS);
         umma::fence_barrier_init();
+    }
+    // The first rows are requested while barriers and tensor memory are set up: with one item per CTA all the rest waits for them (77 tokens x 16 heads
+    // 14.3 -> 13.8 us)
+    if (warp == X_WARPS + Y_WARPS + COPY_X) {
+        if (umma::elect_one()) {
+            umma::mbar_init(&sh.ldin, 1);
+            umma::fence_barrier_init();
+            follow_stream();
+            const Walk w(p.L);
+            request_rows<DT, SCALAR>(w, 0, maps, base, sh);
+            if (Rows<DT, SCALAR>::LATE_Q) request_q<DT, SCALAR>(w, maps, base, sh);
+        }
+        __syncwarp();
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -665,7 +687,7 @@ __global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const Mkda
         if (umma::elect_one()) {
             switch (warp - X_WARPS - Y_WARPS) {
                 case 0: intra_mm1<DT, SCALAR>(p, base, tmem, sh); break;
-                case 1: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
+                case COPY_X: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
                 case 2: intra_copy_y<DT>(p, maps, base, sh); break;
                 default: intra_mm3(p, base, tmem, sh);
             }

@@ -304,7 +304,12 @@ def intra(dims, dtype, scalar, n=STEPS):
     wait, arrive = r.agent("products Y")
     for k in range(n):
         wait("hand", k), wait("opA", k)
-        arrive("mmV", k), wait("opV", k), arrive("mmU", k), arrive("mmN", k)
+        arrive("mmV", k)
+        if k + 1 == n:
+            arrive("mmN", k)
+        wait("opV", k), arrive("mmU", k)
+        if k + 1 < n:
+            arrive("mmN", k)
     wait, arrive = r.agent("copies X")
 
     def load_rows(k):
