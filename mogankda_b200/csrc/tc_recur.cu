@@ -213,7 +213,7 @@ __device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainM
     if (tid == 0) umma::bulk_store_wait_read();
 }
 
-template <int OUT>
+template <int OUT, bool NORM>
 __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg_order, const MkdaOutFwd& o, const ChainMaps& maps) {
     using namespace rc;
     using L = RecurLayout<(OUT >= 0)>;
@@ -238,10 +238,6 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
         umma::mbar_init(&sh.gFree, 4);
         umma::fence_barrier_init();
     }
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tmem = sh.tmem;
     follow_stream();
     const int seg = seg_order ? seg_order[blockIdx.z] : blockIdx.z;
 
@@ -254,13 +250,18 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
         const int w = p.warm_start[seg * HV + h];
         if (w > c_beg) { cut = true; c_beg = trans ? c_end : w; }
     }
+    umma::fence_before_sync();
+    __syncthreads();                                       // the table entries have travelled while barriers and tensor memory were set up
+    umma::fence_after_sync();
+    const uint32_t tmem = sh.tmem;
     const int n = c_end - c_beg;
     const bool save_h = OUT >= 0 && p.h;
     // Where the chain itself is what takes the time (no norm: a short epilogue), the output's products stand behind the chain's, and without
     // states to save their place is a second buffer for nw^T, which each step starts with.  In the gap in front of X the products held X up
     // whenever their tile or their accumulator was late: 5.4 -> 4.7 k cycles per step (scalar gate, 64 chains of 32 steps: 107 -> 95 us; of 256
     // steps with states saved: 1073 -> 971).  With the norm the epilogue or HBM is the bound, and the other order is faster by 5 %.
-    const bool late = OUT >= 0 && !o.has_norm;
+    // (At compile time, and the table entries read in front of the first barrier: two steps x 16 chains with the norm 12.0 -> 11.7 us.)
+    constexpr bool late = OUT >= 0 && !NORM;
     const int dn = L::D > 1 || (late && !save_h) ? 2 : 1;
     auto buf_n = [&](int k) { return base + (L::D > 1 ? L::N + (k & 1) * L::T : (k & 1) && dn == 2 ? L::S : L::N); };
     auto n_bar = [&](int k) { return &sh.fullN[dn == 2 ? k & 1 : 0]; };
@@ -345,10 +346,9 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
             }
             __syncwarp();
         } else if (OUT >= 0 && warp >= 20) {
-            if (o.has_norm) recur_epilogue<OUT < 0 ? 0 : OUT, true>(o, maps, sh, base, h, c_beg, n);
-            else recur_epilogue<OUT < 0 ? 0 : OUT, false>(o, maps, sh, base, h, c_beg, n);
-        } else if (OUT > 0 && warp == WARP_GATE) {
-            if (o.has_norm && umma::elect_one()) {
+            recur_epilogue<OUT < 0 ? 0 : OUT, NORM>(o, maps, sh, base, h, c_beg, n);
+        } else if (OUT > 0 && NORM && warp == WARP_GATE) {
+            if (umma::elect_one()) {
                 for (int k = 0; k < n; ++k) {              // rows past the chunk's end belong to the next sequence (or read as zeros) and are never used
                     const int start = o.L.chunk_start[c_beg + k];
                     if (k) {
@@ -459,11 +459,11 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
 }
 
 __global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p, const int* seg_order) {
-    recur_body<-1>(p, seg_order, MkdaOutFwd{}, ChainMaps{});
+    recur_body<-1, false>(p, seg_order, MkdaOutFwd{}, ChainMaps{});
 }
-template <int OUT>
+template <int OUT, bool NORM>
 __global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const int* seg_order, const __grid_constant__ ChainMaps maps) {
-    recur_body<OUT>(p.r, seg_order, p.o, maps);
+    recur_body<OUT, NORM>(p.r, seg_order, p.o, maps);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -691,10 +691,10 @@ int launch_recur_fwd_tc(const MkdaRecurFwd* p, const int* seg_order, cudaStream_
     return check_launch("recur_fwd");
 }
 
-template <int OUT>
-static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
+template <int OUT, bool NORM>
+static int launch_chain_fwd_tc_n(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
     using L = RecurLayout<true>;
-    auto kern = chain_fwd_tc_kernel<OUT>;
+    auto kern = chain_fwd_tc_kernel<OUT, NORM>;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "chain_fwd")) return e;
     static const int regs = kernel_registers((const void*)kern);
     if (regs < L::REGS) return set_error(MKDA_ERR_LAUNCH, "chain_fwd: built with fewer registers than its warps redistribute");
@@ -702,12 +702,16 @@ static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, const int* seg_order, cu
     memset(&maps, 0, sizeof(maps));
     const unsigned long long rows = (unsigned long long)p->o.L.TT, cols = (unsigned long long)p->o.L.HV * 128;
     int e = 0;
-    if (p->o.has_norm && OUT != MKDA_F32) e = make_rows_map(&maps.gate, p->o.gate, 2, rows, cols, "chain_fwd");
+    if (NORM && OUT != MKDA_F32) e = make_rows_map(&maps.gate, p->o.gate, 2, rows, cols, "chain_fwd");
     if (!e && p->o.o_raw) e = make_rows_map(&maps.raw, p->o.o_raw, 4, rows, cols, "chain_fwd", 16);
     if (!e) e = make_rows_map(&maps.out, p->o.out, p->o.out_dtype == MKDA_F32 ? 4 : 2, rows, cols, "chain_fwd", 16);
     if (e) return e;
     launch(kern, dim3(1, p->r.L.HV, p->r.L.NS), L::THREADS, L::SMEM, stream, *p, seg_order, maps);
     return check_launch("chain_fwd");
+}
+template <int OUT>
+static int launch_chain_fwd_tc_t(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
+    return p->o.has_norm ? launch_chain_fwd_tc_n<OUT, true>(p, seg_order, stream) : launch_chain_fwd_tc_n<OUT, false>(p, seg_order, stream);
 }
 int launch_chain_fwd_tc(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream) {
     switch (p->o.has_norm ? p->o.gate_dtype : p->o.out_dtype) {
