@@ -94,16 +94,17 @@ def wants_segments(chunks_per_seq, HV, seg_chunks, sm_count=None, cost_ratio=2.5
     direction and a second pass in the backward direction, about 2.5 x the serial work over a layer step, plus the prefix
     combine.  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
     warm-up truncation, which shortens the two extra passes to a few chunks wherever the gate decays).  With few chains the four passes of a
-    cut call take a segment each however small the share is: about 374 us for segments of 32 chunks, at 2.1 us per chunk for the pre-pass and 3
-    for the others, against 6 us per chunk uncut; without the pre-passes about 205.  So sequences of up to two segments (1.25 where truncation is
-    allowed) are left alone.  45 + 42 + 42 chunks x 16 heads took 415 us in the serial kernels and combines when cut, 280 uncut.  Decided from the
+    cut call take a segment each however small the share is, so sequences of up to 1.85 segments (1.2 where truncation is allowed) are left alone.
+    Uncut / cut, one sequence x 4 to 32 heads: training 0.93 to 0.99 of the time at 54 chunks, 0.98 to 1.03 at 58, 1.02 to 1.07 at 62; forward only 0.90 to 1.04
+    at 54, 0.94 to 1.11 at 58, 0.98 to 1.16 at 62 (few heads gain most by the cut); with truncation 0.94 to 0.98 at 37, 1.00 to 1.04 at 40.
+    45 + 42 + 42 chunks x 16 heads took 415 us in the serial kernels and combines when cut, 280 uncut.  Decided from the
     lengths alone (host), never from data; it plays the role of the reference's intra-card CP decision
     (mogan_kda/ops/gated_delta_rule/chunk/cp/context.py:252-283, cp/autocp/decision.py:54-123)."""
     longest = max(chunks_per_seq, default=0)
     if seg_chunks <= 0 or longest <= seg_chunks:
         return False
     even_share = sum(chunks_per_seq) * HV / (sm_count or _sm_count())
-    return longest > max(cost_ratio * even_share, (0.5 + 0.6 * cost_ratio) * seg_chunks)
+    return longest > max(cost_ratio * even_share, (0.55 + 0.52 * cost_ratio) * seg_chunks)
 
 
 # Entries: (static key, the cu_seqlens tensor itself, its version counter, layout).  The entry keeps the tensor alive

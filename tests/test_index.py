@@ -54,6 +54,9 @@ def test_segment_chooser():
     assert not wants_segments([8, 20, 32], 32, 32, sm_count=148)
     # one long sequence, few heads: the GPU cannot be filled without cutting
     assert wants_segments([1024], 32, 32, sm_count=148)
+    # one sequence, few heads: from 60 chunks on (39 where the pre-passes may be truncated)
+    assert [wants_segments([n], 8, 32, sm_count=148) for n in (59, 60)] == [False, True]
+    assert [wants_segments([n], 8, 32, sm_count=148, cost_ratio=1.25) for n in (38, 39)] == [False, True]
     # many documents of similar length fill the GPU on their own
     assert not wants_segments([40] * 100, 32, 32, sm_count=148)
     # a packed batch dominated by one document: its chain is far longer than the even share
