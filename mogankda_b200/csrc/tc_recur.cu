@@ -213,14 +213,16 @@ __device__ __forceinline__ void recur_epilogue(const MkdaOutFwd& o, const ChainM
     if (tid == 0) umma::bulk_store_wait_read();
 }
 
-template <int OUT, bool NORM>
+template <int OUT, bool NORM, bool SPLIT>
 __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg_order, const MkdaOutFwd& o, const ChainMaps& maps) {
     using namespace rc;
     using L = RecurLayout<(OUT >= 0)>;
+    static_assert(!SPLIT || OUT < 0, "chain_fwd takes whole rows");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
     RecurShared& sh = *reinterpret_cast<RecurShared*>(base + L::TILES);
-    const bool trans = blockIdx.x == 1;
+    const bool trans = (SPLIT ? blockIdx.x >> 1 : blockIdx.x) == 1;
+    const int v0 = SPLIT ? 64 * (blockIdx.x & 1) : 0;      // first of this CTA's rows of the transposed state, which are lanes 0, 1, ...
     const int h = blockIdx.y, HV = p.L.HV;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
@@ -233,7 +235,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
         for (uint64_t* b : {&sh.fullN[0], &sh.fullN[1], &sh.fullK[0], &sh.fullK[1], &sh.fullU[0], &sh.fullU[1], &sh.fullQ, &sh.fullA, &sh.mm1[0], &sh.mm1[1],
                             &sh.mm2[0], &sh.mm2[1], &sh.mmS, &sh.mmO, &sh.fullG, &sh.freed[0], &sh.freed[1]})
             umma::mbar_init(b, 1);
-        for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree[0], &sh.uFree[1], &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, COMPUTE / 32);
+        for (uint64_t* b : {&sh.opS, &sh.opV, &sh.uFree[0], &sh.uFree[1], &sh.ready[0], &sh.ready[1]}) umma::mbar_init(b, SPLIT ? COMPUTE / 64 : COMPUTE / 32);
         umma::mbar_init(&sh.oFree, 4);
         umma::mbar_init(&sh.gFree, 4);
         umma::fence_barrier_init();
@@ -289,7 +291,14 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
                     umma::bulk_load(sh.gl[k & 3], p.gl + ((size_t)(c_beg + k) * HV + h) * DK, DK * 4, bar);
                 };
                 auto load_k = [&](int k) { if (k < n) one(buf_k(k), p.kbar, k, &sh.fullK[k % L::D]); };
-                auto load_u = [&](int k) { if (k < n && !trans) one(buf_u(k), p.u, k, &sh.fullU[k % L::D]); };
+                auto load_u = [&](int k) {
+                    if (k >= n || trans) return;
+                    if (!SPLIT) return one(buf_u(k), p.u, k, &sh.fullU[k % L::D]);
+                    const uint8_t* src = reinterpret_cast<const uint8_t*>(p.u) + ((size_t)(c_beg + k) * HV + h) * umma::CHUNK_TILE_BYTES + 128 * v0;
+                    umma::mbar_expect_tx(&sh.fullU[k % L::D], umma::CHUNK_TILE_BYTES / 2);
+                    umma::bulk_load(buf_u(k), src, 8192, &sh.fullU[k % L::D]);
+                    umma::bulk_load(buf_u(k) + 16384, src + 16384, 8192, &sh.fullU[k % L::D]);
+                };
                 auto load_q = [&](int k) { if (OUT >= 0 && k < n) one(base + L::Q, o.qs, k, &sh.fullQ); };
                 auto load_a = [&](int k) {
                     if (OUT < 0 || k >= n) return;
@@ -375,17 +384,17 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
             }
             __syncwarp();
         }
-    } else {
+    } else if (!SPLIT || (warp & 3) < 2) {
         if (OUT >= 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-        const int cg = warp >> 2, row = (warp & 3) * 32 + lane;
+        const int cg = warp >> 2, row = (warp & 3) * 32 + lane, vrow = v0 + row;
         const bool vf = p.state_v_first != 0;
         float s[32];
         const int h0row = p.seg_h0 ? p.seg_h0[seg] : seg;
         if (!trans && !cut && p.h0 && h0row >= 0) {
-            load_state(p.h0 + ((size_t)h0row * HV + h) * DK * DV, vf && !p.h0_k_first, row, cg, s);
+            load_state(p.h0 + ((size_t)h0row * HV + h) * DK * DV, vf && !p.h0_k_first, vrow, cg, s);
         } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) s[j] = trans && !cut && cg * 32 + j == row ? 1.f : 0.f;
+            for (int j = 0; j < 32; ++j) s[j] = trans && !cut && cg * 32 + j == vrow ? 1.f : 0.f;
         }
         // u^T of step k into the accumulator that its first product adds to
         auto preload_u = [&](int k) {
@@ -421,7 +430,7 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
                 stage_state(base + L::S, row, cg, hi);
                 umma::signal(&sh.ready[0], lane);
             } else if (OUT < 0 && p.h && !trans) {
-                save_state_tile(reinterpret_cast<uint8_t*>(p.h) + it * umma::STATE_TILE_BYTES, row, cg, hi, lo);
+                save_state_tile(reinterpret_cast<uint8_t*>(p.h) + it * umma::STATE_TILE_BYTES, vrow, cg, hi, lo);
             }
             wait_mma(&sh.mm1[k & 1], step_par(k));
             {
@@ -430,8 +439,8 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
                 signal_tmem(&sh.opV, lane);
                 if (p.Vd && !trans) {
                     uint8_t* tile = reinterpret_cast<uint8_t*>(p.Vd) + it * umma::CHUNK_TILE_BYTES;
-                    store_pair(tile, 128, row, 2 * cg, vh);
-                    store_pair(tile + 16384, 128, row, 2 * cg, vl);
+                    store_pair(tile, 128, vrow, 2 * cg, vh);
+                    store_pair(tile + 16384, 128, vrow, 2 * cg, vl);
                 }
             }
             if (save_h) {
@@ -447,10 +456,10 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
         }
         // transition: M[K out][K in] with this thread holding row `row` = K in; state: [K][V] or [V][K]
         if (trans) {
-            if (p.mt) store_state(p.mt + ((size_t)seg * HV + h) * DK * DK, false, row, cg, s);
+            if (p.mt) store_state(p.mt + ((size_t)seg * HV + h) * DK * DK, false, vrow, cg, s);
         } else if (p.ht) {
             const int r = p.seg_ht ? p.seg_ht[seg] : seg;
-            if (r >= 0) store_state(p.ht + ((size_t)r * HV + h) * DK * DV, vf, row, cg, s);
+            if (r >= 0) store_state(p.ht + ((size_t)r * HV + h) * DK * DV, vf, vrow, cg, s);
         }
     }
     umma::fence_before_sync();
@@ -458,13 +467,19 @@ __device__ __forceinline__ void recur_body(const MkdaRecurFwd& p, const int* seg
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(RecurLayout<false>::THREADS, 1) recur_fwd_tc_kernel(const MkdaRecurFwd p, const int* seg_order) {
-    recur_body<-1, false>(p, seg_order, MkdaOutFwd{}, ChainMaps{});
+    recur_body<-1, false, SPLIT>(p, seg_order, MkdaOutFwd{}, ChainMaps{});
 }
 template <int OUT, bool NORM>
 __global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_kernel(const MkdaChainFwd p, const int* seg_order, const __grid_constant__ ChainMaps maps) {
-    recur_body<OUT, NORM>(p.r, seg_order, p.o, maps);
+    recur_body<OUT, NORM, false>(p.r, seg_order, p.o, maps);
 }
+// Rows of the transposed state (v) never meet: S^T nw, Vd^T kbar and their reverses contract over K and over tokens.  So with at most half as many
+// chains as SMs a chain is shared between two CTAs of 64 rows each, with the same bits: a step is bound by what one SM moves (192 or 240 KB at 35 B per
+// cycle, half of it the saved states and Vd), and that is 112 or 128 KB then.  recur_fwd 45 steps x 48 chains 131 -> 99 us, 16 x 32 48.5 -> 37.5, 4 x 4
+// 15.2 -> 11.9; bwd_dh 150 -> 113, 56 -> 43, 15.7 -> 12.2, 256 x 64 894 -> 702.  (chain_fwd gained nothing: 256 x 64 996, 32 x 64 95 us.)
+static bool split_chains(long long chains) { return 2 * chains <= sm_count(); }
 
 // ---------------------------------------------------------------------------------------------------------
 // The pre-pass of a cut call: state from zero and transition of a segment in ONE CTA, when there are more of them than SMs.  A chain of its own
@@ -685,9 +700,11 @@ int launch_recur_fwd_tc(const MkdaRecurFwd* p, const int* seg_order, cudaStream_
         return check_launch("recur_fwd");
     }
     using L = RecurLayout<false>;
-    auto kern = recur_fwd_tc_kernel;
+    const int per_segment = p->want_transition ? 2 : 1;
+    const bool split = split_chains((long long)per_segment * p->L.HV * p->L.NS);
+    auto kern = split ? recur_fwd_tc_kernel<true> : recur_fwd_tc_kernel<false>;
     if (int e = ensure_smem((const void*)kern, L::SMEM, "recur_fwd")) return e;
-    launch(kern, dim3(p->want_transition ? 2 : 1, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream, *p, seg_order);
+    launch(kern, dim3(split ? 2 * per_segment : per_segment, p->L.HV, p->L.NS), L::THREADS, L::SMEM, stream, *p, seg_order);
     return check_launch("recur_fwd");
 }
 
@@ -738,12 +755,13 @@ constexpr int DH_K = 2 * DH_SET, DH_N = DH_K + 32 * rc::KB, DH_TILES = DH_N + 32
 constexpr int DH_SMEM = DH_TILES + (int)sizeof(DhShared);
 static_assert(DH_SMEM <= 232448, "shared memory of one CTA");
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwdDh p, const int* seg_order) {
     using namespace rc;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
     DhShared& sh = *reinterpret_cast<DhShared*>(base + DH_TILES);
-    const int h = blockIdx.y, HV = p.L.HV;
+    const int h = blockIdx.y, HV = p.L.HV, v0 = SPLIT ? 64 * blockIdx.x : 0;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (umma::smem_u32(base) & 1023) {                     // ... and nothing runs if that ever fails to hold
         follow_stream();
@@ -753,7 +771,7 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
     if (warp == 0) umma::tmem_alloc(&sh.tmem, 512);
     if (tid == 0) {
         for (uint64_t* b : {&sh.fullA[0], &sh.fullA[1], &sh.fullK, &sh.fullN, &sh.mm1, &sh.mm2}) umma::mbar_init(b, 1);
-        for (uint64_t* b : {&sh.opS, &sh.opV}) umma::mbar_init(b, COMPUTE / 32);
+        for (uint64_t* b : {&sh.opS, &sh.opV}) umma::mbar_init(b, SPLIT ? COMPUTE / 64 : COMPUTE / 32);
         umma::fence_barrier_init();
     }
     umma::fence_before_sync();
@@ -782,8 +800,14 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
             };
             auto set_a = [&](int k) {
                 uint64_t* bar = &sh.fullA[k & 1];
-                umma::mbar_expect_tx(bar, 2 * umma::CHUNK_TILE_BYTES + umma::QUARTER_TILE_BYTES + DK * 4);
-                load((k & 1) * DH_SET, p.dO_in_t, item(k), umma::CHUNK_TILE_BYTES, bar);
+                umma::mbar_expect_tx(bar, (SPLIT ? 3 : 4) * umma::CHUNK_TILE_BYTES / 2 + umma::QUARTER_TILE_BYTES + DK * 4);
+                if (SPLIT) {                               // one 64-column block of the hi and of the lo tile; the products read the other block unloaded:
+                    const uint8_t* src = reinterpret_cast<const uint8_t*>(p.dO_in_t) + item(k) * umma::CHUNK_TILE_BYTES + 128 * v0;
+                    umma::bulk_load(base + (k & 1) * DH_SET, src, 8192, bar);              // accumulator lanes that nobody looks at
+                    umma::bulk_load(base + (k & 1) * DH_SET + 16384, src + 16384, 8192, bar);
+                } else {
+                    load((k & 1) * DH_SET, p.dO_in_t, item(k), umma::CHUNK_TILE_BYTES, bar);
+                }
                 load((k & 1) * DH_SET + 65536, p.Aqk, item(k), umma::QUARTER_TILE_BYTES, bar);
                 load((k & 1) * DH_SET + 32768, p.qs, item(k), umma::CHUNK_TILE_BYTES, bar);
                 umma::bulk_load(sh.gl[k & 3], p.gl + item(k) * DK, DK * 4, bar);
@@ -827,8 +851,8 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
             }
         }
         __syncwarp();
-    } else {
-        const int cg = warp >> 2, row = (warp & 3) * 32 + lane;
+    } else if (!SPLIT || (warp & 3) < 2) {
+        const int cg = warp >> 2, row = v0 + (warp & 3) * 32 + lane;
         const bool vf = p.state_v_first != 0;
         float s[32];
         const int drow = p.seg_dht ? p.seg_dht[seg] : seg;
@@ -873,9 +897,10 @@ __global__ void __launch_bounds__(rc::THREADS, 1) bwd_dh_tc_kernel(const MkdaBwd
 }
 
 int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stream) {
-    auto kern = bwd_dh_tc_kernel;
+    const bool split = split_chains((long long)p->L.HV * p->L.NS);
+    auto kern = split ? bwd_dh_tc_kernel<true> : bwd_dh_tc_kernel<false>;
     if (int e = ensure_smem((const void*)kern, DH_SMEM, "bwd_dh")) return e;
-    launch(kern, dim3(1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream, *p, seg_order);
+    launch(kern, dim3(split ? 2 : 1, p->L.HV, p->L.NS), rc::THREADS, DH_SMEM, stream, *p, seg_order);
     return check_launch("bwd_dh");
 }
 

@@ -93,3 +93,19 @@ def test_state_and_transition_in_one_cta(lens, seg, vfirst, monkeypatch):
     _, _, ht3, mt3 = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, **kw)
     assert torch.equal(ht3[-1], ht[0]) and torch.equal(ht3[0], ht[-1]) and (ht3[1:-1] == 7).all() and torch.equal(mt3, mt)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("epi,scalar,dtype", [("silu", False, torch.float32), (None, False, torch.bfloat16), (None, True, torch.float16)])
+@pytest.mark.parametrize("T", [1, 64, 193])
+def test_a_chain_shared_by_two_ctas(T, epi, scalar, dtype):
+    """Up to half as many (sequence, head) chains as SMs: two CTAs share a chain, 64 rows of the transposed state each.  A sequence has the same bits
+    alone (shared) and among so many others that no chain is, states in and out in both layouts, forward only and with a backward pass."""
+    HV, N = 4, torch.cuda.get_device_properties(0).multi_processor_count // 8 + 1
+    gate = "precomputed" if scalar else "eda"
+    lv, do, dht, opts, epi = make_inputs(B=N, T=T, HK=2, HV=HV, dtype=dtype, gate=gate, scalar=scalar, epi=epi, seed=41)
+    first = lambda t: t[:1].contiguous() if t.dim() >= 3 and t.shape[0] == N else t          # noqa: E731
+    for vfirst in (False, True):
+        many = run(mk.chunk_delta_rule, lv, do, dht, opts, epi, vfirst=vfirst)
+        one = run(mk.chunk_delta_rule, {k: first(t) for k, t in lv.items()}, first(do), first(dht), opts, epi, vfirst=vfirst)
+        for k in ("o", "ht", "dq", "dk", "dv", "dg", "dbeta", "dh0"):
+            assert torch.equal(many[k][:1], one[k]), k
