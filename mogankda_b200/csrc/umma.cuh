@@ -46,15 +46,6 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& 
     unpack2(add2(pack2(a, b), pack2(__uint_as_float((h << 16) ^ 0x80000000u), __uint_as_float((h & 0xffff0000u) ^ 0x80000000u))), ra, rb);
     l = pack_bf16x2(ra, rb);
 }
-// ... and what the two halves leave (2^-18 of the value), as a third pair
-__device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& l, uint32_t& rest) {
-    h = pack_bf16x2(a, b);
-    float ra, rb, sa, sb;
-    unpack2(add2(pack2(a, b), pack2(__uint_as_float((h << 16) ^ 0x80000000u), __uint_as_float((h & 0xffff0000u) ^ 0x80000000u))), ra, rb);
-    l = pack_bf16x2(ra, rb);
-    unpack2(add2(pack2(ra, rb), pack2(__uint_as_float((l << 16) ^ 0x80000000u), __uint_as_float((l & 0xffff0000u) ^ 0x80000000u))), sa, sb);
-    rest = pack_bf16x2(sa, sb);
-}
 __device__ __forceinline__ void store_split8(uint8_t* hi, uint8_t* lo, int R, int r, int k8, const float (&v)[8]) {
     uint32_t h[4], l[4];
 #pragma unroll
@@ -414,12 +405,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-    float x[8];
-    tmem_ld8(taddr, x);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(x[i]);
 }
 // two 8-column reads behind one wait
 __device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, float (&a)[8], float (&b)[8]) {

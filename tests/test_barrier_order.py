@@ -360,3 +360,80 @@ def test_bwd_dh():
 @pytest.mark.parametrize("dtype", ["fp16", "fp32"])
 def test_intra_fwd(dtype, scalar):
     assert intra(_slots("tc_intra.cu", "Shared"), dtype, scalar).late_waits() == []
+
+
+def bwd_chunk(dims, scalar, from_hbm, n=STEPS):
+    """bwd_chunk: compute warps a (row block 0), b (row block 3), one thread that issues products, one that copies, one warp for the per-row scalars."""
+    slots = {k: (d[0] if d else 1) for k, d in dims.items()}
+    slots["mmI"] = slots["opI"] = 1                        # [4] are the row blocks
+    r = Roles(slots)
+    r.count = {**dict.fromkeys(("opW", "free", "opI3", "syncTop", "syncMid", "syncEnd"), 2), "fullS": 2}
+    if scalar:
+        r.count["opI0"] = 2
+    for w in "ab":
+        wait, arrive = r.agent("compute" + w)
+
+        def sync(name, k):
+            arrive(name, k), wait(name, k)
+        for k in range(n):
+            wait("rows", k)
+            sync("syncTop", k)
+            wait("mmW", k), arrive("opW", k)
+            wait("fullS", k), wait("fullT", k), wait("mmL", k), wait("mmT", k)
+            sync("syncMid", k)
+            arrive("free", k)
+            if scalar or w == "a":
+                arrive("opI3", k) if not scalar else None
+                arrive("opI0", k)
+            else:
+                arrive("opI3", k)
+            wait("mmI0" if scalar or w == "a" else "mmI3", k)
+            sync("syncEnd", k)
+    wait, arrive = r.agent("products")
+    wait("fullW", 0), arrive("mmW", 0)
+    for k in range(n):
+        wait("fullS", k), wait("opW", k), arrive("mmL", k)
+        wait("fullT", k), arrive("mmT", k)
+        if not scalar:
+            wait("opI3", k), arrive("mmI3", k)
+        wait("opI0", k), arrive("mmI0", k)
+        if k + 1 < n:
+            wait("mmI0", k), wait("fullW", k + 1), arrive("mmW", k + 1)
+    wait, arrive = r.agent("copies")
+    arrive("fullW", 0), arrive("fullS", 0)
+    for k in range(n):
+        if k:
+            wait("mmI0", k - 1)
+            if not scalar:
+                arrive("fullW", k)
+        arrive("fullS", k)                                 # dO: the second part of its bytes
+        wait("mmW", k), arrive("fullT", k)
+        if k + 1 == n:
+            break
+        if from_hbm:
+            wait("mmL", k)
+        wait("free", k)
+        if scalar:
+            arrive("fullW", k + 1)
+        arrive("fullS", k + 1)
+    wait, arrive = r.agent("rows")
+    for k in range(n):
+        if k:
+            wait("free", k - 1)
+        arrive("rows", k)
+    return r
+
+
+@pytest.mark.parametrize("from_hbm", [False, True])
+@pytest.mark.parametrize("scalar", [False, True])
+def test_bwd_chunk(scalar, from_hbm):
+    """... and no role waits for a phase of a barrier without having waited for the one in front of it: a wait by parity would return at once if that
+    were still to come."""
+    r = bwd_chunk(_slots("tc_bwd_chunk.cu", "Shared"), scalar, from_hbm)
+    assert r.late_waits() == []
+    for name, ops in r.agents.items():
+        seen = {}
+        for what, bar, phase in ops:
+            if what == "wait":
+                assert phase == seen.get(bar, 0), (name, bar, phase)
+                seen[bar] = phase + 1
