@@ -246,9 +246,11 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
 }
 
 // Tables and per-row scalars of an item: requested two items ahead of their use, written once the item in front has passed its state products.
-template <bool SCALAR, bool SPREAD>
+template <int DT, bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared& sh, int lane) {
     using namespace bc;
+    constexpr uint32_t ROW = DT == MKDA_F32 ? 512 : 256;
+    const bool from_hbm = (size_t)p.L.NC * p.L.HV > (256u << 20) / (272u << 10);          // as for the tiles
     uint32_t n = 0;
     for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
         const int start = p.L.chunk_start[w.chunk()], len = p.L.chunk_len[w.chunk()], h = w.head(), hk = w.hk();
@@ -278,6 +280,20 @@ __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared
         __syncwarp();
         if (lane == 0) umma::arrive(&sh.rows[n & 1]);
         __syncwarp();
+        if (from_hbm) {                                    // the rows of v, g, k and q start on their way into L2
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int i = lane + 32 * m;
+                if (i >= len) continue;
+                const size_t tk = ((size_t)(start + i) * p.L.HK + hk), tv = ((size_t)(start + i) * p.L.HV + h);
+                umma::l2_prefetch(static_cast<const uint8_t*>(p.v) + tv * ROW, ROW);
+                if (!SCALAR) umma::l2_prefetch(p.g_c + tv * 128, 512);
+                if (w.j == 0) {
+                    umma::l2_prefetch(static_cast<const uint8_t*>(p.k) + tk * ROW, ROW);
+                    umma::l2_prefetch(static_cast<const uint8_t*>(p.q) + tk * ROW, ROW);
+                }
+            }
+        }
     }
 }
 
@@ -774,7 +790,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
             if (elect_one()) bwd_chunk_load<SCALAR, SPREAD>(p, base, sh);
             __syncwarp();
         } else if (warp == WARP_ROWS) {
-            bwd_chunk_rows<SCALAR, SPREAD>(p, sh, threadIdx.x & 31);
+            bwd_chunk_rows<DT, SCALAR, SPREAD>(p, sh, threadIdx.x & 31);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
