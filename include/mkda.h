@@ -122,6 +122,8 @@ typedef struct {
     float* q_rstd_out; float* k_rstd_out;          /* also written, [TT,HK], or NULL */
 } MkdaIntraFwd;
 int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream);
+/* The same without A, which only a backward pass reads (the field is not looked at). */
+int mkda_intra_fwd_forward_only(const MkdaIntraFwd* p, void* stream);
 
 /* State tile: how the per-chunk states `h` (state entering a chunk) and `dh` (gradient of the state leaving it) travel
  * between the kernels.  One tile per (chunk, v-head), MKDA_STATE_TILE_BYTES each, is the tensor-core operand itself: the

@@ -122,7 +122,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     }
     keep.want(&s.g_c, c.scalar_gate ? row / 128 : row);
     keep.want(&s.beta_e, (int64_t)c.TT * c.HV * 4);
-    keep.want(&s.A, c.tiles(MKDA_QUARTER_TILE_BYTES));
+    if (need_bwd) keep.want(&s.A, c.tiles(MKDA_QUARTER_TILE_BYTES));
     keep.want(&s.Aqk, c.tiles(MKDA_QUARTER_TILE_BYTES));
     keep.want(&s.nw, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.kbar, c.tiles(MKDA_CHUNK_TILE_BYTES));
@@ -163,7 +163,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.scale = c.scale;
         p.l2 = c.l2; p.l2_eps = 1e-6f; p.q_rstd_out = s.q_rstd; p.k_rstd_out = s.k_rstd;
         p.A = s.A; p.Aqk = s.Aqk; p.nw = s.nw; p.u = u; p.kbar = s.kbar; p.qs = s.qs; p.gl = s.gl;
-        check_rc(mkda_intra_fwd(&p, st), "mkda_intra_fwd");
+        check_rc(need_bwd ? mkda_intra_fwd(&p, st) : mkda_intra_fwd_forward_only(&p, st), "mkda_intra_fwd");
     }
     Tensor ht;
     if (c.want_ht) ht = c.states(c.N);

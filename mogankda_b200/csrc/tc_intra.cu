@@ -482,7 +482,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
                 for (int e = 0; e < 8; ++e)
                     if (k8 * 8 + e > r) a8[e] = 0.f;
             }
-            store_split8(At, At + 8192, 64, r, k8, a8);
+            if (p.A) store_split8(At, At + 8192, 64, r, k8, a8);         // a forward-only call has no use for it
             store_split8(base + A_, base + A_ + 8192, 64, r, k8, a8);
         }
         // beta v in two halves, one after the other in the same place: u is formed in front of nw, as soon as the low half is there.  fp32 rows are read
