@@ -23,7 +23,7 @@
 // beta goes to v and k 2^g and not into A, whose diagonal stays exact.  With A diag(beta) as the operand a bf16 v would be one as it stands and take a
 // product less per k-step (6 to 12 % of the kernel), but a rounded beta on the diagonal is an error that all 128 values of a row have in common:
 // dh0 1.03 times as far from fp64 (geometric mean of 90 bf16 layers; 1.4 at worst), fp32 gradients 1.08, final states 1.2.
-// An item takes 12 to 13 k cycles (18 k before): shared memory (operands, tiles and rows of X) and the latency of Y are about as long.
+// An item takes 16 k cycles, all of them X's (rows 3 k, operands 5 k, L2 statistics 1.5 k, nw and u 2.9 k, tiles 3 k), 11 k of them Y's; 12 k with a scalar gate, Y's.
 // 6 k packed tokens x 32 heads 240 -> 190 us, 32 k tokens x 32 heads 1121 -> 860, scalar gate 4 x 2000 tokens x 16 heads 129 -> 99.
 #include "host.h"
 #include "intra.cuh"

@@ -2,7 +2,7 @@
 
 An mbarrier is waited for by the parity of a phase: the wait has to be made before the NEXT phase of the barrier completes, or it blocks on the phase
 after that.  So for every wait something must keep the next phase from completing until the waiter has passed.  The roles of the kernels that carry
-the state and of the WY preparation are restated here as sequences of arrivals and waits; every role is held in front of each of its waits while all
+the state, of the WY preparation and of the chunk backward are restated here as sequences of arrivals and waits; every role is held in front of each of its waits while all
 others run as far as they can (copies and products complete at once), and the barrier it is held at must not have gone past the phase it waits for.
 The system is monotone, so this covers every schedule.
 
