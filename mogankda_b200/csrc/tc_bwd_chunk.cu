@@ -193,6 +193,8 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
     }
 }
 
+// Every tile is read here for the last time and may leave L2 at once, which keeps what comes next: the tiles that bwd_dh has written, and the gradients for
+// the kernels behind (1B shape 201 -> 193 us, fp16 4 x 1000 tokens 66 -> 63, short documents 248 -> 242, 64k packed tokens no difference).
 // S and Vd of the next item are requested once the state products and dgl of the current one are done, dO, dVd and A once the intra-chunk products
 // are, dS' once dVd and A have been read.
 template <bool SCALAR, bool SPREAD>
@@ -202,13 +204,13 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
     const bool from_hbm = (size_t)p.L.NC * p.L.HV > (256u << 20) / (272u << 10);          // twice L2 (126 MB)
     auto request_s = [&](size_t it) {
         umma::mbar_expect_tx(&sh.fullS, umma::STATE_TILE_BYTES + 2 * umma::CHUNK_TILE_BYTES);
-        umma::bulk_load(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
-        umma::bulk_load(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
+        umma::bulk_load_last(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
+        umma::bulk_load_last(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
     };
     auto request_w = [&](size_t it) {
         umma::mbar_expect_tx(&sh.fullW, umma::CHUNK_TILE_BYTES + umma::QUARTER_TILE_BYTES);
-        umma::bulk_load(base + W_, src(p.dVd_t, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullW);
-        umma::bulk_load(base + A_, src(p.A, it, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES, &sh.fullW);
+        umma::bulk_load_last(base + W_, src(p.dVd_t, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullW);
+        umma::bulk_load_last(base + A_, src(p.A, it, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES, &sh.fullW);
     };
     uint32_t n = 0;
     for (ItemWalk<SPREAD> w(p.L); w.valid(); ++n) {
@@ -222,10 +224,10 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
         if (n && !SCALAR) request_w(it);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            umma::bulk_load(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
+            umma::bulk_load_last(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
         umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read
         umma::mbar_expect_tx(&sh.fullT, umma::STATE_TILE_BYTES);
-        umma::bulk_load(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
+        umma::bulk_load_last(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
         w.next();
         if (!w.valid()) break;
         const size_t in = w.item();

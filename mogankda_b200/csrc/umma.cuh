@@ -328,6 +328,13 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+// The same for what nobody reads again: its lines are the first to leave L2, which keeps what the next kernel wants.
+__device__ __forceinline__ void bulk_load_last(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 :: "r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)), "l"(policy) : "memory");
+}
 // Tiled copy of one 64 x 128 box of a row tensor (host.h: make_rows_map) starting at element column x (x times the element
 // size a multiple of 16 bytes) and row y; lands as a dense [64][128] block at the 128-byte aligned `smem_dst`, completion
 // counted in bytes (the whole box, rows past the tensor's end included) on `bar`.
