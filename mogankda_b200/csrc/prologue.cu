@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(32 * GB_WARPS, 2) gate_bwd_kernel(const MkdaGa
     float4 bias = splat4(0.f);
     if (p.dt_bias) bias = *reinterpret_cast<const float4*>(p.dt_bias + h * 128 + 4 * lane);
     float4 pa = splat4(0.f), pb = splat4(0.f);
-    for (int c = blockIdx.y; c < p.L.NC; c += gridDim.y) {
+    for (int c = p.L.NC - 1 - (int)blockIdx.y; c >= 0; c -= (int)gridDim.y) {       // the latest tiles first: they are in L2 (1B shape 41.2 -> 39.9 us)
         const int start = p.L.chunk_start[c], len = p.L.chunk_len[c];
         float4 vals[GB_ROWS], xs[GB_ROWS];
 #pragma unroll
