@@ -33,7 +33,7 @@
 // channel and 16 tokens in registers from the first use to the last; its anchors are scalars, the column tiles go into tensor memory (over Dq and Dk),
 // and of the intra-chunk part only [Qr; beta Kr] and the weights are in shared memory.  That leaves room there: S and Vd of the next item travel from the
 // middle of this one on, where everything used to wait for its end (232 KB at 44 B per cycle while the epilogue wrote 96 KB, and nothing before).
-// (Operands by token rows, as the forward kernel builds them: k, q, g requested twice, the column tiles 4.2 k cycles instead of 1.8 k.)
+// (Operands by token rows, as the forward kernel builds them: k, q and g requested twice, 2.5 k cycles each time, and 144 KB of operands in shared memory.)
 // dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
 // An item takes 23 k cycles (26 k before): 1B shape 223 -> 201 us, 64 k packed tokens x 32 heads 3.64 -> 3.29 ms, short documents 267 -> 250 us, fp16 4 x 1000
 // tokens 74 -> 66, scalar gate 4 x 16 k tokens x 16 heads 1313 -> 1249; with the hints below 193 us, 2.84 to 3.2 ms, 242 us, 63, 1210.
