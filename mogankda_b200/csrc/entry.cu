@@ -3,16 +3,18 @@
 
 using namespace mkda;
 
-static int intra_fwd(const MkdaIntraFwd* p, bool forward_only, void* stream) {
-    if (!p || !p->q || !p->k || !p->v || !p->g_c || !p->beta || (!p->A && !forward_only) || !p->Aqk || !p->nw || !p->u || !p->kbar || !p->qs || !p->gl)
+static int intra_fwd(const MkdaIntraFwd* given, bool forward_only, void* stream) {
+    if (!given) return set_error(MKDA_ERR_ARG, "intra_fwd: null argument");
+    MkdaIntraFwd call = *given;
+    if (forward_only) call.A = nullptr;                    // whatever stands there
+    const MkdaIntraFwd* p = &call;
+    if (!p->q || !p->k || !p->v || !p->g_c || !p->beta || (!p->A && !forward_only) || !p->Aqk || !p->nw || !p->u || !p->kbar || !p->qs || !p->gl)
         return set_error(MKDA_ERR_ARG, "intra_fwd: null argument");
     if (any_misaligned(p->q, p->k, p->v, p->g_c, p->A, p->Aqk, p->nw, p->u, p->kbar, p->qs, p->gl))
         return set_error(MKDA_ERR_ARG, "intra_fwd: tensors must be 16-byte aligned");
     if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "intra_fwd: HV must be a multiple of HK");
     if (p->L.NC == 0) return MKDA_OK;
-    MkdaIntraFwd call = *p;
-    if (forward_only) call.A = nullptr;
-    return launch_intra_fwd_tc(&call, (cudaStream_t)stream);
+    return launch_intra_fwd_tc(p, (cudaStream_t)stream);
 }
 extern "C" int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream) { return intra_fwd(p, false, stream); }
 extern "C" int mkda_intra_fwd_forward_only(const MkdaIntraFwd* p, void* stream) { return intra_fwd(p, true, stream); }

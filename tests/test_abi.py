@@ -102,6 +102,21 @@ def test_entry_points_reject_misaligned_tensors_without_launching():
     assert b"16-byte aligned" in lib.mkda_last_error()
 
 
+@pytest.mark.parametrize("A", [0, 0x40010, 0x40001])
+def test_forward_only_does_not_look_at_A(lib, A):
+    """A host may leave the field of mkda_intra_fwd_forward_only as it is; mkda_intra_fwd needs it, aligned.  Without chunks: nothing is launched."""
+    from mogankda_b200 import _lib
+    p = _lib.STRUCTS["MkdaIntraFwd"]()
+    p.L.HK, p.L.HV, p.L.NC, p.A = 1, 1, 0, A
+    for f in ("q", "k", "v", "g_c", "beta", "Aqk", "nw", "u", "kbar", "qs", "gl"):
+        setattr(p, f, 0x30000)
+    assert lib.mkda_intra_fwd_forward_only(ctypes.byref(p), None) == 0
+    assert lib.mkda_intra_fwd(ctypes.byref(p), None) == (0 if A and A % 16 == 0 else _lib.MKDA_ERR_ARG)
+    p.nw = 0x30001
+    assert lib.mkda_intra_fwd_forward_only(ctypes.byref(p), None) == _lib.MKDA_ERR_ARG
+    assert lib.mkda_intra_fwd_forward_only(None, None) == _lib.MKDA_ERR_ARG
+
+
 @pytest.mark.parametrize("scalar", [False, True])
 def test_parameter_tensors_of_other_sizes_are_refused(lib, scalar):
     """The kernels take the sizes of A_log, dt_bias and the norm's tensors from v and g; a smaller one would be read, and its gradient written,
