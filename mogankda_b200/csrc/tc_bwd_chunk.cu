@@ -689,7 +689,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
             }
             if (SCALAR) umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, c0), umma::tmem_addr(tmem, warp, 64 + c0), x, y);
             else umma::tmem_ld8x2(umma::tmem_addr(tmem, warp, 32 * cg + 8 * hf), umma::tmem_addr(tmem, warp, 32 * cg + 16 + 8 * hf), x, y);
-            // Rows past the end come out as zeros: it.rk, it.rq and it.beta are 0 there, the tiles' rows and the weights too, and every other factor is finite.
+            // Rows past the end: it.rk, it.rq and it.beta are 0 there, the tiles' rows and the weights too; but 0 times what is not finite is not 0, and
+            // these rows leave as zeros whatever the others hold.
             float bsv[8], dgs[8];
 #pragma unroll
             for (int r4 = 0; r4 < 2; ++r4) {               // the rows' scalars four at a time: one broadcast read each instead of four
@@ -712,11 +713,12 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
 #pragma unroll
                     for (int o = 0; o < 2; ++o) {
                         const int io = i + o;
-                        if (first_of_group) { oq[io * DK] = dqv[o]; ok[io * DK] = dkv[o]; }
-                        else { red_add(oq + io * DK, dqv[o]); red_add(ok + io * DK, dkv[o]); }
-                        if (SCALAR) dgs[2 * pr + o] = dgv[o];
-                        else if (io == len - 1) dg_last = dgv[o];
-                        else og[io * DK] = dgv[o];
+                        const float dq = io < len ? dqv[o] : 0.f, dk = io < len ? dkv[o] : 0.f, dg = io < len ? dgv[o] : 0.f;
+                        if (first_of_group) { oq[io * DK] = dq; ok[io * DK] = dk; }
+                        else { red_add(oq + io * DK, dq); red_add(ok + io * DK, dk); }
+                        if (SCALAR) dgs[2 * pr + o] = dg;
+                        else if (io == len - 1) dg_last = dg;
+                        else og[io * DK] = dg;
                     }
                 }
             }

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import mogankda_b200 as mk
+from mogankda_b200.index import get_layout
 from oracle import kda_oracle as orc
 from tests.common import compare, make_inputs, run
 
@@ -34,3 +35,38 @@ def test_ragged_chunks_have_the_same_gradients_everywhere(dtype, l2, scalar):
     with torch.no_grad():
         forward = run(mk.chunk_delta_rule, {k: t for k, t in many_lv.items() if k != "h0"}, rep(do), rep(dht), many_opts, epi, grads=False)
     assert torch.equal(forward["o"], lone["o"]) and torch.equal(forward["ht"], lone["ht"])
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_rows_past_the_end_are_zero_whatever_the_others_hold(dtype, scalar):
+    """dq_v, dk_v and dgp leave as tiles of 64 rows, and a caller may add up whole tiles: rows past the end of a chunk are zero also where q, k or the states
+    are not finite.  One, some and no rows missing, in the first, a middle and the last block of 16, two v-heads per q/k head."""
+    from mogankda_b200 import ops
+    lens, HK, HV = (1, 15, 16, 31, 40, 63, 64), 2, 4
+    T, cu = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, _, opts, _ = make_inputs(T=T, HK=HK, HV=HV, cu=tuple(cu), dtype=dtype, gate="precomputed", scalar=scalar, epi=None, h0=False, seed=61)
+    lay = get_layout(1, T, opts["cu_seqlens"], lv["q"].device, 32)
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "precomputed", None, None, -5.0, HV, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    rq, rk = ops.l2norm_rstd(lv["q"]), ops.l2norm_rstd(lv["k"])
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], rq, rk, g_c, be, 128 ** -0.5, HK, HV, scalar_gate=scalar)
+    h, Vd, _, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV)
+    dh, dVd, dO, _ = ops.bwd_dh(lay, do, kbar, qs, gl, Aqk, nw, HK, HV)
+    last = torch.tensor(cu[1:], device="cuda") - 1
+
+    def at_last(t, x):
+        t = t.clone()
+        t[0, last, :, 5] = x
+        return t
+
+    def tile(t, x):          # one value of the high half of every state
+        t = t.clone()
+        t.view(torch.bfloat16).reshape(lay.NC, HV, -1)[..., 7] = x
+        return t
+
+    for x in (float("inf"), float("nan")):
+        for q, k, S, dS in ((lv["q"], at_last(lv["k"], x), h, dh), (at_last(lv["q"], x), lv["k"], h, dh), (lv["q"], lv["k"], tile(h, x), dh),
+                            (lv["q"], lv["k"], h, tile(dh, x))):
+            for t in ops.bwd_chunk(lay, q, k, lv["v"], rq, rk, g_c, be, A, S, dS, Vd, dO, dVd, 128 ** -0.5, HK, HV, lv["beta"], True, 2.0, scalar_gate=scalar)[:3]:
+                for c, n in enumerate(lay.chunk_len.tolist()):
+                    assert (t[c, :, n:] == 0).all(), (x, c, n)
