@@ -97,9 +97,10 @@ def test_state_and_transition_in_one_cta(lens, seg, vfirst, monkeypatch):
 
 @pytest.mark.parametrize("epi,scalar,dtype", [("silu", False, torch.float32), (None, False, torch.bfloat16), (None, True, torch.float16)])
 @pytest.mark.parametrize("T", [1, 64, 193])
-def test_a_chain_shared_by_two_ctas(T, epi, scalar, dtype):
-    """Up to half as many (sequence, head) chains as SMs: two CTAs share a chain, 64 rows of the transposed state each.  A sequence has the same bits
-    alone (shared) and among so many others that no chain is, states in and out in both layouts, forward only and with a backward pass."""
+def test_a_sequence_alone_and_among_many(T, epi, scalar, dtype):
+    """A sequence has the same bits alone (serial kernels by two CTAs per chain where they are separate ones, few items) and among so many others that no
+    chain is shared, states in and out in both layouts, forward only and with a backward pass; forward only without a state to start from, which
+    a continuation of at most 16 tokens would take to another kernel."""
     HV, N = 4, torch.cuda.get_device_properties(0).multi_processor_count // 8 + 1
     gate = "precomputed" if scalar else "eda"
     lv, do, dht, opts, epi = make_inputs(B=N, T=T, HK=2, HV=HV, dtype=dtype, gate=gate, scalar=scalar, epi=epi, seed=41)
@@ -109,3 +110,42 @@ def test_a_chain_shared_by_two_ctas(T, epi, scalar, dtype):
         one = run(mk.chunk_delta_rule, {k: first(t) for k, t in lv.items()}, first(do), first(dht), opts, epi, vfirst=vfirst)
         for k in ("o", "ht", "dq", "dk", "dv", "dg", "dbeta", "dh0"):
             assert torch.equal(many[k][:1], one[k]), k
+        lone = {k: t for k, t in lv.items() if k != "h0"}
+        with torch.no_grad():
+            many = run(mk.chunk_delta_rule, lone, do, dht, opts, epi, vfirst=vfirst, grads=False)
+            one = run(mk.chunk_delta_rule, {k: first(t) for k, t in lone.items()}, first(do), first(dht), opts, epi, vfirst=vfirst, grads=False)
+        for k in ("o", "ht"):
+            assert torch.equal(many[k][:1], one[k]), k
+
+
+@pytest.mark.parametrize("vfirst", [False, True])
+@pytest.mark.parametrize("lens", [(1,), (64, 0), (193, 65, 0, 128)])
+def test_a_chain_shared_by_two_ctas(lens, vfirst):
+    """recur_fwd and bwd_dh: up to half as many (sequence, head) chains as SMs, those of the transitions counted, are shared by two CTAs of 64 rows of the
+    transposed state each.  Every sequence, an empty one too, has the bits that it has among so many copies that no chain is shared: states, Vd, final
+    states and transitions (a state to start from keeps state and transition in CTAs of their own), and their reverses."""
+    from mogankda_b200 import ops
+    HV, N, sms = 4, len(lens), torch.cuda.get_device_properties(0).multi_processor_count
+    times = sms // (2 * HV * N) + 1
+    T, cu = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, dht, opts, _ = make_inputs(T=T, HK=HV, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi=None, seed=43)
+    assert 2 * 2 * HV * N <= sms < 2 * HV * N * times
+
+    def serial(copies, transition):
+        rep = lambda t, dim: torch.cat([t] * copies, dim)                                  # noqa: E731
+        many = torch.tensor([0] + [c + T * r for r in range(copies) for c in cu[1:]], dtype=torch.int32, device="cuda")
+        lay = get_layout(1, T * copies, many, lv["q"].device, 32)
+        q, k, v, g, b = (rep(lv[n], 1) for n in ("q", "k", "v", "g", "beta"))
+        g_c, be = ops.gate_cumsum_fwd(lay, g, "kimi", lv["A_log"], lv["dt_bias"], -5.0, HV, beta_raw=b, beta_sigmoid=True, beta_scale=2.0)
+        _, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, q, k, v, ops.l2norm_rstd(q), ops.l2norm_rstd(k), g_c, be, 128 ** -0.5, HV, HV)
+        h, Vd, ht, mt = ops.recur_fwd(lay, nw, u, kbar, gl, HV, HV, h0=rep(lv["h0"], 0), state_v_first=vfirst, want_transition=transition)
+        dh, dVd, _, dh0 = ops.bwd_dh(lay, rep(do, 1), kbar, qs, gl, Aqk, nw, HV, HV, dht=rep(dht, 0), state_v_first=vfirst)
+        _, _, _, short = ops.bwd_dh(lay, rep(do, 1), kbar, qs, gl, Aqk, nw, HV, HV, dht=rep(dht, 0), state_v_first=vfirst, store=False)
+        return dict(h=h, Vd=Vd, ht=ht, dh=dh, dVd=dVd, dh0=dh0, dh0_only=short, **(dict(mt=mt) if transition else {}))
+
+    for transition in (False, True):
+        shared, whole = serial(1, transition), serial(times, transition)
+        for k, t in shared.items():
+            assert torch.isfinite(t.view(torch.bfloat16) if k in ("h", "Vd", "dh", "dVd") else t).all(), k
+            for r in range(times):
+                assert torch.equal(whole[k][r * t.shape[0]:(r + 1) * t.shape[0]].view(torch.int32), t.view(torch.int32)), (k, r, transition)
