@@ -36,7 +36,8 @@
 // (Operands by token rows, as the forward kernel builds them: k, q and g requested twice, 2.5 k cycles each time, and 144 KB of operands in shared memory.)
 // dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
 // An item takes 23 k cycles (26 k before): 1B shape 223 -> 201 us, 64 k packed tokens x 32 heads 3.64 -> 3.29 ms, short documents 267 -> 250 us, fp16 4 x 1000
-// tokens 74 -> 66, scalar gate 4 x 16 k tokens x 16 heads 1313 -> 1249; with the hints below 193 us, 2.84 to 3.2 ms, 242 us, 63, 1210.
+// tokens 74 -> 66, scalar gate 4 x 16 k tokens x 16 heads 1313 -> 1249; with the hints of rows and the loads that leave L2 first 193 us, 3.23 ms, 242 us, 63,
+// 1210 (64 k tokens on other boxes, whose clocks differ: 2.84 to 3.12 ms).
 // Shared memory (KB): S [0,64) | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> weights [64,96), scratch in dW pieces | Vd^T [128,160) |
 // dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Qr; beta Kr].
 // TMEM columns: R_I 32 I; [D1; Z] 128, later C_I 128 + {0, 16, 48, 96}; dW 320, later Dq 320 and Dk 384, later column tiles 288 + {0, 16, 48, 96}; Db 448.
@@ -193,15 +194,18 @@ __device__ __forceinline__ void bwd_chunk_issue(const MkdaBwdChunk& p, uint8_t* 
     }
 }
 
+// Do the tiles of all items (272 KB each) take more than twice L2 (126 MB)?  What comes next is hinted into L2 then.
+__device__ __forceinline__ bool from_hbm(const MkdaLayout& L) { return (size_t)L.NC * L.HV > (256u << 20) / (272u << 10); }
+
 // Every tile is read here for the last time and may leave L2 at once, which keeps what comes next: the tiles that bwd_dh has written, and the gradients for
 // the kernels behind (1B shape 201 -> 193 us, fp16 4 x 1000 tokens 66 -> 63, short documents 248 -> 242, 64k packed tokens no difference).
 // S and Vd of the next item are requested once the state products and dgl of the current one are done, dO, dVd and A once the intra-chunk products
-// are, dS' once dVd and A have been read.
+// are (with a scalar gate, whose products leave the place of dVd and A alone, these two go with S and Vd), dS' once dVd and A have been read.
 template <bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     auto src = [](const void* t, size_t it, uint32_t bytes, uint32_t off = 0) { return static_cast<const uint8_t*>(t) + it * bytes + off; };
-    const bool from_hbm = (size_t)p.L.NC * p.L.HV > (256u << 20) / (272u << 10);          // twice L2 (126 MB)
+    const bool hints = from_hbm(p.L);
     auto request_s = [&](size_t it) {
         umma::mbar_expect_tx(&sh.fullS, umma::STATE_TILE_BYTES + 2 * umma::CHUNK_TILE_BYTES);
         umma::bulk_load_last(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
@@ -234,7 +238,7 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
         // Hints for what finds no room before the epilogue (3.47 -> 3.23 ms on 64k packed tokens x 32 heads, 1315 -> 1250 us on 4 x 16k x 16 heads with a
         // scalar gate, when all of the item's tiles waited for it).  Not where the tiles of all items come close to fitting into L2 as they are: 512
         // items lose 3 % by it.
-        if (from_hbm) {
+        if (hints) {
             umma::mbar_wait(&sh.mmL, n & 1);
             umma::l2_prefetch(src(p.dVd_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
             umma::l2_prefetch(src(p.A, in, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES);
@@ -247,12 +251,13 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
     }
 }
 
-// Tables and per-row scalars of an item: requested two items ahead of their use, written once the item in front has passed its state products.
+// Tables and per-row scalars of item n: requested in the middle of item n - 2, written in the middle of item n - 1 to the place of those of item n - 2, which
+// everyone is done with by then.
 template <int DT, bool SCALAR, bool SPREAD>
 __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared& sh, int lane) {
     using namespace bc;
     constexpr uint32_t ROW = DT == MKDA_F32 ? 512 : 256;
-    const bool from_hbm = (size_t)p.L.NC * p.L.HV > (256u << 20) / (272u << 10);          // as for the tiles
+    const bool hints = from_hbm(p.L);
     uint32_t n = 0;
     for (ItemWalk<SPREAD> w(p.L); w.valid(); w.next(), ++n) {
         const int start = p.L.chunk_start[w.chunk()], len = p.L.chunk_len[w.chunk()], h = w.head(), hk = w.hk();
@@ -282,7 +287,7 @@ __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared
         __syncwarp();
         if (lane == 0) umma::arrive(&sh.rows[n & 1]);
         __syncwarp();
-        if (from_hbm) {                                    // the rows of v, g, k and q start on their way into L2
+        if (hints) {                                       // the rows of v, g, k and q start on their way into L2
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const int i = lane + 32 * m;

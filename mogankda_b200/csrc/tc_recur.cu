@@ -1,7 +1,8 @@
 // Serial state recurrences on the Blackwell tensor cores.
 //
 // One CTA per (v-head, segment) carries the whole 128 x 128 state, TRANSPOSED: accumulator lane = v, columns = K index.  The fp32 state
-// lives in the registers of 512 compute threads (thread = one lane x 32 columns); each step it is split into packed bf16 hi / lo pairs in
+// lives in the registers of 512 compute threads (thread = one lane x 32 columns); with few chains recur_fwd and bwd_dh take two CTAs of 64 rows
+// and 256 working compute threads each (split_chains).  Each step the state is split into packed bf16 hi / lo pairs in
 // tensor memory, where the products take it as their left operand, and the products' result comes back from an fp32 accumulator:
 //   forward   D^T = u^T + S^T nw^T = Vd^T        S^T <- S^T diag(gl) + Vd^T kbar
 //   reverse   D^T = dO^T Aqk + dS^T kbar^T = dVd^T      dS^T <- dS^T diag(gl) + dO^T (scale q 2^g) + dVd^T nw
@@ -476,9 +477,11 @@ __global__ void __launch_bounds__(RecurLayout<true>::THREADS, 1) chain_fwd_tc_ke
     recur_body<OUT, NORM, false>(p.r, seg_order, p.o, maps);
 }
 // Rows of the transposed state (v) never meet: S^T nw, Vd^T kbar and their reverses contract over K and over tokens.  So with at most half as many
-// chains as SMs a chain is shared between two CTAs of 64 rows each, with the same bits: a step is bound by what one SM moves (192 or 240 KB at 35 B per
-// cycle, half of it the saved states and Vd), and that is 112 or 128 KB then.  recur_fwd 45 steps x 48 chains 131 -> 99 us, 16 x 32 48.5 -> 37.5, 4 x 4
-// 15.2 -> 11.9; bwd_dh 150 -> 113, 56 -> 43, 15.7 -> 12.2, 256 x 64 894 -> 702.  (chain_fwd gained nothing: 256 x 64 996, 32 x 64 95 us.)
+// chains as SMs a chain is shared between two CTAs of 64 rows each, with the same bits.  Per step and SM a forward CTA moves 128 KB then
+// instead of 192 (nw and kbar whole, u, h and Vd by halves) in 4.0 instead of 5.5 k cycles, a reverse one 176 instead of 240 KB (nw, kbar, qs, Aqk whole,
+// dO, dh and dVd by halves) in 4.6 instead of 6.9 k: 33 to 39 B per cycle all four.  recur_fwd 45 steps x 48 chains 131 -> 99 us, 16 x 32 48.5 -> 37.5, 4 x 4
+// 15.2 -> 11.9; bwd_dh 150 -> 113, 56 -> 43, 15.7 -> 12.2, 256 x 64 894 -> 702.  (chain_fwd, with its single buffers kept, gained nothing: 256 x 64
+// 996 us, 32 x 64 95; what its step waits for has not been shown.)
 static bool split_chains(long long chains) { return 2 * chains <= sm_count(); }
 
 // ---------------------------------------------------------------------------------------------------------
