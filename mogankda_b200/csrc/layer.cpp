@@ -69,9 +69,12 @@ bool spread_v_heads(const Call& c) {
 
 // Output in the kernel of the state chain, or in one of its own?  In units of 1000 SM cycles per chunk: a chain step takes 6
 // without the output; with it 8.5 (a backward pass follows) or 6.5, and 12 or 9 when the gated norm is fused; a kernel of its own takes 7
-// (11 with the norm) per chunk and SM and 6 to launch, and has all SMs.  (Measured when the output's products stood in front of the chain's also
-// without a norm; such a step takes 7.2 or 4.7 now, and the line has not been taken again.)  So the separate kernel is the better one where a few long
+// (11 with the norm) per chunk and SM and 6 to launch, and has all SMs.  So the separate kernel is the better one where a few long
 // chains leave SMs idle: fp16 4 x 1000 tokens x 8 heads 75 instead of 96 us, 64k packed tokens x 32 heads 2260 instead of 1770 us.
+// These units are older than the kernels: a step takes 7.2 or 4.7 without a norm, where the output's products stand behind the chain's, and 4.0 by itself
+// where two CTAs share the chain.  Over 1, 2, 4 ... 64 steps x 4 to 128 chains, with and without norm and backward pass, the line takes the fused kernel 19
+// times in 280 where the separate ones are faster, by 1 to 21 % and between 4 and 72 chains (norm, forward only: 8 steps x 32 chains 37.9 us against 31.4,
+// 64 x 48 268 against 241), and never the other way round.
 bool output_in_chain(const Call& c, bool need_bwd) {
     const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     const double share = (double)c.NC * c.HV / sms, steps = std::max((double)c.chain, share);

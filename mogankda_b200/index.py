@@ -95,9 +95,11 @@ def wants_segments(chunks_per_seq, HV, seg_chunks, sm_count=None, cost_ratio=2.5
     combine.  So: cut when the critical path is longer than 2.5 even shares (``cost_ratio``; 1.25 when the caller allows
     warm-up truncation, which shortens the two extra passes to a few chunks wherever the gate decays).  With few chains the four passes of a
     cut call take a segment each however small the share is, so sequences of up to 1.85 segments (1.2 where truncation is allowed) are left alone.
-    Uncut / cut, one sequence x 4 to 32 heads: training 0.93 to 0.99 of the time at 54 chunks, 0.98 to 1.03 at 58, 1.02 to 1.07 at 62; forward only 0.90 to 1.04
-    at 54, 0.94 to 1.11 at 58, 0.98 to 1.16 at 62 (few heads gain most by the cut); with truncation 0.94 to 0.98 at 37, 1.00 to 1.04 at 40.
-    45 + 42 + 42 chunks x 16 heads took 415 us in the serial kernels and combines when cut, 280 uncut.  Decided from the
+    The line is older than chains shared by two CTAs, by which uncut calls gained most.  Time uncut / cut now, one sequence x 4, 8, 16, 32, 48 heads: training
+    0.90 0.92 0.93 0.94 0.89 at 58 chunks, 0.95 0.96 0.96 0.95 0.92 at 62, 1.03 1.02 1.00 0.92 0.91 at 72, 1.20 1.17 1.11 1.01 0.96 at 90, 1.68 1.51 1.27 0.92
+    0.98 at 160; forward only 0.91 0.92 0.93 0.95 1.02 at 58, 0.94 0.95 0.96 0.98 1.05 at 62, 1.03 1.03 1.01 1.00 1.10 at 72, 1.71 1.48 1.43 1.04 1.18 at 160;
+    with truncation at 40 chunks 1.03 1.02 1.02 1.00 0.91 and 1.02 1.02 1.02 0.93 1.04.  So up to 70 chunks, and in training with 32 heads and more also
+    beyond, the cut costs up to 13 %.  Decided from the
     lengths alone (host), never from data; it plays the role of the reference's intra-card CP decision
     (mogan_kda/ops/gated_delta_rule/chunk/cp/context.py:252-283, cp/autocp/decision.py:54-123)."""
     longest = max(chunks_per_seq, default=0)
