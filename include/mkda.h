@@ -124,6 +124,9 @@ typedef struct {
 int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream);
 /* The same without A, which only a backward pass reads (the field is not looked at). */
 int mkda_intra_fwd_forward_only(const MkdaIntraFwd* p, void* stream);
+/* mkda_gate_cumsum_fwd and mkda_intra_fwd in one kernel, for at most as many (chunk, v-head) pairs as the device has SMs.  Of `p`, the fields g_c and beta are not looked at, of `g` the field L; beta_raw is needed.
+ * g->g_c, g->beta_out and p->A are what a backward pass reads: each may be NULL and is then not written. */
+int mkda_gate_intra_fwd(const MkdaGateFwd* g, const MkdaIntraFwd* p, void* stream);
 
 /* State tile: how the per-chunk states `h` (state entering a chunk) and `dh` (gradient of the state leaving it) travel
  * between the kernels.  One tile per (chunk, v-head), MKDA_STATE_TILE_BYTES each, is the tensor-core operand itself: the

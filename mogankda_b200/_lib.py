@@ -16,7 +16,8 @@ ENTRY_POINTS = (
     "mkda_recur_fwd", "mkda_out_fwd", "mkda_epilogue_bwd", "mkda_epilogue_bwd_tiles", "mkda_bwd_dh", "mkda_bwd_chunk",
     "mkda_qk_grad_finish", "mkda_state_combine", "mkda_warmup_chunks", "mkda_selftest_umma", "mkda_selftest_wait", "mkda_epilogue_bwd_noalloc",
 )
-ORDERED_ENTRY_POINTS = ("mkda_recur_fwd_ordered", "mkda_chain_fwd_ordered", "mkda_bwd_dh_ordered")      # with the order of the segments
+# with a third argument: the order of the segments, the second struct
+ORDERED_ENTRY_POINTS = ("mkda_recur_fwd_ordered", "mkda_chain_fwd_ordered", "mkda_bwd_dh_ordered", "mkda_gate_intra_fwd")
 ENUMS = {}
 STRUCTS = {}
 

@@ -14,10 +14,28 @@ static int intra_fwd(const MkdaIntraFwd* given, bool forward_only, void* stream)
         return set_error(MKDA_ERR_ARG, "intra_fwd: tensors must be 16-byte aligned");
     if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "intra_fwd: HV must be a multiple of HK");
     if (p->L.NC == 0) return MKDA_OK;
-    return launch_intra_fwd_tc(p, (cudaStream_t)stream);
+    return launch_intra_fwd_tc(p, nullptr, (cudaStream_t)stream);
 }
 extern "C" int mkda_intra_fwd(const MkdaIntraFwd* p, void* stream) { return intra_fwd(p, false, stream); }
 extern "C" int mkda_intra_fwd_forward_only(const MkdaIntraFwd* p, void* stream) { return intra_fwd(p, true, stream); }
+
+extern "C" int mkda_gate_intra_fwd(const MkdaGateFwd* g, const MkdaIntraFwd* p, void* stream) {
+    if (!g || !p || !g->x || !g->beta_raw || !p->q || !p->k || !p->v || !p->Aqk || !p->nw || !p->u || !p->kbar || !p->qs || !p->gl)
+        return set_error(MKDA_ERR_ARG, "gate_intra_fwd: null argument");
+    if (any_misaligned(p->q, p->k, p->v, p->A, p->Aqk, p->nw, p->u, p->kbar, p->qs, p->gl) ||
+        (!p->scalar_gate && any_misaligned(g->x, g->dt_bias, g->g_c)))
+        return set_error(MKDA_ERR_ARG, "gate_intra_fwd: tensors must be 16-byte aligned");
+    if (g->scalar_gate != p->scalar_gate) return set_error(MKDA_ERR_ARG, "gate_intra_fwd: one decay per token, or one per channel?");
+    if (g->mode != MKDA_GATE_PRECOMPUTED && !(g->lower_bound < 0.f)) return set_error(MKDA_ERR_ARG, "gate_intra_fwd: lower_bound must be < 0");
+    for (int dt : {g->x_dtype, g->beta_dtype})
+        if (dt < MKDA_F32 || dt > MKDA_F16) return set_error(MKDA_ERR_ARG, "gate_intra_fwd: unsupported dtype");
+    if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "gate_intra_fwd: HV must be a multiple of HK");
+    if (p->L.NC == 0) return MKDA_OK;
+    if ((long long)p->L.NC * p->L.HV > sm_count()) return set_error(MKDA_ERR_ARG, "gate_intra_fwd: more (chunk, v-head) pairs than SMs");
+    MkdaGateFwd gate = *g;
+    gate.L = p->L;
+    return launch_intra_fwd_tc(p, &gate, (cudaStream_t)stream);
+}
 
 extern "C" int mkda_recur_fwd_ordered(const MkdaRecurFwd* p, const int* seg_order, void* stream) {
     if (!p || !p->nw || !p->u || !p->kbar || !p->gl) return set_error(MKDA_ERR_ARG, "recur_fwd: null argument");

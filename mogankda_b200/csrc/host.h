@@ -54,7 +54,7 @@ int launch_chain_fwd_tc(const MkdaChainFwd* p, const int* seg_order, cudaStream_
 int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stream);
 int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();
-int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream);
+int launch_intra_fwd_tc(const MkdaIntraFwd* p, const MkdaGateFwd* gate, cudaStream_t stream);      // gate: formed there, or NULL
 int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream);
 int tc_bwd_chunk_status(unsigned int* out);
 int tc_bwd_chunk_status_clear();

@@ -67,6 +67,11 @@ bool spread_v_heads(const Call& c) {
     return groups <= 2 * sms && (groups * G + sms - 1) / sms < G * ((groups + sms - 1) / sms);
 }
 
+// The gate in intra_fwd where that has at most one item per SM: a kernel and its cold start less (77 tokens x 16 heads 28.5 -> 26.1 us, 5.1 + 13.2 us of
+// kernels -> 15.9).  With more items its work is not free, neither in intra_fwd's own warps nor in warps beside them, an item ahead: 3.5 items per SM 54 us against
+// 40 + 8, 24 items 258 against 189 + 38.
+bool gate_in_intra(const Call& c) { return (int64_t)c.NC * c.HV <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
+
 // Output in the kernel of the state chain, or in one of its own?  In units of 1000 SM cycles per chunk: a chain step takes 6
 // without the output; with it 8.5 (a backward pass follows) or 6.5, and 12 or 9 when the gated norm is fused; a kernel of its own takes 7
 // (11 with the norm) per chunk and SM and 6 to launch, and has all SMs.  So the separate kernel is the better one where a few long
@@ -123,8 +128,11 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
         keep.want(&s.q_rstd, (int64_t)c.TT * c.HK * 4);
         keep.want(&s.k_rstd, (int64_t)c.TT * c.HK * 4);
     }
-    keep.want(&s.g_c, c.scalar_gate ? row / 128 : row);
-    keep.want(&s.beta_e, (int64_t)c.TT * c.HV * 4);
+    const bool one_kernel = gate_in_intra(c);
+    if (need_bwd || !one_kernel) {
+        keep.want(&s.g_c, c.scalar_gate ? row / 128 : row);
+        keep.want(&s.beta_e, (int64_t)c.TT * c.HV * 4);
+    }
     if (need_bwd) keep.want(&s.A, c.tiles(MKDA_QUARTER_TILE_BYTES));
     keep.want(&s.Aqk, c.tiles(MKDA_QUARTER_TILE_BYTES));
     keep.want(&s.nw, c.tiles(MKDA_CHUNK_TILE_BYTES));
@@ -153,20 +161,22 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     const int* order = segment_order(c);
 
     {
-        MkdaGateFwd p{};
-        p.L = L; p.x = in.x.data_ptr(); p.x_dtype = dtype_code(in.x); p.scalar_gate = c.scalar_gate;
-        p.A_log = fptr(alog); p.dt_bias = fptr(bias); p.mode = c.mode; p.lower_bound = c.lower_bound;
-        p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta); p.beta_sigmoid = c.beta_sigmoid;
-        p.beta_scale = c.beta_scale; p.beta_out = s.beta_e; p.g_c = s.g_c;
-        check_rc(mkda_gate_cumsum_fwd(&p, st), "mkda_gate_cumsum_fwd");
-    }
-    {
+        MkdaGateFwd g{};
+        g.L = L; g.x = in.x.data_ptr(); g.x_dtype = dtype_code(in.x); g.scalar_gate = c.scalar_gate;
+        g.A_log = fptr(alog); g.dt_bias = fptr(bias); g.mode = c.mode; g.lower_bound = c.lower_bound;
+        g.beta_raw = in.beta.data_ptr(); g.beta_dtype = dtype_code(in.beta); g.beta_sigmoid = c.beta_sigmoid;
+        g.beta_scale = c.beta_scale; g.beta_out = s.beta_e; g.g_c = s.g_c;
         MkdaIntraFwd p{};
         p.L = L; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
         p.g_c = s.g_c; p.beta = s.beta_e; p.scalar_gate = c.scalar_gate; p.scale = c.scale;
         p.l2 = c.l2; p.l2_eps = 1e-6f; p.q_rstd_out = s.q_rstd; p.k_rstd_out = s.k_rstd;
         p.A = s.A; p.Aqk = s.Aqk; p.nw = s.nw; p.u = u; p.kbar = s.kbar; p.qs = s.qs; p.gl = s.gl;
-        check_rc(need_bwd ? mkda_intra_fwd(&p, st) : mkda_intra_fwd_forward_only(&p, st), "mkda_intra_fwd");
+        if (one_kernel) {
+            check_rc(mkda_gate_intra_fwd(&g, &p, st), "mkda_gate_intra_fwd");
+        } else {
+            check_rc(mkda_gate_cumsum_fwd(&g, st), "mkda_gate_cumsum_fwd");
+            check_rc(need_bwd ? mkda_intra_fwd(&p, st) : mkda_intra_fwd_forward_only(&p, st), "mkda_intra_fwd");
+        }
     }
     Tensor ht;
     if (c.want_ht) ht = c.states(c.N);

@@ -25,10 +25,12 @@
 // dh0 1.03 times as far from fp64 (geometric mean of 90 bf16 layers; 1.4 at worst), fp32 gradients 1.08, final states 1.2.
 // An item takes 16 k cycles, all of them X's (rows 3 k, operands 5 k, L2 statistics 1.5 k, nw and u 2.9 k, tiles 3 k), 11 k of them Y's; 12 k with a scalar gate, Y's.
 // 6 k packed tokens x 32 heads 240 -> 190 us, 32 k tokens x 32 heads 1121 -> 860, scalar gate 4 x 2000 tokens x 16 heads 129 -> 99.
+#include "gate.cuh"
 #include "host.h"
 #include "intra.cuh"
 
 #include <string.h>
+#include <type_traits>
 
 namespace mkda {
 
@@ -78,7 +80,13 @@ struct Shared {
 constexpr int SMEM = TILES + (int)sizeof(Shared);
 static_assert(SMEM <= 232448, "shared memory of one CTA");
 
-struct Maps { CUtensorMap k, q, g, v; };
+struct Maps { CUtensorMap k, q, g, v; };                    // g: the cumsum, or the raw gate of a kernel that forms it
+
+// G = MkdaGateFwd: the gate is formed here too, for calls of at most one item per CTA (then a compile-time fact): X waits for its rows anyway, and 2.7 us of
+// its time replace a kernel of 5.1 us (77 tokens x 16 heads).
+struct NoGate {};
+template <class G> constexpr bool GATED = std::is_same<G, MkdaGateFwd>::value;
+constexpr int RAW_X = BK;                                   // raw gate of the item, fp32 or 16 bits: nothing else is there yet
 
 __device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 __device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
@@ -108,7 +116,8 @@ struct Walk {
         table();
     }
 };
-__device__ __forceinline__ int item_count(const MkdaLayout& L) { return (L.NC * L.HV - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x; }
+template <bool ONE>
+__device__ __forceinline__ int item_count(const MkdaLayout& L) { return ONE ? 1 : (L.NC * L.HV - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x; }
 
 // eight consecutive floats by the threads c = 0..7 of a row: the two 16-byte halves in an order that keeps the eight off each other's banks
 __device__ __forceinline__ void lds8_swapped(const float* p, bool s, f32x2 (&v)[4]) {
@@ -124,6 +133,54 @@ __device__ __forceinline__ void lds_raw8(const uint8_t* row, int k8, Raw8& r) {
         r.a = *reinterpret_cast<const uint4*>(row + k8 * 16);
     }
 }
+
+// ---- the gate and its chunk-local inclusive cumsum (log2), summed in the same order as by the kernels that do nothing else (prologue.cu) ----
+// One decay per token, by one warp: the raw values of rows 2 l and 2 l + 1 in, their cumsum out (the last valid one past the end).  Groups of eight rows,
+// then the groups in order.
+__device__ __forceinline__ void scalar_cumsum(const MkdaGateFwd& p, int h, int len, float& a, float& b, int lane) {
+    const float E = p.A_log ? expf(p.A_log[h]) : 1.f, bias = p.dt_bias ? p.dt_bias[h] : 0.f;
+    a = 2 * lane < len ? gate_value(p.mode, a + bias, E, p.lower_bound) : 0.f;
+    const float v = 2 * lane + 1 < len ? gate_value(p.mode, b + bias, E, p.lower_bound) : 0.f;
+    b = __fadd_rn(a, v);
+#pragma unroll
+    for (int j = 1; j < 4; ++j) {
+        const float t = __shfl_up_sync(0xffffffffu, b, 1);
+        if ((lane & 3) == j) { a = __fadd_rn(t, a); b = __fadd_rn(a, v); }
+    }
+    float pre = 0.f;
+#pragma unroll
+    for (int w = 0; w < 7; ++w) {
+        const float t = __shfl_sync(0xffffffffu, b, 4 * w + 3);
+        if (w < (lane >> 2)) pre += t;
+    }
+    a = (pre + a) * RCP_LN2;
+    b = (pre + b) * RCP_LN2;
+}
+// One decay per channel, by X: thread = 16 rows of a channel, four at a time: all of it is fetched cold, once, so short code is fast code.
+// `raw` -> `rows`, both [64][128]; E and the bias were requested before the rows were waited for.
+__device__ __forceinline__ void channel_cumsum(const MkdaGateFwd& p, const uint8_t* raw, float* rows, float (&tot)[5][DK], size_t first, int len, float E, float bias) {
+    const int ch = threadIdx.x & 127, b = threadIdx.x >> 7;
+    float run = 0.f, pre = 0.f;
+#pragma unroll 1
+    for (int r = 16 * b; r < 16 * b + 16; r += 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float g = gate_value(p.mode, ld1(raw, p.x_dtype, (r + i) * 128 + ch) + bias, E, p.lower_bound);
+            if (r + i < len) run = __fadd_rn(run, g);      // not contracted with the gate's last product
+            rows[(r + i) * 128 + ch] = run;
+        }
+    }
+    tot[b][ch] = run;
+    sync_x();
+    for (int w = 0; w < b; ++w) pre += tot[w][ch];
+#pragma unroll 4
+    for (int r = 16 * b; r < 16 * b + 16; ++r) {
+        const float g = (pre + rows[r * 128 + ch]) * RCP_LN2;
+        rows[r * 128 + ch] = g;
+        if (p.g_c && r < len) p.g_c[first + (size_t)r * p.L.HV * 128] = g;
+    }
+    sync_x();
+}
 }  // namespace in
 
 // ---- X ----------------------------------------------------------------------------------------------------------------------------------
@@ -133,8 +190,8 @@ __device__ __forceinline__ void lds_raw8(const uint8_t* row, int k8, Raw8& r) {
 // over channels, Gamma_ij = (k_i . k_j) 2^(g_i - g_j), so the products are plain K K^T / Q K^T (one product over a stacked
 // [K; Q] tile; bf16 rows have no low half) and the decay is applied to the accumulators, element by element and for i >= j only: nothing is
 // anchored, no exponent is ever positive, and any g <= 0 is in range (the per-channel path needs g >= -5 per token).
-template <int DT, bool SCALAR>
-__device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, uint32_t tmem, in::Shared& sh) {
+template <int DT, bool SCALAR, class G>
+__device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, uint8_t* base, uint32_t tmem, in::Shared& sh) {
     using namespace in;
     using R = Rows<DT, SCALAR>;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c8 = tid & 7;
@@ -162,14 +219,24 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
         stage(U, base + UT, 1.f);
         umma::signal(&sh.uReady, lane);
     };
-    const int count = item_count(p.L);
+    const int count = item_count<GATED<G>>(p.L);
     for (int it = 0; it < count; ++it) {
         const uint32_t par = it & 1;
         float* beta = sh.beta[par];
         float* gs = &sh.ga[0][0] + par * CH;                // SCALAR: the cumsum of every row, two items (rows past the end: the last valid one)
         // ---- this item's rows into registers; park the anchor rows of g ----
+        float E = 1.f, bias = 0.f, raw0 = 0.f, raw1 = 0.f;   // of a gate that is formed here, and beta or a scalar gate before it is
+        if constexpr (GATED<G> && !SCALAR) {
+            const int h = blockIdx.x % p.L.HV;
+            if (gate.A_log) E = expf(gate.A_log[h]);
+            if (gate.dt_bias) bias = gate.dt_bias[h * 128 + (tid & 127)];
+        }
         umma::mbar_wait(&sh.ldin, par);
         const int len = sh.info[it & 3].len;
+        if constexpr (GATED<G> && !SCALAR) {
+            const size_t first = ((size_t)sh.info[0].start * p.L.HV + sh.info[0].h) * 128 + (tid & 127);
+            channel_cumsum(gate, base + RAW_X, reinterpret_cast<float*>(base + RAW_G), sh.ga, first, len, E, bias);
+        }
         Raw8 wk[2], wq[2];
         f32x2 vg[2][4];
 #pragma unroll
@@ -199,8 +266,18 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
         {   // beta (and a scalar gate's cumsum), used once the products are done
             const size_t HV = p.L.HV;
             const int i = sh.info[it & 3].start + min(tid & (CH - 1), len - 1), h = sh.info[it & 3].h;
-            if (tid < CH) cp_async4(&beta[tid], p.beta + i * HV + h);
-            else if (SCALAR && tid < 2 * CH) cp_async4(gs + tid - CH, p.g_c + i * HV + h);
+            if constexpr (GATED<G>) {
+                if (tid < CH) {
+                    raw0 = ld1(gate.beta_raw, gate.beta_dtype, i * HV + h);
+                } else if (SCALAR && warp == 2) {           // two rows per lane
+                    const size_t first = (size_t)sh.info[it & 3].start * HV + h;
+                    raw0 = ld1(gate.x, gate.x_dtype, first + min(2 * lane, len - 1) * HV);
+                    raw1 = ld1(gate.x, gate.x_dtype, first + min(2 * lane + 1, len - 1) * HV);
+                }
+            } else {
+                if (tid < CH) cp_async4(&beta[tid], p.beta + i * HV + h);
+                else if (SCALAR && tid < 2 * CH) cp_async4(gs + tid - CH, p.g_c + i * HV + h);
+            }
         }
         umma::fence_before_sync();
         sync_x();
@@ -292,8 +369,22 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, uint8_t* base, ui
             const int i = tid & (CH - 1), x = tid >> 6;
             sh.rs[x][i] = p.k_rstd ? (x ? p.q_rstd : p.k_rstd)[(size_t)(sh.info[it & 3].start + min(i, len - 1)) * p.L.HK + sh.info[it & 3].hk] : 1.f;
         }
-        cp_async_wait_all();
-        if (tid < CH && tid >= len) beta[tid] = 0.f;
+        if constexpr (GATED<G>) {
+            const size_t HV = p.L.HV, first = (size_t)sh.info[it & 3].start * HV + sh.info[it & 3].h;
+            if (tid < CH) {
+                const float b = gate.beta_sigmoid ? gate.beta_scale * sigmoidf_(raw0) : raw0;
+                beta[tid] = tid < len ? b : 0.f;
+                if (gate.beta_out && tid < len) gate.beta_out[first + tid * HV] = b;
+            } else if (SCALAR && warp == 2) {
+                scalar_cumsum(gate, sh.info[it & 3].h, len, raw0, raw1, lane);
+                *reinterpret_cast<float2*>(gs + 2 * lane) = make_float2(raw0, raw1);
+                if (gate.g_c && 2 * lane < len) gate.g_c[first + 2 * lane * HV] = raw0;
+                if (gate.g_c && 2 * lane + 1 < len) gate.g_c[first + (2 * lane + 1) * HV] = raw1;
+            }
+        } else {
+            cp_async_wait_all();
+            if (tid < CH && tid >= len) beta[tid] = 0.f;
+        }
         __syncwarp();
         if (lane == 0) umma::arrive(&sh.rows);
         if (it) read_out(it - 1);
@@ -397,14 +488,14 @@ __device__ __forceinline__ void invert_unit_lower(float* M, float* T, uint64_t* 
     product(M + 2 * MB, T, M + MB, -1.f);
 }
 
-template <int DT, bool SCALAR>
+template <int DT, bool SCALAR, bool ONE>
 __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, uint32_t tmem, in::Shared& sh) {
     using namespace in;
     constexpr int YT = 32 * Y_WARPS;
     const int tid = threadIdx.x & (YT - 1), warp = threadIdx.x >> 5, lane = tid & 31, q = warp & 3;
     const size_t HV = p.L.HV;
     float* M = reinterpret_cast<float*>(base + M_);
-    const int count = item_count(p.L);
+    const int count = item_count<ONE>(p.L);
     for (int it = 0; it < count; ++it) {
         const uint32_t par = it & 1;
         const float* beta = sh.beta[par];
@@ -530,10 +621,10 @@ __device__ __forceinline__ uint8_t* fresh(uint8_t* smem) {
     asm volatile("" : "+l"(smem));
     return smem;
 }
-template <int DT, bool SCALAR>
+template <int DT, bool SCALAR, bool ONE>
 __device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, uint32_t tmem, in::Shared& sh) {
     using namespace in;
-    const int count = item_count(p.L);
+    const int count = item_count<ONE>(p.L);
     for (int it = 0; it < count; ++it) {
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
@@ -554,9 +645,10 @@ __device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, 
         umma::commit(&sh.mm1[it & 1]);
     }
 }
+template <bool ONE>
 __device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, uint32_t tmem, in::Shared& sh) {
     using namespace in;
-    const int count = item_count(p.L);
+    const int count = item_count<ONE>(p.L);
     for (int it = 0; it < count; ++it) {
         const uint32_t par = it & 1;
         umma::wait_mma(&sh.hand, par);                      // beta k 2^g
@@ -585,26 +677,28 @@ template <int DT, bool SCALAR>
 __device__ __forceinline__ void request_q(const in::Walk& w, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     umma::tma_load_rows(base + in::Rows<DT, SCALAR>::Q, &maps.q, w.hk * 128, w.start, &sh.ldin);
 }
-template <int DT, bool SCALAR>
-__device__ __forceinline__ void request_rows(const in::Walk& w, int it, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+template <int DT, bool SCALAR, class G>
+__device__ __forceinline__ void request_rows(const G& gate, const in::Walk& w, int it, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     using R = in::Rows<DT, SCALAR>;
     auto& i = sh.info[it & 3];
     i.item = w.item(); i.start = w.start; i.len = w.len; i.h = w.h; i.hk = w.hk;
-    umma::mbar_expect_tx(&sh.ldin, 2 * R::BYTES + (SCALAR ? 0u : 32768u));
-    if (!SCALAR) umma::tma_load_rows(base + in::RAW_G, &maps.g, w.h * 128, w.start, &sh.ldin);
+    uint32_t g_bytes = SCALAR ? 0u : 32768u;
+    if constexpr (in::GATED<G> && !SCALAR) g_bytes = gate.x_dtype == MKDA_F32 ? 32768u : 16384u;
+    umma::mbar_expect_tx(&sh.ldin, 2 * R::BYTES + g_bytes);
+    if (!SCALAR) umma::tma_load_rows(base + (in::GATED<G> ? in::RAW_X : in::RAW_G), &maps.g, w.h * 128, w.start, &sh.ldin);
     umma::tma_load_rows(base + R::K, &maps.k, w.hk * 128, w.start, &sh.ldin);
     if (!R::LATE_Q) request_q<DT, SCALAR>(w, maps, base, sh);
 }
-template <int DT, bool SCALAR>
-__device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
+template <int DT, bool SCALAR, class G>
+__device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const G& gate, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     using namespace in;
     using R = Rows<DT, SCALAR>;
     Walk w(p.L);                                            // the first item's rows are on their way
     for (int it = 0; w.valid(); ++it) {
         const size_t item = w.item();
-        w.next();
+        if (GATED<G>) w.c = w.NC; else w.next();
         umma::mbar_wait(&sh.mm1[it & 1], (it >> 1) & 1);    // the operands are dead
-        if (w.valid()) request_rows<DT, SCALAR>(w, it + 1, maps, base, sh);
+        if (w.valid()) request_rows<DT, SCALAR>(gate, w, it + 1, maps, base, sh);
         umma::mbar_wait(&sh.acc, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + item * umma::QUARTER_TILE_BYTES, base + AQ, umma::QUARTER_TILE_BYTES);
         umma::mbar_wait(&sh.hand, it & 1);
@@ -615,7 +709,7 @@ __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const in::Ma
         if (R::LATE_Q && w.valid()) request_q<DT, SCALAR>(w, maps, base, sh);
     }
 }
-template <int DT>
+template <int DT, bool ONE>
 __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Maps& maps, uint8_t* base, in::Shared& sh) {
     using namespace in;
     auto load_v = [&](const Walk& w) {                      // two boxes of 64 channels: rows in the layout of an operand tile
@@ -628,7 +722,7 @@ __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Ma
     load_v(w);
     for (uint32_t it = 0; w.valid(); ++it) {
         const size_t item = w.item();
-        w.next();
+        if (ONE) w.c = w.NC; else w.next();
         umma::mbar_wait(&sh.nwReady, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + item * umma::CHUNK_TILE_BYTES, base + BK, umma::CHUNK_TILE_BYTES);
         umma::mbar_wait(&sh.uReady, it & 1);
@@ -641,9 +735,10 @@ __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Ma
     }
 }
 
-template <int DT, bool SCALAR>
-__global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const __grid_constant__ in::Maps maps) {
+template <int DT, bool SCALAR, class G>
+__global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const MkdaIntraFwd p, const G gate, const __grid_constant__ in::Maps maps) {
     using namespace in;
+    constexpr bool ONE = GATED<G>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
     Shared& sh = *reinterpret_cast<Shared*>(base + TILES);
@@ -668,7 +763,7 @@ __global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const Mkda
             umma::fence_barrier_init();
             follow_stream();
             const Walk w(p.L);
-            request_rows<DT, SCALAR>(w, 0, maps, base, sh);
+            request_rows<DT, SCALAR>(gate, w, 0, maps, base, sh);
             if (Rows<DT, SCALAR>::LATE_Q) request_q<DT, SCALAR>(w, maps, base, sh);
         }
         __syncwarp();
@@ -680,17 +775,17 @@ __global__ void __launch_bounds__(in::THREADS, 1) intra_fwd_tc_kernel(const Mkda
     follow_stream();
     if (warp < X_WARPS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(X_REGS));
-        intra_x<DT, SCALAR>(p, base, tmem, sh);
+        intra_x<DT, SCALAR>(p, gate, base, tmem, sh);
     } else if (warp < X_WARPS + Y_WARPS) {
-        intra_y<DT, SCALAR>(p, base, tmem, sh);
+        intra_y<DT, SCALAR, ONE>(p, base, tmem, sh);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(ISSUE_REGS));
         if (umma::elect_one()) {
             switch (warp - X_WARPS - Y_WARPS) {
-                case 0: intra_mm1<DT, SCALAR>(p, base, tmem, sh); break;
-                case COPY_X: intra_copy_x<DT, SCALAR>(p, maps, base, sh); break;
-                case 2: intra_copy_y<DT>(p, maps, base, sh); break;
-                default: intra_mm3(p, base, tmem, sh);
+                case 0: intra_mm1<DT, SCALAR, ONE>(p, base, tmem, sh); break;
+                case COPY_X: intra_copy_x<DT, SCALAR>(p, gate, maps, base, sh); break;
+                case 2: intra_copy_y<DT, ONE>(p, maps, base, sh); break;
+                default: intra_mm3<ONE>(p, base, tmem, sh);
             }
         }
         __syncwarp();
@@ -708,9 +803,9 @@ int tc_intra_status_clear() {
     return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess ? 0 : -1;
 }
 
-template <int DT, bool SCALAR>
-static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, cudaStream_t stream) {
-    auto kern = intra_fwd_tc_kernel<DT, SCALAR>;
+template <int DT, bool SCALAR, class G>
+static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, const G& gate, cudaStream_t stream) {
+    auto kern = intra_fwd_tc_kernel<DT, SCALAR, G>;
     if (int e = ensure_smem((const void*)kern, in::SMEM, "intra_fwd")) return e;
     static const int regs = kernel_registers((const void*)kern);
     if (regs < in::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "intra_fwd: built with fewer registers than its warps redistribute");
@@ -720,23 +815,31 @@ static int launch_intra_fwd_tc_t(const MkdaIntraFwd* p, cudaStream_t stream) {
     constexpr int ES = DT == MKDA_F32 ? 4 : 2;
     int e = make_rows_map(&maps.k, p->k, ES, rows, k_cols, "intra_fwd");
     if (!e) e = make_rows_map(&maps.q, p->q, ES, rows, k_cols, "intra_fwd");
-    if (!e && !SCALAR) e = make_rows_map(&maps.g, p->g_c, 4, rows, v_cols, "intra_fwd");
+    if constexpr (in::GATED<G>) {
+        if (!e && !SCALAR) e = make_rows_map(&maps.g, gate.x, gate.x_dtype == MKDA_F32 ? 4 : 2, rows, v_cols, "intra_fwd");
+    } else {
+        if (!e && !SCALAR) e = make_rows_map(&maps.g, p->g_c, 4, rows, v_cols, "intra_fwd");
+    }
     if (!e && DT != MKDA_F32) e = make_rows_map(&maps.v, p->v, 2, rows, v_cols, "intra_fwd", CH, 64);
     if (e) return e;
     const int items = p->L.NC * p->L.HV;
-    launch(kern, items < sm_count() ? items : sm_count(), in::THREADS, in::SMEM, stream, *p, maps);
+    launch(kern, items < sm_count() ? items : sm_count(), in::THREADS, in::SMEM, stream, *p, gate, maps);
     return check_launch("intra_fwd");
 }
-int launch_intra_fwd_tc(const MkdaIntraFwd* p, cudaStream_t stream) {
+template <class G>
+static int launch_intra_fwd_tc_g(const MkdaIntraFwd* p, const G& gate, cudaStream_t stream) {
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {
-        case MKDA_F32 * 2: return launch_intra_fwd_tc_t<MKDA_F32, false>(p, stream);
-        case MKDA_BF16 * 2: return launch_intra_fwd_tc_t<MKDA_BF16, false>(p, stream);
-        case MKDA_F16 * 2: return launch_intra_fwd_tc_t<MKDA_F16, false>(p, stream);
-        case MKDA_F32 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_F32, true>(p, stream);
-        case MKDA_BF16 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_BF16, true>(p, stream);
-        case MKDA_F16 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_F16, true>(p, stream);
+        case MKDA_F32 * 2: return launch_intra_fwd_tc_t<MKDA_F32, false>(p, gate, stream);
+        case MKDA_BF16 * 2: return launch_intra_fwd_tc_t<MKDA_BF16, false>(p, gate, stream);
+        case MKDA_F16 * 2: return launch_intra_fwd_tc_t<MKDA_F16, false>(p, gate, stream);
+        case MKDA_F32 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_F32, true>(p, gate, stream);
+        case MKDA_BF16 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_BF16, true>(p, gate, stream);
+        case MKDA_F16 * 2 + 1: return launch_intra_fwd_tc_t<MKDA_F16, true>(p, gate, stream);
     }
     return set_error(MKDA_ERR_ARG, "intra_fwd: unsupported dtype");
+}
+int launch_intra_fwd_tc(const MkdaIntraFwd* p, const MkdaGateFwd* gate, cudaStream_t stream) {
+    return gate ? launch_intra_fwd_tc_g(p, *gate, stream) : launch_intra_fwd_tc_g(p, in::NoGate{}, stream);
 }
 
 }  // namespace mkda

@@ -160,3 +160,23 @@ def test_a_host_module_of_another_header_is_refused(lib, tmp_path):
         run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, LD_PRELOAD=preload), capture_output=True, text=True)
         assert (run.returncode == 0) == ok, run.stderr
         assert ok or "struct sizes differ" in run.stderr
+
+
+def test_gate_and_intra_in_one_kernel_refuses_what_it_does_not_take(lib):
+    """Without chunks: nothing is launched where the arguments are accepted."""
+    from mogankda_b200 import _lib
+    g, p = _lib.STRUCTS["MkdaGateFwd"](), _lib.STRUCTS["MkdaIntraFwd"]()
+    p.L.HK, p.L.HV, p.L.NC, g.lower_bound, g.mode = 1, 1, 0, -5.0, _lib.MKDA_GATE_EDA
+    for s, names in ((p, ("q", "k", "v", "Aqk", "nw", "u", "kbar", "qs", "gl")), (g, ("x", "beta_raw"))):
+        for f in names:
+            setattr(s, f, 0x30000)
+    call = lambda: lib.mkda_gate_intra_fwd(ctypes.byref(g), ctypes.byref(p), None)      # noqa: E731
+    assert call() == 0
+    for s, f, bad in ((g, "beta_raw", 0), (g, "x", 0x30008), (g, "g_c", 0x30008), (p, "A", 0x30008), (g, "x_dtype", 7), (g, "beta_dtype", -1), (g, "lower_bound", 0.0),
+                      (g, "scalar_gate", 1), (p, "nw", 0), (p.L, "HK", 0)):
+        good = getattr(s, f)
+        setattr(s, f, bad)
+        assert call() == _lib.MKDA_ERR_ARG, f
+        setattr(s, f, good)
+    assert call() == 0
+    assert lib.mkda_gate_intra_fwd(None, ctypes.byref(p), None) == _lib.MKDA_ERR_ARG and lib.mkda_gate_intra_fwd(ctypes.byref(g), None, None) == _lib.MKDA_ERR_ARG

@@ -86,3 +86,40 @@ def test_ragged_chunks(dtype, scalar):
         x, y = x.view(torch.int32), y.view(torch.int32).view(TIMES, *x.shape)
         for c in range(0, TIMES, 2):
             assert torch.equal(y[c], x)
+
+
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("mode,x_dtype", [("eda", torch.float32), ("kimi", torch.bfloat16), ("gdn", torch.float16), ("precomputed", torch.float32)])
+@pytest.mark.parametrize("dtype,scalar", [(torch.bfloat16, False), (torch.float16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_gate_in_the_kernel(dtype, scalar, mode, x_dtype, keep):
+    """mkda_gate_intra_fwd gives the bits of mkda_gate_cumsum_fwd and mkda_intra_fwd, whether or not it leaves behind what a backward pass reads."""
+    import ctypes
+    from mogankda_b200 import _lib
+    T, gen = sum(LENS), torch.Generator(device="cuda").manual_seed(7)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")                        # noqa: E731
+    q, k, v, b = r(1, T, HK, 128).to(dtype), r(1, T, HK, 128).to(dtype), r(1, T, HV, 128).to(dtype), r(1, T, HV).to(x_dtype)
+    x = r(1, T, HV, *(() if scalar else (128,)))
+    x = (-x.abs() if mode == "precomputed" else x).to(x_dtype)
+    A_log, bias = (None, None) if mode == "precomputed" else (0.1 * r(HV), 0.1 * r(*(x.shape[2:])).reshape(-1))
+    cu = torch.tensor([0, *torch.tensor(LENS).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    lay = get_layout(1, T, cu, q.device)
+    g_c, be = ops.gate_cumsum_fwd(lay, x, mode, A_log, bias, -5.0, HV, beta_raw=b, beta_sigmoid=True, beta_scale=2.0)
+    want = ops.intra_fwd(lay, q, k, v, ops.l2norm_rstd(q), ops.l2norm_rstd(k), g_c, be, 128 ** -0.5, HK, HV, scalar)
+    got = [torch.full_like(t, float("nan")) for t in want]
+    g_out, b_out = torch.full_like(g_c, float("nan")), torch.full_like(be, float("nan"))
+    rq, rk = ops.l2norm_rstd(q), ops.l2norm_rstd(k)
+    g, p = _lib.STRUCTS["MkdaGateFwd"](), _lib.STRUCTS["MkdaIntraFwd"]()
+    g.x, g.x_dtype, g.scalar_gate, g.mode, g.lower_bound = ops._ptr(x), ops._dt(x), int(scalar), ops.GATE_MODES[mode], -5.0
+    g.A_log, g.dt_bias = ops._ptr(A_log), ops._ptr(bias)
+    g.beta_raw, g.beta_dtype, g.beta_sigmoid, g.beta_scale = ops._ptr(b), ops._dt(b), 1, 2.0
+    p.L = ops._layout_struct(lay, HK, HV)
+    p.q, p.k, p.v, p.qkv_dtype, p.q_rstd, p.k_rstd = ops._ptr(q), ops._ptr(k), ops._ptr(v), ops._dt(q), ops._ptr(rq), ops._ptr(rk)
+    p.scale, p.scalar_gate = 128 ** -0.5, int(scalar)
+    p.Aqk, p.nw, p.u, p.kbar, p.qs, p.gl = (ops._ptr(t) for t in got[1:])
+    if keep:
+        p.A, g.g_c, g.beta_out = ops._ptr(got[0]), ops._ptr(g_out), ops._ptr(b_out)
+    assert _lib.load().mkda_gate_intra_fwd(ctypes.byref(g), ctypes.byref(p), ops._stream()) == 0
+    for a, c in zip((*got[not keep:], *((g_out, b_out) if keep else ())), (*want[not keep:], *((g_c, be) if keep else ()))):
+        assert torch.equal(a.view(torch.int32), c.view(torch.int32))
+    if not keep:
+        assert g_out.isnan().all() and b_out.isnan().all() and got[0].isnan().all()
