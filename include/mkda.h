@@ -348,6 +348,9 @@ typedef struct {
                                 * CTAs one by one; mkda_qk_grad_finish adds the tiles */
 } MkdaBwdChunk;
 int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream);
+/* The same with dq and dk as mkda_qk_grad_finish would leave them, [TT,HK,128] in qkv_dtype (tokens outside every chunk are not written), where nothing has
+ * to be done for that: HV = HK, and no q_rstd and k_rstd.  The fields dq_v, dk_v and per_v_head are not looked at. */
+int mkda_bwd_chunk_finish(const MkdaBwdChunk* p, void* dq, void* dk, void* stream);
 
 /* Sum over the v-heads sharing a q/k head, then L2-norm backward; writes dq and dk in the input dtype (one launch for
  * both).  Replaces group_reduce_vector (mogan_kda/ops/utils/group_reduce.py:60-79) and l2norm_bwd

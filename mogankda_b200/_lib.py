@@ -16,8 +16,8 @@ ENTRY_POINTS = (
     "mkda_recur_fwd", "mkda_out_fwd", "mkda_epilogue_bwd", "mkda_epilogue_bwd_tiles", "mkda_bwd_dh", "mkda_bwd_chunk",
     "mkda_qk_grad_finish", "mkda_state_combine", "mkda_warmup_chunks", "mkda_selftest_umma", "mkda_selftest_wait", "mkda_epilogue_bwd_noalloc",
 )
-# with a third argument: the order of the segments, the second struct
-ORDERED_ENTRY_POINTS = ("mkda_recur_fwd_ordered", "mkda_chain_fwd_ordered", "mkda_bwd_dh_ordered", "mkda_gate_intra_fwd")
+# with more arguments than the struct and the stream: the order of the segments, a second struct, dq and dk
+LONGER_ENTRY_POINTS = {"mkda_recur_fwd_ordered": 3, "mkda_chain_fwd_ordered": 3, "mkda_bwd_dh_ordered": 3, "mkda_gate_intra_fwd": 3, "mkda_bwd_chunk_finish": 4}
 ENUMS = {}
 STRUCTS = {}
 
@@ -80,10 +80,10 @@ def load():
         raise MkdaError(f"{path} is missing: build it with `python -m mogankda_b200.build` (no CPU or library fallback exists)")
     lib = ctypes.CDLL(path)
     lib.mkda_last_error.restype = ctypes.c_char_p
-    for name in ENTRY_POINTS + ORDERED_ENTRY_POINTS:
+    for name in (*ENTRY_POINTS, *LONGER_ENTRY_POINTS):
         fn = getattr(lib, name)
         fn.restype = ctypes.c_int
-        fn.argtypes = [ctypes.c_void_p] * (3 if name in ORDERED_ENTRY_POINTS else 2)
+        fn.argtypes = [ctypes.c_void_p] * LONGER_ENTRY_POINTS.get(name, 2)
     n = len(STRUCT_ORDER)
     sizes = (ctypes.c_int * n)()
     cnt = lib.mkda_struct_sizes(sizes, n)

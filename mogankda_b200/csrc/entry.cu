@@ -85,14 +85,22 @@ extern "C" int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, voi
 }
 extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) { return mkda_bwd_dh_ordered(p, nullptr, stream); }
 
-extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) {
-    if (!p || !p->q || !p->k || !p->v || !p->g_c || !p->beta || !p->A || !p->h || !p->dh || !p->Vd || !p->dO_t || !p->dVd_t ||
-        !p->dq_v || !p->dk_v || !p->dgp || !p->dbeta || !p->dv)
+static int bwd_chunk(const MkdaBwdChunk* given, bool finish, void* dq, void* dk, void* stream) {
+    if (!given || (finish && (!dq || !dk))) return set_error(MKDA_ERR_ARG, "bwd_chunk: null argument");
+    MkdaBwdChunk call = *given;
+    if (finish) call.dq_v = call.dk_v = nullptr;           // whatever stands there
+    const MkdaBwdChunk* p = &call;
+    if (!p->q || !p->k || !p->v || !p->g_c || !p->beta || !p->A || !p->h || !p->dh || !p->Vd || !p->dO_t || !p->dVd_t ||
+        (!finish && (!p->dq_v || !p->dk_v)) || !p->dgp || !p->dbeta || !p->dv)
         return set_error(MKDA_ERR_ARG, "bwd_chunk: null argument");
-    if (any_misaligned(p->q, p->k, p->v, p->g_c, p->A, p->h, p->dh, p->Vd, p->dO_t, p->dVd_t, p->dq_v, p->dk_v, p->dgp, p->dv))
+    if (any_misaligned(p->q, p->k, p->v, p->g_c, p->A, p->h, p->dh, p->Vd, p->dO_t, p->dVd_t, p->dq_v, p->dk_v, p->dgp, p->dv, dq, dk))
         return set_error(MKDA_ERR_ARG, "bwd_chunk: tensors must be 16-byte aligned");
     if (p->beta_sigmoid && !p->beta_raw) return set_error(MKDA_ERR_ARG, "bwd_chunk: sigmoid beta needs the raw input");
     if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "bwd_chunk: HV must be a multiple of HK");
+    if (finish && (p->L.HK != p->L.HV || p->q_rstd || p->k_rstd))
+        return set_error(MKDA_ERR_ARG, "bwd_chunk_finish: needs one v-head per q/k head and rows that are not normalised");
     if (p->L.NC == 0) return MKDA_OK;
-    return launch_bwd_chunk_tc(p, (cudaStream_t)stream);
+    return launch_bwd_chunk_tc(p, dq, dk, (cudaStream_t)stream);
 }
+extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) { return bwd_chunk(p, false, nullptr, nullptr, stream); }
+extern "C" int mkda_bwd_chunk_finish(const MkdaBwdChunk* p, void* dq, void* dk, void* stream) { return bwd_chunk(p, true, dq, dk, stream); }

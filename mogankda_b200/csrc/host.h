@@ -55,7 +55,7 @@ int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stre
 int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, const MkdaGateFwd* gate, cudaStream_t stream);      // gate: formed there, or NULL
-int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream);
+int launch_bwd_chunk_tc(const MkdaBwdChunk* p, void* dq, void* dk, cudaStream_t stream);      // dq, dk: rows instead of tiles, or NULL
 int tc_bwd_chunk_status(unsigned int* out);
 int tc_bwd_chunk_status_clear();
 int tc_intra_status(unsigned int* out);

@@ -240,8 +240,11 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     tmp.want(&dh, c.tiles(MKDA_STATE_TILE_BYTES));
     tmp.want(&dVd, c.tiles(tile));
     const bool spread = spread_v_heads(c);
-    tmp.want(&dq_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
-    tmp.want(&dk_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
+    const bool finished = !c.l2 && c.HV == c.HK;          // dq and dk leave the chunk kernel as they are
+    if (!finished) {
+        tmp.want(&dq_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
+        tmp.want(&dk_v, (int64_t)c.NC * (spread ? c.HV : c.HK) * tile);
+    }
     tmp.want(&dgp, c.tiles(c.scalar_gate ? 256 : tile));
     if (c.has_ep && in.ep_w.defined()) tmp.want(&part_w, (int64_t)w_rows * 512);
     if (c.mode != MKDA_GATE_PRECOMPUTED) {
@@ -289,6 +292,8 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     check_rc(mkda_bwd_dh_ordered(&full, order, st), "mkda_bwd_dh");
     g.v = c.rows_out(c.HV, in.v.scalar_type());
     g.beta = c.like_out(in.beta);
+    g.q = c.rows_out(c.HK, in.q.scalar_type());
+    g.k = c.rows_out(c.HK, in.k.scalar_type());
     {
         MkdaBwdChunk p{};
         p.L = L; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.v = in.v.data_ptr(); p.qkv_dtype = c.qkv_dtype;
@@ -296,7 +301,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         p.dh = dh; p.Vd = s.Vd; p.dO_t = dO; p.dVd_t = dVd; p.scale = c.scale; p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta);
         p.beta_sigmoid = c.beta_sigmoid; p.beta_scale = c.beta_scale; p.dq_v = dq_v; p.dk_v = dk_v; p.dgp = dgp; p.dbeta = g.beta.data_ptr();
         p.dbeta_dtype = dtype_code(g.beta); p.dv = g.v.data_ptr(); p.per_v_head = spread;
-        check_rc(mkda_bwd_chunk(&p, st), "mkda_bwd_chunk");
+        check_rc(finished ? mkda_bwd_chunk_finish(&p, g.q.data_ptr(), g.k.data_ptr(), st) : mkda_bwd_chunk(&p, st), "mkda_bwd_chunk");
     }
     g.x = c.like_out(in.x);
     {
@@ -316,9 +321,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         auto cast = [](Tensor& t, const Tensor& like) { if (t.defined() && t.scalar_type() != like.scalar_type()) t = t.to(like.scalar_type()); };
         cast(g.ep_w, in.ep_w); cast(g.dt_bias, in.dt_bias); cast(g.A_log, in.A_log);
     }
-    g.q = c.rows_out(c.HK, in.q.scalar_type());
-    g.k = c.rows_out(c.HK, in.k.scalar_type());
-    {
+    if (!finished) {
         MkdaQkGrad p{};
         p.L = L; p.dq_v = dq_v; p.dk_v = dk_v; p.q = in.q.data_ptr(); p.k = in.k.data_ptr(); p.x_dtype = c.qkv_dtype;
         p.q_rstd = s.q_rstd; p.k_rstd = s.k_rstd; p.dq = g.q.data_ptr(); p.dk = g.k.data_ptr(); p.per_v_head = spread;

@@ -85,6 +85,11 @@ struct Scratch {
 };
 static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
 
+// dq and dk by token rows, [TT,HK,128] in the type of q and k, instead of fp32 tiles: with one v-head per q/k head and no L2 norm to go back through nothing is
+// left to be done (4 x 16 k tokens x 16 heads, scalar gate: 241 us of qk_grad_finish less; this kernel, half of its dq and dk less to write, takes as long as
+// before, 1224 us, and 1260 where two lanes exchange values for 4-byte stores)
+struct Finished { void *dq, *dk; };
+
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 using umma::elect_one;
 using umma::signal;
@@ -305,8 +310,8 @@ __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared
 }
 
 // Compute warps.  Thread (q, lane, cg): accumulator lane `row` = 32 q + lane, columns or rows [16 cg, 16 cg + 16).
-template <int DT, bool SCALAR, bool SPREAD>
-__device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
+__device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const bc::Finished& fin, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int q = warp & 3, cg = warp >> 2, row = q * 32 + lane;
@@ -626,8 +631,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
         if (tid < len && p.beta_sigmoid) raw_beta = ld1(p.beta_raw, p.beta_dtype, (size_t)(start + tid) * HV + h);
         const bool first_of_group = it.first;
         const size_t obk = it.group * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
-        float* __restrict__ oq = p.dq_v + obk;
-        float* __restrict__ ok = p.dk_v + obk;
+        float* __restrict__ oq = FINISH ? nullptr : p.dq_v + obk;
+        float* __restrict__ ok = FINISH ? nullptr : p.dk_v + obk;
+        const size_t orow = ((size_t)start * HK + hk) * 128 + row;
         float* __restrict__ og = SCALAR ? p.dgp + (size_t)it.item * CH : p.dgp + it.item * (size_t)(CH * DK) + row;
         f32x2 cs2 = 0;
         float dg_last = 0.f;
@@ -719,7 +725,9 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
                     for (int o = 0; o < 2; ++o) {
                         const int io = i + o;
                         const float dq = io < len ? dqv[o] : 0.f, dk = io < len ? dkv[o] : 0.f, dg = io < len ? dgv[o] : 0.f;
-                        if (first_of_group) { oq[io * DK] = dq; ok[io * DK] = dk; }
+                        if (FINISH) {
+                            if (io < len) { st1(fin.dq, DT, orow + (size_t)io * HK * 128, dq); st1(fin.dk, DT, orow + (size_t)io * HK * 128, dk); }
+                        } else if (first_of_group) { oq[io * DK] = dq; ok[io * DK] = dk; }
                         else { red_add(oq + io * DK, dq); red_add(ok + io * DK, dk); }
                         if (SCALAR) dgs[2 * pr + o] = dg;
                         else if (io == len - 1) dg_last = dg;
@@ -769,8 +777,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, uint8_t
     }
 }
 
-template <int DT, bool SCALAR, bool SPREAD>
-__global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p) {
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
+__global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p, const bc::Finished fin) {
     using namespace bc;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
@@ -803,35 +811,37 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        bwd_chunk_compute<DT, SCALAR, SPREAD>(p, base, sh);
+        bwd_chunk_compute<DT, SCALAR, SPREAD, FINISH>(p, fin, base, sh);
     }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(sh.tmem, 512);
 }
 
-template <int DT, bool SCALAR, bool SPREAD>
-static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, cudaStream_t stream) {
-    auto kern = bwd_chunk_tc_kernel<DT, SCALAR, SPREAD>;
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
+static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, const bc::Finished& fin, cudaStream_t stream) {
+    auto kern = bwd_chunk_tc_kernel<DT, SCALAR, SPREAD, FINISH>;
     if (int e = ensure_smem((const void*)kern, bc::SMEM, "bwd_chunk")) return e;
     static const int regs = kernel_registers((const void*)kern);
     if (regs < bc::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "bwd_chunk: built with fewer registers than its warps redistribute");
     const int groups = p->L.NC * (SPREAD ? p->L.HV : p->L.HK);              // a CTA takes whole (chunk, q/k head) groups
-    launch(kern, groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream, *p);
+    launch(kern, groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream, *p, fin);
     return check_launch("bwd_chunk");
 }
 template <int DT, bool SCALAR>
-static int launch_bwd_chunk_tc_s(const MkdaBwdChunk* p, cudaStream_t stream) {
-    return p->per_v_head ? launch_bwd_chunk_tc_t<DT, SCALAR, true>(p, stream) : launch_bwd_chunk_tc_t<DT, SCALAR, false>(p, stream);
+static int launch_bwd_chunk_tc_s(const MkdaBwdChunk* p, const bc::Finished& fin, cudaStream_t stream) {
+    if (fin.dq) return launch_bwd_chunk_tc_t<DT, SCALAR, true, true>(p, fin, stream);
+    return p->per_v_head ? launch_bwd_chunk_tc_t<DT, SCALAR, true, false>(p, fin, stream) : launch_bwd_chunk_tc_t<DT, SCALAR, false, false>(p, fin, stream);
 }
-int launch_bwd_chunk_tc(const MkdaBwdChunk* p, cudaStream_t stream) {
+int launch_bwd_chunk_tc(const MkdaBwdChunk* p, void* dq, void* dk, cudaStream_t stream) {
+    const bc::Finished fin{dq, dk};
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {
-        case MKDA_F32 * 2: return launch_bwd_chunk_tc_s<MKDA_F32, false>(p, stream);
-        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_s<MKDA_BF16, false>(p, stream);
-        case MKDA_F16 * 2: return launch_bwd_chunk_tc_s<MKDA_F16, false>(p, stream);
-        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F32, true>(p, stream);
-        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_BF16, true>(p, stream);
-        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F16, true>(p, stream);
+        case MKDA_F32 * 2: return launch_bwd_chunk_tc_s<MKDA_F32, false>(p, fin, stream);
+        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_s<MKDA_BF16, false>(p, fin, stream);
+        case MKDA_F16 * 2: return launch_bwd_chunk_tc_s<MKDA_F16, false>(p, fin, stream);
+        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F32, true>(p, fin, stream);
+        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_BF16, true>(p, fin, stream);
+        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F16, true>(p, fin, stream);
     }
     return set_error(MKDA_ERR_ARG, "bwd_chunk: unsupported dtype");
 }

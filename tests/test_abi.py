@@ -180,3 +180,22 @@ def test_gate_and_intra_in_one_kernel_refuses_what_it_does_not_take(lib):
         setattr(s, f, good)
     assert call() == 0
     assert lib.mkda_gate_intra_fwd(None, ctypes.byref(p), None) == _lib.MKDA_ERR_ARG and lib.mkda_gate_intra_fwd(ctypes.byref(g), None, None) == _lib.MKDA_ERR_ARG
+
+
+def test_finished_chunk_backward_refuses_what_is_left_to_finish(lib):
+    """Without chunks: nothing is launched where the arguments are accepted."""
+    from mogankda_b200 import _lib
+    p = _lib.STRUCTS["MkdaBwdChunk"]()
+    p.L.HK, p.L.HV, p.L.NC = 2, 2, 0
+    for f in ("q", "k", "v", "g_c", "beta", "A", "h", "dh", "Vd", "dO_t", "dVd_t", "dgp", "dbeta", "dv"):
+        setattr(p, f, 0x30000)
+    p.dq_v = 0x30001                                       # not looked at
+    call = lambda dq=0x30000, dk=0x30000: lib.mkda_bwd_chunk_finish(ctypes.byref(p), dq, dk, None)      # noqa: E731
+    assert call() == 0
+    assert call(dq=0) == call(dk=0) == call(dk=0x30008) == _lib.MKDA_ERR_ARG
+    for obj, f, bad in ((p.L, "HV", 4), (p, "q_rstd", 0x30000), (p, "k_rstd", 0x30000), (p, "dv", 0)):
+        good = getattr(obj, f)
+        setattr(obj, f, bad)
+        assert call() == _lib.MKDA_ERR_ARG, f
+        setattr(obj, f, good)
+    assert lib.mkda_bwd_chunk(ctypes.byref(p), None) == _lib.MKDA_ERR_ARG

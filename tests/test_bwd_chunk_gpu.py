@@ -70,3 +70,31 @@ def test_rows_past_the_end_are_zero_whatever_the_others_hold(dtype, scalar):
             for t in ops.bwd_chunk(lay, q, k, lv["v"], rq, rk, g_c, be, A, S, dS, Vd, dO, dVd, 128 ** -0.5, HK, HV, lv["beta"], True, 2.0, scalar_gate=scalar)[:3]:
                 for c, n in enumerate(lay.chunk_len.tolist()):
                     assert (t[c, :, n:] == 0).all(), (x, c, n)
+
+
+@pytest.mark.parametrize("scalar", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_finished_dq_and_dk(dtype, scalar, monkeypatch):
+    """mkda_bwd_chunk_finish leaves the bits of mkda_bwd_chunk and mkda_qk_grad_finish (no L2 norm, one v-head per q/k head), and nothing outside the chunks."""
+    import ctypes
+    from mogankda_b200 import _lib, ops
+    lens, H = (1, 15, 16, 17, 33, 63, 64, 65), 3
+    T, cu = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, _, opts, _ = make_inputs(T=T, HK=H, HV=H, cu=tuple(cu), dtype=dtype, gate="precomputed", scalar=scalar, l2=False, epi=None, h0=False, seed=67)
+    lay = get_layout(1, T, opts["cu_seqlens"], lv["q"].device, 32)
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "precomputed", None, None, -5.0, H, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, 128 ** -0.5, H, H, scalar_gate=scalar)
+    h, Vd, _, _ = ops.recur_fwd(lay, nw, u, kbar, gl, H, H)
+    dh, dVd, dO, _ = ops.bwd_dh(lay, do, kbar, qs, gl, Aqk, nw, H, H)
+    args = (lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, A, h, dh, Vd, dO, dVd, 128 ** -0.5, H, H, lv["beta"], True, 2.0)
+    want = ops.bwd_chunk(*args, scalar_gate=scalar)
+    rows = ops.qk_grad_finish(lay, want[0], want[1], lv["q"], lv["k"], None, None, H, H)
+    # a row more in front and behind: outside every chunk
+    got = [torch.full((T + 2, H, 128), 7.0, dtype=dtype, device="cuda") for _ in range(2)]
+    monkeypatch.setattr(_lib, "call", lambda name, p, *a: _lib.load().mkda_bwd_chunk_finish(ctypes.byref(p), *(ctypes.c_void_p(t[1:].data_ptr()) for t in got), ctypes.c_void_p(a[0])))
+    out = ops.bwd_chunk(*args, scalar_gate=scalar)
+    monkeypatch.undo()
+    for t, w in zip(got, rows):
+        assert torch.equal(t[1:-1], w.view(T, H, 128)) and (t[[0, -1]] == 7).all()
+    for a, b in zip(out[2:], want[2:]):
+        assert torch.equal(a, b)
