@@ -316,6 +316,9 @@ typedef struct {
 } MkdaBwdDh;
 int mkda_bwd_dh(const MkdaBwdDh* p, void* stream);
 int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, void* stream);
+/* The same for bf16 rows d_o, which are read where they are; only chunks of fewer than 64 tokens need tiles, of which the high halves are used: those of
+ * dO_in_t, or, if that is NULL, those that are then written to dO_t.  Both may be NULL if there is no such chunk. */
+int mkda_bwd_dh_rows(const MkdaBwdDh* p, const int* seg_order, void* stream);
 
 /* Every gradient that is local to a (chunk, v-head) once the state gradients are known, in one kernel:
  *  - through Vd = A diag(beta)(V - k~ S): dv, the WY part of dbeta, dAqk and dL = -strictlower(A^T dVd Vd^T) (K3a of bwd_post_kda,
@@ -348,9 +351,12 @@ typedef struct {
                                 * CTAs one by one; mkda_qk_grad_finish adds the tiles */
 } MkdaBwdChunk;
 int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream);
-/* The same with dq and dk as mkda_qk_grad_finish would leave them, [TT,HK,128] in qkv_dtype (tokens outside every chunk are not written), where nothing has
- * to be done for that: HV = HK, and no q_rstd and k_rstd.  The fields dq_v, dk_v and per_v_head are not looked at. */
-int mkda_bwd_chunk_finish(const MkdaBwdChunk* p, void* dq, void* dk, void* stream);
+/* The same with tensors by token rows in the place of tiles, each where it is not NULL.
+ * d_o: dO as bf16 rows [TT,HV,128], for qkv_dtype bf16 too.  Of dO_t only the tiles of chunks of fewer than 64 tokens are read, of these the high halves
+ *   (mkda_bwd_dh_rows leaves them there); it may be NULL if there are none.
+ * dq and dk (both or neither): as mkda_qk_grad_finish would leave them, [TT,HK,128] in qkv_dtype (tokens outside every chunk are not written), where nothing
+ *   has to be done for that: HV = HK, and no q_rstd and k_rstd.  The fields dq_v, dk_v and per_v_head are then not looked at. */
+int mkda_bwd_chunk_rows(const MkdaBwdChunk* p, const void* d_o, void* dq, void* dk, void* stream);
 
 /* Sum over the v-heads sharing a q/k head, then L2-norm backward; writes dq and dk in the input dtype (one launch for
  * both).  Replaces group_reduce_vector (mogan_kda/ops/utils/group_reduce.py:60-79) and l2norm_bwd

@@ -16,8 +16,9 @@ ENTRY_POINTS = (
     "mkda_recur_fwd", "mkda_out_fwd", "mkda_epilogue_bwd", "mkda_epilogue_bwd_tiles", "mkda_bwd_dh", "mkda_bwd_chunk",
     "mkda_qk_grad_finish", "mkda_state_combine", "mkda_warmup_chunks", "mkda_selftest_umma", "mkda_selftest_wait", "mkda_epilogue_bwd_noalloc",
 )
-# with more arguments than the struct and the stream: the order of the segments, a second struct, dq and dk
-LONGER_ENTRY_POINTS = {"mkda_recur_fwd_ordered": 3, "mkda_chain_fwd_ordered": 3, "mkda_bwd_dh_ordered": 3, "mkda_gate_intra_fwd": 3, "mkda_bwd_chunk_finish": 4}
+# with more arguments than the struct and the stream: the order of the segments, a second struct, dO, dq and dk as rows
+LONGER_ENTRY_POINTS = {"mkda_recur_fwd_ordered": 3, "mkda_chain_fwd_ordered": 3, "mkda_bwd_dh_ordered": 3, "mkda_gate_intra_fwd": 3, "mkda_bwd_dh_rows": 3,
+                       "mkda_bwd_chunk_rows": 5}
 ENUMS = {}
 STRUCTS = {}
 

@@ -69,38 +69,55 @@ extern "C" int mkda_chain_fwd_ordered(const MkdaChainFwd* p, const int* seg_orde
 }
 extern "C" int mkda_chain_fwd(const MkdaChainFwd* p, void* stream) { return mkda_chain_fwd_ordered(p, nullptr, stream); }
 
-extern "C" int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, void* stream) {
-    if (!p || !(p->dO_in_t || (p->d_o && p->dO_t)) || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw)
-        return set_error(MKDA_ERR_ARG, "bwd_dh: null argument");
+static int check_bwd_dh(const MkdaBwdDh* p, bool source) {
+    if (!p || !source || !p->kbar || !p->qs || !p->gl || !p->Aqk || !p->nw) return set_error(MKDA_ERR_ARG, "bwd_dh: null argument");
     if (any_misaligned(p->d_o, p->dO_in_t, p->kbar, p->qs, p->gl, p->Aqk, p->nw, p->dh, p->dVd_t, p->dO_t))
         return set_error(MKDA_ERR_ARG, "bwd_dh: tensors must be 16-byte aligned");
     if (any_misaligned32(p->dh, p->dVd_t) || (p->state_v_first && any_misaligned32(p->dht, p->dh0)))
         return set_error(MKDA_ERR_ARG, "bwd_dh: saved tiles and [V,K] states must be 32-byte aligned");
+    return MKDA_OK;
+}
+extern "C" int mkda_bwd_dh_ordered(const MkdaBwdDh* p, const int* seg_order, void* stream) {
+    if (int e = check_bwd_dh(p, p && (p->dO_in_t || (p->d_o && p->dO_t)))) return e;
     if (p->L.NS == 0) return MKDA_OK;
-    if (p->dO_in_t) return launch_bwd_dh_tc(p, seg_order, (cudaStream_t)stream);
+    if (p->dO_in_t) return launch_bwd_dh_tc(p, seg_order, false, (cudaStream_t)stream);
     if (int e = launch_rows_to_tiles(p->L, p->d_o, p->do_dtype, p->dO_t, (cudaStream_t)stream)) return e;
     MkdaBwdDh q = *p;
     q.dO_in_t = p->dO_t;
-    return launch_bwd_dh_tc(&q, seg_order, (cudaStream_t)stream);
+    return launch_bwd_dh_tc(&q, seg_order, false, (cudaStream_t)stream);
+}
+extern "C" int mkda_bwd_dh_rows(const MkdaBwdDh* p, const int* seg_order, void* stream) {
+    if (int e = check_bwd_dh(p, p && p->d_o)) return e;
+    if (p->do_dtype != MKDA_BF16) return set_error(MKDA_ERR_ARG, "bwd_dh_rows: unsupported dtype");
+    if (p->L.NS == 0) return MKDA_OK;
+    MkdaBwdDh q = *p;
+    if (!q.dO_in_t && q.dO_t) {
+        if (int e = launch_ragged_rows_to_tiles(q.L, q.d_o, q.dO_t, (cudaStream_t)stream)) return e;
+        q.dO_in_t = q.dO_t;
+    }
+    return launch_bwd_dh_tc(&q, seg_order, true, (cudaStream_t)stream);
 }
 extern "C" int mkda_bwd_dh(const MkdaBwdDh* p, void* stream) { return mkda_bwd_dh_ordered(p, nullptr, stream); }
 
-static int bwd_chunk(const MkdaBwdChunk* given, bool finish, void* dq, void* dk, void* stream) {
+static int bwd_chunk(const MkdaBwdChunk* given, const void* d_o, bool finish, void* dq, void* dk, void* stream) {
     if (!given || (finish && (!dq || !dk))) return set_error(MKDA_ERR_ARG, "bwd_chunk: null argument");
     MkdaBwdChunk call = *given;
     if (finish) call.dq_v = call.dk_v = nullptr;           // whatever stands there
     const MkdaBwdChunk* p = &call;
-    if (!p->q || !p->k || !p->v || !p->g_c || !p->beta || !p->A || !p->h || !p->dh || !p->Vd || !p->dO_t || !p->dVd_t ||
+    if (!p->q || !p->k || !p->v || !p->g_c || !p->beta || !p->A || !p->h || !p->dh || !p->Vd || (!p->dO_t && !d_o) || !p->dVd_t ||
         (!finish && (!p->dq_v || !p->dk_v)) || !p->dgp || !p->dbeta || !p->dv)
         return set_error(MKDA_ERR_ARG, "bwd_chunk: null argument");
-    if (any_misaligned(p->q, p->k, p->v, p->g_c, p->A, p->h, p->dh, p->Vd, p->dO_t, p->dVd_t, p->dq_v, p->dk_v, p->dgp, p->dv, dq, dk))
+    if (any_misaligned(p->q, p->k, p->v, p->g_c, p->A, p->h, p->dh, p->Vd, p->dO_t, p->dVd_t, p->dq_v, p->dk_v, p->dgp, p->dv, d_o, dq, dk))
         return set_error(MKDA_ERR_ARG, "bwd_chunk: tensors must be 16-byte aligned");
     if (p->beta_sigmoid && !p->beta_raw) return set_error(MKDA_ERR_ARG, "bwd_chunk: sigmoid beta needs the raw input");
     if (p->L.HK <= 0 || p->L.HV % p->L.HK) return set_error(MKDA_ERR_ARG, "bwd_chunk: HV must be a multiple of HK");
     if (finish && (p->L.HK != p->L.HV || p->q_rstd || p->k_rstd))
-        return set_error(MKDA_ERR_ARG, "bwd_chunk_finish: needs one v-head per q/k head and rows that are not normalised");
+        return set_error(MKDA_ERR_ARG, "bwd_chunk_rows: finished dq and dk need one v-head per q/k head and rows that are not normalised");
+    if (d_o && p->qkv_dtype != MKDA_BF16) return set_error(MKDA_ERR_ARG, "bwd_chunk_rows: rows of dO are taken in bf16 calls only");
     if (p->L.NC == 0) return MKDA_OK;
-    return launch_bwd_chunk_tc(p, dq, dk, (cudaStream_t)stream);
+    return launch_bwd_chunk_tc(p, d_o, dq, dk, (cudaStream_t)stream);
 }
-extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) { return bwd_chunk(p, false, nullptr, nullptr, stream); }
-extern "C" int mkda_bwd_chunk_finish(const MkdaBwdChunk* p, void* dq, void* dk, void* stream) { return bwd_chunk(p, true, dq, dk, stream); }
+extern "C" int mkda_bwd_chunk(const MkdaBwdChunk* p, void* stream) { return bwd_chunk(p, nullptr, false, nullptr, nullptr, stream); }
+extern "C" int mkda_bwd_chunk_rows(const MkdaBwdChunk* p, const void* d_o, void* dq, void* dk, void* stream) {
+    return bwd_chunk(p, d_o, dq || dk, dq, dk, stream);
+}

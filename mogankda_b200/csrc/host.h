@@ -49,13 +49,14 @@ int launch_out_fwd_tc(const MkdaOutFwd* p, cudaStream_t stream);
 int tc_chunk_status(unsigned int* out);
 int tc_chunk_status_clear();
 int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void* tiles, cudaStream_t stream);
+int launch_ragged_rows_to_tiles(const MkdaLayout& L, const void* rows, void* tiles, cudaStream_t stream);
 int launch_recur_fwd_tc(const MkdaRecurFwd* p, const int* seg_order, cudaStream_t stream);
 int launch_chain_fwd_tc(const MkdaChainFwd* p, const int* seg_order, cudaStream_t stream);
-int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, cudaStream_t stream);
+int launch_bwd_dh_tc(const MkdaBwdDh* p, const int* seg_order, bool rows, cudaStream_t stream);
 int tc_recur_status(unsigned int* out);
 int tc_recur_status_clear();
 int launch_intra_fwd_tc(const MkdaIntraFwd* p, const MkdaGateFwd* gate, cudaStream_t stream);      // gate: formed there, or NULL
-int launch_bwd_chunk_tc(const MkdaBwdChunk* p, void* dq, void* dk, cudaStream_t stream);      // dq, dk: rows instead of tiles, or NULL
+int launch_bwd_chunk_tc(const MkdaBwdChunk* p, const void* d_o, void* dq, void* dk, cudaStream_t stream);      // rows instead of tiles, or NULL
 int tc_bwd_chunk_status(unsigned int* out);
 int tc_bwd_chunk_status_clear();
 int tc_intra_status(unsigned int* out);

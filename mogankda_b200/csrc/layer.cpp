@@ -236,7 +236,9 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     const int64_t tile = MKDA_CHUNK_TILE_BYTES, seg_states = (int64_t)c.NS * c.HV * 65536;
     const int w_rows = std::min(c.NC * c.HV, MKDA_EPILOGUE_MAX_PART_ROWS);
     const int g_rows = std::min(c.NC, 256), g_width = c.scalar_gate ? c.HV : c.HV * 128;
-    tmp.want(&dO, c.tiles(tile));
+    // bf16 gradients of an output without a norm are operands as they stand; only chunks that are not full need tiles
+    const bool rows = !c.has_ep && c.qkv_dtype == MKDA_BF16 && dy.scalar_type() == at::kBFloat16, ragged = !c.covers_all || (int64_t)c.NC * 64 != c.TT;
+    if (!rows || ragged) tmp.want(&dO, c.tiles(tile));
     tmp.want(&dh, c.tiles(MKDA_STATE_TILE_BYTES));
     tmp.want(&dVd, c.tiles(tile));
     const bool spread = spread_v_heads(c);
@@ -278,7 +280,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     if (c.segmented) {
         // pre-pass from zero: only the gradient entering each segment is wanted, nothing per chunk is stored
         d.dh0 = dloc; d.warm_end = s.warm_end;
-        check_rc(mkda_bwd_dh_ordered(&d, order, st), "mkda_bwd_dh");
+        check_rc(rows ? mkda_bwd_dh_rows(&d, order, st) : mkda_bwd_dh_ordered(&d, order, st), "mkda_bwd_dh");
         MkdaCombine m{};
         m.NG = c.N; m.HV = c.HV; m.grp_seg_off = c.grp_off; m.hs = dloc; m.ms = s.ms; m.carry = fptr(dht); m.reverse = 1; m.s_in = g_in;
         m.s_out = fptr(g.h0); m.carry_v_first = c.vf; m.out_v_first = c.vf;
@@ -289,7 +291,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
     }
     full.dh = dh; full.dVd_t = dVd;
     if (c.segmented) full.dO_in_t = dO;                    // already in tile form
-    check_rc(mkda_bwd_dh_ordered(&full, order, st), "mkda_bwd_dh");
+    check_rc(rows ? mkda_bwd_dh_rows(&full, order, st) : mkda_bwd_dh_ordered(&full, order, st), "mkda_bwd_dh");
     g.v = c.rows_out(c.HV, in.v.scalar_type());
     g.beta = c.like_out(in.beta);
     g.q = c.rows_out(c.HK, in.q.scalar_type());
@@ -301,7 +303,7 @@ Grads run_backward(const Call& c, const Inputs& in, Saved& s, Tensor dy, Tensor 
         p.dh = dh; p.Vd = s.Vd; p.dO_t = dO; p.dVd_t = dVd; p.scale = c.scale; p.beta_raw = in.beta.data_ptr(); p.beta_dtype = dtype_code(in.beta);
         p.beta_sigmoid = c.beta_sigmoid; p.beta_scale = c.beta_scale; p.dq_v = dq_v; p.dk_v = dk_v; p.dgp = dgp; p.dbeta = g.beta.data_ptr();
         p.dbeta_dtype = dtype_code(g.beta); p.dv = g.v.data_ptr(); p.per_v_head = spread;
-        check_rc(finished ? mkda_bwd_chunk_finish(&p, g.q.data_ptr(), g.k.data_ptr(), st) : mkda_bwd_chunk(&p, st), "mkda_bwd_chunk");
+        check_rc(mkda_bwd_chunk_rows(&p, rows ? dy.data_ptr() : nullptr, finished ? g.q.data_ptr() : nullptr, finished ? g.k.data_ptr() : nullptr, st), "mkda_bwd_chunk");
     }
     g.x = c.like_out(in.x);
     {

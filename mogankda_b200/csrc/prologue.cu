@@ -532,6 +532,24 @@ __global__ void __launch_bounds__(256) rows_to_tiles_kernel(const MkdaLayout L, 
     }
 }
 
+// The high halves only (all there is of bf16 rows), of the chunks that are not full; a block looks at four heads of one chunk.
+__global__ void __launch_bounds__(256) ragged_rows_to_tiles_kernel(const MkdaLayout L, const uint16_t* rows, uint8_t* tiles) {
+    follow_stream();
+    const int HV = L.HV, c = blockIdx.x, start = L.chunk_start[c], len = L.chunk_len[c];
+    if (len == CH) return;
+    const int k8 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+    for (int h = 4 * blockIdx.y; h < min(4 * (int)blockIdx.y + 4, HV); ++h) {
+        uint8_t* tile = tiles + ((size_t)c * HV + h) * 32768;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + 16 * i;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (r < len) v = *reinterpret_cast<const uint4*>(rows + ((size_t)(start + r) * HV + h) * 128 + k8 * 8);
+            *reinterpret_cast<uint4*>(tile + umma::tile_chunk_offset(64, r, k8)) = v;
+        }
+    }
+}
+
 // Warm-up truncation table: one CTA per (segment, v-head), one thread per key channel (see MkdaWarmup).
 // gl = 2^gL may have underflowed to zero: log2 gives -inf, i.e. fully decayed.
 __global__ void __launch_bounds__(128) warmup_chunks_kernel(const MkdaWarmup p) {
@@ -565,6 +583,11 @@ int launch_rows_to_tiles(const MkdaLayout& L, const void* rows, int dtype, void*
         case MKDA_F16: launch(rows_to_tiles_kernel<MKDA_F16>, grid, 256, 0, stream, L, rows, t); break;
         default: return set_error(MKDA_ERR_ARG, "bwd_dh: unsupported dtype");
     }
+    return check_launch("rows_to_tiles");
+}
+int launch_ragged_rows_to_tiles(const MkdaLayout& L, const void* rows, void* tiles, cudaStream_t stream) {
+    if (L.NC == 0 || L.HV == 0) return MKDA_OK;
+    launch(ragged_rows_to_tiles_kernel, dim3(L.NC, (L.HV + 3) / 4), 256, 0, stream, L, static_cast<const uint16_t*>(rows), static_cast<uint8_t*>(tiles));
     return check_launch("rows_to_tiles");
 }
 

@@ -44,6 +44,8 @@
 #include "host.h"
 #include "intra.cuh"
 
+#include <type_traits>
+
 namespace mkda {
 
 namespace bc {
@@ -85,11 +87,21 @@ struct Scratch {
 };
 static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
 
+// dO as bf16 rows, as in bwd_dh: full chunks' are fetched from where they are, the others' as tiles, of either the high half only.  The low half below which the
+// low half of dW is stacked is zeros: written once, or, where beta dLs passes through its place, again in each epilogue (two stores per thread; fetched from a
+// block of zeros in L2 the kernel took 1336 us at 4 x 16 k tokens x 16 heads, 1190 to 1235 so, and 1210 to 1255 with tiles).
+struct NoRows {};
+template <class R> constexpr bool ROWS = std::is_same<R, CUtensorMap>::value;
+
 // dq and dk by token rows, [TT,HK,128] in the type of q and k, instead of fp32 tiles: with one v-head per q/k head and no L2 norm to go back through nothing is
 // left to be done (4 x 16 k tokens x 16 heads, scalar gate: 241 us of qk_grad_finish less; this kernel, half of its dq and dk less to write, takes as long as
 // before, 1224 us, and 1260 where two lanes exchange values for 4-byte stores)
 struct Finished { void *dq, *dk; };
 
+__device__ __forceinline__ void no_low_half(uint8_t* base) {
+#pragma unroll
+    for (int i = 2; i < 4; ++i) *reinterpret_cast<uint4*>(base + o_piece(i) + 16 * threadIdx.x) = make_uint4(0, 0, 0, 0);
+}
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 using umma::elect_one;
 using umma::signal;
@@ -206,13 +218,13 @@ __device__ __forceinline__ bool from_hbm(const MkdaLayout& L) { return (size_t)L
 // the kernels behind (1B shape 201 -> 193 us, fp16 4 x 1000 tokens 66 -> 63, short documents 248 -> 242, 64k packed tokens no difference).
 // S and Vd of the next item are requested once the state products and dgl of the current one are done, dO, dVd and A once the intra-chunk products
 // are (with a scalar gate, whose products leave the place of dVd and A alone, these two go with S and Vd), dS' once dVd and A have been read.
-template <bool SCALAR, bool SPREAD>
-__device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* base, bc::Shared& sh) {
+template <bool SCALAR, bool SPREAD, class R>
+__device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, const R& rows, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     auto src = [](const void* t, size_t it, uint32_t bytes, uint32_t off = 0) { return static_cast<const uint8_t*>(t) + it * bytes + off; };
     const bool hints = from_hbm(p.L);
     auto request_s = [&](size_t it) {
-        umma::mbar_expect_tx(&sh.fullS, umma::STATE_TILE_BYTES + 2 * umma::CHUNK_TILE_BYTES);
+        umma::mbar_expect_tx(&sh.fullS, umma::STATE_TILE_BYTES + (ROWS<R> ? 3 : 4) * umma::CHUNK_TILE_BYTES / 2);
         umma::bulk_load_last(base + S_, src(p.h, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullS);
         umma::bulk_load_last(base + V_, src(p.Vd, it, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES, &sh.fullS);
     };
@@ -222,8 +234,16 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
         umma::bulk_load_last(base + A_, src(p.A, it, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES, &sh.fullW);
     };
     uint32_t n = 0;
-    for (ItemWalk<SPREAD> w(p.L); w.valid(); ++n) {
+    ItemWalk<SPREAD> w(p.L);
+    int start = 0, len = 0;                                // of the next item's chunk, read an item ahead
+    auto look = [&]() {
+        if (!ROWS<R> || !w.valid()) return;
+        start = p.L.chunk_start[w.chunk()]; len = p.L.chunk_len[w.chunk()];
+    };
+    look();
+    for (; w.valid(); ++n) {
         const size_t it = w.item();
+        const int x = w.head() * 128;
         if (n) {
             umma::mbar_wait(&sh.mmI[0], (n & 1) ^ 1);
         } else {
@@ -231,14 +251,23 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
             request_s(it);
         }
         if (n && !SCALAR) request_w(it);
+        if constexpr (ROWS<R>) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            umma::bulk_load_last(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
+            for (int i = 0; i < 2; ++i) {
+                if (len == CH || !p.dO_t) umma::tma_load_rows(base + o_piece(i), &rows, x + 64 * i, start, &sh.fullS);
+                else umma::bulk_load_last(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                umma::bulk_load_last(base + o_piece(i), src(p.dO_t, it, umma::CHUNK_TILE_BYTES, 8192 * i), 8192, &sh.fullS);
+        }
         umma::mbar_wait(&sh.mmW, n & 1);                 // dVd and A have been read
         umma::mbar_expect_tx(&sh.fullT, umma::STATE_TILE_BYTES);
         umma::bulk_load_last(base + T_, src(p.dh, it, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES, &sh.fullT);
         w.next();
         if (!w.valid()) break;
+        look();
         const size_t in = w.item();
         // Hints for what finds no room before the epilogue (3.47 -> 3.23 ms on 64k packed tokens x 32 heads, 1315 -> 1250 us on 4 x 16k x 16 heads with a
         // scalar gate, when all of the item's tiles waited for it).  Not where the tiles of all items come close to fitting into L2 as they are: 512
@@ -247,7 +276,16 @@ __device__ __forceinline__ void bwd_chunk_load(const MkdaBwdChunk& p, uint8_t* b
             umma::mbar_wait(&sh.mmL, n & 1);
             umma::l2_prefetch(src(p.dVd_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
             umma::l2_prefetch(src(p.A, in, umma::QUARTER_TILE_BYTES), umma::QUARTER_TILE_BYTES);
-            umma::l2_prefetch(src(p.dO_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
+            if constexpr (ROWS<R>) {
+                if (len == CH || !p.dO_t) {
+                    umma::tma_prefetch_rows(&rows, w.head() * 128, start);
+                    umma::tma_prefetch_rows(&rows, w.head() * 128 + 64, start);
+                } else {
+                    umma::l2_prefetch(src(p.dO_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES / 2);
+                }
+            } else {
+                umma::l2_prefetch(src(p.dO_t, in, umma::CHUNK_TILE_BYTES), umma::CHUNK_TILE_BYTES);
+            }
             umma::l2_prefetch(src(p.dh, in, umma::STATE_TILE_BYTES), umma::STATE_TILE_BYTES);
         }
         umma::mbar_wait(&sh.free, n & 1);
@@ -310,7 +348,7 @@ __device__ __forceinline__ void bwd_chunk_rows(const MkdaBwdChunk& p, bc::Shared
 }
 
 // Compute warps.  Thread (q, lane, cg): accumulator lane `row` = 32 q + lane, columns or rows [16 cg, 16 cg + 16).
-template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH, bool ROWS>
 __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const bc::Finished& fin, uint8_t* base, bc::Shared& sh) {
     using namespace bc;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -638,6 +676,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const b
         f32x2 cs2 = 0;
         float dg_last = 0.f;
         wait_mma(&sh.mmI[SCALAR ? 0 : cg], par);
+        if (ROWS && SCALAR) no_low_half(base);             // for the next item's products, which follow this warp's next signal
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int c0 = 16 * cg + 8 * hf;
@@ -777,8 +816,8 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const b
     }
 }
 
-template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
-__global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p, const bc::Finished fin) {
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH, class R>
+__global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const MkdaBwdChunk p, const bc::Finished fin, const __grid_constant__ R rows) {
     using namespace bc;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw;                              // no static shared memory: the dynamic block starts on a 1024-byte boundary
@@ -796,6 +835,7 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
         for (int I = 0; I < 4; ++I) umma::mbar_init(&sh.opI[I], SCALAR ? COMPUTE / 32 : 4 * (I + 1));
         umma::fence_barrier_init();
     }
+    if (ROWS<R> && threadIdx.x < COMPUTE) no_low_half(base);
     publish();
     follow_stream();
     if (warp >= COMPUTE / 32) {
@@ -804,44 +844,55 @@ __global__ void __launch_bounds__(bc::THREADS, 1) bwd_chunk_tc_kernel(const Mkda
             if (elect_one()) bwd_chunk_issue<SCALAR, SPREAD>(p, base, sh);
             __syncwarp();
         } else if (warp == WARP_LOAD) {
-            if (elect_one()) bwd_chunk_load<SCALAR, SPREAD>(p, base, sh);
+            if (elect_one()) bwd_chunk_load<SCALAR, SPREAD>(p, rows, base, sh);
             __syncwarp();
         } else if (warp == WARP_ROWS) {
             bwd_chunk_rows<DT, SCALAR, SPREAD>(p, sh, threadIdx.x & 31);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        bwd_chunk_compute<DT, SCALAR, SPREAD, FINISH>(p, fin, base, sh);
+        bwd_chunk_compute<DT, SCALAR, SPREAD, FINISH, ROWS<R>>(p, fin, base, sh);
     }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(sh.tmem, 512);
 }
 
-template <int DT, bool SCALAR, bool SPREAD, bool FINISH>
-static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, const bc::Finished& fin, cudaStream_t stream) {
-    auto kern = bwd_chunk_tc_kernel<DT, SCALAR, SPREAD, FINISH>;
+template <int DT, bool SCALAR, bool SPREAD, bool FINISH, class R>
+static int launch_bwd_chunk_tc_t(const MkdaBwdChunk* p, const bc::Finished& fin, const R& rows, cudaStream_t stream) {
+    auto kern = bwd_chunk_tc_kernel<DT, SCALAR, SPREAD, FINISH, R>;
     if (int e = ensure_smem((const void*)kern, bc::SMEM, "bwd_chunk")) return e;
     static const int regs = kernel_registers((const void*)kern);
     if (regs < bc::LAUNCH_REGS) return set_error(MKDA_ERR_LAUNCH, "bwd_chunk: built with fewer registers than its warps redistribute");
     const int groups = p->L.NC * (SPREAD ? p->L.HV : p->L.HK);              // a CTA takes whole (chunk, q/k head) groups
-    launch(kern, groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream, *p, fin);
+    launch(kern, groups < sm_count() ? groups : sm_count(), bc::THREADS, bc::SMEM, stream, *p, fin, rows);
     return check_launch("bwd_chunk");
 }
-template <int DT, bool SCALAR>
-static int launch_bwd_chunk_tc_s(const MkdaBwdChunk* p, const bc::Finished& fin, cudaStream_t stream) {
-    if (fin.dq) return launch_bwd_chunk_tc_t<DT, SCALAR, true, true>(p, fin, stream);
-    return p->per_v_head ? launch_bwd_chunk_tc_t<DT, SCALAR, true, false>(p, fin, stream) : launch_bwd_chunk_tc_t<DT, SCALAR, false, false>(p, fin, stream);
+template <int DT, bool SCALAR, class R>
+static int launch_bwd_chunk_tc_r(const MkdaBwdChunk* p, const bc::Finished& fin, const R& rows, cudaStream_t stream) {
+    if (fin.dq) return launch_bwd_chunk_tc_t<DT, SCALAR, true, true>(p, fin, rows, stream);
+    return p->per_v_head ? launch_bwd_chunk_tc_t<DT, SCALAR, true, false>(p, fin, rows, stream) : launch_bwd_chunk_tc_t<DT, SCALAR, false, false>(p, fin, rows, stream);
 }
-int launch_bwd_chunk_tc(const MkdaBwdChunk* p, void* dq, void* dk, cudaStream_t stream) {
+template <int DT, bool SCALAR>
+static int launch_bwd_chunk_tc_s(const MkdaBwdChunk* p, const bc::Finished& fin, const void* d_o, cudaStream_t stream) {
+    if constexpr (DT == MKDA_BF16) {
+        if (d_o) {
+            CUtensorMap map;
+            if (int e = make_rows_map(&map, d_o, 2, (unsigned long long)p->L.TT, (unsigned long long)p->L.HV * 128, "bwd_chunk", CH, 64)) return e;
+            return launch_bwd_chunk_tc_r<DT, SCALAR>(p, fin, map, stream);
+        }
+    }
+    return launch_bwd_chunk_tc_r<DT, SCALAR>(p, fin, bc::NoRows{}, stream);
+}
+int launch_bwd_chunk_tc(const MkdaBwdChunk* p, const void* d_o, void* dq, void* dk, cudaStream_t stream) {
     const bc::Finished fin{dq, dk};
     switch (p->qkv_dtype * 2 + (p->scalar_gate ? 1 : 0)) {
-        case MKDA_F32 * 2: return launch_bwd_chunk_tc_s<MKDA_F32, false>(p, fin, stream);
-        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_s<MKDA_BF16, false>(p, fin, stream);
-        case MKDA_F16 * 2: return launch_bwd_chunk_tc_s<MKDA_F16, false>(p, fin, stream);
-        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F32, true>(p, fin, stream);
-        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_BF16, true>(p, fin, stream);
-        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F16, true>(p, fin, stream);
+        case MKDA_F32 * 2: return launch_bwd_chunk_tc_s<MKDA_F32, false>(p, fin, d_o, stream);
+        case MKDA_BF16 * 2: return launch_bwd_chunk_tc_s<MKDA_BF16, false>(p, fin, d_o, stream);
+        case MKDA_F16 * 2: return launch_bwd_chunk_tc_s<MKDA_F16, false>(p, fin, d_o, stream);
+        case MKDA_F32 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F32, true>(p, fin, d_o, stream);
+        case MKDA_BF16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_BF16, true>(p, fin, d_o, stream);
+        case MKDA_F16 * 2 + 1: return launch_bwd_chunk_tc_s<MKDA_F16, true>(p, fin, d_o, stream);
     }
     return set_error(MKDA_ERR_ARG, "bwd_chunk: unsupported dtype");
 }

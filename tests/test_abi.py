@@ -190,7 +190,7 @@ def test_finished_chunk_backward_refuses_what_is_left_to_finish(lib):
     for f in ("q", "k", "v", "g_c", "beta", "A", "h", "dh", "Vd", "dO_t", "dVd_t", "dgp", "dbeta", "dv"):
         setattr(p, f, 0x30000)
     p.dq_v = 0x30001                                       # not looked at
-    call = lambda dq=0x30000, dk=0x30000: lib.mkda_bwd_chunk_finish(ctypes.byref(p), dq, dk, None)      # noqa: E731
+    call = lambda dq=0x30000, dk=0x30000: lib.mkda_bwd_chunk_rows(ctypes.byref(p), None, dq, dk, None)      # noqa: E731
     assert call() == 0
     assert call(dq=0) == call(dk=0) == call(dk=0x30008) == _lib.MKDA_ERR_ARG
     for obj, f, bad in ((p.L, "HV", 4), (p, "q_rstd", 0x30000), (p, "k_rstd", 0x30000), (p, "dv", 0)):

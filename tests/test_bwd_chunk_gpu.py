@@ -75,7 +75,7 @@ def test_rows_past_the_end_are_zero_whatever_the_others_hold(dtype, scalar):
 @pytest.mark.parametrize("scalar", [False, True])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_finished_dq_and_dk(dtype, scalar, monkeypatch):
-    """mkda_bwd_chunk_finish leaves the bits of mkda_bwd_chunk and mkda_qk_grad_finish (no L2 norm, one v-head per q/k head), and nothing outside the chunks."""
+    """mkda_bwd_chunk_rows leaves the bits of mkda_bwd_chunk and mkda_qk_grad_finish (no L2 norm, one v-head per q/k head), and nothing outside the chunks."""
     import ctypes
     from mogankda_b200 import _lib, ops
     lens, H = (1, 15, 16, 17, 33, 63, 64, 65), 3
@@ -91,10 +91,59 @@ def test_finished_dq_and_dk(dtype, scalar, monkeypatch):
     rows = ops.qk_grad_finish(lay, want[0], want[1], lv["q"], lv["k"], None, None, H, H)
     # a row more in front and behind: outside every chunk
     got = [torch.full((T + 2, H, 128), 7.0, dtype=dtype, device="cuda") for _ in range(2)]
-    monkeypatch.setattr(_lib, "call", lambda name, p, *a: _lib.load().mkda_bwd_chunk_finish(ctypes.byref(p), *(ctypes.c_void_p(t[1:].data_ptr()) for t in got), ctypes.c_void_p(a[0])))
+    monkeypatch.setattr(_lib, "call", lambda name, p, *a: _lib.load().mkda_bwd_chunk_rows(ctypes.byref(p), None, *(ctypes.c_void_p(t[1:].data_ptr()) for t in got), ctypes.c_void_p(a[0])))
     out = ops.bwd_chunk(*args, scalar_gate=scalar)
     monkeypatch.undo()
     for t, w in zip(got, rows):
         assert torch.equal(t[1:-1], w.view(T, H, 128)) and (t[[0, -1]] == 7).all()
     for a, b in zip(out[2:], want[2:]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("finish", [False, True])
+@pytest.mark.parametrize("times", [1, 12])
+@pytest.mark.parametrize("lens", [(1, 15, 64, 65, 63, 128), (64, 128, 192)])
+@pytest.mark.parametrize("scalar", [False, True])
+def test_rows_of_dO(scalar, lens, times, finish, monkeypatch):
+    """mkda_bwd_dh_rows and mkda_bwd_chunk_rows on bf16 rows give the bits of the tiles, chains shared between two CTAs or not, one and many items per CTA; full
+    chunks have no tile, and of the others' the low halves are not looked at."""
+    import ctypes
+    from mogankda_b200 import _lib, ops
+    lens, HK, HV = lens * times, 2, 2 if finish else 4
+    T, cu = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, dht, opts, _ = make_inputs(T=T, HK=HK, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="precomputed", scalar=scalar, l2=False, epi=None, h0=False, seed=71)
+    lay = get_layout(1, T, opts["cu_seqlens"], lv["q"].device, 32)
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "precomputed", None, None, -5.0, HV, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, 128 ** -0.5, HK, HV, scalar_gate=scalar)
+    h, Vd, _, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV)
+    do = do.to(torch.bfloat16).contiguous()
+
+    def both():
+        dh, dVd, dO, dh0 = ops.bwd_dh(lay, do, kbar, qs, gl, Aqk, nw, HK, HV, want_dh0=True)
+        if rows:
+            t = dO.view(torch.bfloat16).reshape(lay.NC, HV, 2, -1)
+            t[:, :, 1] = float("nan")
+            t[lay.chunk_len == 64] = float("nan")
+        out = ops.bwd_chunk(lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, A, h, dh, Vd, dO, dVd, 128 ** -0.5, HK, HV, lv["beta"], True, 2.0, scalar_gate=scalar)
+        return dh, dVd, dh0, *out
+
+    rows = False
+    want = both()
+    fin = ops.qk_grad_finish(lay, want[3], want[4], lv["q"], lv["k"], None, None, HK, HV)
+    rows, got_q, got_k = True, torch.empty_like(lv["q"]), torch.empty_like(lv["k"])
+
+    def call(name, p, *args):
+        lib, stream = _lib.load(), args[-1]
+        if name == "mkda_bwd_dh_ordered":
+            assert lib.mkda_bwd_dh_rows(ctypes.byref(p), *args) == 0
+        else:
+            dq, dk = (got_q.data_ptr(), got_k.data_ptr()) if finish else (None, None)
+            assert lib.mkda_bwd_chunk_rows(ctypes.byref(p), do.data_ptr(), dq, dk, stream) == 0
+    monkeypatch.setattr(_lib, "call", call)
+    got = both()
+    monkeypatch.undo()
+    for i, (a, b) in enumerate(zip(got, want)):
+        if not (finish and i in (3, 4)):
+            assert torch.equal(a.view(torch.int32) if a.dtype == torch.float32 else a, b.view(torch.int32) if b.dtype == torch.float32 else b), i
+    if finish:
+        assert torch.equal(got_q.view(-1), fin[0].view(-1)) and torch.equal(got_k.view(-1), fin[1].view(-1))
