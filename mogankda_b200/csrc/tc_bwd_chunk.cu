@@ -94,8 +94,8 @@ struct NoRows {};
 template <class R> constexpr bool ROWS = std::is_same<R, CUtensorMap>::value;
 
 // dq and dk by token rows, [TT,HK,128] in the type of q and k, instead of fp32 tiles: with one v-head per q/k head and no L2 norm to go back through nothing is
-// left to be done (4 x 16 k tokens x 16 heads, scalar gate: 241 us of qk_grad_finish less; this kernel, half of its dq and dk less to write, takes as long as
-// before, 1224 us, and 1260 where two lanes exchange values for 4-byte stores)
+// left to be done (4 x 16 k tokens x 16 heads, scalar gate: 241 us of qk_grad_finish less; this kernel, half of its dq and dk less to write, takes 1310 us instead
+// of 1270: 256-byte pieces 4 KB apart; with the same stores to one block it takes 1240.  Two lanes that exchange values for 4-byte stores: 1260 where it was 1224)
 struct Finished { void *dq, *dk; };
 
 __device__ __forceinline__ void no_low_half(uint8_t* base) {
@@ -671,7 +671,10 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const b
         const size_t obk = it.group * (size_t)(CH * DK) + row;      // dq / dk: one tile per q/k head
         float* __restrict__ oq = FINISH ? nullptr : p.dq_v + obk;
         float* __restrict__ ok = FINISH ? nullptr : p.dk_v + obk;
-        const size_t orow = ((size_t)start * HK + hk) * 128 + row;
+        constexpr int FB = DT == MKDA_F32 ? 4 : 2;
+        const size_t frow = (((size_t)start * HK + hk) * 128 + row) * FB;
+        const uint32_t fpitch = HK * 128 * FB;
+        char *fq = static_cast<char*>(fin.dq) + frow, *fk = static_cast<char*>(fin.dk) + frow;
         float* __restrict__ og = SCALAR ? p.dgp + (size_t)it.item * CH : p.dgp + it.item * (size_t)(CH * DK) + row;
         f32x2 cs2 = 0;
         float dg_last = 0.f;
@@ -765,7 +768,7 @@ __device__ __forceinline__ void bwd_chunk_compute(const MkdaBwdChunk& p, const b
                         const int io = i + o;
                         const float dq = io < len ? dqv[o] : 0.f, dk = io < len ? dkv[o] : 0.f, dg = io < len ? dgv[o] : 0.f;
                         if (FINISH) {
-                            if (io < len) { st1(fin.dq, DT, orow + (size_t)io * HK * 128, dq); st1(fin.dk, DT, orow + (size_t)io * HK * 128, dk); }
+                            if (io < len) { st1(fq + (uint32_t)io * fpitch, DT, 0, dq); st1(fk + (uint32_t)io * fpitch, DT, 0, dk); }
                         } else if (first_of_group) { oq[io * DK] = dq; ok[io * DK] = dk; }
                         else { red_add(oq + io * DK, dq); red_add(ok + io * DK, dk); }
                         if (SCALAR) dgs[2 * pr + o] = dg;
