@@ -254,12 +254,23 @@ __global__ void __launch_bounds__(256) gate_bwd_scalar_kernel(const MkdaGateBwd 
 // rounds (21 us).
 constexpr int RED_OUTS = 8, RED_LANES = 128;
 __host__ __device__ inline int reduce_blocks(const MkdaReduce& j) { return (j.cols / j.group + RED_OUTS - 1) / RED_OUTS; }
+// the job of a block, and its block of that job (no index that is not a constant: the struct would be copied to local memory by every thread)
+__device__ __forceinline__ MkdaReduce reduce_job(const MkdaReduceMulti& p, int& blk) {
+    MkdaReduce q = p.job[0];
+#pragma unroll
+    for (int job = 0; job < 2; ++job) {
+        const int n = reduce_blocks(p.job[job]);
+        if (blk < n) break;
+        blk -= n;
+        q = p.job[job + 1];
+    }
+    return q;
+}
 __global__ void __launch_bounds__(1024) reduce_kernel(const MkdaReduceMulti p) {
     follow_stream();
     __shared__ float part[RED_OUTS][RED_LANES + 4];
-    int blk = blockIdx.x, job = 0;
-    while (job < 2 && blk >= reduce_blocks(p.job[job])) { blk -= reduce_blocks(p.job[job]); ++job; }
-    const MkdaReduce q = p.job[job];
+    int blk = blockIdx.x;
+    const MkdaReduce q = reduce_job(p, blk);
     const int o = threadIdx.x & (RED_OUTS - 1), l = threadIdx.x / RED_OUTS, j = blk * RED_OUTS + o, outs = q.cols / q.group, terms = q.rows * q.group;
     float s = 0.f;
     if (j < outs) {
