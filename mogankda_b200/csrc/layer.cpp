@@ -72,19 +72,16 @@ bool spread_v_heads(const Call& c) {
 // 40 + 8, 24 items 258 against 189 + 38.
 bool gate_in_intra(const Call& c) { return (int64_t)c.NC * c.HV <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
 
-// Output in the kernel of the state chain, or in one of its own?  In units of 1000 SM cycles per chunk: a chain step takes 6
-// without the output; with it 8.5 (a backward pass follows) or 6.5, and 12 or 9 when the gated norm is fused; a kernel of its own takes 7
-// (11 with the norm) per chunk and SM and 6 to launch, and has all SMs.  So the separate kernel is the better one where a few long
-// chains leave SMs idle: fp16 4 x 1000 tokens x 8 heads 75 instead of 96 us, 64k packed tokens x 32 heads 2260 instead of 1770 us.
-// These units are older than the kernels: a step takes 7.2 or 4.7 without a norm, where the output's products stand behind the chain's, and 4.0 by itself
-// where two CTAs share the chain.  Over 1, 2, 4 ... 64 steps x 4 to 128 chains, with and without norm and backward pass, the line takes the fused kernel 19
-// times in 280 where the separate ones are faster, by 1 to 21 % and between 4 and 72 chains (norm, forward only: 8 steps x 32 chains 37.9 us against 31.4,
-// 64 x 48 268 against 241), and never the other way round.
+// Output in the kernel of the state chain, or in one of its own?  A separate one has all SMs where a few chains leave some idle, and where there are at most half as
+// many chains as SMs two CTAs share a chain of it; with more chains the fused kernel was never behind.  Costs in units of 1000 SM cycles, fitted to both over 1, 2, 4 ...
+// 64 steps x 4 to 128 chains, with and without norm and backward pass: a fused step takes 4.9 (7.9 if a backward pass follows), 7.8 (11.4) with the norm, a shared one
+// without the output 4.2, the separate output 8.8 (8.5) per chunk and SM and 7 to launch.  Of 280 shapes 6 are on the wrong side, by 2 to 5 %; the line before, older than
+// shared chains, had 13, by up to 16 % (norm, forward only: 8 steps x 32 chains 36.2 us fused, 31.2 separate; 64 x 48 258 and 240).
 bool output_in_chain(const Call& c, bool need_bwd) {
     const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    const double share = (double)c.NC * c.HV / sms, steps = std::max((double)c.chain, share);
-    const double fused = steps * (c.has_ep ? (need_bwd ? 12.0 : 9.0) : (need_bwd ? 8.5 : 6.5));
-    return fused <= steps * 6.0 + share * (c.has_ep ? 11.0 : 7.0) + 6.0;
+    if (2.0 * c.NS * c.HV > sms) return true;
+    const double share = (double)c.NC * c.HV / sms, steps = c.chain;
+    return steps * (c.has_ep ? (need_bwd ? 11.4 : 7.8) : (need_bwd ? 7.9 : 4.9)) <= steps * 4.2 + share * (c.has_ep ? 8.5 : 8.8) + 7.0;
 }
 
 // Segments longest first, unless all of them run at once.  In the order of the documents a long one that starts late is waited for at the end:
