@@ -59,6 +59,8 @@ int launch_intra_fwd_tc(const MkdaIntraFwd* p, const MkdaGateFwd* gate, cudaStre
 int launch_bwd_chunk_tc(const MkdaBwdChunk* p, const void* d_o, void* dq, void* dk, cudaStream_t stream);      // rows instead of tiles, or NULL
 int tc_bwd_chunk_status(unsigned int* out);
 int tc_bwd_chunk_status_clear();
+int step_status(unsigned int* out);
+int step_status_clear();
 int tc_intra_status(unsigned int* out);
 int tc_intra_status_clear();
 }  // namespace mkda

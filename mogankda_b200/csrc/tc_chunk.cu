@@ -137,12 +137,15 @@ __global__ void __launch_bounds__(512, 1) out_fwd_tc_kernel(const MkdaOutFwd p) 
     tc_end(&sh, tmem, 64);
 }
 
-int tc_chunk_status(unsigned int* out) {
-    return cudaMemcpyFromSymbol(out, umma::g_timeout_flag, sizeof(unsigned int)) == cudaSuccess ? 0 : -1;
+int tc_chunk_status(unsigned int* out) {                   // and of the step kernel
+    unsigned int step = 0;
+    if (cudaMemcpyFromSymbol(out, umma::g_timeout_flag, sizeof(unsigned int)) != cudaSuccess || step_status(&step) != 0) return -1;
+    *out |= step;
+    return 0;
 }
 int tc_chunk_status_clear() {
     const unsigned int z = 0;
-    return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess ? 0 : -1;
+    return cudaMemcpyToSymbol(umma::g_timeout_flag, &z, sizeof(z)) == cudaSuccess && step_status_clear() == 0 ? 0 : -1;
 }
 
 template <int GDT>

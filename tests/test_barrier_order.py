@@ -437,3 +437,28 @@ def test_bwd_chunk(scalar, from_hbm):
             if what == "wait":
                 assert phase == seen.get(bar, 0), (name, bar, phase)
                 seen[bar] = phase + 1
+
+
+def step(dims, n=STEPS):
+    """step_fwd_vk: compute warps a and b, one warp that fetches what the items are and their states."""
+    r = Roles({k: (d[0] if d else 1) for k, d in dims.items()})
+    r.count = {"empty": 2}
+    wait, arrive = r.agent("load")
+    for k in range(n + 1):                                 # the last one says that there are no more
+        if k >= 2:
+            wait("empty", k - 2)
+        arrive("known", k)
+        if k < n:
+            arrive("full", k)
+    for w in "ab":
+        wait, arrive = r.agent("compute" + w)
+        wait("known", 0)
+        for k in range(n):
+            wait("full", k), arrive("empty", k), wait("known", k + 1)
+    return r
+
+
+def test_step_fwd_vk():
+    dims = _slots("step.cu", "Shared")
+    assert step(dims).late_waits() == []
+    assert step({k: [] for k in dims}).late_waits() != []

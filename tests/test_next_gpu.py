@@ -100,3 +100,33 @@ def test_api_errors_follow_the_reference_conventions():
         mk.chunk_gated_delta_rule(*args)                                     # ... and the scalar entry point a scalar one
     with pytest.raises(AssertionError):
         mk.chunk_delta_rule(*args, gate_mode="eda")                          # eda needs A_log
+
+
+@pytest.mark.parametrize("HV", [1, 16])
+@pytest.mark.parametrize("dtype,norm,scalar", [(torch.bfloat16, True, False), (torch.float16, False, False), (torch.float32, True, False),
+                                               (torch.float32, False, True)])
+@pytest.mark.parametrize("lens", [(1, 16, 2, 0, 15, 3), (1,) * 40, (3, 70, 16, 17, 1)])
+def test_steps_with_a_state_in_either_layout(lens, dtype, norm, scalar, HV):
+    """[V,K] states have a step kernel of their own: up to several items per CTA, empty sequences, and longer ones in the batch, which it leaves alone.  The sums over
+    128 channels are formed in another order, 2^-24 x 128 of their terms at most (states of size 0.1, |k| = 1, 16 tokens): 1e-5 of the largest value."""
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    r = lambda *s: torch.randn(*s, generator=gen, device="cuda")                        # noqa: E731
+    T, N, HK = sum(lens), len(lens), max(HV // 2, 1)
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    q, k, v, beta, h0 = r(1, T, HK, 128).to(dtype), r(1, T, HK, 128).to(dtype), r(1, T, HV, 128).to(dtype), torch.rand(1, T, HV, generator=gen, device="cuda"), 0.1 * r(N, HV, 128, 128)
+    g = -torch.rand(1, T, HV, *(() if scalar else (128,)), generator=gen, device="cuda")
+    epi = dict(weight=r(128), gate=r(1, T, HV, 128).to(dtype), act="silu", eps=1e-6) if norm else None
+
+    def call(vf):
+        f = mk.chunk_gated_delta_rule if scalar else mk.chunk_kda
+        kw = {} if scalar else dict(gate_mode="precomputed", beta_mode="precomputed", output_norm=epi)
+        with torch.no_grad():
+            return f(q, k, v, g, beta, initial_state=h0.transpose(2, 3).contiguous() if vf else h0, output_final_state=True, use_qk_l2norm_in_kernel=True, cu_seqlens=cu,
+                     state_v_first=vf, **kw)
+    (o, ht), (ov, htv) = call(False), call(True)
+    tol = 2.0 ** -8 if o.dtype == torch.bfloat16 else 2.0 ** -10 if o.dtype == torch.float16 else 1e-5
+    assert (o.float() - ov.float()).abs().max() <= tol * o.float().abs().max()
+    assert (ht - htv.transpose(2, 3)).abs().max() <= 1e-5 * ht.abs().max()
+    for n, length in enumerate(lens):
+        if length == 0:
+            assert torch.equal(htv[n], h0[n].transpose(1, 2))
