@@ -543,21 +543,28 @@ __global__ void __launch_bounds__(256) rows_to_tiles_kernel(const MkdaLayout L, 
     }
 }
 
-// The high halves only (all there is of bf16 rows), of the chunks that are not full; a block looks at four heads of one chunk.
+// The high halves only (all there is of bf16 rows), of the chunks that are not full; a block looks at four heads of one chunk, all their rows in flight (one head
+// after the other: 10.3 us instead of 3.8 where rows_to_tiles took 4.5, 2188 tokens x 8 heads in a few documents).
 __global__ void __launch_bounds__(256) ragged_rows_to_tiles_kernel(const MkdaLayout L, const uint16_t* rows, uint8_t* tiles) {
     follow_stream();
-    const int HV = L.HV, c = blockIdx.x, start = L.chunk_start[c], len = L.chunk_len[c];
+    const int HV = L.HV, c = blockIdx.x, start = L.chunk_start[c], len = L.chunk_len[c], h0 = 4 * blockIdx.y;
     if (len == CH) return;
     const int k8 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
-    for (int h = 4 * blockIdx.y; h < min(4 * (int)blockIdx.y + 4, HV); ++h) {
-        uint8_t* tile = tiles + ((size_t)c * HV + h) * 32768;
+    uint4 v[4][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int r = r0 + 16 * i;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (r < len) v = *reinterpret_cast<const uint4*>(rows + ((size_t)(start + r) * HV + h) * 128 + k8 * 8);
-            *reinterpret_cast<uint4*>(tile + umma::tile_chunk_offset(64, r, k8)) = v;
+            v[e][i] = make_uint4(0, 0, 0, 0);
+            if (r < len && h0 + e < HV) v[e][i] = *reinterpret_cast<const uint4*>(rows + ((size_t)(start + r) * HV + h0 + e) * 128 + k8 * 8);
         }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (h0 + e >= HV) return;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(tiles + ((size_t)c * HV + h0 + e) * 32768 + umma::tile_chunk_offset(64, r0 + 16 * i, k8)) = v[e][i];
     }
 }
 
