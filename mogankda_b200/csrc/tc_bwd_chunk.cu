@@ -37,7 +37,7 @@
 // dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
 // An item takes 23 k cycles (26 k before): 1B shape 223 -> 201 us, 64 k packed tokens x 32 heads 3.64 -> 3.29 ms, short documents 267 -> 250 us, fp16 4 x 1000
 // tokens 74 -> 66, scalar gate 4 x 16 k tokens x 16 heads 1313 -> 1249; with the hints of rows and the loads that leave L2 first 193 us, 3.23 ms, 242 us, 63,
-// 1210 (64 k tokens on other boxes, whose clocks differ: 2.84 to 3.12 ms).
+// 1210 (64 k tokens on other boxes, whose clocks differ: 2.84 to 3.12 ms); with waits that do not read the clock first 180 us, 229, 61.
 // Shared memory (KB): S [0,64) | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> weights [64,96), scratch in dW pieces | Vd^T [128,160) |
 // dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Qr; beta Kr].
 // TMEM columns: R_I 32 I; [D1; Z] 128, later C_I 128 + {0, 16, 48, 96}; dW 320, later Dq 320 and Dk 384, later column tiles 288 + {0, 16, 48, 96}; Db 448.
