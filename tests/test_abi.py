@@ -199,3 +199,20 @@ def test_finished_chunk_backward_refuses_what_is_left_to_finish(lib):
         assert call() == _lib.MKDA_ERR_ARG, f
         setattr(obj, f, good)
     assert lib.mkda_bwd_chunk(ctypes.byref(p), None) == _lib.MKDA_ERR_ARG
+
+
+def test_reverse_chain_on_rows_refuses_other_rows(lib):
+    """Without segments: nothing is launched where the arguments are accepted."""
+    from mogankda_b200 import _lib
+    p = _lib.STRUCTS["MkdaBwdDh"]()
+    p.L.NS, p.do_dtype = 0, _lib.MKDA_BF16
+    for f in ("d_o", "kbar", "qs", "gl", "Aqk", "nw"):
+        setattr(p, f, 0x30000)
+    call = lambda: lib.mkda_bwd_dh_rows(ctypes.byref(p), None, None)                    # noqa: E731
+    assert call() == 0                                     # no tiles: no chunk is ragged
+    for f, bad in (("d_o", 0), ("d_o", 0x30002), ("do_dtype", _lib.MKDA_F16), ("dO_t", 0x30008), ("nw", 0), ("dh", 0x30010)):
+        good = getattr(p, f)
+        setattr(p, f, bad)
+        assert call() == _lib.MKDA_ERR_ARG, f
+        setattr(p, f, good)
+    assert lib.mkda_bwd_dh_rows(None, None, None) == _lib.MKDA_ERR_ARG
