@@ -72,16 +72,21 @@ bool spread_v_heads(const Call& c) {
 // 40 + 8, 24 items 258 against 189 + 38.
 bool gate_in_intra(const Call& c) { return (int64_t)c.NC * c.HV <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
 
-// Output in the kernel of the state chain, or in one of its own?  A separate one has all SMs where a few chains leave some idle, and where there are at most half as
-// many chains as SMs two CTAs share a chain of it; with more chains the fused kernel was never behind.  Costs in units of 1000 SM cycles, fitted to both over 1, 2, 4 ...
-// 64 steps x 4 to 128 chains, with and without norm and backward pass: a fused step takes 4.9 (7.9 if a backward pass follows), 7.8 (11.4) with the norm, a shared one
-// without the output 4.2, the separate output 8.8 (8.5) per chunk and SM and 7 to launch.  Of 280 shapes 6 are on the wrong side, by 2 to 5 %; the line before, older than
-// shared chains, had 13, by up to 16 % (norm, forward only: 8 steps x 32 chains 36.2 us fused, 31.2 separate; 64 x 48 258 and 240).
+// Output in the kernel of the state chain, or in one of its own?  A separate one has all SMs where a few chains, or the last steps of a few long ones among many
+// short, leave some idle; with at most half as many chains as SMs two CTAs share a chain of it besides.  In units of 1000 SM cycles, the shared
+// ones fitted to 280 equal batches of 4 to 128 chains x 1 to 64 steps, the others to 656 equal and unequal ones of 60 to 700 chains x 1 to 48, with and without norm and
+// backward pass: a step of the chain without the output takes 4.2 shared and 5.5 not, with it 4.9 and 5.5 (7.9 and 6.8 if a backward pass follows), with the norm 7.8 and 7.3 (11.4 and 9.8); the separate output 8.5 with the norm and 8.8
+// without per chunk and SM, and 7 to launch.  What takes the steps is the longest chain, or the even share of all.  Times in us with norm and backward pass, fused and
+// separate, x 16 heads: documents of 3000, 2000, 1500, 1000 and 692 tokens 420 and 377, one of 2048 and 12 of 512 307 and 285, five of 1536 equal ones
+// 279 and 291; x 8 heads one of 1024 and 30 of 64 137 and 111.  (A line for equal chains alone, all calls of more than half as many chains as SMs fused: 53 of 656 on the
+// wrong side by up to 51 %; this one 4, by up to 5 %.)  Forward only the separate kernels allocate states and Vd, 96 KB per chunk and head, that the fused one
+// never writes: 3 % has to be gained for that.
 bool output_in_chain(const Call& c, bool need_bwd) {
-    const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    if (2.0 * c.NS * c.HV > sms) return true;
-    const double share = (double)c.NC * c.HV / sms, steps = c.chain;
-    return steps * (c.has_ep ? (need_bwd ? 11.4 : 7.8) : (need_bwd ? 7.9 : 4.9)) <= steps * 4.2 + share * (c.has_ep ? 8.5 : 8.8) + 7.0;
+    const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount, share = (double)c.NC * c.HV / sms;
+    const bool shared = 2.0 * c.NS * c.HV <= sms;
+    const double fused = c.has_ep ? (need_bwd ? (shared ? 11.4 : 9.8) : (shared ? 7.8 : 7.3)) : (need_bwd ? (shared ? 7.9 : 6.8) : (shared ? 4.9 : 5.5));
+    const double steps = shared ? c.chain : std::max((double)c.chain, share);
+    return steps * fused <= (need_bwd ? 1.0 : 1.03) * (steps * (shared ? 4.2 : 5.5) + share * (c.has_ep ? 8.5 : 8.8) + 7.0);
 }
 
 // Segments longest first, unless all of them run at once.  In the order of the documents a long one that starts late is waited for at the end:

@@ -149,3 +149,41 @@ def test_a_chain_shared_by_two_ctas(lens, vfirst):
             assert torch.isfinite(t.view(torch.bfloat16) if k in ("h", "Vd", "dh", "dVd") else t).all(), k
             for r in range(times):
                 assert torch.equal(whole[k][r * t.shape[0]:(r + 1) * t.shape[0]].view(torch.int32), t.view(torch.int32)), (k, r, transition)
+
+
+# chunks of the documents, v-heads, norm, backward pass -> output in a kernel of its own.  148 SMs; faster by (us, fused and separate) ...
+@pytest.mark.parametrize("chunks,HV,norm,train,apart", [
+    ((47, 32, 24, 16, 11), 16, True, True, True),          # 420, 377: more chains than half the SMs, but the longest sets the time
+    ((32, *[8] * 12), 16, True, True, True),               # 307, 285
+    ((48, *[1] * 12), 8, True, False, True),               # 246, 209
+    ((48, *[1] * 12), 8, False, True, True),               # 231, 207
+    ((48, *[1] * 12), 8, False, False, False),             # without a norm and forward only the fused step is no longer than that of the state alone
+    ((24,) * 5, 16, True, True, False),                    # 279, 291: equal chains
+    ((24,) * 8, 16, True, False, False),                   # 317, 416
+    ((24,) * 4, 16, True, True, True),                     # 258, 242: chains that two CTAs share
+    ((24,) * 4, 16, True, False, False),                   # 219, 236
+])
+def test_output_in_the_chain_or_apart(chunks, HV, norm, train, apart):
+    """The faster one also where chains are of unequal length: gate, WY preparation and chain are three launches, a separate output is one more.  Either way each
+    document has the bits of its own call."""
+    from mogankda_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("measured on 148 SMs")
+    lens = [64 * n - 3 for n in chunks]
+    cu = [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, _, _, opts, epi = make_inputs(T=cu[-1], HK=HV // 2, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi="silu" if norm else None, h0=False, seed=53)
+    assert not get_layout(1, cu[-1], opts["cu_seqlens"], lv["q"].device, 32, HV).segmented
+
+    def call(lv, cu):
+        with torch.set_grad_enabled(train):
+            norm_ = dict(weight=lv["ep_w"], gate=lv["ep_gate"], act=epi, eps=1e-6) if norm else None
+            before = _lib.launch_count()
+            o, ht = mk.chunk_kda(lv["q"].detach().requires_grad_(train), lv["k"], lv["v"], lv["g"], lv["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"],
+                                 output_norm=norm_, **dict(opts, cu_seqlens=cu))
+            return o.detach(), ht.detach(), _lib.launch_count() - before
+    o, ht, launches = call(lv, opts["cu_seqlens"])
+    assert launches == 3 + apart
+    for d in (0, len(lens) - 1):
+        s, e = cu[d], cu[d + 1]
+        one = call({k: (t[:, s:e].contiguous() if t.dim() >= 3 and t.shape[1] == cu[-1] else t) for k, t in lv.items()}, None)
+        assert torch.equal(o[:, s:e], one[0]) and torch.equal(ht[d:d + 1], one[1]), d
