@@ -270,10 +270,9 @@ def test_activation_checkpointing_frees_the_intermediates(T, epi):
     f, q, grads = _training_call(T, epi, 109)
     ref = grads(*f(q))
     gc.collect()
-    asked_for = lambda: torch.cuda.memory_stats()["requested_bytes.all.current"]       # noqa: E731  (the blocks may be up to 1 MB larger, as the tests before left them)
-    before = asked_for()
+    before = torch.cuda.memory_allocated()
     o, ht = checkpoint(f, q, use_reentrant=False)
-    held = asked_for() - before - o.numel() * o.element_size() - ht.numel() * 4
+    held = torch.cuda.memory_allocated() - before - o.numel() * o.element_size() - ht.numel() * 4
     assert held < 1 << 16, held
     for a, b in zip(ref, grads(o, ht)):
         assert torch.equal(a, b)
