@@ -141,11 +141,14 @@ static_assert(STEP_MAX <= WARPS, "a warp prepares one token");
 struct Shared {
     uint64_t known[2], full[2], empty[2];                  // what the item is | its state has landed | has been read
     struct { int item, start, len; } info[4];              // item < 0: no more
+    int gave_up;                                           // a wait of a compute warp has
     __align__(16) float k[STEP_MAX][DK], q[STEP_MAX][DK], d[STEP_MAX][DK], v[STEP_MAX][DV], o[STEP_MAX][DV], beta[STEP_MAX];
 };
 constexpr int SMEM = 2 * STATE * 4 + (int)sizeof(Shared);
 static_assert(SMEM <= 232448, "shared memory of one CTA");
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+// What the items are, and that there are no more, stands behind a wait: one that gives up ends the walk, for all lanes of its warp
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, umma::mbar_wait(bar, parity)); }
 
 // Four elements as they lie in memory, widened where they are used
 __device__ __forceinline__ void ldraw4(const void* base, int dtype, size_t idx, uint4& r) {
@@ -159,11 +162,12 @@ __device__ __forceinline__ float4 widen4(const uint4& r, int dtype) {
 }
 }  // namespace st
 
-// Items and their states, ahead of the compute warps
+// Items and their states, ahead of the compute warps.  Returns once no copy is on its way into shared memory
 __device__ __forceinline__ void step_load(const MkdaStepFwd& p, float* states, st::Shared& sh, int lane) {
     using namespace st;
     const int HV = p.L.HV, items = p.N * HV;
     int j = 0;
+    auto landed = [&](int i) { if (i >= 0) (void)umma::mbar_wait(&sh.full[i & 1], (i >> 1) & 1); };
     for (int it = blockIdx.x;; it += gridDim.x) {
         int start = 0, len = 0;
         if (it < items) {
@@ -172,12 +176,12 @@ __device__ __forceinline__ void step_load(const MkdaStepFwd& p, float* states, s
             if (p.short_only && (chunks != 1 || len > STEP_MAX)) continue;
         }
         const int s = j & 1;
-        if (j >= 2) umma::mbar_wait(&sh.empty[s], ((j - 2) >> 1) & 1);
+        if (j >= 2 && !wait_warp(&sh.empty[s], ((j - 2) >> 1) & 1)) break;
         if (lane == 0) {
             sh.info[j & 3] = {it < items ? it : -1, start, len};
             umma::arrive(&sh.known[s]);
         }
-        if (it >= items) return;
+        if (it >= items) break;
         if (!p.h0) {
             if (lane == 0) umma::arrive(&sh.full[s]);
         } else {
@@ -189,6 +193,8 @@ __device__ __forceinline__ void step_load(const MkdaStepFwd& p, float* states, s
         }
         ++j;
     }
+    landed(j - 2);
+    landed(j - 1);
 }
 
 __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaStepFwd p) {
@@ -199,6 +205,7 @@ __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaS
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31, HV = p.L.HV, HK = p.L.HK, G = HV / HK;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) { umma::mbar_init(&sh.known[i], 1); umma::mbar_init(&sh.full[i], 1); umma::mbar_init(&sh.empty[i], WARPS); }
+        sh.gave_up = 0;
         umma::fence_barrier_init();
     }
     __syncthreads();
@@ -211,8 +218,13 @@ __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaS
     uint4 rk, rq, rv, rx, rz;
     float rb = 0.f;
     int item = -1, start = 0, len = 0;
+    volatile int* gave_up = &sh.gave_up;                   // written between two block-wide barriers, read behind the second: all compute warps leave together
     auto request = [&](int j) {                            // item j: its tokens
-        umma::mbar_wait(&sh.known[j & 1], (j >> 1) & 1);
+        item = -1;
+        if (!wait_warp(&sh.known[j & 1], (j >> 1) & 1)) {
+            *gave_up = 1;
+            return;
+        }
         item = sh.info[j & 3].item; start = sh.info[j & 3].start; len = sh.info[j & 3].len;
         if (item < 0 || t >= len) return;
         const int h = item % HV;
@@ -224,7 +236,8 @@ __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaS
         rb = ld1(p.beta, p.beta_dtype, th);
     };
     request(0);
-    for (int j = 0; item >= 0; ++j) {
+    sync_compute();
+    for (int j = 0, end = *gave_up; item >= 0 && !end; ++j) {
         const int h = item % HV, n_tok = len, first = start;
         const size_t so = (size_t)item * DK * DV;
         float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -256,14 +269,15 @@ __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaS
         }
         sync_compute();
         float S[4][8];                                     // channel 4 lane + i, value 8 warp + v
-        umma::mbar_wait(&sh.full[j & 1], (j >> 1) & 1);
+        const bool here = umma::mbar_wait(&sh.full[j & 1], (j >> 1) & 1);
+        if (!here) *gave_up = 1;
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
             const float4 a = p.h0 ? *reinterpret_cast<const float4*>(states + (j & 1) * STATE + (8 * warp + v) * DK + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
             S[0][v] = a.x; S[1][v] = a.y; S[2][v] = a.z; S[3][v] = a.w;
         }
         __syncwarp();
-        if (lane == 0) umma::arrive(&sh.empty[j & 1]);
+        if (here && lane == 0) umma::arrive(&sh.empty[j & 1]);
         request(j + 1);
         for (int s = 0; s < n_tok; ++s) {
             const float4 d4 = *reinterpret_cast<const float4*>(sh.d[s] + 4 * lane), k4 = *reinterpret_cast<const float4*>(sh.k[s] + 4 * lane),
@@ -295,6 +309,7 @@ __global__ void __launch_bounds__(st::THREADS, 1) step_fwd_vk_kernel(const MkdaS
                 *reinterpret_cast<float4*>(p.ht + so + (size_t)(8 * warp + v) * DK + 4 * lane) = make_float4(S[0][v], S[1][v], S[2][v], S[3][v]);
         }
         sync_compute();
+        end = *gave_up;
         if (t < n_tok) {                                   // output rows: lane = 4 values
             float4 o = *reinterpret_cast<const float4*>(&sh.o[t][4 * lane]);
             if (p.has_norm) {

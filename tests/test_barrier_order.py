@@ -462,3 +462,95 @@ def test_step_fwd_vk():
     dims = _slots("step.cu", "Shared")
     assert step(dims).late_waits() == []
     assert step({k: [] for k in dims}).late_waits() != []
+
+
+def _step_with_a_failure(n, fails):
+    """step_fwd_vk over n items with two compute warps.  `fails`: (agent, i): its i-th wait gives up; what can go on no more gives up too, except at the block-wide
+    barrier, where it would hang.  Barriers go by parity, as they do.  Returns the waits made by each agent."""
+    done, info, state, waits = {}, [None] * 4, {"gave_up": False}, {}
+
+    def arrive(bar, count=1):
+        done[bar] = done.get(bar, 0) + 1 / count
+
+    def load():
+        j = 0
+        for it in range(n + 1):
+            if j >= 2 and not (yield ("empty", j - 2)):
+                break
+            info[j & 3] = (j, it if it < n else -1)
+            arrive(("known", j & 1))
+            if it == n:
+                break
+            arrive(("full", j & 1))
+            j += 1
+        for i in (j - 2, j - 1):
+            if i >= 0:
+                yield ("full", i)
+
+    def compute():
+        def request(j):
+            if not (yield ("known", j)):
+                state["gave_up"] = True
+                return -1
+            assert info[j & 3][0] == j
+            return info[j & 3][1]
+        item = yield from request(0)
+        yield "sync"
+        j = 0
+        while item >= 0 and not state["gave_up"]:
+            assert item == j
+            yield "sync"
+            here = yield ("full", j)
+            if here:
+                arrive(("empty", j & 1), 2)
+            else:
+                state["gave_up"] = True
+            item = yield from request(j + 1)
+            yield "sync"
+            j += 1
+
+    agents = {"load": load(), "a": compute(), "b": compute()}
+    at = {name: next(a) for name, a in agents.items()}
+
+    def step(name, value):
+        try:
+            at[name] = agents[name].send(value)
+        except StopIteration:
+            del at[name]
+    while at:
+        moved = False
+        for name in list(at):
+            if at[name] == "sync":
+                continue
+            bar, k = at[name]
+            if (name, waits.get(name, 0)) == fails:
+                ok = False
+            elif int(done.get((bar, k & 1), 0) + 1e-9) & 1 != (k >> 1) & 1:
+                ok = True
+            else:
+                continue
+            waits[name] = waits.get(name, 0) + 1
+            step(name, ok)
+            moved = True
+        if not moved and all(at.get(w) == "sync" for w in "ab"):
+            for w in "ab":
+                step(w, None)
+            moved = True
+        if not moved:
+            late = [name for name in at if at[name] != "sync"]
+            assert late, f"{fails}: the compute warps disagree on the number of block-wide barriers: {at}"
+            for name in late:
+                waits[name] = waits.get(name, 0) + 1
+                step(name, False)
+    return waits
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7])
+def test_step_fwd_vk_comes_to_its_end_when_a_wait_gives_up(n):
+    """Whichever it is: no warp reads what an item is without having been told, all compute warps leave behind the same block-wide barrier, and what the kernel does
+    hangs on no wait whose outcome it drops."""
+    for name, waits in _step_with_a_failure(n, None).items():
+        for i in range(waits):
+            _step_with_a_failure(n, (name, i))
+    code = open(os.path.join(CSRC, "step.cu")).read()
+    assert "mbar_wait" in code and not re.findall(r"(?:[;{}]|(?<!\(void)\))\s*umma::mbar_wait\(", code)         # (void): it is over either way
