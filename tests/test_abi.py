@@ -216,3 +216,21 @@ def test_reverse_chain_on_rows_refuses_other_rows(lib):
         assert call() == _lib.MKDA_ERR_ARG, f
         setattr(p, f, good)
     assert lib.mkda_bwd_dh_rows(None, None, None) == _lib.MKDA_ERR_ARG
+
+
+def test_chunk_backward_on_rows_of_dO_refuses_other_rows(lib):
+    """Without chunks: nothing is launched where the arguments are accepted.  dO as rows or as tiles; one of them there has to be."""
+    from mogankda_b200 import _lib
+    p = _lib.STRUCTS["MkdaBwdChunk"]()
+    p.L.HK, p.L.HV, p.L.NC, p.qkv_dtype = 1, 2, 0, _lib.MKDA_BF16
+    for f in ("q", "k", "v", "g_c", "beta", "A", "h", "dh", "Vd", "dO_t", "dVd_t", "dq_v", "dk_v", "dgp", "dbeta", "dv"):
+        setattr(p, f, 0x30000)
+    call = lambda d_o: lib.mkda_bwd_chunk_rows(ctypes.byref(p), d_o, None, None, None)  # noqa: E731
+    assert call(0x30000) == call(None) == 0
+    assert call(0x30002) == call(0x30008) == _lib.MKDA_ERR_ARG
+    for dt in (_lib.MKDA_F16, _lib.MKDA_F32):
+        p.qkv_dtype = dt
+        assert call(0x30000) == _lib.MKDA_ERR_ARG and call(None) == 0
+    p.qkv_dtype, p.dO_t = _lib.MKDA_BF16, None
+    assert call(0x30000) == 0 and call(None) == _lib.MKDA_ERR_ARG
+    assert lib.mkda_bwd_chunk(ctypes.byref(p), None) == _lib.MKDA_ERR_ARG

@@ -147,3 +147,42 @@ def test_rows_of_dO(scalar, lens, times, finish, monkeypatch):
             assert torch.equal(a.view(torch.int32) if a.dtype == torch.float32 else a, b.view(torch.int32) if b.dtype == torch.float32 else b), i
     if finish:
         assert torch.equal(got_q.view(-1), fin[0].view(-1)) and torch.equal(got_k.view(-1), fin[1].view(-1))
+
+
+@pytest.mark.parametrize("times", [1, 12])
+@pytest.mark.parametrize("lens", [(1, 15, 64, 65, 63, 128), (64, 128, 192)])
+@pytest.mark.parametrize("scalar", [False, True])
+def test_rows_of_dO_with_v_heads_spread_and_without_tiles(scalar, lens, times, monkeypatch):
+    """The bits of the tiles also with a dq and dk tile per v-head, and where no chunk is ragged without any tiles of dO."""
+    import ctypes
+    from mogankda_b200 import _lib, ops
+    full, lens, HK, HV = all(n % 64 == 0 for n in lens), lens * times, 2, 4
+    T, cu = sum(lens), [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, do, _, opts, _ = make_inputs(T=T, HK=HK, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="precomputed", scalar=scalar, l2=False, epi=None, h0=False, seed=73)
+    lay = get_layout(1, T, opts["cu_seqlens"], lv["q"].device, 32)
+    g_c, be = ops.gate_cumsum_fwd(lay, lv["g"], "precomputed", None, None, -5.0, HV, beta_raw=lv["beta"], beta_sigmoid=True, beta_scale=2.0)
+    A, Aqk, nw, u, kbar, qs, gl = ops.intra_fwd(lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, 128 ** -0.5, HK, HV, scalar_gate=scalar)
+    h, Vd, _, _ = ops.recur_fwd(lay, nw, u, kbar, gl, HK, HV)
+    do = do.to(torch.bfloat16).contiguous()
+    lib, both = _lib.load(), []
+
+    def call(name, p, *args):
+        if name == "mkda_bwd_chunk":
+            p.per_v_head, p.dq_v, p.dk_v = 1, dq.data_ptr(), dk.data_ptr()
+        if rows and full:
+            p.dO_t = None
+        if name == "mkda_bwd_dh_ordered":
+            assert (lib.mkda_bwd_dh_rows if rows else lib.mkda_bwd_dh_ordered)(ctypes.byref(p), *args) == 0
+        elif rows:
+            assert lib.mkda_bwd_chunk_rows(ctypes.byref(p), do.data_ptr(), None, None, *args) == 0
+        else:
+            assert lib.mkda_bwd_chunk(ctypes.byref(p), *args) == 0
+    monkeypatch.setattr(_lib, "call", call)
+    for rows in (False, True):
+        dq, dk = (torch.full((lay.NC, HV, 64, 128), float("nan"), device="cuda") for _ in range(2))
+        dh, dVd, dO, dh0 = ops.bwd_dh(lay, do, kbar, qs, gl, Aqk, nw, HK, HV, want_dh0=True)
+        out = ops.bwd_chunk(lay, lv["q"], lv["k"], lv["v"], None, None, g_c, be, A, h, dh, Vd, dO, dVd, 128 ** -0.5, HK, HV, lv["beta"], True, 2.0, scalar_gate=scalar)
+        both.append((dh, dVd, dh0, dq, dk, *out[2:]))
+    for i, (a, b) in enumerate(zip(*both)):
+        assert torch.equal(a.view(torch.int32) if a.dtype == torch.float32 else a, b.view(torch.int32) if b.dtype == torch.float32 else b), i
+    assert not torch.isnan(both[1][3]).any() and not torch.isnan(both[1][4]).any()
