@@ -80,13 +80,14 @@ bool gate_in_intra(const Call& c) { return (int64_t)c.NC * c.HV <= at::cuda::get
 // separate, x 16 heads: documents of 3000, 2000, 1500, 1000 and 692 tokens 420 and 377, one of 2048 and 12 of 512 307 and 285, five of 1536 equal ones
 // 279 and 291; x 8 heads one of 1024 and 30 of 64 137 and 111.  (A line for equal chains alone, all calls of more than half as many chains as SMs fused: 53 of 656 on the
 // wrong side by up to 51 %; this one 4, by up to 5 %.)  Forward only the separate kernels allocate states and Vd, 96 KB per chunk and head, that the fused one
-// never writes: 3 % has to be gained for that.
+// never writes: 3 % has to be gained for more than 64 MB of them.  (For any number: two documents of 256 tokens x 16 heads 38.2 us instead of 36.8.)
 bool output_in_chain(const Call& c, bool need_bwd) {
     const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount, share = (double)c.NC * c.HV / sms;
     const bool shared = 2.0 * c.NS * c.HV <= sms;
     const double fused = c.has_ep ? (need_bwd ? (shared ? 11.4 : 9.8) : (shared ? 7.8 : 7.3)) : (need_bwd ? (shared ? 7.9 : 6.8) : (shared ? 4.9 : 5.5));
     const double steps = shared ? c.chain : std::max((double)c.chain, share);
-    return steps * fused <= (need_bwd ? 1.0 : 1.03) * (steps * (shared ? 4.2 : 5.5) + share * (c.has_ep ? 8.5 : 8.8) + 7.0);
+    const bool costly = !need_bwd && c.tiles(MKDA_STATE_TILE_BYTES + MKDA_CHUNK_TILE_BYTES) > 64 << 20;
+    return steps * fused <= (costly ? 1.03 : 1.0) * (steps * (shared ? 4.2 : 5.5) + share * (c.has_ep ? 8.5 : 8.8) + 7.0);
 }
 
 // Segments longest first, unless all of them run at once.  In the order of the documents a long one that starts late is waited for at the end:

@@ -187,3 +187,18 @@ def test_output_in_the_chain_or_apart(chunks, HV, norm, train, apart):
         s, e = cu[d], cu[d + 1]
         one = call({k: (t[:, s:e].contiguous() if t.dim() >= 3 and t.shape[1] == cu[-1] else t) for k, t in lv.items()}, None)
         assert torch.equal(o[:, s:e], one[0]) and torch.equal(ht[d:d + 1], one[1]), d
+
+
+@pytest.mark.parametrize("chunks,HV", [((4,) * 4, 8), ((4, 4), 16)])       # 38.1 us fused and 36.6 separate; 38.2, 36.8
+def test_output_apart_in_small_calls(chunks, HV):
+    """States and Vd that only the separate kernels allocate are no reason to stay with the slower one where they are a few MB."""
+    from mogankda_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("measured on 148 SMs")
+    cu = [0, *torch.tensor([64 * n for n in chunks]).cumsum(0).tolist()]
+    lv, _, _, opts, epi = make_inputs(T=cu[-1], HK=HV // 2, HV=HV, cu=tuple(cu), dtype=torch.bfloat16, gate="kimi", epi="silu", h0=False, seed=61)
+    before = _lib.launch_count()
+    with torch.no_grad():
+        mk.chunk_kda(lv["q"], lv["k"], lv["v"], lv["g"], lv["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"],
+                     output_norm=dict(weight=lv["ep_w"], gate=lv["ep_gate"], act=epi, eps=1e-6), **opts)
+    assert _lib.launch_count() - before == 3               # gate and WY preparation, chain, output
