@@ -73,21 +73,23 @@ bool spread_v_heads(const Call& c) {
 bool gate_in_intra(const Call& c) { return (int64_t)c.NC * c.HV <= at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
 
 // Output in the kernel of the state chain, or in one of its own?  A separate one has all SMs where a few chains, or the last steps of a few long ones among many
-// short, leave some idle; with at most half as many chains as SMs two CTAs share a chain of it besides.  In units of 1000 SM cycles, the shared
-// ones fitted to 280 equal batches of 4 to 128 chains x 1 to 64 steps, the others to 656 equal and unequal ones of 60 to 700 chains x 1 to 48, with and without norm and
-// backward pass: a step of the chain without the output takes 4.2 shared and 5.5 not, with it 4.9 and 5.5 (7.9 and 6.8 if a backward pass follows), with the norm 7.8 and 7.3 (11.4 and 9.8); the separate output 8.5 with the norm and 8.8
-// without per chunk and SM, and 7 to launch.  What takes the steps is the longest chain, or the even share of all.  Times in us with norm and backward pass, fused and
-// separate, x 16 heads: documents of 3000, 2000, 1500, 1000 and 692 tokens 420 and 377, one of 2048 and 12 of 512 307 and 285, five of 1536 equal ones
-// 279 and 291; x 8 heads one of 1024 and 30 of 64 137 and 111.  (A line for equal chains alone, all calls of more than half as many chains as SMs fused: 53 of 656 on the
-// wrong side by up to 51 %; this one 4, by up to 5 %.)  Forward only the separate kernels allocate states and Vd, 96 KB per chunk and head, that the fused one
-// never writes: 3 % has to be gained for more than 64 MB of them.  (For any number: two documents of 256 tokens x 16 heads 38.2 us instead of 36.8.)
-bool output_in_chain(const Call& c, bool need_bwd) {
+// short, leave some idle; with at most half as many chains as SMs two CTAs share a chain of it besides.  In units of 1000 SM cycles a step of the chain without the
+// output takes 4.2 shared and 5.5 not, with it what `step` says; the separate output takes 8.5 with a norm and 8.8 without per chunk and SM, and 7 to launch (8.4 with a 32-bit gate).  What takes the
+// steps is the longest chain, or the even share of all.  Fitted to 656 equal and unequal batches of 60 to 700 chains x 1 to 48 steps and, each with and without backward
+// pass, norm and 16-bit types, 266 of 4 to 400 chains.  Of the latter at most 3 in 266 are on the wrong side by 2 % or more, by up to 7 %.
+// Times in us with norm and backward pass, fused and separate, x 16 heads: documents of 3000, 2000, 1500, 1000 and 692 tokens 421 and 374, one of 2048 and 12
+// of 512 345 and 338, five of 1536 279 and 291; x 8 heads one of 1024 and 30 of 64 137 and 110.
+// The rows of a 32-bit gate have no place in the shared memory of the fused kernel, whose epilogue fetches them from where they are, 16 at a time: 20 k cycles for
+// a step of 10.  Forward only, x 16 heads, one document of 48 chunks and 30 of one 674 and 285 us, six of 48 chunks with a backward pass 1021 and 621.
+bool output_in_chain(const Call& c, bool need_bwd, bool gate_32_bits) {
+    static const double step[3][2][2] = {{{7.8, 7.3}, {11.4, 9.8}}, {{12.6, 19.2}, {12.6, 21.0}}, {{4.9, 5.5}, {7.9, 7.2}}};      // 16-bit gate, 32-bit, no norm; backward pass; not shared
     const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount, share = (double)c.NC * c.HV / sms;
     const bool shared = 2.0 * c.NS * c.HV <= sms;
-    const double fused = c.has_ep ? (need_bwd ? (shared ? 11.4 : 9.8) : (shared ? 7.8 : 7.3)) : (need_bwd ? (shared ? 7.9 : 6.8) : (shared ? 4.9 : 5.5));
-    const double steps = shared ? c.chain : std::max((double)c.chain, share);
+    const double steps = shared ? c.chain : std::max((double)c.chain, share), fused = step[c.has_ep ? gate_32_bits : 2][need_bwd][!shared];
+    // forward only the separate kernels allocate states and Vd, 96 KB per chunk and head, that the fused one never writes: 3 % has to be gained for more than 64 MB of
+    // them (for any number: two documents of 256 tokens x 16 heads 38.2 us instead of 36.8)
     const bool costly = !need_bwd && c.tiles(MKDA_STATE_TILE_BYTES + MKDA_CHUNK_TILE_BYTES) > 64 << 20;
-    return steps * fused <= (costly ? 1.03 : 1.0) * (steps * (shared ? 4.2 : 5.5) + share * (c.has_ep ? 8.5 : 8.8) + 7.0);
+    return steps * fused <= (costly ? 1.03 : 1.0) * (steps * (shared ? 4.2 : 5.5) + share * (c.has_ep ? 8.5 : 8.8) + (gate_32_bits ? 8.4 : 7.0));
 }
 
 // Segments longest first, unless all of them run at once.  In the order of the documents a long one that starts late is waited for at the end:
@@ -142,7 +144,7 @@ std::pair<Tensor, Tensor> run_forward(const Call& c, const Inputs& in, bool need
     keep.want(&s.kbar, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.qs, c.tiles(MKDA_CHUNK_TILE_BYTES));
     keep.want(&s.gl, c.tiles(512));
-    const bool fused = output_in_chain(c, need_bwd);
+    const bool fused = output_in_chain(c, need_bwd, c.has_ep && in.ep_gate.scalar_type() == at::kFloat);
     if (need_bwd || !fused) {
         keep.want(&s.h, c.tiles(MKDA_STATE_TILE_BYTES));
         keep.want(&s.Vd, c.tiles(MKDA_CHUNK_TILE_BYTES));

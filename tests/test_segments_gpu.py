@@ -202,3 +202,36 @@ def test_output_apart_in_small_calls(chunks, HV):
         mk.chunk_kda(lv["q"], lv["k"], lv["v"], lv["g"], lv["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"],
                      output_norm=dict(weight=lv["ep_w"], gate=lv["ep_gate"], act=epi, eps=1e-6), **opts)
     assert _lib.launch_count() - before == 3               # gate and WY preparation, chain, output
+
+
+# ... and with a 32-bit gate (us, fused and separate)
+@pytest.mark.parametrize("chunks,HV,train,apart", [
+    ((48, *[1] * 30), 16, False, True),                    # 674, 285
+    ((48,) * 6, 16, True, True),                           # 1021, 621
+    ((16,) * 8, 8, False, True),                           # chains that two CTAs share
+    ((1,) * 2, 4, False, False),                           # one step: 27.5, 28.9
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_output_apart_from_the_chain_with_a_32_bit_gate(dtype, chunks, HV, train, apart):
+    """The fused kernel has no place for the rows of such a gate and fetches them while everything waits.  The gate's type decides, not that of q, k and v; the bits are
+    those of each document's own call."""
+    from mogankda_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("measured on 148 SMs")
+    lens = [64 * n - 3 for n in chunks]
+    cu = [0, *torch.tensor(lens).cumsum(0).tolist()]
+    lv, _, _, opts, epi = make_inputs(T=cu[-1], HK=HV // 2, HV=HV, cu=tuple(cu), dtype=dtype, gate="kimi", epi="silu", h0=False, seed=59)
+
+    def call(lv, cu):
+        with torch.set_grad_enabled(train):
+            before = _lib.launch_count()
+            o, ht = mk.chunk_kda(lv["q"].detach().requires_grad_(train), lv["k"], lv["v"], lv["g"], lv["beta"], A_log=lv["A_log"], dt_bias=lv["dt_bias"],
+                                 output_norm=dict(weight=lv["ep_w"], gate=lv["ep_gate"].float(), act=epi, eps=1e-6), **dict(opts, cu_seqlens=cu))
+            return o.detach(), ht.detach(), _lib.launch_count() - before
+    o, ht, launches = call(lv, opts["cu_seqlens"])
+    one_kernel = sum(chunks) * HV <= 148                   # gate and WY preparation
+    assert launches == 3 - one_kernel + apart
+    for d in (0, len(lens) - 1):
+        s, e = cu[d], cu[d + 1]
+        one = call({k: (t[:, s:e].contiguous() if t.dim() >= 3 and t.shape[1] == cu[-1] else t) for k, t in lv.items()}, None)
+        assert torch.equal(o[:, s:e], one[0]) and torch.equal(ht[d:d + 1], one[1]), d
