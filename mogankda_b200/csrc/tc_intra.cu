@@ -212,10 +212,10 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
                 store_split8(tile, tile + 16384, 128, (warp & 3) * 32 + lane, 2 * (warp >> 2) + m, o);
             }
         };
-        umma::wait_mma<true>(&sh.mmN, it & 1);
+        umma::wait_mma(&sh.mmN, it & 1);
         stage(NW, base + BK, -1.f);
         umma::signal(&sh.nwReady, lane);
-        umma::wait_mma<true>(&sh.mmU, it & 1);
+        umma::wait_mma(&sh.mmU, it & 1);
         stage(U, base + UT, 1.f);
         umma::signal(&sh.uReady, lane);
     };
@@ -231,7 +231,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
             if (gate.A_log) E = expf(gate.A_log[h]);
             if (gate.dt_bias) bias = gate.dt_bias[h * 128 + (tid & 127)];
         }
-        umma::mbar_wait<true>(&sh.ldin, par);
+        umma::mbar_wait(&sh.ldin, par);
         const int len = sh.info[it & 3].len;
         if constexpr (GATED<G> && !SCALAR) {
             const size_t first = ((size_t)sh.info[0].start * p.L.HV + sh.info[0].h) * 128 + (tid & 127);
@@ -251,7 +251,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
             if (!SCALAR) {
                 const float* g = reinterpret_cast<const float*>(base + RAW_G) + k8 * 8;
                 lds8_swapped(g + rr * 128, odd, vg[hf]);
-                if (it && hf == 0) umma::mbar_wait<true>(&sh.hand, par ^ 1);             // nobody reads the previous item's last row any more
+                if (it && hf == 0) umma::mbar_wait(&sh.hand, par ^ 1);             // nobody reads the previous item's last row any more
                 if ((r & 15) == 0) sts_halves(sh.ga[r >> 4], k8, vg[hf]);
                 if (r == len - 1) sts_halves(sh.ga[4], k8, vg[hf]);
                 if ((r & 15) == 0 && r >= 32) {
@@ -311,7 +311,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
                 unpack8<DT>(wk[hf], x8);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) { x8[e] = mul2(x8[e], both(COL_DOWN)); t8[e] = mul2(x8[e], ex2f2_(mul2(d[e], both(-1.f)))); }
-                if (it && hf == 0) umma::mbar_wait<true>(&sh.khFree, par ^ 1);           // the tiles under the column tiles have left
+                if (it && hf == 0) umma::mbar_wait(&sh.khFree, par ^ 1);           // the tiles under the column tiles have left
                 store_split8(base, base + KC_BYTES, KC_ROWS, kc_row(I0) + r, k8, t8);
 #pragma unroll
                 for (int I = 1; I < 4; ++I) {
@@ -331,7 +331,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
         }
         // ---- L2 scales, while the products run: they are applied to what comes out (Gamma and Q K^T are bilinear in the rows) and to the tiles
         // below.  Four sums (k, q of two half rows) over eight threads; lane bit 2 ends up choosing the half, bit 1 between k and q ----
-        if (SCALAR && it) umma::mbar_wait<true>(&sh.khFree, par ^ 1);     // Y has used the previous item's
+        if (SCALAR && it) umma::mbar_wait(&sh.khFree, par ^ 1);     // Y has used the previous item's
         if (p.l2) {
             float t[2][2];
 #pragma unroll
@@ -388,8 +388,8 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
         __syncwarp();
         if (lane == 0) umma::arrive(&sh.rows);
         if (it) read_out(it - 1);
-        umma::wait_mma<true>(&sh.mm1[par], (it >> 1) & 1);
-        umma::mbar_wait<true>(&sh.rows, par);
+        umma::wait_mma(&sh.mm1[par], (it >> 1) & 1);
+        umma::mbar_wait(&sh.rows, par);
         // ---- over the dead operands: the state kernels' scaled operands, kbar = k 2^(gL - g) (gL = last valid row) and scale q 2^g; beta k 2^g for Y ----
         const float gLs = SCALAR ? gs[CH - 1] : 0.f;
 #pragma unroll
@@ -413,7 +413,7 @@ __device__ __forceinline__ void intra_x(const MkdaIntraFwd& p, const G& gate, ui
 #pragma unroll
             for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(t8[e], sq) : mul2(mul2(t8[e], sq), e8[e]);
             store_split8(base + QS, base + QS + 16384, 64, r, k8, t8);
-            if (it && hf == 0) umma::mbar_wait<true>(&sh.bkFree, par ^ 1);               // nw^T of the previous item has left
+            if (it && hf == 0) umma::mbar_wait(&sh.bkFree, par ^ 1);               // nw^T of the previous item has left
 #pragma unroll
             for (int e = 0; e < 4; ++e) t8[e] = SCALAR ? mul2(x8[e], sb) : mul2(mul2(x8[e], sb), e8[e]);
             store_split8(base + BK, base + BK + 16384, 64, r, k8, t8);
@@ -473,7 +473,7 @@ __device__ __forceinline__ void invert_unit_lower(float* M, float* T, uint64_t* 
             *reinterpret_cast<float2*>(D + (24 + g) * LD + 8 * nt + 2 * t) = make_float2(-z[nt][2], -z[nt][3]);
         }
     }
-    if (it) umma::mbar_wait<true>(free, (it & 1) ^ 1);
+    if (it) umma::mbar_wait(free, (it & 1) ^ 1);
     sync_y();
     // 32 x 32 block (rows 32.., columns 0..31): a tile of 16 x 8 per warp
     const int m0 = 16 * (y >> 2), n0 = 8 * (y & 3);
@@ -502,8 +502,8 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
         const float* gs = &sh.ga[0][0] + par * CH;
         // ---- I + L and Aqk from the accumulators ----
         // per channel: warp quadrant = row block (16 rows of Gamma, then 16 rows of Q K^T); scalar gate: 64 rows of K K^T, then of Q K^T
-        umma::mbar_wait<true>(&sh.rows, par);
-        umma::wait_mma<true>(&sh.mm1[par], (it >> 1) & 1);
+        umma::mbar_wait(&sh.rows, par);
+        umma::wait_mma(&sh.mm1[par], (it >> 1) & 1);
         const int len = sh.info[it & 3].len;
         {
             const int i = SCALAR ? (q & 1) * 32 + lane : 16 * q + (lane & 15);
@@ -580,7 +580,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
         // from global memory, there is no place for them (6 k packed tokens x 32 heads all the same 344 -> 243 us by the split into two groups)
         constexpr int N = 4;
         uint32_t lo[N][4];
-        if (DT != MKDA_F32) umma::mbar_wait<true>(&sh.fullV, par);
+        if (DT != MKDA_F32) umma::mbar_wait(&sh.fullV, par);
         Raw8 raw[N];
 #pragma unroll
         for (int n = 0; n < N; ++n) {
@@ -603,7 +603,7 @@ __device__ __forceinline__ void intra_y(const MkdaIntraFwd& p, uint8_t* base, ui
             *reinterpret_cast<uint4*>(base + V_ + umma::tile_chunk_offset(64, r, i & 15)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }
         umma::signal(&sh.opA, lane);
-        umma::wait_mma<true>(&sh.mmV, par);
+        umma::wait_mma(&sh.mmV, par);
 #pragma unroll
         for (int n = 0; n < N; ++n) {
             const int i = tid + YT * n;
@@ -628,7 +628,7 @@ __device__ __forceinline__ void intra_mm1(const MkdaIntraFwd& p, uint8_t* smem, 
     for (int it = 0; it < count; ++it) {
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-            umma::wait_mma<true>(&sh.op1[hf], it & 1);
+            umma::wait_mma(&sh.op1[hf], it & 1);
             uint8_t* base = fresh(smem);
             uint8_t* kq = base + KQ + hf * 16384;
             if (SCALAR) {      // D[m][j]: lanes 0..63 = K K^T rows, lanes 64..127 = Q K^T rows; columns j = K rows of the same tile
@@ -651,8 +651,8 @@ __device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, 
     const int count = item_count<ONE>(p.L);
     for (int it = 0; it < count; ++it) {
         const uint32_t par = it & 1;
-        umma::wait_mma<true>(&sh.hand, par);                      // beta k 2^g
-        umma::wait_mma<true>(&sh.opA, par);
+        umma::wait_mma(&sh.hand, par);                      // beta k 2^g
+        umma::wait_mma(&sh.opA, par);
         uint8_t* base = fresh(smem);
         const umma::Opnd a = umma::opnd_k(base + A_, base + A_ + 8192, 64), v = umma::opnd_mn(base + V_, nullptr, 64);
         auto product_nw = [&]() {
@@ -664,7 +664,7 @@ __device__ __forceinline__ void intra_mm3(const MkdaIntraFwd& p, uint8_t* smem, 
         // Of the last item nw comes first, under Y's writing of the low half (77 tokens 13.8 -> 13.4 us).  In front of other items that would hold up
         // what waits for u: 14 items per SM 123 -> 129 us
         if (it + 1 == count) product_nw();
-        umma::wait_mma<true>(&sh.opV, par);
+        umma::wait_mma(&sh.opV, par);
         umma::Opnd hi = a;
         hi.lo = 0;
         umma::gemm(tmem + U, v, hi, 128, 64, 64, 1u);
@@ -697,11 +697,11 @@ __device__ __forceinline__ void intra_copy_x(const MkdaIntraFwd& p, const G& gat
     for (int it = 0; w.valid(); ++it) {
         const size_t item = w.item();
         if (GATED<G>) w.c = w.NC; else w.next();
-        umma::mbar_wait<true>(&sh.mm1[it & 1], (it >> 1) & 1);    // the operands are dead
+        umma::mbar_wait(&sh.mm1[it & 1], (it >> 1) & 1);    // the operands are dead
         if (w.valid()) request_rows<DT, SCALAR>(gate, w, it + 1, maps, base, sh);
-        umma::mbar_wait<true>(&sh.acc, it & 1);
+        umma::mbar_wait(&sh.acc, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.Aqk) + item * umma::QUARTER_TILE_BYTES, base + AQ, umma::QUARTER_TILE_BYTES);
-        umma::mbar_wait<true>(&sh.hand, it & 1);
+        umma::mbar_wait(&sh.hand, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.kbar) + item * umma::CHUNK_TILE_BYTES, base + KB, umma::CHUNK_TILE_BYTES);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.qs) + item * umma::CHUNK_TILE_BYTES, base + QS, umma::CHUNK_TILE_BYTES);
         umma::bulk_store_wait_read();
@@ -723,9 +723,9 @@ __device__ __forceinline__ void intra_copy_y(const MkdaIntraFwd& p, const in::Ma
     for (uint32_t it = 0; w.valid(); ++it) {
         const size_t item = w.item();
         if (ONE) w.c = w.NC; else w.next();
-        umma::mbar_wait<true>(&sh.nwReady, it & 1);
+        umma::mbar_wait(&sh.nwReady, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.nw) + item * umma::CHUNK_TILE_BYTES, base + BK, umma::CHUNK_TILE_BYTES);
-        umma::mbar_wait<true>(&sh.uReady, it & 1);
+        umma::mbar_wait(&sh.uReady, it & 1);
         umma::bulk_store(reinterpret_cast<uint8_t*>(p.u) + item * umma::CHUNK_TILE_BYTES, base + UT, umma::CHUNK_TILE_BYTES);
         umma::bulk_store_wait_read_but<1>();
         umma::arrive(&sh.bkFree);

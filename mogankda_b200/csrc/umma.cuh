@@ -260,16 +260,13 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
     atomicExch(flag, 1u);
     return false;
 }
-template <bool CLOCK_FIRST = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     // Bounded by wall time (SM clock): ~70 ms for the first wait that fails on a device, ~35 us afterwards, so a broken
     // launch drains quickly instead of serialising one long timeout per CTA.  The flag stays set until
     // mkda_device_status_clear().  It is looked at only by a wait that has already taken ~35 us: read up front it put a global load, i.e.
     // 0.7 k cycles of latency and thousands under a saturated memory system, in front of every wait of every kernel.
     // The clock is read once a first attempt has failed: most waits are over when they are made, and those of a thread that issues products or copies
-    // follow one another (bwd_chunk 191 -> 180 us at the 1B shape, 241 -> 229 short documents; recur_fwd_pair 347 -> 327, chain_fwd 94 -> 88 and 144 -> 141).  Not in intra_fwd
-    // (CLOCK_FIRST), whose 24 warps wait longer than they issue: 40.2 us so and 39.5 with the clock first (fp16 4 x 1000 tokens), 119.4 and 118.0 (1B shape),
-    // 837 and 833 (32 k tokens x 32 heads), 16.0 and 15.8 (77 tokens x 16).  One attempt in the loop and the clock behind it is slower than either, in every kernel.
+    // follow one another (bwd_chunk 191 -> 180 us at the 1B shape, 241 -> 229 short documents; recur_fwd_pair 347 -> 327, chain_fwd 94 -> 88 and 144 -> 141).
     const uint32_t addr = smem_u32(bar);
     auto done = [&]() {
         uint32_t ok;
@@ -278,7 +275,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
             : "=r"(ok) : "r"(addr), "r"(parity), "r"(1000u) : "memory");
         return ok != 0;
     };
-    if (!CLOCK_FIRST && done()) return true;
+    if (done()) return true;
     const long long t0 = clock64();
     long long limit = 1ll << 16;
     for (;;) {
@@ -310,9 +307,8 @@ __device__ __forceinline__ void signal_tmem(uint64_t* bar, int lane) {
     __syncwarp();
     if (lane == 0) arrive(bar);
 }
-template <bool CLOCK_FIRST = false>
 __device__ __forceinline__ void wait_mma(uint64_t* bar, uint32_t parity) {
-    mbar_wait<CLOCK_FIRST>(bar, parity);
+    mbar_wait(bar, parity);
     fence_after_sync();
 }
 __device__ __forceinline__ bool elect_one() {
