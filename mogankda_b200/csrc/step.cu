@@ -3,10 +3,13 @@
 //   S <- diag(2^g) S        S <- S + k (beta (v - k^T S))        o = scale q^T S, then the optional gated RMSNorm
 // The state is read and written once and everything in between, gate and L2 norm included, stays on chip.  [K,V] states: one CTA per (sequence, v-head) with the
 // state in registers (thread = one v x 64 key channels).  [V,K] states: a kernel of its own (below).
-// What bounds it: 128 KB of state traffic per CTA.  The chunk path spends the same traffic several times over (operand tiles of 64 rows of
-// which a few are real, and five launches): 63 us of kernels for one token of 8 sequences x 32 heads, against 9 us here (33.5 MB of states).
-// Up to how many tokens: a token costs 1.6 us there, a chunk the same for any number of rows.  16 tokens, whole call with cold caches, here
-// and by chunks: 43 / 52 us (8 sequences x 32 heads), 221 / 316 us (64 x 32), 29 / 30 us (1 x 32); one token 18 / 50, 80 / 306, 14 / 30.
+// What bounds it: 128 KB of state traffic per (sequence, v-head).  The chunk path spends the same traffic several times over (operand tiles of 64 rows of
+// which a few are real, and three or four launches).
+// Up to how many tokens: a token costs time here, while a chunk takes the same for any number of rows.  Whole calls with cold caches, 32 heads, by steps / by chunks in us:
+//                        [K,V] states: 1 token      8          16          [V,K] states: 1       8           16
+//   one sequence                   14.3 / 31.7   18.5 / 31.7   28.7 / 31.7         12.3 / 33.8   16.4 / 33.8   20.4 / 33.8
+//   8                              18.4 / 50.0   28.7 / 50.2   43.0 / 50.2         18.4 / 54.3   26.6 / 54.3   36.9 / 54.3
+//   64                             79.9 / 269    137 / 269     223 / 273           67.6 / 302    123 / 306     197 / 310
 #include "common.cuh"
 #include "gate.cuh"
 #include "host.h"
@@ -133,8 +136,10 @@ __global__ void __launch_bounds__(256, 2) step_fwd_kernel(const MkdaStepFwd p) {
 // A row of the state is 512 bytes of one value: a warp has 8 values and all 128 key channels of them, a lane four of the channels, and sums over the channels are
 // sums over a warp.  A persistent CTA per SM walks the (sequence, v-head) items: a warp of its own fetches the states of the next two into shared memory while this
 // one's is updated in registers and the last one's is on its way out, and the tokens of the next item are requested before this one's are worked through.
-// (The kernel above read and wrote such a state in 16-byte pieces 512 bytes apart: one token of 8 sequences x 32 heads 15.0 -> 10.6 us, of 64 110 -> 64, of one 11.7
-// -> 8.1 for 4 tokens.  [K,V] states in this form: 8.9 -> 11.3 us, 75.9 -> 75.0, 16 tokens of 64 sequences 218 -> 242; they stay where they are.)
+// Launches one after another over states that are not in L2, x 32 heads, us: by the kernel above, which read and wrote such a state in 16-byte pieces 512 bytes
+// apart, and by this one: one token of 1, 8, 64, 256 sequences 9.7 -> 6.3, 16.0 -> 12.6, 110 -> 61, 422 -> 223; 16 tokens 22.7 -> 15.0, 38.3 -> 30.5, 259 -> 188, 979 -> 727.
+// Among longer sequences, which one warp passes over: 64 of one token and 64 of 200 116 -> 65, 8 and 248 34 -> 28, 24 and 1000 of 70 135 -> 126.
+// ([K,V] states in this form: one token of 8 8.9 -> 11.3, 16 tokens of 64 218 -> 242; they stay where they are.)
 namespace st {
 constexpr int WARPS = 16, THREADS = 32 * (WARPS + 1), STATE = DK * DV;      // floats of a state
 static_assert(STEP_MAX <= WARPS, "a warp prepares one token");

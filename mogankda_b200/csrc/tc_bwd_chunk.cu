@@ -35,9 +35,10 @@
 // middle of this one on, where everything used to wait for its end (232 KB at 44 B per cycle while the epilogue wrote 96 KB, and nothing before).
 // (Operands by token rows, as the forward kernel builds them: k, q and g requested twice, 2.5 k cycles each time, and 144 KB of operands in shared memory.)
 // dW of the next item is computed under the epilogue: Dq and Dk leave their columns early, as the starting values of the row products.
-// An item takes 23 k cycles (26 k before): 1B shape 223 -> 201 us, 64 k packed tokens x 32 heads 3.64 -> 3.29 ms, short documents 267 -> 250 us, fp16 4 x 1000
-// tokens 74 -> 66, scalar gate 4 x 16 k tokens x 16 heads 1313 -> 1249; with the hints of rows and the loads that leave L2 first 193 us, 3.23 ms, 242 us, 63,
-// 1210 (64 k tokens on other boxes, whose clocks differ: 2.84 to 3.12 ms); with waits that do not read the clock first 180 us, 229, 61.
+// An item takes 23 k cycles (26 k by token rows).  Now: 1B shape 180 us, short documents 230, fp16 4 x 1000 tokens 61, 64 k packed tokens x 32 heads 2.84 to 3.26 ms, scalar
+// gate 4 x 16 k tokens x 16 heads 1190 us; where a launch lasts a millisecond its clock is that of the power cap, and the same launch again and again takes 1157 to 1317.
+// The 1B shape on the way here: 223 by token rows, 201 by channels, 193 with the hints of rows and the loads that leave L2 first, 180 with waits that look before they
+// read the clock.
 // Shared memory (KB): S [0,64) | stacked [dO; dW] [64,128): 8 KB pieces, dO even, dW odd -> weights [64,96), scratch in dW pieces | Vd^T [128,160) |
 // dVd^T [160,192), A [192,208) -> dS' [160,224) -> [Qr; beta Kr].
 // TMEM columns: R_I 32 I; [D1; Z] 128, later C_I 128 + {0, 16, 48, 96}; dW 320, later Dq 320 and Dk 384, later column tiles 288 + {0, 16, 48, 96}; Db 448.
@@ -89,13 +90,14 @@ static_assert(sizeof(Scratch) <= 8 * KB, "scratch");
 
 // dO as bf16 rows, as in bwd_dh: full chunks' are fetched from where they are, the others' as tiles, of either the high half only.  The low half below which the
 // low half of dW is stacked is zeros: written once, or, where beta dLs passes through its place, again in each epilogue (two stores per thread; fetched from a
-// block of zeros in L2 the kernel took 1336 us at 4 x 16 k tokens x 16 heads, 1190 to 1235 so, and 1210 to 1255 with tiles).
+// block of zeros in L2 8 % slower).  The products still multiply it.  This kernel gains from rows with one decay per channel (4 x 16 k tokens x 16 heads, in turn: 1527 to 1729 us
+// with tiles, 1431 to 1516 with rows) and not with a scalar gate (1157 to 1317, 1233 to 1373); the pass that writes tiles, 120 us, is gone in both.
 struct NoRows {};
 template <class R> constexpr bool ROWS = std::is_same<R, CUtensorMap>::value;
 
 // dq and dk by token rows, [TT,HK,128] in the type of q and k, instead of fp32 tiles: with one v-head per q/k head and no L2 norm to go back through nothing is
-// left to be done (4 x 16 k tokens x 16 heads, scalar gate: 241 us of qk_grad_finish less; this kernel, half of its dq and dk less to write, takes 1310 us instead
-// of 1270: 256-byte pieces 4 KB apart; with the same stores to one block it takes 1240.  Two lanes that exchange values for 4-byte stores: 1260 where it was 1224)
+// left to be done.  4 x 16 k tokens x 16 heads, scalar gate, in the whole call: this kernel 1190 us (1187 with tiles: half the bytes, but 256-byte pieces 4 KB apart), and
+// 237 us of qk_grad_finish less.  (Two lanes that exchange values for 4-byte stores: 3 % slower.  Rows staged in shared memory have not been tried.)
 struct Finished { void *dq, *dk; };
 
 __device__ __forceinline__ void no_low_half(uint8_t* base) {

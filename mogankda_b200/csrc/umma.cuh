@@ -267,6 +267,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     // 0.7 k cycles of latency and thousands under a saturated memory system, in front of every wait of every kernel.
     // The clock is read once a first attempt has failed: most waits are over when they are made, and those of a thread that issues products or copies
     // follow one another (bwd_chunk 191 -> 180 us at the 1B shape, 241 -> 229 short documents; recur_fwd_pair 347 -> 327, chain_fwd 94 -> 88 and 144 -> 141).
+    // intra_fwd is the mixed one: 3 to 6 % faster with as many q/k heads as v-heads (15.8 k tokens x 16 244 -> 232 us, 32 k 495 -> 461), up to 1 % slower with half
+    // as many (1B shape 118.0 -> 119.4, 32 k tokens x 32 833 -> 837).  One attempt in the loop with the clock behind it is slower in every kernel (327 -> 352, 560 -> 575).
     const uint32_t addr = smem_u32(bar);
     auto done = [&]() {
         uint32_t ok;
